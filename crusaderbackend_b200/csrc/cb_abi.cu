@@ -381,8 +381,8 @@ int cb_gemm(cb_ctx* ctx, int transA, int transB, int M, int N, int K, const floa
     return finish(ctx, "cb_gemm");
 }
 
-// C (+)= sum over `count` operand pairs of op(A[b]) * op(B[b]): the batch is folded into the contraction, one launch on
-// the tensor-core path (the k-blocks walk the pairs); the CUDA-core fp32 path adds the pairs one after the other.
+// C (+)= sum over `count` operand pairs of op(A[b]) * op(B[b]): the batch is folded into the contraction, one launch (the
+// k-blocks walk the pairs).
 int cb_gemm_batch_reduce(cb_ctx* ctx, int transA, int transB, int M, int N, int K, const float* A, int lda, const float* B,
                          int ldb, float* C, int ldc, int count, long long strideA, long long strideB, int accumulate) {
     if (int rc_enter = enter(ctx)) return rc_enter;
@@ -405,18 +405,11 @@ int cb_gemm_batch_reduce(cb_ctx* ctx, int transA, int transB, int M, int N, int 
     g.C = C; g.ldc = ldc; g.strideC = 0; g.out_mode = 0;
     g.accumulate = accumulate ? 1 : 0;
     g.kfold = count;
-    int rc = CB_OK;
-    if (ctx->math != CB_MATH_FP32 && umma_gemm_eligible(g)) {
+    int rc;
+    if (ctx->math != CB_MATH_FP32 && umma_gemm_eligible(g))
         rc = launch_umma_gemm(ctx, g, ctx->math == CB_MATH_3XTF32);
-    } else {
-        g.kfold = 1;
-        for (int b = 0; b < count && rc == CB_OK; ++b) {
-            g.P = B + (long long)b * strideB;
-            g.Q = A + (long long)b * strideA;
-            g.accumulate = (accumulate || b > 0) ? 1 : 0;
-            rc = launch_simt_gemm(ctx, g);
-        }
-    }
+    else
+        rc = launch_simt_gemm(ctx, g);
     if (rc != CB_OK) return rc;
     return finish(ctx, "cb_gemm_batch_reduce");
 }

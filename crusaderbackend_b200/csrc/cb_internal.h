@@ -150,6 +150,8 @@ void filter_cache_destroy(cb_ctx* ctx);
 bool umma_gemm_eligible(const GemmCall& g);
 int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3);
 int launch_simt_gemm(cb_ctx* ctx, const GemmCall& g);
+// Clears the output matrices of a call whose partial products are added into them with atomics.
+int gemm_zero_output(cb_ctx* ctx, const GemmCall& g);
 
 // BatchNorm on one group of samples of a batch (statistics per group; neighbours.cu).
 int bn_fwd_group(cb_ctx* ctx, const float* X, const float* beta, const float* gamma, const float* R, float* Y, int relu, int N,

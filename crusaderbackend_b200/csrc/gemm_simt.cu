@@ -1,0 +1,323 @@
+// CUDA-core fp32 GEMM: CB_MATH_FP32 and every operand pair TMA cannot address, on the shared main loop of simt_core.cuh,
+// and split-K kernels for thin products.
+#include <utility>
+
+#include "simt_core.cuh"
+
+namespace cb {
+namespace {
+
+using simt::kBK;
+
+struct SimtParams {
+    int I, J, K, batch;
+    const float* P; long long ldp, strideP;
+    const float* Q; long long ldq, strideQ;
+    int p_mn, q_mn;
+    float* C; long long ldc, strideC; int out_mode, accumulate, atomic_out;
+    const float* bias_i; const float* bias_j; int relu;
+    int splits, k_per_split;  // k_per_split counts k-slices of 16 (simt_gemm_kernel) or k (thin_gemm_*)
+    int slices;               // k-slices of the whole contraction
+    int per_fold;             // k-slices of one operand pair (batch folded into the contraction), else = slices
+};
+
+// Copies of one operand: element (e, k) at base + e * ld + k (K-major) or base + k * ld + e (MN-major). A slice that lies
+// inside the matrix (`inside`, the same for the whole CTA) needs no tests: pointer and one constant step.
+template <bool MN, int EXT, int NW>
+__device__ __forceinline__ void load_operand(uint32_t dst, const float* base, long long ld, int e0, int E, int k0, int K) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    typedef simt::MnLanes<EXT, NW> M;
+    typedef simt::KLanes<EXT, NW> L;
+    constexpr int kCopies = MN ? M::kCopies : L::kCopies;
+    const int e = MN ? M::e(warp, lane) : L::e(warp, lane, 0), k = MN ? M::k(warp, 0) : L::k(warp, lane);
+    constexpr int kStepE = MN ? 0 : L::kStep, kStepK = MN ? M::kStep : 0;  // between a thread's consecutive copies
+    const float* src = base + (MN ? (long long)(k0 + k) * ld + e0 + e : (long long)(e0 + e) * ld + k0 + k);
+    const long long step = (long long)(MN ? kStepK : kStepE) * ld;
+    dst += simt::slot<EXT>(k, e);
+    if (e0 + EXT <= E && k0 + kBK <= K) {
+#pragma unroll
+        for (int r = 0; r < kCopies; ++r, src += step) simt::cp_async4(dst + simt::slot<EXT>(r * kStepK, r * kStepE), src, true);
+    } else {
+#pragma unroll
+        for (int r = 0; r < kCopies; ++r, src += step) {
+            const bool ok = e0 + e + r * kStepE < E && k0 + k + r * kStepK < K;
+            simt::cp_async4(dst + simt::slot<EXT>(r * kStepK, r * kStepE), ok ? src : base, ok);
+        }
+    }
+}
+
+template <class T, bool P_MN, bool Q_MN>
+struct GemmSource {
+    const SimtParams& p;
+    int b, i0, j0, slice0;
+    __device__ __forceinline__ void begin(int) {}
+    __device__ __forceinline__ void load(int t, uint32_t dst) {
+        int s = slice0 + t, pair = b;
+        if (p.per_fold != p.slices) {
+            pair = s / p.per_fold;
+            s -= pair * p.per_fold;
+        }
+        load_operand<P_MN, T::BM, T::NW>(dst, p.P + pair * p.strideP, p.ldp, i0, p.I, s * kBK, p.K);
+        load_operand<Q_MN, T::BN, T::NW>(dst + simt::kOperandBytes<T::BM>, p.Q + pair * p.strideQ, p.ldq, j0, p.J, s * kBK, p.K);
+    }
+};
+
+// 1000 x 777 x 1501 NN: 267 us with the 64 x 64 tile of scalar loads and 4 x 4 outputs this replaces (8.7 TFLOP/s).
+template <class T, bool P_MN, bool Q_MN>
+__global__ void __launch_bounds__(T::NT, T::kMinCtas) simt_gemm_kernel(const SimtParams p) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int b = blockIdx.z / p.splits, split = blockIdx.z - b * p.splits;
+    const int i0 = blockIdx.x * T::BM, j0 = blockIdx.y * T::BN;
+    GemmSource<T, P_MN, Q_MN> src{p, b, i0, j0, split * p.k_per_split};
+    simt::Acc<T> acc;
+    simt::main_loop<T>(src, min(p.k_per_split, p.slices - src.slice0), (uint32_t)__cvta_generic_to_shared(smem), acc);
+    float* Cb = p.C + (long long)b * p.strideC;
+    simt::for_outputs<T>(acc, i0, j0, [&](int j, int i, float (&v)[4]) {
+        if (j >= p.J) return;
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            if (i + x >= p.I) return;
+            float y = v[x];
+            if (split == 0) {
+                if (p.bias_i) y += p.bias_i[i + x];
+                if (p.bias_j) y += p.bias_j[j];
+            }
+            float* dst = p.out_mode == 0 ? Cb + (long long)j * p.ldc + i + x : Cb + (long long)(i + x) * p.ldc + j;
+            if (p.atomic_out) {
+                atomicAdd(dst, y);
+            } else {
+                if (p.accumulate) y += *dst;
+                if (p.relu) y = fmaxf(y, 0.f);
+                *dst = y;
+            }
+        }
+    });
+}
+
+// Thin products (I <= 16, classifier layers and single samples): bound by reading the wide operand once, so the thin one
+// is staged in shared memory, the contraction is split over enough CTAs to have the whole GPU loading, and the partial
+// sums meet in C through atomics (or stay in one CTA on deterministic contexts). IT: I rounded up to 4, 8 or 16.
+constexpr int kThinK = 256;  // k of a staged piece
+
+template <int IT>
+__device__ __forceinline__ void stage_thin(float (&sP)[IT][kThinK], const SimtParams& p, int k0, int k1) {
+    for (int e = threadIdx.x; e < IT * kThinK; e += 256) {
+        // consecutive threads along whichever index is contiguous in memory
+        const int i = p.p_mn ? e % IT : e / kThinK, kk = p.p_mn ? e / IT : e % kThinK;
+        const int k = k0 + kk;
+        sP[i][kk] = (i < p.I && k < k1) ? (p.p_mn ? p.P[(long long)k * p.ldp + i] : p.P[(long long)i * p.ldp + k]) : 0.f;
+    }
+}
+__device__ __forceinline__ void store_thin(const SimtParams& p, int i, int j, float v, bool first) {
+    if (i >= p.I || j >= p.J) return;
+    if (first) {
+        if (p.bias_i) v += p.bias_i[i];
+        if (p.bias_j) v += p.bias_j[j];
+    }
+    float* dst = p.out_mode == 0 ? p.C + (long long)j * p.ldc + i : p.C + (long long)i * p.ldc + j;
+    if (p.atomic_out) {
+        atomicAdd(dst, v);
+    } else {
+        if (p.accumulate) v += *dst;
+        if (p.relu) v = fmaxf(v, 0.f);
+        *dst = v;
+    }
+}
+
+// Wide operand with k contiguous: lanes walk k, a warp holds 4 rows of it against all IT thin ones, and one butterfly
+// that halves the accumulators at every step replaces a full reduction of each.
+template <int IT>
+__global__ void __launch_bounds__(256) thin_gemm_k_kernel(const SimtParams p) {
+    __shared__ float sP[IT][kThinK];
+    constexpr int NV = 4 * IT;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int j0 = blockIdx.x * 32 + warp * 4;
+    const int k_begin = blockIdx.y * p.k_per_split, k_end = min(p.K, k_begin + p.k_per_split);
+    float acc[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[v] = 0.f;
+    const float* row[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) row[r] = p.Q + (long long)min(j0 + r, p.J - 1) * p.ldq;
+    for (int k0 = k_begin; k0 < k_end; k0 += kThinK) {
+        stage_thin<IT>(sP, p, k0, k_end);
+        __syncthreads();
+#pragma unroll 2
+        for (int kk = lane; kk < kThinK; kk += 32) {
+            float q[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) q[r] = k0 + kk < k_end ? row[r][k0 + kk] : 0.f;
+#pragma unroll
+            for (int i = 0; i < IT; ++i) {
+                const float a = sP[i][kk];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) acc[i * 4 + r] = fmaf(a, q[r], acc[i * 4 + r]);
+            }
+        }
+        __syncthreads();
+    }
+    // after the step with offset o a lane keeps the half of its values that its bit o selects
+    int base = 0, n = NV;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int v = 0; v < NV / 2; ++v)
+                if (v < n) {
+                    const float give = up ? acc[v] : acc[v + n], keep = up ? acc[v + n] : acc[v];
+                    acc[v] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+            base += up ? n : 0;
+        } else {
+            acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+        }
+    }
+    constexpr int kLeft = NV > 32 ? NV / 32 : 1;   // values a lane is left with
+    if (NV < 32 && (lane & (32 / NV - 1)) != 0) return;  // the last steps left equal values in several lanes
+#pragma unroll
+    for (int v = 0; v < kLeft; ++v) store_thin(p, (base + v) >> 2, j0 + ((base + v) & 3), acc[v], blockIdx.y == 0);
+}
+
+// Wide operand with j contiguous: lanes are 32 consecutive j, the eight warps take every eighth k of the piece, and the
+// thin values are shared-memory broadcasts.
+template <int IT>
+__global__ void __launch_bounds__(256) thin_gemm_mn_kernel(const SimtParams p) {
+    __shared__ float sP[IT][kThinK];
+    __shared__ float part[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int j = blockIdx.x * 32 + lane;
+    const int k_begin = blockIdx.y * p.k_per_split, k_end = min(p.K, k_begin + p.k_per_split);
+    float acc[IT];
+#pragma unroll
+    for (int i = 0; i < IT; ++i) acc[i] = 0.f;
+    const float* col = p.Q + min(j, p.J - 1);
+    for (int k0 = k_begin; k0 < k_end; k0 += kThinK) {
+        stage_thin<IT>(sP, p, k0, k_end);
+        __syncthreads();
+#pragma unroll 8
+        for (int kk = warp; kk < kThinK; kk += 8) {
+            const float q = k0 + kk < k_end ? col[(long long)(k0 + kk) * p.ldq] : 0.f;
+#pragma unroll
+            for (int i = 0; i < IT; ++i) acc[i] = fmaf(sP[i][kk], q, acc[i]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+        part[warp][lane] = acc[i];
+        __syncthreads();
+        if (warp == (i & 7)) {
+            float v = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) v += part[w][lane];
+            store_thin(p, i, j, v, blockIdx.y == 0);
+        }
+        __syncthreads();
+    }
+}
+
+cudaError_t launch_thin(cb_ctx* ctx, const SimtParams& sp, dim3 grid) {
+    typedef void (*Kernel)(const SimtParams);
+    static const Kernel kernels[2][3] = {{thin_gemm_k_kernel<4>, thin_gemm_k_kernel<8>, thin_gemm_k_kernel<16>},
+                                         {thin_gemm_mn_kernel<4>, thin_gemm_mn_kernel<8>, thin_gemm_mn_kernel<16>}};
+    kernels[sp.q_mn ? 1 : 0][sp.I <= 4 ? 0 : (sp.I <= 8 ? 1 : 2)]<<<grid, 256, 0, ctx->stream>>>(sp);
+    return cudaGetLastError();
+}
+
+template <class T>
+cudaError_t launch_tile(cb_ctx* ctx, const SimtParams& sp, dim3 grid) {
+    typedef void (*Kernel)(const SimtParams);
+    static const Kernel forms[4] = {simt_gemm_kernel<T, false, false>, simt_gemm_kernel<T, false, true>,
+                                    simt_gemm_kernel<T, true, false>, simt_gemm_kernel<T, true, true>};
+    const Kernel k = forms[(sp.p_mn ? 2 : 0) + (sp.q_mn ? 1 : 0)];
+    cudaError_t e = raise_dynamic_smem_once(k, ctx->device, ctx->max_smem_optin, nullptr);
+    if (e != cudaSuccess) return e;
+    k<<<grid, T::NT, T::kSmem, ctx->stream>>>(sp);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+int gemm_zero_output(cb_ctx* ctx, const GemmCall& g) {
+    // rows of the output as laid out in memory: out_mode 0 -> J rows of I floats, 1 -> I rows of J floats
+    const size_t width = (size_t)(g.out_mode == 0 ? g.I : g.J) * 4;
+    const size_t height = (size_t)(g.out_mode == 0 ? g.J : g.I);
+    for (int b = 0; b < g.batch; ++b) {
+        cudaError_t e = cudaMemset2DAsync(g.C + (long long)b * g.strideC, (size_t)g.ldc * 4, 0, width, height,
+                                          ctx->stream);
+        if (e != cudaSuccess) return check_cuda(ctx, e, "cudaMemset2DAsync(split-K output)");
+    }
+    return CB_OK;
+}
+
+
+int launch_simt_gemm(cb_ctx* ctx, const GemmCall& g_in) {
+    GemmCall g = g_in;
+    if (g.J <= 16 && g.I > 16) {  // put the thin extent on the I side: D'[j][i] with the operands' roles swapped
+        std::swap(g.I, g.J);
+        std::swap(g.P, g.Q); std::swap(g.ldp, g.ldq); std::swap(g.strideP, g.strideQ); std::swap(g.p_mn, g.q_mn);
+        std::swap(g.ep.bias_i, g.ep.bias_j);
+        g.out_mode ^= 1;
+    }
+    const int fold = g.kfold > 1 ? g.kfold : 1;
+    const bool may_split = !ctx->deterministic && g.ep.relu == 0;
+    SimtParams sp{};
+    sp.I = g.I; sp.J = g.J; sp.K = g.K; sp.batch = g.batch;
+    sp.P = g.P; sp.ldp = g.ldp; sp.strideP = g.strideP; sp.p_mn = g.p_mn;
+    sp.Q = g.Q; sp.ldq = g.ldq; sp.strideQ = g.strideQ; sp.q_mn = g.q_mn;
+    sp.C = g.C; sp.ldc = g.ldc; sp.strideC = g.strideC; sp.out_mode = g.out_mode; sp.accumulate = g.accumulate;
+    sp.bias_i = g.ep.bias_i; sp.bias_j = g.ep.bias_j; sp.relu = g.ep.relu;
+    // A tile of 32 or more rows would be mostly padding; below 64 k the tiled kernel's one or two slices cost no more.
+    if (g.I <= 16 && g.batch == 1 && fold == 1 && g.J >= 32 && g.K >= 64) {
+        const int jblocks = (g.J + 31) / 32;
+        int splits = 1;
+        if (may_split) {
+            splits = (2 * ctx->sm_count + jblocks - 1) / jblocks;
+            if (splits > g.K / 64) splits = g.K / 64;
+            if (splits < 1) splits = 1;
+        }
+        int kps = (g.K + splits - 1) / splits;
+        kps = ((kps + 31) / 32) * 32;
+        splits = (g.K + kps - 1) / kps;
+        sp.splits = splits; sp.k_per_split = kps;
+        sp.atomic_out = splits > 1 ? 1 : 0;
+        if (sp.atomic_out && !g.accumulate) {
+            int rc = gemm_zero_output(ctx, g);
+            if (rc != CB_OK) return rc;
+        }
+        if (splits > 65535) return fail(ctx, CB_EUNSUPPORTED, "thin gemm: contraction too long");
+        cudaError_t e = launch_thin(ctx, sp, dim3((unsigned)jblocks, (unsigned)splits));
+        if (e != cudaSuccess) return check_cuda(ctx, e, "thin_gemm_kernel launch");
+        ctx->launches += 1;
+        ctx->last_kernel = "simt_fp32";
+        return CB_OK;
+    }
+    sp.per_fold = (g.K + kBK - 1) / kBK;
+    if ((long long)sp.per_fold * fold > (1LL << 30)) return fail(ctx, CB_EUNSUPPORTED, "simt gemm: contraction longer than 2^34");
+    sp.slices = sp.per_fold * fold;
+    const simt::Choice c = simt::choose_tile(ctx->sm_count, g.I, g.J, sp.slices, g.batch, may_split);
+    sp.splits = c.splits; sp.k_per_split = c.per_split;
+    sp.atomic_out = c.splits > 1 ? 1 : 0;
+    if ((long long)g.batch * c.splits > 65535) return fail(ctx, CB_EUNSUPPORTED, "simt gemm: batch*splits > 65535");
+    if (sp.atomic_out && !g.accumulate) {
+        int rc = gemm_zero_output(ctx, g);
+        if (rc != CB_OK) return rc;
+    }
+    cudaError_t e = cudaSuccess;
+    const int rc_grid = simt::with_tile(c.tile, [&](auto tile) {
+        typedef decltype(tile) T;
+        const long long gy = ((long long)g.J + T::BN - 1) / T::BN;
+        if (gy > 65535) return fail(ctx, CB_EUNSUPPORTED, "simt gemm: more than 65535 column tiles");
+        e = launch_tile<T>(ctx, sp, dim3((unsigned)((g.I + T::BM - 1) / T::BM), (unsigned)gy, (unsigned)(g.batch * c.splits)));
+        return (int)CB_OK;
+    });
+    if (rc_grid != CB_OK) return rc_grid;
+    if (e != cudaSuccess) return check_cuda(ctx, e, "simt_gemm_kernel launch");
+    ctx->launches += 1;
+    ctx->last_kernel = "simt_fp32";
+    return CB_OK;
+}
+
+}  // namespace cb

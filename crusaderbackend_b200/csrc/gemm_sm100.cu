@@ -418,147 +418,6 @@ __global__ void __launch_bounds__(X3 ? 64 + 32 * kEpiWarps + 128 : 64 + 32 * kEp
     }
 }
 
-// ------------------------------------------------------------------ CUDA-core fp32 kernel (any shape / alignment)
-// 64x64 tile, 16-deep k slices, 256 threads x (4x4) outputs. Exact fp32 FMA in k order.
-struct SimtParams {
-    int I, J, K, batch;
-    const float* P; long long ldp, strideP; int p_mn;
-    const float* Q; long long ldq, strideQ; int q_mn;
-    float* C; long long ldc, strideC; int out_mode, accumulate, atomic_out;
-    const float* bias_i; const float* bias_j; int relu;
-    int splits, k_per_split;
-};
-
-__global__ void __launch_bounds__(256) simt_gemm_kernel(const SimtParams p) {
-    __shared__ float sP[16][64 + 4];
-    __shared__ float sQ[16][64 + 4];
-    const int b = blockIdx.z / p.splits;
-    const int split = blockIdx.z - b * p.splits;
-    const int i0 = blockIdx.x * 64, j0 = blockIdx.y * 64;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const float* Pb = p.P + (long long)b * p.strideP;
-    const float* Qb = p.Q + (long long)b * p.strideQ;
-    const int k_begin = split * p.k_per_split;
-    const int k_end = min(p.K, k_begin + p.k_per_split);
-    float acc[4][4] = {};
-    for (int k0 = k_begin; k0 < k_end; k0 += 16) {
-        for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-            int kk, r;
-            if (p.p_mn) { r = e & 63; kk = e >> 6; } else { kk = e & 15; r = e >> 4; }
-            const int i = i0 + r, k = k0 + kk;
-            float v = 0.f;
-            if (i < p.I && k < k_end) v = p.p_mn ? Pb[(long long)k * p.ldp + i] : Pb[(long long)i * p.ldp + k];
-            sP[kk][r] = v;
-        }
-        for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-            int kk, r;
-            if (p.q_mn) { r = e & 63; kk = e >> 6; } else { kk = e & 15; r = e >> 4; }
-            const int j = j0 + r, k = k0 + kk;
-            float v = 0.f;
-            if (j < p.J && k < k_end) v = p.q_mn ? Qb[(long long)k * p.ldq + j] : Qb[(long long)j * p.ldq + k];
-            sQ[kk][r] = v;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            float a[4], c[4];
-#pragma unroll
-            for (int x = 0; x < 4; ++x) { a[x] = sP[kk][tx + 16 * x]; c[x] = sQ[kk][ty + 16 * x]; }
-#pragma unroll
-            for (int x = 0; x < 4; ++x)
-#pragma unroll
-                for (int y = 0; y < 4; ++y) acc[x][y] = fmaf(a[x], c[y], acc[x][y]);
-        }
-        __syncthreads();
-    }
-    float* Cb = p.C + (long long)b * p.strideC;
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) {
-            const int i = i0 + tx + 16 * x, j = j0 + ty + 16 * y;
-            if (i < p.I && j < p.J) {
-                float v = acc[x][y];
-                if (split == 0) {
-                    if (p.bias_i) v += p.bias_i[i];
-                    if (p.bias_j) v += p.bias_j[j];
-                }
-                float* dst = p.out_mode == 0 ? Cb + (long long)j * p.ldc + i : Cb + (long long)i * p.ldc + j;
-                if (p.atomic_out) {
-                    atomicAdd(dst, v);
-                } else {
-                    if (p.accumulate) v += *dst;
-                    if (p.relu) v = fmaxf(v, 0.f);
-                    *dst = v;
-                }
-            }
-        }
-}
-
-// Thin products (I <= 16, e.g. the 128 x 10 x 4096 dense-layer shape): HBM/latency-bound, so K is split over many CTAs,
-// one warp per output row j with lanes striding k (128-bit-coalesced reads of Q when it is K-major), the I thin
-// outputs per lane reduced with warp shuffles and added atomically into C (or stored when K is not split).
-__global__ void __launch_bounds__(256) skinny_gemm_kernel(const SimtParams p) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int j = blockIdx.x * 8 + warp;
-    if (j >= p.J) return;
-    const int split = blockIdx.y;
-    const int k0 = split * p.k_per_split, k1 = min(p.K, k0 + p.k_per_split);
-    float acc[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-    for (int k = k0 + lane; k < k1; k += 32) {
-        const float q = p.q_mn ? p.Q[(long long)k * p.ldq + j] : p.Q[(long long)j * p.ldq + k];
-        if (p.p_mn) {
-            const float* pr = p.P + (long long)k * p.ldp;
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                if (i < p.I) acc[i] = fmaf(q, pr[i], acc[i]);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                if (i < p.I) acc[i] = fmaf(q, p.P[(long long)i * p.ldp + k], acc[i]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        float v = acc[i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        acc[i] = v;
-    }
-    if (lane < p.I) {
-        float v = 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (i == lane) v = acc[i];
-        if (split == 0) {
-            if (p.bias_i) v += p.bias_i[lane];
-            if (p.bias_j) v += p.bias_j[j];
-        }
-        float* dst = p.out_mode == 0 ? p.C + (long long)j * p.ldc + lane : p.C + (long long)lane * p.ldc + j;
-        if (p.atomic_out) {
-            atomicAdd(dst, v);
-        } else {
-            if (p.accumulate) v += *dst;
-            if (p.relu) v = fmaxf(v, 0.f);
-            *dst = v;
-        }
-    }
-}
-
-int zero_output(cb_ctx* ctx, const GemmCall& g) {
-    // rows of the output as laid out in memory: out_mode 0 -> J rows of I floats, 1 -> I rows of J floats
-    const size_t width = (size_t)(g.out_mode == 0 ? g.I : g.J) * 4;
-    const size_t height = (size_t)(g.out_mode == 0 ? g.J : g.I);
-    for (int b = 0; b < g.batch; ++b) {
-        cudaError_t e = cudaMemset2DAsync(g.C + (long long)b * g.strideC, (size_t)g.ldc * 4, 0, width, height,
-                                          ctx->stream);
-        if (e != cudaSuccess) return check_cuda(ctx, e, "cudaMemset2DAsync(split-K output)");
-    }
-    return CB_OK;
-}
-
 template <bool P_MN, bool Q_MN>
 cudaError_t launch_variant(cb_ctx* ctx, bool x3, dim3 grid, size_t smem, const CUtensorMap& tp, const CUtensorMap& tq,
                            const GemmParams& gp) {
@@ -718,7 +577,7 @@ int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3) {
     }
 
     if (gp.atomic_out && !g.accumulate) {
-        int rc = zero_output(ctx, g);
+        int rc = gemm_zero_output(ctx, g);
         if (rc != CB_OK) return rc;
     }
 
@@ -734,78 +593,6 @@ int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3) {
     if (e != cudaSuccess) return check_cuda(ctx, e, "umma_gemm_kernel launch");
     ctx->launches += 1;
     ctx->last_kernel = x3 ? "umma_3xtf32" : "umma_tf32";
-    return CB_OK;
-}
-
-int launch_simt_gemm(cb_ctx* ctx, const GemmCall& g_in) {
-    GemmCall g = g_in;
-    if (g.J <= 16 && g.I > 16) {  // put the thin extent on the I side: D'[j][i] with the operands' roles swapped
-        std::swap(g.I, g.J);
-        std::swap(g.P, g.Q); std::swap(g.ldp, g.ldq); std::swap(g.strideP, g.strideQ); std::swap(g.p_mn, g.q_mn);
-        std::swap(g.ep.bias_i, g.ep.bias_j);
-        g.out_mode ^= 1;
-    }
-    if (g.I <= 16 && g.batch == 1 && g.J >= 32 && g.K >= 256) {
-        SimtParams sp{};
-        sp.I = g.I; sp.J = g.J; sp.K = g.K; sp.batch = 1;
-        sp.P = g.P; sp.ldp = g.ldp; sp.p_mn = g.p_mn;
-        sp.Q = g.Q; sp.ldq = g.ldq; sp.q_mn = g.q_mn;
-        sp.C = g.C; sp.ldc = g.ldc; sp.out_mode = g.out_mode; sp.accumulate = g.accumulate;
-        sp.bias_i = g.ep.bias_i; sp.bias_j = g.ep.bias_j; sp.relu = g.ep.relu;
-        const int jblocks = (g.J + 7) / 8;
-        int splits = 1;
-        if (!ctx->deterministic && g.ep.relu == 0) {
-            splits = (2 * ctx->sm_count + jblocks - 1) / jblocks;
-            if (splits > g.K / 128) splits = g.K / 128;
-            if (splits < 1) splits = 1;
-        }
-        int kps = (g.K + splits - 1) / splits;
-        kps = ((kps + 31) / 32) * 32;
-        splits = (g.K + kps - 1) / kps;
-        sp.splits = splits; sp.k_per_split = kps;
-        sp.atomic_out = splits > 1 ? 1 : 0;
-        if (sp.atomic_out && !g.accumulate) {
-            int rc = zero_output(ctx, g);
-            if (rc != CB_OK) return rc;
-        }
-        skinny_gemm_kernel<<<dim3(jblocks, splits), 256, 0, ctx->stream>>>(sp);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return check_cuda(ctx, e, "skinny_gemm_kernel launch");
-        ctx->launches += 1;
-        ctx->last_kernel = "simt_fp32";
-        return CB_OK;
-    }
-    SimtParams sp{};
-    sp.I = g.I; sp.J = g.J; sp.K = g.K; sp.batch = g.batch;
-    sp.P = g.P; sp.ldp = g.ldp; sp.strideP = g.strideP; sp.p_mn = g.p_mn;
-    sp.Q = g.Q; sp.ldq = g.ldq; sp.strideQ = g.strideQ; sp.q_mn = g.q_mn;
-    sp.C = g.C; sp.ldc = g.ldc; sp.strideC = g.strideC; sp.out_mode = g.out_mode;
-    sp.accumulate = g.accumulate;
-    sp.bias_i = g.ep.bias_i; sp.bias_j = g.ep.bias_j; sp.relu = g.ep.relu;
-    const int ti = (g.I + 63) / 64, tj = (g.J + 63) / 64;
-    long long tiles = (long long)ti * tj * g.batch;
-    int splits = 1;
-    if (!ctx->deterministic && g.ep.relu == 0 && tiles * 2 <= ctx->sm_count && g.K >= 512) {
-        splits = (int)(2LL * ctx->sm_count / tiles);
-        if (splits > g.K / 128) splits = g.K / 128;
-        if (splits < 1) splits = 1;
-    }
-    int kps = (g.K + splits - 1) / splits;
-    kps = ((kps + 15) / 16) * 16;
-    splits = (g.K + kps - 1) / kps;
-    sp.splits = splits; sp.k_per_split = kps;
-    sp.atomic_out = splits > 1 ? 1 : 0;
-    if ((long long)g.batch * splits > 65535) return fail(ctx, CB_EUNSUPPORTED, "simt gemm: batch*splits > 65535");
-    if (sp.atomic_out && !g.accumulate) {
-        int rc = zero_output(ctx, g);
-        if (rc != CB_OK) return rc;
-    }
-    dim3 grid(ti, tj, g.batch * splits);
-    simt_gemm_kernel<<<grid, 256, 0, ctx->stream>>>(sp);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return check_cuda(ctx, e, "simt_gemm_kernel launch");
-    ctx->launches += 1;
-    ctx->last_kernel = "simt_fp32";
     return CB_OK;
 }
 

@@ -229,3 +229,14 @@ def test_bias_add_and_bias_grad(torch_cuda, ctxs):
     assert orc.max_err_norm(db.cpu().numpy(), orc.conv_bias_grad(Y0) + 1.0) <= 2e-6
     ctx.convBiasGrad(torch.from_numpy(Y0).cuda(), db, accumulate=False)
     assert orc.max_err_norm(db.cpu().numpy(), orc.conv_bias_grad(Y0)) <= 2e-6
+
+
+@pytest.mark.parametrize("geo", [(1, 1, 5, 5, 1, 1, 1, 0), (3, 5, 8, 9, 33, 3, 1, 1), (2, 7, 13, 11, 31, 3, 2, 1), (2, 4, 10, 10, 65, 2, 3, 0),
+                                 (1, 2, 20, 21, 3, 17, 1, 8), (1, 3, 33, 31, 8, 7, 2, 3), (4, 33, 7, 7, 64, 3, 1, 1), (2, 6, 9, 9, 5, 1, 3, 0)])
+def test_cuda_core_convolution_tiles_and_phases(torch_cuda, ctxs, geo):
+    """The fp32 kernels on pixel counts, channel counts and contraction lengths around their tiles, strides whose phases
+    have different taps (or none), and filters on both sides of the 15-tap limit of the tap masks."""
+    N, IC, H, W, OC, F, s, p = geo
+    c = conv_case(("simt", geo), N, IC, H, W, OC, F, s, p, bias=True)
+    kern = check_three_passes(torch_cuda, ctxs["fp32"], "fp32", c, dW0=orc.normal((OC, IC, F, F), "simt", geo, "dW0"))
+    assert all(k == "simt_fp32" for k in kern), kern

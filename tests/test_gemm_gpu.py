@@ -276,3 +276,22 @@ def test_golden_reference_sgemm_nta(torch_cuda, ctxs, golden):
         A, B, Cc = (torch.from_numpy(x[k]).cuda() for k in ("A", "B", "C0"))
         ctxs["3xtf32"].sgemmNTA(A, B, Cc)
         assert orc.max_err_norm(Cc.cpu().numpy(), golden[name + "/C"]) <= 2e-5, name
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("M,N,K", [(64, 64, 16), (65, 33, 17), (33, 129, 15), (128, 128, 63), (129, 31, 65), (1, 300, 1000), (512, 65, 257),
+                                   (700, 700, 49), (16, 97, 64), (4, 33, 255), (9, 260, 1025), (2, 1025, 4097)])
+def test_cuda_core_tiles_at_their_edges(torch_cuda, ctxs, M, N, K, form):
+    """The fp32 kernel's tiles (64 or 128 rows, 32 to 128 columns, slices of 16 k, contraction split or whole) one element
+    below, at and above their sizes, with and without splitting (deterministic contexts never split), and the thin kernels
+    (an extent of at most 16) around their pieces of 256 k and groups of 4, 8 and 16."""
+    torch = torch_cuda
+    A, B = make_operands(M, N, K, form, ("edges", M, N, K, form))
+    ref = orc.gemm_f64(A, B, *FORMS[form])
+    ctx = ctxs["fp32"]
+    for det in (False, True):
+        ctx.set_deterministic(det)
+        got = run_gemm(torch, ctx, A, B, M, N, form)
+        ctx.set_deterministic(False)
+        assert ctx.last_kernel == "simt_fp32"
+        assert orc.max_err_norm(got, ref) <= TOL["fp32"]
