@@ -1,7 +1,8 @@
 """Thin Python face of the C ABI for tests and benchmarks.
 
 torch is used only to own device memory and streams; every computation goes through
-libcrusader_b200.so. Function names follow the reference's seblas operations
+libcrusader_b200.so, called by the extension module _native (csrc/bind.cpp), which reads the tensors'
+extents, strides and pointers natively. Function names follow the reference's seblas operations
 (seblas/operations/cuGEMM.cuh:12-21, cuConv.cuh:20-42, cuLinear.cuh:14-18).
 """
 from __future__ import annotations
@@ -16,12 +17,20 @@ from ._lib import CB_MATH_3XTF32, CB_MATH_FP32, CB_MATH_TF32, CrusaderError
 MATH_MODES = {"tf32": CB_MATH_TF32, "3xtf32": CB_MATH_3XTF32, "fp32": CB_MATH_FP32}
 
 
-def _ptr(t: torch.Tensor | None) -> int | None:
-    if t is None:
-        return None
-    if not t.is_cuda or t.dtype != torch.float32:
-        raise ValueError("operands must be fp32 CUDA tensors")
-    return t.data_ptr()
+_native = None
+
+
+def _load_native(lib: C.CDLL):
+    """The extension module, attached to the loaded library; missing, it is an error like a missing library."""
+    global _native
+    if _native is None:
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise RuntimeError("crusaderbackend_b200._native has not been built (python -m crusaderbackend_b200.build)") from e
+        module.attach(lib._handle, CrusaderError)
+        _native = module
+    return _native
 
 
 class Context:
@@ -29,6 +38,7 @@ class Context:
 
     def __init__(self, device: int = 0, math: str = "tf32", sync: bool = False, stream: torch.cuda.Stream | None = None):
         self.lib = _lib.load()
+        self._native = _load_native(self.lib)
         if not torch.cuda.is_available():
             raise RuntimeError("crusader_b200 needs a CUDA device; there is no CPU path")
         self.device = device
@@ -40,6 +50,7 @@ class Context:
         if rc != 0:
             raise CrusaderError(rc, "cb_create failed")
         self.h = h
+        self._hv = h.value  # what the native calls take
         self.set_math(math)
         self.set_sync(sync)
 
@@ -52,6 +63,7 @@ class Context:
         if getattr(self, "h", None):
             self.lib.cb_destroy(self.h)
             self.h = None
+            self._hv = 0
 
     def __del__(self):
         try:
@@ -91,195 +103,110 @@ class Context:
              accumulate: bool = False) -> torch.Tensor:
         """C = op(A) @ op(B) (+ C). 2-D row-major operands, or 3-D with a leading batch dimension
         (a 2-D A or B is shared by every batch, as in seblas::sgemm)."""
-        def mat(t):
-            if t.dim() == 2:
-                return 1, t.shape[0], t.shape[1], t.stride(0), 0
-            return t.shape[0], t.shape[1], t.shape[2], t.stride(1), t.stride(0)
-        for t in (A, B, C_):
-            if t.stride(-1) != 1:
-                raise ValueError("operands must be row-major (unit inner stride)")
-        ba, ra, ca, lda, sa = mat(A)
-        bb, rb, cb, ldb, sb = mat(B)
-        bc, M, N, ldc, sc = mat(C_)
-        K = ra if transA else ca
-        if (ca if transA else ra) != M or (cb if transB else rb) != K or (rb if transB else cb) != N:
-            raise ValueError("gemm: shapes do not agree")
-        batch = bc
-        if ba not in (1, batch) or bb not in (1, batch):
-            raise ValueError("gemm: batch sizes do not agree")
-        self._check(self.lib.cb_gemm(self.h, int(transA), int(transB), M, N, K, _ptr(A), lda, _ptr(B), ldb,
-                                     _ptr(C_), ldc, batch, sa if ba == batch else 0, sb if bb == batch else 0, sc,
-                                     int(accumulate)))
-        return C_
+        return self._native.gemm(self._hv, A, B, C_, transA, transB, accumulate)
 
     # ---- seblas-named GEMMs
     def sgemm(self, A, B, Cout):
         """seblas::sgemm: C[b] = A @ B[b] (seblas/operations/cuGEMM.cu:1649)."""
-        return self.gemm(A, B, Cout)
+        return self._native.gemm(self._hv, A, B, Cout, False, False, False)
 
     def sgemmTN(self, A, B, Cout):
         """seblas::sgemmTN: C[b] = A^T @ B[b], A stored K x M (seblas/operations/cuGEMM.cu:1667)."""
-        return self.gemm(A, B, Cout, transA=True)
+        return self._native.gemm(self._hv, A, B, Cout, True, False, False)
 
     def sgemmNT(self, A, B, Cout):
         """seblas::sgemmNT: C = A @ B^T, B stored N x K (seblas/operations/cuGEMM.cu:1685)."""
-        return self.gemm(A, B, Cout, transB=True)
+        return self._native.gemm(self._hv, A, B, Cout, False, True, False)
 
     def sgemmNTA(self, A, B, Cout):
         """seblas::sgemmNTA: C += sum over n of A[n] @ B[n]^T, A n x M x K, B n x N x K, C M x N
         (seblas/operations/cuGEMM.cu:1701); the batch is folded into the contraction, one launch."""
-        if A.dim() != 3 or B.dim() != 3 or Cout.dim() != 2:
-            raise ValueError("sgemmNTA: A and B are 3-D (batch first), C is 2-D")
-        for t in (A, B, Cout):
-            if t.stride(-1) != 1:
-                raise ValueError("operands must be row-major (unit inner stride)")
-        n, M, K = A.shape
-        if B.shape[0] != n or B.shape[2] != K or tuple(Cout.shape) != (M, B.shape[1]):
-            raise ValueError("sgemmNTA: shapes do not agree")
-        self._check(self.lib.cb_gemm_batch_reduce(self.h, 0, 1, M, B.shape[1], K, _ptr(A), A.stride(1), _ptr(B), B.stride(1),
-                                                  _ptr(Cout), Cout.stride(0), n, A.stride(0), B.stride(0), 1))
-        return Cout
+        return self._native.gemm_nta(self._hv, A, B, Cout)
 
     # ---- convolution: arguments in the order of seblas::conv / convDerive / convError
-    @staticmethod
-    def _geo(W, X, stride, pad):
-        N, IC, IH, IW = X.shape
-        OC, IC2, FH, FW = W.shape
-        if IC2 != IC:
-            raise ValueError("conv: channel counts do not agree")
-        return [N, IC, IH, IW, OC, FH, FW, stride[0], stride[1], pad[0], pad[1]]
-
     def conv(self, A, B, Cout, strideH=1, strideW=1, padH=0, padW=0, biases=None, relu=False):
         """seblas::conv(A=filters OC x IC x FH x FW, B=input N x IC x IH x IW, C=output), seblas/operations/cuConv.cu:757."""
-        geo = self._geo(A, B, (strideH, strideW), (padH, padW))
-        self._check(self.lib.cb_conv_fwd(self.h, _ptr(A), _ptr(B), _ptr(Cout), _ptr(biases), *geo, int(relu)))
-        return Cout
+        return self._native.conv(self._hv, A, B, Cout, strideH, strideW, padH, padW, biases, relu)
 
     def convDerive(self, A, B, Cout, strideH=1, strideW=1, padH=0, padW=0):
         """seblas::convDerive(A=filters, B=dY, C=dX), seblas/operations/cuConv.cu:774."""
-        geo = self._geo(A, Cout, (strideH, strideW), (padH, padW))
-        self._check(self.lib.cb_conv_dgrad(self.h, _ptr(A), _ptr(B), _ptr(Cout), *geo))
-        return Cout
+        return self._native.conv_dgrad(self._hv, A, B, Cout, strideH, strideW, padH, padW)
 
     def convError(self, A, B, Cout, strideH=1, strideW=1, padH=0, padW=0, accumulate=True):
         """seblas::convError(A=dY, B=input, C=filter gradient, accumulated), seblas/operations/cuConv.cu:793.
         Returns A, as the reference does."""
-        geo = self._geo(Cout, B, (strideH, strideW), (padH, padW))
-        self._check(self.lib.cb_conv_wgrad(self.h, _ptr(A), _ptr(B), _ptr(Cout), *geo, int(accumulate)))
-        return A
+        return self._native.conv_wgrad(self._hv, A, B, Cout, strideH, strideW, padH, padW, accumulate)
 
     def convBias(self, Y, biases):
-        N, Cc, H, W = Y.shape
-        self._check(self.lib.cb_conv_bias(self.h, _ptr(Y), _ptr(biases), N, Cc, H * W))
-        return Y
+        return self._native.conv_bias(self._hv, Y, biases)
 
     def convBiasGrad(self, dY, db, accumulate=False):
-        N, Cc, H, W = dY.shape
-        self._check(self.lib.cb_conv_bias_grad(self.h, _ptr(dY), _ptr(db), N, Cc, H * W, int(accumulate)))
-        return db
+        return self._native.conv_bias_grad(self._hv, dY, db, accumulate)
 
     # ---- linear: seblas::linear / linearXGrad / linearParamGrad (seblas/operations/cuLinear.cu:1052-1115)
     def linear(self, X, W, B, Y):
-        batch, IN = X.shape[0], X.numel() // X.shape[0]
-        self._check(self.lib.cb_linear_fwd(self.h, _ptr(X), _ptr(W), _ptr(B), _ptr(Y), batch, IN, W.shape[-2]))
-        return Y
+        return self._native.linear(self._hv, X, W, B, Y)
 
     def linearXGrad(self, dY, W, dX):
-        batch = dX.shape[0]
-        self._check(self.lib.cb_linear_xgrad(self.h, _ptr(dY), _ptr(W), _ptr(dX), batch, W.shape[-1], W.shape[-2]))
-        return dX
+        return self._native.linear_xgrad(self._hv, dY, W, dX)
 
     def linearParamGrad(self, dY, X, dW, dB):
-        batch = X.shape[0]
-        self._check(self.lib.cb_linear_paramgrad(self.h, _ptr(dY), _ptr(X), _ptr(dW), _ptr(dB), batch, dW.shape[-1],
-                                                 dW.shape[-2]))
-        return dW
+        return self._native.linear_paramgrad(self._hv, dY, X, dW, dB)
 
     # ---- neighbours
     def batchNorm(self, X, beta, gamma, mean, var, Y, xHat):
-        N = X.shape[0]
-        self._check(self.lib.cb_bn_fwd(self.h, _ptr(X), _ptr(beta), _ptr(gamma), _ptr(mean), _ptr(var), _ptr(Y),
-                                       _ptr(xHat), N, X.numel() // N))
-        return Y
+        return self._native.bn_fwd(self._hv, X, beta, gamma, mean, var, Y, xHat)
 
     def batchNormGrad(self, dY, gamma, X, dX):
-        N = X.shape[0]
-        self._check(self.lib.cb_bn_bwd(self.h, _ptr(dY), _ptr(gamma), _ptr(X), _ptr(dX), N, X.numel() // N))
-        return dX
+        return self._native.bn_bwd(self._hv, dY, gamma, X, dX)
 
     def batchNormParamGrads(self, dY, xHat, dGamma, dBeta):
-        N = dY.shape[0]
-        self._check(self.lib.cb_bn_paramgrad(self.h, _ptr(dY), _ptr(xHat), _ptr(dGamma), _ptr(dBeta), N,
-                                             dY.numel() // N))
+        return self._native.bn_paramgrad(self._hv, dY, xHat, dGamma, dBeta)
 
     def batchNormGradFused(self, dY, gamma, X, dX, dGamma, dBeta, relu_out=None):
-        N = X.shape[0]
-        self._check(self.lib.cb_bn_bwd_fused(self.h, _ptr(dY), _ptr(gamma), _ptr(X), _ptr(dX), _ptr(dGamma), _ptr(dBeta),
-                                             _ptr(relu_out), N, X.numel() // N))
-        return dX
+        return self._native.bn_bwd_fused(self._hv, dY, gamma, X, dX, dGamma, dBeta, relu_out)
 
     def batchNormRelu(self, X, beta, gamma, Y):
-        N = X.shape[0]
-        self._check(self.lib.cb_bn_fwd_relu(self.h, _ptr(X), _ptr(beta), _ptr(gamma), _ptr(Y), N, X.numel() // N))
-        return Y
+        return self._native.bn_fwd_relu(self._hv, X, beta, gamma, Y)
 
     def addRelu(self, A, B, Out):
-        self._check(self.lib.cb_add_relu(self.h, _ptr(A), _ptr(B), _ptr(Out), A.numel()))
-        return Out
+        return self._native.add_relu(self._hv, A, B, Out)
 
     def reluGrad2(self, Y, dY, dA, dB=None):
-        self._check(self.lib.cb_relu_grad2(self.h, _ptr(Y), _ptr(dY), _ptr(dA), _ptr(dB), Y.numel()))
-        return dA
+        return self._native.relu_grad2(self._hv, Y, dY, dA, dB)
 
     def relu(self, X, Y):
-        self._check(self.lib.cb_relu(self.h, _ptr(X), _ptr(Y), X.numel()))
-        return Y
+        return self._native.relu(self._hv, X, Y)
 
     def reluGradFast(self, X, dY, dX):
-        self._check(self.lib.cb_relu_grad(self.h, _ptr(X), _ptr(dY), _ptr(dX), X.numel()))
-        return dX
+        return self._native.relu_grad(self._hv, X, dY, dX)
 
     def tensor_op(self, op: int, A, B=None, scalar: float = 0.0):
-        self._check(self.lib.cb_tensor_op(self.h, op, _ptr(A), _ptr(B), scalar, A.numel()))
-        return A
+        return self._native.tensor_op(self._hv, op, A, B, scalar)
 
     def grad_handover(self, dA, dAReserve):
-        self._check(self.lib.cb_grad_handover(self.h, _ptr(dA), _ptr(dAReserve), dA.numel()))
-        return dA
+        return self._native.grad_handover(self._hv, dA, dAReserve)
 
     def avgPool(self, X, Y, rangeH=2, rangeW=2):
-        N, Cc, H, W = X.shape
-        self._check(self.lib.cb_avgpool(self.h, _ptr(X), _ptr(Y), N * Cc, H, W, rangeH, rangeW))
-        return Y
+        return self._native.avgpool(self._hv, X, Y, rangeH, rangeW)
 
     def avgPoolBack(self, dX, dY, rangeH=2, rangeW=2):
-        N, Cc, H, W = dX.shape
-        self._check(self.lib.cb_avgpool_back(self.h, _ptr(dX), _ptr(dY), N * Cc, H, W, rangeH, rangeW))
-        return dX
+        return self._native.avgpool_back(self._hv, dX, dY, rangeH, rangeW)
 
     def globalAvgPool(self, X, Y):
-        N, Cc, H, W = X.shape
-        self._check(self.lib.cb_global_avgpool(self.h, _ptr(X), _ptr(Y), N * Cc, H * W))
-        return Y
+        return self._native.global_avgpool(self._hv, X, Y)
 
     def globalAvgPoolBack(self, dX, dY):
-        N, Cc, H, W = dX.shape
-        self._check(self.lib.cb_global_avgpool_back(self.h, _ptr(dX), _ptr(dY), N * Cc, H * W))
-        return dX
+        return self._native.global_avgpool_back(self._hv, dX, dY)
 
     def softmax(self, A, out, step=None):
-        rows = A.shape[0]
-        step = step or A.numel() // rows
-        self._check(self.lib.cb_softmax(self.h, _ptr(A), _ptr(out), A.numel() // step, step))
-        return out
+        return self._native.softmax(self._hv, A, out, step or 0)
 
     def crossEntropy(self, Y, labels, dY=None, loss=None):
-        self._check(self.lib.cb_cross_entropy(self.h, _ptr(Y), _ptr(labels), _ptr(dY), _ptr(loss), Y.numel()))
-        return loss
+        return self._native.cross_entropy(self._hv, Y, labels, dY, loss)
 
     def momentumApply(self, X, Xgrad, V, lr, beta, l2=0.0, is_weight=False):
-        self._check(self.lib.cb_momentum(self.h, _ptr(X), _ptr(Xgrad), _ptr(V), X.numel(), lr, beta, l2,
-                                         int(is_weight)))
+        return self._native.momentum(self._hv, X, Xgrad, V, lr, beta, l2, is_weight)
 
     def momentumApplyMulti(self, params, grads, moms, is_weight, lr, beta, l2):
         n = len(params)

@@ -9,6 +9,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -17,6 +18,8 @@ CSRC = PKG / "csrc"
 LIB_DIR = PKG / "lib"
 OBJ_DIR = PKG / "build"
 LIB_PATH = LIB_DIR / "libcrusader_b200.so"
+BIND_SRC = CSRC / "bind.cpp"
+BIND_PATH = PKG / ("_native" + sysconfig.get_config_var("EXT_SUFFIX"))  # the CPython face (csrc/bind.cpp)
 
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
@@ -46,10 +49,32 @@ def needs_build() -> bool:
     return any(p.stat().st_mtime > t for p in _sources() + _headers())
 
 
+def build_bind(force: bool = False, verbose: bool = False) -> Path:
+    """Compiles the CPython extension module. It is host code only: torch's headers for reading tensors, the C ABI's
+    header for the signatures; the CUDA library itself is resolved at run time."""
+    import torch
+    sources = [BIND_SRC, PKG.parent / "include" / "crusader_b200.h"]
+    if not force and BIND_PATH.exists() and BIND_PATH.stat().st_mtime > max(p.stat().st_mtime for p in sources):
+        return BIND_PATH
+    inc = Path(torch.__file__).resolve().parent / "include"
+    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-isystem", str(inc), "-isystem", str(inc / "torch" / "csrc" / "api" / "include"),
+           "-isystem", sysconfig.get_paths()["include"], str(BIND_SRC), "-o", str(BIND_PATH),
+           "-L", str(inc.parent / "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {BIND_SRC.name}:\n{r.stdout}\n{r.stderr}")
+    return BIND_PATH
+
+
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False, trace: bool = False) -> Path:
     """trace=True builds a second library, libcrusader_b200_trace.so, with the kernels' time-stamp instrumentation
     (-DCB_TRACE) compiled in; the product library never carries it."""
     lib_path = LIB_DIR / "libcrusader_b200_trace.so" if trace else LIB_PATH
+    if not trace:
+        build_bind(force, verbose)
     if not force and not trace and not needs_build():
         return LIB_PATH
     nvcc = _nvcc()

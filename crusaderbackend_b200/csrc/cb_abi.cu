@@ -144,21 +144,23 @@ int encode_tmap(cb_ctx* ctx, CUtensorMap* out, const void* base, int rank, const
     for (int i = 0; i + 1 < rank; ++i) gs[i] = strides_bytes[i];
     // The encoding is a pure function of these values: a context keeps what it has encoded (bounded: a caller that
     // walks through ever new addresses starts over at 4096 entries).
-    struct Key {
-        const void* base;
-        cuuint64_t gd[5], gs[4];
-        cuuint32_t bd[5], es[5];
-        int rank, swizzle;
-    } key{};  // value-initialised: padding bytes are zero, the bytes are the hash key
-    std::string kbytes;
+    TmapKey key{};
+    key.w[0] = (uint64_t)reinterpret_cast<uintptr_t>(base);
+    key.w[1] = (uint64_t)rank << 32 | (uint64_t)swizzle_bytes;
+    for (int i = 0; i < 5; ++i) {
+        key.w[2 + i] = gd[i];
+        key.w[7 + i] = (uint64_t)bd[i] << 32 | es[i];
+    }
+    for (int i = 0; i < 4; ++i) key.w[12 + i] = gs[i];
+    uint64_t hash = 0;
+    for (uint64_t w : key.w) {
+        hash = (hash ^ w) * 0x9E3779B97F4A7C15ull;
+        hash ^= hash >> 29;
+    }
     if (ctx) {
-        key.base = base; key.rank = rank; key.swizzle = swizzle_bytes;
-        for (int i = 0; i < 5; ++i) { key.gd[i] = gd[i]; key.bd[i] = bd[i]; key.es[i] = es[i]; }
-        for (int i = 0; i < 4; ++i) key.gs[i] = gs[i];
-        kbytes.assign(reinterpret_cast<const char*>(&key), sizeof(key));
-        auto it = ctx->tmap_cache.find(kbytes);
-        if (it != ctx->tmap_cache.end()) {
-            *out = it->second;
+        auto it = ctx->tmap_cache.find(hash);
+        if (it != ctx->tmap_cache.end() && std::memcmp(&it->second.key, &key, sizeof(key)) == 0) {
+            *out = it->second.map;
             ++ctx->tmap_hits;
             return CB_OK;
         }
@@ -182,7 +184,7 @@ int encode_tmap(cb_ctx* ctx, CUtensorMap* out, const void* base, int rank, const
     }
     if (ctx) {
         if (ctx->tmap_cache.size() >= 4096) ctx->tmap_cache.clear();
-        ctx->tmap_cache.emplace(std::move(kbytes), *out);
+        ctx->tmap_cache[hash] = TmapEntry{key, *out};
         ++ctx->tmap_misses;
     }
     return CB_OK;

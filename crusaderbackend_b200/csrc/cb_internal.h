@@ -12,6 +12,15 @@
 
 #include "../../include/crusader_b200.h"
 
+// What a tensor map encodes, as words: base, rank and swizzle, extents, box and element strides, byte strides.
+struct TmapKey {
+    uint64_t w[16];
+};
+struct TmapEntry {
+    TmapKey key;
+    CUtensorMap map;
+};
+
 struct cb_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -41,7 +50,7 @@ struct cb_ctx {
     int wgrad_grid_cap = 0;        // > 0: most CTAs a weight-gradient kernel uses (contexts that run beside another stream)
     // Encoded tensor maps by (base pointer, extents, strides, box, swizzle): a training loop presents the same few
     // hundred (tensor, tiling) pairs every step, so the encode runs once per pair (encode_tmap, cb_abi.cu).
-    std::unordered_map<std::string, CUtensorMap> tmap_cache;
+    std::unordered_map<uint64_t, TmapEntry> tmap_cache;  // by the hash of the key
     long long tmap_hits = 0, tmap_misses = 0;
 };
 
