@@ -67,22 +67,31 @@ int finish(cb_ctx* ctx, const char* what);
 // that an earlier kernel may have written or may still read.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_dep_on(cudaStream_t stream, bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                          Args&&... args) {
+                          int cluster, Args&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {  // consecutive blocks in x form clusters of this many CTAs
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = (unsigned)cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1u : 0u;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 template <typename... KArgs, typename... Args>
 cudaError_t launch_dep(cb_ctx* ctx, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
-    return launch_dep_on(ctx->stream, ctx->pdl != 0, kernel, grid, block, smem, std::forward<Args>(args)...);
+    return launch_dep_on(ctx->stream, ctx->pdl != 0, kernel, grid, block, smem, 1, std::forward<Args>(args)...);
 }
 
 // Raises cudaFuncAttributeMaxDynamicSharedMemorySize of `kernel` to the most this device allows (opt-in limit minus
@@ -120,7 +129,7 @@ struct Epilogue {
 
 // D[i][j] = sum_k P[i][k] * Q[j][k]; i < I tiles of 128 (UMMA M), j < J (UMMA N).
 // p_mn / q_mn: operand stored with the i / j index contiguous (MN-major) instead of k (K-major).
-// out_mode 0: C[j*ldc + i]; out_mode 1: C[i*ldc + j].
+// out_mode 0: C[j*ldc + i]; out_mode 1: C[i*ldc + j] (CUDA-core kernels only).
 struct GemmCall {
     int I = 0, J = 0, K = 0, batch = 1;
     const float* P = nullptr; long long ldp = 0, strideP = 0; int p_mn = 0;

@@ -70,6 +70,20 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
         : "memory");
     return ok;
 }
+// Non-blocking: 1 when the phase has completed. Issued a step ahead of the wait, its latency hides behind other work.
+__device__ __forceinline__ uint32_t mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok;
+}
 
 // Status codes a kernel may leave in the context's device status word.
 enum : int {
@@ -94,13 +108,17 @@ __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.
 
 __device__ __forceinline__ bool mbar_wait_for(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
                                               int code, uint64_t limit_ns) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = globaltimer_ns();
-    for (uint32_t it = 1;; ++it) {
+    // Reading %globaltimer costs ~600 clocks: a wait that looked at it whenever its first poll failed bound every pipeline
+    // of this library to one k-block per ~700 clocks, whatever the block's size. Each poll suspends the thread in hardware
+    // for a while, so the clock (and the abort flag) come in only on every 64th.
+    uint64_t t0 = 0;
+    for (uint32_t it = 0;; ++it) {
         if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 63u) == 0u) {
+        if ((it & 63u) == 63u) {
             if (*abort_flag) return false;
-            if (globaltimer_ns() - t0 > limit_ns) break;
+            const uint64_t now = globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > limit_ns) break;
         }
     }
     *abort_flag = 1;
@@ -121,21 +139,25 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int lane, volatile int* abort_flag,
                                                int* status, int code, uint32_t max_sleep_ns) {
     int ok = 1;
-    if (lane == 0 && !mbar_try_wait(bar, parity)) {
-        const uint64_t t0 = globaltimer_ns();
+    if (lane == 0) {
+        uint64_t t0 = 0;
         uint32_t ns = 32;
-        for (;;) {
+        for (uint32_t it = 0; !mbar_try_wait(bar, parity); ++it) {
             if (max_sleep_ns) {
                 __nanosleep(ns);
                 if (ns < max_sleep_ns) ns <<= 1;
             }
-            if (mbar_try_wait(bar, parity)) break;
-            if (*abort_flag) { ok = 0; break; }
-            if (globaltimer_ns() - t0 > CB_WAIT_LIMIT_NS) {
-                *abort_flag = 1;
-                atomicCAS(status, 0, code);
-                ok = 0;
-                break;
+            if ((it & 15u) == 15u) {  // the clock is expensive to read (see mbar_wait_for)
+                if (*abort_flag) { ok = 0; break; }
+                const uint64_t now = globaltimer_ns();
+                if (t0 == 0) {
+                    t0 = now;
+                } else if (now - t0 > CB_WAIT_LIMIT_NS) {
+                    *abort_flag = 1;
+                    atomicCAS(status, 0, code);
+                    ok = 0;
+                    break;
+                }
             }
         }
     }
@@ -143,6 +165,25 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, in
     if (ok)
         for (int i = 0; i < 1024 && !mbar_try_wait(bar, parity); ++i) {}
     return ok != 0;
+}
+
+// Whole converged warp, for the roles whose every instruction delays the pipeline (TMA producer, UMMA issuer): all lanes
+// poll, and the loop's control goes through warp votes, which the compiler knows to be uniform — the code after the wait
+// then keeps its operands in uniform registers. Same bound and abort behaviour as mbar_wait.
+__device__ __forceinline__ bool mbar_wait_uniform(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+    uint64_t t0 = 0;
+    for (uint32_t it = 0;; ++it) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if ((it & 63u) == 63u) {
+            if (__any_sync(0xffffffffu, *abort_flag)) return false;
+            const uint64_t now = globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            else if (__any_sync(0xffffffffu, now - t0 > CB_WAIT_LIMIT_NS)) break;
+        }
+    }
+    *abort_flag = 1;
+    atomicCAS(status, 0, code);
+    return false;
 }
 
 // After an abort: gives work that is still in flight a bounded chance to land before the CTA releases what it targets.
@@ -154,6 +195,23 @@ __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity, int* s
         if ((it & 63u) == 63u && globaltimer_ns() - t0 > 1000000ull) break;
     }
     atomicCAS(status, 0, 107 /* CBK_TIMEOUT_DRAIN */);
+}
+
+// ---------------------------------------------------------------- thread-block clusters
+// Every thread of every CTA of the cluster; orders shared-memory writes before it against reads after it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// 16 bytes at this CTA's shared-memory address `addr`, read from CTA `rank` of the cluster.
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
+    float4 v;
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(remote)
+                 : "memory");
+    return v;
 }
 
 // generic-proxy writes (st.shared) -> visible to the async proxy (TMA / tcgen05 operand reads)
@@ -174,6 +232,40 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* tm,
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], "
         "[%2];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(tm)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+        : "memory");
+}
+// Whole converged warp, every lane with the same arguments, one elected lane acts: like umma_tf32_elect, this keeps the
+// operands in uniform registers (a one-lane branch moves each of them there first).
+__device__ __forceinline__ void mbar_expect_tx_elect(uint32_t bar, uint32_t bytes) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t"
+        "}\n" ::"r"(bar),
+        "r"(bytes)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_elect(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int c0, int c1, int c2) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t"
+        "}\n" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(tm)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_elect(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int c0, int c1, int c2,
+                                                  int c3) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], "
+        "[%2];\n\t"
+        "}\n" ::"r"(dst),
         "l"(reinterpret_cast<uint64_t>(tm)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
         : "memory");
 }

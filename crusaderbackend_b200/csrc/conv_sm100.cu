@@ -999,7 +999,7 @@ int launch_conv(cb_ctx* err_ctx, const ConvEnv& env, const ConvPlan& q, const fl
     const int grid = per_split * q.nsplit;
     const int taps = FW == 1 ? TAPS_1 : (FW == 3 ? TAPS_3 : (pW == 1 ? TAPS_2L : TAPS_2R));
     cudaError_t e = launch_dep_on(env.stream, err_ctx && err_ctx->pdl, kernels[q.ew == 8 ? 0 : 1][taps], dim3((unsigned)grid),
-                                  dim3((unsigned)(64 + 32 * q.ew)), smem, tmIn, tmW, tmOut, p);
+                                  dim3((unsigned)(64 + 32 * q.ew)), smem, 1, tmIn, tmW, tmOut, p);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return check_cuda(err_ctx, e, "umma_conv_kernel launch");
     return CB_OK;
