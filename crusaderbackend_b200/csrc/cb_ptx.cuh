@@ -362,18 +362,6 @@ __device__ __forceinline__ void umma_tf32_elect(uint32_t d_tmem, uint64_t desc_a
         "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// kElect: called by the whole converged warp (elected lane issues); otherwise by the one issuing thread.
-template <bool kElect>
-__device__ __forceinline__ void umma_tf32_sel(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                              uint32_t accumulate) {
-    if (kElect) umma_tf32_elect(d_tmem, desc_a, desc_b, idesc, accumulate);
-    else umma_tf32(d_tmem, desc_a, desc_b, idesc, accumulate);
-}
-template <bool kElect>
-__device__ __forceinline__ void tc_commit_sel(uint32_t bar) {
-    if (kElect) tc_commit_elect(bar);
-    else tc_commit(bar);
-}
 // Whole-warp: 32 lanes x 16 consecutive fp32 columns starting at taddr (lane field = warp's quarter).
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(

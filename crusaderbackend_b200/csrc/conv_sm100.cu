@@ -64,7 +64,6 @@ struct ConvParams {
     long long out_batch;      // elements between consecutive images of the output
     ConvEpilogue ep;
     int c_wrap;         // > 0: input channels from c_wrap on are read again from channel (c - c_wrap) (3xTF32 form)
-    int issue_uniform;  // the MMA warp issues as a whole with an elected lane (wide accumulators) instead of from lane 0
     int* status;
     long long* trace;
     int dbg;       // development probes of the trace build
@@ -187,7 +186,7 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
                      const __grid_constant__ CUtensorMap tmOut, const ConvParams p) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ ConvSmem cs;
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // uniform for the compiler too
     const int lane = threadIdx.x & 31;
     volatile int* abort_flag = &cs.abort_flag;
 
@@ -210,7 +209,7 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(smem_u32(&cs.tfull[a]), 1);
-            mbar_init(smem_u32(&cs.tempty[a]), 32 * kEpiWarps);
+            mbar_init(smem_u32(&cs.tempty[a]), kEpiWarps);
         }
         mbar_init(smem_u32(&cs.wbar), 1);
         mbar_init(smem_u32(&cs.drain), 1);
@@ -234,56 +233,57 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
     griddep_launch();
     const uint32_t tmem_base = cs.tmem_base;
     const uint32_t acc_stride = (uint32_t)p.tmem_cols >> 1;
-    uint32_t armed = 0, armed_parity = 0;  // producer lane: stages armed at least once / parity of their last arming
+    uint32_t fills = 0;  // producer: stages filled so far
     if (threadIdx.x == 0) CB_TRACE_EVENT(p.trace, 2);
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        {
             // resident filter slice: one box [FW taps][OCs rows][32 channels] per (filter row, channel group)
             const uint32_t wbar = smem_u32(&cs.wbar);
-            mbar_expect_tx(wbar, p.w_bytes);
+            mbar_expect_tx_elect(wbar, p.w_bytes);
             const int boxes = p.FH * p.CG;
             for (int b = 0; b < boxes; ++b)
-                tma_load_3d(w_base + (uint32_t)b * p.NQ * kRowBytes, &tmW, wbar, 0, oc0, b * p.FW);
+                tma_load_3d_elect(w_base + (uint32_t)b * p.NQ * kRowBytes, &tmW, wbar, 0, oc0, b * p.FW);
         }
-        __syncwarp();
-        uint32_t s = 0, ph = 0;
+        uint32_t s = 0, ph = 0, ahead = 0;
         bool ok = true;
         for (int tile = tile0; tile < p.tiles && ok; tile += tile_step) {
+            // the tile's four lines; lines past the end use an image index >= N: their boxes are zero-filled
+            int n[4], h0[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int g = 4 * tile + j;  // 32-bit: a 64-bit division costs ~100 cycles on this path
+                n[j] = g / p.LPI;
+                h0[j] = (g - n[j] * p.LPI) * p.L;
+            }
             for (int cb = 0; cb < p.NCB; ++cb) {
-                ok = conv_warp_wait(smem_u32(&cs.empty[s]), ph ^ 1u, lane, abort_flag, p.status, CBK_TIMEOUT_EMPTY);
-                if (!ok) break;
-                if (lane == 0) {
-                    const uint32_t full = smem_u32(&cs.full[s]);
-                    const uint32_t dst0 = st_base + s * p.stage_bytes;
-                    mbar_expect_tx(full, p.stage_bytes);
-                    armed |= 1u << s;
-                    armed_parity = (armed_parity & ~(1u << s)) | (ph << s);
-                    int c0 = cb * p.KS * kCB;
-                    if (p.c_wrap && c0 >= p.c_wrap) c0 -= p.c_wrap;  // third channel group of the 3xTF32 form: x_hi again
-                    if (p.shared_rows) {
-                        // W == 32: the tile is 4 consecutive rows of one image; ONE box (32 px, 8*KS channels, FH+3
-                        // rows) lands as [row][channel][128 B]; rows above / below the image are zero-filled
-                        const int g = 4 * tile;  // 32-bit: a 64-bit division costs ~100 cycles on this path
-                        const int n = g / p.LPI;
-                        const int h0 = g - n * p.LPI;
-                        tma_load_4d(dst0, &tmIn, full, 0, c0, h0 - p.pH, n);
-                    } else {
-                        for (int fh = 0; fh < p.FH; ++fh) {
-                            for (int j = 0; j < 4; ++j) {
-                                const int g = 4 * tile + j;
-                                // lines past the end use an image index >= N: the whole box is zero-filled
-                                const int n = g / p.LPI;
-                                const int h0 = (g - n * p.LPI) * p.L;
-                                tma_load_3d(dst0 + (uint32_t)(fh * 4 + j) * p.block_bytes, &tmIn, full,
-                                            (h0 + fh - p.pH) * p.W, c0, n);
-                            }
-                        }
+                if (!__all_sync(0xffffffffu, ahead)) {
+                    ok = mbar_wait_uniform(smem_u32(&cs.empty[s]), ph ^ 1u, abort_flag, p.status, CBK_TIMEOUT_EMPTY);
+                    if (!ok) break;
+                }
+                const uint32_t s1 = s + 1 == (uint32_t)p.stages ? 0u : s + 1, ph1 = s1 ? ph : ph ^ 1u;
+                ahead = mbar_test(smem_u32(&cs.empty[s1]), ph1 ^ 1u);
+                const uint32_t full = smem_u32(&cs.full[s]);
+                const uint32_t dst0 = st_base + s * p.stage_bytes;
+                mbar_expect_tx_elect(full, p.stage_bytes);
+                int c0 = cb * p.KS * kCB;
+                if (p.c_wrap && c0 >= p.c_wrap) c0 -= p.c_wrap;  // third channel group of the 3xTF32 form: x_hi again
+                if (p.shared_rows) {
+                    // W == 32: the tile is 4 consecutive rows of one image; ONE box (32 px, 8*KS channels, FH+3
+                    // rows) lands as [row][channel][128 B]; rows above / below the image are zero-filled
+                    tma_load_4d_elect(dst0, &tmIn, full, 0, c0, h0[0] - p.pH, n[0]);
+                } else {
+                    for (int fh = 0; fh < p.FH; ++fh) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            tma_load_3d_elect(dst0 + (uint32_t)(fh * 4 + j) * p.block_bytes, &tmIn, full,
+                                              (h0[j] + fh - p.pH) * p.W, c0, n[j]);
                     }
                 }
-                __syncwarp();
-                if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
+                ++fills;
+                s = s1;
+                ph = ph1;
             }
         }
     } else if (warp == 1) {
@@ -302,88 +302,46 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
         const uint32_t fh_units = (p.shared_rows ? 1u : 4u) * blk_units;  // between consecutive filter rows of P
         const uint32_t q_group_units = (uint32_t)p.NQ * (kRowBytes >> 4);  // one (filter row, 32-channel group) of Q
         const uint32_t q_fh_units = (uint32_t)p.CG * q_group_units;        // between consecutive filter rows of Q
-        uint32_t s = 0, ph = 0, lt = 0;
-        bool ok = conv_warp_wait(smem_u32(&cs.wbar), 0, lane, abort_flag, p.status, CBK_TIMEOUT_FULL);
+        // The whole warp runs the loop with the same values (waits go through votes) and one elected lane issues, so that
+        // the descriptors stay in uniform registers; the next stage's barrier is tested while this one's UMMAs are issued.
+        uint32_t s = 0, ph = 0, lt = 0, ahead = 0;
+        bool ok = mbar_wait_uniform(smem_u32(&cs.wbar), 0, abort_flag, p.status, CBK_TIMEOUT_FULL);
         if (lane == 0) CB_TRACE_EVENT(p.trace, 4);
-#ifdef CB_TRACE
-        long long t_tempty = 0, t_full = 0, t_issue = 0;
-#endif
         for (int tile = tile0; tile < p.tiles && ok; tile += tile_step, ++lt) {
             const uint32_t a = lt & 1u;
-#ifdef CB_TRACE
-            const long long c_t0 = clock64();
-#endif
-            ok = conv_warp_wait(smem_u32(&cs.tempty[a]), ((lt >> 1) & 1u) ^ 1u, lane, abort_flag, p.status,
-                                CBK_TIMEOUT_TMEM_EMPTY);
+            ok = mbar_wait_uniform(smem_u32(&cs.tempty[a]), ((lt >> 1) & 1u) ^ 1u, abort_flag, p.status, CBK_TIMEOUT_TMEM_EMPTY);
             if (!ok) break;
             tc_fence_after();
-#ifdef CB_TRACE
-            t_tempty += clock64() - c_t0;
-#endif
             const uint32_t d_tmem = tmem_base + a * acc_stride;
-            int ti = 0;
+            uint32_t acc = 0u;
             for (int cb = 0; cb < p.NCB; ++cb) {
-#ifdef CB_TRACE
-                const long long c_f0 = clock64();
-#endif
-                ok = conv_warp_wait(smem_u32(&cs.full[s]), ph, lane, abort_flag, p.status, CBK_TIMEOUT_FULL);
-                if (!ok) break;
+                if (!__all_sync(0xffffffffu, ahead)) {
+                    ok = mbar_wait_uniform(smem_u32(&cs.full[s]), ph, abort_flag, p.status, CBK_TIMEOUT_FULL);
+                    if (!ok) break;
+                }
+                const uint32_t s1 = s + 1 == (uint32_t)p.stages ? 0u : s + 1, ph1 = s1 ? ph : ph ^ 1u;
+                ahead = mbar_test(smem_u32(&cs.full[s1]), ph1);
                 tc_fence_after();
-#ifdef CB_TRACE
-                const long long c_f1 = clock64();
-                t_full += c_f1 - c_f0;
-#endif
                 if (lane == 0 && lt == 0 && cb == 0) CB_TRACE_EVENT(p.trace, 5);
                 const uint64_t pbase = descP0 + (uint64_t)(((st_base + s * p.stage_bytes) >> 4) & 0x3FFFu);
                 const uint32_t ks0 = (uint32_t)(cb * p.KS);  // first K step of the stage: channels [8 ks0, ..)
-                if (p.issue_uniform) {
-                    // Wide accumulators (long MMA phases): the whole warp runs the loop with the same values and one
-                    // elected lane issues, so that the descriptors stay in uniform registers — from a one-lane branch a
-                    // descriptor that changes between UMMAs costs ~110 cycles of issue, more than a 128 x 192 x 8 UMMA
-                    // takes (measured with the UMMA-only loop of peak_sm100.cu). Narrow accumulators measured slower
-                    // this way and keep the one-lane form.
-                    for (int fh = 0; fh < p.FH; ++fh) {
-                        const uint64_t prow = pbase + (uint64_t)((uint32_t)fh * fh_units);
-                        const uint64_t qrow = descQ0 + (uint64_t)((uint32_t)fh * q_fh_units);
-                        for (int kk = 0; kk < p.KS; ++kk, ++ti) {
-                            const uint32_t ks = ks0 + (uint32_t)kk;
-                            umma_tf32_elect(d_tmem, prow + (uint64_t)((uint32_t)kk * 64u),
-                                            qrow + (uint64_t)((ks >> 2) * q_group_units + (ks & 3u) * 2u), idesc, ti != 0 ? 1u : 0u);
-                        }
+                for (int fh = 0; fh < p.FH; ++fh) {
+                    const uint64_t prow = pbase + (uint64_t)((uint32_t)fh * fh_units);
+                    const uint64_t qrow = descQ0 + (uint64_t)((uint32_t)fh * q_fh_units);
+                    for (int kk = 0; kk < p.KS; ++kk) {
+                        const uint32_t ks = ks0 + (uint32_t)kk;
+                        umma_tf32_elect(d_tmem, prow + (uint64_t)((uint32_t)kk * 64u),
+                                        qrow + (uint64_t)((ks >> 2) * q_group_units + (ks & 3u) * 2u), idesc, acc);
+                        acc = 1u;
                     }
-                    tc_commit_elect(smem_u32(&cs.empty[s]));
-                    if (cb == p.NCB - 1) tc_commit_elect(smem_u32(&cs.tfull[a]));
-                } else if (lane == 0) {
-                    for (int fh = 0; fh < p.FH; ++fh) {
-                        const uint64_t prow = pbase + (uint64_t)((uint32_t)fh * fh_units);
-                        const uint64_t qrow = descQ0 + (uint64_t)((uint32_t)fh * q_fh_units);
-                        for (int kk = 0; kk < p.KS; ++kk, ++ti) {
-                            const uint32_t ks = ks0 + (uint32_t)kk;
-                            umma_tf32(d_tmem, prow + (uint64_t)((uint32_t)kk * 64u),
-                                      qrow + (uint64_t)((ks >> 2) * q_group_units + (ks & 3u) * 2u), idesc, ti != 0 ? 1u : 0u);
-                        }
-                    }
-                    tc_commit(smem_u32(&cs.empty[s]));
-                    if (cb == p.NCB - 1) tc_commit(smem_u32(&cs.tfull[a]));
                 }
+                tc_commit_elect(smem_u32(&cs.empty[s]));
+                if (cb == p.NCB - 1) tc_commit_elect(smem_u32(&cs.tfull[a]));
                 if (lane == 0 && lt == 0 && cb == p.NCB - 1) CB_TRACE_EVENT(p.trace, 6);
-                __syncwarp();
-#ifdef CB_TRACE
-                t_issue += clock64() - c_f1;
-#endif
-                if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
+                s = s1;
+                ph = ph1;
             }
         }
-#ifdef CB_TRACE
-        if (lane == 0 && p.trace) {
-            // behind the 1024 x 16 event slots: per-CTA sums of the issuer's waits and issue time
-            long long* sums = p.trace + 1024 * 16 + (long long)blockIdx.x * 4;
-            sums[0] = t_tempty;
-            sums[1] = t_full;
-            sums[2] = t_issue;
-            sums[3] = (long long)p.stages * 10000 + p.KS * 1000 + p.NCB * 100 + p.nsplit;
-        }
-#endif
     } else {
         // ------------------------------------------------------------ epilogue (warps 2 ..)
         // One scheduler cannot hide the shuffle and store latencies of a single warp, so every TMEM lane quarter is
@@ -399,8 +357,7 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
         const bool has_left = col > 0, has_right = col < p.W - 1;
         for (int tile = tile0; tile < p.tiles && ok; tile += tile_step, ++lt) {
             const uint32_t a = lt & 1u;
-            ok = mbar_wait(smem_u32(&cs.tfull[a]), (lt >> 1) & 1u, abort_flag, p.status, CBK_TIMEOUT_TMEM_FULL);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = mbar_wait_uniform(smem_u32(&cs.tfull[a]), (lt >> 1) & 1u, abort_flag, p.status, CBK_TIMEOUT_TMEM_FULL);
             if (!ok) break;
             tc_fence_after();
             if (threadIdx.x == 64 && lt == 0) CB_TRACE_EVENT(p.trace, 7);
@@ -416,7 +373,8 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
 #ifdef CB_TRACE
             if (p.dbg & 1) {  // development probe: leave the accumulator unread (how fast is the MMA phase alone?)
                 tc_fence_before();
-                mbar_arrive(smem_u32(&cs.tempty[a]));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&cs.tempty[a]));
                 continue;
             }
 #endif
@@ -424,7 +382,8 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
                 conv_epilogue_chunk<TAPS>(p, &tmOut, t_row, c, oc0, img, plane, pix, n, valid, has_left, has_right,
                                     my_stage + buf * 1024u, lane, threadIdx.x == 64 && lt == 0 && c == 0);
             tc_fence_before();
-            mbar_arrive(smem_u32(&cs.tempty[a]));
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&cs.tempty[a]));
             if (threadIdx.x == 64 && lt == 0) CB_TRACE_EVENT(p.trace, 8);
             if (threadIdx.x == 64) CB_TRACE_EVENT(p.trace, 10);
         }
@@ -440,12 +399,11 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
         // finish before the shared memory and TMEM are released.
         if (warp == 0 && lane == 0) {
             mbar_drain(smem_u32(&cs.wbar), 0, p.status);
-            for (int st = 0; st < p.stages; ++st)
-                if ((armed >> st) & 1u) mbar_drain(smem_u32(&cs.full[st]), (armed_parity >> st) & 1u, p.status);
+            const uint32_t n = (uint32_t)p.stages;  // stage st was last filled as number st + n * round: parity of the round
+            for (uint32_t st = 0; st < n && st < fills; ++st) mbar_drain(smem_u32(&cs.full[st]), ((fills - 1 - st) / n) & 1u, p.status);
         }
         if (warp == 1) {  // the commit comes from the lane that issued the MMAs
-            if (p.issue_uniform) tc_commit_elect(smem_u32(&cs.drain));
-            else if (lane == 0) tc_commit(smem_u32(&cs.drain));
+            tc_commit_elect(smem_u32(&cs.drain));
             if (lane == 0) mbar_drain(smem_u32(&cs.drain), 0, p.status);
         }
         __syncthreads();
@@ -907,13 +865,6 @@ int launch_conv(cb_ctx* err_ctx, const ConvEnv& env, const ConvPlan& q, const fl
     p.out_batch = out_batch ? out_batch : (long long)q.Cout * (long long)plane;
     p.ep = ep;
     p.status = env.status;
-    {
-        static const int forced = [] {
-            const char* e = std::getenv("CB_CONV_ISSUE");  // development override: 0 one lane, 1 whole warp
-            return e ? std::atoi(e) : -1;
-        }();
-        p.issue_uniform = forced >= 0 ? forced : (q.NQ >= 160 ? 1 : 0);
-    }
     p.trace = err_ctx ? err_ctx->trace : nullptr;
 #ifdef CB_TRACE
     {

@@ -48,7 +48,6 @@ struct WgradParams {
     int rows_cf;
     long long oc_stride, base_off;
     float* dW;
-    int issue_uniform;               // the MMA warp issues as a whole with an elected lane instead of from lane 0
     int* status;
     long long* trace;
 };
@@ -98,7 +97,7 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
                       const WgradParams p) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ WgradSmem ws;
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // uniform for the compiler too
     const int lane = threadIdx.x & 31;
     volatile int* abort_flag = &ws.abort_flag;
     const uint32_t st_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -112,7 +111,7 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
         for (int s = 0; s < p.stages; ++s) {
             mbar_init(smem_u32(&ws.full[s]), 1);
             mbar_init(smem_u32(&ws.empty[s]), 1);
-            mbar_init(smem_u32(&ws.xf[s]), 32 * kShiftWarps);
+            mbar_init(smem_u32(&ws.xf[s]), kShiftWarps);
         }
         mbar_init(smem_u32(&ws.tfull), 1);
         mbar_init(smem_u32(&ws.drain), 1);
@@ -138,135 +137,92 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
     const uint32_t tmem_base = ws.tmem_base;
     if (threadIdx.x == 0) CB_TRACE_EVENT(p.trace, 2);
 
-    uint32_t armed = 0, armed_parity = 0;  // producer lane: stages armed at least once / parity of their last arming
+    uint32_t fills = 0;  // producer: stages filled so far
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        uint32_t s = 0, ph = 0;
-        bool ok = true;
-        for (int g = blockIdx.x; g < p.vgroups && ok; g += gridDim.x) {
-            ok = conv_warp_wait(smem_u32(&ws.empty[s]), ph ^ 1u, lane, abort_flag, p.status, CBK_TIMEOUT_EMPTY);
-            if (!ok) break;
-            if (lane == 0) {
-                const uint32_t full = smem_u32(&ws.full[s]);
-                mbar_expect_tx(full, (uint32_t)p.lps * (p.a_bytes + set_bytes));
-                armed |= 1u << s;
-                armed_parity = (armed_parity & ~(1u << s)) | (ph << s);
-                // 3xTF32 form: the two small cross terms first, while the accumulator is small (the tensor core's
-                // fp32 accumulation error is relative to what the accumulator holds), the hi x hi products last
-                const int pass = g / p.groups, gg = g - pass * p.groups;
-                const bool x3 = p.vgroups > p.groups;
-                const CUtensorMap* mx = (x3 && pass == 0) ? &tmXlo : &tmX;
-                const CUtensorMap* my = (x3 && pass == 1) ? &tmdYlo : &tmdY;
-                for (int l = 0; l < p.lps; ++l) {
-                    const uint32_t stg = st_base + s * p.stage_bytes + (uint32_t)l * p.line_bytes;
-                    // lines past the end use an image index >= N: their boxes are zero-filled and add nothing
-                    const int gi = gg * p.lps + l;  // total_lines < 2^29 (checked on the host)
-                    const int n = gi / p.LPI;
-                    const int h0 = (gi - n * p.LPI) * p.L;
-                    if (p.rows_cf) {
-                        tma_load_4d(stg, mx, full, 0, h0 - p.pH, 0, n);
-                    } else {
-                        for (int fh = 0; fh < p.FH; ++fh)
-                            tma_load_3d(stg + (uint32_t)fh * p.Cp * kRowBytes, mx, full, (h0 + fh - p.pH) * p.W, 0, n);
-                    }
-                    tma_load_3d(stg + p.a_bytes + (uint32_t)centre * set_bytes, my, full, h0 * p.W, 0, n);
+        uint32_t s = 0, ph = 0, ahead = 0;
+        const bool x3 = p.vgroups > p.groups;
+        for (int g = blockIdx.x; g < p.vgroups; g += gridDim.x) {
+            if (!__all_sync(0xffffffffu, ahead) &&
+                !mbar_wait_uniform(smem_u32(&ws.empty[s]), ph ^ 1u, abort_flag, p.status, CBK_TIMEOUT_EMPTY))
+                break;
+            const uint32_t s1 = s + 1 == (uint32_t)p.stages ? 0u : s + 1, ph1 = s1 ? ph : ph ^ 1u;
+            ahead = mbar_test(smem_u32(&ws.empty[s1]), ph1 ^ 1u);
+            const uint32_t full = smem_u32(&ws.full[s]);
+            mbar_expect_tx_elect(full, (uint32_t)p.lps * (p.a_bytes + set_bytes));
+            // 3xTF32 form: the two small cross terms first, while the accumulator is small (the tensor core's
+            // fp32 accumulation error is relative to what the accumulator holds), the hi x hi products last
+            const int pass = x3 ? g / p.groups : 0, gg = g - pass * p.groups;
+            const CUtensorMap* mx = (x3 && pass == 0) ? &tmXlo : &tmX;
+            const CUtensorMap* my = (x3 && pass == 1) ? &tmdYlo : &tmdY;
+            // lines past the end use an image index >= N: their boxes are zero-filled and add nothing
+            const int g0 = gg * p.lps;  // total_lines < 2^29 (checked on the host)
+            int n = g0 / p.LPI, line = g0 - n * p.LPI;
+            for (int l = 0; l < p.lps; ++l) {
+                const uint32_t stg = st_base + s * p.stage_bytes + (uint32_t)l * p.line_bytes;
+                const int h0 = line * p.L;
+                if (p.rows_cf) {
+                    tma_load_4d_elect(stg, mx, full, 0, h0 - p.pH, 0, n);
+                } else {
+                    for (int fh = 0; fh < p.FH; ++fh)
+                        tma_load_3d_elect(stg + (uint32_t)fh * p.Cp * kRowBytes, mx, full, (h0 + fh - p.pH) * p.W, 0, n);
+                }
+                tma_load_3d_elect(stg + p.a_bytes + (uint32_t)centre * set_bytes, my, full, h0 * p.W, 0, n);
+                if (++line == p.LPI) {
+                    line = 0;
+                    ++n;
                 }
             }
-            __syncwarp();
-            if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
+            ++fills;
+            s = s1;
+            ph = ph1;
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ UMMA issuer
         const uint32_t idesc = umma_idesc_tf32(128, (uint32_t)p.NQ, 0u, 0u);
         const uint64_t desc0 = umma_smem_desc(0, 16u, 1024u, UMMA_SW_128B);  // K-major 128-byte rows; address added per stage
-        uint32_t s = 0, ph = 0;
-        bool ok = true;
+        // The whole warp runs the loop with the same values (waits go through votes) and one elected lane issues: the
+        // descriptors stay in uniform registers (see umma_tf32_elect).
+        const bool shifted = p.FW > 1;
+        uint32_t s = 0, ph = 0, ahead = 0;
         bool first_line = true;
-#ifdef CB_TRACE
-        long long t_full = 0, t_xf = 0, t_issue = 0;
-#endif
-        for (int g = blockIdx.x; g < p.vgroups && ok; g += gridDim.x) {
-#ifdef CB_TRACE
-            const long long c0 = clock64();
-#endif
-            ok = conv_warp_wait(smem_u32(&ws.full[s]), ph, lane, abort_flag, p.status, CBK_TIMEOUT_FULL);
-            if (!ok) break;
-#ifdef CB_TRACE
-            const long long c1 = clock64();
-#endif
-            if (p.FW > 1) {
-                ok = conv_warp_wait(smem_u32(&ws.xf[s]), ph, lane, abort_flag, p.status, CBK_TIMEOUT_XFORM);
-                if (!ok) break;
-            }
+        for (int g = blockIdx.x; g < p.vgroups; g += gridDim.x) {
+            // with shifted copies the shift warps' arrival implies that the copies' source has landed; the rest of the
+            // stage is part of the same transaction count
+            if (!__all_sync(0xffffffffu, ahead) &&
+                !mbar_wait_uniform(smem_u32(shifted ? &ws.xf[s] : &ws.full[s]), ph, abort_flag, p.status,
+                                   shifted ? CBK_TIMEOUT_XFORM : CBK_TIMEOUT_FULL))
+                break;
+            const uint32_t s1 = s + 1 == (uint32_t)p.stages ? 0u : s + 1, ph1 = s1 ? ph : ph ^ 1u;
+            ahead = mbar_test(smem_u32(shifted ? &ws.xf[s1] : &ws.full[s1]), ph1);
             tc_fence_after();
-#ifdef CB_TRACE
-            const long long c2 = clock64();
-            t_full += c1 - c0;
-            t_xf += c2 - c1;
-#endif
             if (lane == 0 && first_line) CB_TRACE_EVENT(p.trace, 5);
-            if (p.issue_uniform) {
-                // the whole warp runs the loop with the same values, one elected lane issues: descriptors that change
-                // from UMMA to UMMA cost ~110 cycles of issue each from a one-lane branch (see umma_tf32_elect)
-                for (int l = 0; l < p.lps; ++l) {
-                    const uint32_t stg = st_base + s * p.stage_bytes + (uint32_t)l * p.line_bytes;
-                    const uint64_t dA0 = desc0 + (uint64_t)((stg >> 4) & 0x3FFFu);
-                    const uint64_t dB0 = desc0 + (uint64_t)(((stg + p.a_bytes) >> 4) & 0x3FFFu);
-                    const uint32_t first = (first_line && l == 0) ? 0u : 1u;
-                    for (int m = 0; m < p.mtiles; ++m) {
-                        const uint64_t dA = dA0 + (uint64_t)(m * (16384 >> 4));
-                        const uint32_t d = tmem_base + (uint32_t)m * p.NQ;
-                        umma_tf32_elect(d, dA, dB0, idesc, first);
-                        umma_tf32_elect(d, dA + 2, dB0 + 2, idesc, 1u);
-                        umma_tf32_elect(d, dA + 4, dB0 + 4, idesc, 1u);
-                        umma_tf32_elect(d, dA + 6, dB0 + 6, idesc, 1u);
-                    }
-                }
-                tc_commit_elect(smem_u32(&ws.empty[s]));
-                if (g + (int)gridDim.x >= p.vgroups) tc_commit_elect(smem_u32(&ws.tfull));
-                if (lane == 0 && first_line) CB_TRACE_EVENT(p.trace, 6);
-                if (lane == 0 && g + (int)gridDim.x >= p.vgroups) CB_TRACE_EVENT(p.trace, 7);
-            } else if (lane == 0) {
-                for (int l = 0; l < p.lps; ++l) {
-                    const uint32_t stg = st_base + s * p.stage_bytes + (uint32_t)l * p.line_bytes;
-                    const uint64_t dA0 = desc0 + (uint64_t)((stg >> 4) & 0x3FFFu);
-                    const uint64_t dB0 = desc0 + (uint64_t)(((stg + p.a_bytes) >> 4) & 0x3FFFu);
-                    const uint32_t first = (first_line && l == 0) ? 0u : 1u;
-                    for (int m = 0; m < p.mtiles; ++m) {
-                        const uint64_t dA = dA0 + (uint64_t)(m * (16384 >> 4));
-                        const uint32_t d = tmem_base + (uint32_t)m * p.NQ;
-                        umma_tf32(d, dA, dB0, idesc, first);
-                        umma_tf32(d, dA + 2, dB0 + 2, idesc, 1u);
-                        umma_tf32(d, dA + 4, dB0 + 4, idesc, 1u);
-                        umma_tf32(d, dA + 6, dB0 + 6, idesc, 1u);
-                    }
-                }
-                tc_commit(smem_u32(&ws.empty[s]));
-                if (first_line) CB_TRACE_EVENT(p.trace, 6);
-                if (g + (int)gridDim.x >= p.vgroups) {
-                    tc_commit(smem_u32(&ws.tfull));
-                    CB_TRACE_EVENT(p.trace, 7);
+            for (int l = 0; l < p.lps; ++l) {
+                const uint32_t stg = st_base + s * p.stage_bytes + (uint32_t)l * p.line_bytes;
+                const uint64_t dA0 = desc0 + (uint64_t)((stg >> 4) & 0x3FFFu);
+                const uint64_t dB0 = desc0 + (uint64_t)(((stg + p.a_bytes) >> 4) & 0x3FFFu);
+                const uint32_t first = (first_line && l == 0) ? 0u : 1u;
+                for (int m = 0; m < p.mtiles; ++m) {
+                    const uint64_t dA = dA0 + (uint64_t)(m * (16384 >> 4));
+                    const uint32_t d = tmem_base + (uint32_t)m * p.NQ;
+                    umma_tf32_elect(d, dA, dB0, idesc, first);
+                    umma_tf32_elect(d, dA + 2, dB0 + 2, idesc, 1u);
+                    umma_tf32_elect(d, dA + 4, dB0 + 4, idesc, 1u);
+                    umma_tf32_elect(d, dA + 6, dB0 + 6, idesc, 1u);
                 }
             }
-            __syncwarp();
-#ifdef CB_TRACE
-            t_issue += clock64() - c2;
-#endif
+            tc_commit_elect(smem_u32(&ws.empty[s]));
+            if (g + (int)gridDim.x >= p.vgroups) tc_commit_elect(smem_u32(&ws.tfull));
+            if (lane == 0 && first_line) CB_TRACE_EVENT(p.trace, 6);
+            if (lane == 0 && g + (int)gridDim.x >= p.vgroups) CB_TRACE_EVENT(p.trace, 7);
             first_line = false;
-            if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
+            s = s1;
+            ph = ph1;
         }
-#ifdef CB_TRACE
-        if (lane == 0 && p.trace) {
-            p.trace[(long long)blockIdx.x * 16 + 13] = t_full;
-            p.trace[(long long)blockIdx.x * 16 + 14] = t_xf;
-            p.trace[(long long)blockIdx.x * 16 + 15] = t_issue;
-        }
-#endif
     } else if (warp < 6) {
         // ------------------------------------------------------------ epilogue: partial sums to the workspace
         const int quarter = warp & 3;
-        bool ok = mbar_wait(smem_u32(&ws.tfull), 0, abort_flag, p.status, CBK_TIMEOUT_TMEM_FULL);
-        ok = __all_sync(0xffffffffu, ok);
+        const bool ok = mbar_wait_warp(smem_u32(&ws.tfull), 0, lane, abort_flag, p.status, CBK_TIMEOUT_TMEM_FULL, 128);
         if (threadIdx.x == 64) CB_TRACE_EVENT(p.trace, 8);
         if (ok) {
             tc_fence_after();
@@ -334,22 +290,25 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
         if (p.FW > 1) {
             const int t = threadIdx.x - 192;
             uint32_t s = 0, ph = 0;
-            bool ok = true;
-            const int per_line = p.OCp * 8;
-            for (int g = blockIdx.x; g < p.vgroups && ok; g += gridDim.x) {
-                ok = mbar_wait(smem_u32(&ws.full[s]), ph, abort_flag, p.status, CBK_TIMEOUT_XFORM_FULL);
-                if (!ok) break;
-                for (int item = t; item < p.lps * per_line; item += 32 * kShiftWarps) {
-                    const int l = item / per_line, rem = item - l * per_line;
-                    const int row = rem >> 3, q = rem & 7;
-                    const uint32_t b0 = st_base + s * p.stage_bytes + (uint32_t)l * p.line_bytes + p.a_bytes + (uint32_t)row * kRowBytes;
-                    const uint32_t src = b0 + (uint32_t)centre * set_bytes;
+            // item = (row, 16-byte chunk) of a line; a thread's items keep their chunk (32 * kShiftWarps is a multiple of 8)
+            const int rows = p.lps * p.OCp, q = t & 7;
+            for (int g = blockIdx.x; g < p.vgroups; g += gridDim.x) {
+                if (!mbar_wait_uniform(smem_u32(&ws.full[s]), ph, abort_flag, p.status, CBK_TIMEOUT_XFORM_FULL)) break;
+                const uint32_t base = st_base + s * p.stage_bytes + p.a_bytes + (uint32_t)centre * set_bytes;
+                int l = 0, row = t >> 3;
+                for (int r = t >> 3; r < rows; r += 4 * kShiftWarps, row += 4 * kShiftWarps) {
+                    while (row >= p.OCp) {
+                        row -= p.OCp;
+                        ++l;
+                    }
+                    const uint32_t src = base + (uint32_t)l * p.line_bytes + (uint32_t)row * kRowBytes;
                     const uint32_t m1 = centre >= 1 ? src - set_bytes : 0u;             // tap fw = pW - 1
                     const uint32_t p1 = centre + 1 < p.FW ? src + set_bytes : 0u;       // tap fw = pW + 1
                     shift_dy_chunk(src, m1, p1, q, p.W);
                 }
                 fence_proxy_async_smem();
-                mbar_arrive(smem_u32(&ws.xf[s]));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&ws.xf[s]));
                 if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
             }
         }
@@ -363,12 +322,11 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
         // shared memory and issued MMAs may still run on its accumulator; both get a bounded chance to finish before
         // the shared memory and TMEM are released.
         if (warp == 0 && lane == 0) {
-            for (int st = 0; st < p.stages; ++st)
-                if ((armed >> st) & 1u) mbar_drain(smem_u32(&ws.full[st]), (armed_parity >> st) & 1u, p.status);
+            const uint32_t n = (uint32_t)p.stages;  // stage st was last filled as number st + n * round: parity of the round
+            for (uint32_t st = 0; st < n && st < fills; ++st) mbar_drain(smem_u32(&ws.full[st]), ((fills - 1 - st) / n) & 1u, p.status);
         }
         if (warp == 1) {  // the commit comes from the lane that issued the MMAs
-            if (p.issue_uniform) tc_commit_elect(smem_u32(&ws.drain));
-            else if (lane == 0) tc_commit(smem_u32(&ws.drain));
+            tc_commit_elect(smem_u32(&ws.drain));
             if (lane == 0) mbar_drain(smem_u32(&ws.drain), 0, p.status);
         }
         __syncthreads();
@@ -591,13 +549,6 @@ static int wgrad_core(cb_ctx* ctx, const float* dY, const float* X, float* dW, i
         return e ? std::atoi(e) : 1;
     }();
     p.atomic = (!ctx->deterministic && allow_atomic) ? 1 : 0;
-    static const int issue_mode = [] {
-        // development override: 0 one lane (default: with back-to-back UMMAs the tensor core's operand fetches starve
-        // the shift warps' shared-memory traffic and every layer shape measured 5-20 % slower), 1 whole warp
-        const char* e = std::getenv("CB_WGRAD_ISSUE");
-        return e ? std::atoi(e) : 0;
-    }();
-    p.issue_uniform = issue_mode;
     static const int allow_direct = [] {
         const char* e = std::getenv("CB_WGRAD_DIRECT");  // development switch, default on
         return e ? std::atoi(e) : 1;
