@@ -23,7 +23,7 @@
 //  * When a layer has fewer pixel tiles than the GPU has CTA slots, the output channels are split over 2 or 4 CTAs
 //    per tile (each fetches only its slice of the packed filter and runs a narrower UMMA), so that small feature maps
 //    still occupy the whole GPU.
-//  * Epilogue (4 or 2 warps per TMEM lane quarter): tcgen05.ld, tap combine, then optional per-channel or
+//  * Epilogue (four warps per TMEM lane quarter): tcgen05.ld, tap combine, then optional per-channel or
 //    per-position scale / shift, bias, accumulation onto the output, ReLU, and stores in which the 32 lanes of a warp
 //    write 128 contiguous bytes.
 //
@@ -59,6 +59,7 @@ struct ConvParams {
     uint32_t w_bytes;         // resident slice of the packed filter
     uint32_t block_bytes;     // one line of a stage: 8 * KS channels x 128 B
     uint32_t stage_bytes;     // nblocks * block_bytes
+    int epi_sets;             // sets of epilogue warps that take the tiles in turn
     int tma_out;              // 1: results leave through TMA stores (2: TMA reduce-adds) staged in shared memory
     float* Out;
     long long out_batch;      // elements between consecutive images of the output
@@ -123,8 +124,8 @@ __device__ __forceinline__ void conv_epilogue_chunk(const ConvParams& p, const C
     if (traced) CB_TRACE_EVENT(p.trace, 14);
     const bool plain = p.ep.scale == nullptr && p.ep.bias == nullptr;
     if (p.tma_out) {
-        // the store issued two chunks ago from this slot must have finished reading it
-        if (lane == 0) tma_store_wait_read<1>();
+        // the store issued from this slot before must have finished reading it
+        if (lane == 0) tma_store_wait_read<0>();
         __syncwarp();
         const uint32_t mine = stage + (uint32_t)(lane * 4);
         if (plain) {
@@ -177,11 +178,13 @@ __device__ __forceinline__ void conv_epilogue_chunk(const ConvParams& p, const C
     if (traced) CB_TRACE_EVENT(p.trace, 15);
 }
 
-// Epilogue warps are a template parameter of the kernel (8 = 2 per TMEM lane quarter is what the planner picks; 16 is
-// kept for experiments). Outputs of at most 32 channels per CTA with a small filter run two CTAs per SM so that their
-// UMMA chains overlap.
+// Epilogue warps: eight (two per TMEM lane quarter) where two CTAs share an SM (outputs of at most 32 channels per CTA with a
+// small filter: their UMMA chains overlap), else sixteen. A warp's chunk of 8 channels is a chain of latencies (TMEM load,
+// shuffles, staging, proxy fence, TMA store: ~1100 clocks), so the chunks of a tile go to different warps, and where a tile
+// has fewer chunks than warps they form sets that take the tiles in turn. 64 -> 64 at 32 x 32 with eight warps was bound by
+// this; 16 -> 16 pays more for the start of 1152 threads an SM than the second eight warps of each CTA gain.
 template <int kEpiWarps, int TAPS>
-__global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
+__global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps == 8 ? 2 : 1)
     umma_conv_kernel(const __grid_constant__ CUtensorMap tmIn, const __grid_constant__ CUtensorMap tmW,
                      const __grid_constant__ CUtensorMap tmOut, const ConvParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -192,7 +195,7 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
 
     const uint32_t w_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t st_base = w_base + p.w_bytes;
-    const uint32_t out_base = st_base + (uint32_t)p.stages * p.stage_bytes;  // epilogue staging: 2 KB per epilogue warp
+    const uint32_t out_base = st_base + (uint32_t)p.stages * p.stage_bytes;  // epilogue staging: 1 KB per epilogue warp
     // this CTA's slice of the output channels and its walk over the pixel tiles
     const int split = (int)blockIdx.x % p.nsplit;
     const int tile0 = (int)blockIdx.x / p.nsplit;
@@ -209,7 +212,7 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(smem_u32(&cs.tfull[a]), 1);
-            mbar_init(smem_u32(&cs.tempty[a]), kEpiWarps);
+            mbar_init(smem_u32(&cs.tempty[a]), (uint32_t)(kEpiWarps / p.epi_sets));
         }
         mbar_init(smem_u32(&cs.wbar), 1);
         mbar_init(smem_u32(&cs.drain), 1);
@@ -238,14 +241,6 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        {
-            // resident filter slice: one box [FW taps][OCs rows][32 channels] per (filter row, channel group)
-            const uint32_t wbar = smem_u32(&cs.wbar);
-            mbar_expect_tx_elect(wbar, p.w_bytes);
-            const int boxes = p.FH * p.CG;
-            for (int b = 0; b < boxes; ++b)
-                tma_load_3d_elect(w_base + (uint32_t)b * p.NQ * kRowBytes, &tmW, wbar, 0, oc0, b * p.FW);
-        }
         uint32_t s = 0, ph = 0, ahead = 0;
         bool ok = true;
         for (int tile = tile0; tile < p.tiles && ok; tile += tile_step) {
@@ -305,6 +300,15 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
         // The whole warp runs the loop with the same values (waits go through votes) and one elected lane issues, so that
         // the descriptors stay in uniform registers; the next stage's barrier is tested while this one's UMMAs are issued.
         uint32_t s = 0, ph = 0, lt = 0, ahead = 0;
+        {
+            // this warp fetches the resident filter slice, while the producer is already at the first stage: one box
+            // [FW taps][OCs rows][32 channels] per (filter row, channel group)
+            const uint32_t wbar = smem_u32(&cs.wbar);
+            mbar_expect_tx_elect(wbar, p.w_bytes);
+            const int boxes = p.FH * p.CG;
+            for (int b = 0; b < boxes; ++b)
+                tma_load_3d_elect(w_base + (uint32_t)b * p.NQ * kRowBytes, &tmW, wbar, 0, oc0, b * p.FW);
+        }
         bool ok = mbar_wait_uniform(smem_u32(&cs.wbar), 0, abort_flag, p.status, CBK_TIMEOUT_FULL);
         if (lane == 0) CB_TRACE_EVENT(p.trace, 4);
         for (int tile = tile0; tile < p.tiles && ok; tile += tile_step, ++lt) {
@@ -323,16 +327,20 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
                 ahead = mbar_test(smem_u32(&cs.full[s1]), ph1);
                 tc_fence_after();
                 if (lane == 0 && lt == 0 && cb == 0) CB_TRACE_EVENT(p.trace, 5);
+                if (lane == 0 && lt == 1 && cb == 0) CB_TRACE_EVENT(p.trace, 3);
                 const uint64_t pbase = descP0 + (uint64_t)(((st_base + s * p.stage_bytes) >> 4) & 0x3FFFu);
-                const uint32_t ks0 = (uint32_t)(cb * p.KS);  // first K step of the stage: channels [8 ks0, ..)
+                // a stage holds 1, 2 or 4 K steps of 8 channels, never across a 32-channel group of the packed filter
+                const uint32_t ks0 = (uint32_t)(cb * p.KS);
+                const uint64_t q0 = descQ0 + (uint64_t)((ks0 >> 2) * q_group_units + (ks0 & 3u) * 2u);
                 for (int fh = 0; fh < p.FH; ++fh) {
-                    const uint64_t prow = pbase + (uint64_t)((uint32_t)fh * fh_units);
-                    const uint64_t qrow = descQ0 + (uint64_t)((uint32_t)fh * q_fh_units);
-                    for (int kk = 0; kk < p.KS; ++kk) {
-                        const uint32_t ks = ks0 + (uint32_t)kk;
-                        umma_tf32_elect(d_tmem, prow + (uint64_t)((uint32_t)kk * 64u),
-                                        qrow + (uint64_t)((ks >> 2) * q_group_units + (ks & 3u) * 2u), idesc, acc);
-                        acc = 1u;
+                    const uint64_t dp = pbase + (uint64_t)((uint32_t)fh * fh_units);
+                    const uint64_t dq = q0 + (uint64_t)((uint32_t)fh * q_fh_units);
+                    umma_tf32_elect(d_tmem, dp, dq, idesc, acc);
+                    acc = 1u;
+                    if (p.KS >= 2) umma_tf32_elect(d_tmem, dp + 64u, dq + 2u, idesc, 1u);
+                    if (p.KS == 4) {
+                        umma_tf32_elect(d_tmem, dp + 128u, dq + 4u, idesc, 1u);
+                        umma_tf32_elect(d_tmem, dp + 192u, dq + 6u, idesc, 1u);
                     }
                 }
                 tc_commit_elect(smem_u32(&cs.empty[s]));
@@ -344,24 +352,18 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
         }
     } else {
         // ------------------------------------------------------------ epilogue (warps 2 ..)
-        // One scheduler cannot hide the shuffle and store latencies of a single warp, so every TMEM lane quarter is
-        // served by several warps that split the channel chunks between them.
         const int quarter = warp & 3;
-        const int slot = (warp - 2) >> 2;
-        const uint32_t my_stage = out_base + (uint32_t)(warp - 2) * 2048u;
-        uint32_t buf = 0;
+        const int per_set = kEpiWarps / 4 / p.epi_sets;           // warps of a set on this lane quarter
+        const int set = ((warp - 2) >> 2) / per_set, slot = ((warp - 2) >> 2) - set * per_set;
+        const uint32_t my_stage = out_base + (uint32_t)(warp - 2) * 1024u;
         uint32_t lt = 0;
         bool ok = true;
         const long long plane = (long long)p.H * p.W;
         const int col = lane & (p.W - 1);
         const bool has_left = col > 0, has_right = col < p.W - 1;
-        for (int tile = tile0; tile < p.tiles && ok; tile += tile_step, ++lt) {
+        lt = (uint32_t)set;
+        for (int tile = tile0 + set * tile_step; tile < p.tiles && ok; tile += p.epi_sets * tile_step, lt += (uint32_t)p.epi_sets) {
             const uint32_t a = lt & 1u;
-            ok = mbar_wait_uniform(smem_u32(&cs.tfull[a]), (lt >> 1) & 1u, abort_flag, p.status, CBK_TIMEOUT_TMEM_FULL);
-            if (!ok) break;
-            tc_fence_after();
-            if (threadIdx.x == 64 && lt == 0) CB_TRACE_EVENT(p.trace, 7);
-            if (threadIdx.x == 64 && lt == 1) CB_TRACE_EVENT(p.trace, 9);
             const int g = 4 * tile + quarter;
             const bool valid = g < (int)p.total_lines;
             const int n = g / p.LPI;
@@ -369,6 +371,11 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
             // lane x of the line is pixel (h0 + x / W, x % W): 32 consecutive floats of the output plane
             float* img = p.Out + (long long)n * p.out_batch;
             const int pix = h0 * p.W + lane;
+            ok = mbar_wait_uniform(smem_u32(&cs.tfull[a]), (lt >> 1) & 1u, abort_flag, p.status, CBK_TIMEOUT_TMEM_FULL);
+            if (!ok) break;
+            tc_fence_after();
+            if (threadIdx.x == 64 && lt == 0) CB_TRACE_EVENT(p.trace, 7);
+            if (threadIdx.x == 64 && lt == 1) CB_TRACE_EVENT(p.trace, 9);
             const uint32_t t_row = tmem_base + a * acc_stride + ((uint32_t)(32 * quarter) << 16);
 #ifdef CB_TRACE
             if (p.dbg & 1) {  // development probe: leave the accumulator unread (how fast is the MMA phase alone?)
@@ -378,17 +385,18 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
                 continue;
             }
 #endif
-            for (int c = slot * 8; c < p.OCs; c += 8 * (kEpiWarps / 4), buf ^= 1u)
+            for (int c = slot * 8; c < p.OCs; c += 8 * per_set)
                 conv_epilogue_chunk<TAPS>(p, &tmOut, t_row, c, oc0, img, plane, pix, n, valid, has_left, has_right,
-                                    my_stage + buf * 1024u, lane, threadIdx.x == 64 && lt == 0 && c == 0);
+                                    my_stage, lane, threadIdx.x == 64 && lt == 0 && c == 0);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&cs.tempty[a]));
             if (threadIdx.x == 64 && lt == 0) CB_TRACE_EVENT(p.trace, 8);
             if (threadIdx.x == 64) CB_TRACE_EVENT(p.trace, 10);
         }
-        // this warp's stores must be complete before its staging memory is released with the CTA
-        if (p.tma_out && lane == 0) tma_store_wait_all<0>();
+        // this warp's stores must have read their staging memory before it is released with the CTA (the writes themselves
+        // are complete when the grid is)
+        if (p.tma_out && lane == 0) tma_store_wait_read<0>();
     }
 
     tc_fence_before();
@@ -397,8 +405,8 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps <= 8 ? 2 : 1)
         // A bounded wait gave up somewhere in this CTA. Copies armed before that may still be in flight towards this
         // CTA's shared memory and issued MMAs may still be running on its accumulators: give both a bounded chance to
         // finish before the shared memory and TMEM are released.
+        if (warp == 1 && lane == 0) mbar_drain(smem_u32(&cs.wbar), 0, p.status);
         if (warp == 0 && lane == 0) {
-            mbar_drain(smem_u32(&cs.wbar), 0, p.status);
             const uint32_t n = (uint32_t)p.stages;  // stage st was last filled as number st + n * round: parity of the round
             for (uint32_t st = 0; st < n && st < fills; ++st) mbar_drain(smem_u32(&cs.full[st]), ((fills - 1 - st) / n) & 1u, p.status);
         }
@@ -709,9 +717,9 @@ struct ConvEnv {
 // Geometry the tensor-core forward / data-gradient kernel covers; fills the derived sizes.
 struct ConvPlan {
     int Cin, Cout, OCp, OCs, nsplit, NQ, CG, L, KS, shared_rows, nblocks, stages;
-    int ew;      // epilogue warps of the kernel instantiation: 8 or 16
     int c_wrap = 0;  // set by the caller before planning: input-channel wrap of the 3xTF32 form (0 = none)
     int ks_max = 4;  // set by the caller before planning: most K steps a stage may carry
+    int ew;      // epilogue warps of the kernel instantiation: 8 or 16
     int per_sm;  // CTAs the plan expects to share an SM (2 for narrow outputs with a small filter, else 1)
     size_t w_bytes;       // one CTA's slice of the packed filter
     size_t w_total_bytes; // the whole packed filter
@@ -722,15 +730,6 @@ struct ConvPlan {
 int forced_nsplit() {
     static const int v = [] {
         const char* e = std::getenv("CB_CONV_NSPLIT");
-        return e ? std::atoi(e) : 0;
-    }();
-    return v;
-}
-
-// Development override of the epilogue warp count (8 or 16); 0 = choose from the output width.
-int forced_ew() {
-    static const int v = [] {
-        const char* e = std::getenv("CB_CONV_EW");
         return e ? std::atoi(e) : 0;
     }();
     return v;
@@ -776,14 +775,11 @@ int plan_conv(ConvPlan& q, int smem_optin, int sm_count, const float* X, int N, 
         c.NQ = FW * c.OCs;
         if (c.NQ > 256) continue;
         c.w_bytes = (size_t)FH * c.CG * c.NQ * kRowBytes;
-        // Two epilogue warps per TMEM lane quarter: with four, the waiting and draining warps took issue slots from the
-        // one thread that feeds the tensor core and the wide layers ran 15 % slower. Narrow outputs with a small filter
-        // are sized so that two CTAs fit one SM (shared memory and TMEM halves).
-        c.ew = 8;
-        if (forced_ew() == 8 || forced_ew() == 16) c.ew = forced_ew();
-        const bool two_per_sm = c.OCs <= 32 && c.w_bytes <= 40 * 1024 && c.ew <= 8;
+        // narrow outputs with a small filter are sized so that two CTAs fit one SM (shared memory and TMEM halves)
+        const bool two_per_sm = c.OCs <= 32 && c.w_bytes <= 40 * 1024;
+        c.ew = two_per_sm ? 8 : 16;
         const long long avail = two_per_sm ? (long long)(smem_optin < 113 * 1024 ? smem_optin : 113 * 1024) : (long long)smem_optin;
-        const long long cap = avail - 4096 - (long long)c.w_bytes - 2048LL * c.ew;  // static shared memory, alignment slack;  // 2 KB of store staging per epilogue warp
+        const long long cap = avail - 4096 - (long long)c.w_bytes - 1024LL * c.ew;  // static shared memory, alignment slack; store staging
         // as many K steps per stage as leaves at least 2 stages: fewer, larger TMA boxes measured faster than a deeper
         // pipeline of small ones
         c.KS = 0;
@@ -854,6 +850,7 @@ int launch_conv(cb_ctx* err_ctx, const ConvEnv& env, const ConvPlan& q, const fl
     if (p.total_lines > (1LL << 29)) return fail(err_ctx, CB_EUNSUPPORTED, "convolution: more than 2^29 lines of 32 pixels");
     p.tiles = (int)((p.total_lines + 3) / 4);
     p.stages = q.stages;
+    p.epi_sets = q.OCs / 8 <= q.ew / 8 ? 2 : 1;
     int cols = 32;
     while (cols < 2 * q.NQ) cols <<= 1;
     p.tmem_cols = cols;
@@ -917,7 +914,7 @@ int launch_conv(cb_ctx* err_ctx, const ConvEnv& env, const ConvPlan& q, const fl
         rc = encode_tmap(err_ctx, &tmOut, Y, 3, dims, str, box, nullptr, 0);
         if (rc != CB_OK) return rc;
     }
-    const size_t smem = q.w_bytes + (size_t)p.stages * q.stage_bytes + 2048u * (size_t)q.ew + 1024;
+    const size_t smem = q.w_bytes + (size_t)p.stages * q.stage_bytes + 1024u * (size_t)q.ew + 1024;
     // per device: the opt-in shared-memory size is raised to the maximum once (several host threads may race here)
     static std::once_flag attr_once[64];
     static cudaError_t attr_error[64] = {};
@@ -928,9 +925,9 @@ int launch_conv(cb_ctx* err_ctx, const ConvEnv& env, const ConvPlan& q, const fl
         {umma_conv_kernel<8, TAPS_1>, umma_conv_kernel<8, TAPS_3>, umma_conv_kernel<8, TAPS_2L>, umma_conv_kernel<8, TAPS_2R>},
         {umma_conv_kernel<16, TAPS_1>, umma_conv_kernel<16, TAPS_3>, umma_conv_kernel<16, TAPS_2L>, umma_conv_kernel<16, TAPS_2R>}};
     auto raise_limits = [&]() -> cudaError_t {
-        for (int a = 0; a < 2; ++a)
-            for (int b = 0; b < 4; ++b) {
-                cudaError_t e = cudaFuncSetAttribute(kernels[a][b], cudaFuncAttributeMaxDynamicSharedMemorySize, env.smem_optin - 3072);
+        for (const auto& row : kernels)
+            for (KernelFn k : row) {
+                cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, env.smem_optin - 3072);
                 if (e != cudaSuccess) return e;
             }
         return cudaSuccess;

@@ -91,6 +91,15 @@ __device__ __forceinline__ void shift_dy_chunk(uint32_t src_row, uint32_t row_m1
     }
 }
 
+// The four K steps (8 pixels each) of one line on one M tile; b_units: from the A tile to the line's B rows.
+__device__ __forceinline__ void issue_line(uint32_t d_tmem, uint64_t dA, uint32_t b_units, uint32_t idesc, uint32_t accumulate) {
+    const uint64_t dB = dA + (uint64_t)b_units;
+    umma_tf32_elect(d_tmem, dA, dB, idesc, accumulate);
+    umma_tf32_elect(d_tmem, dA + 2, dB + 2, idesc, 1u);
+    umma_tf32_elect(d_tmem, dA + 4, dB + 4, idesc, 1u);
+    umma_tf32_elect(d_tmem, dA + 6, dB + 6, idesc, 1u);
+}
+
 __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
     umma_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmdY,
                       const __grid_constant__ CUtensorMap tmXlo, const __grid_constant__ CUtensorMap tmdYlo,
@@ -184,6 +193,7 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
         // The whole warp runs the loop with the same values (waits go through votes) and one elected lane issues: the
         // descriptors stay in uniform registers (see umma_tf32_elect).
         const bool shifted = p.FW > 1;
+        const uint32_t line_units = p.line_bytes >> 4, a_units = p.a_bytes >> 4;  // descriptor address units
         uint32_t s = 0, ph = 0, ahead = 0;
         bool first_line = true;
         for (int g = blockIdx.x; g < p.vgroups; g += gridDim.x) {
@@ -197,19 +207,18 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
             ahead = mbar_test(smem_u32(shifted ? &ws.xf[s1] : &ws.full[s1]), ph1);
             tc_fence_after();
             if (lane == 0 && first_line) CB_TRACE_EVENT(p.trace, 5);
-            for (int l = 0; l < p.lps; ++l) {
-                const uint32_t stg = st_base + s * p.stage_bytes + (uint32_t)l * p.line_bytes;
-                const uint64_t dA0 = desc0 + (uint64_t)((stg >> 4) & 0x3FFFu);
-                const uint64_t dB0 = desc0 + (uint64_t)(((stg + p.a_bytes) >> 4) & 0x3FFFu);
-                const uint32_t first = (first_line && l == 0) ? 0u : 1u;
-                for (int m = 0; m < p.mtiles; ++m) {
-                    const uint64_t dA = dA0 + (uint64_t)(m * (16384 >> 4));
-                    const uint32_t d = tmem_base + (uint32_t)m * p.NQ;
-                    umma_tf32_elect(d, dA, dB0, idesc, first);
-                    umma_tf32_elect(d, dA + 2, dB0 + 2, idesc, 1u);
-                    umma_tf32_elect(d, dA + 4, dB0 + 4, idesc, 1u);
-                    umma_tf32_elect(d, dA + 6, dB0 + 6, idesc, 1u);
-                }
+            const uint64_t stg = desc0 + (uint64_t)(((st_base + s * p.stage_bytes) >> 4) & 0x3FFFu);
+            if (p.lps == 4 && p.mtiles == 1) {  // the narrow layers: 16 small UMMAs, whose loop would cost as much as they do
+#pragma unroll
+                for (uint32_t l = 0; l < 4; ++l)
+                    issue_line(tmem_base, stg + (uint64_t)(l * line_units), a_units, idesc, first_line && l == 0 ? 0u : 1u);
+            } else {
+                for (uint32_t l = 0; l < (uint32_t)p.lps; ++l)
+                    for (uint32_t m = 0; m < (uint32_t)p.mtiles; ++m) {
+                        const uint32_t shift = m * (16384u >> 4);
+                        issue_line(tmem_base + m * (uint32_t)p.NQ, stg + (uint64_t)(l * line_units + shift), a_units - shift, idesc,
+                                   first_line && l == 0 ? 0u : 1u);
+                    }
             }
             tc_commit_elect(smem_u32(&ws.empty[s]));
             if (g + (int)gridDim.x >= p.vgroups) tc_commit_elect(smem_u32(&ws.tfull));
@@ -219,9 +228,38 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
             s = s1;
             ph = ph1;
         }
-    } else if (warp < 6) {
-        // ------------------------------------------------------------ epilogue: partial sums to the workspace
-        const int quarter = warp & 3;
+    } else {
+        // ------------------------------------------------------------ shift warps (6..): fw = 0 and fw = 2 copies of dY
+        if (warp >= 6 && p.FW > 1) {
+            const int t = threadIdx.x - 192;
+            uint32_t s = 0, ph = 0;
+            // item = (row, 16-byte chunk) of a line; a thread's items keep their chunk (32 * kShiftWarps is a multiple of 8)
+            const int rows = p.lps * p.OCp, q = t & 7;
+            for (int g = blockIdx.x; g < p.vgroups; g += gridDim.x) {
+                if (!mbar_wait_uniform(smem_u32(&ws.full[s]), ph, abort_flag, p.status, CBK_TIMEOUT_XFORM_FULL)) break;
+                const uint32_t base = st_base + s * p.stage_bytes + p.a_bytes + (uint32_t)centre * set_bytes;
+                int l = 0, row = t >> 3;
+                for (int r = t >> 3; r < rows; r += 4 * kShiftWarps, row += 4 * kShiftWarps) {
+                    while (row >= p.OCp) {
+                        row -= p.OCp;
+                        ++l;
+                    }
+                    const uint32_t src = base + (uint32_t)l * p.line_bytes + (uint32_t)row * kRowBytes;
+                    const uint32_t m1 = centre >= 1 ? src - set_bytes : 0u;             // tap fw = pW - 1
+                    const uint32_t p1 = centre + 1 < p.FW ? src + set_bytes : 0u;       // tap fw = pW + 1
+                    shift_dy_chunk(src, m1, p1, q, p.W);
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&ws.xf[s]));
+                if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
+            }
+        }
+
+        // ------------------------------------------------------------ epilogue: twelve warps, three per TMEM lane quarter
+        // (four warps alone spent 4000 clocks on the tile of a 64-channel layer)
+        const int quarter = warp & 3, slot = (warp - 2) >> 2;
+        constexpr int kEpiSlots = (4 + kShiftWarps) / 4;
         const bool ok = mbar_wait_warp(smem_u32(&ws.tfull), 0, lane, abort_flag, p.status, CBK_TIMEOUT_TMEM_FULL, 128);
         if (threadIdx.x == 64) CB_TRACE_EVENT(p.trace, 8);
         if (ok) {
@@ -247,7 +285,7 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
                     pw = phase & 1;
                 }
                 const uint32_t t_row = tmem_base + (uint32_t)m * p.NQ + ((uint32_t)(32 * quarter) << 16);
-                for (int c0 = 0; c0 < p.NQ; c0 += 16) {
+                for (int c0 = slot * 16; c0 < p.NQ; c0 += 16 * kEpiSlots) {
                     uint32_t v[16];
                     tmem_ld16(t_row + (uint32_t)c0, v);
                     tmem_ld_wait();
@@ -269,7 +307,7 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
                 // partial[cta][col][row]: for one column the warp's 32 rows are 128 contiguous bytes
                 float* dst = p.partial + (p.atomic ? 0LL : (long long)blockIdx.x * p.NQ * rows_tot) + r;
                 const uint32_t t_row = tmem_base + (uint32_t)m * p.NQ + ((uint32_t)(32 * quarter) << 16);
-                for (int c = 0; c < p.NQ; c += 16) {
+                for (int c = slot * 16; c < p.NQ; c += 16 * kEpiSlots) {
                     uint32_t v[16];
                     tmem_ld16(t_row + (uint32_t)c, v);
                     tmem_ld_wait();
@@ -283,33 +321,6 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
                         }
                     }
                 }
-            }
-        }
-    } else {
-        // ------------------------------------------------------------ shift warps: fw = 0 and fw = 2 copies of dY
-        if (p.FW > 1) {
-            const int t = threadIdx.x - 192;
-            uint32_t s = 0, ph = 0;
-            // item = (row, 16-byte chunk) of a line; a thread's items keep their chunk (32 * kShiftWarps is a multiple of 8)
-            const int rows = p.lps * p.OCp, q = t & 7;
-            for (int g = blockIdx.x; g < p.vgroups; g += gridDim.x) {
-                if (!mbar_wait_uniform(smem_u32(&ws.full[s]), ph, abort_flag, p.status, CBK_TIMEOUT_XFORM_FULL)) break;
-                const uint32_t base = st_base + s * p.stage_bytes + p.a_bytes + (uint32_t)centre * set_bytes;
-                int l = 0, row = t >> 3;
-                for (int r = t >> 3; r < rows; r += 4 * kShiftWarps, row += 4 * kShiftWarps) {
-                    while (row >= p.OCp) {
-                        row -= p.OCp;
-                        ++l;
-                    }
-                    const uint32_t src = base + (uint32_t)l * p.line_bytes + (uint32_t)row * kRowBytes;
-                    const uint32_t m1 = centre >= 1 ? src - set_bytes : 0u;             // tap fw = pW - 1
-                    const uint32_t p1 = centre + 1 < p.FW ? src + set_bytes : 0u;       // tap fw = pW + 1
-                    shift_dy_chunk(src, m1, p1, q, p.W);
-                }
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&ws.xf[s]));
-                if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
             }
         }
     }
@@ -339,15 +350,24 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
         // the whole CTA adds the staged tile into dW: consecutive threads, consecutive addresses within a run
         const int total = p.OC * p.run;
         float* out = p.dW + p.base_off;
+        // every CTA starts at another place of the filter: in step they would all add into the same few lines at once
+        const int chunk = (p.vec4 ? 4 : 1) * (int)blockDim.x, chunks = (total + chunk - 1) / chunk, padded = chunks * chunk;
+        const int rotation = (int)((long long)blockIdx.x * chunks / gridDim.x);
         if (p.vec4) {  // runs start on 16-byte boundaries and are whole float4s: one vector add per four weights
-            for (int i = 4 * (int)threadIdx.x; i < total; i += 4 * (int)blockDim.x) {
+            for (int k = 4 * (int)threadIdx.x; k < padded; k += chunk) {
+                int i = k + rotation * chunk;
+                if (i >= padded) i -= padded;
+                if (i >= total) continue;
                 const int oc = i / p.run, j = i - oc * p.run;
                 float4 v;
                 asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(st_base + 4u * (uint32_t)i));
                 asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(out + (long long)oc * p.oc_stride + j), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
             }
         } else {
-            for (int i = threadIdx.x; i < total; i += blockDim.x) {
+            for (int k = threadIdx.x; k < padded; k += blockDim.x) {
+                int i = k + rotation * chunk;
+                if (i >= padded) i -= padded;
+                if (i >= total) continue;
                 const int oc = i / p.run, j = i - oc * p.run;
                 float v;
                 asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(st_base + 4u * (uint32_t)i));
