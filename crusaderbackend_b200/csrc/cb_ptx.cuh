@@ -285,6 +285,11 @@ __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* tm, uint32_
                  "r"(src), "r"(c0), "r"(c1), "r"(c2)
                  : "memory");
 }
+// One thread. global[0 .. bytes) += shared[0 .. bytes) as fp32; both addresses on 16 bytes, bytes a multiple of 16.
+__device__ __forceinline__ void bulk_reduce_add_f32(float* dst, uint32_t src, uint32_t bytes) {
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes)
+                 : "memory");
+}
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Waits until at most N of this thread's committed store groups are still READING their shared-memory source.
 template <int N>

@@ -29,6 +29,7 @@ struct WgradParams {
     int Cp, OCp, NQ, mtiles, rowsA;  // rowsA = FH * Cp valid accumulator rows
     int L, LPI;
     long long total_lines;
+    int nsplit;                      // CTAs that share a line group, each taking OCp of the output channels (below)
     int lps;                         // lines per pipeline stage
     int groups;                      // ceil(total_lines / lps)
     // 3xTF32 in one launch: the line groups are walked three times, as (lo part of X, dY), (X, lo part of dY) and
@@ -111,6 +112,9 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
     volatile int* abort_flag = &ws.abort_flag;
     const uint32_t st_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t set_bytes = (uint32_t)p.OCp * kRowBytes;
+    // this CTA's output channels and its walk over the line groups
+    const int oc_first = ((int)blockIdx.x % p.nsplit) * p.OCp, oc_here = min(p.OCp, p.OC - oc_first);
+    const int cta = (int)blockIdx.x / p.nsplit, ctas = (int)gridDim.x / p.nsplit;
     const int centre = p.pW;  // (fw, oc) rows of the N side: the unshifted copy is the tap with fw - pW == 0
 
     if (threadIdx.x == 0) {
@@ -151,7 +155,7 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
         // ------------------------------------------------------------ TMA producer
         uint32_t s = 0, ph = 0, ahead = 0;
         const bool x3 = p.vgroups > p.groups;
-        for (int g = blockIdx.x; g < p.vgroups; g += gridDim.x) {
+        for (int g = cta; g < p.vgroups; g += ctas) {
             if (!__all_sync(0xffffffffu, ahead) &&
                 !mbar_wait_uniform(smem_u32(&ws.empty[s]), ph ^ 1u, abort_flag, p.status, CBK_TIMEOUT_EMPTY))
                 break;
@@ -176,7 +180,7 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
                     for (int fh = 0; fh < p.FH; ++fh)
                         tma_load_3d_elect(stg + (uint32_t)fh * p.Cp * kRowBytes, mx, full, (h0 + fh - p.pH) * p.W, 0, n);
                 }
-                tma_load_3d_elect(stg + p.a_bytes + (uint32_t)centre * set_bytes, my, full, h0 * p.W, 0, n);
+                tma_load_3d_elect(stg + p.a_bytes + (uint32_t)centre * set_bytes, my, full, h0 * p.W, oc_first, n);
                 if (++line == p.LPI) {
                     line = 0;
                     ++n;
@@ -196,7 +200,7 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
         const uint32_t line_units = p.line_bytes >> 4, a_units = p.a_bytes >> 4;  // descriptor address units
         uint32_t s = 0, ph = 0, ahead = 0;
         bool first_line = true;
-        for (int g = blockIdx.x; g < p.vgroups; g += gridDim.x) {
+        for (int g = cta; g < p.vgroups; g += ctas) {
             // with shifted copies the shift warps' arrival implies that the copies' source has landed; the rest of the
             // stage is part of the same transaction count
             if (!__all_sync(0xffffffffu, ahead) &&
@@ -221,9 +225,9 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
                     }
             }
             tc_commit_elect(smem_u32(&ws.empty[s]));
-            if (g + (int)gridDim.x >= p.vgroups) tc_commit_elect(smem_u32(&ws.tfull));
+            if (g + ctas >= p.vgroups) tc_commit_elect(smem_u32(&ws.tfull));
             if (lane == 0 && first_line) CB_TRACE_EVENT(p.trace, 6);
-            if (lane == 0 && g + (int)gridDim.x >= p.vgroups) CB_TRACE_EVENT(p.trace, 7);
+            if (lane == 0 && g + ctas >= p.vgroups) CB_TRACE_EVENT(p.trace, 7);
             first_line = false;
             s = s1;
             ph = ph1;
@@ -235,7 +239,7 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
             uint32_t s = 0, ph = 0;
             // item = (row, 16-byte chunk) of a line; a thread's items keep their chunk (32 * kShiftWarps is a multiple of 8)
             const int rows = p.lps * p.OCp, q = t & 7;
-            for (int g = blockIdx.x; g < p.vgroups; g += gridDim.x) {
+            for (int g = cta; g < p.vgroups; g += ctas) {
                 if (!mbar_wait_uniform(smem_u32(&ws.full[s]), ph, abort_flag, p.status, CBK_TIMEOUT_XFORM_FULL)) break;
                 const uint32_t base = st_base + s * p.stage_bytes + p.a_bytes + (uint32_t)centre * set_bytes;
                 int l = 0, row = t >> 3;
@@ -295,12 +299,13 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
                         const uint32_t dst = st_base + 4u * (uint32_t)(oc0 * p.run + roff + sw);
 #pragma unroll
                         for (int e = 0; e < 16; ++e)
-                            if (oc0 + e < p.OC)
+                            if (oc0 + e < oc_here)
                                 asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + 4u * (uint32_t)(e * p.run)), "f"(__uint_as_float(v[e])) : "memory");
                     }
                     __syncwarp();  // the next tcgen05.ld is warp-wide
                 }
             }
+            if (p.direct) fence_proxy_async_smem();  // the tile leaves through bulk copies
             for (int m = 0; m < p.mtiles && !p.direct; ++m) {
                 const int r = m * 128 + 32 * quarter + lane;
                 if (m * 128 + 32 * quarter >= p.rowsA) continue;  // warp-uniform: no valid row in this quarter
@@ -347,24 +352,28 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
         tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
     }
     if (p.direct && !ws.abort_flag) {
-        // the whole CTA adds the staged tile into dW: consecutive threads, consecutive addresses within a run
-        const int total = p.OC * p.run;
-        float* out = p.dW + p.base_off;
-        // every CTA starts at another place of the filter: in step they would all add into the same few lines at once
-        const int chunk = (p.vec4 ? 4 : 1) * (int)blockDim.x, chunks = (total + chunk - 1) / chunk, padded = chunks * chunk;
-        const int rotation = (int)((long long)blockIdx.x * chunks / gridDim.x);
-        if (p.vec4) {  // runs start on 16-byte boundaries and are whole float4s: one vector add per four weights
-            for (int k = 4 * (int)threadIdx.x; k < padded; k += chunk) {
-                int i = k + rotation * chunk;
-                if (i >= padded) i -= padded;
-                if (i >= total) continue;
-                const int oc = i / p.run, j = i - oc * p.run;
-                float4 v;
-                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(st_base + 4u * (uint32_t)i));
-                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(out + (long long)oc * p.oc_stride + j), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+        // The staged tile is added into dW, every CTA starting at another place of it: in step they would all add into the
+        // same few lines at once.
+        float* out = p.dW + p.base_off + (long long)oc_first * p.oc_stride;
+        if (p.vec4) {
+            // runs start on 16-byte boundaries and are whole float4s: bulk copies that add on arrival, of a run each or,
+            // where the runs are contiguous, of 4 KB (the same through vector atomics of 448 threads took 10,000 clocks for
+            // a 64-channel layer, most of the kernel)
+            const bool whole = p.oc_stride == p.run;
+            const int total = oc_here * p.run, piece = whole ? 1024 : p.run;  // floats
+            const int pieces = (total + piece - 1) / piece;
+            const int rotation = (int)((long long)cta * pieces / ctas);
+            for (int k = threadIdx.x; k < pieces; k += blockDim.x) {
+                const int i = k + rotation < pieces ? k + rotation : k + rotation - pieces;
+                const int n = min(piece, total - i * piece);
+                bulk_reduce_add_f32(out + (long long)i * (whole ? piece : p.oc_stride), st_base + 4u * (uint32_t)(i * piece), 4u * (uint32_t)n);
             }
+            tma_store_commit();
+            tma_store_wait_read<0>();
         } else {
-            for (int k = threadIdx.x; k < padded; k += blockDim.x) {
+            const int total = oc_here * p.run, chunk = (int)blockDim.x, padded = (total + chunk - 1) / chunk * chunk;
+            const int rotation = (int)((long long)cta * (padded / chunk) / ctas);
+            for (int k = threadIdx.x; k < padded; k += chunk) {
                 int i = k + rotation * chunk;
                 if (i >= padded) i -= padded;
                 if (i >= total) continue;
@@ -481,23 +490,6 @@ struct LoParts {
     long long x_batch = 0, dy_batch = 0;
 };
 
-// Development override of the lines per stage (1, 2 or 4); 0 = choose from the stage size.
-int forced_lps() {
-    static const int v = [] {
-        const char* e = std::getenv("CB_WGRAD_LPS");
-        return e ? std::atoi(e) : 0;
-    }();
-    return v;
-}
-// Development override of the fewest line groups a CTA takes; 0 = from the 256-pixel rule.
-int forced_min_groups() {
-    static const int v = [] {
-        const char* e = std::getenv("CB_WGRAD_MINGROUPS");
-        return e ? std::atoi(e) : 0;
-    }();
-    return v;
-}
-
 }  // namespace
 
 // dW (+)= contraction over the pixels of N x Cin x IH x IW planes `X` and N x OC x IH x IW planes `dY` with taps
@@ -512,32 +504,71 @@ static int wgrad_core(cb_ctx* ctx, const float* dY, const float* X, float* dW, i
     const int L = 32 / IW;
     if (IH % L) return CB_EUNSUPPORTED;
     const int Cp = (Cin + 7) / 8 * 8;
-    const int OCp = (OC + 15) / 16 * 16;
-    const int NQ = FW * OCp;
     const int rowsA = FH * Cp;
     const int mtiles = (rowsA + 127) / 128;
-    if (NQ > 256 || Cp > 256 || OCp > 128 || mtiles * NQ > 512) return CB_EUNSUPPORTED;
+    if (Cp > 256 || (OC + 15) / 16 * 16 > 128) return CB_EUNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(X) & 15u) || (reinterpret_cast<uintptr_t>(dY) & 15u)) return CB_EUNSUPPORTED;
-    int rows_stage = rowsA + NQ;
-    if (rows_stage < mtiles * 128) rows_stage = mtiles * 128;
-    const uint32_t line_bytes = ((uint32_t)rows_stage * kRowBytes + 1023u) & ~1023u;
     const long long smem_cap = (long long)ctx->max_smem_optin - 2048;
-    if (smem_cap / line_bytes < 2) return CB_EUNSUPPORTED;
-    int lps = 1;
-    for (int cand = 4; cand >= 2; cand >>= 1)
-        if (smem_cap / ((long long)cand * line_bytes) >= 3) { lps = cand; break; }
-    if (forced_lps() && smem_cap / ((long long)forced_lps() * line_bytes) >= 2) lps = forced_lps();
-    const uint32_t stage_bytes = (uint32_t)lps * line_bytes;
-    long long stages = smem_cap / stage_bytes;
-    if (stages > kConvMaxStages) stages = kConvMaxStages;
+    const int max_ctas = ctx->wgrad_grid_cap > 0 && ctx->wgrad_grid_cap < ctx->sm_count ? ctx->wgrad_grid_cap : ctx->sm_count;
+    const long long total_lines = (long long)N * (IH / L), passes = lo.x ? 3 : 1;
+    if (total_lines > (1LL << 29)) return CB_EUNSUPPORTED;
+    const int run = s2 ? IC_src * 9 : Cin * FH * FW;
+    // The output channels of a line group go to one CTA or are shared by two or four. An SM adds into global memory at about
+    // 14 bytes a clock whatever the form of the atomics, so a 64-channel layer's 147 KB tile takes 10,000 clocks to leave a
+    // CTA; sharing divides that (and the UMMAs of a line) while X is fetched once more for each share. Small maps gain
+    // (64 -> 64 at 8 x 8), large ones, bound by fetching, do not. Clocks of a launch by candidate:
+    struct Shape {
+        int nsplit, OCp, NQ, lps, grid;
+        uint32_t line_bytes;
+        long long stages;
+    } sh{};
+    double best_cost = 1e300;
+    for (int ns = 1; ns <= 4; ns <<= 1) {
+        Shape c{};
+        c.nsplit = ns;
+        c.OCp = ((OC + ns - 1) / ns + 15) / 16 * 16;
+        if (ns > 1 && (ctx->deterministic || c.OCp * (ns - 1) >= OC)) break;
+        c.NQ = FW * c.OCp;
+        if (c.NQ > 256 || mtiles * c.NQ > 512) continue;
+        int rows_stage = rowsA + c.NQ;
+        if (rows_stage < mtiles * 128) rows_stage = mtiles * 128;
+        c.line_bytes = ((uint32_t)rows_stage * kRowBytes + 1023u) & ~1023u;
+        if (smem_cap / c.line_bytes < 2) continue;
+        // as many lines per stage as leave three stages: the hand-offs between the roles are paid per stage
+        c.lps = 1;
+        for (int cand = 4; cand >= 2; cand >>= 1)
+            if (smem_cap / ((long long)cand * c.line_bytes) >= 3) { c.lps = cand; break; }
+        c.stages = smem_cap / ((long long)c.lps * c.line_bytes);
+        if (c.stages > kConvMaxStages) c.stages = kConvMaxStages;
+        const long long tile_bytes = 4LL * c.OCp * run;
+        if (ns > 1 && tile_bytes > c.stages * c.lps * (long long)c.line_bytes) continue;  // only the staged flush knows shares
+        const long long groups = (total_lines + c.lps - 1) / c.lps * passes;
+        long long per_share = max_ctas / ns;
+        if (per_share < 1) break;
+        if (per_share > groups) per_share = groups;
+        c.grid = (int)per_share * ns;
+        const double umma = c.NQ <= 96 ? 58.0 : 0.52 * c.NQ, fetch = (rowsA + c.OCp) * kRowBytes / 27.0;
+        const double issue = 4.0 * mtiles * umma + 60.0;
+        const double line = issue > fetch ? issue : fetch;
+        const double cost = (double)((groups + per_share - 1) / per_share) * c.lps * line + (double)tile_bytes / 14.0 +
+                            12.0 * mtiles * c.NQ;
+        if (cost < best_cost) {
+            best_cost = cost;
+            sh = c;
+        }
+    }
+    if (sh.nsplit == 0) return CB_EUNSUPPORTED;
+    const int OCp = sh.OCp, NQ = sh.NQ, lps = sh.lps, grid = sh.grid;
+    const uint32_t line_bytes = sh.line_bytes, stage_bytes = (uint32_t)lps * line_bytes;
+    const long long stages = sh.stages;
 
     WgradParams p{};
     p.N = N; p.Cin = Cin; p.H = IH; p.W = IW; p.OC = OC;
     p.FH = FH; p.FW = FW; p.pH = pH; p.pW = pW;
     p.Cp = Cp; p.OCp = OCp; p.NQ = NQ; p.mtiles = mtiles; p.rowsA = rowsA;
     p.L = L; p.LPI = IH / L;
-    p.total_lines = (long long)N * p.LPI;
-    if (p.total_lines > (1LL << 29)) return CB_EUNSUPPORTED;
+    p.total_lines = total_lines;
+    p.nsplit = sh.nsplit;
     p.stages = (int)stages;
     int cols = 32;
     while (cols < mtiles * NQ) cols <<= 1;
@@ -550,45 +581,16 @@ static int wgrad_core(cb_ctx* ctx, const float* dY, const float* X, float* dW, i
     p.vgroups = lo.x ? 3 * p.groups : p.groups;
     p.status = ctx->d_status;
     p.trace = ctx->trace;
-    // One CTA per line group up to the SM count: fewer, longer CTAs (fewer partial sums to write and reduce) measured
-    // slower on every layer shape of the models.
-    int min_groups = forced_min_groups() ? forced_min_groups() : 1;
-    int grid = p.vgroups / min_groups;
-    if (grid < 1) grid = 1;
-    if (grid > ctx->sm_count) grid = ctx->sm_count;
-    static const int max_grid = [] {
-        const char* e = std::getenv("CB_WGRAD_MAXGRID");  // development override
-        return e ? std::atoi(e) : 0;
-    }();
-    if (max_grid > 0 && grid > max_grid) grid = max_grid;
-    else if (max_grid == 0 && ctx->wgrad_grid_cap > 0 && grid > ctx->wgrad_grid_cap) grid = ctx->wgrad_grid_cap;
     // Partial sums: one tile per CTA added in a fixed order by the second kernel (deterministic contexts), or one
     // zero-filled tile that every CTA adds into with atomics and the second kernel moves into dW and clears again.
-    static const int allow_atomic = [] {
-        const char* e = std::getenv("CB_WGRAD_ATOMIC");  // development switch, default on
-        return e ? std::atoi(e) : 1;
-    }();
-    p.atomic = (!ctx->deterministic && allow_atomic) ? 1 : 0;
-    static const int allow_direct = [] {
-        const char* e = std::getenv("CB_WGRAD_DIRECT");  // development switch, default on
-        return e ? std::atoi(e) : 1;
-    }();
+    p.atomic = ctx->deterministic ? 0 : 1;
     p.s2 = s2; p.IC_src = IC_src;
-    static const int allow_cf = [] {
-        const char* e = std::getenv("CB_WGRAD_ROWBOX");  // development switch, default on
-        return e ? std::atoi(e) : 1;
-    }();
-    p.rows_cf = (allow_cf && IW == 32 && FH > 1 && !s2) ? 1 : 0;
-    p.run = s2 ? IC_src * 9 : Cin * FH * FW;
+    p.rows_cf = (IW == 32 && FH > 1 && !s2) ? 1 : 0;
+    p.run = run;
     p.oc_stride = s2 ? (long long)IC_src * 9 : (long long)IC_total * FH * FW;
     p.base_off = s2 ? 0 : ((long long)oc_off * IC_total + c_off) * FH * FW;
     p.dW = dW;
-    static const long long direct_limit = [] {
-        const char* e = std::getenv("CB_WGRAD_DIRECT_LIMIT");  // development override: most weights of a direct launch
-        return e ? std::atoll(e) : 1LL << 30;
-    }();
-    p.direct = (p.atomic && allow_direct && (long long)OC * p.run * 4 <= stages * (long long)stage_bytes &&
-                (long long)OC * p.run <= direct_limit) ? 1 : 0;
+    p.direct = (p.atomic && 4LL * OCp * p.run <= stages * (long long)stage_bytes) ? 1 : 0;
     p.vec4 = ((p.run & 3) == 0 && (p.oc_stride & 3) == 0 && (p.base_off & 3) == 0 &&
               (reinterpret_cast<uintptr_t>(dW) & 15u) == 0) ? 1 : 0;
     int rc;
