@@ -4,6 +4,7 @@
 // two gradients (the reference's weight-gradient map at :570-571 is wrong for stride > 1 and is not reproduced).
 #include <cstdlib>
 
+#include "cb_ptx.cuh"
 #include "simt_core.cuh"
 
 namespace cb {
@@ -138,6 +139,8 @@ template <class T, bool MASK>
 __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_gather_simt(const __grid_constant__ GatherParams p) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ TapK table[2 * simt::kBK];
+    griddep_wait();
+    griddep_launch();
     const int set = blockIdx.z / p.splits, split = blockIdx.z - set * p.splits;
     const PixelSet& s = p.sets[set];
     const long long pixels = (long long)p.N * s.UH * s.UW;
@@ -274,6 +277,8 @@ __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_wgrad_simt(const Wgra
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ PixelK table[2 * simt::kBK];
     __shared__ TapI rows[T::BM];
+    griddep_wait();
+    griddep_launch();
     const int i0 = blockIdx.x * T::BM;
     const int taps = p.g.FH * p.g.FW;
     for (int e = threadIdx.x; e < T::BM; e += T::NT) {
@@ -337,8 +342,8 @@ int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, 
             if (er != cudaSuccess) return er;
             const long long gx = (pixels + T::BM - 1) / T::BM, gy = (p.OUTC + T::BN - 1) / T::BN, gz = (long long)count * c.splits;
             if (gx > 0x7fffffffLL || gy > 65535 || gz > 65535) return cudaErrorInvalidConfiguration;
-            kernel<<<dim3((unsigned)gx, (unsigned)gy, (unsigned)gz), T::NT, T::kSmem, ctx->stream>>>(p);
-            return cudaGetLastError();
+            er = launch_dep(ctx, kernel, dim3((unsigned)gx, (unsigned)gy, (unsigned)gz), dim3(T::NT), T::kSmem, p);
+            return er == cudaSuccess ? cudaGetLastError() : er;
         });
         if (e != cudaSuccess) return check_cuda(ctx, e, who);
         ctx->launches += 1;
@@ -403,8 +408,8 @@ int simt_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, con
         if (er != cudaSuccess) return er;
         const long long gx = (I + T::BM - 1) / T::BM, gy = (g.OC + T::BN - 1) / T::BN;
         if (gy > 65535 || c.splits > 65535) return cudaErrorInvalidConfiguration;
-        kernel<<<dim3((unsigned)gx, (unsigned)gy, (unsigned)c.splits), T::NT, T::kSmem, ctx->stream>>>(p);
-        return cudaGetLastError();
+        er = launch_dep(ctx, kernel, dim3((unsigned)gx, (unsigned)gy, (unsigned)c.splits), dim3(T::NT), T::kSmem, p);
+        return er == cudaSuccess ? cudaGetLastError() : er;
     });
     if (e != cudaSuccess) return check_cuda(ctx, e, who);
     ctx->launches += 1;
@@ -431,6 +436,8 @@ int make_geo(cb_ctx* ctx, ConvGeo& g, int N, int IC, int IH, int IW, int OC, int
 // lo[n][i] = lo part of x[n*x_batch + i], written densely (per elements per image)
 __global__ void tf32_lo_kernel(const float* __restrict__ x, float* __restrict__ lo, long long n, long long per,
                                long long x_batch) {
+    griddep_wait();
+    griddep_launch();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const long long img = i / per;
         const float v = x[img * x_batch + (i - img * per)];

@@ -490,6 +490,8 @@ __device__ __forceinline__ float pack_value(const PackJob& j, long long i) {
 }
 
 __global__ void pack_filter_kernel(const PackJob j) {
+    griddep_wait();
+    griddep_launch();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < j.total; i += (long long)gridDim.x * blockDim.x)
         j.Wp[i] = pack_value(j, i);
 }
@@ -827,8 +829,8 @@ PackJob make_job(const PackSpec& ps, const ConvPlan& q, const float* W, float* d
 int launch_pack(cb_ctx* err_ctx, const ConvEnv& env, const PackJob& j) {
     int grid = (int)((j.total + 255) / 256);
     if (grid > env.sm_count * 8) grid = env.sm_count * 8;
-    pack_filter_kernel<<<grid, 256, 0, env.stream>>>(j);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_dep_on(env.stream, err_ctx && err_ctx->pdl, pack_filter_kernel, dim3((unsigned)grid), dim3(256), 0, 1, j);
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return check_cuda(err_ctx, e, "pack_filter_kernel launch");
     return CB_OK;
 }

@@ -2,6 +2,7 @@
 // and split-K kernels for thin products.
 #include <utility>
 
+#include "cb_ptx.cuh"
 #include "simt_core.cuh"
 
 namespace cb {
@@ -66,6 +67,8 @@ struct GemmSource {
 template <class T, bool P_MN, bool Q_MN>
 __global__ void __launch_bounds__(T::NT, T::kMinCtas) simt_gemm_kernel(const SimtParams p) {
     extern __shared__ __align__(16) uint8_t smem[];
+    griddep_wait();
+    griddep_launch();
     const int b = blockIdx.z / p.splits, split = blockIdx.z - b * p.splits;
     const int i0 = blockIdx.x * T::BM, j0 = blockIdx.y * T::BN;
     GemmSource<T, P_MN, Q_MN> src{p, b, i0, j0, split * p.k_per_split};
@@ -130,6 +133,8 @@ template <int IT>
 __global__ void __launch_bounds__(256) thin_gemm_k_kernel(const SimtParams p) {
     __shared__ float sP[IT][kThinK];
     constexpr int NV = 4 * IT;
+    griddep_wait();
+    griddep_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int j0 = blockIdx.x * 32 + warp * 4;
     const int k_begin = blockIdx.y * p.k_per_split, k_end = min(p.K, k_begin + p.k_per_split);
@@ -185,7 +190,9 @@ __global__ void __launch_bounds__(256) thin_gemm_k_kernel(const SimtParams p) {
 template <int IT>
 __global__ void __launch_bounds__(256) thin_gemm_mn_kernel(const SimtParams p) {
     __shared__ float sP[IT][kThinK];
-    __shared__ float part[8][32];
+    __shared__ float part[IT][8][32];
+    griddep_wait();
+    griddep_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int j = blockIdx.x * 32 + lane;
     const int k_begin = blockIdx.y * p.k_per_split, k_end = min(p.K, k_begin + p.k_per_split);
@@ -196,25 +203,23 @@ __global__ void __launch_bounds__(256) thin_gemm_mn_kernel(const SimtParams p) {
     for (int k0 = k_begin; k0 < k_end; k0 += kThinK) {
         stage_thin<IT>(sP, p, k0, k_end);
         __syncthreads();
+        const int n = min(kThinK, k_end - k0);
 #pragma unroll 8
-        for (int kk = warp; kk < kThinK; kk += 8) {
-            const float q = k0 + kk < k_end ? col[(long long)(k0 + kk) * p.ldq] : 0.f;
+        for (int kk = warp; kk < n; kk += 8) {
+            const float q = col[(long long)(k0 + kk) * p.ldq];
 #pragma unroll
             for (int i = 0; i < IT; ++i) acc[i] = fmaf(sP[i][kk], q, acc[i]);
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < IT; ++i) {
-        part[warp][lane] = acc[i];
-        __syncthreads();
-        if (warp == (i & 7)) {
-            float v = 0.f;
+    for (int i = 0; i < IT; ++i) part[i][warp][lane] = acc[i];
+    __syncthreads();
+    for (int i = warp; i < IT; i += 8) {
+        float v = 0.f;
 #pragma unroll
-            for (int w = 0; w < 8; ++w) v += part[w][lane];
-            store_thin(p, i, j, v, blockIdx.y == 0);
-        }
-        __syncthreads();
+        for (int w = 0; w < 8; ++w) v += part[i][w][lane];
+        store_thin(p, i, j, v, blockIdx.y == 0);
     }
 }
 
@@ -222,8 +227,8 @@ cudaError_t launch_thin(cb_ctx* ctx, const SimtParams& sp, dim3 grid) {
     typedef void (*Kernel)(const SimtParams);
     static const Kernel kernels[2][3] = {{thin_gemm_k_kernel<4>, thin_gemm_k_kernel<8>, thin_gemm_k_kernel<16>},
                                          {thin_gemm_mn_kernel<4>, thin_gemm_mn_kernel<8>, thin_gemm_mn_kernel<16>}};
-    kernels[sp.q_mn ? 1 : 0][sp.I <= 4 ? 0 : (sp.I <= 8 ? 1 : 2)]<<<grid, 256, 0, ctx->stream>>>(sp);
-    return cudaGetLastError();
+    cudaError_t e = launch_dep(ctx, kernels[sp.q_mn ? 1 : 0][sp.I <= 4 ? 0 : (sp.I <= 8 ? 1 : 2)], grid, dim3(256), 0, sp);
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 template <class T>
@@ -234,8 +239,8 @@ cudaError_t launch_tile(cb_ctx* ctx, const SimtParams& sp, dim3 grid) {
     const Kernel k = forms[(sp.p_mn ? 2 : 0) + (sp.q_mn ? 1 : 0)];
     cudaError_t e = raise_dynamic_smem_once(k, ctx->device, ctx->max_smem_optin, nullptr);
     if (e != cudaSuccess) return e;
-    k<<<grid, T::NT, T::kSmem, ctx->stream>>>(sp);
-    return cudaGetLastError();
+    e = launch_dep(ctx, k, grid, dim3(T::NT), T::kSmem, sp);
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 }  // namespace
@@ -274,8 +279,8 @@ int launch_simt_gemm(cb_ctx* ctx, const GemmCall& g_in) {
         const int jblocks = (g.J + 31) / 32;
         int splits = 1;
         if (may_split) {
-            splits = (2 * ctx->sm_count + jblocks - 1) / jblocks;
-            if (splits > g.K / 64) splits = g.K / 64;
+            splits = 2 * ctx->sm_count / jblocks;
+            if (splits > g.K / 128) splits = g.K / 128;
             if (splits < 1) splits = 1;
         }
         int kps = (g.K + splits - 1) / splits;

@@ -1,6 +1,7 @@
 // Dense-layer entry points lowered onto the GEMM core. Shapes follow seblas::linear / linearXGrad /
 // linearParamGrad (seblas/operations/cuLinear.cu:1052-1115): X is batch x IN, W is OUT x IN, Y is batch x OUT.
 #include "cb_internal.h"
+#include "cb_ptx.cuh"
 
 namespace cb {
 namespace {
@@ -10,10 +11,13 @@ namespace {
 __global__ void __launch_bounds__(256) colsum_add_kernel(const float* __restrict__ dY, float* __restrict__ db,
                                                          int batch, int OUT) {
     __shared__ float part[8][32];
+    griddep_wait();
+    griddep_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int m = blockIdx.x * 32 + lane;
     float s = 0.f;
     if (m < OUT)
+#pragma unroll 8
         for (int n = warp; n < batch; n += 8) s += dY[(long long)n * OUT + m];
     part[warp][lane] = s;
     __syncthreads();
@@ -87,8 +91,8 @@ int cb_linear_paramgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW,
         if (rc != CB_OK) return rc;
     }
     if (db) {
-        colsum_add_kernel<<<(OUT + 31) / 32, 256, 0, ctx->stream>>>(dY, db, batch, OUT);
-        cudaError_t e = cudaGetLastError();
+        cudaError_t e = launch_dep(ctx, colsum_add_kernel, dim3((unsigned)((OUT + 31) / 32)), dim3(256), 0, dY, db, batch, OUT);
+        if (e == cudaSuccess) e = cudaGetLastError();
         if (e != cudaSuccess) return check_cuda(ctx, e, "cb_linear_paramgrad: bias gradient");
         ctx->launches += 1;
     }

@@ -256,6 +256,9 @@ __global__ void __launch_bounds__(256) bn_fwd_par_kernel(const float* __restrict
     const long long p = ((long long)blockIdx.x * PB + threadIdx.x) * 4;
     const bool live = p < P;
     const int g = threadIdx.y;
+    // the parameters are fetched with the samples: behind the sums their latency would be paid on its own
+    const float4 ga = live ? *reinterpret_cast<const float4*>(gamma + p) : f4_zero();
+    const float4 be = live ? *reinterpret_cast<const float4*>(beta + p) : f4_zero();
     float4 x[SPT];
     float4 s[1] = {f4_zero()};
 #pragma unroll
@@ -280,7 +283,6 @@ __global__ void __launch_bounds__(256) bn_fwd_par_kernel(const float* __restrict
     if (!live) return;
     const float4 inv = make_float4(1.0f / sqrtf(v.x + 1e-8f), 1.0f / sqrtf(v.y + 1e-8f), 1.0f / sqrtf(v.z + 1e-8f),
                                    1.0f / sqrtf(v.w + 1e-8f));
-    const float4 ga = *reinterpret_cast<const float4*>(gamma + p), be = *reinterpret_cast<const float4*>(beta + p);
 #pragma unroll
     for (int i = 0; i < SPT; ++i) {
         const int n = g + G * i;
@@ -318,6 +320,7 @@ __global__ void __launch_bounds__(256, SPT <= 4 ? 4 : 1) bn_bwd_par_kernel(const
     const long long p = ((long long)blockIdx.x * PB + threadIdx.x) * 4;
     const bool live = p < P;
     const int g = threadIdx.y;
+    const float4 ga = live ? *reinterpret_cast<const float4*>(gamma + p) : f4_zero();
     float4 x[SPT], dy[SPT];
     float4 s[1] = {f4_zero()};
 #pragma unroll
@@ -340,7 +343,6 @@ __global__ void __launch_bounds__(256, SPT <= 4 ? 4 : 1) bn_bwd_par_kernel(const
     const float invN = 1.0f / (float)N;
     bn_block_sums<1, G>(s, red, tot);
     const float4 m = make_float4(s[0].x * invN, s[0].y * invN, s[0].z * invN, s[0].w * invN);
-    const float4 ga = live ? *reinterpret_cast<const float4*>(gamma + p) : f4_zero();
     // sums of xc^2, dy * xc (dxhat = dy * gamma is factored out below), dy and xc, in one exchange
     float4 sums[4] = {f4_zero(), f4_zero(), f4_zero(), f4_zero()};
 #pragma unroll
@@ -397,10 +399,13 @@ __global__ void __launch_bounds__(256) bn_paramgrad_par_kernel(const float* __re
                                                                float* __restrict__ dgamma, float* __restrict__ dbeta,
                                                                int N, long long P) {
     __shared__ float4 red[16][16];
+    griddep_wait();
+    griddep_launch();
     const long long p = ((long long)blockIdx.x * 16 + threadIdx.x) * 4;
     const bool live = p < P;
     float4 sg = f4_zero(), sb = f4_zero();
     if (live) {
+#pragma unroll 4
         for (int n = threadIdx.y; n < N; n += 16) {
             const float4 h = *reinterpret_cast<const float4*>(xhat + (long long)n * P + p);
             const float4 d = *reinterpret_cast<const float4*>(dY + (long long)n * P + p);
@@ -498,21 +503,35 @@ __device__ __forceinline__ float ew(float a, float b, float c, float s) {
     }
 }
 
-// out[i] = f(a[i], b[i], s). OP_ADD_ZERO_B additionally clears b (gradient hand-over in the backward pass).
+// out[i] = f(a[i], b[i], s). OP_ADD_ZERO_B additionally clears b (gradient hand-over in the backward pass). Bound by memory:
+// four 16-byte vectors a thread are in flight at a time, and a launch begins under the tail of the one before.
 template <int OP, bool VEC>
-__global__ void eltwise_kernel(const float* __restrict__ a, float* __restrict__ b, float* __restrict__ out, float s,
-                               long long n) {
+__global__ void __launch_bounds__(kThreads) eltwise_kernel(const float* __restrict__ a, float* __restrict__ b, float* __restrict__ out,
+                                                           float s, long long n) {
+    griddep_wait();
+    griddep_launch();
     const long long stride = (long long)gridDim.x * blockDim.x;
     if (VEC) {
+        constexpr int U = 4;
         const long long nv = n >> 2;
-        for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += stride) {
-            float4 x = a ? reinterpret_cast<const float4*>(a)[i] : make_float4(0, 0, 0, 0);
-            float4 y = b ? reinterpret_cast<const float4*>(b)[i] : make_float4(0, 0, 0, 0);
-            float4 r;
-            r.x = ew<OP>(x.x, y.x, 0, s); r.y = ew<OP>(x.y, y.y, 0, s);
-            r.z = ew<OP>(x.z, y.z, 0, s); r.w = ew<OP>(x.w, y.w, 0, s);
-            reinterpret_cast<float4*>(out)[i] = r;
-            if (OP == OP_ADD_ZERO_B) reinterpret_cast<float4*>(b)[i] = make_float4(0, 0, 0, 0);
+        for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; i0 < nv; i0 += U * stride) {
+            float4 x[U], y[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const long long i = i0 + u * stride;
+                x[u] = a && i < nv ? reinterpret_cast<const float4*>(a)[i] : make_float4(0, 0, 0, 0);
+                y[u] = b && i < nv ? reinterpret_cast<const float4*>(b)[i] : make_float4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const long long i = i0 + u * stride;
+                if (i >= nv) break;
+                float4 r;
+                r.x = ew<OP>(x[u].x, y[u].x, 0, s); r.y = ew<OP>(x[u].y, y[u].y, 0, s);
+                r.z = ew<OP>(x[u].z, y[u].z, 0, s); r.w = ew<OP>(x[u].w, y[u].w, 0, s);
+                reinterpret_cast<float4*>(out)[i] = r;
+                if (OP == OP_ADD_ZERO_B) reinterpret_cast<float4*>(b)[i] = make_float4(0, 0, 0, 0);
+            }
         }
     } else {
         for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -527,10 +546,9 @@ template <int OP>
 int launch_eltwise(cb_ctx* ctx, const float* a, float* b, float* out, float s, long long n, const char* what) {
     if (n == 0) return CB_OK;
     const bool vec = (n % 4 == 0) && aligned16(a) && aligned16(b) && aligned16(out);
-    const int grid = grid_for(ctx, vec ? n / 4 : n);
-    if (vec) eltwise_kernel<OP, true><<<grid, kThreads, 0, ctx->stream>>>(a, b, out, s, n);
-    else eltwise_kernel<OP, false><<<grid, kThreads, 0, ctx->stream>>>(a, b, out, s, n);
-    cudaError_t e = cudaGetLastError();
+    const int grid = vec ? grid_for(ctx, n / 4, 4 * kThreads) : grid_for(ctx, n);
+    cudaError_t e = launch_dep(ctx, vec ? eltwise_kernel<OP, true> : eltwise_kernel<OP, false>, dim3((unsigned)grid), dim3(kThreads), 0, a, b, out, s, n);
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return check_cuda(ctx, e, what);
     ctx->launches += 1;
     return finish(ctx, what);
@@ -914,7 +932,7 @@ int cb_bn_paramgrad(cb_ctx* ctx, const float* dY, const float* xhat, float* dgam
     if (!dY || !xhat || !dgamma || !dbeta) return fail(ctx, CB_EINVAL, "cb_bn_paramgrad: null operand");
     const bool vec = (P % 4 == 0) && aligned16(xhat) && aligned16(dY);
     if (vec && aligned16(dgamma) && aligned16(dbeta)) {
-        bn_paramgrad_par_kernel<<<(unsigned)((P / 4 + 15) / 16), dim3(16, 16), 0, ctx->stream>>>(dY, xhat, dgamma, dbeta, N, P);
+        launch_dep(ctx, bn_paramgrad_par_kernel, dim3((unsigned)((P / 4 + 15) / 16)), dim3(16, 16), 0, dY, xhat, dgamma, dbeta, N, P);
         return done(ctx, "cb_bn_paramgrad");
     }
     if (vec) bn_paramgrad_kernel<4><<<grid_for(ctx, P / 4, 128), 128, 0, ctx->stream>>>(dY, xhat, dgamma, dbeta, N, P);
