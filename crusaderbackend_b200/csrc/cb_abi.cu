@@ -78,6 +78,7 @@ static int grow_block(cb_ctx* ctx, void** block, size_t* have, size_t bytes, siz
         return CB_ENOMEM;
     }
     *have = want;
+    ctx->scratch_epoch += 1;
     return CB_OK;
 }
 

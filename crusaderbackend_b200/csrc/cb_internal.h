@@ -34,6 +34,7 @@ struct cb_ctx {
     size_t workspace2_bytes = 0;
     void* workspace3 = nullptr;    // scratch: lo parts and partial results of the 3xTF32 convolutions
     size_t workspace3_bytes = 0;
+    long long scratch_epoch = 0;   // counts the reallocations of the scratch blocks above: recorded graphs hold their addresses
     int workspace_frozen = 0;      // 1: a call that would need a larger scratch block fails instead of reallocating
     long long launches = 0;
     int sm_count = 148;
@@ -151,18 +152,17 @@ struct ConvEpilogue {
 };
 // Tensor-core convolution paths. Each returns CB_EUNSUPPORTED, before any work is queued, when the geometry is outside
 // what it covers. in/out batch strides: elements between consecutive images, 0 = densely packed.
+// x3: 3xTF32 in one tensor-core pass.
 int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const ConvEpilogue& ep, int N, int IC, int IH,
                   int IW, int OC, int FH, int FW, int sH, int sW, int pH, int pW, bool dgrad_of, long long in_batch,
-                  long long out_batch);
-// 3xTF32 forward / data gradient in one tensor-core pass (stride 1; conv_sm100.cu), else CB_EUNSUPPORTED.
-int umma_conv_fwd_x3(cb_ctx* ctx, const float* W, const float* X, float* Y, const ConvEpilogue& ep, int N, int IC, int IH,
-                     int IW, int OC, int FH, int FW, int pH, int pW, bool dgrad_of, long long in_batch, long long out_batch);
+                  long long out_batch, bool x3 = false);
 // x3: 3xTF32 in one launch (the kernel walks (lo of X, dY), (X, lo of dY), (X, dY) into one accumulator).
 int umma_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, int N, int IC, int IH, int IW, int OC,
                     int FH, int FW, int sH, int sW, int pH, int pW, int accumulate, long long dy_batch, long long x_batch,
                     bool x3 = false);
 // Packed-filter cache of a context (conv_sm100.cu).
 int filter_cache_repack_all(cb_ctx* ctx);
+bool filter_cache_fresh(const cb_ctx* ctx);  // no convolution would re-pack a filter it has seen before
 void filter_cache_destroy(cb_ctx* ctx);
 
 bool umma_gemm_eligible(const GemmCall& g);

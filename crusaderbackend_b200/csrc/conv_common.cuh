@@ -20,6 +20,9 @@ __host__ __device__ __forceinline__ int s2_tap(int phase, int t) { return phase 
 //   space_to_depth2: Xs[n][phase*C + c][i][j] = X[n][c][2i + (phase >> 1)][2j + (phase & 1)]
 //   subsample2:      Xsub[nc][i][j] = X[nc][2i][2j]
 int launch_space_to_depth2(cb_ctx* ctx, const float* X, float* Xs, int N, int C, int H, int W);
+// space_to_depth2_split: the same followed, Cp planes later, by the lo parts of its values (3xTF32), planes 4C .. Cp zeroed;
+// X on 16 bytes, W a multiple of 4
+int launch_space_to_depth2_split(cb_ctx* ctx, const float* X, float* X2, int N, int C, int Cp, int H, int W);
 int launch_subsample2(cb_ctx* ctx, const float* X, float* Xsub, long long NC, int H, int W);
 
 }  // namespace cb

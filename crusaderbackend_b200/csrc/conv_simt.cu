@@ -476,15 +476,9 @@ int grid_el(const cb_ctx* ctx, long long n) {
 static int conv_3xtf32(cb_ctx* ctx, const float* W, const float* In, float* Out, const ConvEpilogue& ep, int N, int IC,
                        int IH, int IW, int OC, int FH, int FW, int sH, int sW, int pH, int pW, bool dgrad_of,
                        long long in_per, long long out_per, long long out_plane, long long in_batch, long long out_batch) {
-    static const int one_pass = [] {
-        const char* e = std::getenv("CB_CONV_X3_ONEPASS");  // development switch, default on
-        return e ? std::atoi(e) : 1;
-    }();
-    if (one_pass && sH == 1 && sW == 1) {
-        // one pass of the tensor-core kernel over three channel groups, when the tripled filter fits
-        const int rc1 = umma_conv_fwd_x3(ctx, W, In, Out, ep, N, IC, IH, IW, OC, FH, FW, pH, pW, dgrad_of, in_batch, out_batch);
-        if (rc1 != CB_EUNSUPPORTED) return rc1;
-    }
+    // one pass of the tensor-core kernel over three channel groups, when the doubled filter fits
+    const int rc1 = umma_conv_fwd(ctx, W, In, Out, ep, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, dgrad_of, in_batch, out_batch, true);
+    if (rc1 != CB_EUNSUPPORTED) return rc1;
     const long long w_elems = (long long)OC * IC * FH * FW;
     const long long in_elems = in_per * N, out_elems = out_per * N;
     auto up = [](long long n) { return (n + 63) & ~63LL; };
@@ -516,41 +510,6 @@ static int conv_3xtf32(cb_ctx* ctx, const float* W, const float* In, float* Out,
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return check_cuda(ctx, e, "3xTF32 convolution");
     ctx->launches += 3;
-    ctx->last_kernel = "umma_3xtf32";
-    return CB_OK;
-}
-
-// 3xTF32 weight gradient: the products dY_hi X_hi, dY_hi X_lo, dY_lo X_hi in ONE launch of the tensor-core kernel
-// (it walks the pixels three times into one accumulator), or, with that switched off, as three accumulating launches
-// (dense tensors only).
-static int wgrad_3xtf32(cb_ctx* ctx, const float* dY, const float* X, float* dW, int N, int IC, int IH, int IW, int OC, int FH,
-                        int FW, int sH, int sW, int pH, int pW, int accumulate, long long x_elems, long long dy_elems,
-                        long long dy_batch, long long x_batch) {
-    static const int onepass = [] {
-        const char* e = std::getenv("CB_WGRAD_X3_ONEPASS");  // development switch, default on
-        return e ? std::atoi(e) : 1;
-    }();
-    if (onepass) {
-        const int rc1 = umma_conv_wgrad(ctx, dY, X, dW, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, accumulate, dy_batch, x_batch, true);
-        if (rc1 == CB_OK) ctx->last_kernel = "umma_3xtf32";
-        return rc1;
-    }
-    if (dy_batch || x_batch) return CB_EUNSUPPORTED;
-    auto up = [](long long n) { return (n + 63) & ~63LL; };
-    int rc = ensure_workspace3(ctx, (size_t)(up(x_elems) + up(dy_elems)) * sizeof(float));
-    if (rc != CB_OK) return rc;
-    float* x_lo = static_cast<float*>(ctx->workspace3);
-    float* dy_lo = x_lo + up(x_elems);
-    rc = umma_conv_wgrad(ctx, dY, X, dW, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, accumulate, 0, 0);
-    if (rc != CB_OK) return rc;
-    tf32_lo_kernel<<<grid_el(ctx, x_elems), 256, 0, ctx->stream>>>(X, x_lo, x_elems, x_elems, x_elems);
-    tf32_lo_kernel<<<grid_el(ctx, dy_elems), 256, 0, ctx->stream>>>(dY, dy_lo, dy_elems, dy_elems, dy_elems);
-    rc = umma_conv_wgrad(ctx, dY, x_lo, dW, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, 1, 0, 0);
-    if (rc == CB_OK) rc = umma_conv_wgrad(ctx, dy_lo, X, dW, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, 1, 0, 0);
-    if (rc != CB_OK) return rc;
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return check_cuda(ctx, e, "3xTF32 weight gradient");
-    ctx->launches += 2;
     ctx->last_kernel = "umma_3xtf32";
     return CB_OK;
 }
@@ -676,8 +635,9 @@ static int conv_wgrad_impl(cb_ctx* ctx, const float* dY, const float* X, float* 
         rc = umma_conv_wgrad(ctx, dY, X, dW, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, accumulate, dy_batch, x_batch);
         if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;
     } else if (ctx->math == CB_MATH_3XTF32) {
-        rc = wgrad_3xtf32(ctx, dY, X, dW, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, accumulate,
-                          (long long)N * IC * IH * IW, (long long)N * OC * g.OH * g.OW, dy_batch, x_batch);
+        // the products dY_hi X_hi, dY_hi X_lo, dY_lo X_hi in one launch that walks the pixels three times
+        rc = umma_conv_wgrad(ctx, dY, X, dW, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, accumulate, dy_batch, x_batch, true);
+        if (rc == CB_OK) ctx->last_kernel = "umma_3xtf32";
         if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;
     }
     rc = simt_conv_wgrad(ctx, dY, X, dW, g, accumulate ? 1 : 0, who);

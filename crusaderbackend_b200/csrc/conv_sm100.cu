@@ -64,6 +64,7 @@ struct ConvParams {
     float* Out;
     long long out_batch;      // elements between consecutive images of the output
     ConvEpilogue ep;
+    int f_wrap;         // > 0: K steps (8 channels) from f_wrap on take the packed filter's rows f_wrap steps earlier (3xTF32)
     int c_wrap;         // > 0: input channels from c_wrap on are read again from channel (c - c_wrap) (3xTF32 form)
     int* status;
     long long* trace;
@@ -81,7 +82,7 @@ struct __align__(8) ConvSmem {
     int abort_flag;
 };
 
-enum { PACK_FWD = 0, PACK_DGRAD = 1, PACK_S2_FWD = 2, PACK_S2_DGRAD = 3, PACK_FWD_X3 = 4, PACK_DGRAD_X3 = 5 };
+enum { PACK_FWD = 0, PACK_DGRAD = 1, PACK_S2_FWD = 2, PACK_S2_DGRAD = 3 };
 constexpr int kMaxTileUmmas = 256;  // most UMMAs of one tile (filter rows x 8-channel steps) a plan may need
 
 // Horizontal tap sets the kernel is instantiated for: the taps' column offsets fw - pW.
@@ -331,7 +332,9 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps == 8 ? 2 : 1)
                 const uint64_t pbase = descP0 + (uint64_t)(((st_base + s * p.stage_bytes) >> 4) & 0x3FFFu);
                 // a stage holds 1, 2 or 4 K steps of 8 channels, never across a 32-channel group of the packed filter
                 const uint32_t ks0 = (uint32_t)(cb * p.KS);
-                const uint64_t q0 = descQ0 + (uint64_t)((ks0 >> 2) * q_group_units + (ks0 & 3u) * 2u);
+                // 3xTF32: the groups [x ; x_lo ; x] meet the packed groups [w ; w_lo] as w, w, w_lo
+                const uint32_t fs0 = p.f_wrap && ks0 >= (uint32_t)p.f_wrap ? ks0 - (uint32_t)p.f_wrap : ks0;
+                const uint64_t q0 = descQ0 + (uint64_t)((fs0 >> 2) * q_group_units + (fs0 & 3u) * 2u);
                 for (int fh = 0; fh < p.FH; ++fh) {
                     const uint64_t dp = pbase + (uint64_t)((uint32_t)fh * fh_units);
                     const uint64_t dq = q0 + (uint64_t)((uint32_t)fh * q_fh_units);
@@ -434,40 +437,19 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps == 8 ? 2 : 1)
 //                  c' = phase*IC + c: row[c'] = W[o][c][s2_tap(ph, fh)][s2_tap(pw, fw)] (zero where no tap lands)
 //   PACK_S2_DGRAD: its adjoint: input channels are the OC planes of dY, output o' = out_first + o indexes (phase, c),
 //                  taps flipped: row[oc] = W[oc][c][s2_tap(ph, 1-fh)][s2_tap(pw, 1-fw)]
+// x3 > 0 (a multiple of 8, at least the pass's input channels): the packed channels are two groups of x3, the filter and its
+// lo part (3xTF32: lo = rna_tf32(w - hi) with hi the 19 bits the tensor core reads).
 struct PackJob {
     const float* W;
     float* Wp;
-    int OC, IC, FHs, FWs, FHc, FWc, OCp, CG, mode, out_first, out_count;
+    int OC, IC, FHs, FWs, FHc, FWc, OCp, CG, mode, out_first, out_count, x3;
     long long total;  // floats of the packed filter
 };
 
-__device__ __forceinline__ float pack_value(const PackJob& j, long long i) {
-    const int c = (int)(i & 31);
-    long long r = i >> 5;
-    const int o = (int)(r % j.OCp);
-    r /= j.OCp;
-    const int fw = (int)(r % j.FWc);
-    r /= j.FWc;
-    const int cg = (int)(r % j.CG);
-    const int fh = (int)(r / j.CG);
-    const int ch = cg * 32 + c;
+// Value of the packed filter at channel ch of row (fh, fw, o), zero outside the filter.
+__device__ __forceinline__ float pack_source(const PackJob& j, int ch, int fh, int fw, int o) {
     const float* W = j.W;
     const int OC = j.OC, IC = j.IC, FHs = j.FHs, FWs = j.FWs;
-    if (j.mode == PACK_FWD_X3 || j.mode == PACK_DGRAD_X3) {
-        // 3xTF32 in one pass: the convolution runs over three groups of input channels [x ; x_lo ; x] against
-        // [w ; w ; w_lo] (the tensor core reads the hi part of whatever it is given), all into one accumulator
-        const int cin = j.mode == PACK_FWD_X3 ? IC : OC;   // input channels of the convolution the kernel runs
-        const int cout = j.mode == PACK_FWD_X3 ? OC : IC;
-        if (o >= cout || ch >= 3 * cin) return 0.f;
-        const int grp = ch / cin, cc = ch - grp * cin;
-        const float w = j.mode == PACK_FWD_X3 ? W[(((long long)o * IC + cc) * FHs + fh) * FWs + fw]
-                                               : W[(((long long)cc * IC + o) * FHs + (FHs - 1 - fh)) * FWs + (FWs - 1 - fw)];
-        if (grp < 2) return w;
-        const float hi = __uint_as_float(__float_as_uint(w) & 0xFFFFE000u);
-        uint32_t r;
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(w - hi));
-        return __uint_as_float(r);
-    }
     if (j.mode == PACK_FWD) {
         if (o < OC && ch < IC) return W[(((long long)o * IC + ch) * FHs + fh) * FWs + fw];
     } else if (j.mode == PACK_DGRAD) {
@@ -487,6 +469,24 @@ __device__ __forceinline__ float pack_value(const PackJob& j, long long i) {
         }
     }
     return 0.f;
+}
+__device__ __forceinline__ float tf32_lo(float x) {
+    uint32_t r;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u)));
+    return __uint_as_float(r);
+}
+__device__ __forceinline__ float pack_value(const PackJob& j, long long i) {
+    const int c = (int)(i & 31);
+    long long r = i >> 5;
+    const int o = (int)(r % j.OCp);
+    r /= j.OCp;
+    const int fw = (int)(r % j.FWc);
+    r /= j.FWc;
+    const int cg = (int)(r % j.CG);
+    const int fh = (int)(r / j.CG);
+    const int ch = cg * 32 + c;
+    if (j.x3 == 0 || ch < j.x3) return pack_source(j, ch, fh, fw, o);
+    return ch < 2 * j.x3 ? tf32_lo(pack_source(j, ch - j.x3, fh, fw, o)) : 0.f;
 }
 
 __global__ void pack_filter_kernel(const PackJob j) {
@@ -676,29 +676,49 @@ static bool vec_ok(const void* a, const void* b, int W) {
     return (W & 3) == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15u) == 0;
 }
 
-// 3xTF32 in one pass: X2[n][c] = X[n][c] and X2[n][C + c] = lo part of X[n][c] (x = hi + lo with hi the 19 bits the
-// tensor core reads, lo = rna_tf32(x - hi)), four pixels per thread; X may be batch-strided, X2 is dense.
-__global__ void tf32_split2_kernel(const float* __restrict__ X, float* __restrict__ X2, long long per4, long long x_batch,
-                                   long long items) {
+// 3xTF32 in one pass: X2[n][c] = X[n][c] and X2[n][Cp + c] = lo part of X[n][c] (x = hi + lo with hi the 19 bits the
+// tensor core reads, lo = rna_tf32(x - hi)), four pixels per thread; planes C .. Cp of both halves are zeroed (Cp: C rounded up
+// to the 8 channels of a K step). X may be batch-strided, X2 is dense.
+__device__ __forceinline__ float4 lo4(float4 v) { return make_float4(tf32_lo(v.x), tf32_lo(v.y), tf32_lo(v.z), tf32_lo(v.w)); }
+__global__ void tf32_split2_kernel(const float* __restrict__ X, float* __restrict__ X2, long long per4, long long perp4,
+                                   long long x_batch, long long items) {
     griddep_wait();
     griddep_launch();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < items; i += (long long)gridDim.x * blockDim.x) {
-        const long long n = i / per4, r = i - n * per4;
-        const float4 v = *reinterpret_cast<const float4*>(X + n * x_batch + 4 * r);
-        float4 lo;
-        const float in[4] = {v.x, v.y, v.z, v.w};
-        float out[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float hi = __uint_as_float(__float_as_uint(in[e]) & 0xFFFFE000u);
-            uint32_t q;
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(q) : "f"(in[e] - hi));
-            out[e] = __uint_as_float(q);
-        }
-        lo = make_float4(out[0], out[1], out[2], out[3]);
-        float* dst = X2 + n * 8 * per4 + 4 * r;   // a sample of X2 holds 2 * per elements = 8 * per4 floats
-        *reinterpret_cast<float4*>(dst) = v;
-        *reinterpret_cast<float4*>(dst + 4 * per4) = lo;
+        const long long n = i / perp4, r = i - n * perp4;
+        const float4 v = r < per4 ? *reinterpret_cast<const float4*>(X + n * x_batch + 4 * r) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4* dst = reinterpret_cast<float4*>(X2) + n * 2 * perp4 + r;
+        dst[0] = v;
+        dst[perp4] = lo4(v);
+    }
+}
+// The same together with the phase split of a stride-2 convolution: X2 holds 2 * Cp planes of H/2 x W/2, the 4 C phase planes
+// of X and, Cp planes later, their lo parts (Cp: 4 C rounded up to a multiple of 8, the planes between zeroed).
+__global__ void space_to_depth2_split_kernel(const float* __restrict__ X, float* __restrict__ X2, int C, int Cp, int H, int W,
+                                             long long items) {
+    griddep_wait();
+    griddep_launch();
+    const int H2 = H / 2, W2 = W / 2, WQ = W / 4;
+    const long long half = (long long)Cp * H2 * W2, pad = (long long)(Cp - 4 * C) * H2 * W2;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < items; i += (long long)gridDim.x * blockDim.x) {
+        const int q = (int)(i % WQ);
+        long long r = i / WQ;
+        const int y = (int)(r % H);
+        r /= H;
+        const int c = (int)(r % C);
+        const long long n = r / C;
+        const float4 v = *reinterpret_cast<const float4*>(X + ((n * C + c) * H + y) * W + 4 * q);
+        const float4 l = lo4(v);
+        const int row = y & 1;
+        float* d0 = X2 + n * 2 * half + ((2LL * row * C + c) * H2 + (y >> 1)) * W2 + 2 * q;  // phase (row, 0)
+        float* d1 = d0 + (long long)C * H2 * W2;                                             // phase (row, 1)
+        *reinterpret_cast<float2*>(d0) = make_float2(v.x, v.z);
+        *reinterpret_cast<float2*>(d1) = make_float2(v.y, v.w);
+        *reinterpret_cast<float2*>(d0 + half) = make_float2(l.x, l.z);
+        *reinterpret_cast<float2*>(d1 + half) = make_float2(l.y, l.w);
+        // the padding planes of an image are spread over its threads
+        const long long per_image = (long long)C * H * WQ, at = i - n * per_image;
+        for (long long z = at; z < pad; z += per_image) X2[n * 2 * half + half - pad + z] = X2[n * 2 * half + 2 * half - pad + z] = 0.f;
     }
 }
 
@@ -719,7 +739,7 @@ struct ConvEnv {
 // Geometry the tensor-core forward / data-gradient kernel covers; fills the derived sizes.
 struct ConvPlan {
     int Cin, Cout, OCp, OCs, nsplit, NQ, CG, L, KS, shared_rows, nblocks, stages;
-    int c_wrap = 0;  // set by the caller before planning: input-channel wrap of the 3xTF32 form (0 = none)
+    int x3 = 0;      // set by the caller before planning: channels of a group of the 3xTF32 form (0: plain)
     int ks_max = 4;  // set by the caller before planning: most K steps a stage may carry
     int ew;      // epilogue warps of the kernel instantiation: 8 or 16
     int per_sm;  // CTAs the plan expects to share an SM (2 for narrow outputs with a small filter, else 1)
@@ -751,7 +771,7 @@ int plan_conv(ConvPlan& q, int smem_optin, int sm_count, const float* X, int N, 
     q.OCp = (q.Cout + 15) / 16 * 16;
     if (q.Cin < 1) return CB_EUNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(X) & 15u) != 0) return CB_EUNSUPPORTED;
-    q.CG = (q.Cin + 31) / 32;
+    q.CG = (q.Cin - q.x3 + 31) / 32;  // the 3xTF32 form packs two groups for three
     q.w_total_bytes = (size_t)FH * q.CG * FW * q.OCp * kRowBytes;
     q.shared_rows = (q.L == 1 && IH % 4 == 0) ? 1 : 0;
     q.nblocks = q.shared_rows ? FH + 3 : FH * 4;
@@ -814,14 +834,14 @@ int plan_conv(ConvPlan& q, int smem_optin, int sm_count, const float* X, int N, 
 
 // How the caller's filter becomes the packed filter of the convolution the kernel runs.
 struct PackSpec {
-    int mode, OC, IC, FHs, FWs, out_first, out_count;
+    int mode, OC, IC, FHs, FWs, out_first, out_count;  // mode and geometry of pack_source
 };
 
 PackJob make_job(const PackSpec& ps, const ConvPlan& q, const float* W, float* dst, int FH, int FW) {
     PackJob j{};
     j.W = W; j.Wp = dst;
     j.OC = ps.OC; j.IC = ps.IC; j.FHs = ps.FHs; j.FWs = ps.FWs; j.FHc = FH; j.FWc = FW;
-    j.OCp = q.OCp; j.CG = q.CG; j.mode = ps.mode; j.out_first = ps.out_first; j.out_count = ps.out_count;
+    j.OCp = q.OCp; j.CG = q.CG; j.x3 = q.x3; j.mode = ps.mode; j.out_first = ps.out_first; j.out_count = ps.out_count;
     j.total = (long long)q.w_total_bytes / 4;
     return j;
 }
@@ -844,7 +864,8 @@ int launch_conv(cb_ctx* err_ctx, const ConvEnv& env, const ConvPlan& q, const fl
     p.N = N; p.Cin = q.Cin; p.H = IH; p.W = IW; p.Cout = q.Cout;
     p.FH = FH; p.FW = FW; p.pH = pH; p.pW = pW;
     p.OCs = q.OCs; p.nsplit = q.nsplit; p.NQ = q.NQ; p.CG = q.CG; p.KS = q.KS;
-    p.c_wrap = q.c_wrap;
+    p.c_wrap = 2 * q.x3;
+    p.f_wrap = q.x3 / kCB;
     p.NCB = (q.Cin + q.KS * kCB - 1) / (q.KS * kCB);
     p.L = q.L; p.LPI = IH / q.L;
     p.shared_rows = q.shared_rows; p.nblocks = q.nblocks;
@@ -998,7 +1019,7 @@ struct FilterCache {
 
 static bool same_job(const PackJob& a, const PackJob& b) {
     return a.W == b.W && a.OC == b.OC && a.IC == b.IC && a.FHs == b.FHs && a.FWs == b.FWs && a.FHc == b.FHc &&
-           a.FWc == b.FWc && a.OCp == b.OCp && a.CG == b.CG && a.mode == b.mode && a.out_first == b.out_first &&
+           a.FWc == b.FWc && a.OCp == b.OCp && a.CG == b.CG && a.mode == b.mode && a.x3 == b.x3 && a.out_first == b.out_first &&
            a.out_count == b.out_count;
 }
 
@@ -1056,6 +1077,14 @@ static int packed_filter(cb_ctx* ctx, const ConvEnv& env, const ConvPlan& q, con
     return CB_OK;
 }
 
+bool filter_cache_fresh(const cb_ctx* ctx) {
+    const FilterCache* fc = static_cast<const FilterCache*>(ctx->filter_cache);
+    if (!ctx->filter_cache_on || !fc) return false;
+    for (const FilterCacheEntry& e : fc->entries)
+        if (e.version != ctx->filter_version) return false;
+    return true;
+}
+
 // Re-packs every cached filter in one launch and marks them current.
 int filter_cache_repack_all(cb_ctx* ctx) {
     ctx->filter_version += 1;
@@ -1106,68 +1135,85 @@ static int conv_on_packed(cb_ctx* ctx, const ConvEnv& env, const ConvPlan& q, co
     return CB_OK;
 }
 
-// 3xTF32 forward / data gradient in ONE pass of the tensor-core kernel (stride 1): x = x_hi + x_lo, w = w_hi + w_lo and
-// y = x_hi w_hi + x_lo w_hi + x_hi w_lo are a single convolution over three groups of input channels, [x ; x_lo ; x]
-// against [w ; w ; w_lo], because the tensor core itself takes the hi part of what it reads. One small pass writes
-// X2 = [x ; x_lo] (dense scratch), the packed filter carries the three weight groups (cached like any other), and the
-// kernel's producer reads channels [0, cin) a second time for the third group. Everything accumulates in one TMEM
-// accumulator and leaves through the ordinary epilogue. CB_EUNSUPPORTED (nothing queued) when the channel count is not
-// a multiple of 8 or the tripled filter does not fit; the caller then composes three passes.
-int umma_conv_fwd_x3(cb_ctx* ctx, const float* W, const float* X, float* Y, const ConvEpilogue& ep, int N, int IC, int IH,
-                     int IW, int OC, int FH, int FW, int pH, int pW, bool dgrad_of, long long in_batch, long long out_batch) {
-    if (!((FH == 1 && pH == 0) || (FH == 3 && pH == 1))) return CB_EUNSUPPORTED;
-    if (!((FW == 1 && pW == 0) || (FW == 3 && pW == 1))) return CB_EUNSUPPORTED;
-    const int cin = dgrad_of ? OC : IC, cout = dgrad_of ? IC : OC;
-    if (cin % 8 || ((long long)IH * IW) % 4) return CB_EUNSUPPORTED;
-    if ((reinterpret_cast<uintptr_t>(X) & 15u) || (in_batch & 3)) return CB_EUNSUPPORTED;
-    ConvEnv env{ctx->stream, ctx->sm_count, ctx->max_smem_optin, ctx->d_status};
-    ConvPlan q{};
-    q.c_wrap = 2 * cin;
-    q.ks_max = (cin % 32 == 0) ? 4 : ((cin % 16 == 0) ? 2 : 1);  // a stage's channels stay inside one group
-    int rc = plan_conv(q, ctx->max_smem_optin, ctx->sm_count, nullptr /* the scratch copy is aligned */, N, 3 * cin, cout, IH, IW,
-                       FH, FW, pH, pW);
+// Plan of one convolution of the path below: cin input channels of IH x IW, cout outputs. With x3 the contraction runs over
+// three groups of channels (see umma_conv_fwd).
+static int plan_pass(const cb_ctx* ctx, ConvPlan& q, bool x3, const float* X, int N, int cin, int cout, int IH, int IW, int FH, int FW,
+                     int pH, int pW) {
+    q = ConvPlan{};
+    if (!x3) return plan_conv(q, ctx->max_smem_optin, ctx->sm_count, X, N, cin, cout, IH, IW, FH, FW, pH, pW);
+    if (((long long)IH * IW) % 4 || (reinterpret_cast<uintptr_t>(X) & 15u)) return CB_EUNSUPPORTED;
+    q.x3 = (cin + 7) / 8 * 8;
+    q.ks_max = q.x3 % 32 == 0 ? 4 : (q.x3 % 16 == 0 ? 2 : 1);  // a stage's channels stay inside one group
+    const int rc = plan_conv(q, ctx->max_smem_optin, ctx->sm_count, nullptr /* the scratch copy is aligned */, N, 3 * q.x3, cout, IH,
+                             IW, FH, FW, pH, pW);
     if (rc != CB_OK) return rc;
-    // A tripled 64-channel filter only fits when the output channels are split four ways; every CTA then re-reads the
-    // input tile for 16 output channels, which pays on small maps (64->64 @8x8: 21 us against 36 composed) and not on
-    // large ones (64->64 @32x32: 207 us against 141).
+    // A filter that only fits when the output channels are split four ways makes every CTA re-read the input for a quarter
+    // of them, which pays on small maps and not on large ones (64 -> 64: 21 us against 36 composed at 8 x 8).
     if (q.nsplit > 2 && ((long long)N * (IH / q.L) + 3) / 4 > ctx->sm_count) return CB_EUNSUPPORTED;
-    const long long per = (long long)cin * IH * IW;
-    rc = ensure_workspace3(ctx, (size_t)N * 2 * per * sizeof(float));
-    if (rc != CB_OK) return rc;
-    float* X2 = static_cast<float*>(ctx->workspace3);
-    const long long items = (long long)N * (per / 4);
-    cudaError_t e = launch_dep(ctx, tf32_split2_kernel, dim3((unsigned)relayout_grid(ctx, items)), dim3(256), 0, X, X2, per / 4,
-                               in_batch ? in_batch : per, items);
+    return CB_OK;
+}
+
+// One planned convolution on `X` (N images of `cin` planes, in_batch floats apart or dense). With q.x3 the input is first
+// written as [x ; x_lo] to scratch.
+static int run_pass(cb_ctx* ctx, const ConvEnv& env, const ConvPlan& q, const PackSpec& ps, const float* W, const float* X, int cin,
+                    float* Y, const ConvEpilogue& ep, int N, int IH, int IW, int FH, int FW, int pH, int pW, long long in_batch,
+                    long long out_batch) {
+    if (q.x3) {
+        const long long plane = (long long)IH * IW, per = cin * plane, perp = q.x3 * plane;
+        if (in_batch & 3) return CB_EUNSUPPORTED;
+        int rc = ensure_workspace3(ctx, (size_t)N * 2 * perp * sizeof(float));
+        if (rc != CB_OK) return rc;
+        float* X2 = static_cast<float*>(ctx->workspace3);
+        const long long items = (long long)N * (perp / 4);
+        cudaError_t e = launch_dep(ctx, tf32_split2_kernel, dim3((unsigned)relayout_grid(ctx, items)), dim3(256), 0, X, X2, per / 4,
+                                   perp / 4, in_batch ? in_batch : per, items);
+        if (e == cudaSuccess) e = cudaGetLastError();
+        if (e != cudaSuccess) return check_cuda(ctx, e, "tf32_split2_kernel launch");
+        ctx->launches += 1;
+        X = X2;
+        in_batch = 2 * perp;
+    }
+    return conv_on_packed(ctx, env, q, ps, W, X, Y, ep, N, IH, IW, FH, FW, pH, pW, in_batch, out_batch);
+}
+
+int launch_space_to_depth2_split(cb_ctx* ctx, const float* X, float* X2, int N, int C, int Cp, int H, int W) {
+    const long long items = (long long)N * C * H * (W / 4);
+    cudaError_t e = launch_dep(ctx, space_to_depth2_split_kernel, dim3((unsigned)relayout_grid(ctx, items)), dim3(256), 0, X, X2, C, Cp, H,
+                               W, items);
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) return check_cuda(ctx, e, "tf32_split2_kernel launch");
+    if (e != cudaSuccess) return check_cuda(ctx, e, "space_to_depth2_split_kernel launch");
     ctx->launches += 1;
-    const PackSpec ps{dgrad_of ? PACK_DGRAD_X3 : PACK_FWD_X3, OC, IC, FH, FW, 0, 0};
-    rc = conv_on_packed(ctx, env, q, ps, W, X2, Y, ep, N, IH, IW, FH, FW, pH, pW, 2 * per, out_batch);
-    if (rc != CB_OK) return rc;
-    ctx->last_kernel = "umma_3xtf32";
     return CB_OK;
 }
 
 // Forward (dgrad_of = false: Y = conv(W, X), full epilogue) or data gradient (dgrad_of = true: X is dY, Y is dX; of the
 // epilogue only `accumulate` applies). Returns CB_EUNSUPPORTED, before any work is queued, for geometries outside the
 // tensor-core kernel.
+//
+// x3: 3xTF32 in ONE pass of the kernel. With x = x_hi + x_lo and w = w_hi + w_lo, y = x_hi w_hi + x_lo w_hi + x_hi w_lo is a
+// single convolution over three groups of input channels, [x ; x_lo ; x] against [w ; w ; w_lo], because the tensor core itself
+// takes the hi part of what it reads. A small kernel writes [x ; x_lo] (dense scratch; for stride 2 in the phase-split layout),
+// the packed filter holds [w ; w_lo] (cached like any other), the kernel reads x a second time and w twice. Everything
+// accumulates in one TMEM accumulator and leaves through the ordinary epilogue. Against three passes into temporaries, their lo
+// parts and a sum: 32 -> 64 stride 2 at 32 x 32, batch 128, three passes of the layer 229 us before.
 int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const ConvEpilogue& ep, int N, int IC, int IH,
                   int IW, int OC, int FH, int FW, int sH, int sW, int pH, int pW, bool dgrad_of, long long in_batch,
-                  long long out_batch) {
+                  long long out_batch, bool x3) {
     ConvEnv env{ctx->stream, ctx->sm_count, ctx->max_smem_optin, ctx->d_status};
     ConvPlan q{};
     int rc;
+    const char* name = x3 ? "umma_3xtf32" : "umma_tf32";
     if (sH == 1 && sW == 1) {
         // ---- stride 1: 1x1 (pad 0) or 3x3 (pad 1) per axis
         if (!((FH == 1 && pH == 0) || (FH == 3 && pH == 1))) return CB_EUNSUPPORTED;
         if (!((FW == 1 && pW == 0) || (FW == 3 && pW == 1))) return CB_EUNSUPPORTED;
-        rc = plan_conv(q, ctx->max_smem_optin, ctx->sm_count, X, N, dgrad_of ? OC : IC, dgrad_of ? IC : OC, IH, IW, FH, FW, pH, pW);
+        const int cin = dgrad_of ? OC : IC, cout = dgrad_of ? IC : OC;
+        rc = plan_pass(ctx, q, x3, X, N, cin, cout, IH, IW, FH, FW, pH, pW);
         if (rc != CB_OK) return rc;
         const PackSpec ps{dgrad_of ? PACK_DGRAD : PACK_FWD, OC, IC, FH, FW, 0, 0};
-        rc = conv_on_packed(ctx, env, q, ps, W, X, Y, ep, N, IH, IW, FH, FW, pH, pW, in_batch, out_batch);
-        if (rc != CB_OK) return rc;
-        ctx->last_kernel = "umma_tf32";
-        return CB_OK;
+        rc = run_pass(ctx, env, q, ps, W, X, cin, Y, ep, N, IH, IW, FH, FW, pH, pW, in_batch, out_batch);
+        if (rc == CB_OK) ctx->last_kernel = name;
+        return rc;
     }
     // ---- stride 2 (square): 3x3 pad 1 through the 4 input phases, 1x1 pad 0 through phase (0,0); dense tensors only
     if (sH != 2 || sW != 2 || FH != FW || pH != pW || (IH & 1) || (IW & 1)) return CB_EUNSUPPORTED;
@@ -1178,8 +1224,9 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
     const ConvEpilogue plain{};
     if (FH == 1) {
         // Y = W * X[:, :, ::2, ::2]  /  dX[:, :, ::2, ::2] = W^T dY, zero elsewhere
-        rc = plan_conv(q, ctx->max_smem_optin, ctx->sm_count, dgrad_of ? X : nullptr /* the sub-sampled copy is aligned */, N,
-                       dgrad_of ? OC : IC, dgrad_of ? IC : OC, H2, W2, 1, 1, 0, 0);
+        const int cin = dgrad_of ? OC : IC;
+        rc = plan_pass(ctx, q, x3, dgrad_of ? X : nullptr /* the sub-sampled copy is aligned */, N, cin, dgrad_of ? IC : OC, H2, W2, 1, 1,
+                       0, 0);
         if (rc != CB_OK) return rc;
         const size_t sub_bytes = (size_t)N * IC * plane2 * sizeof(float);
         rc = ensure_workspace2(ctx, sub_bytes);
@@ -1188,9 +1235,9 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
         const PackSpec ps{dgrad_of ? PACK_DGRAD : PACK_FWD, OC, IC, 1, 1, 0, 0};
         if (!dgrad_of) {
             rc = launch_subsample2(ctx, X, sub, (long long)N * IC, IH, IW);
-            if (rc == CB_OK) rc = conv_on_packed(ctx, env, q, ps, W, sub, Y, ep, N, H2, W2, 1, 1, 0, 0, 0, 0);
+            if (rc == CB_OK) rc = run_pass(ctx, env, q, ps, W, sub, cin, Y, ep, N, H2, W2, 1, 1, 0, 0, 0, 0);
         } else {
-            rc = conv_on_packed(ctx, env, q, ps, W, X /* = dY */, sub, plain, N, H2, W2, 1, 1, 0, 0, 0, 0);
+            rc = run_pass(ctx, env, q, ps, W, X /* = dY */, cin, sub, plain, N, H2, W2, 1, 1, 0, 0, 0, 0);
             const long long n_full = (long long)N * IC * IH * IW;
             if (rc == CB_OK) {
                 if (vec_ok(sub, Y, IW))
@@ -1205,25 +1252,33 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
         if (rc != CB_OK) return rc;
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return check_cuda(ctx, e, "stride-2 1x1 convolution");
-        ctx->last_kernel = "umma_tf32";
+        ctx->last_kernel = name;
         return CB_OK;
     }
     const int C4 = 4 * IC;
     const size_t s2d_bytes = (size_t)N * C4 * plane2 * sizeof(float);
     if (!dgrad_of) {
         // Xs[n][phase*IC + c] = X[n][c][phase rows / cols]; Y = 2x2 convolution (taps at -1, 0) over the 4*IC planes
-        rc = ensure_workspace2(ctx, s2d_bytes);
-        if (rc != CB_OK) return rc;
-        float* Xs = static_cast<float*>(ctx->workspace2);
-        rc = plan_conv(q, ctx->max_smem_optin, ctx->sm_count, Xs, N, C4, OC, H2, W2, 2, 2, 1, 1);
-        if (rc != CB_OK) return rc;
-        rc = launch_space_to_depth2(ctx, X, Xs, N, IC, IH, IW);
-        if (rc != CB_OK) return rc;
         const PackSpec ps{PACK_S2_FWD, OC, IC, 3, 3, 0, 0};
-        rc = conv_on_packed(ctx, env, q, ps, W, Xs, Y, ep, N, H2, W2, 2, 2, 1, 1, 0, 0);
+        rc = plan_pass(ctx, q, x3, nullptr /* the re-laid-out copy is aligned */, N, C4, OC, H2, W2, 2, 2, 1, 1);
         if (rc != CB_OK) return rc;
-        ctx->last_kernel = "umma_tf32";
-        return CB_OK;
+        if (x3) {
+            if (!vec_ok(X, nullptr, IW)) return CB_EUNSUPPORTED;
+            const long long perp = 2LL * q.x3 * plane2;
+            rc = ensure_workspace3(ctx, (size_t)N * perp * sizeof(float));
+            if (rc != CB_OK) return rc;
+            float* X2 = static_cast<float*>(ctx->workspace3);
+            rc = launch_space_to_depth2_split(ctx, X, X2, N, IC, q.x3, IH, IW);
+            if (rc == CB_OK) rc = conv_on_packed(ctx, env, q, ps, W, X2, Y, ep, N, H2, W2, 2, 2, 1, 1, perp, 0);
+        } else {
+            rc = ensure_workspace2(ctx, s2d_bytes);
+            if (rc != CB_OK) return rc;
+            float* Xs = static_cast<float*>(ctx->workspace2);
+            rc = launch_space_to_depth2(ctx, X, Xs, N, IC, IH, IW);
+            if (rc == CB_OK) rc = conv_on_packed(ctx, env, q, ps, W, Xs, Y, ep, N, H2, W2, 2, 2, 1, 1, 0, 0);
+        }
+        if (rc == CB_OK) ctx->last_kernel = name;
+        return rc;
     }
     // data gradient: dXs (4*IC phase planes) = adjoint 2x2 convolution (taps at 0, +1) over dY, in channel groups small
     // enough for the accumulator (FW * roundup16(channels) <= 256), then interleaved back into dX
@@ -1234,12 +1289,12 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
     rc = ensure_workspace2(ctx, s2d_bytes);
     if (rc != CB_OK) return rc;
     float* dXs = static_cast<float*>(ctx->workspace2);
-    rc = plan_conv(q, ctx->max_smem_optin, ctx->sm_count, X /* = dY */, N, OC, per_group, H2, W2, 2, 2, 0, 0);
+    rc = plan_pass(ctx, q, x3, X /* = dY */, N, OC, per_group, H2, W2, 2, 2, 0, 0);
     if (rc != CB_OK) return rc;
     for (int g = 0; g < groups; ++g) {
         const PackSpec ps{PACK_S2_DGRAD, OC, IC, 3, 3, g * per_group, per_group};
-        rc = conv_on_packed(ctx, env, q, ps, W, X /* = dY */, dXs + (size_t)g * N * per_group * plane2, plain, N, H2, W2, 2, 2,
-                            0, 0, 0, 0);
+        rc = run_pass(ctx, env, q, ps, W, X /* = dY */, OC, dXs + (size_t)g * N * per_group * plane2, plain, N, H2, W2, 2, 2, 0, 0, 0,
+                      0);
         if (rc != CB_OK) return rc;
     }
     const long long n_full = (long long)N * IC * IH * IW;
@@ -1251,7 +1306,7 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return check_cuda(ctx, e, "depth_to_space2_kernel launch");
     ctx->launches += 1;
-    ctx->last_kernel = "umma_tf32";
+    ctx->last_kernel = name;
     return CB_OK;
 }
 

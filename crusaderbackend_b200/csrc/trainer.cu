@@ -100,6 +100,26 @@ struct ParamEntry {
     int d0, d1, d2, d3;
 };
 
+// Everything a recorded pass depends on besides the model's own buffers.
+struct PassKey {
+    const float *images, *labels;
+    int backward, math, deterministic, bn_grad_swap, bn_groups, pdl;
+    long long scratch_epoch;
+    bool operator==(const PassKey& o) const {
+        return images == o.images && labels == o.labels && backward == o.backward && math == o.math && deterministic == o.deterministic &&
+               bn_grad_swap == o.bn_grad_swap && bn_groups == o.bn_groups && pdl == o.pdl && scratch_epoch == o.scratch_epoch;
+    }
+};
+struct RecordedPass {
+    PassKey key;
+    int seen = 0;                  // eager calls with this key so far
+    bool unusable = false;         // recording it failed: stays eager
+    cudaGraphExec_t exec = nullptr;
+    long long launches = 0;        // kernels of a replay on the context's stream ...
+    std::vector<long long> side_launches;  // ... and on each weight-gradient stream
+    unsigned long long used = 0;
+};
+
 }  // namespace
 
 struct cbt_model {
@@ -139,6 +159,10 @@ struct cbt_model {
     std::vector<int*> side_own_status;
     std::vector<char> side_used;
     int side_next = 0;
+    // recorded passes (run_recorded): the eager call sequence of a forward or backward pass as an executable graph
+    std::vector<RecordedPass> recorded;
+    cudaStream_t record_stream = nullptr;
+    unsigned long long record_clock = 0;
     // .crseq image of the model (ResNets): top-level operand ids, the words of the info section (uuid words flagged: a
     // file's own block numbering is accepted on load), and the parameter entries in the order the file stores them
     std::vector<uint32_t> crseq_ids, crseq_info;
@@ -149,6 +173,8 @@ struct cbt_model {
 extern "C" int cbt_set_wgrad_streams(cbt_model* m, int n);
 
 namespace {
+
+void drop_recorded(cbt_model* m);
 
 int new_tensor(cbt_model* m, int n, int c, int h, int w) {
     TensorBuf b;
@@ -532,6 +558,7 @@ int cbt_densenet_create(cbt_model** out, cb_ctx* ctx, int batch, int growth, int
 int cbt_set_wgrad_streams(cbt_model* m, int n) {
     if (!m || n < 0 || n > 4) return CB_EINVAL;
     cudaStreamSynchronize(m->ctx->stream);
+    drop_recorded(m);
     release_side_streams(m);
     for (int s = 0; s < n; ++s) {
         cudaStream_t st = nullptr;
@@ -571,6 +598,8 @@ long long cbt_side_launches(const cbt_model* m) {
 int cbt_destroy(cbt_model* m) {
     if (!m) return CB_EINVAL;
     cudaStreamSynchronize(m->ctx->stream);
+    drop_recorded(m);
+    if (m->record_stream) cudaStreamDestroy(m->record_stream);
     release_side_streams(m);
     for (void* p : m->owned) cudaFree(p);
     if (m->mom_table) cudaFree(m->mom_table);
@@ -606,6 +635,7 @@ int cbt_bind(cbt_model* m, float* params, float* grads, float* momentum) {
         m->err = "flat parameter buffers must be 16-byte aligned";
         return CB_EINVAL;
     }
+    drop_recorded(m);  // they hold the addresses of the buffers bound before
     m->P = params; m->G = grads; m->M = momentum;
     const int n = (int)m->params.size();
     std::vector<float*> w(n), g(n), mo(n);
@@ -738,14 +768,118 @@ int cbt_load_crseq(cbt_model* m, const char* path, unsigned* epoch) {
     return cbt_params_changed(m);
 }
 
+}  // extern "C"
+
+namespace {
+
+void drop_recorded(cbt_model* m) {
+    if (m->recorded.empty()) return;
+    cudaStreamSynchronize(m->ctx->stream);
+    for (RecordedPass& r : m->recorded)
+        if (r.exec) cudaGraphExecDestroy(r.exec);
+    m->recorded.clear();
+}
+
+// Runs `pass` (the calls of a forward or backward pass on the context's stream). A program that steps a model without a
+// graph of its own issues 30 to 300 launches a step from the host, at about 3 us each, which bounds small models and small
+// batches. So a pass that comes back with the same buffers and settings is recorded on its third call, and later calls
+// launch the recording. Eager as before: the first calls, streams that are being captured, sync mode, data-parallel models
+// (their collectives are ordered call by call), calls that find a filter's packed copy stale, and passes whose recording
+// fails. A recording is keyed by everything it has baked in, scratch blocks included; at most kMostRecorded are kept.
+template <class F>
+int run_recorded(cbt_model* m, bool backward, F pass) {
+    constexpr size_t kMostRecorded = 8;
+    constexpr int kSeenBeforeRecording = 2;
+    cb_ctx* ctx = m->ctx;
+    if (m->comm || ctx->sync || !cb::filter_cache_fresh(ctx)) return pass();
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return pass();
+    }
+    if (cap != cudaStreamCaptureStatusNone) return pass();
+    PassKey key{m->t[m->input].a, m->labels, backward ? 1 : 0, ctx->math, ctx->deterministic, m->bn_grad_swap, m->bn_groups, ctx->pdl,
+                ctx->scratch_epoch};
+    for (const cb_ctx* c : m->side) key.scratch_epoch += c->scratch_epoch;  // only ever grow: the sum changes with any of them
+    RecordedPass* r = nullptr;
+    for (RecordedPass& e : m->recorded)
+        if (e.key == key) { r = &e; break; }
+    if (!r) {
+        if (m->recorded.size() == kMostRecorded) {
+            size_t oldest = 0;
+            for (size_t i = 1; i < m->recorded.size(); ++i)
+                if (m->recorded[i].used < m->recorded[oldest].used) oldest = i;
+            if (m->recorded[oldest].exec) {
+                cudaStreamSynchronize(ctx->stream);
+                cudaGraphExecDestroy(m->recorded[oldest].exec);
+            }
+            m->recorded.erase(m->recorded.begin() + (long)oldest);
+        }
+        m->recorded.push_back(RecordedPass{});
+        r = &m->recorded.back();
+        r->key = key;
+    }
+    r->used = ++m->record_clock;
+    if (!r->exec) {
+        if (r->unusable || r->seen < kSeenBeforeRecording) {
+            ++r->seen;
+            return pass();
+        }
+        r->unusable = true;  // until the recording is complete
+        if (!m->record_stream && cudaStreamCreateWithFlags(&m->record_stream, cudaStreamNonBlocking) != cudaSuccess) return pass();
+        const long long l0 = ctx->launches;
+        std::vector<long long> s0;
+        for (const cb_ctx* c : m->side) s0.push_back(c->launches);
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        cudaStream_t callers = ctx->stream;
+        if (cudaStreamBeginCapture(m->record_stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+            cudaGetLastError();
+            return pass();
+        }
+        ctx->stream = m->record_stream;
+        const int rc = pass();
+        ctx->stream = callers;
+        cudaError_t e = cudaStreamEndCapture(m->record_stream, &graph);
+        if (rc == CB_OK && e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+        if (graph) cudaGraphDestroy(graph);
+        r->launches = ctx->launches - l0;
+        r->side_launches.clear();
+        for (size_t i = 0; i < m->side.size(); ++i) r->side_launches.push_back(m->side[i]->launches - s0[i]);
+        // nothing of the recording has run yet
+        ctx->launches = l0;
+        for (size_t i = 0; i < m->side.size(); ++i) m->side[i]->launches = s0[i];
+        if (rc != CB_OK || e != cudaSuccess || !exec) {
+            cudaGetLastError();
+            m->err.clear();
+            return pass();
+        }
+        r->exec = exec;
+        r->unusable = false;
+    }
+    cudaError_t e = cudaGraphLaunch(r->exec, ctx->stream);
+    if (e != cudaSuccess) { m->err = cudaGetErrorString(e); return CB_ECUDA; }
+    ctx->launches += r->launches;
+    for (size_t i = 0; i < m->side.size(); ++i) m->side[i]->launches += r->side_launches[i];
+    return CB_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
 // Forward pass on `images` (batch x 3 x H x W, device) with one-hot `labels` (batch x classes, device). The images are
 // read in place (no copy): they must stay unchanged until cbt_backward has run. Leaves the softmax in the last tensor
 // and the summed loss in the model's device loss word (after cbt_backward for models with the fused head).
+static int forward_ops(cbt_model* m, const float* labels);
 int cbt_forward(cbt_model* m, const float* images, const float* labels) {
     if (!m || !m->P || !images || !labels) return CB_EINVAL;
-    cb_ctx* ctx = m->ctx;
     m->t[m->input].a = const_cast<float*>(images);
     m->labels = const_cast<float*>(labels);
+    return run_recorded(m, false, [&] { return forward_ops(m, labels); });
+}
+static int forward_ops(cbt_model* m, const float* labels) {
+    cb_ctx* ctx = m->ctx;
     cudaError_t e;
     for (const Op& o : m->ops) {
         const TensorBuf& x = m->t[o.in0];
@@ -863,8 +997,12 @@ static int dp_release_buckets(cbt_model* m, int op_index) {
 
 // Backward pass: fills the flat gradient buffer (accumulating into it, as every seblas parameter-gradient kernel
 // does; cbt_update zeroes it again).
+static int backward_ops(cbt_model* m);
 int cbt_backward(cbt_model* m) {
     if (!m || !m->G) return CB_EINVAL;
+    return run_recorded(m, true, [&] { return backward_ops(m); });
+}
+static int backward_ops(cbt_model* m) {
     cb_ctx* ctx = m->ctx;
     m->side_next = 0;
     std::fill(m->side_used.begin(), m->side_used.end(), 0);

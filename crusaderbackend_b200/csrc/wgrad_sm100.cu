@@ -696,6 +696,7 @@ int umma_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, int
         return rc;
     };
     if (N < 1 || ((long long)IH * IW & 3)) return CB_EUNSUPPORTED;
+    if (((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(dY)) & 15u) || (x3 && ((x_batch | dy_batch) & 3))) return CB_EUNSUPPORTED;
     if (sH == 1 && sW == 1) {
         if (!((FH == 1 && pH == 0) || (FH == 3 && pH == 1))) return CB_EUNSUPPORTED;
         if (!((FW == 1 && pW == 0) || (FW == 3 && pW == 1))) return CB_EUNSUPPORTED;
@@ -757,18 +758,28 @@ int umma_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, int
         return wgrad_core(ctx, dY, sub, dW, N, IC, H2, W2, OC, 1, 1, 0, 0, accumulate, 0, IC, 0, 0, 0, 0, 0, lo);
     }
     if (4 * IC > 256) return CB_EUNSUPPORTED;
+    if (x3) {
+        // phase planes and their lo parts in one pass
+        const long long half = 4LL * IC * plane2, dy_per = (long long)OC * plane2;
+        int rc = ensure_workspace2(ctx, (size_t)N * 2 * half * sizeof(float));
+        if (rc == CB_OK) rc = ensure_workspace3(ctx, (size_t)N * dy_per * sizeof(float));
+        if (rc != CB_OK) return rc;
+        float* X2 = static_cast<float*>(ctx->workspace2);
+        float* yl = static_cast<float*>(ctx->workspace3);
+        rc = launch_space_to_depth2_split(ctx, X, X2, N, IC, 4 * IC, IH, IW);
+        if (rc == CB_OK) rc = launch_lo(ctx, dY, yl, N, dy_per, 0);
+        if (rc != CB_OK) return rc;
+        LoParts lo;
+        lo.x = X2 + half; lo.x_batch = 2 * half; lo.dy = yl; lo.dy_batch = dy_per;
+        return wgrad_core(ctx, dY, X2, dW, N, 4 * IC, H2, W2, OC, 2, 2, 1, 1, accumulate, 1, IC, 0, 2 * half, 0, 0, 0, lo);
+    }
     const long long n_el = (long long)N * 4 * IC * plane2;
     int rc = ensure_workspace2(ctx, (size_t)n_el * sizeof(float));
     if (rc != CB_OK) return rc;
     float* Xs = static_cast<float*>(ctx->workspace2);
     rc = launch_space_to_depth2(ctx, X, Xs, N, IC, IH, IW);
     if (rc != CB_OK) return rc;
-    LoParts lo;
-    if (x3) {
-        rc = make_lo(Xs, 4LL * IC * plane2, 0, dY, (long long)OC * plane2, 0, lo);
-        if (rc != CB_OK) return rc;
-    }
-    return wgrad_core(ctx, dY, Xs, dW, N, 4 * IC, H2, W2, OC, 2, 2, 1, 1, accumulate, 1, IC, 0, 0, 0, 0, 0, lo);
+    return wgrad_core(ctx, dY, Xs, dW, N, 4 * IC, H2, W2, OC, 2, 2, 1, 1, accumulate, 1, IC, 0, 0);
 }
 
 }  // namespace cb

@@ -240,3 +240,21 @@ def test_cuda_core_convolution_tiles_and_phases(torch_cuda, ctxs, geo):
     c = conv_case(("simt", geo), N, IC, H, W, OC, F, s, p, bias=True)
     kern = check_three_passes(torch_cuda, ctxs["fp32"], "fp32", c, dW0=orc.normal((OC, IC, F, F), "simt", geo, "dW0"))
     assert all(k == "simt_fp32" for k in kern), kern
+
+
+@pytest.mark.parametrize("geo", [(2, 3, 16, 16, 3, 1), (2, 20, 16, 24, 3, 1), (4, 6, 32, 40, 3, 2), (2, 5, 16, 16, 1, 2), (3, 64, 32, 64, 3, 1),
+                                 (2, 32, 64, 64, 3, 2), (1, 13, 16, 48, 3, 2)])
+def test_3xtf32_in_one_pass_pads_channels_and_covers_stride_2(torch_cuda, ctxs, geo):
+    """The one-pass 3xTF32 form: channel counts that are no multiple of a K step (padded planes of the scratch copy), filters
+    whose two packed groups need an output-channel split, the phase-split layout of stride 2; and the launches of a pass."""
+    N, IC, H, OC, F, s = geo
+    p = 1 if F == 3 else 0
+    ctx = ctxs["3xtf32"]
+    c = conv_case(("x3one", geo), N, IC, H, H, OC, F, s, p)
+    kern = check_three_passes(torch_cuda, ctx, "3xtf32", c)
+    assert all(k == "umma_3xtf32" for k in kern), kern
+    W, X = (torch_cuda.from_numpy(c[k]).cuda() for k in ("W", "X"))
+    Y = torch_cuda.empty(c["dY"].shape, device="cuda")
+    l0 = ctx.launches
+    ctx.conv(W, X, Y, s, s, p, p)
+    assert ctx.launches - l0 <= 4  # re-layout, split, filter, convolution

@@ -295,3 +295,40 @@ def test_densenet_bc_100_forward_backward(torch_cuda):
         tr.close()
         ctx.close()
     assert np.isfinite(losses["fp32"]) and abs(losses["fp32"] - losses["tf32"]) <= 0.01 * abs(losses["fp32"])
+
+
+@pytest.mark.parametrize("streams", [0, 2])
+def test_recorded_passes_match_eager_ones(streams):
+    """Forward and backward passes that come back with the same buffers are recorded on their third call: the same bits and
+    the same launch count as a context in sync mode, which never records, over alternating batches, a change of math mode,
+    a reallocation of the context's scratch and a change of the weight-gradient streams."""
+    import torch
+    from crusaderbackend_b200.api import Context
+    from crusaderbackend_b200.train import ResNetTrainer
+    torch.manual_seed(5)
+    batches = [(torch.randn(8, 3, 16, 16, device="cuda"), torch.eye(10, device="cuda")[torch.randint(0, 10, (8,))].contiguous()) for _ in range(2)]
+    wide = torch.randn(256, 64, 32, 32, device="cuda")
+    W = torch.randn(64, 64, 3, 3, device="cuda")
+    results = []
+    for sync in (True, False):
+        ctx = Context(0, math="tf32", sync=sync)
+        ctx.set_deterministic(True)
+        tr = ResNetTrainer(ctx, batch=8, blocks_per_stage=1, image_hw=16)
+        tr.set_wgrad_streams(streams)
+        tr.init_params("recorded")
+        losses, l0 = [], tr.launches
+        for i in range(14):
+            if i == 8:
+                ctx.set_math("3xtf32")
+                ctx.conv(W, wide, torch.empty_like(wide), 1, 1, 1, 1)   # grows the scratch the recordings hold
+                ctx.set_math("tf32")
+            if i == 11:
+                tr.set_wgrad_streams(streams)
+            tr.step(*batches[i % 2], lr=1e-3)
+            losses.append(tr.loss())
+        results.append((losses, tr.params.clone(), tr.momentum.clone(), tr.launches - l0))
+        tr.close()
+        ctx.close()
+    (la, pa, ma, na), (lb, pb, mb, nb) = results
+    assert la == lb and torch.equal(pa, pb) and torch.equal(ma, mb)
+    assert na == nb
