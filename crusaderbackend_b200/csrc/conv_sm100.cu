@@ -579,91 +579,90 @@ __global__ void upsample2_zero_kernel(const float* __restrict__ dXsub, float* __
     }
 }
 
-// Vector forms of the four re-layout kernels for 16-byte aligned tensors with W % 4 == 0: one thread moves four
-// consecutive pixels of an input row (a 16-byte access on the full-resolution side, two 8-byte accesses on the
-// half-resolution side), so every access is coalesced.
-__global__ void space_to_depth2_vec_kernel(const float* __restrict__ X, float* __restrict__ Xs, int C, int H, int W,
-                                           long long items) {
+// Vector forms of the four re-layout kernels for 16-byte aligned tensors with W % 4 == 0: one item is four consecutive pixels
+// of an input row (a 16-byte access on the full-resolution side, two 8-byte accesses on the half-resolution side), so every
+// access is coalesced. kRelayoutItems items a thread are loaded before the first is stored.
+struct PlaneIndex {      // item -> (plane n * C + c, row y, quad q)
+    FastDiv wq, h, c;
+};
+constexpr int kRelayoutItems = 4;
+__global__ void __launch_bounds__(256) space_to_depth2_vec_kernel(const float* __restrict__ X, float* __restrict__ Xs, const PlaneIndex ix,
+                                                                  int W2, long long plane2, uint32_t items) {
     griddep_wait();
     griddep_launch();
-    const int H2 = H / 2, W2 = W / 2, WQ = W / 4;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < items;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int q = (int)(i % WQ);
-        long long r = i / WQ;
-        const int y = (int)(r % H);
-        r /= H;
-        const int c = (int)(r % C);
-        const long long n = r / C;
-        const float4 v = *reinterpret_cast<const float4*>(X + ((n * C + c) * H + y) * W + 4 * q);
-        const int row = y & 1;
-        float* d0 = Xs + (((n * 4 + 2 * row) * C + c) * H2 + (y >> 1)) * W2 + 2 * q;  // phase (row, 0)
-        float* d1 = d0 + (long long)C * H2 * W2;                                       // phase (row, 1)
-        *reinterpret_cast<float2*>(d0) = make_float2(v.x, v.z);
-        *reinterpret_cast<float2*>(d1) = make_float2(v.y, v.w);
-    }
-}
-__global__ void depth_to_space2_vec_kernel(const float* __restrict__ dXs, float* __restrict__ dX, int N, int C, int H, int W,
-                                           int per_group, long long items, int accumulate) {
-    griddep_wait();
-    griddep_launch();
-    const int H2 = H / 2, W2 = W / 2, WQ = W / 4;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < items;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int q = (int)(i % WQ);
-        long long r = i / WQ;
-        const int y = (int)(r % H);
-        r /= H;
-        const int c = (int)(r % C);
-        const long long n = r / C;
-        float2 ph[2];
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < items; i0 += kRelayoutItems * stride) {
+        float4 v[kRelayoutItems];
 #pragma unroll
-        for (int col = 0; col < 2; ++col) {
-            const int og = ((y & 1) * 2 + col) * C + c;
-            const int g = og / per_group, o = og - g * per_group;
-            ph[col] = *reinterpret_cast<const float2*>(dXs + ((((long long)g * N + n) * per_group + o) * H2 + (y >> 1)) * W2 + 2 * q);
+        for (int u = 0; u < kRelayoutItems; ++u)
+            if (i0 + u * stride < items) v[u] = reinterpret_cast<const float4*>(X)[i0 + u * stride];
+#pragma unroll
+        for (int u = 0; u < kRelayoutItems; ++u) {
+            if (i0 + u * stride >= items) break;
+            uint32_t q, y, c;
+            const uint32_t n = ix.c.split(ix.h.split(ix.wq.split(i0 + u * stride, q), y), c);
+            float* d0 = Xs + ((long long)(n * 4 + 2 * (y & 1)) * ix.c.d + c) * plane2 + (y >> 1) * W2 + 2 * q;  // phase (row, 0)
+            *reinterpret_cast<float2*>(d0) = make_float2(v[u].x, v[u].z);
+            *reinterpret_cast<float2*>(d0 + ix.c.d * plane2) = make_float2(v[u].y, v[u].w);                     // phase (row, 1)
         }
-        float4* dst = reinterpret_cast<float4*>(dX + ((n * C + c) * H + y) * W + 4 * q);
-        float4 v = make_float4(ph[0].x, ph[1].x, ph[0].y, ph[1].y);
-        if (accumulate) {
-            const float4 old = *dst;
-            v = make_float4(old.x + v.x, old.y + v.y, old.z + v.z, old.w + v.w);
-        }
-        *dst = v;
     }
 }
-__global__ void subsample2_vec_kernel(const float* __restrict__ X, float* __restrict__ Xsub, long long NC, int H, int W,
-                                      long long items) {
+__global__ void __launch_bounds__(256) depth_to_space2_vec_kernel(const float* __restrict__ dXs, float* __restrict__ dX, const PlaneIndex ix,
+                                                                  int N, int W2, long long plane2, const FastDiv group, uint32_t items,
+                                                                  int accumulate) {
     griddep_wait();
     griddep_launch();
-    const int H2 = H / 2, W2 = W / 2, WQ = W / 4;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < items;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int q = (int)(i % WQ);
-        const long long r = i / WQ;
-        const int ii = (int)(r % H2);
-        const long long nc = r / H2;
-        const float4 v = *reinterpret_cast<const float4*>(X + (nc * H + 2 * ii) * W + 4 * q);
-        *reinterpret_cast<float2*>(Xsub + (nc * H2 + ii) * W2 + 2 * q) = make_float2(v.x, v.z);
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < items; i0 += kRelayoutItems * stride) {
+        float4 v[kRelayoutItems];
+#pragma unroll
+        for (int u = 0; u < kRelayoutItems; ++u) {
+            if (i0 + u * stride >= items) break;
+            uint32_t q, y, c;
+            const uint32_t n = ix.c.split(ix.h.split(ix.wq.split(i0 + u * stride, q), y), c);
+            float2 ph[2];
+#pragma unroll
+            for (uint32_t col = 0; col < 2; ++col) {
+                uint32_t o;
+                const uint32_t g = group.split(((y & 1) * 2 + col) * ix.c.d + c, o);
+                ph[col] = *reinterpret_cast<const float2*>(dXs + (((long long)g * N + n) * group.d + o) * plane2 + (y >> 1) * W2 + 2 * q);
+            }
+            v[u] = make_float4(ph[0].x, ph[1].x, ph[0].y, ph[1].y);
+            if (accumulate) {
+                const float4 old = reinterpret_cast<const float4*>(dX)[i0 + u * stride];
+                v[u] = make_float4(old.x + v[u].x, old.y + v[u].y, old.z + v[u].z, old.w + v[u].w);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kRelayoutItems; ++u)
+            if (i0 + u * stride < items) reinterpret_cast<float4*>(dX)[i0 + u * stride] = v[u];
     }
 }
-__global__ void upsample2_zero_vec_kernel(const float* __restrict__ dXsub, float* __restrict__ dX, int H, int W,
-                                          long long items, int accumulate) {
+// item: four pixels of an even row
+__global__ void __launch_bounds__(256) subsample2_vec_kernel(const float* __restrict__ X, float* __restrict__ Xsub, const FastDiv wq, int W,
+                                                             uint32_t items) {
     griddep_wait();
     griddep_launch();
-    const int H2 = H / 2, W2 = W / 2, WQ = W / 4;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < items;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int q = (int)(i % WQ);
-        const long long r = i / WQ;
-        const int y = (int)(r % H);
-        const long long nc = r / H;
-        float4* dst = reinterpret_cast<float4*>(dX + (nc * H + y) * W + 4 * q);
-        if (y & 1) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < items; i += gridDim.x * blockDim.x) {
+        uint32_t q;
+        const uint32_t row = wq.split(i, q);  // plane * H/2 + output row: H is even, so input row 2 * row of the stack of planes
+        const float4 v = *reinterpret_cast<const float4*>(X + 2LL * row * W + 4 * q);
+        reinterpret_cast<float2*>(Xsub)[i] = make_float2(v.x, v.z);
+    }
+}
+__global__ void __launch_bounds__(256) upsample2_zero_vec_kernel(const float* __restrict__ dXsub, float* __restrict__ dX, const FastDiv wq,
+                                                                 uint32_t items, int accumulate) {
+    griddep_wait();
+    griddep_launch();
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < items; i += gridDim.x * blockDim.x) {
+        uint32_t q;
+        const uint32_t row = wq.split(i, q);  // row of the stack of planes
+        float4* dst = reinterpret_cast<float4*>(dX) + i;
+        if (row & 1) {
             if (!accumulate) *dst = make_float4(0.f, 0.f, 0.f, 0.f);
             continue;
         }
-        const float2 a = *reinterpret_cast<const float2*>(dXsub + (nc * H2 + (y >> 1)) * W2 + 2 * q);
+        const float2 a = reinterpret_cast<const float2*>(dXsub)[(row >> 1) * wq.d + q];
         if (accumulate) {
             const float4 old = *dst;
             *dst = make_float4(old.x + a.x, old.y, old.z + a.y, old.w);
@@ -672,6 +671,8 @@ __global__ void upsample2_zero_vec_kernel(const float* __restrict__ dXsub, float
         }
     }
 }
+// the vector kernels index items, and step past the end by up to kRelayoutItems grids, in 32 bits
+constexpr long long kMostItems = 1LL << 30;
 static bool vec_ok(const void* a, const void* b, int W) {
     return (W & 3) == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15u) == 0;
 }
@@ -680,50 +681,65 @@ static bool vec_ok(const void* a, const void* b, int W) {
 // tensor core reads, lo = rna_tf32(x - hi)), four pixels per thread; planes C .. Cp of both halves are zeroed (Cp: C rounded up
 // to the 8 channels of a K step). X may be batch-strided, X2 is dense.
 __device__ __forceinline__ float4 lo4(float4 v) { return make_float4(tf32_lo(v.x), tf32_lo(v.y), tf32_lo(v.z), tf32_lo(v.w)); }
-__global__ void tf32_split2_kernel(const float* __restrict__ X, float* __restrict__ X2, long long per4, long long perp4,
-                                   long long x_batch, long long items) {
+__global__ void __launch_bounds__(256) tf32_split2_kernel(const float* __restrict__ X, float* __restrict__ X2, long long per4,
+                                                          const FastDiv perp4, long long x_batch, uint32_t items) {
     griddep_wait();
     griddep_launch();
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < items; i += (long long)gridDim.x * blockDim.x) {
-        const long long n = i / perp4, r = i - n * perp4;
-        const float4 v = r < per4 ? *reinterpret_cast<const float4*>(X + n * x_batch + 4 * r) : make_float4(0.f, 0.f, 0.f, 0.f);
-        float4* dst = reinterpret_cast<float4*>(X2) + n * 2 * perp4 + r;
-        dst[0] = v;
-        dst[perp4] = lo4(v);
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < items; i0 += kRelayoutItems * stride) {
+        float4 v[kRelayoutItems];
+        uint32_t n[kRelayoutItems], r[kRelayoutItems];
+#pragma unroll
+        for (int u = 0; u < kRelayoutItems; ++u) {
+            n[u] = perp4.split(i0 + u * stride, r[u]);
+            v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i0 + u * stride < items && r[u] < per4) v[u] = *reinterpret_cast<const float4*>(X + n[u] * x_batch + 4LL * r[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < kRelayoutItems; ++u) {
+            if (i0 + u * stride >= items) break;
+            float4* dst = reinterpret_cast<float4*>(X2) + 2LL * n[u] * perp4.d + r[u];
+            dst[0] = v[u];
+            dst[perp4.d] = lo4(v[u]);
+        }
     }
 }
 // The same together with the phase split of a stride-2 convolution: X2 holds 2 * Cp planes of H/2 x W/2, the 4 C phase planes
 // of X and, Cp planes later, their lo parts (Cp: 4 C rounded up to a multiple of 8, the planes between zeroed).
-__global__ void space_to_depth2_split_kernel(const float* __restrict__ X, float* __restrict__ X2, int C, int Cp, int H, int W,
-                                             long long items) {
+__global__ void __launch_bounds__(256) space_to_depth2_split_kernel(const float* __restrict__ X, float* __restrict__ X2, const PlaneIndex ix,
+                                                                    int Cp, int W2, long long plane2, uint32_t items) {
     griddep_wait();
     griddep_launch();
-    const int H2 = H / 2, W2 = W / 2, WQ = W / 4;
-    const long long half = (long long)Cp * H2 * W2, pad = (long long)(Cp - 4 * C) * H2 * W2;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < items; i += (long long)gridDim.x * blockDim.x) {
-        const int q = (int)(i % WQ);
-        long long r = i / WQ;
-        const int y = (int)(r % H);
-        r /= H;
-        const int c = (int)(r % C);
-        const long long n = r / C;
-        const float4 v = *reinterpret_cast<const float4*>(X + ((n * C + c) * H + y) * W + 4 * q);
-        const float4 l = lo4(v);
-        const int row = y & 1;
-        float* d0 = X2 + n * 2 * half + ((2LL * row * C + c) * H2 + (y >> 1)) * W2 + 2 * q;  // phase (row, 0)
-        float* d1 = d0 + (long long)C * H2 * W2;                                             // phase (row, 1)
-        *reinterpret_cast<float2*>(d0) = make_float2(v.x, v.z);
-        *reinterpret_cast<float2*>(d1) = make_float2(v.y, v.w);
-        *reinterpret_cast<float2*>(d0 + half) = make_float2(l.x, l.z);
-        *reinterpret_cast<float2*>(d1 + half) = make_float2(l.y, l.w);
-        // the padding planes of an image are spread over its threads
-        const long long per_image = (long long)C * H * WQ, at = i - n * per_image;
-        for (long long z = at; z < pad; z += per_image) X2[n * 2 * half + half - pad + z] = X2[n * 2 * half + 2 * half - pad + z] = 0.f;
+    const uint32_t stride = gridDim.x * blockDim.x, C = ix.c.d;
+    const long long half = Cp * plane2, pad = (Cp - 4LL * C) * plane2;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < items; i0 += kRelayoutItems * stride) {
+        float4 v[kRelayoutItems];
+#pragma unroll
+        for (int u = 0; u < kRelayoutItems; ++u)
+            if (i0 + u * stride < items) v[u] = reinterpret_cast<const float4*>(X)[i0 + u * stride];
+#pragma unroll
+        for (int u = 0; u < kRelayoutItems; ++u) {
+            if (i0 + u * stride >= items) break;
+            uint32_t q, y, c;
+            const uint32_t n = ix.c.split(ix.h.split(ix.wq.split(i0 + u * stride, q), y), c);
+            const float4 l = lo4(v[u]);
+            float* image = X2 + n * 2 * half;
+            float* d0 = image + (2LL * (y & 1) * C + c) * plane2 + (y >> 1) * W2 + 2 * q;  // phase (row, 0)
+            float* d1 = d0 + C * plane2;                                                   // phase (row, 1)
+            *reinterpret_cast<float2*>(d0) = make_float2(v[u].x, v[u].z);
+            *reinterpret_cast<float2*>(d1) = make_float2(v[u].y, v[u].w);
+            *reinterpret_cast<float2*>(d0 + half) = make_float2(l.x, l.z);
+            *reinterpret_cast<float2*>(d1 + half) = make_float2(l.y, l.w);
+            // the padding planes of an image are spread over its items
+            const uint32_t per_image = C * ix.h.d * ix.wq.d;
+            for (long long z = i0 + u * stride - n * per_image; z < pad; z += per_image)
+                image[half - pad + z] = image[2 * half - pad + z] = 0.f;
+        }
     }
 }
 
-int relayout_grid(const cb_ctx* ctx, long long n) {
-    long long g = (n + 255) / 256;
+int relayout_grid(const cb_ctx* ctx, long long n, int per_thread = 1) {
+    long long g = (n + 256LL * per_thread - 1) / (256LL * per_thread);
     const long long cap = (long long)ctx->sm_count * 16;
     return (int)(g > cap ? cap : (g < 1 ? 1 : g));
 }
@@ -980,8 +996,9 @@ int launch_conv(cb_ctx* err_ctx, const ConvEnv& env, const ConvPlan& q, const fl
 
 int launch_space_to_depth2(cb_ctx* ctx, const float* X, float* Xs, int N, int C, int H, int W) {
     const long long n_el = (long long)N * C * H * W;
-    cudaError_t e = vec_ok(X, Xs, W)
-                        ? launch_dep(ctx, space_to_depth2_vec_kernel, dim3((unsigned)relayout_grid(ctx, n_el / 4)), dim3(256), 0, X, Xs, C, H, W, n_el / 4)
+    cudaError_t e = vec_ok(X, Xs, W) && n_el / 4 <= kMostItems
+                        ? launch_dep(ctx, space_to_depth2_vec_kernel, dim3((unsigned)relayout_grid(ctx, n_el / 4, kRelayoutItems)), dim3(256), 0, X, Xs,
+                                     PlaneIndex{FastDiv(W / 4), FastDiv(H), FastDiv(C)}, W / 2, (long long)(H / 2) * (W / 2), (uint32_t)(n_el / 4))
                         : launch_dep(ctx, space_to_depth2_kernel, dim3((unsigned)relayout_grid(ctx, n_el)), dim3(256), 0, X, Xs, C, H, W, n_el);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return check_cuda(ctx, e, "space_to_depth2_kernel launch");
@@ -991,8 +1008,9 @@ int launch_space_to_depth2(cb_ctx* ctx, const float* X, float* Xs, int N, int C,
 int launch_subsample2(cb_ctx* ctx, const float* X, float* Xsub, long long NC, int H, int W) {
     const long long n_sub = NC * (H / 2) * (W / 2);
     const long long n_items = NC * (H / 2) * (W / 4);
-    cudaError_t e = vec_ok(X, Xsub, W)
-                        ? launch_dep(ctx, subsample2_vec_kernel, dim3((unsigned)relayout_grid(ctx, n_items)), dim3(256), 0, X, Xsub, NC, H, W, n_items)
+    cudaError_t e = vec_ok(X, Xsub, W) && n_items <= kMostItems
+                        ? launch_dep(ctx, subsample2_vec_kernel, dim3((unsigned)relayout_grid(ctx, n_items)), dim3(256), 0, X, Xsub, FastDiv(W / 4), W,
+                                     (uint32_t)n_items)
                         : launch_dep(ctx, subsample2_kernel, dim3((unsigned)relayout_grid(ctx, n_sub)), dim3(256), 0, X, Xsub, NC, H, W, n_sub);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return check_cuda(ctx, e, "subsample2_kernel launch");
@@ -1165,8 +1183,9 @@ static int run_pass(cb_ctx* ctx, const ConvEnv& env, const ConvPlan& q, const Pa
         if (rc != CB_OK) return rc;
         float* X2 = static_cast<float*>(ctx->workspace3);
         const long long items = (long long)N * (perp / 4);
-        cudaError_t e = launch_dep(ctx, tf32_split2_kernel, dim3((unsigned)relayout_grid(ctx, items)), dim3(256), 0, X, X2, per / 4,
-                                   perp / 4, in_batch ? in_batch : per, items);
+        if (items > kMostItems) return CB_EUNSUPPORTED;
+        cudaError_t e = launch_dep(ctx, tf32_split2_kernel, dim3((unsigned)relayout_grid(ctx, items, kRelayoutItems)), dim3(256), 0, X, X2,
+                                   per / 4, FastDiv(perp / 4), in_batch ? in_batch : per, (uint32_t)items);
         if (e == cudaSuccess) e = cudaGetLastError();
         if (e != cudaSuccess) return check_cuda(ctx, e, "tf32_split2_kernel launch");
         ctx->launches += 1;
@@ -1178,8 +1197,9 @@ static int run_pass(cb_ctx* ctx, const ConvEnv& env, const ConvPlan& q, const Pa
 
 int launch_space_to_depth2_split(cb_ctx* ctx, const float* X, float* X2, int N, int C, int Cp, int H, int W) {
     const long long items = (long long)N * C * H * (W / 4);
-    cudaError_t e = launch_dep(ctx, space_to_depth2_split_kernel, dim3((unsigned)relayout_grid(ctx, items)), dim3(256), 0, X, X2, C, Cp, H,
-                               W, items);
+    if (items > kMostItems) return CB_EUNSUPPORTED;
+    cudaError_t e = launch_dep(ctx, space_to_depth2_split_kernel, dim3((unsigned)relayout_grid(ctx, items, kRelayoutItems)), dim3(256), 0, X,
+                               X2, PlaneIndex{FastDiv(W / 4), FastDiv(H), FastDiv(C)}, Cp, W / 2, (long long)(H / 2) * (W / 2), (uint32_t)items);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return check_cuda(ctx, e, "space_to_depth2_split_kernel launch");
     ctx->launches += 1;
@@ -1240,9 +1260,9 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
             rc = run_pass(ctx, env, q, ps, W, X /* = dY */, cin, sub, plain, N, H2, W2, 1, 1, 0, 0, 0, 0);
             const long long n_full = (long long)N * IC * IH * IW;
             if (rc == CB_OK) {
-                if (vec_ok(sub, Y, IW))
+                if (vec_ok(sub, Y, IW) && n_full / 4 <= kMostItems)
                     launch_dep(ctx, upsample2_zero_vec_kernel, dim3((unsigned)relayout_grid(ctx, n_full / 4)), dim3(256), 0,
-                               (const float*)sub, Y /* = dX */, IH, IW, n_full / 4, ep.accumulate ? 1 : 0);
+                               (const float*)sub, Y /* = dX */, FastDiv(IW / 4), (uint32_t)(n_full / 4), ep.accumulate ? 1 : 0);
                 else
                     launch_dep(ctx, upsample2_zero_kernel, dim3((unsigned)relayout_grid(ctx, n_full)), dim3(256), 0, (const float*)sub,
                                Y /* = dX */, IH, IW, n_full, ep.accumulate ? 1 : 0);
@@ -1298,9 +1318,10 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
         if (rc != CB_OK) return rc;
     }
     const long long n_full = (long long)N * IC * IH * IW;
-    cudaError_t e = vec_ok(dXs, Y, IW)
-                        ? launch_dep(ctx, depth_to_space2_vec_kernel, dim3((unsigned)relayout_grid(ctx, n_full / 4)), dim3(256), 0,
-                                     (const float*)dXs, Y /* = dX */, N, IC, IH, IW, per_group, n_full / 4, ep.accumulate ? 1 : 0)
+    cudaError_t e = vec_ok(dXs, Y, IW) && n_full / 4 <= kMostItems
+                        ? launch_dep(ctx, depth_to_space2_vec_kernel, dim3((unsigned)relayout_grid(ctx, n_full / 4, kRelayoutItems)), dim3(256), 0,
+                                     (const float*)dXs, Y /* = dX */, PlaneIndex{FastDiv(IW / 4), FastDiv(IH), FastDiv(IC)}, N, W2, plane2,
+                                     FastDiv(per_group), (uint32_t)(n_full / 4), ep.accumulate ? 1 : 0)
                         : launch_dep(ctx, depth_to_space2_kernel, dim3((unsigned)relayout_grid(ctx, n_full)), dim3(256), 0,
                                      (const float*)dXs, Y /* = dX */, N, IC, IH, IW, per_group, n_full, ep.accumulate ? 1 : 0);
     if (e == cudaSuccess) e = cudaGetLastError();

@@ -450,33 +450,44 @@ __global__ void __launch_bounds__(32 * kReduceGroups) wgrad_reduce_kernel(float*
 
 // lo[n][i] = rna_tf32(x - hi(x)) of x[n * x_batch + i], hi = the 19 bits the tensor core reads; four elements per
 // thread, lo dense with `per4` float4 per image.
-__global__ void tf32_lo4_kernel(const float* __restrict__ x, float* __restrict__ lo, long long per4, long long x_batch,
-                                long long items) {
+__global__ void __launch_bounds__(256) tf32_lo4_kernel(const float* __restrict__ x, float* __restrict__ lo, const FastDiv per4,
+                                                       long long x_batch, uint32_t items) {
     griddep_wait();
     griddep_launch();
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < items; i += (long long)gridDim.x * blockDim.x) {
-        const long long n = i / per4, r = i - n * per4;
-        const float4 v = *reinterpret_cast<const float4*>(x + n * x_batch + 4 * r);
-        const float in[4] = {v.x, v.y, v.z, v.w};
-        float out[4];
+    constexpr int U = 4;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < items; i0 += U * stride) {
+        float4 v[U];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float hi = __uint_as_float(__float_as_uint(in[e]) & 0xFFFFE000u);
-            uint32_t q;
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(q) : "f"(in[e] - hi));
-            out[e] = __uint_as_float(q);
+        for (int u = 0; u < U; ++u) {
+            uint32_t r;
+            const uint32_t n = per4.split(i0 + u * stride, r);
+            if (i0 + u * stride < items) v[u] = *reinterpret_cast<const float4*>(x + n * x_batch + 4LL * r);
         }
-        reinterpret_cast<float4*>(lo)[i] = make_float4(out[0], out[1], out[2], out[3]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (i0 + u * stride >= items) break;
+            const float in[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+            float out[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                uint32_t q;
+                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(q) : "f"(in[e] - __uint_as_float(__float_as_uint(in[e]) & 0xFFFFE000u)));
+                out[e] = __uint_as_float(q);
+            }
+            reinterpret_cast<float4*>(lo)[i0 + u * stride] = make_float4(out[0], out[1], out[2], out[3]);
+        }
     }
 }
 
 int launch_lo(cb_ctx* ctx, const float* x, float* lo, long long images, long long per, long long x_batch) {
     const long long items = images * (per / 4);
-    long long g = (items + 255) / 256;
+    if (items > (1LL << 30)) return CB_EUNSUPPORTED;  // 32-bit item indexes
+    long long g = (items + 1023) / 1024;
     const long long cap = (long long)ctx->sm_count * 16;
     if (g > cap) g = cap;
     if (g < 1) g = 1;
-    cudaError_t e = launch_dep(ctx, tf32_lo4_kernel, dim3((unsigned)g), dim3(256), 0, x, lo, per / 4, x_batch ? x_batch : per, items);
+    cudaError_t e = launch_dep(ctx, tf32_lo4_kernel, dim3((unsigned)g), dim3(256), 0, x, lo, FastDiv(per / 4), x_batch ? x_batch : per, (uint32_t)items);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return check_cuda(ctx, e, "tf32_lo4_kernel launch");
     ctx->launches += 1;
