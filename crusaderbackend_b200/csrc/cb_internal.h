@@ -57,6 +57,23 @@ struct cb_ctx {
 
 namespace cb {
 
+// Division of n < 2^31 by a run-time constant as a multiply and a shift: the re-layout kernels move 16 bytes a thread and
+// their 64-bit index divisions took longer than that (space_to_depth2 of 17 MB 16 us).
+struct FastDiv {
+    uint32_t d, m, s;
+    __host__ explicit FastDiv(long long divisor = 1) : d((uint32_t)divisor), m(0), s(0) {
+        while ((1ull << s) < d) ++s;
+        m = (uint32_t)(((1ull << 32) * ((1ull << s) - d)) / d + 1);
+    }
+    __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(n, m) + n) >> s; }
+    // n = q * d + r
+    __device__ __forceinline__ uint32_t split(uint32_t n, uint32_t& r) const {
+        const uint32_t q = div(n);
+        r = n - q * d;
+        return q;
+    }
+};
+
 int fail(cb_ctx* ctx, int code, const std::string& msg);
 int check_cuda(cb_ctx* ctx, cudaError_t e, const char* what);
 // Text for a CBK_* code a kernel left in a status word.

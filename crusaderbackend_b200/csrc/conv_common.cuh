@@ -11,23 +11,6 @@ constexpr int kCB = 8;          // input channels per UMMA K step
 constexpr int kConvMaxStages = 8;
 constexpr int kRowBytes = 128;  // one line of 32 floats
 
-// Division of n < 2^31 by a run-time constant as a multiply and a shift: the re-layout kernels move 16 bytes a thread and
-// their 64-bit index divisions took longer than that (space_to_depth2 of 17 MB 16 us).
-struct FastDiv {
-    uint32_t d, m, s;
-    __host__ explicit FastDiv(long long divisor = 1) : d((uint32_t)divisor), m(0), s(0) {
-        while ((1ull << s) < d) ++s;
-        m = (uint32_t)(((1ull << 32) * ((1ull << s) - d)) / d + 1);
-    }
-    __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(n, m) + n) >> s; }
-    // n = q * d + r
-    __device__ __forceinline__ uint32_t split(uint32_t n, uint32_t& r) const {
-        const uint32_t q = div(n);
-        r = n - q * d;
-        return q;
-    }
-};
-
 // Source filter tap of the stride-2 convolution that lands on (input phase, tap of the 2x2 phase convolution):
 // with ih = 2 oh + fh - 1, tap fh = 0 reads phase 1 at row oh - 1, fh = 1 phase 0 at row oh, fh = 2 phase 1 at row oh.
 __host__ __device__ __forceinline__ int s2_tap(int phase, int t) { return phase == 1 ? (t == 0 ? 0 : 2) : (t == 1 ? 1 : -1); }

@@ -443,7 +443,7 @@ struct PackJob {
     const float* W;
     float* Wp;
     int OC, IC, FHs, FWs, FHc, FWc, OCp, CG, mode, out_first, out_count, x3;
-    long long total;  // floats of the packed filter
+    unsigned total;   // floats of the packed filter (of at most a few hundred kilobytes)
 };
 
 // Value of the packed filter at channel ch of row (fh, fw, o), zero outside the filter.
@@ -451,9 +451,9 @@ __device__ __forceinline__ float pack_source(const PackJob& j, int ch, int fh, i
     const float* W = j.W;
     const int OC = j.OC, IC = j.IC, FHs = j.FHs, FWs = j.FWs;
     if (j.mode == PACK_FWD) {
-        if (o < OC && ch < IC) return W[(((long long)o * IC + ch) * FHs + fh) * FWs + fw];
+        if (o < OC && ch < IC) return W[((o * IC + ch) * FHs + fh) * FWs + fw];
     } else if (j.mode == PACK_DGRAD) {
-        if (o < IC && ch < OC) return W[(((long long)ch * IC + o) * FHs + (FHs - 1 - fh)) * FWs + (FWs - 1 - fw)];
+        if (o < IC && ch < OC) return W[((ch * IC + o) * FHs + (FHs - 1 - fh)) * FWs + (FWs - 1 - fw)];
     } else if (j.mode == PACK_S2_FWD) {
         if (o < OC && ch < 4 * IC) {
             const int phase = ch / IC, cc = ch - phase * IC;
@@ -475,15 +475,15 @@ __device__ __forceinline__ float tf32_lo(float x) {
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u)));
     return __uint_as_float(r);
 }
-__device__ __forceinline__ float pack_value(const PackJob& j, long long i) {
+__device__ __forceinline__ float pack_value(const PackJob& j, unsigned i) {
     const int c = (int)(i & 31);
-    long long r = i >> 5;
-    const int o = (int)(r % j.OCp);
-    r /= j.OCp;
-    const int fw = (int)(r % j.FWc);
-    r /= j.FWc;
-    const int cg = (int)(r % j.CG);
-    const int fh = (int)(r / j.CG);
+    unsigned r = i >> 5;
+    const int o = (int)(r % (unsigned)j.OCp);
+    r /= (unsigned)j.OCp;
+    const int fw = (int)(r % (unsigned)j.FWc);
+    r /= (unsigned)j.FWc;
+    const int cg = (int)(r % (unsigned)j.CG);
+    const int fh = (int)(r / (unsigned)j.CG);
     const int ch = cg * 32 + c;
     if (j.x3 == 0 || ch < j.x3) return pack_source(j, ch, fh, fw, o);
     return ch < 2 * j.x3 ? tf32_lo(pack_source(j, ch - j.x3, fh, fw, o)) : 0.f;
@@ -492,16 +492,14 @@ __device__ __forceinline__ float pack_value(const PackJob& j, long long i) {
 __global__ void pack_filter_kernel(const PackJob j) {
     griddep_wait();
     griddep_launch();
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < j.total; i += (long long)gridDim.x * blockDim.x)
-        j.Wp[i] = pack_value(j, i);
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < j.total; i += gridDim.x * blockDim.x) j.Wp[i] = pack_value(j, i);
 }
 // Every cached filter of a context in one launch: blockIdx.y indexes a device table of jobs.
 __global__ void pack_filter_table_kernel(const PackJob* __restrict__ jobs) {
     griddep_wait();
     griddep_launch();
     const PackJob j = jobs[blockIdx.y];
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < j.total; i += (long long)gridDim.x * blockDim.x)
-        j.Wp[i] = pack_value(j, i);
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < j.total; i += gridDim.x * blockDim.x) j.Wp[i] = pack_value(j, i);
 }
 
 // ---- re-layout kernels of the stride-2 path (memory-bound, one element per thread, coalesced on the write side)
@@ -858,7 +856,7 @@ PackJob make_job(const PackSpec& ps, const ConvPlan& q, const float* W, float* d
     j.W = W; j.Wp = dst;
     j.OC = ps.OC; j.IC = ps.IC; j.FHs = ps.FHs; j.FWs = ps.FWs; j.FHc = FH; j.FWc = FW;
     j.OCp = q.OCp; j.CG = q.CG; j.x3 = q.x3; j.mode = ps.mode; j.out_first = ps.out_first; j.out_count = ps.out_count;
-    j.total = (long long)q.w_total_bytes / 4;
+    j.total = (unsigned)(q.w_total_bytes / 4);
     return j;
 }
 

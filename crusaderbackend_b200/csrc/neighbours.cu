@@ -168,34 +168,6 @@ __global__ void bn_bwd_kernel(const float* __restrict__ dY, const float* __restr
     }
 }
 
-template <int VEC>
-__global__ void bn_paramgrad_kernel(const float* __restrict__ dY, const float* __restrict__ xhat,
-                                    float* __restrict__ dgamma, float* __restrict__ dbeta, int N, long long P) {
-    const long long nvec = P / VEC;
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nvec;
-         v += (long long)gridDim.x * blockDim.x) {
-        const long long p = v * VEC;
-        float sg[VEC], sb[VEC];
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) { sg[e] = 0.f; sb[e] = 0.f; }
-        for (int n = 0; n < N; ++n) {
-            float h[VEC], dy[VEC];
-            if (VEC == 4) {
-                *reinterpret_cast<float4*>(h) = *reinterpret_cast<const float4*>(xhat + n * P + p);
-                *reinterpret_cast<float4*>(dy) = *reinterpret_cast<const float4*>(dY + n * P + p);
-            } else {
-                h[0] = xhat[n * P + p];
-                dy[0] = dY[n * P + p];
-            }
-#pragma unroll
-            for (int e = 0; e < VEC; ++e) { sb[e] += dy[e]; sg[e] += dy[e] * h[e]; }
-        }
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) { dgamma[p + e] = sg[e]; dbeta[p + e] = sb[e]; }
-    }
-}
-
-
 // ------------------------------------------------------------------ BatchNorm, batch-parallel form
 // Block = 16 float4 position vectors (64 positions, 256 contiguous bytes per sample) x 16 batch groups. Every thread
 // keeps its SPT samples (n = group, group + 16, ...) in registers, so X (and dY) are read from HBM exactly once;
@@ -218,10 +190,10 @@ __device__ __forceinline__ float4 bn_group_sum(float4 v, float4 (*red)[16]) {
 // Sums, over the G batch groups of a block, of Q float4 quantities per position vector; every thread returns the totals
 // of its position. The G x (Q float4) values go through shared memory once: thread (x, g) with g < 4 Q adds component
 // g & 3 of quantity g >> 2 over the groups in group order (a fixed order: deterministic), and everyone reads the
-// totals back. red: Q * 1024 floats, tot: Q * (1024 / G) floats.
-template <int Q, int G>
+// totals back. red: Q * 4 T floats (T threads), tot: Q * (4 T / G) floats.
+template <int Q, int G, int T>
 __device__ __forceinline__ void bn_block_sums(float4 (&v)[Q], float* red, float* tot) {
-    constexpr int W = (256 / G) * 4;  // floats per group row: the block's positions
+    constexpr int W = (T / G) * 4;  // floats per group row: the block's positions
     static_assert(G >= 4 * Q, "one summing thread per (quantity, component)");
     const int x = threadIdx.x, g = threadIdx.y;
 #pragma unroll
@@ -239,17 +211,36 @@ __device__ __forceinline__ void bn_block_sums(float4 (&v)[Q], float* red, float*
     for (int q = 0; q < Q; ++q) v[q] = *reinterpret_cast<const float4*>(tot + q * W + x * 4);
 }
 
-// Block = 256 / G float4 position vectors x G batch groups (G = 16, 32 or 64: more groups for small maps, so that the
-// grid still covers the GPU); thread (x, g) keeps samples n = g, g + G, ... (SPT of them) in registers.
-template <int SPT, int G>
-__global__ void __launch_bounds__(256) bn_fwd_par_kernel(const float* __restrict__ X, const float* __restrict__ beta,
+// Block = T / G float4 position vectors x G batch groups; thread (x, g) keeps samples n = g, g + G, ... (SPT of them) in
+// registers (the launchers below choose).
+// Positions p .. p+3 of a sample (or of a parameter): one 16-byte access, or, where P is no multiple of 4 or a tensor is not on
+// 16 bytes (V false), up to four of 4 bytes.
+template <bool V>
+__device__ __forceinline__ float4 ld4(const float* __restrict__ row, long long p, long long P) {
+    if (V) return *reinterpret_cast<const float4*>(row + p);
+    return make_float4(row[p], p + 1 < P ? row[p + 1] : 0.f, p + 2 < P ? row[p + 2] : 0.f, p + 3 < P ? row[p + 3] : 0.f);
+}
+template <bool V>
+__device__ __forceinline__ void st4(float* row, long long p, long long P, float4 v) {
+    if (V) {
+        *reinterpret_cast<float4*>(row + p) = v;
+        return;
+    }
+    row[p] = v.x;
+    if (p + 1 < P) row[p + 1] = v.y;
+    if (p + 2 < P) row[p + 2] = v.z;
+    if (p + 3 < P) row[p + 3] = v.w;
+}
+
+template <int T, int G, int SPT, bool V>
+__global__ void __launch_bounds__(T) bn_fwd_par_kernel(const float* __restrict__ X, const float* __restrict__ beta,
                                                          const float* __restrict__ gamma, float* __restrict__ mean,
                                                          float* __restrict__ var, float* __restrict__ Y,
                                                          float* __restrict__ xhat, const float* __restrict__ res, int N,
                                                          long long P, int relu, long long xs) {
     // xs: floats between consecutive samples of X (P when dense; larger for a channel-prefix view of a wider tensor)
-    constexpr int PB = 256 / G;
-    __shared__ __align__(16) float red[1024];
+    constexpr int PB = T / G;
+    __shared__ __align__(16) float red[4 * T];
     __shared__ __align__(16) float tot[PB * 4];
     griddep_wait();
     griddep_launch();
@@ -257,18 +248,18 @@ __global__ void __launch_bounds__(256) bn_fwd_par_kernel(const float* __restrict
     const bool live = p < P;
     const int g = threadIdx.y;
     // the parameters are fetched with the samples: behind the sums their latency would be paid on its own
-    const float4 ga = live ? *reinterpret_cast<const float4*>(gamma + p) : f4_zero();
-    const float4 be = live ? *reinterpret_cast<const float4*>(beta + p) : f4_zero();
+    const float4 ga = live ? ld4<V>(gamma, p, P) : f4_zero();
+    const float4 be = live ? ld4<V>(beta, p, P) : f4_zero();
     float4 x[SPT];
     float4 s[1] = {f4_zero()};
 #pragma unroll
     for (int i = 0; i < SPT; ++i) {
         const int n = g + G * i;
-        x[i] = (live && n < N) ? *reinterpret_cast<const float4*>(X + (long long)n * xs + p) : f4_zero();
+        x[i] = (live && n < N) ? ld4<V>(X + (long long)n * xs, p, P) : f4_zero();
         s[0] = f4_add(s[0], x[i]);
     }
     const float invN = 1.0f / (float)N;
-    bn_block_sums<1, G>(s, red, tot);
+    bn_block_sums<1, G, T>(s, red, tot);
     const float4 m = make_float4(s[0].x * invN, s[0].y * invN, s[0].z * invN, s[0].w * invN);
     float4 q[1] = {f4_zero()};
 #pragma unroll
@@ -278,7 +269,7 @@ __global__ void __launch_bounds__(256) bn_fwd_par_kernel(const float* __restrict
             q[0] = f4_add(q[0], make_float4(a * a, b * b, c * c, d * d));
         }
     }
-    bn_block_sums<1, G>(q, red, tot);
+    bn_block_sums<1, G, T>(q, red, tot);
     const float4 v = make_float4(q[0].x * invN, q[0].y * invN, q[0].z * invN, q[0].w * invN);
     if (!live) return;
     const float4 inv = make_float4(1.0f / sqrtf(v.x + 1e-8f), 1.0f / sqrtf(v.y + 1e-8f), 1.0f / sqrtf(v.z + 1e-8f),
@@ -290,58 +281,58 @@ __global__ void __launch_bounds__(256) bn_fwd_par_kernel(const float* __restrict
             const float4 h = make_float4((x[i].x - m.x) * inv.x, (x[i].y - m.y) * inv.y, (x[i].z - m.z) * inv.z,
                                          (x[i].w - m.w) * inv.w);
             float4 y = make_float4(h.x * ga.x + be.x, h.y * ga.y + be.y, h.z * ga.z + be.z, h.w * ga.w + be.w);
-            if (res) y = f4_add(y, *reinterpret_cast<const float4*>(res + (long long)n * P + p));  // shortcut add
+            if (res) y = f4_add(y, ld4<V>(res + (long long)n * P, p, P));  // shortcut add
             if (relu) y = make_float4(fmaxf(y.x, 0.f), fmaxf(y.y, 0.f), fmaxf(y.z, 0.f), fmaxf(y.w, 0.f));
-            *reinterpret_cast<float4*>(Y + (long long)n * P + p) = y;
-            if (xhat) *reinterpret_cast<float4*>(xhat + (long long)n * P + p) = h;
+            st4<V>(Y + (long long)n * P, p, P, y);
+            if (xhat) st4<V>(xhat + (long long)n * P, p, P, h);
         }
     }
     if (g == 0) {
-        if (mean) *reinterpret_cast<float4*>(mean + p) = m;
-        if (var) *reinterpret_cast<float4*>(var + p) = v;
+        if (mean) st4<V>(mean, p, P, m);
+        if (var) st4<V>(var, p, P, v);
     }
 }
 
 // Data gradient (statistics recomputed from X as seblas::batchNormGrad does) and, when dgamma / dbeta are given, the
 // parameter gradients dbeta = sum dy, dgamma = sum dy * xhat of seblas::batchNormParamGrads in the same pass.
-template <int SPT, int G>
-__global__ void __launch_bounds__(256, SPT <= 4 ? 4 : 1) bn_bwd_par_kernel(const float* __restrict__ dY, const float* __restrict__ gamma,
+template <int T, int G, int SPT, bool V>
+__global__ void __launch_bounds__(T, SPT <= 4 ? 1024 / T : 1) bn_bwd_par_kernel(const float* __restrict__ dY, const float* __restrict__ gamma,
                                                          const float* __restrict__ X, float* __restrict__ dX,
                                                          float* __restrict__ dgamma, float* __restrict__ dbeta,
                                                          const float* __restrict__ relu_out, float* __restrict__ dres,
                                                          int dres_add, int pg_add, int N, long long P, long long xs,
                                                          long long dxs, int dx_add) {
     // xs / dxs: floats between consecutive samples of X / dX (P when dense); dx_add: dX += instead of dX =
-    constexpr int PB = 256 / G;
-    __shared__ __align__(16) float red[4 * 1024];
+    constexpr int PB = T / G;
+    __shared__ __align__(16) float red[16 * T];
     __shared__ __align__(16) float tot[4 * PB * 4];
     griddep_wait();
     griddep_launch();
     const long long p = ((long long)blockIdx.x * PB + threadIdx.x) * 4;
     const bool live = p < P;
     const int g = threadIdx.y;
-    const float4 ga = live ? *reinterpret_cast<const float4*>(gamma + p) : f4_zero();
+    const float4 ga = live ? ld4<V>(gamma, p, P) : f4_zero();
     float4 x[SPT], dy[SPT];
     float4 s[1] = {f4_zero()};
 #pragma unroll
     for (int i = 0; i < SPT; ++i) {
         const int n = g + G * i;
         const bool on = live && n < N;
-        x[i] = on ? *reinterpret_cast<const float4*>(X + (long long)n * xs + p) : f4_zero();
-        dy[i] = on ? *reinterpret_cast<const float4*>(dY + (long long)n * P + p) : f4_zero();
+        x[i] = on ? ld4<V>(X + (long long)n * xs, p, P) : f4_zero();
+        dy[i] = on ? ld4<V>(dY + (long long)n * P, p, P) : f4_zero();
         if (relu_out && on) {  // the ReLU that followed this layer in the forward pass: dy passes where its output is > 0
-            const float4 r = *reinterpret_cast<const float4*>(relu_out + (long long)n * P + p);
+            const float4 r = ld4<V>(relu_out + (long long)n * P, p, P);
             dy[i] = make_float4(r.x > 0.f ? dy[i].x : 0.f, r.y > 0.f ? dy[i].y : 0.f, r.z > 0.f ? dy[i].z : 0.f,
                                 r.w > 0.f ? dy[i].w : 0.f);
         }
         if (dres && on) {  // the shortcut that was added before that ReLU receives the same masked gradient
-            float4* d = reinterpret_cast<float4*>(dres + (long long)n * P + p);
-            *d = dres_add ? f4_add(*d, dy[i]) : dy[i];
+            float* d = dres + (long long)n * P;
+            st4<V>(d, p, P, dres_add ? f4_add(ld4<V>(d, p, P), dy[i]) : dy[i]);
         }
         s[0] = f4_add(s[0], x[i]);
     }
     const float invN = 1.0f / (float)N;
-    bn_block_sums<1, G>(s, red, tot);
+    bn_block_sums<1, G, T>(s, red, tot);
     const float4 m = make_float4(s[0].x * invN, s[0].y * invN, s[0].z * invN, s[0].w * invN);
     // sums of xc^2, dy * xc (dxhat = dy * gamma is factored out below), dy and xc, in one exchange
     float4 sums[4] = {f4_zero(), f4_zero(), f4_zero(), f4_zero()};
@@ -356,7 +347,7 @@ __global__ void __launch_bounds__(256, SPT <= 4 ? 4 : 1) bn_bwd_par_kernel(const
             sums[3] = f4_add(sums[3], xc);
         }
     }
-    bn_block_sums<4, G>(sums, red, tot);
+    bn_block_sums<4, G, T>(sums, red, tot);
     const float4 sq = sums[0], sdx = sums[1], sd = sums[2], sxc = sums[3];
     if (!live) return;
     float o_inv[4], o_dvar[4], o_dmean[4];
@@ -378,23 +369,24 @@ __global__ void __launch_bounds__(256, SPT <= 4 ? 4 : 1) bn_bwd_par_kernel(const
             o.y = dy[i].y * gav[1] * o_inv[1] + o_dvar[1] * x[i].y * 2.0f * invN + o_dmean[1] * invN;
             o.z = dy[i].z * gav[2] * o_inv[2] + o_dvar[2] * x[i].z * 2.0f * invN + o_dmean[2] * invN;
             o.w = dy[i].w * gav[3] * o_inv[3] + o_dvar[3] * x[i].w * 2.0f * invN + o_dmean[3] * invN;
-            float4* dst = reinterpret_cast<float4*>(dX + (long long)n * dxs + p);
-            *dst = dx_add ? f4_add(*dst, o) : o;
+            float* dst = dX + (long long)n * dxs;
+            st4<V>(dst, p, P, dx_add ? f4_add(ld4<V>(dst, p, P), o) : o);
         }
     }
     if (g == 0 && dgamma && dbeta) {
         float4 gb = sd;
         float4 gg = make_float4(sdx.x * o_inv[0], sdx.y * o_inv[1], sdx.z * o_inv[2], sdx.w * o_inv[3]);  // sum dy * xhat
         if (pg_add) {  // a later group of a batch whose statistics are taken per group
-            gb = f4_add(gb, *reinterpret_cast<const float4*>(dbeta + p));
-            gg = f4_add(gg, *reinterpret_cast<const float4*>(dgamma + p));
+            gb = f4_add(gb, ld4<V>(dbeta, p, P));
+            gg = f4_add(gg, ld4<V>(dgamma, p, P));
         }
-        *reinterpret_cast<float4*>(dbeta + p) = gb;
-        *reinterpret_cast<float4*>(dgamma + p) = gg;
+        st4<V>(dbeta, p, P, gb);
+        st4<V>(dgamma, p, P, gg);
     }
 }
 
 // Parameter gradients alone (seblas::batchNormParamGrads): one pass over dY and xhat, batch-parallel.
+template <bool V>
 __global__ void __launch_bounds__(256) bn_paramgrad_par_kernel(const float* __restrict__ dY, const float* __restrict__ xhat,
                                                                float* __restrict__ dgamma, float* __restrict__ dbeta,
                                                                int N, long long P) {
@@ -407,8 +399,8 @@ __global__ void __launch_bounds__(256) bn_paramgrad_par_kernel(const float* __re
     if (live) {
 #pragma unroll 4
         for (int n = threadIdx.y; n < N; n += 16) {
-            const float4 h = *reinterpret_cast<const float4*>(xhat + (long long)n * P + p);
-            const float4 d = *reinterpret_cast<const float4*>(dY + (long long)n * P + p);
+            const float4 h = ld4<V>(xhat + (long long)n * P, p, P);
+            const float4 d = ld4<V>(dY + (long long)n * P, p, P);
             sb = f4_add(sb, d);
             sg = f4_add(sg, make_float4(d.x * h.x, d.y * h.y, d.z * h.z, d.w * h.w));
         }
@@ -416,69 +408,55 @@ __global__ void __launch_bounds__(256) bn_paramgrad_par_kernel(const float* __re
     sg = bn_group_sum(sg, red);
     sb = bn_group_sum(sb, red);
     if (live && threadIdx.y == 0) {
-        *reinterpret_cast<float4*>(dgamma + p) = sg;
-        *reinterpret_cast<float4*>(dbeta + p) = sb;
+        st4<V>(dgamma, p, P, sg);
+        st4<V>(dbeta, p, P, sb);
     }
 }
 
 // Eligibility of the batch-parallel kernels: non-zero when N <= 256 (16 samples per thread at 16 groups).
 inline int bn_spt(int N) { return N <= 256 ? 1 : 0; }
 
-// Batch groups per block: 32 when every group still gets two samples, else 16 (measured on the ResNet-56 step at
-// batch 128 / 64 / 16: 32 groups beat 16 and 64 on every map size once N >= 64); then the samples per thread, the
-// smallest power of two >= ceil(N / groups).
-struct BnShape { int groups, spt; unsigned grid; };
-inline BnShape bn_shape(const cb_ctx* ctx, int N, long long P) {
-    static const int forced = [] {
-        const char* e = std::getenv("CB_BN_GROUPS");  // development override: 16, 32 or 64
-        return e ? std::atoi(e) : 0;
-    }();
-    int G = N >= 64 ? 32 : 16;
-    static const int small64 = [] {
-        const char* e = std::getenv("CB_BN_SMALL64");  // development switch, default on
-        return e ? std::atoi(e) : 1;
-    }();
-    if (small64 && G == 32 && N >= 128 && (P / 4 + 7) / 8 < ctx->sm_count) G = 64;  // maps too small to fill the GPU at 32
-    if (forced == 16 || forced == 32 || forced == 64) G = forced;
-    const int need = (N + G - 1) / G;
-    int spt = 1;
-    while (spt < need) spt <<= 1;
-    const int pb = 256 / G;
-    return BnShape{G, spt, (unsigned)((P / 4 + pb - 1) / pb)};
+// Launches one instantiation: T threads as T / G vectors of 16 bytes (what a sample contributes contiguously) x G batch groups,
+// SPT samples a thread (G * SPT >= N).
+template <int T, int G, typename... KArgs, typename... Args>
+void launch_bn(cb_ctx* ctx, void (*kernel)(KArgs...), long long P, Args... args) {
+    constexpr int pb = T / G;
+    launch_dep(ctx, kernel, dim3((unsigned)(((P + 3) / 4 + pb - 1) / pb)), dim3((unsigned)pb, (unsigned)G), 0, args...);
 }
 
-#define BN_DISPATCH(shape, KERNEL, ...)                                                                        \
-    do {                                                                                                       \
-        const dim3 blk_((unsigned)(256 / (shape).groups), (unsigned)(shape).groups);                            \
-        switch ((shape).groups * 100 + (shape).spt) {                                                          \
-            case 1601: launch_dep(ctx, KERNEL<1, 16>, dim3((shape).grid), blk_, 0, __VA_ARGS__); break;        \
-            case 1602: launch_dep(ctx, KERNEL<2, 16>, dim3((shape).grid), blk_, 0, __VA_ARGS__); break;        \
-            case 1604: launch_dep(ctx, KERNEL<4, 16>, dim3((shape).grid), blk_, 0, __VA_ARGS__); break;        \
-            case 1608: launch_dep(ctx, KERNEL<8, 16>, dim3((shape).grid), blk_, 0, __VA_ARGS__); break;        \
-            case 1616: launch_dep(ctx, KERNEL<16, 16>, dim3((shape).grid), blk_, 0, __VA_ARGS__); break;       \
-            case 3201: launch_dep(ctx, KERNEL<1, 32>, dim3((shape).grid), blk_, 0, __VA_ARGS__); break;        \
-            case 3202: launch_dep(ctx, KERNEL<2, 32>, dim3((shape).grid), blk_, 0, __VA_ARGS__); break;        \
-            case 3204: launch_dep(ctx, KERNEL<4, 32>, dim3((shape).grid), blk_, 0, __VA_ARGS__); break;        \
-            case 3208: launch_dep(ctx, KERNEL<8, 32>, dim3((shape).grid), blk_, 0, __VA_ARGS__); break;        \
-            case 6401: launch_dep(ctx, KERNEL<1, 64>, dim3((shape).grid), blk_, 0, __VA_ARGS__); break;        \
-            case 6402: launch_dep(ctx, KERNEL<2, 64>, dim3((shape).grid), blk_, 0, __VA_ARGS__); break;        \
-            default: launch_dep(ctx, KERNEL<4, 64>, dim3((shape).grid), blk_, 0, __VA_ARGS__); break;          \
-        }                                                                                                      \
-    } while (0)
-
+// Sixteen groups (256 contiguous bytes of a sample) as long as four samples a thread suffice, and for wide layers, which are
+// bound by DRAM, also with eight; otherwise thirty-two. Measured, us, 16 against 32 groups: N 64, P 135168 10.9 / 14.1;
+// 80, 128000 15.5 / 17.9; 128, 131072 24.3 / 27.1; 128, 16384 4.5 / 3.7; 173, 111616 38.2 / 34.4.
 void launch_bn_fwd_par(cb_ctx* ctx, const float* X, const float* beta, const float* gamma, float* mean, float* var, float* Y,
-                       float* xhat, const float* res, int N, long long P, int relu, long long xs = 0) {
-    const BnShape sh = bn_shape(ctx, N, P);
+                       float* xhat, const float* res, int N, long long P, int relu, long long xs = 0, bool vec = true) {
     if (xs == 0) xs = P;
-    BN_DISPATCH(sh, bn_fwd_par_kernel, X, beta, gamma, mean, var, Y, xhat, res, N, P, relu, xs);
+#define CB_BN(T, G, SPT) launch_bn<T, G>(ctx, vec ? bn_fwd_par_kernel<T, G, SPT, true> : bn_fwd_par_kernel<T, G, SPT, false>, P, X, beta, gamma, mean, var, Y, xhat, res, N, P, relu, xs)
+    if (N <= 16) CB_BN(256, 16, 1);
+    else if (N <= 32) CB_BN(256, 16, 2);
+    else if (N <= 64) CB_BN(256, 16, 4);
+    else if (N <= 128 && P >= 65536) CB_BN(256, 16, 8);
+    else if (N <= 128) CB_BN(256, 32, 4);
+    else CB_BN(256, 32, 8);
+#undef CB_BN
 }
+// The backward kernel holds two tensors' samples: never more than four a thread (eight cost half its occupancy: N 128,
+// P 131072 with sixteen groups 70 us against 47). N 64: sixteen groups 27.3 / 28.0 at P 135168 and 8.1 / 8.9 at 49152, but
+// 3.0 / 2.5 at 4096. N 173, P 111616: 512 threads in 64 groups 69 us against 95 with eight samples in 32.
 void launch_bn_bwd_par(cb_ctx* ctx, const float* dY, const float* gamma, const float* X, float* dX, float* dgamma,
                        float* dbeta, const float* relu_out, float* dres, int dres_add, int pg_add, int N, long long P,
-                       long long xs = 0, long long dxs = 0, int dx_add = 0) {
-    const BnShape sh = bn_shape(ctx, N, P);
+                       long long xs = 0, long long dxs = 0, int dx_add = 0, bool vec = true) {
     if (xs == 0) xs = P;
     if (dxs == 0) dxs = P;
-    BN_DISPATCH(sh, bn_bwd_par_kernel, dY, gamma, X, dX, dgamma, dbeta, relu_out, dres, dres_add, pg_add, N, P, xs, dxs, dx_add);
+#define CB_BN(T, G, SPT)                                                                                                          \
+    launch_bn<T, G>(ctx, vec ? bn_bwd_par_kernel<T, G, SPT, true> : bn_bwd_par_kernel<T, G, SPT, false>, P, dY, gamma, X, dX, dgamma, dbeta, relu_out, dres, dres_add, pg_add, N, P, xs, \
+                    dxs, dx_add)
+    if (N <= 16) CB_BN(256, 16, 1);
+    else if (N <= 32) CB_BN(256, 16, 2);
+    else if (N < 64 || (N == 64 && P >= 32768)) CB_BN(256, 16, 4);
+    else if (N == 64) CB_BN(256, 32, 2);
+    else if (N <= 128) CB_BN(256, 32, 4);
+    else CB_BN(512, 64, 4);
+#undef CB_BN
 }
 
 // ------------------------------------------------------------------ elementwise
@@ -597,6 +575,43 @@ __global__ void avgpool_back_kernel(float* __restrict__ dX, const float* __restr
             o = n * ys + ((c - n * C) * OH + oh) * (long long)OW + ow;
         }
         dX[i] = (oh < OH && ow < OW) ? dY[o] * inv : 0.f;
+    }
+}
+// 2 x 2 windows on maps with W % 4 == 0 and 16-byte aligned dense rows, the transitions of the DenseNets: a thread moves four
+// input pixels of a row, index division by multiply and shift (38 MB of gradient: 35 us with an element and two 64-bit
+// divisions a thread). ys as above.
+struct PoolIndex {
+    FastDiv wq, oh, c;  // quads of an input row, output rows, channels
+};
+__global__ void __launch_bounds__(kThreads) avgpool2_kernel(const float* __restrict__ X, float* __restrict__ Y, const PoolIndex ix,
+                                                            long long ys, uint32_t items) {
+    griddep_wait();
+    griddep_launch();
+    const uint32_t stride = gridDim.x * blockDim.x, wq = ix.wq.d;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < items; i += stride) {
+        uint32_t q, oh, c;
+        const uint32_t row = ix.wq.split(i, q);            // (n * C + c) * OH + oh
+        const uint32_t n = ix.c.split(ix.oh.split(row, oh), c);
+        const float4* src = reinterpret_cast<const float4*>(X) + 2LL * row * wq + q;
+        const float4 a = src[0], b = src[wq];
+        float* dst = Y + n * ys + (c * ix.oh.d + oh) * 2LL * wq + 2 * q;
+        *reinterpret_cast<float2*>(dst) = make_float2((((a.x + a.y) + b.x) + b.y) * 0.25f, (((a.z + a.w) + b.z) + b.w) * 0.25f);
+    }
+}
+__global__ void __launch_bounds__(kThreads) avgpool2_back_kernel(float* __restrict__ dX, const float* __restrict__ dY, const PoolIndex ix,
+                                                                 long long ys, uint32_t items) {
+    griddep_wait();
+    griddep_launch();
+    const uint32_t stride = gridDim.x * blockDim.x, wq = ix.wq.d;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < items; i += stride) {
+        uint32_t q, oh, c;
+        const uint32_t row = ix.wq.split(i, q);
+        const uint32_t n = ix.c.split(ix.oh.split(row, oh), c);
+        const float2 d = *reinterpret_cast<const float2*>(dY + n * ys + (c * ix.oh.d + oh) * 2LL * wq + 2 * q);
+        const float4 v = make_float4(d.x * 0.25f, d.x * 0.25f, d.y * 0.25f, d.y * 0.25f);
+        float4* dst = reinterpret_cast<float4*>(dX) + 2LL * row * wq + q;
+        dst[0] = v;
+        dst[wq] = v;
     }
 }
 // Global average pool: one warp per (n,c) plane.
@@ -746,7 +761,7 @@ __global__ void slice_add_kernel(float* __restrict__ dst, const float* __restric
 // Forward, one CTA per sample: global average pooling over the H*W plane of every channel, the dense layer
 // logits = W pooled + b, the softmax y = exp(x - max) / (sum + 1e-10), the loss gradient y - label and the sample's
 // loss -sum(log(y + 1e-10) * label): what GlobalAvgPool, Linear, Softmax and the cross-entropy pair do in four launches.
-__global__ void __launch_bounds__(256) head_fwd_kernel(const float* __restrict__ X, const float* __restrict__ W,
+__global__ void __launch_bounds__(1024) head_fwd_kernel(const float* __restrict__ X, const float* __restrict__ W,
                                                        const float* __restrict__ b, const float* __restrict__ labels,
                                                        float* __restrict__ pooled, float* __restrict__ logits,
                                                        float* __restrict__ probs, float* __restrict__ dlogits,
@@ -759,7 +774,8 @@ __global__ void __launch_bounds__(256) head_fwd_kernel(const float* __restrict__
     const float* Xn = X + (long long)n * C * HW;
     // pooling: a warp takes four channels at a time so that their loads are in flight together; each channel is summed
     // lane-strided, then across the lanes
-    for (int c0 = warp * 4; c0 < C; c0 += 32) {
+    const int warps = blockDim.x >> 5;
+    for (int c0 = warp * 4; c0 < C; c0 += 4 * warps) {
         float s[4] = {0.f, 0.f, 0.f, 0.f};
         for (int i = lane; i < HW; i += 32) {
 #pragma unroll
@@ -777,7 +793,7 @@ __global__ void __launch_bounds__(256) head_fwd_kernel(const float* __restrict__
     }
     __syncthreads();
     // logits: one warp per class, lanes stride the channels (coalesced weight rows), summed across the lanes
-    for (int m = warp; m < M; m += 8) {
+    for (int m = warp; m < M; m += warps) {
         float a = 0.f;
         for (int c = lane; c < C; c += 32) a = fmaf(W[(long long)m * C + c], sh[c], a);
         a = warp_sum(a);
@@ -825,7 +841,15 @@ __global__ void __launch_bounds__(256) head_bwd_kernel(const float* __restrict__
         }
         __syncthreads();
         float* out = dX + (long long)n * C * HW;
-        for (int i = threadIdx.x; i < C * HW; i += blockDim.x) out[i] = sh[i / HW];
+        if ((HW & 3) == 0 && (reinterpret_cast<uintptr_t>(dX) & 15u) == 0) {
+            const unsigned quads = (unsigned)HW / 4;
+            for (unsigned i = threadIdx.x; i < (unsigned)C * quads; i += blockDim.x) {
+                const float v = sh[i / quads];
+                reinterpret_cast<float4*>(out)[i] = make_float4(v, v, v, v);
+            }
+        } else {
+            for (int i = threadIdx.x; i < C * HW; i += blockDim.x) out[i] = sh[i / HW];
+        }
         return;
     }
     const int w_ctas = (M * C + 255) / 256;
@@ -900,8 +924,9 @@ int cb_bn_fwd(cb_ctx* ctx, const float* X, const float* beta, const float* gamma
     if (!X || !beta || !gamma || !Y) return fail(ctx, CB_EINVAL, "cb_bn_fwd: null operand");
     const bool vec = (P % 4 == 0) && aligned16(X) && aligned16(Y) && (!xhat || aligned16(xhat));
     const int spt = bn_spt(N);
-    if (vec && spt > 0 && aligned16(beta) && aligned16(gamma) && (!mean || aligned16(mean)) && (!var || aligned16(var))) {
-        launch_bn_fwd_par(ctx, X, beta, gamma, mean, var, Y, xhat, nullptr, N, P, 0);
+    if (spt > 0) {
+        launch_bn_fwd_par(ctx, X, beta, gamma, mean, var, Y, xhat, nullptr, N, P, 0, 0,
+                          vec && aligned16(beta) && aligned16(gamma) && (!mean || aligned16(mean)) && (!var || aligned16(var)));
         return done(ctx, "cb_bn_fwd");
     }
     if (vec) bn_fwd_kernel<4><<<grid_for(ctx, P / 4, 128), 128, 0, ctx->stream>>>(X, beta, gamma, mean, var, Y, xhat, N, P);
@@ -916,8 +941,8 @@ int cb_bn_bwd(cb_ctx* ctx, const float* dY, const float* gamma, const float* X, 
     if (!dY || !gamma || !X || !dX) return fail(ctx, CB_EINVAL, "cb_bn_bwd: null operand");
     const bool vec = (P % 4 == 0) && aligned16(X) && aligned16(dY) && aligned16(dX);
     const int spt = bn_spt(N);
-    if (vec && spt > 0 && aligned16(gamma)) {
-        launch_bn_bwd_par(ctx, dY, gamma, X, dX, nullptr, nullptr, nullptr, nullptr, 0, 0, N, P);
+    if (spt > 0) {
+        launch_bn_bwd_par(ctx, dY, gamma, X, dX, nullptr, nullptr, nullptr, nullptr, 0, 0, N, P, 0, 0, 0, vec && aligned16(gamma));
         return done(ctx, "cb_bn_bwd");
     }
     if (vec) bn_bwd_kernel<4><<<grid_for(ctx, P / 4, 128), 128, 0, ctx->stream>>>(dY, gamma, X, dX, N, P);
@@ -930,13 +955,9 @@ int cb_bn_paramgrad(cb_ctx* ctx, const float* dY, const float* xhat, float* dgam
     if (N < 0 || P < 0) return fail(ctx, CB_EINVAL, "cb_bn_paramgrad: negative extent");
     if (P == 0) return CB_OK;
     if (!dY || !xhat || !dgamma || !dbeta) return fail(ctx, CB_EINVAL, "cb_bn_paramgrad: null operand");
-    const bool vec = (P % 4 == 0) && aligned16(xhat) && aligned16(dY);
-    if (vec && aligned16(dgamma) && aligned16(dbeta)) {
-        launch_dep(ctx, bn_paramgrad_par_kernel, dim3((unsigned)((P / 4 + 15) / 16)), dim3(16, 16), 0, dY, xhat, dgamma, dbeta, N, P);
-        return done(ctx, "cb_bn_paramgrad");
-    }
-    if (vec) bn_paramgrad_kernel<4><<<grid_for(ctx, P / 4, 128), 128, 0, ctx->stream>>>(dY, xhat, dgamma, dbeta, N, P);
-    else bn_paramgrad_kernel<1><<<grid_for(ctx, P, 128), 128, 0, ctx->stream>>>(dY, xhat, dgamma, dbeta, N, P);
+    const bool vec = (P % 4 == 0) && aligned16(xhat) && aligned16(dY) && aligned16(dgamma) && aligned16(dbeta);
+    launch_dep(ctx, vec ? bn_paramgrad_par_kernel<true> : bn_paramgrad_par_kernel<false>, dim3((unsigned)(((P + 3) / 4 + 15) / 16)), dim3(16, 16), 0,
+               dY, xhat, dgamma, dbeta, N, P);
     return done(ctx, "cb_bn_paramgrad");
 }
 
@@ -1073,13 +1094,38 @@ int cb_grad_handover(cb_ctx* ctx, float* dA, float* dA_reserve, long long n) {
     return launch_eltwise<OP_ADD_ZERO_B>(ctx, dA, dA_reserve, dA, 0.f, n, "cb_grad_handover");
 }
 
+inline bool pool2_ok(const float* wide, const float* pooled, long long N, int C, int H, int W, int rH, int rW, long long ys) {
+    return rH == 2 && rW == 2 && (H & 1) == 0 && (W & 3) == 0 && aligned16(wide) && aligned16(pooled) && (ys & 1) == 0 &&
+           N * C * H * W < (1LL << 31);
+}
+static void launch_avgpool(cb_ctx* ctx, const float* X, float* Y, long long N, int C, int H, int W, int rH, int rW, long long ys) {
+    if (pool2_ok(X, Y, N, C, H, W, rH, rW, ys)) {
+        const long long items = N * C * (H / 2) * (W / 4);
+        launch_dep(ctx, avgpool2_kernel, dim3((unsigned)grid_for(ctx, items)), dim3(kThreads), 0, X, Y,
+                   PoolIndex{FastDiv(W / 4), FastDiv(H / 2), FastDiv(C)}, ys ? ys : (long long)C * (H / 2) * (W / 2), (uint32_t)items);
+        return;
+    }
+    const long long total = N * C * (H / rH) * (W / rW);
+    avgpool_kernel<<<grid_for(ctx, total), kThreads, 0, ctx->stream>>>(X, Y, total, H, W, rH, rW, C, ys);
+}
+static void launch_avgpool_back(cb_ctx* ctx, float* dX, const float* dY, long long N, int C, int H, int W, int rH, int rW,
+                                long long ys) {
+    if (pool2_ok(dX, dY, N, C, H, W, rH, rW, ys)) {
+        const long long items = N * C * (H / 2) * (W / 4);
+        launch_dep(ctx, avgpool2_back_kernel, dim3((unsigned)grid_for(ctx, items)), dim3(kThreads), 0, dX, dY,
+                   PoolIndex{FastDiv(W / 4), FastDiv(H / 2), FastDiv(C)}, ys ? ys : (long long)C * (H / 2) * (W / 2), (uint32_t)items);
+        return;
+    }
+    const long long total = N * C * H * W;
+    avgpool_back_kernel<<<grid_for(ctx, total), kThreads, 0, ctx->stream>>>(dX, dY, total, H, W, rH, rW, C, ys);
+}
 int cb_avgpool(cb_ctx* ctx, const float* X, float* Y, long long NC, int H, int W, int rH, int rW) {
     if (int rc_enter = enter(ctx)) return rc_enter;
     if (NC < 0 || H < 0 || W < 0 || rH < 1 || rW < 1) return fail(ctx, CB_EINVAL, "cb_avgpool: bad extent");
     const long long total = NC * (H / rH) * (W / rW);
     if (total == 0) return CB_OK;
     if (!X || !Y) return fail(ctx, CB_EINVAL, "cb_avgpool: null operand");
-    avgpool_kernel<<<grid_for(ctx, total), kThreads, 0, ctx->stream>>>(X, Y, total, H, W, rH, rW, 1, 0);
+    launch_avgpool(ctx, X, Y, NC, 1, H, W, rH, rW, 0);
     return done(ctx, "cb_avgpool");
 }
 
@@ -1091,7 +1137,7 @@ int cb_avgpool_ex(cb_ctx* ctx, const float* X, float* Y, int N, int C, int H, in
     if (!X || !Y) return fail(ctx, CB_EINVAL, "cb_avgpool_ex: null operand");
     if (y_batch_stride && y_batch_stride < (long long)C * (H / rH) * (W / rW))
         return fail(ctx, CB_EINVAL, "cb_avgpool_ex: batch stride smaller than one pooled sample");
-    avgpool_kernel<<<grid_for(ctx, total), kThreads, 0, ctx->stream>>>(X, Y, total, H, W, rH, rW, C, y_batch_stride);
+    launch_avgpool(ctx, X, Y, N, C, H, W, rH, rW, y_batch_stride);
     return done(ctx, "cb_avgpool_ex");
 }
 
@@ -1104,7 +1150,7 @@ int cb_avgpool_back_ex(cb_ctx* ctx, float* dX, const float* dY, int N, int C, in
     if (!dX || !dY) return fail(ctx, CB_EINVAL, "cb_avgpool_back_ex: null operand");
     if (dy_batch_stride && dy_batch_stride < (long long)C * (H / rH) * (W / rW))
         return fail(ctx, CB_EINVAL, "cb_avgpool_back_ex: batch stride smaller than one pooled sample");
-    avgpool_back_kernel<<<grid_for(ctx, total), kThreads, 0, ctx->stream>>>(dX, dY, total, H, W, rH, rW, C, dy_batch_stride);
+    launch_avgpool_back(ctx, dX, dY, N, C, H, W, rH, rW, dy_batch_stride);
     return done(ctx, "cb_avgpool_back_ex");
 }
 
@@ -1114,7 +1160,7 @@ int cb_avgpool_back(cb_ctx* ctx, float* dX, const float* dY, long long NC, int H
     const long long total = NC * H * W;
     if (total == 0) return CB_OK;
     if (!dX || !dY) return fail(ctx, CB_EINVAL, "cb_avgpool_back: null operand");
-    avgpool_back_kernel<<<grid_for(ctx, total), kThreads, 0, ctx->stream>>>(dX, dY, total, H, W, rH, rW, 1, 0);
+    launch_avgpool_back(ctx, dX, dY, NC, 1, H, W, rH, rW, 0);
     return done(ctx, "cb_avgpool_back");
 }
 
@@ -1166,7 +1212,7 @@ int cb_head_fwd(cb_ctx* ctx, const float* X, const float* W, const float* b, con
     if (N == 0) return CB_OK;
     if (!X || !W || !labels || !pooled || !logits || !probs || !dlogits || !loss_per_sample)
         return fail(ctx, CB_EINVAL, "cb_head_fwd: null operand");
-    launch_dep(ctx, head_fwd_kernel, dim3((unsigned)N), dim3(256), (size_t)(C + 32) * sizeof(float), X, W, b, labels, pooled, logits, probs,
+    launch_dep(ctx, head_fwd_kernel, dim3((unsigned)N), dim3((long long)C * HW > 8192 ? 1024u : 256u), (size_t)(C + 32) * sizeof(float), X, W, b, labels, pooled, logits, probs,
                dlogits, loss_per_sample, C, HW, M);
     return done(ctx, "cb_head_fwd");
 }

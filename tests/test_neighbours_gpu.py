@@ -121,6 +121,13 @@ def test_batchnorm(torch_cuda, ctxs, shape):
         assert orc.max_err_norm(dg2.cpu().numpy().ravel(), rdg_m) <= 2e-5
         assert orc.max_err_norm(db2.cpu().numpy().ravel(), rdb_m) <= F32
 
+@pytest.mark.parametrize("shape", [(16, 5, 3, 7), (17, 5, 3, 7), (32, 1, 2, 9), (33, 5, 3, 7), (64, 5, 3, 7), (64, 33, 32, 32), (65, 1, 1, 2),
+                                   (65, 67, 31, 32), (128, 3, 3, 3), (129, 3, 4, 4), (256, 5, 3, 7), (256, 2, 3, 6), (257, 3, 3, 3)])
+def test_batchnorm_block_shapes(torch_cuda, ctxs, shape):
+    """Either side of each batch at which the block shape changes, with and without 16-byte vectors (P % 4)."""
+    test_batchnorm(torch_cuda, ctxs, shape)
+
+
 
 def test_golden_batchnorm(torch_cuda, ctxs, golden):
     from tests.golden.make_golden import CASES, inputs
