@@ -47,7 +47,7 @@ struct GatherParams {
     const float* Wt; int w_ch, w_out, FW;                    // filter strides: contraction channel, output channel; width
     float* Out; long long out_batch; int OUTC, OHH, OWW;     // output channels, rows, columns
     int N, sgn;
-    int splits, per_split, atomic_out;
+    int splits, per_split, atomic_out, tap_major;
     ConvEpilogue ep;
     PixelSet sets[kMaxSets]; // blockIdx.z = set * splits + split
 };
@@ -99,7 +99,8 @@ struct GatherSource {
             TapK e{0, 0xffffffffu, -1, 0};
             if (k < s.K) {
                 const int taps = s.TH * s.TW;
-                const int c = k / taps, r = k - c * taps;
+                // the order in which a pixel's products are added: channel by channel, or (data gradient) tap by tap
+                const int c = p.tap_major ? k % p.C : k / taps, r = p.tap_major ? k / p.C : k - c * taps;
                 const int th = r / s.TW, tw = r - th * s.TW;
                 e.off = (c * p.H + p.sgn * th) * p.W + p.sgn * tw;
                 e.bits = tap_bits<MASK>(th, tw, p.sgn);
@@ -309,12 +310,13 @@ __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_wgrad_simt(const Wgra
 }
 
 // One launch for up to four pixel sets. The contraction is split over CTAs where the output alone does not fill the GPU and the
-// epilogue is a plain sum (the output is then cleared first).
+// epilogue is a plain sum (the output is then cleared first), except in the passes of a model: atomic sums come in any order, and
+// one rounding more or less in an activation moves the gradients of a deep model by percents from one run to the next.
 int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, const char* who) {
     const long long out_elems = (long long)p.OUTC * p.OHH * p.OWW;
     if ((long long)p.C * p.H * p.W >= (1LL << 29) || out_elems >= (1LL << 31) || (long long)p.C * p.w_ch >= (1LL << 31))
         return fail(ctx, CB_EUNSUPPORTED, std::string(who) + ": an image or filter of more than 2^29 values");
-    bool may_split = !ctx->deterministic && !p.ep.scale && !p.ep.relu;
+    bool may_split = !ctx->deterministic && !ctx->model_pass && !p.ep.scale && !p.ep.relu;
     int most = 0;
     for (int i = 0; i < nsets; ++i) most = sets[i].K > most ? sets[i].K : most;
     const simt::Choice c = simt::choose_tile(ctx->sm_count, (long long)p.N * sets[0].UH * sets[0].UW * nsets, p.OUTC,
@@ -367,7 +369,7 @@ int simt_conv_dgrad(cb_ctx* ctx, const float* W, const float* dY, float* dX, con
     p.In = dY; p.in_batch = g.y_batch; p.C = g.OC; p.H = g.OH; p.W = g.OW;
     p.Wt = W; p.w_ch = g.IC * g.FH * g.FW; p.w_out = g.FH * g.FW; p.FW = g.FW;
     p.Out = dX; p.out_batch = g.x_batch; p.OUTC = g.IC; p.OHH = g.IH; p.OWW = g.IW;
-    p.N = g.N; p.sgn = -1; p.ep.accumulate = accumulate;
+    p.N = g.N; p.sgn = -1; p.ep.accumulate = accumulate; p.tap_major = 1;
     std::vector<PixelSet> sets;
     for (int a = 0; a < g.sH; ++a)
         for (int b = 0; b < g.sW; ++b) {

@@ -65,7 +65,8 @@ struct ConvParams {
     long long out_batch;      // elements between consecutive images of the output
     ConvEpilogue ep;
     int f_wrap;         // > 0: K steps (8 channels) from f_wrap on take the packed filter's rows f_wrap steps earlier (3xTF32)
-    int c_wrap;         // > 0: input channels from c_wrap on are read again from channel (c - c_wrap) (3xTF32 form)
+    int c_wrap;         // > 0: input channels from c_wrap on are read again from channel (c - c_wrap) (3xTF32 form), and of the
+                        // channels before it the second half comes first
     int* status;
     long long* trace;
     int dbg;       // development probes of the trace build
@@ -264,7 +265,8 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps == 8 ? 2 : 1)
                 const uint32_t dst0 = st_base + s * p.stage_bytes;
                 mbar_expect_tx_elect(full, p.stage_bytes);
                 int c0 = cb * p.KS * kCB;
-                if (p.c_wrap && c0 >= p.c_wrap) c0 -= p.c_wrap;  // third channel group of the 3xTF32 form: x_hi again
+                if (p.c_wrap)  // 3xTF32: [x ; x_lo] in memory is read as x_lo, x, x
+                    c0 = c0 >= p.c_wrap ? c0 - p.c_wrap : (2 * c0 >= p.c_wrap ? c0 - p.c_wrap / 2 : c0 + p.c_wrap / 2);
                 if (p.shared_rows) {
                     // W == 32: the tile is 4 consecutive rows of one image; ONE box (32 px, 8*KS channels, FH+3
                     // rows) lands as [row][channel][128 B]; rows above / below the image are zero-filled
@@ -332,7 +334,7 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps == 8 ? 2 : 1)
                 const uint64_t pbase = descP0 + (uint64_t)(((st_base + s * p.stage_bytes) >> 4) & 0x3FFFu);
                 // a stage holds 1, 2 or 4 K steps of 8 channels, never across a 32-channel group of the packed filter
                 const uint32_t ks0 = (uint32_t)(cb * p.KS);
-                // 3xTF32: the groups [x ; x_lo ; x] meet the packed groups [w ; w_lo] as w, w, w_lo
+                // 3xTF32: the groups [x_lo ; x ; x] meet the packed groups [w ; w_lo] as w, w_lo, w
                 const uint32_t fs0 = p.f_wrap && ks0 >= (uint32_t)p.f_wrap ? ks0 - (uint32_t)p.f_wrap : ks0;
                 const uint64_t q0 = descQ0 + (uint64_t)((fs0 >> 2) * q_group_units + (fs0 & 3u) * 2u);
                 for (int fh = 0; fh < p.FH; ++fh) {
@@ -817,13 +819,14 @@ int plan_conv(ConvPlan& q, int smem_optin, int sm_count, const float* X, int N, 
         const long long avail = two_per_sm ? (long long)(smem_optin < 113 * 1024 ? smem_optin : 113 * 1024) : (long long)smem_optin;
         const long long cap = avail - 4096 - (long long)c.w_bytes - 1024LL * c.ew;  // static shared memory, alignment slack; store staging
         // as many K steps per stage as leaves at least 2 stages: fewer, larger TMA boxes measured faster than a deeper
-        // pipeline of small ones
+        // pipeline of small ones. The steps of a stage are also the order in which a pixel's products are added, so they
+        // are chosen as if every plan staged for sixteen epilogue warps: no result depends on how many a plan has.
         c.KS = 0;
         for (int ks = 4; ks >= 1; ks >>= 1) {
             if (ks > cin8 && ks > 1) continue;
             if (ks > q.ks_max) continue;
-            const long long st = cap / ((long long)c.nblocks * ks * kCB * kRowBytes);
-            if (st >= 2) {
+            const long long bytes = (long long)c.nblocks * ks * kCB * kRowBytes, st = cap / bytes;
+            if ((cap - 1024LL * (16 - c.ew)) / bytes >= 2) {
                 c.KS = ks;
                 c.stages = (int)(st > kConvMaxStages ? kConvMaxStages : st);
                 break;
@@ -879,7 +882,7 @@ int launch_conv(cb_ctx* err_ctx, const ConvEnv& env, const ConvPlan& q, const fl
     p.FH = FH; p.FW = FW; p.pH = pH; p.pW = pW;
     p.OCs = q.OCs; p.nsplit = q.nsplit; p.NQ = q.NQ; p.CG = q.CG; p.KS = q.KS;
     p.c_wrap = 2 * q.x3;
-    p.f_wrap = q.x3 / kCB;
+    p.f_wrap = p.c_wrap / kCB;
     p.NCB = (q.Cin + q.KS * kCB - 1) / (q.KS * kCB);
     p.L = q.L; p.LPI = IH / q.L;
     p.shared_rows = q.shared_rows; p.nblocks = q.nblocks;
@@ -1209,11 +1212,13 @@ int launch_space_to_depth2_split(cb_ctx* ctx, const float* X, float* X2, int N, 
 // tensor-core kernel.
 //
 // x3: 3xTF32 in ONE pass of the kernel. With x = x_hi + x_lo and w = w_hi + w_lo, y = x_hi w_hi + x_lo w_hi + x_hi w_lo is a
-// single convolution over three groups of input channels, [x ; x_lo ; x] against [w ; w ; w_lo], because the tensor core itself
-// takes the hi part of what it reads. A small kernel writes [x ; x_lo] (dense scratch; for stride 2 in the phase-split layout),
-// the packed filter holds [w ; w_lo] (cached like any other), the kernel reads x a second time and w twice. Everything
-// accumulates in one TMEM accumulator and leaves through the ordinary epilogue. Against three passes into temporaries, their lo
-// parts and a sum: 32 -> 64 stride 2 at 32 x 32, batch 128, three passes of the layer 229 us before.
+// single convolution over three groups of input channels, [x_lo ; x ; x] against [w ; w_lo ; w], because the tensor core itself
+// takes the hi part of what it reads. The two corrections come first: TMEM truncates every addition at the accumulator's
+// magnitude, which they leave small (against double, 64 -> 64 channels, 3x3: 5.3e-7, and 2.3e-6 with x w first). A small kernel
+// writes [x ; x_lo] (dense scratch; for stride 2 in the phase-split layout), the packed filter holds [w ; w_lo] (cached like any
+// other), the kernel reads x a second time and w twice. Everything accumulates in one TMEM accumulator and leaves through the
+// ordinary epilogue. Against three passes into temporaries, their lo parts and a sum: 32 -> 64 stride 2 at 32 x 32, batch 128,
+// three passes of the layer 229 us before.
 int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const ConvEpilogue& ep, int N, int IC, int IH,
                   int IW, int OC, int FH, int FW, int sH, int sW, int pH, int pW, bool dgrad_of, long long in_batch,
                   long long out_batch, bool x3) {

@@ -187,23 +187,33 @@ __device__ __forceinline__ float4 bn_group_sum(float4 v, float4 (*red)[16]) {
     return t;
 }
 
-// Sums, over the G batch groups of a block, of Q float4 quantities per position vector; every thread returns the totals
-// of its position. The G x (Q float4) values go through shared memory once: thread (x, g) with g < 4 Q adds component
-// g & 3 of quantity g >> 2 over the groups in group order (a fixed order: deterministic), and everyone reads the
-// totals back. red: Q * 4 T floats (T threads), tot: Q * (4 T / G) floats.
-template <int Q, int G, int T>
+// Sums, over the R * G batch groups of a block (R a thread), of Q float4 quantities per position vector; every thread returns
+// the totals of its position. The values go through shared memory once: thread (x, g) with g < 4 Q adds component g & 3 of
+// quantity g >> 2 over the groups in group order (a fixed order: deterministic), and everyone reads the totals back.
+// red: R * Q * 4 T floats (T threads), tot: Q * (4 T / G) floats.
+// With R = 2 the values of groups 0 .. G-1 are put ahead by bn_put and v holds those of groups G .. 2G-1.
+template <int Q, int G, int R, int T>
+__device__ __forceinline__ void bn_put(float4 (&v)[Q], float* red) {
+    constexpr int W = (T / G) * 4;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        *reinterpret_cast<float4*>(red + (q * R * G + threadIdx.y) * W + threadIdx.x * 4) = v[q];
+        v[q] = f4_zero();
+    }
+}
+template <int Q, int G, int R, int T>
 __device__ __forceinline__ void bn_block_sums(float4 (&v)[Q], float* red, float* tot) {
     constexpr int W = (T / G) * 4;  // floats per group row: the block's positions
     static_assert(G >= 4 * Q, "one summing thread per (quantity, component)");
     const int x = threadIdx.x, g = threadIdx.y;
 #pragma unroll
-    for (int q = 0; q < Q; ++q) *reinterpret_cast<float4*>(red + (q * G + g) * W + x * 4) = v[q];
+    for (int q = 0; q < Q; ++q) *reinterpret_cast<float4*>(red + ((q * R + R - 1) * G + g) * W + x * 4) = v[q];
     __syncthreads();
     if (g < 4 * Q) {
-        const float* src = red + (g >> 2) * G * W + x * 4 + (g & 3);
+        const float* src = red + (g >> 2) * R * G * W + x * 4 + (g & 3);
         float t = 0.f;
 #pragma unroll
-        for (int k = 0; k < G; ++k) t += src[k * W];
+        for (int k = 0; k < R * G; ++k) t += src[k * W];
         tot[(g >> 2) * W + x * 4 + (g & 3)] = t;
     }
     __syncthreads();
@@ -211,8 +221,6 @@ __device__ __forceinline__ void bn_block_sums(float4 (&v)[Q], float* red, float*
     for (int q = 0; q < Q; ++q) v[q] = *reinterpret_cast<const float4*>(tot + q * W + x * 4);
 }
 
-// Block = T / G float4 position vectors x G batch groups; thread (x, g) keeps samples n = g, g + G, ... (SPT of them) in
-// registers (the launchers below choose).
 // Positions p .. p+3 of a sample (or of a parameter): one 16-byte access, or, where P is no multiple of 4 or a tensor is not on
 // 16 bytes (V false), up to four of 4 bytes.
 template <bool V>
@@ -232,7 +240,10 @@ __device__ __forceinline__ void st4(float* row, long long p, long long P, float4
     if (p + 3 < P) row[p + 3] = v.w;
 }
 
-template <int T, int G, int SPT, bool V>
+// Block = T / G float4 position vectors x G rows of threads; thread (x, g) keeps samples n = g, g + G, ... (SPT of them) in
+// registers. Sample n counts to batch group n mod R G, whose members are added in ascending order, then the groups: the order,
+// and with it every bit of the statistics, depends on R G alone, so the launchers below choose G by speed.
+template <int T, int G, int SPT, int R, bool V>
 __global__ void __launch_bounds__(T) bn_fwd_par_kernel(const float* __restrict__ X, const float* __restrict__ beta,
                                                          const float* __restrict__ gamma, float* __restrict__ mean,
                                                          float* __restrict__ var, float* __restrict__ Y,
@@ -240,7 +251,7 @@ __global__ void __launch_bounds__(T) bn_fwd_par_kernel(const float* __restrict__
                                                          long long P, int relu, long long xs) {
     // xs: floats between consecutive samples of X (P when dense; larger for a channel-prefix view of a wider tensor)
     constexpr int PB = T / G;
-    __shared__ __align__(16) float red[4 * T];
+    __shared__ __align__(16) float red[R * 4 * T];
     __shared__ __align__(16) float tot[PB * 4];
     griddep_wait();
     griddep_launch();
@@ -251,25 +262,31 @@ __global__ void __launch_bounds__(T) bn_fwd_par_kernel(const float* __restrict__
     const float4 ga = live ? ld4<V>(gamma, p, P) : f4_zero();
     const float4 be = live ? ld4<V>(beta, p, P) : f4_zero();
     float4 x[SPT];
-    float4 s[1] = {f4_zero()};
+    float4 s[1] = {f4_zero()}, s0[1] = {f4_zero()};
 #pragma unroll
     for (int i = 0; i < SPT; ++i) {
         const int n = g + G * i;
         x[i] = (live && n < N) ? ld4<V>(X + (long long)n * xs, p, P) : f4_zero();
-        s[0] = f4_add(s[0], x[i]);
+        if (R == 2 && i % 2 == 0) s0[0] = f4_add(s0[0], x[i]);
+        else s[0] = f4_add(s[0], x[i]);
     }
+    if (R == 2) bn_put<1, G, R, T>(s0, red);
     const float invN = 1.0f / (float)N;
-    bn_block_sums<1, G, T>(s, red, tot);
+    bn_block_sums<1, G, R, T>(s, red, tot);
     const float4 m = make_float4(s[0].x * invN, s[0].y * invN, s[0].z * invN, s[0].w * invN);
     float4 q[1] = {f4_zero()};
 #pragma unroll
-    for (int i = 0; i < SPT; ++i) {
-        if (g + G * i < N) {
-            const float a = x[i].x - m.x, b = x[i].y - m.y, c = x[i].z - m.z, d = x[i].w - m.w;
-            q[0] = f4_add(q[0], make_float4(a * a, b * b, c * c, d * d));
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int i = 0; i < SPT; ++i) {
+            if (i % R == r && g + G * i < N) {
+                const float a = x[i].x - m.x, b = x[i].y - m.y, c = x[i].z - m.z, d = x[i].w - m.w;
+                q[0] = f4_add(q[0], make_float4(a * a, b * b, c * c, d * d));
+            }
         }
+        if (r + 1 < R) bn_put<1, G, R, T>(q, red);
     }
-    bn_block_sums<1, G, T>(q, red, tot);
+    bn_block_sums<1, G, R, T>(q, red, tot);
     const float4 v = make_float4(q[0].x * invN, q[0].y * invN, q[0].z * invN, q[0].w * invN);
     if (!live) return;
     const float4 inv = make_float4(1.0f / sqrtf(v.x + 1e-8f), 1.0f / sqrtf(v.y + 1e-8f), 1.0f / sqrtf(v.z + 1e-8f),
@@ -295,7 +312,7 @@ __global__ void __launch_bounds__(T) bn_fwd_par_kernel(const float* __restrict__
 
 // Data gradient (statistics recomputed from X as seblas::batchNormGrad does) and, when dgamma / dbeta are given, the
 // parameter gradients dbeta = sum dy, dgamma = sum dy * xhat of seblas::batchNormParamGrads in the same pass.
-template <int T, int G, int SPT, bool V>
+template <int T, int G, int SPT, int R, bool V>
 __global__ void __launch_bounds__(T, SPT <= 4 ? 1024 / T : 1) bn_bwd_par_kernel(const float* __restrict__ dY, const float* __restrict__ gamma,
                                                          const float* __restrict__ X, float* __restrict__ dX,
                                                          float* __restrict__ dgamma, float* __restrict__ dbeta,
@@ -304,7 +321,7 @@ __global__ void __launch_bounds__(T, SPT <= 4 ? 1024 / T : 1) bn_bwd_par_kernel(
                                                          long long dxs, int dx_add) {
     // xs / dxs: floats between consecutive samples of X / dX (P when dense); dx_add: dX += instead of dX =
     constexpr int PB = T / G;
-    __shared__ __align__(16) float red[16 * T];
+    __shared__ __align__(16) float red[R * 16 * T];
     __shared__ __align__(16) float tot[4 * PB * 4];
     griddep_wait();
     griddep_launch();
@@ -313,7 +330,7 @@ __global__ void __launch_bounds__(T, SPT <= 4 ? 1024 / T : 1) bn_bwd_par_kernel(
     const int g = threadIdx.y;
     const float4 ga = live ? ld4<V>(gamma, p, P) : f4_zero();
     float4 x[SPT], dy[SPT];
-    float4 s[1] = {f4_zero()};
+    float4 s[1] = {f4_zero()}, s0[1] = {f4_zero()};
 #pragma unroll
     for (int i = 0; i < SPT; ++i) {
         const int n = g + G * i;
@@ -329,25 +346,31 @@ __global__ void __launch_bounds__(T, SPT <= 4 ? 1024 / T : 1) bn_bwd_par_kernel(
             float* d = dres + (long long)n * P;
             st4<V>(d, p, P, dres_add ? f4_add(ld4<V>(d, p, P), dy[i]) : dy[i]);
         }
-        s[0] = f4_add(s[0], x[i]);
+        if (R == 2 && i % 2 == 0) s0[0] = f4_add(s0[0], x[i]);
+        else s[0] = f4_add(s[0], x[i]);
     }
+    if (R == 2) bn_put<1, G, R, T>(s0, red);
     const float invN = 1.0f / (float)N;
-    bn_block_sums<1, G, T>(s, red, tot);
+    bn_block_sums<1, G, R, T>(s, red, tot);
     const float4 m = make_float4(s[0].x * invN, s[0].y * invN, s[0].z * invN, s[0].w * invN);
     // sums of xc^2, dy * xc (dxhat = dy * gamma is factored out below), dy and xc, in one exchange
     float4 sums[4] = {f4_zero(), f4_zero(), f4_zero(), f4_zero()};
 #pragma unroll
-    for (int i = 0; i < SPT; ++i) {
-        if (g + G * i < N) {
-            const float4 xc = make_float4(x[i].x - m.x, x[i].y - m.y, x[i].z - m.z, x[i].w - m.w);
-            x[i] = xc;  // keep the centred value
-            sums[0] = f4_add(sums[0], make_float4(xc.x * xc.x, xc.y * xc.y, xc.z * xc.z, xc.w * xc.w));
-            sums[1] = f4_add(sums[1], make_float4(dy[i].x * xc.x, dy[i].y * xc.y, dy[i].z * xc.z, dy[i].w * xc.w));
-            sums[2] = f4_add(sums[2], dy[i]);
-            sums[3] = f4_add(sums[3], xc);
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int i = 0; i < SPT; ++i) {
+            if (i % R == r && g + G * i < N) {
+                const float4 xc = make_float4(x[i].x - m.x, x[i].y - m.y, x[i].z - m.z, x[i].w - m.w);
+                x[i] = xc;  // keep the centred value
+                sums[0] = f4_add(sums[0], make_float4(xc.x * xc.x, xc.y * xc.y, xc.z * xc.z, xc.w * xc.w));
+                sums[1] = f4_add(sums[1], make_float4(dy[i].x * xc.x, dy[i].y * xc.y, dy[i].z * xc.z, dy[i].w * xc.w));
+                sums[2] = f4_add(sums[2], dy[i]);
+                sums[3] = f4_add(sums[3], xc);
+            }
         }
+        if (r + 1 < R) bn_put<4, G, R, T>(sums, red);
     }
-    bn_block_sums<4, G, T>(sums, red, tot);
+    bn_block_sums<4, G, R, T>(sums, red, tot);
     const float4 sq = sums[0], sdx = sums[1], sd = sums[2], sxc = sums[3];
     if (!live) return;
     float o_inv[4], o_dvar[4], o_dmean[4];
@@ -424,38 +447,49 @@ void launch_bn(cb_ctx* ctx, void (*kernel)(KArgs...), long long P, Args... args)
     launch_dep(ctx, kernel, dim3((unsigned)(((P + 3) / 4 + pb - 1) / pb)), dim3((unsigned)pb, (unsigned)G), 0, args...);
 }
 
-// Sixteen groups (256 contiguous bytes of a sample) as long as four samples a thread suffice, and for wide layers, which are
-// bound by DRAM, also with eight; otherwise thirty-two. Measured, us, 16 against 32 groups: N 64, P 135168 10.9 / 14.1;
-// 80, 128000 15.5 / 17.9; 128, 131072 24.3 / 27.1; 128, 16384 4.5 / 3.7; 173, 111616 38.2 / 34.4.
+// Batch groups: 16 below a batch of 64, 32 from there, 64 for maps too narrow to give every SM a block of 32. From a batch of 64
+// on and for wide layers, which are bound by DRAM, sixteen rows of threads (256 contiguous bytes of a sample) hold the 32 groups.
+// Measured, us, forward, 16 against 32 rows: N 64, P 135168 12.3 / 14.8, 49152 5.8 / 6.3, 21888 4.1 / 3.5; 80, 128000 15.8 / 19.7;
+// 128, 131072 24.4 / 31.4; 173, 111616 38.2 / 34.4. 512 threads in 32 rows: N 64, P 135168 18.0.
+inline bool bn_narrow(const cb_ctx* ctx, int N, long long P) { return N >= 128 && (P / 4 + 7) / 8 < ctx->sm_count; }
 void launch_bn_fwd_par(cb_ctx* ctx, const float* X, const float* beta, const float* gamma, float* mean, float* var, float* Y,
                        float* xhat, const float* res, int N, long long P, int relu, long long xs = 0, bool vec = true) {
     if (xs == 0) xs = P;
-#define CB_BN(T, G, SPT) launch_bn<T, G>(ctx, vec ? bn_fwd_par_kernel<T, G, SPT, true> : bn_fwd_par_kernel<T, G, SPT, false>, P, X, beta, gamma, mean, var, Y, xhat, res, N, P, relu, xs)
-    if (N <= 16) CB_BN(256, 16, 1);
-    else if (N <= 32) CB_BN(256, 16, 2);
-    else if (N <= 64) CB_BN(256, 16, 4);
-    else if (N <= 128 && P >= 65536) CB_BN(256, 16, 8);
-    else if (N <= 128) CB_BN(256, 32, 4);
-    else CB_BN(256, 32, 8);
+#define CB_BN(T, G, SPT, R)                                                                                                      \
+    launch_bn<T, G>(ctx, vec ? bn_fwd_par_kernel<T, G, SPT, R, true> : bn_fwd_par_kernel<T, G, SPT, R, false>, P, X, beta, gamma, \
+                      mean, var, Y, xhat, res, N, P, relu, xs)
+    if (N <= 16) CB_BN(256, 16, 1, 1);
+    else if (N <= 32) CB_BN(256, 16, 2, 1);
+    else if (N < 64) CB_BN(256, 16, 4, 1);
+    else if (N == 64 && P >= 32768) CB_BN(256, 16, 4, 2);
+    else if (N == 64) CB_BN(256, 32, 2, 1);
+    else if (bn_narrow(ctx, N, P) && N == 128) CB_BN(256, 64, 2, 1);
+    else if (bn_narrow(ctx, N, P)) CB_BN(256, 64, 4, 1);
+    else if (N <= 128 && P >= 65536) CB_BN(256, 16, 8, 2);
+    else if (N <= 128) CB_BN(256, 32, 4, 1);
+    else CB_BN(256, 32, 8, 1);
 #undef CB_BN
 }
 // The backward kernel holds two tensors' samples: never more than four a thread (eight cost half its occupancy: N 128,
-// P 131072 with sixteen groups 70 us against 47). N 64: sixteen groups 27.3 / 28.0 at P 135168 and 8.1 / 8.9 at 49152, but
-// 3.0 / 2.5 at 4096. N 173, P 111616: 512 threads in 64 groups 69 us against 95 with eight samples in 32.
+// P 131072 with sixteen rows 70 us against 47; N 173, P 111616: 512 threads in 64 rows 69 us against 95 with eight samples in 32).
+// Thirty-two groups in sixteen rows pay only where dX is added to, one more tensor through DRAM (a DenseNet-100 step of batch 64
+// 3580 -> 3545 us); without, N 64, P 135168 26.6 us against 25.8.
 void launch_bn_bwd_par(cb_ctx* ctx, const float* dY, const float* gamma, const float* X, float* dX, float* dgamma,
                        float* dbeta, const float* relu_out, float* dres, int dres_add, int pg_add, int N, long long P,
                        long long xs = 0, long long dxs = 0, int dx_add = 0, bool vec = true) {
     if (xs == 0) xs = P;
     if (dxs == 0) dxs = P;
-#define CB_BN(T, G, SPT)                                                                                                          \
-    launch_bn<T, G>(ctx, vec ? bn_bwd_par_kernel<T, G, SPT, true> : bn_bwd_par_kernel<T, G, SPT, false>, P, dY, gamma, X, dX, dgamma, dbeta, relu_out, dres, dres_add, pg_add, N, P, xs, \
+#define CB_BN(T, G, SPT, R)                                                                                                          \
+    launch_bn<T, G>(ctx, vec ? bn_bwd_par_kernel<T, G, SPT, R, true> : bn_bwd_par_kernel<T, G, SPT, R, false>, P, dY, gamma, X, dX, dgamma, dbeta, relu_out, dres, dres_add, pg_add, N, P, xs, \
                     dxs, dx_add)
-    if (N <= 16) CB_BN(256, 16, 1);
-    else if (N <= 32) CB_BN(256, 16, 2);
-    else if (N < 64 || (N == 64 && P >= 32768)) CB_BN(256, 16, 4);
-    else if (N == 64) CB_BN(256, 32, 2);
-    else if (N <= 128) CB_BN(256, 32, 4);
-    else CB_BN(512, 64, 4);
+    if (N <= 16) CB_BN(256, 16, 1, 1);
+    else if (N <= 32) CB_BN(256, 16, 2, 1);
+    else if (N < 64) CB_BN(256, 16, 4, 1);
+    else if (N == 64 && dx_add && P >= 32768) CB_BN(256, 16, 4, 2);
+    else if (N == 64) CB_BN(256, 32, 2, 1);
+    else if (bn_narrow(ctx, N, P) && N == 128) CB_BN(256, 64, 2, 1);
+    else if (N <= 128) CB_BN(256, 32, 4, 1);
+    else CB_BN(512, 64, 4, 1);
 #undef CB_BN
 }
 

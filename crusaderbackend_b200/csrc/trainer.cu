@@ -787,10 +787,16 @@ void drop_recorded(cbt_model* m) {
 // (their collectives are ordered call by call), calls that find a filter's packed copy stale, and passes whose recording
 // fails. A recording is keyed by everything it has baked in, scratch blocks included; at most kMostRecorded are kept.
 template <class F>
-int run_recorded(cbt_model* m, bool backward, F pass) {
+int run_recorded(cbt_model* m, bool backward, F ops) {
     constexpr size_t kMostRecorded = 8;
     constexpr int kSeenBeforeRecording = 2;
     cb_ctx* ctx = m->ctx;
+    auto pass = [&] {
+        ctx->model_pass = true;
+        const int rc = ops();
+        ctx->model_pass = false;
+        return rc;
+    };
     if (m->comm || ctx->sync || !cb::filter_cache_fresh(ctx)) return pass();
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess) {
