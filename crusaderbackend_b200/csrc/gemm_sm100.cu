@@ -514,6 +514,7 @@ TileChoice search_tile(int sm_count, const ClusterRoom& room, int smem_cap, cons
     TileChoice best{0, 16, 2, 1};
     double best_cost = 1e300;
     const int j_gran = g.q_mn ? 32 : 16;
+    const bool full = !x3 && (double)g.batch * g.I * g.J >= 1.5 * sm_count * 128 * 256;
     for (int mi = 1; mi <= 2; ++mi) {
         if (mi == 2 && g.I <= 128) continue;
         for (int bn = 256; bn >= 16; bn >>= 1) {
@@ -531,7 +532,11 @@ TileChoice search_tile(int sm_count, const ClusterRoom& room, int smem_cap, cons
             // shared-memory traffic of the split; a finished tile ~20 a column until its successor's epilogue can start.
             const double pipe = 2.1 * mi * bn_eff;
             const double own = x3 ? (stages >= 4 ? 300.0 + hi / 27.0 : (stages == 3 ? hi / 20.0 : hi / 17.0)) : 430.0 + (mi > 1 ? 150.0 : 0.0);
-            const double kb_cyc = x3 ? (3.0 * pipe > own ? 3.0 * pipe : own) : (pipe > own ? pipe : own);
+            double kb_cyc = x3 ? (3.0 * pipe > own ? 3.0 * pipe : own) : (pipe > own ? pipe : own);
+            // Over several waves every SM fetches all the time: ~53 bytes a clock each from L2, and the tall tile, which reads
+            // two thirds of the bytes a product, also draws less of the power that caps the clock. 8192^3: 128 x 256 1748 us,
+            // 256 x 256 1510, 256 x 128 1940; 4096^3: 247, 213, 279; 5000 x 2500 x 800: 43, 46, 50.
+            if (full && hi / 53.0 > kb_cyc) kb_cyc = hi / 53.0;
             for (int splits = 1; splits <= kMaxCluster; splits <<= 1) {
                 if (splits > 1 && (mi > 1 || num_kb < 2 * splits || tiles > room.of[splits])) break;
                 const double per = (double)((num_kb + splits - 1) / splits);
@@ -540,6 +545,7 @@ TileChoice search_tile(int sm_count, const ClusterRoom& room, int smem_cap, cons
                 const double waves = (double)(((long long)(tiles * splits) + sm_count - 1) / sm_count);
                 const double main = per * kb_cyc, out = 300.0 + 20.0 * mi * bn_eff;
                 double cost = waves * (main > out ? main : out) + 13.0 * mi * bn_eff;
+                if (full && mi > 1) cost += 0.5 * waves * out;  // both accumulators are the tile's: little overlaps its way out
                 if (splits > 1) cost += 4300.0 + 10.0 * bn_eff;  // two cluster barriers, the partial tiles' way through memory
                 if (cost < best_cost) {
                     best_cost = cost;
