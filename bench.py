@@ -394,8 +394,8 @@ def resnet56_3xtf32_section(torch, local):
     tr.close()
     ctx.close()
     return {"ms_per_step": round(ms, 3), "images_per_s": round(GLOBAL_BATCH / ms * 1e3, 1),
-            "note": "3xTF32: convolutions of up to 32 channels (and 64 channels on 8x8 maps) in one tensor-core pass over "
-                    "[x; x_lo; x] x [w; w; w_lo], the others as three passes"}
+            "note": "3xTF32: convolutions in one tensor-core pass over [x_lo; x; x] x [w; w_lo; w], three passes where the filter "
+                    "needs a four-way split of the output channels on a large map"}
 
 
 def densenet_section(torch, local):
