@@ -187,7 +187,7 @@ bool umma_gemm_eligible(const GemmCall& g);
 int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3);
 int launch_simt_gemm(cb_ctx* ctx, const GemmCall& g);
 // Clears the output matrices of a call whose partial products are added into them with atomics.
-int gemm_zero_output(cb_ctx* ctx, const GemmCall& g);
+int clear_output(cb_ctx* ctx, float* p, long long width, long long ld, long long rows, long long stride, long long batch, const char* who);
 
 // BatchNorm on one group of samples of a batch (statistics per group; neighbours.cu).
 int bn_fwd_group(cb_ctx* ctx, const float* X, const float* beta, const float* gamma, const float* R, float* Y, int relu, int N,

@@ -323,8 +323,8 @@ int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, 
                                              (most + simt::kBK - 1) / simt::kBK, 1, may_split);
     p.splits = c.splits; p.per_split = c.per_split; p.atomic_out = c.splits > 1 ? 1 : 0;
     if (p.atomic_out && !p.ep.accumulate) {
-        cudaError_t e = cudaMemset2DAsync(p.Out, (size_t)p.out_batch * 4, 0, (size_t)out_elems * 4, (size_t)p.N, ctx->stream);
-        if (e != cudaSuccess) return check_cuda(ctx, e, who);
+        const int rc = clear_output(ctx, p.Out, out_elems, p.out_batch, p.N, 0, 1, who);
+        if (rc != CB_OK) return rc;
     }
     bool mask = true;
     for (int i = 0; i < nsets; ++i) mask = mask && sets[i].TH <= kMaskTaps && sets[i].TW <= kMaskTaps;
@@ -400,10 +400,11 @@ int simt_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, con
     const simt::Choice c = simt::choose_tile(ctx->sm_count, I, g.OC, (pixels + simt::kBK - 1) / simt::kBK, 1, !ctx->deterministic);
     p.splits = c.splits; p.per_split = c.per_split;
     p.mode = c.splits > 1 ? 2 : (accumulate ? 1 : 0);
-    cudaError_t e = cudaSuccess;
-    if (p.mode == 2 && !accumulate) e = cudaMemsetAsync(dW, 0, (size_t)I * g.OC * sizeof(float), ctx->stream);
-    if (e != cudaSuccess) return check_cuda(ctx, e, who);
-    e = simt::with_tile(c.tile, [&](auto tile) {
+    if (p.mode == 2 && !accumulate) {
+        const int rc = clear_output(ctx, dW, I * g.OC, I * g.OC, 1, 0, 1, who);
+        if (rc != CB_OK) return rc;
+    }
+    cudaError_t e = simt::with_tile(c.tile, [&](auto tile) {
         typedef decltype(tile) T;
         auto kernel = mask ? conv_wgrad_simt<T, true> : conv_wgrad_simt<T, false>;
         cudaError_t er = raise_dynamic_smem_once(kernel, ctx->device, ctx->max_smem_optin, nullptr);

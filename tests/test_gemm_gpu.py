@@ -331,3 +331,17 @@ def test_tall_tiles_over_several_waves(torch_cuda, ctxs, M, N, K, form):
     C = torch.full((M, N), float("nan"), device="cuda")
     ctxs["tf32"].gemm(torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda(), C, transA=tA, transB=tB)
     assert orc.max_err_norm(C.cpu().numpy(), orc.gemm_f64(A, B, tA, tB)) <= TOL["tf32"]
+
+
+@pytest.mark.parametrize("pad,gap", [(0, 0), (3, 0), (0, 7), (1, 2)])
+@pytest.mark.parametrize("batch,M,N,K", [(1, 65, 67, 2051), (5, 33, 64, 1025), (3, 64, 64, 700)])
+def test_split_products_clear_their_output(torch_cuda, ctxs, batch, M, N, K, pad, gap):
+    """CUDA-core products that split the contraction: rows `pad` floats and matrices `gap` rows apart; what lies between stays."""
+    torch = torch_cuda
+    A = torch.from_numpy(orc.uniform_pm1((M, K), "clr", M, "A")).cuda()
+    B = torch.from_numpy(orc.uniform_pm1((batch, K, N), "clr", M, "B")).cuda()
+    whole = torch.full((batch, M + gap, N + pad), 7.0, device="cuda")
+    ctxs["fp32"].gemm(A, B, whole[:, :M, :N])
+    want = np.stack([orc.gemm_f64(A.cpu().numpy(), b) for b in B.cpu().numpy()])
+    assert orc.max_err_norm(whole[:, :M, :N].cpu().numpy(), want) <= TOL["fp32"]
+    assert bool((whole[:, M:, :] == 7).all()) and bool((whole[:, :, N:] == 7).all())
