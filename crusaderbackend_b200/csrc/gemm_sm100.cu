@@ -44,6 +44,7 @@ struct GemmParams {
     int mi, bn;            // P sub-tiles per CTA tile, UMMA N
     int stages;
     int num_kb, splits, kb_per_split;
+    int kgroups;           // > 1: clusters (or CTAs) that share a tile's contraction and add their sums into a cleared C
     int kb_per_fold;       // > 0: the k-blocks walk `kfold` operand pairs of kb_per_fold blocks each (their products are summed)
     int kc;                // k-blocks per accumulation chunk: the accumulator is drained to C every kc blocks
     int tmem_cols;         // allocated TMEM columns (power of two >= 2*bn)
@@ -80,13 +81,14 @@ __device__ __forceinline__ uint64_t desc_mn(uint32_t addr) {
 }
 
 struct WorkItem {
-    int b, i0, j0, kb0, kb1, split;
+    int b, i0, j0, kb0, kb1, split, kgroup;
 };
 
 __device__ __forceinline__ WorkItem decode_work(const GemmParams& p, int w) {
     WorkItem it;
-    const int tile = w / p.splits;
-    it.split = w - tile * p.splits;
+    const int part = w / p.splits, tile = part / p.kgroups;
+    it.split = w - part * p.splits;
+    it.kgroup = part - tile * p.kgroups;
     const int per_batch = p.tiles_i * p.tiles_j;
     it.b = tile / per_batch;
     int r = tile - it.b * per_batch;
@@ -99,7 +101,7 @@ __device__ __forceinline__ WorkItem decode_work(const GemmParams& p, int w) {
     const int tj = group * gw + (rg - ti * jw);
     it.i0 = ti * 128 * p.mi;
     it.j0 = tj * p.bn;
-    it.kb0 = it.split * p.kb_per_split;
+    it.kb0 = (it.kgroup * p.splits + it.split) * p.kb_per_split;
     it.kb1 = min(p.num_kb, it.kb0 + p.kb_per_split);
     return it;
 }
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(96 + 32 * kEpiWarps + (X3 ? 32 * kSplitWarps :
     const uint32_t tmem_base = ps.tmem_base;
     const uint32_t acc_stride = (uint32_t)p.tmem_cols >> 1;  // column offset of accumulator 1
 
-    const int total_work = p.batch * p.tiles_i * p.tiles_j * p.splits;
+    const int total_work = p.batch * p.tiles_i * p.tiles_j * p.kgroups * p.splits;
     uint32_t fills = 0;  // producer warps: stages filled so far
     constexpr int kQWarp = 2 + kEpiWarps + (X3 ? kSplitWarps : 0);
 
@@ -303,7 +305,7 @@ __global__ void __launch_bounds__(96 + 32 * kEpiWarps + (X3 ? 32 * kSplitWarps :
             float* Cb = p.C + (long long)it.b * p.strideC;
             const int nchunks = (it.kb1 - it.kb0 + p.kc - 1) / p.kc;
             for (int ch = 0; ch < nchunks && ok; ++ch) {
-                const bool add_bias = ch == 0;
+                const bool add_bias = ch == 0 && it.kgroup == 0;
                 const bool add_old = p.accumulate || ch > 0;      // later chunks add onto what this thread wrote
                 const bool relu_now = p.relu && ch == nchunks - 1;
                 const bool plain = p.bias_i == nullptr && p.bias_j == nullptr && !relu_now;
@@ -336,7 +338,7 @@ __global__ void __launch_bounds__(96 + 32 * kEpiWarps + (X3 ? 32 * kSplitWarps :
                         if (!i_ok) continue;
                         const int j = it.j0 + c, n = p.J - j;  // columns from here on
                         float* dst = Cb + (long long)j * p.ldc + i;
-                        if (plain && !add_old && n >= 16) {
+                        if (plain && !add_old && n >= 16 && p.kgroups == 1) {
 #pragma unroll
                             for (int e = 0; e < 16; ++e, dst += p.ldc) *dst = __uint_as_float(r[e]);
                             continue;
@@ -346,6 +348,10 @@ __global__ void __launch_bounds__(96 + 32 * kEpiWarps + (X3 ? 32 * kSplitWarps :
                             if (e >= n) break;
                             float v = __uint_as_float(r[e]) + bi;
                             if (p.bias_j != nullptr && add_bias) v += p.bias_j[j + e];
+                            if (p.kgroups > 1) {
+                                atomicAdd(dst, v);
+                                continue;
+                            }
                             if (add_old) v += *dst;
                             if (relu_now) v = fmaxf(v, 0.f);
                             *dst = v;
@@ -430,8 +436,15 @@ __global__ void __launch_bounds__(96 + 32 * kEpiWarps + (X3 ? 32 * kSplitWarps :
             for (int r = 0; r < 8; ++r)
                 if (r < p.splits) { v[0] += part[r].x; v[1] += part[r].y; v[2] += part[r].z; v[3] += part[r].w; }
             const int live = min(4, p.I - i);
-            const float bj = p.bias_j ? p.bias_j[j] : 0.f;
+            const bool with_bias = it.kgroup == 0;
+            const float bj = p.bias_j && with_bias ? p.bias_j[j] : 0.f;
             float* dst = Cb + (long long)j * p.ldc + i;
+            if (p.kgroups > 1) {
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+                    if (x < live) atomicAdd(dst + x, v[x] + bj + (p.bias_i && with_bias ? p.bias_i[i + x] : 0.f));
+                continue;
+            }
 #pragma unroll
             for (int x = 0; x < 4; ++x)
                 if (x < live) {
@@ -473,7 +486,7 @@ GemmKernel kernel_for(bool p_mn, bool q_mn) {
 }
 
 struct TileChoice {
-    int mi, bn, stages, splits;
+    int mi, bn, stages, splits, kgroups;
 };
 // How many clusters of 2 / 4 / 8 CTAs of this kernel the device holds at once. An SM holds one CTA and a cluster lies within
 // one GPC, so this is less than SMs / size; a grid beyond it runs its last clusters as a second wave (512^3 as 16 clusters
@@ -510,8 +523,8 @@ const ClusterRoom& cluster_room(const cb_ctx* ctx) {
 
 // Tile and contraction split by a model in SM clocks. Splits are the CTAs of one cluster, which add their partial tiles
 // through each other's shared memory: reproducible, no clearing launch, no atomics, any epilogue.
-TileChoice search_tile(int sm_count, const ClusterRoom& room, int smem_cap, const GemmCall& g, int num_kb, bool x3) {
-    TileChoice best{0, 16, 2, 1};
+TileChoice search_tile(int sm_count, const ClusterRoom& room, int smem_cap, const GemmCall& g, int num_kb, bool x3, bool may_add) {
+    TileChoice best{0, 16, 2, 1, 1};
     double best_cost = 1e300;
     const int j_gran = g.q_mn ? 32 : 16;
     const bool full = !x3 && (double)g.batch * g.I * g.J >= 1.5 * sm_count * 128 * 256;
@@ -549,9 +562,26 @@ TileChoice search_tile(int sm_count, const ClusterRoom& room, int smem_cap, cons
                 if (splits > 1) cost += 4300.0 + 10.0 * bn_eff;  // two cluster barriers, the partial tiles' way through memory
                 if (cost < best_cost) {
                     best_cost = cost;
-                    best = TileChoice{mi, bn_eff, stages, splits};
+                    best = TileChoice{mi, bn_eff, stages, splits, 1};
                 }
             }
+            // From about a thousand k on (a batch folded into K, mostly) several clusters on a tile, or single CTAs, which spare
+            // the cluster's barriers and the partial tile's room beside the stages, may add their sums into a cleared output.
+            // 242 x 116, 18 pairs of K 576, 3xTF32: 33.9 us in clusters alone, 12.4 now; 128 x 10, 64 pairs of K 2048: 286 and 32;
+            // 128 x 128 x 4096, TF32: 10.4 and 7.4. Shorter ones gain nothing (512^3 8.1, 8.2).
+            if (!may_add || mi > 1 || num_kb < 32) continue;
+            for (int size = 1; size <= kMaxCluster; size <<= 1)
+                for (int groups = 2; tiles * groups <= (size > 1 ? room.of[size] : sm_count); ++groups) {
+                    const int parts = groups * size, per = (num_kb + parts - 1) / parts;
+                    if ((parts - 1) * per >= num_kb) continue;  // an empty share
+                    if (size > 1 && x3 && per > kChunk3x && 2 * stage + 128 * bn_eff * 4 > smem_cap) continue;
+                    // atomic adds leave an SM at three a clock
+                    const double cost = per * kb_cyc + 5000.0 + 13.0 * bn_eff + 43.0 * bn_eff / size + (size > 1 ? 4300.0 + 10.0 * bn_eff : 0.0);
+                    if (cost < best_cost) {
+                        best_cost = cost;
+                        best = TileChoice{1, bn_eff, stages, size, groups};
+                    }
+                }
         }
     }
     return best;
@@ -576,16 +606,17 @@ int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3) {
     const int smem_cap = ctx->max_smem_optin - 2048;  // static barriers + 1 KB alignment slack
     // the search takes about a microsecond and depends on these numbers only: a thread keeps the last shapes' answers
     struct Known {
-        int I, J, batch, num_kb, q_mn, x3, sm_count, smem_cap;
+        int I, J, batch, num_kb, q_mn, x3, sm_count, smem_cap, may_add;
         TileChoice choice;
     };
     static thread_local Known table[64];
+    const bool may_add = !ctx->deterministic && !ctx->model_pass && !g.ep.relu;
     const uint32_t h = ((uint32_t)g.I * 0x9E3779B1u) ^ ((uint32_t)g.J * 0x85EBCA77u) ^ ((uint32_t)num_kb * 0xC2B2AE3Du) ^ (uint32_t)g.batch * 31u;
     Known& known = table[(h >> 20) & 63u];
     if (known.I != g.I || known.J != g.J || known.batch != g.batch || known.num_kb != num_kb || known.q_mn != g.q_mn ||
-        known.x3 != (int)x3 || known.sm_count != ctx->sm_count || known.smem_cap != smem_cap)
-        known = Known{g.I, g.J, g.batch, num_kb, g.q_mn, x3 ? 1 : 0, ctx->sm_count, smem_cap,
-                      search_tile(ctx->sm_count, cluster_room(ctx), smem_cap, g, num_kb, x3)};
+        known.x3 != (int)x3 || known.sm_count != ctx->sm_count || known.smem_cap != smem_cap || known.may_add != (int)may_add)
+        known = Known{g.I, g.J, g.batch, num_kb, g.q_mn, x3 ? 1 : 0, ctx->sm_count, smem_cap, may_add ? 1 : 0,
+                      search_tile(ctx->sm_count, cluster_room(ctx), smem_cap, g, num_kb, x3, may_add)};
     const TileChoice choice = known.choice;
     if (choice.mi == 0) return fail(ctx, CB_EUNSUPPORTED, "umma gemm: no tile configuration fits");
 
@@ -596,8 +627,9 @@ int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3) {
     gp.tiles_j = (g.J + gp.bn - 1) / gp.bn;
     gp.num_kb = num_kb;
     gp.splits = choice.splits;
-    gp.kb_per_split = (num_kb + gp.splits - 1) / gp.splits;
-    gp.splits = (num_kb + gp.kb_per_split - 1) / gp.kb_per_split;  // no empty split
+    gp.kgroups = choice.kgroups;
+    gp.kb_per_split = (num_kb + gp.splits * gp.kgroups - 1) / (gp.splits * gp.kgroups);
+    if (gp.kgroups == 1) gp.splits = (num_kb + gp.kb_per_split - 1) / gp.kb_per_split;  // no empty split
     const bool cluster = gp.splits > 1;
     // 3xTF32: the tensor core's fp32 accumulation error grows with the number of accumulated products, so the
     // accumulator is drained into C (round-to-nearest fp32 adds) every 512 k
@@ -660,7 +692,7 @@ int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3) {
         if (rc != CB_OK) return rc;
     }
 
-    const long long work = (long long)gp.batch * gp.tiles_i * gp.tiles_j * gp.splits;
+    const long long work = (long long)gp.batch * gp.tiles_i * gp.tiles_j * gp.kgroups * gp.splits;
     const int hi = gp.mi * kPTileBytes + gp.bn * kBK * 4;
     const int stage = x3 ? 2 * hi : hi;
     int tile_bytes = 0;
@@ -679,6 +711,10 @@ int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3) {
     if (smem < gp.tile_offset + (size_t)tile_bytes + 1024) smem = gp.tile_offset + (size_t)tile_bytes + 1024;
     const GemmKernel kernel = x3 ? (cluster ? kernel_for<true, true>(g.p_mn, g.q_mn) : kernel_for<true, false>(g.p_mn, g.q_mn))
                                  : (cluster ? kernel_for<false, true>(g.p_mn, g.q_mn) : kernel_for<false, false>(g.p_mn, g.q_mn));
+    if (gp.kgroups > 1 && !g.accumulate) {
+        const int rc = clear_output(ctx, g.C, g.I, g.ldc, g.J, g.strideC, g.batch, "clear of a split product");
+        if (rc != CB_OK) return rc;
+    }
     int bound = 0;
     cudaError_t e = raise_dynamic_smem_once(kernel, ctx->device, ctx->max_smem_optin, &bound);
     if (e == cudaSuccess && (int)smem > bound) e = cudaErrorInvalidValue;

@@ -301,8 +301,8 @@ def test_cuda_core_tiles_at_their_edges(torch_cuda, ctxs, M, N, K, form):
 @pytest.mark.parametrize("M,N,K", [(128, 16, 4096), (130, 20, 1028), (256, 128, 8192), (96, 260, 644), (16, 8, 2080), (300, 100, 4100), (1, 4, 576)])
 def test_contraction_split_over_a_cluster(torch_cuda, ctxs, M, N, K, math):
     """Outputs of a few tiles with a long contraction: the CTAs of a cluster add their partial tiles through each other's
-    shared memory. Tile edges in both extents, shares of several accumulation chunks (3xTF32), overwrite and accumulate,
-    and the same bits from a deterministic context and on every run."""
+    shared memory, or, on default contexts, single CTAs and clusters add theirs with atomics. Tile edges in both extents, shares
+    of several accumulation chunks (3xTF32), overwrite and accumulate, and the same bits on every run of a deterministic context."""
     torch = torch_cuda
     A, B = make_operands(M, N, K, "NT", ("cluster", M, N, K))
     ref = orc.gemm_f64(A, B, *FORMS["NT"])
@@ -312,8 +312,10 @@ def test_contraction_split_over_a_cluster(torch_cuda, ctxs, M, N, K, math):
     ctx.gemm(dA, dB, C, transB=True)
     assert ctx.last_kernel.startswith("umma")
     assert orc.max_err_norm(C.cpu().numpy(), ref) <= TOL[math]
-    first = C.clone()
     ctx.set_deterministic(True)
+    ctx.gemm(dA, dB, C, transB=True)
+    first = C.clone()
+    assert orc.max_err_norm(C.cpu().numpy(), ref) <= TOL[math]
     ctx.gemm(dA, dB, C, transB=True)
     ctx.set_deterministic(False)
     assert torch.equal(C, first)
