@@ -527,7 +527,7 @@ TileChoice search_tile(int sm_count, const ClusterRoom& room, int smem_cap, cons
     TileChoice best{0, 16, 2, 1, 1};
     double best_cost = 1e300;
     const int j_gran = g.q_mn ? 32 : 16;
-    const bool full = !x3 && (double)g.batch * g.I * g.J >= 1.5 * sm_count * 128 * 256;
+    const bool full = !x3 && (double)g.batch * g.I * g.J > (double)sm_count * 128 * 256;
     for (int mi = 1; mi <= 2; ++mi) {
         if (mi == 2 && g.I <= 128) continue;
         for (int bn = 256; bn >= 16; bn >>= 1) {
@@ -546,9 +546,10 @@ TileChoice search_tile(int sm_count, const ClusterRoom& room, int smem_cap, cons
             const double pipe = 2.1 * mi * bn_eff;
             const double own = x3 ? (stages >= 4 ? 300.0 + hi / 27.0 : (stages == 3 ? hi / 20.0 : hi / 17.0)) : 430.0 + (mi > 1 ? 150.0 : 0.0);
             double kb_cyc = x3 ? (3.0 * pipe > own ? 3.0 * pipe : own) : (pipe > own ? pipe : own);
-            // Over several waves every SM fetches all the time: ~53 bytes a clock each from L2, and the tall tile, which reads
+            // Beyond one wave (`full`) every SM fetches all the time: ~53 bytes a clock each from L2, and the tall tile, which reads
             // two thirds of the bytes a product, also draws less of the power that caps the clock. 8192^3: 128 x 256 1748 us,
-            // 256 x 256 1510, 256 x 128 1940; 4096^3: 247, 213, 279; 5000 x 2500 x 800: 43, 46, 50.
+            // 256 x 256 1510, 256 x 128 1940; 4096^3: 247, 213, 279; 5000 x 2500 x 800: 43, 46, 50;
+            // 4096 x 1200 x 1500: 55, 40.
             if (full && hi / 53.0 > kb_cyc) kb_cyc = hi / 53.0;
             for (int splits = 1; splits <= kMaxCluster; splits <<= 1) {
                 if (splits > 1 && (mi > 1 || num_kb < 2 * splits || tiles > room.of[splits])) break;
