@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "cb_internal.h"
+#include "cb_ptx.cuh"
 
 namespace {
 
@@ -100,13 +101,14 @@ struct ParamEntry {
     int d0, d1, d2, d3;
 };
 
-// Everything a recorded pass depends on besides the model's own buffers.
+// Everything a recorded pass depends on besides the model's own buffers. Of the caller's images and labels that is only where
+// they lie in a 16-byte word (floats past it): kernels are chosen by alignment, and the buffers a recording reads lie likewise.
 struct PassKey {
-    const float *images, *labels;
+    int images_at, labels_at;
     int backward, math, deterministic, bn_grad_swap, bn_groups, pdl;
     long long scratch_epoch;
     bool operator==(const PassKey& o) const {
-        return images == o.images && labels == o.labels && backward == o.backward && math == o.math && deterministic == o.deterministic &&
+        return images_at == o.images_at && labels_at == o.labels_at && backward == o.backward && math == o.math && deterministic == o.deterministic &&
                bn_grad_swap == o.bn_grad_swap && bn_groups == o.bn_groups && pdl == o.pdl && scratch_epoch == o.scratch_epoch;
     }
 };
@@ -114,11 +116,36 @@ struct RecordedPass {
     PassKey key;
     int seen = 0;                  // eager calls with this key so far
     bool unusable = false;         // recording it failed: stays eager
+    cudaGraph_t graph = nullptr;   // kept for its first node, which copies the caller's images and labels (forward passes)
     cudaGraphExec_t exec = nullptr;
+    const float *images = nullptr, *labels = nullptr;  // what that node copies now
     long long launches = 0;        // kernels of a replay on the context's stream ...
     std::vector<long long> side_launches;  // ... and on each weight-gradient stream
     unsigned long long used = 0;
 };
+
+int floats_past_16(const float* p) { return (int)((reinterpret_cast<uintptr_t>(p) & 15u) >> 2); }
+
+// dst and src lie alike in their 16-byte words, so one alignment test serves both.
+__device__ __forceinline__ void copy_alike(const float* __restrict__ src, float* __restrict__ dst, long long n) {
+    const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+    long long tail = 0;
+    if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+        for (long long i = first; i < n / 4; i += step) reinterpret_cast<float4*>(dst)[i] = reinterpret_cast<const float4*>(src)[i];
+        tail = n / 4 * 4;
+    }
+    for (long long i = tail + first; i < n; i += step) dst[i] = src[i];
+}
+// First kernel of a recorded forward pass: what the caller passes in is the one thing that differs from step to step. The copy is
+// bound by its launch: a ResNet-8 step of batch 16 / 128 takes 1.7 / 0.5 us more with it; without, a loop over new tensors ran
+// eagerly (166 against 153 us of GPU time at batch 16, 166 against 11 us of host time).
+__global__ void __launch_bounds__(256) stage_inputs_kernel(const float* images, float* own_images, long long n_images,
+                                                           const float* labels, float* own_labels, long long n_labels) {
+    cb::griddep_wait();
+    cb::griddep_launch();
+    copy_alike(images, own_images, n_images);
+    copy_alike(labels, own_labels, n_labels);
+}
 
 }  // namespace
 
@@ -134,7 +161,10 @@ struct cbt_model {
     float* M = nullptr;
     float* scratch = nullptr;      // one activation-sized temporary for accumulating data gradients
     long long scratch_elems = 0;
-    float* labels = nullptr;       // device copy of the one-hot labels of the current step (caller-owned pointer)
+    float* labels = nullptr;       // the one-hot labels of the current step (caller-owned pointer, like the input's)
+    float* own_images = nullptr;   // copies that recorded passes read; four floats longer than a batch (PassKey)
+    float* own_labels = nullptr;
+    bool input_own = false;        // they hold the batch of the last forward pass
     float* loss_dev = nullptr;     // device word: summed loss of the current step
     float* loss_n = nullptr;       // per-sample losses of the current step (fused head)
     int input = -1, logits = -1, probs = -1;
@@ -163,6 +193,7 @@ struct cbt_model {
     std::vector<RecordedPass> recorded;
     cudaStream_t record_stream = nullptr;
     unsigned long long record_clock = 0;
+    long long replays = 0;         // passes that ran as a recording
     // .crseq image of the model (ResNets): top-level operand ids, the words of the info section (uuid words flagged: a
     // file's own block numbering is accepted on load), and the parameter entries in the order the file stores them
     std::vector<uint32_t> crseq_ids, crseq_info;
@@ -397,6 +428,8 @@ int finalize_model(cbt_model* m, int x, int classes) {
     int rc = dev_alloc(m, &m->scratch, biggest);
     if (rc == CB_OK) rc = dev_alloc(m, &m->loss_dev, 4);
     if (rc == CB_OK) rc = dev_alloc(m, &m->loss_n, m->batch);
+    if (rc == CB_OK) rc = dev_alloc(m, &m->own_images, m->t[m->input].size() + 4);
+    if (rc == CB_OK) rc = dev_alloc(m, &m->own_labels, (long long)m->batch * classes + 4);
     if (rc == CB_OK) {
         const char* env = std::getenv("CBT_WGRAD_STREAMS");
         int n = env ? std::atoi(env) : 2;
@@ -587,6 +620,9 @@ int cbt_set_wgrad_streams(cbt_model* m, int n) {
     return CB_OK;
 }
 
+// Forward and backward passes that ran as a recording (run_recorded) so far.
+long long cbt_replays(const cbt_model* m) { return m ? m->replays : 0; }
+
 // Kernel launches made so far on the weight-gradient streams (the context's own counter does not see them).
 long long cbt_side_launches(const cbt_model* m) {
     long long n = 0;
@@ -772,20 +808,58 @@ int cbt_load_crseq(cbt_model* m, const char* path, unsigned* epoch) {
 
 namespace {
 
+void release(RecordedPass& r) {
+    if (r.exec) cudaGraphExecDestroy(r.exec);
+    if (r.graph) cudaGraphDestroy(r.graph);
+    r.exec = nullptr;
+    r.graph = nullptr;
+}
+
 void drop_recorded(cbt_model* m) {
     if (m->recorded.empty()) return;
     cudaStreamSynchronize(m->ctx->stream);
-    for (RecordedPass& r : m->recorded)
-        if (r.exec) cudaGraphExecDestroy(r.exec);
+    for (RecordedPass& r : m->recorded) release(r);
     m->recorded.clear();
 }
 
-// Runs `pass` (the calls of a forward or backward pass on the context's stream). A program that steps a model without a
-// graph of its own issues 30 to 300 launches a step from the host, at about 3 us each, which bounds small models and small
-// batches. So a pass that comes back with the same buffers and settings is recorded on its third call, and later calls
-// launch the recording. Eager as before: the first calls, streams that are being captured, sync mode, data-parallel models
-// (their collectives are ordered call by call), calls that find a filter's packed copy stale, and passes whose recording
-// fails. A recording is keyed by everything it has baked in, scratch blocks included; at most kMostRecorded are kept.
+// The launch of stage_inputs_kernel for one set of caller's buffers, as a stream launch and as the parameters of a graph node.
+struct StageInputs {
+    const float *images, *labels;
+    float *own_images, *own_labels;
+    long long n_images, n_labels;
+    unsigned grid;
+    StageInputs(const cbt_model* m, const float* images_, const float* labels_)
+        : images(images_), labels(labels_), own_images(m->own_images + floats_past_16(images_)),
+          own_labels(m->own_labels + floats_past_16(labels_)), n_images(m->t[m->input].size()), n_labels((long long)m->batch * m->classes) {
+        const long long blocks = (n_images / 4 + 255) / 256, most = 8LL * m->ctx->sm_count;
+        grid = (unsigned)(blocks < 1 ? 1 : (blocks > most ? most : blocks));
+    }
+    cudaError_t launch(cb_ctx* ctx) const {
+        return cb::launch_dep(ctx, stage_inputs_kernel, dim3(grid), dim3(256), 0, images, own_images, n_images, labels, own_labels, n_labels);
+    }
+    cudaError_t set(cudaGraphExec_t exec, cudaGraph_t graph) {
+        cudaGraphNode_t node = nullptr;
+        size_t n = 1;
+        cudaError_t e = cudaGraphGetRootNodes(graph, &node, &n);
+        if (e != cudaSuccess) return e;
+        void* args[] = {&images, &own_images, &n_images, &labels, &own_labels, &n_labels};
+        cudaKernelNodeParams kp{};
+        kp.func = reinterpret_cast<void*>(stage_inputs_kernel);
+        kp.gridDim = dim3(grid);
+        kp.blockDim = dim3(256);
+        kp.kernelParams = args;
+        return cudaGraphExecKernelNodeSetParams(exec, node, &kp);
+    }
+};
+
+// Runs `ops` (the calls of a forward or backward pass on the context's stream). A program that steps a model without a graph
+// of its own issues 30 to 300 launches a step from the host, at about 3 us each, which bounds small models and small batches.
+// So a pass that comes back with the same settings is recorded on its third call, and later calls launch the recording.
+// The caller's images and labels may be other buffers every time: a recorded forward pass begins with a copy of them into the
+// model's own (its node is given the new addresses before a launch), and the passes read those. Eager, and reading the caller's
+// buffers: the first calls, streams that are being captured, sync mode, data-parallel models (their collectives are ordered call
+// by call), calls that find a filter's packed copy stale, passes whose recording fails, and a backward pass whose forward pass
+// was eager. A recording is keyed by everything it has baked in, scratch blocks included; at most kMostRecorded are kept.
 template <class F>
 int run_recorded(cbt_model* m, bool backward, F ops) {
     constexpr size_t kMostRecorded = 8;
@@ -804,8 +878,9 @@ int run_recorded(cbt_model* m, bool backward, F ops) {
         return pass();
     }
     if (cap != cudaStreamCaptureStatusNone) return pass();
-    PassKey key{m->t[m->input].a, m->labels, backward ? 1 : 0, ctx->math, ctx->deterministic, m->bn_grad_swap, m->bn_groups, ctx->pdl,
-                ctx->scratch_epoch};
+    float*& input = m->t[m->input].a;
+    PassKey key{floats_past_16(input), floats_past_16(m->labels), backward ? 1 : 0, ctx->math, ctx->deterministic, m->bn_grad_swap,
+                m->bn_groups, ctx->pdl, ctx->scratch_epoch};
     for (const cb_ctx* c : m->side) key.scratch_epoch += c->scratch_epoch;  // only ever grow: the sum changes with any of them
     RecordedPass* r = nullptr;
     for (RecordedPass& e : m->recorded)
@@ -815,10 +890,8 @@ int run_recorded(cbt_model* m, bool backward, F ops) {
             size_t oldest = 0;
             for (size_t i = 1; i < m->recorded.size(); ++i)
                 if (m->recorded[i].used < m->recorded[oldest].used) oldest = i;
-            if (m->recorded[oldest].exec) {
-                cudaStreamSynchronize(ctx->stream);
-                cudaGraphExecDestroy(m->recorded[oldest].exec);
-            }
+            if (m->recorded[oldest].exec) cudaStreamSynchronize(ctx->stream);
+            release(m->recorded[oldest]);
             m->recorded.erase(m->recorded.begin() + (long)oldest);
         }
         m->recorded.push_back(RecordedPass{});
@@ -826,47 +899,66 @@ int run_recorded(cbt_model* m, bool backward, F ops) {
         r->key = key;
     }
     r->used = ++m->record_clock;
+    if (r->seen < kSeenBeforeRecording || r->unusable || (backward && !m->input_own)) {
+        ++r->seen;
+        return pass();
+    }
+    const float *images = input, *labels = m->labels;
+    StageInputs stage(m, images, labels);
     if (!r->exec) {
-        if (r->unusable || r->seen < kSeenBeforeRecording) {
-            ++r->seen;
-            return pass();
-        }
         r->unusable = true;  // until the recording is complete
         if (!m->record_stream && cudaStreamCreateWithFlags(&m->record_stream, cudaStreamNonBlocking) != cudaSuccess) return pass();
         const long long l0 = ctx->launches;
         std::vector<long long> s0;
         for (const cb_ctx* c : m->side) s0.push_back(c->launches);
-        cudaGraph_t graph = nullptr;
-        cudaGraphExec_t exec = nullptr;
         cudaStream_t callers = ctx->stream;
         if (cudaStreamBeginCapture(m->record_stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             cudaGetLastError();
             return pass();
         }
         ctx->stream = m->record_stream;
+        cudaError_t e = backward ? cudaSuccess : stage.launch(ctx);
+        input = stage.own_images;
+        m->labels = stage.own_labels;
         const int rc = pass();
+        input = const_cast<float*>(images);
+        m->labels = const_cast<float*>(labels);
         ctx->stream = callers;
-        cudaError_t e = cudaStreamEndCapture(m->record_stream, &graph);
-        if (rc == CB_OK && e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-        if (graph) cudaGraphDestroy(graph);
+        const cudaError_t end = cudaStreamEndCapture(m->record_stream, &r->graph);
+        if (e == cudaSuccess) e = end;
+        if (rc == CB_OK && e == cudaSuccess) e = cudaGraphInstantiate(&r->exec, r->graph, 0);
+        size_t roots = 0;
+        if (rc == CB_OK && e == cudaSuccess && !backward) e = cudaGraphGetRootNodes(r->graph, nullptr, &roots);
+        r->images = images;
+        r->labels = labels;
         r->launches = ctx->launches - l0;
         r->side_launches.clear();
         for (size_t i = 0; i < m->side.size(); ++i) r->side_launches.push_back(m->side[i]->launches - s0[i]);
         // nothing of the recording has run yet
         ctx->launches = l0;
         for (size_t i = 0; i < m->side.size(); ++i) m->side[i]->launches = s0[i];
-        if (rc != CB_OK || e != cudaSuccess || !exec) {
+        if (rc != CB_OK || e != cudaSuccess || !r->exec || (!backward && roots != 1)) {
             cudaGetLastError();
+            release(*r);
             m->err.clear();
             return pass();
         }
-        r->exec = exec;
         r->unusable = false;
+    }
+    if (!backward && (r->images != images || r->labels != labels)) {
+        if (stage.set(r->exec, r->graph) != cudaSuccess) {
+            cudaGetLastError();
+            return pass();
+        }
+        r->images = images;
+        r->labels = labels;
     }
     cudaError_t e = cudaGraphLaunch(r->exec, ctx->stream);
     if (e != cudaSuccess) { m->err = cudaGetErrorString(e); return CB_ECUDA; }
+    if (!backward) m->input_own = true;
     ctx->launches += r->launches;
     for (size_t i = 0; i < m->side.size(); ++i) m->side[i]->launches += r->side_launches[i];
+    ++m->replays;
     return CB_OK;
 }
 
@@ -875,17 +967,19 @@ int run_recorded(cbt_model* m, bool backward, F ops) {
 extern "C" {
 
 // Forward pass on `images` (batch x 3 x H x W, device) with one-hot `labels` (batch x classes, device). The images are
-// read in place (no copy): they must stay unchanged until cbt_backward has run. Leaves the softmax in the last tensor
+// read in place unless the pass runs as a recording: they must stay unchanged until cbt_backward has run. Leaves the softmax in the last tensor
 // and the summed loss in the model's device loss word (after cbt_backward for models with the fused head).
-static int forward_ops(cbt_model* m, const float* labels);
+static int forward_ops(cbt_model* m);
 int cbt_forward(cbt_model* m, const float* images, const float* labels) {
     if (!m || !m->P || !images || !labels) return CB_EINVAL;
     m->t[m->input].a = const_cast<float*>(images);
     m->labels = const_cast<float*>(labels);
-    return run_recorded(m, false, [&] { return forward_ops(m, labels); });
+    m->input_own = false;
+    return run_recorded(m, false, [&] { return forward_ops(m); });
 }
-static int forward_ops(cbt_model* m, const float* labels) {
+static int forward_ops(cbt_model* m) {
     cb_ctx* ctx = m->ctx;
+    const float* labels = m->labels;
     cudaError_t e;
     for (const Op& o : m->ops) {
         const TensorBuf& x = m->t[o.in0];

@@ -40,6 +40,7 @@ TRAIN_SIGNATURES = {
     "cbt_dp_world": (_i, [C.c_void_p]),
     "cbt_set_wgrad_streams": (_i, [C.c_void_p, _i]),
     "cbt_side_launches": (_ll, [C.c_void_p]),
+    "cbt_replays": (_ll, [C.c_void_p]),
     "cbt_save_crseq": (_i, [C.c_void_p, C.c_char_p, C.c_uint]),
     "cbt_load_crseq": (_i, [C.c_void_p, C.c_char_p, C.POINTER(C.c_uint)]),
 }
@@ -182,6 +183,11 @@ class ResNetTrainer:
     def launches(self) -> int:
         """Kernel launches so far: the context's stream plus the weight-gradient streams."""
         return int(self.ctx.launches) + int(self.lib.cbt_side_launches(self.h))
+
+    @property
+    def replays(self) -> int:
+        """Forward and backward passes so far that ran as a recording of the executor's own."""
+        return int(self.lib.cbt_replays(self.h))
 
     def set_bn_groups(self, groups: int):
         """BatchNorm statistics per group of batch/groups consecutive samples (what `groups` data-parallel ranks compute)."""

@@ -48,6 +48,10 @@ int cbt_params_changed(cbt_model* m);
 int cbt_forward(cbt_model* m, const float* images, const float* labels_onehot);
 int cbt_backward(cbt_model* m);
 int cbt_update(cbt_model* m, float lr, float beta, float l2);
+/* A pass that comes back with the same settings is recorded as a CUDA graph on its third call and replayed from then on,
+ * whatever buffers the images and labels of a call are in (a replayed forward pass first copies them, a launch that
+ * cb_launch_count leaves out). Not in sync mode, on a stream that is being captured, or data-parallel. Replays so far: */
+long long cbt_replays(const cbt_model* m);
 
 /* The convolution weight gradients of cbt_backward run on `n` CUDA streams of the executor's own (0..4; 0: on the
  * context's stream). Only the update needs them, so they fill the SMs that the chain of data-gradient and BatchNorm

@@ -332,3 +332,63 @@ def test_recorded_passes_match_eager_ones(streams):
     (la, pa, ma, na), (lb, pb, mb, nb) = results
     assert la == lb and torch.equal(pa, pb) and torch.equal(ma, mb)
     assert na == nb
+
+
+def train_on_new_tensors(torch, cls, sync, math="tf32", classes=10, steps=9, shift=0, eager_forwards=(), **shape):
+    """Steps on other tensors every time, spoilt once the step is queued. shift: floats by which they start past 16 bytes;
+    eager_forwards: steps whose forward pass runs in sync mode, which never records, and whose backward pass does not."""
+    from crusaderbackend_b200.api import Context
+    ctx = Context(0, math=math, sync=sync)
+    ctx.set_deterministic(True)
+    tr = cls(ctx, batch=8, image_hw=16, classes=classes, **shape)
+    tr.init_params("new tensors")
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    kept, losses, l0 = [], [], tr.launches
+    for i in range(steps):
+        images = torch.empty(8 * 3 * 16 * 16 + 4, device="cuda")[shift:shift + 8 * 3 * 16 * 16].view(8, 3, 16, 16)
+        labels = torch.empty(8 * classes + 4, device="cuda")[shift:shift + 8 * classes].view(8, classes)
+        images.copy_(torch.randn(images.shape, generator=gen, device="cuda"))
+        labels.copy_(torch.eye(classes, device="cuda")[torch.randint(0, classes, (8,), generator=gen, device="cuda")])
+        kept += [images, labels]     # no address comes back
+        if i in eager_forwards:
+            ctx.set_sync(True)
+        tr.forward(images, labels)
+        ctx.set_sync(sync)
+        tr.backward()
+        tr.update(1e-3)
+        losses.append(tr.loss_tensor())
+        images.fill_(float("nan"))
+        labels.fill_(float("nan"))
+    out = [float(x) for x in losses], tr.params.clone(), tr.momentum.clone(), tr.launches - l0
+    replays = tr.replays
+    tr.close()
+    ctx.close()
+    return out, replays
+
+
+def assert_same_run(torch, eager, recorded):
+    (la, pa, ma, na), (lb, pb, mb, nb) = eager, recorded
+    assert la == lb and torch.equal(pa, pb) and torch.equal(ma, mb) and na == nb
+
+
+@pytest.mark.parametrize("model", ["resnet", "densenet"])
+@pytest.mark.parametrize("shift", [0, 1, 2])
+def test_recordings_serve_new_input_tensors(torch_cuda, model, shift):
+    """A loop that yields new images and labels every step replays its passes from the third step on, with the bits of a
+    context that never records, also where the tensors do not start on 16 bytes."""
+    from crusaderbackend_b200.train import DenseNetTrainer, ResNetTrainer
+    cls, shape = (ResNetTrainer, dict(blocks_per_stage=1)) if model == "resnet" else (DenseNetTrainer, dict(growth=4, layers=2))
+    eager, none = train_on_new_tensors(torch_cuda, cls, True, shift=shift, **shape)
+    recorded, replays = train_on_new_tensors(torch_cuda, cls, False, shift=shift, **shape)
+    assert none == 0 and replays >= 2 * 6
+    assert_same_run(torch_cuda, eager, recorded)
+
+
+def test_backward_after_an_eager_forward_reads_its_images(torch_cuda):
+    """The backward pass after an eager forward pass reads the caller's images, not the batch of an earlier replay, although
+    it has a recording of its own."""
+    from crusaderbackend_b200.train import ResNetTrainer
+    eager, _ = train_on_new_tensors(torch_cuda, ResNetTrainer, True, blocks_per_stage=1)
+    recorded, replays = train_on_new_tensors(torch_cuda, ResNetTrainer, False, eager_forwards=(5, 6), blocks_per_stage=1)
+    assert replays >= 2 * 4
+    assert_same_run(torch_cuda, eager, recorded)
