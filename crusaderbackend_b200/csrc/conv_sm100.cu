@@ -1098,7 +1098,8 @@ static int packed_filter(cb_ctx* ctx, const ConvEnv& env, const ConvPlan& q, con
 
 bool filter_cache_fresh(const cb_ctx* ctx) {
     const FilterCache* fc = static_cast<const FilterCache*>(ctx->filter_cache);
-    if (!ctx->filter_cache_on || !fc) return false;
+    if (!ctx->filter_cache_on) return false;
+    if (!fc) return true;  // nothing was ever packed: fp32 mode, or no map the tensor cores take
     for (const FilterCacheEntry& e : fc->entries)
         if (e.version != ctx->filter_version) return false;
     return true;

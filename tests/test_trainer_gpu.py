@@ -334,18 +334,19 @@ def test_recorded_passes_match_eager_ones(streams):
     assert na == nb
 
 
-def train_on_new_tensors(torch, cls, sync, math="tf32", classes=10, steps=9, shift=0, eager_forwards=(), **shape):
+def train_on_new_tensors(torch, cls, sync, math="tf32", classes=10, hw=16, steps=9, shift=0, eager_forwards=(),
+                         **shape):
     """Steps on other tensors every time, spoilt once the step is queued. shift: floats by which they start past 16 bytes;
     eager_forwards: steps whose forward pass runs in sync mode, which never records, and whose backward pass does not."""
     from crusaderbackend_b200.api import Context
     ctx = Context(0, math=math, sync=sync)
     ctx.set_deterministic(True)
-    tr = cls(ctx, batch=8, image_hw=16, classes=classes, **shape)
+    tr = cls(ctx, batch=8, image_hw=hw, classes=classes, **shape)
     tr.init_params("new tensors")
     gen = torch.Generator(device="cuda").manual_seed(11)
     kept, losses, l0 = [], [], tr.launches
     for i in range(steps):
-        images = torch.empty(8 * 3 * 16 * 16 + 4, device="cuda")[shift:shift + 8 * 3 * 16 * 16].view(8, 3, 16, 16)
+        images = torch.empty(8 * 3 * hw * hw + 4, device="cuda")[shift:shift + 8 * 3 * hw * hw].view(8, 3, hw, hw)
         labels = torch.empty(8 * classes + 4, device="cuda")[shift:shift + 8 * classes].view(8, classes)
         images.copy_(torch.randn(images.shape, generator=gen, device="cuda"))
         labels.copy_(torch.eye(classes, device="cuda")[torch.randint(0, classes, (8,), generator=gen, device="cuda")])
@@ -391,4 +392,15 @@ def test_backward_after_an_eager_forward_reads_its_images(torch_cuda):
     eager, _ = train_on_new_tensors(torch_cuda, ResNetTrainer, True, blocks_per_stage=1)
     recorded, replays = train_on_new_tensors(torch_cuda, ResNetTrainer, False, eager_forwards=(5, 6), blocks_per_stage=1)
     assert replays >= 2 * 4
+    assert_same_run(torch_cuda, eager, recorded)
+
+
+@pytest.mark.parametrize("math,hw,classes", [("fp32", 16, 10), ("fp32", 16, 40), ("tf32", 12, 10)])
+def test_models_on_the_cuda_cores_are_recorded(torch_cuda, math, hw, classes):
+    """fp32 mode and maps the tensor cores do not take have no packed filters that could be stale: their passes replay too."""
+    from crusaderbackend_b200.train import ResNetTrainer
+    args = dict(math=math, hw=hw, classes=classes, blocks_per_stage=1)
+    eager, _ = train_on_new_tensors(torch_cuda, ResNetTrainer, True, **args)
+    recorded, replays = train_on_new_tensors(torch_cuda, ResNetTrainer, False, **args)
+    assert replays >= 2 * 6
     assert_same_run(torch_cuda, eager, recorded)
