@@ -94,3 +94,25 @@ def test_tensor_maps_are_encoded_once_per_tensor_and_tiling():
     _, m3 = read()
     assert m3 == m2 + 1 and torch.equal(C1, C2)
     ctx.close()
+
+
+@pytest.mark.parametrize("ic,oc,stride,math", [(32, 64, 2, "3xtf32"), (32, 64, 1, "3xtf32"), (16, 16, 2, "3xtf32"), (32, 64, 2, "tf32")])
+def test_scratch_of_one_pass_serves_the_layers_other_passes(ic, oc, stride, math):
+    """The scratch a context allocates for a layer's forward pass and data gradient is enough for its weight gradient, and
+    that of a forward pass for a data gradient over twice the channels: a frozen context runs them."""
+    import torch
+    from crusaderbackend_b200.api import Context
+    ctx = Context(0, math=math, sync=True)
+    o = 32 // stride
+    W, X = torch.randn(oc, ic, 3, 3, device="cuda"), torch.randn(4, ic, 32, 32, device="cuda")
+    dY, dX, dW = torch.randn(4, oc, o, o, device="cuda"), torch.empty_like(X), torch.zeros_like(W)
+    g = (stride, stride, 1, 1)
+    ctx.conv(W, X, torch.empty_like(dY), *g)
+    if stride == 2:
+        ctx.convDerive(W, dY, dX, *g)
+    assert ctx.lib.cb_freeze_workspace(ctx.h, 1) == 0
+    ctx.convDerive(W, dY, dX, *g)
+    ctx.convError(dY, X, dW, *g)
+    ref = torch.nn.grad.conv2d_weight(X.double(), W.shape, dY.double(), stride=stride, padding=1)
+    assert (dW - ref).abs().max() <= (1e-5 if math == "3xtf32" else 2e-3) * ref.abs().max()
+    ctx.close()
