@@ -307,7 +307,8 @@ int launch_simt_gemm(cb_ctx* ctx, const GemmCall& g_in) {
         g.out_mode ^= 1;
     }
     const int fold = g.kfold > 1 ? g.kfold : 1;
-    const bool may_split = !ctx->deterministic && g.ep.relu == 0;
+    // no atomic sums in a model's passes: one rounding in an activation moves the gradients of a deep model by percents
+    const bool may_split = !ctx->deterministic && !ctx->model_pass && g.ep.relu == 0;
     SimtParams sp{};
     sp.I = g.I; sp.J = g.J; sp.K = g.K; sp.batch = g.batch;
     sp.P = g.P; sp.ldp = g.ldp; sp.strideP = g.strideP; sp.p_mn = g.p_mn;

@@ -404,3 +404,25 @@ def test_models_on_the_cuda_cores_are_recorded(torch_cuda, math, hw, classes):
     recorded, replays = train_on_new_tensors(torch_cuda, ResNetTrainer, False, **args)
     assert replays >= 2 * 6
     assert_same_run(torch_cuda, eager, recorded)
+
+
+def test_dense_layer_of_a_model_sums_in_one_order(torch_cuda):
+    """More than 32 classes on 300 features: the forward product would be split over atomic adds if it were a call of its own.
+    In a model it takes the launches, and gives the bits, of a deterministic context."""
+    torch = torch_cuda
+    from crusaderbackend_b200.api import Context
+    from crusaderbackend_b200.train import DenseNetTrainer
+    _, _, dimg, _ = make_batch(torch, 8, 8, 40, "dense order")
+    dlab = torch.eye(40, device="cuda")[:8].contiguous()
+    results = []
+    for deterministic in (True, False):
+        ctx = Context(0, math="fp32", sync=True)
+        ctx.set_deterministic(deterministic)
+        tr = DenseNetTrainer(ctx, batch=8, growth=40, layers=4, image_hw=8, classes=40)
+        tr.init_params("dense order")
+        l0 = tr.launches
+        tr.forward(dimg, dlab)
+        results.append((tr.launches - l0, tr.tensor(-1, (8, 40)).clone()))
+        tr.close()
+        ctx.close()
+    assert results[0][0] == results[1][0] and torch.equal(results[0][1], results[1][1])
