@@ -263,7 +263,8 @@ __global__ void __launch_bounds__(256) clear_kernel(float* __restrict__ p, const
 }  // namespace
 
 // Clears the output of a product whose contraction is split over atomic adds. One launch that chains to the kernels around it: a
-// cudaMemset2DAsync per matrix of a batch took longer than the product (8 x 129 x 131 x 133: 24.7 us).
+// cudaMemset2DAsync per matrix of a batch took longer than the product (8 x 129 x 131 x 133: 24.7 us). Split outputs are small, so
+// 32-bit indexes do: at most 32 tiles of 128 x 128 an SM on the CUDA cores, half a tile of 128 x 256 an SM on the tensor cores.
 int clear_output(cb_ctx* ctx, float* p, long long width, long long ld, long long rows, long long stride, long long batch, const char* who) {
     if (ld == width) {
         width *= rows;
@@ -275,12 +276,6 @@ int clear_output(cb_ctx* ctx, float* p, long long width, long long ld, long long
         batch = 1;
     }
     const long long n = width * rows * batch;
-    if (n >= (1LL << 31) || width >= (1LL << 31)) {
-        cudaError_t e = cudaSuccess;
-        for (long long b = 0; b < batch && e == cudaSuccess; ++b)
-            e = cudaMemset2DAsync(p + b * stride, (size_t)ld * 4, 0, (size_t)width * 4, (size_t)rows, ctx->stream);
-        return e == cudaSuccess ? CB_OK : check_cuda(ctx, e, who);
-    }
     const bool vec = rows * batch == 1 && (n & 3) == 0 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0;
     const uint32_t items = (uint32_t)(vec ? n / 4 : n);
     long long grid = ((long long)items + 1023) / 1024;
