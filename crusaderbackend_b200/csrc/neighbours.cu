@@ -447,8 +447,12 @@ void launch_bn(cb_ctx* ctx, void (*kernel)(KArgs...), long long P, Args... args)
     launch_dep(ctx, kernel, dim3((unsigned)(((P + 3) / 4 + pb - 1) / pb)), dim3((unsigned)pb, (unsigned)G), 0, args...);
 }
 
-// Batch groups: 16 below a batch of 64, 32 from there, 64 for maps too narrow to give every SM a block of 32. From a batch of 64
-// on and for wide layers, which are bound by DRAM, sixteen rows of threads (256 contiguous bytes of a sample) hold the 32 groups.
+// Two rules. How many batch groups a sum has, which decides its bits, depends on the batch (and on narrowness) alone: 16 below a
+// batch of 64, 32 from there, 64 for maps too narrow to give every SM a block of 32. These are the groups these kernels have always
+// had: a step through fifty BatchNorms with other groups gives gradients that differ by 2 % (ResNet-56) to 10 % (DenseNet-100) in
+// its very first update, and a training run could not be compared with one of an earlier version (16 groups at a batch of 64 would
+// save 5 % of the DenseNet-100 step). How many rows of threads share the groups is free, and chosen by speed: sixteen
+// (256 contiguous bytes of a sample) where a thread then holds few enough samples and the layer is wide enough to be bound by DRAM.
 // Measured, us, forward, 16 against 32 rows: N 64, P 135168 12.3 / 14.8, 49152 5.8 / 6.3, 21888 4.1 / 3.5; 80, 128000 15.8 / 19.7;
 // 128, 131072 24.4 / 31.4; 173, 111616 38.2 / 34.4. 512 threads in 32 rows: N 64, P 135168 18.0.
 inline bool bn_narrow(const cb_ctx* ctx, int N, long long P) { return N >= 128 && (P / 4 + 7) / 8 < ctx->sm_count; }
@@ -461,9 +465,9 @@ void launch_bn_fwd_par(cb_ctx* ctx, const float* X, const float* beta, const flo
     if (N <= 16) CB_BN(256, 16, 1, 1);
     else if (N <= 32) CB_BN(256, 16, 2, 1);
     else if (N < 64) CB_BN(256, 16, 4, 1);
-    else if (N == 64 && P >= 32768) CB_BN(256, 16, 4, 2);
-    else if (N == 64) CB_BN(256, 32, 2, 1);
-    else if (bn_narrow(ctx, N, P) && N == 128) CB_BN(256, 64, 2, 1);
+    else if (N <= 64 && P >= 32768) CB_BN(256, 16, 4, 2);
+    else if (N <= 64) CB_BN(256, 32, 2, 1);
+    else if (bn_narrow(ctx, N, P) && N <= 128) CB_BN(256, 64, 2, 1);
     else if (bn_narrow(ctx, N, P)) CB_BN(256, 64, 4, 1);
     else if (N <= 128 && P >= 65536) CB_BN(256, 16, 8, 2);
     else if (N <= 128) CB_BN(256, 32, 4, 1);
@@ -472,8 +476,10 @@ void launch_bn_fwd_par(cb_ctx* ctx, const float* X, const float* beta, const flo
 }
 // The backward kernel holds two tensors' samples: never more than four a thread (eight cost half its occupancy: N 128,
 // P 131072 with sixteen rows 70 us against 47; N 173, P 111616: 512 threads in 64 rows 69 us against 95 with eight samples in 32).
-// Thirty-two groups in sixteen rows pay only where dX is added to, one more tensor through DRAM (a DenseNet-100 step of batch 64
-// 3580 -> 3545 us); without, N 64, P 135168 26.6 us against 25.8.
+// Four samples a thread in sixteen rows end at a batch of 64, where thirty-two groups begin, so that form serves this one batch:
+// only where dX is added to, one more tensor through DRAM. A DenseNet-100 step of batch 64 takes 3557 us with it, 3575 with 32 rows
+// of 8 vectors, 3632 with 512 threads in 32 rows of 16 (batch 96: 4654 and 4689, so from 65 on rows stay at 128 bytes). Dense tensors
+// behind a flushed L2, 16 against 32 rows: P 49152 25.5 / 22.6, 135168 49.2 / 47.1, 270336 81.9 / 84.0; without dX += 26.6 / 25.8.
 void launch_bn_bwd_par(cb_ctx* ctx, const float* dY, const float* gamma, const float* X, float* dX, float* dgamma,
                        float* dbeta, const float* relu_out, float* dres, int dres_add, int pg_add, int N, long long P,
                        long long xs = 0, long long dxs = 0, int dx_add = 0, bool vec = true) {
@@ -485,9 +491,9 @@ void launch_bn_bwd_par(cb_ctx* ctx, const float* dY, const float* gamma, const f
     if (N <= 16) CB_BN(256, 16, 1, 1);
     else if (N <= 32) CB_BN(256, 16, 2, 1);
     else if (N < 64) CB_BN(256, 16, 4, 1);
-    else if (N == 64 && dx_add && P >= 32768) CB_BN(256, 16, 4, 2);
-    else if (N == 64) CB_BN(256, 32, 2, 1);
-    else if (bn_narrow(ctx, N, P) && N == 128) CB_BN(256, 64, 2, 1);
+    else if (N <= 64 && dx_add && P >= 32768) CB_BN(256, 16, 4, 2);
+    else if (N <= 64) CB_BN(256, 32, 2, 1);
+    else if (bn_narrow(ctx, N, P) && N <= 128) CB_BN(256, 64, 2, 1);
     else if (N <= 128) CB_BN(256, 32, 4, 1);
     else CB_BN(512, 64, 4, 1);
 #undef CB_BN

@@ -128,6 +128,26 @@ def test_batchnorm_block_shapes(torch_cuda, ctxs, shape):
     test_batchnorm(torch_cuda, ctxs, shape)
 
 
+@pytest.mark.parametrize("N,P", [(63, 32768), (64, 32764), (64, 32768), (64, 33280), (65, 32768), (128, 65536), (129, 32768)])
+def test_batchnorm_sums_do_not_depend_on_the_block_shape(torch_cuda, ctxs, N, P):
+    """Adding onto dX picks other rows of threads for some batches and widths, not other batch groups: the same bits as the form
+    that assigns, plus one rounded addition."""
+    torch = torch_cuda
+    ctx = ctxs["fp32"]
+    gen = torch.Generator(device="cuda").manual_seed(N * 7 + P)
+    dY, X, dX0 = (torch.randn(N, P, generator=gen, device="cuda") for _ in range(3))
+    g = torch.randn(P, generator=gen, device="cuda")
+    p = lambda t: t.data_ptr()  # noqa: E731
+    out = []
+    for accumulate, dX in ((0, torch.full_like(X, float("nan"))), (1, dX0.clone())):
+        dg, db = torch.empty_like(g), torch.empty_like(g)
+        ctx._check(ctx.lib.cb_bn_bwd_fused_ex(ctx.h, p(dY), p(g), p(X), p(dX), p(dg), p(db), 0, N, P, 0, 0, accumulate))
+        out.append((dX, dg, db))
+    ctx.synchronize()
+    (a, ga, ba), (b, gb, bb) = out
+    assert torch.equal(ga, gb) and torch.equal(ba, bb) and torch.equal(dX0 + a, b)
+
+
 
 def test_golden_batchnorm(torch_cuda, ctxs, golden):
     from tests.golden.make_golden import CASES, inputs
