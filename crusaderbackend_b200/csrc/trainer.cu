@@ -1002,6 +1002,10 @@ static int forward_ops(cbt_model* m) {
                     // statistics per group of consecutive samples: what each GPU of a data-parallel run computes on its shard
                     const long long P = (long long)x.c * x.h * x.w;
                     const int ng = x.n / m->bn_groups;
+                    if (x.bstride) {
+                        m->err = "BatchNorm groups are not combined with views";
+                        return CB_EUNSUPPORTED;
+                    }
                     if (o.xhat >= 0 || x.n % m->bn_groups) {
                         m->err = "BatchNorm groups need the fused kernels (N <= 256, C*H*W % 4 == 0) and a batch divisible by the group count";
                         return CB_EUNSUPPORTED;

@@ -426,3 +426,22 @@ def test_dense_layer_of_a_model_sums_in_one_order(torch_cuda):
         tr.close()
         ctx.close()
     assert results[0][0] == results[1][0] and torch.equal(results[0][1], results[1][1])
+
+
+def test_batchnorm_groups_refuse_views(torch_cuda):
+    """A dense block's BatchNorm reads a channel prefix of a wider tensor, whose samples are not P apart: groups of samples are
+    refused by the forward pass as by the backward pass."""
+    torch = torch_cuda
+    from crusaderbackend_b200.api import Context, CrusaderError
+    from crusaderbackend_b200.train import DenseNetTrainer
+    _, _, dimg, dlab = make_batch(torch, 8, 16, 10, "groups")
+    ctx = Context(0, math="fp32", sync=True)
+    tr = DenseNetTrainer(ctx, batch=8, growth=4, layers=2, image_hw=16, classes=10)
+    tr.init_params("groups")
+    tr.set_bn_groups(2)
+    with pytest.raises(CrusaderError, match="views"):
+        tr.forward(dimg, dlab)
+    tr.set_bn_groups(1)
+    tr.forward(dimg, dlab)
+    tr.close()
+    ctx.close()
