@@ -445,3 +445,67 @@ def test_batchnorm_groups_refuse_views(torch_cuda):
     tr.forward(dimg, dlab)
     tr.close()
     ctx.close()
+
+
+def test_recordings_beyond_the_most_that_are_kept(torch_cuda):
+    """Six settings make twelve recordings where eight are kept: over two rounds every setting's passes are recorded, evicted and
+    recorded again, with the bits and launches of a context that never records."""
+    torch = torch_cuda
+    from crusaderbackend_b200.api import Context
+    from crusaderbackend_b200.train import ResNetTrainer
+    _, _, dimg, dlab = make_batch(torch, 8, 16, 10, "evicted")
+    results = []
+    for sync in (True, False):
+        ctx = Context(0, math="tf32", sync=sync)
+        ctx.set_deterministic(True)
+        tr = ResNetTrainer(ctx, batch=8, blocks_per_stage=1, image_hw=16)
+        tr.init_params("evicted")
+        l0, per_setting = tr.launches, []
+        for _ in range(2):
+            for math in ("tf32", "3xtf32"):
+                ctx.set_math(math)
+                for groups in (1, 2, 4):
+                    tr.set_bn_groups(groups)
+                    before = tr.replays
+                    for _ in range(6):   # at most: stale filters, larger scratch, twice eager, then replays
+                        tr.step(dimg, dlab, lr=1e-4)
+                    per_setting.append(tr.replays - before)
+        results.append((tr.params.clone(), tr.momentum.clone(), tr.launches - l0, per_setting))
+        tr.close()
+        ctx.close()
+    (pa, ma, na, ra), (pb, mb, nb, rb) = results
+    assert torch.equal(pa, pb) and torch.equal(ma, mb) and na == nb
+    assert not any(ra) and min(rb) >= 2
+    assert rb[6:] == [8] * 6   # second round: everything was evicted, so two eager steps come first again
+
+
+def test_pass_that_cannot_be_recorded(torch_cuda):
+    """A forward pass that fails, and with it its recording, reports its error every time; the model works when its setting is
+    put right, and its other recordings are untouched."""
+    torch = torch_cuda
+    from crusaderbackend_b200.api import Context, CrusaderError
+    from crusaderbackend_b200.train import ResNetTrainer
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    dimg = torch.randn(264, 3, 8, 8, generator=gen, device="cuda")   # no batch groups above 256 samples
+    dlab = torch.eye(10, device="cuda")[torch.arange(264, device="cuda") % 10].contiguous()
+    results = []
+    for sync in (True, False):
+        ctx = Context(0, math="tf32", sync=sync)
+        ctx.set_deterministic(True)
+        tr = ResNetTrainer(ctx, batch=264, blocks_per_stage=1, image_hw=8)
+        tr.init_params("failing")
+        losses = []
+        for i in range(10):
+            if i in (3, 6):
+                tr.set_bn_groups(2)
+                for _ in range(4):
+                    with pytest.raises(CrusaderError, match="fused kernels"):
+                        tr.forward(dimg, dlab)
+                tr.set_bn_groups(1)
+            tr.step(dimg, dlab, lr=1e-5)
+            losses.append(tr.loss())
+        results.append((losses, tr.params.clone(), tr.replays))
+        tr.close()
+        ctx.close()
+    (la, pa, _), (lb, pb, replays) = results
+    assert la == lb and torch.equal(pa, pb) and replays >= 2 * 6
