@@ -538,7 +538,7 @@ static int conv_fwd_impl(cb_ctx* ctx, const float* W, const float* X, float* Y, 
     const long long npix = (long long)N * g.OH * g.OW;
     if (npix == 0 || OC == 0) return CB_OK;
     if (!W || !X || !Y) return fail(ctx, CB_EINVAL, std::string(who) + ": null operand");
-    if (ctx->math == CB_MATH_TF32) {  // tensor cores; 3xTF32 = three such passes; FP32 (and uncovered geometries) = CUDA cores
+    if (ctx->math == CB_MATH_TF32) {  // tensor cores; 3xTF32: conv_3xtf32; FP32 and uncovered geometries: CUDA cores
         rc = umma_conv_fwd(ctx, W, X, Y, ep, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, false, xb, yb);
         if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;
     } else if (ctx->math == CB_MATH_3XTF32) {

@@ -23,9 +23,9 @@
 //  * When a layer has fewer pixel tiles than the GPU has CTA slots, the output channels are split over 2 or 4 CTAs
 //    per tile (each fetches only its slice of the packed filter and runs a narrower UMMA), so that small feature maps
 //    still occupy the whole GPU.
-//  * Epilogue (four warps per TMEM lane quarter): tcgen05.ld, tap combine, then optional per-channel or
-//    per-position scale / shift, bias, accumulation onto the output, ReLU, and stores in which the 32 lanes of a warp
-//    write 128 contiguous bytes.
+//  * Epilogue (two warps per TMEM lane quarter where two CTAs share an SM, else four): tcgen05.ld, tap combine, then
+//    optional per-channel or per-position scale / shift, bias, ReLU, and 1 KB of staging a warp that leaves by TMA store, or
+//    by TMA reduce-add where it adds onto the output; outputs TMA cannot address are written directly, 128 bytes a warp.
 //
 // Covered geometry: stride 1, filter 1x1 (pad 0) or 3x3 (pad 1) per axis, W in {8,16,32}, (32/W) | H,
 // FW * OC(rounded to 16) <= 256 per CTA, packed filter slice <= ~150 KB; stride 2 through the phase split below.

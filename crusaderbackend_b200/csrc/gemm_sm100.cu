@@ -3,7 +3,8 @@
 // One persistent, warp-specialised kernel computes D[i][j] = sum_k P[i][k] * Q[j][k]:
 //   warp 0      TMA producer of P: cp.async.bulk.tensor tiles into 128B-swizzled shared memory, mbarrier pipeline
 //   last warp   TMA producer of Q
-//   warp 1      UMMA issuer: one lane issues tcgen05.mma kind::tf32 (M=128, N=bn, K=8), accumulators in TMEM
+//   warp 1      UMMA issuer: the whole warp runs the loop and one elected lane issues tcgen05.mma kind::tf32 (M=128, N=bn,
+//               K=8), accumulators in TMEM
 //   warps 2..17 epilogue: tcgen05.ld -> registers -> bias/ReLU -> global stores (four warps per TMEM lane quarter)
 //   then (3xTF32 only) eight split warps: write lo = a - tf32(a) beside each stage
 // P is the operand on the UMMA M side (128 TMEM lanes), Q the one on the N side (TMEM columns). Each operand

@@ -19,8 +19,9 @@ namespace {
 // A pipeline stage carries `lps` such lines (1, 2 or 4: as many as leave at least three stages), so that the per-stage
 // hand-offs between the producer, the shift warps and the MMA issuer are paid once per 32*lps pixels. Every CTA walks
 // its share of the line groups accumulating D[(fh,c)][(fw,oc)] in TMEM (the whole K split across CTAs). Its tile then
-// leaves in one of two ways: laid out in filter order in the (by then idle) pipeline stages and added into dW with
-// vector atomics by the whole CTA (`direct`, the default: one launch), or written to the workspace as a partial, column
+// leaves in one of two ways: laid out in filter order in the (by then idle) pipeline stages and added into dW by bulk
+// copies that add on arrival, or by scalar atomics where dW's runs are not whole 16-byte words (`direct`, the default: one
+// launch), or written to the workspace as a partial, column
 // by column (the 32 lanes of a warp hold 32 consecutive rows: full 128-byte lines), for a second kernel that adds the
 // partials in a fixed order (deterministic contexts).
 struct WgradParams {
@@ -40,7 +41,7 @@ struct WgradParams {
     float* partial;                  // [gridDim.x][NQ][mtiles * 128]; with `atomic`: ONE such tile that every CTA adds into
     int atomic;
     // direct != 0: no second kernel. The CTA lays its tile out in the idle pipeline stages in the order of the filter
-    // block it belongs to (`OC` runs of `run` floats) and adds the runs into dW with coalesced atomics:
+    // block it belongs to (`OC` runs of `run` floats) and adds the runs into dW (vec4 != 0: by bulk copies):
     // dW[base_off + oc * oc_stride + j] += tile[oc * run + j]. dW must already hold what the sums are added to.
     int direct, vec4, run, s2, IC_src;
     // rows_cf != 0 (32-pixel-wide maps): a line is one image row, so the FH vertically shifted X blocks of a line are

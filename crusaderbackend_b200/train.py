@@ -206,7 +206,7 @@ class ResNetTrainer:
         self.allreduce_grads()
         self.update(lr, beta, l2)
 
-    # ---- whole step as one CUDA graph (launch-bound otherwise: ~700 kernels per ResNet-56 step)
+    # ---- whole step as one CUDA graph (296 kernels per ResNet-56 step)
     def capture_step(self, images, labels_onehot, lr, beta=0.9, l2=1e-4, warmup=2, include_allreduce=True):
         """Runs `warmup` eager steps (workspace growth, packed filters, NCCL set-up), then records forward + backward
         (with the gradient allreduce of a distributed trainer) + update into a torch.cuda.CUDAGraph that reads the

@@ -326,7 +326,7 @@ def test_contraction_split_over_a_cluster(torch_cuda, ctxs, M, N, K, math):
 @pytest.mark.parametrize("form", ["NN", "NT", "TN"])
 @pytest.mark.parametrize("M,N,K", [(2900, 2600, 72), (2945, 2564, 132), (4100, 1800, 36)])
 def test_tall_tiles_over_several_waves(torch_cuda, ctxs, M, N, K, form):
-    """Outputs of more than one and a half waves, where a CTA holds 256 rows: last tile with rows in one or both halves."""
+    """Outputs of more than one wave, where a CTA holds 256 rows: last tile with rows in one or both halves."""
     torch = torch_cuda
     A, B = make_operands(M, N, K, form, ("tall", M, N, K, form))
     tA, tB = FORMS[form]
