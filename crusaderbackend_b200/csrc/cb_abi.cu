@@ -83,12 +83,8 @@ static int grow_block(cb_ctx* ctx, void** block, size_t* have, size_t bytes, siz
 }
 
 int ensure_workspace(cb_ctx* ctx, size_t bytes) { return grow_block(ctx, &ctx->workspace, &ctx->workspace_bytes, bytes, bytes >> 2); }
-// The passes of a convolution layer ask for different multiples of the same activations, one after the other: a 3xTF32 stride-2
-// layer's data gradient for its phase planes, its weight gradient for the planes and their lo parts. With room for twice the
-// first request the passes that follow need no second wait, free and allocation.
-static size_t layer_slack(size_t bytes) { return bytes < (size_t(64) << 20) ? bytes : size_t(64) << 20; }
-int ensure_workspace2(cb_ctx* ctx, size_t bytes) { return grow_block(ctx, &ctx->workspace2, &ctx->workspace2_bytes, bytes, layer_slack(bytes)); }
-int ensure_workspace3(cb_ctx* ctx, size_t bytes) { return grow_block(ctx, &ctx->workspace3, &ctx->workspace3_bytes, bytes, layer_slack(bytes)); }
+int ensure_workspace2(cb_ctx* ctx, size_t bytes) { return grow_block(ctx, &ctx->workspace2, &ctx->workspace2_bytes, bytes, 0); }
+int ensure_workspace3(cb_ctx* ctx, size_t bytes) { return grow_block(ctx, &ctx->workspace3, &ctx->workspace3_bytes, bytes, 0); }
 
 int ensure_wgrad_acc(cb_ctx* ctx, size_t bytes) {
     if (bytes <= ctx->wgrad_acc_bytes) return CB_OK;

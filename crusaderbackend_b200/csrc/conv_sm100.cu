@@ -1173,6 +1173,13 @@ static int plan_pass(const cb_ctx* ctx, ConvPlan& q, bool x3, const float* X, in
     return CB_OK;
 }
 
+// 3xTF32 scratch of a layer: `channels`, the most that either of its tensors has, with their lo parts. A forward pass or data
+// gradient asks for what the layer's other passes will need as well: every growth is a wait for the device, a free and an
+// allocation, 0.3 ms whatever the size.
+static int ensure_split_scratch(cb_ctx* ctx, int N, int channels, long long plane) {
+    return ensure_workspace3(ctx, (size_t)N * 2 * ((channels + 7) / 8 * 8) * plane * sizeof(float));
+}
+
 // One planned convolution on `X` (N images of `cin` planes, in_batch floats apart or dense). With q.x3 the input is first
 // written as [x ; x_lo] to scratch.
 static int run_pass(cb_ctx* ctx, const ConvEnv& env, const ConvPlan& q, const PackSpec& ps, const float* W, const float* X, int cin,
@@ -1233,6 +1240,7 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
         if (!((FW == 1 && pW == 0) || (FW == 3 && pW == 1))) return CB_EUNSUPPORTED;
         const int cin = dgrad_of ? OC : IC, cout = dgrad_of ? IC : OC;
         rc = plan_pass(ctx, q, x3, X, N, cin, cout, IH, IW, FH, FW, pH, pW);
+        if (rc == CB_OK && x3) rc = ensure_split_scratch(ctx, N, IC > OC ? IC : OC, (long long)IH * IW);
         if (rc != CB_OK) return rc;
         const PackSpec ps{dgrad_of ? PACK_DGRAD : PACK_FWD, OC, IC, FH, FW, 0, 0};
         rc = run_pass(ctx, env, q, ps, W, X, cin, Y, ep, N, IH, IW, FH, FW, pH, pW, in_batch, out_batch);
@@ -1254,6 +1262,7 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
         if (rc != CB_OK) return rc;
         const size_t sub_bytes = (size_t)N * IC * plane2 * sizeof(float);
         rc = ensure_workspace2(ctx, sub_bytes);
+        if (rc == CB_OK && x3) rc = ensure_split_scratch(ctx, N, IC > OC ? IC : OC, plane2);
         if (rc != CB_OK) return rc;
         float* sub = static_cast<float*>(ctx->workspace2);
         const PackSpec ps{dgrad_of ? PACK_DGRAD : PACK_FWD, OC, IC, 1, 1, 0, 0};
@@ -1289,7 +1298,7 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
         if (x3) {
             if (!vec_ok(X, nullptr, IW)) return CB_EUNSUPPORTED;
             const long long perp = 2LL * q.x3 * plane2;
-            rc = ensure_workspace3(ctx, (size_t)N * perp * sizeof(float));
+            rc = ensure_split_scratch(ctx, N, C4 > OC ? C4 : OC, plane2);
             if (rc != CB_OK) return rc;
             float* X2 = static_cast<float*>(ctx->workspace3);
             rc = launch_space_to_depth2_split(ctx, X, X2, N, IC, q.x3, IH, IW);
@@ -1310,11 +1319,11 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
     while (groups <= 4 && 2 * ((C4 / groups + 15) / 16 * 16) > 256) groups *= 2;
     if (groups > 4) return CB_EUNSUPPORTED;
     const int per_group = C4 / groups;
-    rc = ensure_workspace2(ctx, s2d_bytes);
+    rc = plan_pass(ctx, q, x3, X /* = dY */, N, OC, per_group, H2, W2, 2, 2, 0, 0);
+    if (rc == CB_OK) rc = ensure_workspace2(ctx, x3 ? 2 * s2d_bytes : s2d_bytes);  // 3xTF32: the weight gradient's lo parts
+    if (rc == CB_OK && x3) rc = ensure_split_scratch(ctx, N, C4 > OC ? C4 : OC, plane2);
     if (rc != CB_OK) return rc;
     float* dXs = static_cast<float*>(ctx->workspace2);
-    rc = plan_pass(ctx, q, x3, X /* = dY */, N, OC, per_group, H2, W2, 2, 2, 0, 0);
-    if (rc != CB_OK) return rc;
     for (int g = 0; g < groups; ++g) {
         const PackSpec ps{PACK_S2_DGRAD, OC, IC, 3, 3, g * per_group, per_group};
         rc = run_pass(ctx, env, q, ps, W, X /* = dY */, OC, dXs + (size_t)g * N * per_group * plane2, plain, N, H2, W2, 2, 2, 0, 0, 0,
