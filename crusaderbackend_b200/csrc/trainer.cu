@@ -162,8 +162,8 @@ struct cbt_model {
     float* scratch = nullptr;      // one activation-sized temporary for accumulating data gradients
     long long scratch_elems = 0;
     float* labels = nullptr;       // the one-hot labels of the current step (caller-owned pointer, like the input's)
-    float* own_images = nullptr;   // copies that recorded passes read; four floats longer than a batch (PassKey)
-    float* own_labels = nullptr;
+    float* own_images = nullptr;   // copies that recorded passes read, allocated with the first recording; both four floats
+    float* own_labels = nullptr;   // longer than a batch (PassKey)
     bool input_own = false;        // they hold the batch of the last forward pass
     float* loss_dev = nullptr;     // device word: summed loss of the current step
     float* loss_n = nullptr;       // per-sample losses of the current step (fused head)
@@ -428,8 +428,6 @@ int finalize_model(cbt_model* m, int x, int classes) {
     int rc = dev_alloc(m, &m->scratch, biggest);
     if (rc == CB_OK) rc = dev_alloc(m, &m->loss_dev, 4);
     if (rc == CB_OK) rc = dev_alloc(m, &m->loss_n, m->batch);
-    if (rc == CB_OK) rc = dev_alloc(m, &m->own_images, m->t[m->input].size() + 4);
-    if (rc == CB_OK) rc = dev_alloc(m, &m->own_labels, (long long)m->batch * classes + 4);
     if (rc == CB_OK) {
         const char* env = std::getenv("CBT_WGRAD_STREAMS");
         int n = env ? std::atoi(env) : 2;
@@ -822,6 +820,20 @@ void drop_recorded(cbt_model* m) {
     m->recorded.clear();
 }
 
+bool make_own_inputs(cbt_model* m) {
+    if (m->own_images) return true;
+    const long long n_images = (m->t[m->input].size() + 7) & ~3LL, n_labels = (long long)m->batch * m->classes + 4;
+    void* p = nullptr;
+    if (cudaMalloc(&p, (size_t)(n_images + n_labels) * sizeof(float)) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    m->owned.push_back(p);
+    m->own_images = static_cast<float*>(p);
+    m->own_labels = m->own_images + n_images;
+    return true;
+}
+
 // The launch of stage_inputs_kernel for one set of caller's buffers, as a stream launch and as the parameters of a graph node.
 struct StageInputs {
     const float *images, *labels;
@@ -904,6 +916,7 @@ int run_recorded(cbt_model* m, bool backward, F ops) {
         return pass();
     }
     const float *images = input, *labels = m->labels;
+    if (!make_own_inputs(m)) return pass();
     StageInputs stage(m, images, labels);
     if (!r->exec) {
         r->unusable = true;  // until the recording is complete
