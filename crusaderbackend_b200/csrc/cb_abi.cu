@@ -58,7 +58,7 @@ int finish(cb_ctx* ctx, const char* what) {
 // on a stream the context used earlier may still read it), and never while the workspace is frozen or the stream is
 // being captured: a captured graph keeps the addresses of the blocks it was recorded with, so a later free would leave
 // it reading released memory.
-static int grow_block(cb_ctx* ctx, void** block, size_t* have, size_t bytes, size_t slack) {
+static int grow_block(cb_ctx* ctx, void** block, size_t* have, size_t bytes, size_t ahead) {
     if (bytes <= *have) return CB_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone)
@@ -71,8 +71,14 @@ static int grow_block(cb_ctx* ctx, void** block, size_t* have, size_t bytes, siz
     if (*block) cudaFree(*block);
     *block = nullptr;
     *have = 0;
-    size_t want = (bytes + slack + 255) & ~size_t(255);
+    auto rounded = [](size_t n) { return (n + 255) & ~size_t(255); };
+    size_t want = rounded(ahead > bytes ? ahead : bytes);
     e = cudaMalloc(block, want);
+    if (e != cudaSuccess && want > rounded(bytes)) {
+        cudaGetLastError();
+        want = rounded(bytes);
+        e = cudaMalloc(block, want);
+    }
     if (e != cudaSuccess) {
         check_cuda(ctx, e, "workspace cudaMalloc");
         return CB_ENOMEM;
@@ -82,13 +88,13 @@ static int grow_block(cb_ctx* ctx, void** block, size_t* have, size_t bytes, siz
     return CB_OK;
 }
 
-int ensure_workspace(cb_ctx* ctx, size_t bytes) { return grow_block(ctx, &ctx->workspace, &ctx->workspace_bytes, bytes, bytes >> 2); }
-int ensure_workspace2(cb_ctx* ctx, size_t bytes) { return grow_block(ctx, &ctx->workspace2, &ctx->workspace2_bytes, bytes, 0); }
-int ensure_workspace3(cb_ctx* ctx, size_t bytes) { return grow_block(ctx, &ctx->workspace3, &ctx->workspace3_bytes, bytes, 0); }
+int ensure_workspace(cb_ctx* ctx, size_t bytes) { return grow_block(ctx, &ctx->workspace, &ctx->workspace_bytes, bytes, bytes + (bytes >> 2)); }
+int ensure_workspace2(cb_ctx* ctx, size_t bytes, size_t ahead) { return grow_block(ctx, &ctx->workspace2, &ctx->workspace2_bytes, bytes, ahead); }
+int ensure_workspace3(cb_ctx* ctx, size_t bytes, size_t ahead) { return grow_block(ctx, &ctx->workspace3, &ctx->workspace3_bytes, bytes, ahead); }
 
 int ensure_wgrad_acc(cb_ctx* ctx, size_t bytes) {
     if (bytes <= ctx->wgrad_acc_bytes) return CB_OK;
-    int rc = grow_block(ctx, &ctx->wgrad_acc, &ctx->wgrad_acc_bytes, bytes, bytes);
+    int rc = grow_block(ctx, &ctx->wgrad_acc, &ctx->wgrad_acc_bytes, bytes, 2 * bytes);
     if (rc != CB_OK) return rc;
     // kept all zero from here on: every call that adds into it also clears what it read
     cudaError_t e = cudaMemset(ctx->wgrad_acc, 0, ctx->wgrad_acc_bytes);

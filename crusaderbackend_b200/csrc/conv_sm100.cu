@@ -1173,22 +1173,22 @@ static int plan_pass(const cb_ctx* ctx, ConvPlan& q, bool x3, const float* X, in
     return CB_OK;
 }
 
-// 3xTF32 scratch of a layer: `channels`, the most that either of its tensors has, with their lo parts. A forward pass or data
-// gradient asks for what the layer's other passes will need as well: every growth is a wait for the device, a free and an
-// allocation, 0.3 ms whatever the size.
-static int ensure_split_scratch(cb_ctx* ctx, int N, int channels, long long plane) {
-    return ensure_workspace3(ctx, (size_t)N * 2 * ((channels + 7) / 8 * 8) * plane * sizeof(float));
+// 3xTF32 scratch of one pass over `channels` input channels and their lo parts; of a layer, when the block has to grow:
+// `layer` is the most channels that either of its tensors has.
+static int ensure_split_scratch(cb_ctx* ctx, int N, int channels, int layer, long long plane) {
+    auto bytes = [&](int c) { return (size_t)N * 2 * ((c + 7) / 8 * 8) * plane * sizeof(float); };
+    return ensure_workspace3(ctx, bytes(channels), bytes(layer));
 }
 
 // One planned convolution on `X` (N images of `cin` planes, in_batch floats apart or dense). With q.x3 the input is first
-// written as [x ; x_lo] to scratch.
+// written as [x ; x_lo] to scratch; `layer`: see ensure_split_scratch.
 static int run_pass(cb_ctx* ctx, const ConvEnv& env, const ConvPlan& q, const PackSpec& ps, const float* W, const float* X, int cin,
-                    float* Y, const ConvEpilogue& ep, int N, int IH, int IW, int FH, int FW, int pH, int pW, long long in_batch,
+                    int layer, float* Y, const ConvEpilogue& ep, int N, int IH, int IW, int FH, int FW, int pH, int pW, long long in_batch,
                     long long out_batch) {
     if (q.x3) {
         const long long plane = (long long)IH * IW, per = cin * plane, perp = q.x3 * plane;
         if (in_batch & 3) return CB_EUNSUPPORTED;
-        int rc = ensure_workspace3(ctx, (size_t)N * 2 * perp * sizeof(float));
+        int rc = ensure_split_scratch(ctx, N, q.x3, layer, plane);
         if (rc != CB_OK) return rc;
         float* X2 = static_cast<float*>(ctx->workspace3);
         const long long items = (long long)N * (perp / 4);
@@ -1240,10 +1240,9 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
         if (!((FW == 1 && pW == 0) || (FW == 3 && pW == 1))) return CB_EUNSUPPORTED;
         const int cin = dgrad_of ? OC : IC, cout = dgrad_of ? IC : OC;
         rc = plan_pass(ctx, q, x3, X, N, cin, cout, IH, IW, FH, FW, pH, pW);
-        if (rc == CB_OK && x3) rc = ensure_split_scratch(ctx, N, IC > OC ? IC : OC, (long long)IH * IW);
         if (rc != CB_OK) return rc;
         const PackSpec ps{dgrad_of ? PACK_DGRAD : PACK_FWD, OC, IC, FH, FW, 0, 0};
-        rc = run_pass(ctx, env, q, ps, W, X, cin, Y, ep, N, IH, IW, FH, FW, pH, pW, in_batch, out_batch);
+        rc = run_pass(ctx, env, q, ps, W, X, cin, IC > OC ? IC : OC, Y, ep, N, IH, IW, FH, FW, pH, pW, in_batch, out_batch);
         if (rc == CB_OK) ctx->last_kernel = name;
         return rc;
     }
@@ -1262,15 +1261,14 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
         if (rc != CB_OK) return rc;
         const size_t sub_bytes = (size_t)N * IC * plane2 * sizeof(float);
         rc = ensure_workspace2(ctx, sub_bytes);
-        if (rc == CB_OK && x3) rc = ensure_split_scratch(ctx, N, IC > OC ? IC : OC, plane2);
         if (rc != CB_OK) return rc;
         float* sub = static_cast<float*>(ctx->workspace2);
         const PackSpec ps{dgrad_of ? PACK_DGRAD : PACK_FWD, OC, IC, 1, 1, 0, 0};
         if (!dgrad_of) {
             rc = launch_subsample2(ctx, X, sub, (long long)N * IC, IH, IW);
-            if (rc == CB_OK) rc = run_pass(ctx, env, q, ps, W, sub, cin, Y, ep, N, H2, W2, 1, 1, 0, 0, 0, 0);
+            if (rc == CB_OK) rc = run_pass(ctx, env, q, ps, W, sub, cin, IC > OC ? IC : OC, Y, ep, N, H2, W2, 1, 1, 0, 0, 0, 0);
         } else {
-            rc = run_pass(ctx, env, q, ps, W, X /* = dY */, cin, sub, plain, N, H2, W2, 1, 1, 0, 0, 0, 0);
+            rc = run_pass(ctx, env, q, ps, W, X /* = dY */, cin, IC > OC ? IC : OC, sub, plain, N, H2, W2, 1, 1, 0, 0, 0, 0);
             const long long n_full = (long long)N * IC * IH * IW;
             if (rc == CB_OK) {
                 if (vec_ok(sub, Y, IW) && n_full / 4 <= kMostItems)
@@ -1298,7 +1296,7 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
         if (x3) {
             if (!vec_ok(X, nullptr, IW)) return CB_EUNSUPPORTED;
             const long long perp = 2LL * q.x3 * plane2;
-            rc = ensure_split_scratch(ctx, N, C4 > OC ? C4 : OC, plane2);
+            rc = ensure_split_scratch(ctx, N, q.x3, C4 > OC ? C4 : OC, plane2);
             if (rc != CB_OK) return rc;
             float* X2 = static_cast<float*>(ctx->workspace3);
             rc = launch_space_to_depth2_split(ctx, X, X2, N, IC, q.x3, IH, IW);
@@ -1320,13 +1318,12 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
     if (groups > 4) return CB_EUNSUPPORTED;
     const int per_group = C4 / groups;
     rc = plan_pass(ctx, q, x3, X /* = dY */, N, OC, per_group, H2, W2, 2, 2, 0, 0);
-    if (rc == CB_OK) rc = ensure_workspace2(ctx, x3 ? 2 * s2d_bytes : s2d_bytes);  // 3xTF32: the weight gradient's lo parts
-    if (rc == CB_OK && x3) rc = ensure_split_scratch(ctx, N, C4 > OC ? C4 : OC, plane2);
+    if (rc == CB_OK) rc = ensure_workspace2(ctx, s2d_bytes, x3 ? 2 * s2d_bytes : 0);  // 3xTF32: the weight gradient has lo parts too
     if (rc != CB_OK) return rc;
     float* dXs = static_cast<float*>(ctx->workspace2);
     for (int g = 0; g < groups; ++g) {
         const PackSpec ps{PACK_S2_DGRAD, OC, IC, 3, 3, g * per_group, per_group};
-        rc = run_pass(ctx, env, q, ps, W, X /* = dY */, OC, dXs + (size_t)g * N * per_group * plane2, plain, N, H2, W2, 2, 2, 0, 0, 0,
+        rc = run_pass(ctx, env, q, ps, W, X /* = dY */, OC, C4 > OC ? C4 : OC, dXs + (size_t)g * N * per_group * plane2, plain, N, H2, W2, 2, 2, 0, 0, 0,
                       0);
         if (rc != CB_OK) return rc;
     }

@@ -116,3 +116,23 @@ def test_scratch_of_one_pass_serves_the_layers_other_passes(ic, oc, stride, math
     ref = torch.nn.grad.conv2d_weight(X.double(), W.shape, dY.double(), stride=stride, padding=1)
     assert (dW - ref).abs().max() <= (1e-5 if math == "3xtf32" else 2e-3) * ref.abs().max()
     ctx.close()
+
+
+def test_frozen_scratch_needs_no_room_for_other_passes():
+    """A context frozen with enough scratch for a 3xTF32 forward pass runs it, although the layer's data gradient, which reads
+    eight times the channels, would need more; that one is refused."""
+    import torch
+    from crusaderbackend_b200._lib import CB_ENOMEM
+    from crusaderbackend_b200.api import Context, CrusaderError
+    ctx = Context(0, math="3xtf32", sync=True)
+    X, W = torch.randn(4, 16, 32, 32, device="cuda"), torch.randn(16, 16, 3, 3, device="cuda")
+    W2, Y2 = torch.randn(128, 16, 1, 1, device="cuda"), torch.empty(4, 128, 32, 32, device="cuda")
+    ctx.conv(W, X, torch.empty_like(X), 1, 1, 1, 1)
+    assert ctx.lib.cb_freeze_workspace(ctx.h, 1) == 0
+    ctx.conv(W2, X, Y2, 1, 1, 0, 0)
+    ref = torch.nn.functional.conv2d(X.double(), W2.double())
+    assert (Y2 - ref).abs().max() <= 1e-5 * ref.abs().max()
+    with pytest.raises(CrusaderError) as exc:
+        ctx.convDerive(W2, Y2, torch.empty_like(X), 1, 1, 0, 0)
+    assert exc.value.code == CB_ENOMEM
+    ctx.close()
