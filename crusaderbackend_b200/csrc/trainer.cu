@@ -870,8 +870,8 @@ struct StageInputs {
 // The caller's images and labels may be other buffers every time: a recorded forward pass begins with a copy of them into the
 // model's own (its node is given the new addresses before a launch), and the passes read those. Eager, and reading the caller's
 // buffers: the first calls, streams that are being captured, sync mode, data-parallel models (their collectives are ordered call
-// by call), calls that find a filter's packed copy stale, passes whose recording fails, and a backward pass whose forward pass
-// was eager. A recording is keyed by everything it has baked in, scratch blocks included; at most kMostRecorded are kept.
+// by call), calls that find a filter's packed copy stale or the filter cache switched off, passes whose recording fails, and a
+// backward pass whose forward pass was eager. A recording is keyed by everything it has baked in, scratch blocks included; at most kMostRecorded are kept.
 template <class F>
 int run_recorded(cbt_model* m, bool backward, F ops) {
     constexpr size_t kMostRecorded = 8;
