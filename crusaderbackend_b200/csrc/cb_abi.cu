@@ -315,6 +315,9 @@ int cb_debug_tmap_stats(cb_ctx* ctx, long long* hits, long long* misses) {
     return CB_OK;
 }
 
+// Development aid: filters in this context's packed-filter cache.
+int cb_debug_cached_filters(cb_ctx* ctx) { return ctx ? cb::filter_cache_size(ctx) : CB_EINVAL; }
+
 #ifdef CB_TRACE
 // Development builds only: the next tensor-core convolution kernels write 16 time stamps per CTA into `buf`, and the
 // forward / data-gradient kernel four more words per CTA (issuer wait and issue sums) behind the first 1024 x 16:

@@ -46,6 +46,7 @@ struct cb_ctx {
     int filter_cache_on = 0;       // packed convolution filters are kept between calls (cb_conv_cache_filters)
     long long filter_version = 0;  // bumped by every call that may have changed a filter's values
     void* filter_cache = nullptr;  // the cache itself (conv_sm100.cu)
+    std::vector<std::pair<const float*, const float*>> bound_params;  // parameter buffers of the models on this context
     int pdl = 1;                   // launch kernels that call griddep_wait with programmatic stream serialization
     void* wgrad_acc = nullptr;     // weight-gradient accumulator [column][row], all zero between calls (wgrad_sm100.cu)
     size_t wgrad_acc_bytes = 0;
@@ -182,6 +183,8 @@ int umma_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, int
 // Packed-filter cache of a context (conv_sm100.cu).
 int filter_cache_repack_all(cb_ctx* ctx);
 bool filter_cache_fresh(const cb_ctx* ctx);  // no convolution would re-pack a filter it has seen before
+int filter_cache_size(const cb_ctx* ctx);
+void filter_cache_forget(cb_ctx* ctx, const float* first, const float* last);  // waits for the device if there is anything to do
 void filter_cache_destroy(cb_ctx* ctx);
 
 bool umma_gemm_eligible(const GemmCall& g);

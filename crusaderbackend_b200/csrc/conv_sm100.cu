@@ -1029,11 +1029,19 @@ struct FilterCacheEntry {
     PackJob job;
     long long version;  // value of cb_ctx::filter_version when the packed copy was last written
 };
+// The jobs of one launch of pack_filter_table_kernel. A table whose launch was captured belongs to the caller's graph as well: it
+// stays until the context goes.
+struct FilterTable {
+    std::vector<PackJob> jobs;
+    PackJob* dev;
+    bool captured;
+};
 struct FilterCache {
     std::vector<FilterCacheEntry> entries;
-    PackJob* dev_table = nullptr;
-    size_t dev_table_entries = 0;
+    std::vector<FilterTable> tables;  // the last one holds every entry (and forgotten ones), unless `changed`
+    bool changed = true;
     long long biggest = 0;
+    std::vector<std::pair<size_t, float*>> spare;  // packed copies of forgotten filters, by size, for the next filters
 };
 
 static bool same_job(const PackJob& a, const PackJob& b) {
@@ -1046,7 +1054,8 @@ void filter_cache_destroy(cb_ctx* ctx) {
     FilterCache* fc = static_cast<FilterCache*>(ctx->filter_cache);
     if (!fc) return;
     for (FilterCacheEntry& e : fc->entries) cudaFree(e.job.Wp);
-    if (fc->dev_table) cudaFree(fc->dev_table);
+    for (FilterTable& t : fc->tables) cudaFree(t.dev);
+    for (auto& s : fc->spare) cudaFree(s.second);
     delete fc;
     ctx->filter_cache = nullptr;
 }
@@ -1076,14 +1085,22 @@ static int packed_filter(cb_ctx* ctx, const ConvEnv& env, const ConvPlan& q, con
         if (cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone)
             return fail(ctx, CB_ENOMEM, "a convolution filter was seen for the first time while the stream is being captured: "
                                         "run the same calls once before the capture so that its packed copy exists");
-        void* d = nullptr;
-        cudaError_t e = cudaMalloc(&d, q.w_total_bytes);
-        if (e != cudaSuccess) {
-            check_cuda(ctx, e, "packed filter cudaMalloc");
-            return CB_ENOMEM;
+        for (size_t i = 0; i < fc->spare.size() && !want.Wp; ++i)
+            if (fc->spare[i].first == q.w_total_bytes) {
+                want.Wp = fc->spare[i].second;
+                fc->spare.erase(fc->spare.begin() + (long)i);
+            }
+        if (!want.Wp) {
+            void* d = nullptr;
+            cudaError_t e = cudaMalloc(&d, q.w_total_bytes);
+            if (e != cudaSuccess) {
+                check_cuda(ctx, e, "packed filter cudaMalloc");
+                return CB_ENOMEM;
+            }
+            want.Wp = static_cast<float*>(d);
         }
-        want.Wp = static_cast<float*>(d);
         fc->entries.push_back(FilterCacheEntry{want, -1});
+        fc->changed = true;
         hit = &fc->entries.back();
     }
     if (hit->version != ctx->filter_version) {
@@ -1105,42 +1122,84 @@ bool filter_cache_fresh(const cb_ctx* ctx) {
     return true;
 }
 
+int filter_cache_size(const cb_ctx* ctx) {
+    const FilterCache* fc = static_cast<const FilterCache*>(ctx->filter_cache);
+    return fc ? (int)fc->entries.size() : 0;
+}
+
 // Re-packs every cached filter in one launch and marks them current.
 int filter_cache_repack_all(cb_ctx* ctx) {
     ctx->filter_version += 1;
     FilterCache* fc = static_cast<FilterCache*>(ctx->filter_cache);
     if (!ctx->filter_cache_on || !fc || fc->entries.empty()) return CB_OK;
-    if (fc->dev_table_entries != fc->entries.size()) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone)
-            return CB_OK;  // filters first seen after the last table build: they re-pack lazily at their next use
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool capturing = cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone;
+    if (fc->changed) {
+        if (capturing) return CB_OK;  // filters first seen after the last table build: they re-pack lazily at their next use
         cudaError_t e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) return check_cuda(ctx, e, "filter table rebuild");
-        if (fc->dev_table) cudaFree(fc->dev_table);
-        fc->dev_table = nullptr;
-        std::vector<PackJob> host(fc->entries.size());
+        if (!fc->tables.empty() && !fc->tables.back().captured) {
+            cudaFree(fc->tables.back().dev);
+            fc->tables.pop_back();
+        }
+        FilterTable t{{}, nullptr, false};
         fc->biggest = 0;
-        for (size_t i = 0; i < host.size(); ++i) {
-            host[i] = fc->entries[i].job;
-            if (host[i].total > fc->biggest) fc->biggest = host[i].total;
+        for (const FilterCacheEntry& en : fc->entries) {
+            t.jobs.push_back(en.job);
+            if (en.job.total > fc->biggest) fc->biggest = en.job.total;
         }
         void* d = nullptr;
-        e = cudaMalloc(&d, sizeof(PackJob) * host.size());
-        if (e == cudaSuccess) e = cudaMemcpy(d, host.data(), sizeof(PackJob) * host.size(), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) return check_cuda(ctx, e, "filter table upload");
-        fc->dev_table = static_cast<PackJob*>(d);
-        fc->dev_table_entries = host.size();
+        e = cudaMalloc(&d, sizeof(PackJob) * t.jobs.size());
+        if (e == cudaSuccess) e = cudaMemcpy(d, t.jobs.data(), sizeof(PackJob) * t.jobs.size(), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {
+            if (d) cudaFree(d);
+            return check_cuda(ctx, e, "filter table upload");
+        }
+        t.dev = static_cast<PackJob*>(d);
+        fc->tables.push_back(std::move(t));
+        fc->changed = false;
     }
+    FilterTable& table = fc->tables.back();
+    table.captured = table.captured || capturing;
     int gx = (int)((fc->biggest + 255) / 256);
     if (gx > 64) gx = 64;
     if (gx < 1) gx = 1;
-    cudaError_t e = launch_dep(ctx, pack_filter_table_kernel, dim3((unsigned)gx, (unsigned)fc->dev_table_entries), dim3(256), 0,
-                               (const PackJob*)fc->dev_table);
+    cudaError_t e = launch_dep(ctx, pack_filter_table_kernel, dim3((unsigned)gx, (unsigned)table.jobs.size()), dim3(256), 0,
+                               (const PackJob*)table.dev);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return check_cuda(ctx, e, "pack_filter_table_kernel launch");
     ctx->launches += 1;
     for (FilterCacheEntry& en : fc->entries) en.version = ctx->filter_version;
     return CB_OK;
+}
+
+// Forgets the filters in [first, last): the memory may be released, and no later launch reads it, nor does a graph that captured
+// one of the tables (its job does nothing from here on).
+void filter_cache_forget(cb_ctx* ctx, const float* first, const float* last) {
+    FilterCache* fc = static_cast<FilterCache*>(ctx->filter_cache);
+    if (!fc) return;
+    auto inside = [&](const PackJob& j) { return j.W >= first && j.W < last; };
+    bool any = false;
+    for (const FilterCacheEntry& e : fc->entries) any = any || inside(e.job);
+    for (const FilterTable& t : fc->tables)
+        for (const PackJob& j : t.jobs) any = any || inside(j);
+    if (!any) return;
+    cudaDeviceSynchronize();  // re-packs in flight, also those of graphs on other streams
+    for (size_t i = fc->entries.size(); i-- > 0;)
+        if (inside(fc->entries[i].job)) {
+            fc->spare.emplace_back((size_t)fc->entries[i].job.total * sizeof(float), fc->entries[i].job.Wp);
+            fc->entries.erase(fc->entries.begin() + (long)i);
+        }
+    for (FilterTable& t : fc->tables) {
+        bool dirty = false;
+        for (PackJob& j : t.jobs)
+            if (inside(j)) {
+                j.total = 0;
+                j.W = nullptr;
+                dirty = true;
+            }
+        if (dirty) cudaMemcpy(t.dev, t.jobs.data(), sizeof(PackJob) * t.jobs.size(), cudaMemcpyHostToDevice);
+    }
 }
 
 static int conv_on_packed(cb_ctx* ctx, const ConvEnv& env, const ConvPlan& q, const PackSpec& ps, const float* W,

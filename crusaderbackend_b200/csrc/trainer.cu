@@ -437,6 +437,22 @@ int finalize_model(cbt_model* m, int x, int classes) {
     return rc;
 }
 
+// The caller may release the bound parameters after this. Packed copies of their filters are forgotten unless another model of the
+// context is bound to the same buffer: its recordings read them.
+void unbind_params(cbt_model* m) {
+    if (!m->P) return;
+    auto& bound = m->ctx->bound_params;
+    const float *first = m->P, *last = m->P + m->param_count;
+    for (size_t i = 0; i < bound.size(); ++i)
+        if (bound[i].first == first && bound[i].second == last) {
+            bound.erase(bound.begin() + (long)i);
+            break;
+        }
+    for (const auto& b : bound)
+        if (b.first < last && first < b.second) return;
+    cb::filter_cache_forget(m->ctx, first, last);
+}
+
 void release_side_streams(cbt_model* m) {
     for (size_t s = 0; s < m->side.size(); ++s) {
         cudaStreamSynchronize(m->side_stream[s]);
@@ -635,6 +651,7 @@ int cbt_destroy(cbt_model* m) {
     drop_recorded(m);
     if (m->record_stream) cudaStreamDestroy(m->record_stream);
     release_side_streams(m);
+    unbind_params(m);
     for (void* p : m->owned) cudaFree(p);
     if (m->mom_table) cudaFree(m->mom_table);
     if (m->comm) {
@@ -670,6 +687,10 @@ int cbt_bind(cbt_model* m, float* params, float* grads, float* momentum) {
         return CB_EINVAL;
     }
     drop_recorded(m);  // they hold the addresses of the buffers bound before
+    if (m->P != params) {
+        unbind_params(m);
+        m->ctx->bound_params.emplace_back(params, params + m->param_count);
+    }
     m->P = params; m->G = grads; m->M = momentum;
     const int n = (int)m->params.size();
     std::vector<float*> w(n), g(n), mo(n);

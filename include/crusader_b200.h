@@ -162,7 +162,8 @@ int cb_conv_wgrad_ex(cb_ctx* ctx, const float* dY, const float* X, float* dW, in
  *     filter in ONE launch on the context's stream (a training step then pays one pack launch instead of two per
  *     convolution).
  * Packed copies are device allocations made at a filter's first use (do that before capturing a CUDA graph) and
- * released by cb_destroy. Default: off — every call packs its filter into the context workspace.
+ * released by cb_destroy. Filters stay allocated as long as the context: cb_filters_changed reads every one the cache has seen
+ * (those of a model's bound parameters until cbt_destroy or another cbt_bind, which forget them). Default: off — every call packs its filter into the context workspace.
  */
 int cb_conv_cache_filters(cb_ctx* ctx, int on);
 int cb_filters_changed(cb_ctx* ctx);

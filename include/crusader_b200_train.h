@@ -36,7 +36,8 @@ int cbt_param_entries(const cbt_model* m);
 int cbt_param_entry(const cbt_model* m, int i, long long* offset, long long* size, int* is_weight, int* kind, int* dims);
 int cbt_op_count(const cbt_model* m);
 
-/* Binds the flat device buffers (cbt_param_count floats each, 16-byte aligned; gradients start at zero). */
+/* Binds the flat device buffers (cbt_param_count floats each, 16-byte aligned; gradients start at zero). The buffers bound before
+ * may be released afterwards, as all of them after cbt_destroy; graphs captured over this model go first. */
 int cbt_bind(cbt_model* m, float* params, float* grads, float* momentum);
 
 /* Must be called after the caller wrote to the bound parameter buffer by any route other than cbt_update (initial

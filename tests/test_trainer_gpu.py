@@ -509,3 +509,90 @@ def test_pass_that_cannot_be_recorded(torch_cuda):
         ctx.close()
     (la, pa, _), (lb, pb, replays) = results
     assert la == lb and torch.equal(pa, pb) and replays >= 2 * 6
+
+
+@pytest.mark.parametrize("math", ["tf32", "3xtf32"])
+def test_models_that_share_a_context_with_a_destroyed_one(torch_cuda, math):
+    """The packed filters of a destroyed model are forgotten, so that its parameters may be released: by the updates of the
+    models that stay, by a graph that was captured while it lived, and by a model that comes after it."""
+    torch = torch_cuda
+    from crusaderbackend_b200.api import Context
+    from crusaderbackend_b200.train import DenseNetTrainer, ResNetTrainer
+    _, _, dimg, dlab = make_batch(torch, 8, 16, 10, "shared")
+
+    def steps(ctx, tr, key, captured=False, between=None):
+        tr.init_params(key)
+        host = tr.params.cpu().numpy()
+        tr.step(dimg, dlab, lr=1e-3)
+        graph = tr.capture_step(dimg, dlab, 1e-3) if captured else None
+        if captured:
+            ctx._check(ctx.lib.cb_freeze_workspace(ctx.h, 0))
+        if between:
+            between()
+        tr.set_params(host)
+        for _ in range(4):
+            graph.replay() if captured else tr.step(dimg, dlab, lr=1e-3)
+        ctx.synchronize()
+        return tr.params.clone()
+
+    def fresh():
+        ctx = Context(0, math=math)
+        ctx.set_deterministic(True)
+        return ctx
+    want = {}
+    for key, captured in (("stays", True), ("after", False)):
+        ctx = fresh()
+        tr = ResNetTrainer(ctx, batch=8, blocks_per_stage=1, image_hw=16)
+        want[key] = steps(ctx, tr, key, captured)
+        alone = ctx.lib.cb_debug_cached_filters(ctx.h)
+        tr.close()
+        assert ctx.lib.cb_debug_cached_filters(ctx.h) == 0 < alone
+        ctx.close()
+
+    ctx = fresh()
+    gone = DenseNetTrainer(ctx, batch=8, growth=4, layers=2, image_hw=16)
+    steps(ctx, gone, "gone")
+    stays = ResNetTrainer(ctx, batch=8, blocks_per_stage=1, image_hw=16)
+
+    def destroy():   # after the capture, whose table holds the filters of both
+        assert ctx.lib.cb_debug_cached_filters(ctx.h) > alone
+        gone.close()
+        for name in ("params", "grads", "momentum"):
+            setattr(gone, name, None)
+        assert ctx.lib.cb_debug_cached_filters(ctx.h) == alone
+    assert torch.equal(steps(ctx, stays, "stays", True, destroy), want["stays"])
+    after = ResNetTrainer(ctx, batch=8, blocks_per_stage=1, image_hw=16)
+    assert torch.equal(steps(ctx, after, "after"), want["after"])
+    assert ctx.lib.cb_debug_cached_filters(ctx.h) == 2 * alone
+    stays.close()
+    after.close()
+    ctx.close()
+
+
+def test_models_that_share_their_parameters(torch_cuda):
+    """A second model bound to the first one's buffers, as for a batch of another size: destroying it leaves the first one's packed
+    filters, which its recorded passes read, as they are."""
+    torch = torch_cuda
+    from crusaderbackend_b200.api import Context
+    from crusaderbackend_b200.train import ResNetTrainer
+    _, _, dimg, dlab = make_batch(torch, 8, 16, 10, "bound twice")
+    results = []
+    for second in (False, True):
+        ctx = Context(0, math="tf32")
+        ctx.set_deterministic(True)
+        tr = ResNetTrainer(ctx, batch=8, blocks_per_stage=1, image_hw=16)
+        tr.init_params("bound twice")
+        for i in range(10):
+            tr.step(dimg, dlab, lr=1e-3)
+            if second and i == 5:
+                other = ResNetTrainer(ctx, batch=4, blocks_per_stage=1, image_hw=16)
+                other._check(other.lib.cbt_bind(other.h, tr.params.data_ptr(), tr.grads.data_ptr(), tr.momentum.data_ptr()))
+                other.forward(dimg[:4], dlab[:4])
+                other.close()
+        results.append((tr.params.clone(), ctx.lib.cb_debug_cached_filters(ctx.h)))
+        assert tr.replays > 0
+        tr.close()
+        assert ctx.lib.cb_debug_cached_filters(ctx.h) == 0
+        ctx.close()
+    assert torch.equal(results[0][0], results[1][0])
+    assert results[0][1] <= results[1][1]   # another batch may pack some filters in another layout as well
