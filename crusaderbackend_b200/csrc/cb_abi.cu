@@ -388,7 +388,7 @@ int cb_gemm(cb_ctx* ctx, int transA, int transB, int M, int N, int K, const floa
     if (ctx->math != CB_MATH_FP32 && umma_gemm_eligible(g))
         rc = launch_umma_gemm(ctx, g, ctx->math == CB_MATH_3XTF32);
     else
-        rc = launch_simt_gemm(ctx, g);
+        rc = launch_fp32_gemm(ctx, g);
     if (rc != CB_OK) return rc;
     return finish(ctx, "cb_gemm");
 }
@@ -421,7 +421,7 @@ int cb_gemm_batch_reduce(cb_ctx* ctx, int transA, int transB, int M, int N, int 
     if (ctx->math != CB_MATH_FP32 && umma_gemm_eligible(g))
         rc = launch_umma_gemm(ctx, g, ctx->math == CB_MATH_3XTF32);
     else
-        rc = launch_simt_gemm(ctx, g);
+        rc = launch_fp32_gemm(ctx, g);
     if (rc != CB_OK) return rc;
     return finish(ctx, "cb_gemm_batch_reduce");
 }

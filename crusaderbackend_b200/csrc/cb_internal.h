@@ -189,7 +189,10 @@ void filter_cache_destroy(cb_ctx* ctx);
 
 bool umma_gemm_eligible(const GemmCall& g);
 int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3);
-int launch_simt_gemm(cb_ctx* ctx, const GemmCall& g);
+// fp32 accuracy: on the CUDA cores, or (launch_split_gemm: CB_EUNSUPPORTED, before any work is queued, where it is not worth it) on the
+// tensor cores.
+int launch_fp32_gemm(cb_ctx* ctx, const GemmCall& g);
+int launch_split_gemm(cb_ctx* ctx, const GemmCall& g);
 // Clears the output matrices of a call whose partial products are added into them with atomics.
 int clear_output(cb_ctx* ctx, float* p, long long width, long long ld, long long rows, long long stride, long long batch, const char* who);
 

@@ -361,6 +361,28 @@ __device__ __forceinline__ void umma_tf32_elect(uint32_t d_tmem, uint64_t desc_a
         "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// D[tmem] (+)= A[tmem] * B[smem desc] for bf16 operands (16 k a step: 8 columns of A, two k a column), fp32 accumulate.
+__device__ __forceinline__ void umma_bf16_ts_elect(uint32_t d_tmem, uint32_t a_tmem, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// Whole-warp: 8 or 4 consecutive columns of the warp's 32 lanes; complete after tmem_st_wait.
+__device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // Whole-warp: 32 lanes x 16 consecutive fp32 columns starting at taddr (lane field = warp's quarter).
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
@@ -419,6 +441,11 @@ __host__ __device__ __forceinline__ uint32_t umma_idesc_tf32(uint32_t m, uint32_
     d |= ((n >> 3) & 0x3Fu) << 17;
     d |= ((m >> 4) & 0x1Fu) << 24;
     return d;
+}
+
+// kind::f16 with bf16 operands (A in TMEM or K-major, B K-major) and fp32 accumulation.
+__host__ __device__ __forceinline__ uint32_t umma_idesc_bf16(uint32_t m, uint32_t n) {
+    return 1u << 4 | 1u << 7 | 1u << 10 | ((n >> 3) & 0x3Fu) << 17 | ((m >> 4) & 0x1Fu) << 24;
 }
 
 }  // namespace cb

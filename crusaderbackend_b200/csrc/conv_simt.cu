@@ -5,85 +5,21 @@
 #include <cstdlib>
 
 #include "cb_ptx.cuh"
+#include "conv_gather.cuh"
 #include "simt_core.cuh"
+#include "split_core.cuh"
 
 namespace cb {
+
+using namespace gather;
+
+// conv_split.cu
+cudaError_t launch_split_gather(cb_ctx* ctx, const GatherParams& p, const split::Choice& c, bool mask, long long pixels, int sets);
+cudaError_t launch_split_wgrad(cb_ctx* ctx, const WgradParams& p, const split::Choice& c, bool mask);
+
 namespace {
 
-struct ConvGeo {
-    int N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, OH, OW;
-    long long x_batch, y_batch;  // elements between consecutive images of the input-side / output-side tensor
-};
-
-__device__ __forceinline__ float apply_epilogue(const ConvEpilogue& ep, float v, int oc, long long pos_idx, float old) {
-    if (ep.scale) {
-        const long long si = ep.per_position ? pos_idx : (long long)oc;
-        v = fmaf(v, ep.scale[si], ep.shift[si]);
-    }
-    if (ep.bias) v += ep.bias[oc];
-    if (ep.accumulate) v += old;
-    if (ep.relu) v = fmaxf(v, 0.f);
-    return v;
-}
-
-// ---- forward and data gradient as D[pixel][channel] = sum_k In(pixel, k) * W(channel, k), k = (input channel, tap)
-//
-// A launch covers a set of output pixels on a regular grid: pixel (u, v) of an image reads In at row hs*u + hb + sgn*th
-// and column ws*v + wb + sgn*tw for its taps (th, tw), and is written at row oh0 + ohs*u, column ow0 + ows*v. The forward
-// pass is one such set (sgn = +1). The data gradient of a strided convolution is sH x sW sets, one for each phase of the
-// input row and column: only every sH-th tap reaches a pixel of a phase, so a set's contraction holds just those taps
-// (sgn = -1) and no products with structural zeros are formed.
-struct PixelSet {
-    int UH, UW;              // pixels of an image in the set
-    int hs, hb, ws, wb;      // first tap's input row / column
-    int oh0, ohs, ow0, ows;  // output row / column
-    int TH, TW;              // taps
-    int wt0, wts, wu0, wus;  // filter row of tap th: wt0 + wts*th; filter column: wu0 + wus*tw
-    int K;                   // channels * TH * TW
-};
-constexpr int kMaxSets = 4;  // pixel sets of one launch: the four phases of a stride-2 data gradient
-struct GatherParams {
-    const float* In; long long in_batch; int C, H, W;       // the tensor the taps read
-    const float* Wt; int w_ch, w_out, FW;                    // filter strides: contraction channel, output channel; width
-    float* Out; long long out_batch; int OUTC, OHH, OWW;     // output channels, rows, columns
-    int N, sgn;
-    int splits, per_split, atomic_out, tap_major;
-    ConvEpilogue ep;
-    PixelSet sets[kMaxSets]; // blockIdx.z = set * splits + split
-};
-
-// Which taps of a pixel lie inside the tensor. Filters of up to 15 x 15 taps keep it as one word, tap rows in the low half
-// and tap columns in the high half, and a tap's test is (mask & bits) == bits; larger ones compare coordinates.
-constexpr int kMaskTaps = 15;
-__device__ __forceinline__ uint32_t range_mask(int first, int sgn, int count, int extent) {
-    // taps t in [0, count) with 0 <= first + sgn * t < extent
-    int lo = sgn > 0 ? -first : first - extent + 1, hi = sgn > 0 ? extent - first : first + 1;
-    lo = min(max(lo, 0), count);
-    hi = min(max(hi, 0), count);
-    return hi > lo ? ((1u << hi) - 1u) & ~((1u << lo) - 1u) : 0u;
-}
-struct Position {
-    int h0, w0;      // coordinates of the first tap
-    uint32_t mask;
-};
-template <bool MASK>
-__device__ __forceinline__ bool tap_inside(const Position& at, uint32_t bits, int H, int W) {
-    if (MASK) return (at.mask & bits) == bits;
-    return (unsigned)(at.h0 + ((int)bits >> 16)) < (unsigned)H && (unsigned)(at.w0 + (short)bits) < (unsigned)W;
-}
-template <bool MASK>
-__device__ __forceinline__ uint32_t tap_bits(int th, int tw, int sgn) {
-    if (MASK) return (1u << th) | (1u << (16 + tw));
-    return ((uint32_t)(sgn * th) << 16) | ((uint32_t)(sgn * tw) & 0xffffu);
-}
-
-// What the copies of one k need: offset from a pixel's first tap, tap test, offset in the filter (-1: past the end).
-struct TapK {
-    int off;
-    uint32_t bits;
-    int woff, pad;
-};
-
+// ---- forward and data gradient
 template <class T, bool MASK>
 struct GatherSource {
     const GatherParams& p;
@@ -94,20 +30,7 @@ struct GatherSource {
     int base;
     int j0, slice0;
     __device__ __forceinline__ void begin(int t) {
-        if (threadIdx.x < simt::kBK) {
-            const int k = (slice0 + t) * simt::kBK + threadIdx.x;
-            TapK e{0, 0xffffffffu, -1, 0};
-            if (k < s.K) {
-                const int taps = s.TH * s.TW;
-                // the order in which a pixel's products are added: channel by channel, or (data gradient) tap by tap
-                const int c = p.tap_major ? k % p.C : k / taps, r = p.tap_major ? k / p.C : k - c * taps;
-                const int th = r / s.TW, tw = r - th * s.TW;
-                e.off = (c * p.H + p.sgn * th) * p.W + p.sgn * tw;
-                e.bits = tap_bits<MASK>(th, tw, p.sgn);
-                e.woff = c * p.w_ch + (s.wt0 + s.wts * th) * p.FW + s.wu0 + s.wus * tw;
-            }
-            table[(t & 1) * simt::kBK + threadIdx.x] = e;
-        }
+        if (threadIdx.x < simt::kBK) table[(t & 1) * simt::kBK + threadIdx.x] = tap_of<MASK>(p, s, (slice0 + t) * simt::kBK + threadIdx.x);
     }
     __device__ __forceinline__ void load(int t, uint32_t dst) {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -151,13 +74,7 @@ __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_gather_simt(const __g
     {
         const long long i = i0 + simt::MnLanes<T::BM, T::NW>::e(threadIdx.x >> 5, threadIdx.x & 31);
         if (i < pixels) {
-            const int per = s.UH * s.UW;
-            const int n = (int)(i / per), r = (int)(i - (long long)n * per);
-            const int u = r / s.UW, v = r - u * s.UW;
-            src.img = p.In + (long long)n * p.in_batch;
-            src.at.h0 = s.hs * u + s.hb;
-            src.at.w0 = s.ws * v + s.wb;
-            if (MASK) src.at.mask = range_mask(src.at.h0, p.sgn, s.TH, p.H) | (range_mask(src.at.w0, p.sgn, s.TW, p.W) << 16);
+            src.at = input_of<MASK>(p, s, i, src.img);
             src.base = src.at.h0 * p.W + src.at.w0;
         }
     }
@@ -175,13 +92,7 @@ __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_gather_simt(const __g
             const long long i = i0 + simt::own_row<T>() + 32 * h + x;
             at[h][x] = -1;
             out[h][x] = p.Out;
-            if (i < pixels) {
-                const int per = s.UH * s.UW;
-                const int n = (int)(i / per), r = (int)(i - (long long)n * per);
-                const int u = r / s.UW, v = r - u * s.UW;
-                at[h][x] = (s.oh0 + s.ohs * u) * p.OWW + s.ow0 + s.ows * v;
-                out[h][x] = p.Out + (long long)n * p.out_batch + at[h][x];
-            }
+            if (i < pixels) at[h][x] = output_of(p, s, i, out[h][x]);
         }
     simt::for_outputs<T>(acc, 0, src.j0, [&](int j, int i, float (&v)[4]) {
         if (j >= p.OUTC) return;
@@ -202,25 +113,7 @@ __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_gather_simt(const __g
     });
 }
 
-// ---- weight gradient as D[(ic, fh, fw)][oc] = sum over pixels of X(pixel + tap) * dY(pixel)
-struct WgradParams {
-    const float* X; const float* dY; float* dW;
-    ConvGeo g;
-    int I;                   // IC * FH * FW
-    int pixels;              // N * OH * OW
-    int splits, per_split;
-    int mode;                // 0 store, 1 add, 2 atomic add
-};
-struct PixelK {
-    long long x, y;          // offsets of the pixel's first tap in X and of the pixel in dY (-1: past the end)
-    Position at;
-    int pad;
-};
-struct TapI {
-    int off;
-    uint32_t bits;
-};
-
+// ---- weight gradient
 template <class T, bool MASK>
 struct WgradSource {
     const WgradParams& p;
@@ -228,21 +121,7 @@ struct WgradSource {
     const TapI* rows;        // [BM]
     int j0, slice0, opix;
     __device__ __forceinline__ void begin(int t) {
-        if (threadIdx.x < simt::kBK) {
-            const ConvGeo& g = p.g;
-            const int k = (slice0 + t) * simt::kBK + threadIdx.x;
-            PixelK e{0, -1, Position{-(1 << 29), 0, 0u}, 0};
-            if (k < p.pixels) {
-                const int n = k / opix, r = k - n * opix;
-                const int oh = r / g.OW, ow = r - oh * g.OW;
-                e.at.h0 = oh * g.sH - g.pH;
-                e.at.w0 = ow * g.sW - g.pW;
-                if (MASK) e.at.mask = range_mask(e.at.h0, 1, g.FH, g.IH) | (range_mask(e.at.w0, 1, g.FW, g.IW) << 16);
-                e.x = (long long)n * g.x_batch + e.at.h0 * g.IW + e.at.w0;
-                e.y = (long long)n * g.y_batch + r;
-            }
-            table[(t & 1) * simt::kBK + threadIdx.x] = e;
-        }
+        if (threadIdx.x < simt::kBK) table[(t & 1) * simt::kBK + threadIdx.x] = pixel_of<MASK>(p, (slice0 + t) * simt::kBK + threadIdx.x);
     }
     __device__ __forceinline__ void load(int t, uint32_t dst) {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -281,17 +160,7 @@ __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_wgrad_simt(const Wgra
     griddep_wait();
     griddep_launch();
     const int i0 = blockIdx.x * T::BM;
-    const int taps = p.g.FH * p.g.FW;
-    for (int e = threadIdx.x; e < T::BM; e += T::NT) {
-        TapI w{-1, 0xffffffffu};  // past the end: the tap test fails
-        if (i0 + e < p.I) {
-            const int ic = (i0 + e) / taps, r = (i0 + e) - ic * taps;
-            const int fh = r / p.g.FW, fw = r - fh * p.g.FW;
-            w.off = (ic * p.g.IH + fh) * p.g.IW + fw;
-            w.bits = tap_bits<MASK>(fh, fw, 1);
-        }
-        rows[e] = w;
-    }
+    for (int e = threadIdx.x; e < T::BM; e += T::NT) rows[e] = row_of<MASK>(p, i0 + e);
     WgradSource<T, MASK> src{p, table, rows, (int)blockIdx.y * T::BN, (int)blockIdx.z * p.per_split, p.g.OH * p.g.OW};
     const int slices = (p.pixels + simt::kBK - 1) / simt::kBK;
     simt::Acc<T> acc;
@@ -309,7 +178,11 @@ __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_wgrad_simt(const Wgra
     });
 }
 
-// One launch for up to four pixel sets. The contraction is split over CTAs where the output alone does not fill the GPU and the
+// Multiplications from which a pass runs at fp32 accuracy on the tensor cores (conv_split.cu).
+constexpr long long kLeastConv = 1LL << 22;
+
+// One launch for up to four pixel sets. In the passes of a model the two that later layers read stay on the CUDA cores (see
+// launch_fp32_gemm). The contraction is split over CTAs where the output alone does not fill the GPU and the
 // epilogue is a plain sum (the output is then cleared first), except in the passes of a model: atomic sums come in any order, and
 // one rounding more or less in an activation moves the gradients of a deep model by percents from one run to the next.
 int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, const char* who) {
@@ -319,9 +192,15 @@ int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, 
     bool may_split = !ctx->deterministic && !ctx->model_pass && !p.ep.scale && !p.ep.relu;
     int most = 0;
     for (int i = 0; i < nsets; ++i) most = sets[i].K > most ? sets[i].K : most;
-    const simt::Choice c = simt::choose_tile(ctx->sm_count, (long long)p.N * sets[0].UH * sets[0].UW * nsets, p.OUTC,
-                                             (most + simt::kBK - 1) / simt::kBK, 1, may_split);
-    p.splits = c.splits; p.per_split = c.per_split; p.atomic_out = c.splits > 1 ? 1 : 0;
+    const long long I = (long long)p.N * sets[0].UH * sets[0].UW * nsets;
+    const bool on_tensor_cores = !ctx->model_pass && split::worth_it(I, p.OUTC, most, 1, kLeastConv);
+    simt::Choice c{};
+    split::Choice sc{};
+    if (on_tensor_cores) sc = split::choose_shape(ctx->sm_count, I, p.OUTC, (most + split::kBK - 1) / split::kBK, 1, may_split, 1.5);
+    else c = simt::choose_tile(ctx->sm_count, I, p.OUTC, (most + simt::kBK - 1) / simt::kBK, 1, may_split);
+    p.splits = on_tensor_cores ? sc.splits : c.splits;
+    p.per_split = on_tensor_cores ? sc.per_split : c.per_split;
+    p.atomic_out = p.splits > 1 ? 1 : 0;
     if (p.atomic_out && !p.ep.accumulate) {
         const int rc = clear_output(ctx, p.Out, out_elems, p.out_batch, p.N, 0, 1, who);
         if (rc != CB_OK) return rc;
@@ -337,7 +216,7 @@ int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, 
             pixels = n > pixels ? n : pixels;
         }
         if (pixels == 0) continue;
-        cudaError_t e = simt::with_tile(c.tile, [&](auto tile) {
+        cudaError_t e = on_tensor_cores ? launch_split_gather(ctx, p, sc, mask, pixels, count) : simt::with_tile(c.tile, [&](auto tile) {
             typedef decltype(tile) T;
             auto kernel = mask ? conv_gather_simt<T, true> : conv_gather_simt<T, false>;
             cudaError_t er = raise_dynamic_smem_once(kernel, ctx->device, ctx->max_smem_optin, nullptr);
@@ -350,7 +229,7 @@ int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, 
         if (e != cudaSuccess) return check_cuda(ctx, e, who);
         ctx->launches += 1;
     }
-    ctx->last_kernel = "simt_fp32";
+    ctx->last_kernel = on_tensor_cores ? "umma_fp32" : "simt_fp32";
     return CB_OK;
 }
 
@@ -397,14 +276,19 @@ int simt_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, con
         return fail(ctx, CB_EUNSUPPORTED, std::string(who) + ": more than 2^31 pixels or filter values");
     const bool mask = g.FH <= kMaskTaps && g.FW <= kMaskTaps;
     p.I = (int)I; p.pixels = (int)pixels;
-    const simt::Choice c = simt::choose_tile(ctx->sm_count, I, g.OC, (pixels + simt::kBK - 1) / simt::kBK, 1, !ctx->deterministic);
-    p.splits = c.splits; p.per_split = c.per_split;
-    p.mode = c.splits > 1 ? 2 : (accumulate ? 1 : 0);
+    const bool on_tensor_cores = split::worth_it(I, g.OC, pixels, 1, kLeastConv);
+    simt::Choice c{};
+    split::Choice sc{};
+    if (on_tensor_cores) sc = split::choose_shape(ctx->sm_count, I, g.OC, (pixels + split::kBK - 1) / split::kBK, 1, !ctx->deterministic, 2.0);
+    else c = simt::choose_tile(ctx->sm_count, I, g.OC, (pixels + simt::kBK - 1) / simt::kBK, 1, !ctx->deterministic);
+    p.splits = on_tensor_cores ? sc.splits : c.splits;
+    p.per_split = on_tensor_cores ? sc.per_split : c.per_split;
+    p.mode = p.splits > 1 ? 2 : (accumulate ? 1 : 0);
     if (p.mode == 2 && !accumulate) {
         const int rc = clear_output(ctx, dW, I * g.OC, I * g.OC, 1, 0, 1, who);
         if (rc != CB_OK) return rc;
     }
-    cudaError_t e = simt::with_tile(c.tile, [&](auto tile) {
+    cudaError_t e = on_tensor_cores ? launch_split_wgrad(ctx, p, sc, mask) : simt::with_tile(c.tile, [&](auto tile) {
         typedef decltype(tile) T;
         auto kernel = mask ? conv_wgrad_simt<T, true> : conv_wgrad_simt<T, false>;
         cudaError_t er = raise_dynamic_smem_once(kernel, ctx->device, ctx->max_smem_optin, nullptr);
@@ -416,7 +300,7 @@ int simt_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, con
     });
     if (e != cudaSuccess) return check_cuda(ctx, e, who);
     ctx->launches += 1;
-    ctx->last_kernel = "simt_fp32";
+    ctx->last_kernel = on_tensor_cores ? "umma_fp32" : "simt_fp32";
     return CB_OK;
 }
 

@@ -1,0 +1,214 @@
+// The three convolution passes at fp32 accuracy on the tensor cores: the gathers of conv_simt.cu (any filter size, stride and padding)
+// feeding the body of split_core.cuh. conv_simt.cu decides which launches come here.
+#include "conv_gather.cuh"
+#include "split_core.cuh"
+
+namespace cb {
+
+using namespace gather;
+
+namespace {
+
+using split::kBK;
+
+// A summing thread's n outputs into memory `step` floats apart. plain: stored, or (add) added to what is there, one atomic add being
+// a read, an addition and a write without the wait for the read. Otherwise value(c, y, old place) is what is stored, or added.
+template <class F>
+__device__ __forceinline__ void store_columns(float* dst, long long step, int n, uint32_t mine, bool plain, bool add, F value) {
+    if (plain) {  // without a branch in the loop: reads of several columns are in flight together
+        if (add)
+#pragma unroll 8
+            for (int c = 0; c < n; ++c, dst += step) atomicAdd(dst, split::staged(mine, c));
+        else
+#pragma unroll 8
+            for (int c = 0; c < n; ++c, dst += step) *dst = split::staged(mine, c);
+        return;
+    }
+#pragma unroll 4
+    for (int c = 0; c < n; ++c, dst += step) {
+        const float y = value(c, split::staged(mine, c), dst);
+        if (add) atomicAdd(dst, y);
+        else *dst = y;
+    }
+}
+
+// Forward and data gradient: rows are pixels, columns output channels.
+template <class S, bool MASK>
+struct SplitGather {
+    static constexpr split::Kind kP = split::MN, kQ = split::K;
+    static constexpr bool kTable = true;
+    typedef split::ShareP<S, kP> SP;
+    typedef split::ShareQ<S, kQ> SQ;
+    const GatherParams& p;
+    const PixelSet& s;
+    TapK* table;             // [kLoaders]
+    const float* img;        // a loader thread's pixel: its image, its taps, offset of the first tap
+    Position at;
+    int base;
+    long long i0, pixels;
+    int j0, block0, part;
+    __device__ __forceinline__ void prepare(int t, int tid) {
+        table[tid] = tap_of<MASK>(p, s, (block0 + t) * kBK + tid);
+    }
+    __device__ __forceinline__ void load(int t, int tid, float (&vp)[SP::kValues], float (&vq)[SQ::kValues]) {
+        const TapK* tab = table + t % (S::kLoaders / kBK) * kBK;
+#pragma unroll
+        for (int x = 0; x < SP::kValues; ++x) {
+            const TapK q = tab[SP::k(tid, x)];
+            const bool ok = tap_inside<MASK>(at, q.bits, p.H, p.W) && (MASK || q.woff >= 0);
+            vp[x] = split::load_if(img + (base + q.off), ok);
+        }
+        const int w0 = tab[SQ::k(tid, 0)].woff, w1 = tab[SQ::k(tid, 0) + 1].woff;
+#pragma unroll
+        for (int u = 0; u < SQ::kUnits; ++u) {
+            const float* row = p.Wt + (long long)min(j0 + SQ::row(tid, u), p.OUTC - 1) * p.w_out;
+            vq[2 * u] = split::load_if(row + w0, w0 >= 0);
+            vq[2 * u + 1] = split::load_if(row + w1, w1 >= 0);
+        }
+    }
+    __device__ __forceinline__ bool covers(int row, int col) const { return i0 + row < pixels && j0 + col < p.OUTC; }
+    __device__ __noinline__ float plain(int row, int col, int blocks) const {
+        const float* image;
+        const Position where = input_of<MASK>(p, s, i0 + row, image);
+        float sum = 0.f;
+        for (int k = block0 * kBK; k < min(s.K, (block0 + blocks) * kBK); ++k) {
+            const TapK q = tap_of<MASK>(p, s, k);
+            const float x = tap_inside<MASK>(where, q.bits, p.H, p.W) ? image[where.h0 * p.W + where.w0 + q.off] : 0.f;
+            sum = fmaf(x, p.Wt[(long long)(j0 + col) * p.w_out + q.woff], sum);
+        }
+        return sum;
+    }
+    __device__ __forceinline__ void store(int row, int first, int n, uint32_t mine) const {
+        if (i0 + row >= pixels) return;
+        float* out;
+        const int place = output_of(p, s, i0 + row, out), plane = p.OHH * p.OWW, j = j0 + first;
+        const bool bias = p.ep.bias && part == 0;
+        store_columns(out + (long long)j * plane, plane, min(n, p.OUTC - j), mine,
+                      p.atomic_out ? !bias : !p.ep.scale && !p.ep.bias && !p.ep.relu, p.atomic_out || (p.ep.accumulate && !p.ep.relu && !p.ep.scale && !p.ep.bias),
+                      [&](int c, float y, const float* dst) {
+                          if (p.atomic_out) return y + p.ep.bias[j + c];
+                          return apply_epilogue(p.ep, y, j + c, (long long)(j + c) * plane + place, p.ep.accumulate ? *dst : 0.f);
+                      });
+    }
+};
+
+template <class S, bool MASK>
+__global__ void __launch_bounds__(S::NT, S::kCtas) conv_gather_split(const __grid_constant__ GatherParams p, int* status) {
+    extern __shared__ uint8_t smem[];
+    __shared__ split::Barriers bars;
+    __shared__ TapK table[S::kLoaders];
+    const int set = blockIdx.z / p.splits, part = blockIdx.z - set * p.splits;
+    const PixelSet& s = p.sets[set];
+    SplitGather<S, MASK> src{p, s, table, p.In, Position{-(1 << 29), 0, 0u}, 0, (long long)blockIdx.x * S::BM, (long long)p.N * s.UH * s.UW,
+                             (int)blockIdx.y * S::BN, part * p.per_split, part};
+    const int blocks = min(p.per_split, (s.K + kBK - 1) / kBK - src.block0);
+    // the grid is sized for the largest set; a share without a block has nothing to add, but a set without any product is still stored
+    if (src.i0 >= src.pixels || (blocks <= 0 && part > 0)) return;
+    const int tid = (int)threadIdx.x - 32 * S::kSumWarps;
+    if (tid >= 0) {
+        const long long i = src.i0 + split::ShareP<S, split::MN>::row(tid, 0);
+        if (i < src.pixels) {
+            src.at = input_of<MASK>(p, s, i, src.img);
+            src.base = src.at.h0 * p.W + src.at.w0;
+        }
+    }
+    split::run<S>(src, max(blocks, 1), smem, bars, nullptr, status);
+}
+
+// Weight gradient: rows are filter positions (ic, fh, fw), columns output channels, the contraction runs over the pixels.
+template <class S, bool MASK>
+struct SplitWgrad {
+    static constexpr split::Kind kP = split::K, kQ = split::K;
+    static constexpr bool kTable = true;
+    typedef split::ShareP<S, kP> SP;
+    typedef split::ShareQ<S, kQ> SQ;
+    const WgradParams& p;
+    PixelK* table;           // [kLoaders]
+    const TapI* rows;        // [BM]
+    int i0, j0, block0, opix;
+    __device__ __forceinline__ void prepare(int t, int tid) {
+        table[tid] = pixel_of<MASK>(p, (block0 + t) * kBK + tid);
+    }
+    __device__ __forceinline__ void load(int t, int tid, float (&vp)[SP::kValues], float (&vq)[SQ::kValues]) {
+        const PixelK* tab = table + t % (S::kLoaders / kBK) * kBK;
+        const PixelK q = tab[SP::k(tid, 0)];
+        const float* first = p.X + q.x;
+#pragma unroll
+        for (int x = 0; x < SP::kValues; ++x) {
+            const TapI w = rows[SP::row(tid, x)];
+            const bool ok = tap_inside<MASK>(q.at, w.bits, p.g.IH, p.g.IW) && (MASK || w.off >= 0);
+            vp[x] = split::load_if(first + w.off, ok);
+        }
+        const long long y0 = tab[SQ::k(tid, 0)].y, y1 = tab[SQ::k(tid, 0) + 1].y;
+#pragma unroll
+        for (int u = 0; u < SQ::kUnits; ++u) {
+            const float* row = p.dY + (long long)min(j0 + SQ::row(tid, u), p.g.OC - 1) * opix;
+            vq[2 * u] = split::load_if(row + y0, y0 >= 0);
+            vq[2 * u + 1] = split::load_if(row + y1, y1 >= 0);
+        }
+    }
+    __device__ __forceinline__ bool covers(int row, int col) const { return i0 + row < p.I && j0 + col < p.g.OC; }
+    __device__ __noinline__ float plain(int row, int col, int blocks) const {
+        const TapI w = row_of<MASK>(p, i0 + row);
+        float sum = 0.f;
+        for (int k = block0 * kBK; k < min(p.pixels, (block0 + blocks) * kBK); ++k) {
+            const PixelK q = pixel_of<MASK>(p, k);
+            const float x = tap_inside<MASK>(q.at, w.bits, p.g.IH, p.g.IW) ? p.X[q.x + w.off] : 0.f;
+            sum = fmaf(x, p.dY[q.y + (long long)(j0 + col) * opix], sum);
+        }
+        return sum;
+    }
+    __device__ __forceinline__ void store(int row, int first, int n, uint32_t mine) const {
+        const int i = i0 + row, j = j0 + first;
+        if (i >= p.I) return;
+        store_columns(p.dW + (long long)j * p.I + i, p.I, min(n, p.g.OC - j), mine, true, p.mode != 0, [](int, float y, const float*) { return y; });
+    }
+};
+
+template <class S, bool MASK>
+__global__ void __launch_bounds__(S::NT, S::kCtas) conv_wgrad_split(const __grid_constant__ WgradParams p, int* status) {
+    extern __shared__ uint8_t smem[];
+    __shared__ split::Barriers bars;
+    __shared__ float patches[split::ShareP<S, split::K>::kPatches];
+    __shared__ PixelK table[S::kLoaders];
+    __shared__ TapI rows[S::BM];
+    const int i0 = blockIdx.x * S::BM;
+    for (int e = threadIdx.x; e < S::BM; e += S::NT) rows[e] = row_of<MASK>(p, i0 + e);  // read behind the barrier of run()
+    SplitWgrad<S, MASK> src{p, table, rows, i0, (int)blockIdx.y * S::BN, (int)blockIdx.z * p.per_split, p.g.OH * p.g.OW};
+    split::run<S>(src, min(p.per_split, (p.pixels + kBK - 1) / kBK - src.block0), smem, bars, patches, status);
+}
+
+template <class F>
+cudaError_t with_shape(int bn, F f) {
+    return bn == 128 ? f(split::Shape<128>{}) : bn == 64 ? f(split::Shape<64>{}) : f(split::Shape<32>{});
+}
+
+}  // namespace
+
+cudaError_t launch_split_gather(cb_ctx* ctx, const GatherParams& p, const split::Choice& c, bool mask, long long pixels, int sets) {
+    return with_shape(c.bn, [&](auto shape) {
+        typedef decltype(shape) S;
+        auto kernel = mask ? conv_gather_split<S, true> : conv_gather_split<S, false>;
+        cudaError_t e = raise_dynamic_smem_once(kernel, ctx->device, ctx->max_smem_optin, nullptr);
+        if (e != cudaSuccess) return e;
+        const long long gx = (pixels + S::BM - 1) / S::BM, gy = (p.OUTC + S::BN - 1) / S::BN, gz = (long long)sets * c.splits;
+        if (gx > 0x7fffffffLL || gy > 65535 || gz > 65535) return cudaErrorInvalidConfiguration;
+        e = launch_dep(ctx, kernel, dim3((unsigned)gx, (unsigned)gy, (unsigned)gz), dim3(S::NT), (size_t)S::kSmem, p, ctx->d_status);
+        return e == cudaSuccess ? cudaGetLastError() : e;
+    });
+}
+
+cudaError_t launch_split_wgrad(cb_ctx* ctx, const WgradParams& p, const split::Choice& c, bool mask) {
+    return with_shape(c.bn, [&](auto shape) {
+        typedef decltype(shape) S;
+        auto kernel = mask ? conv_wgrad_split<S, true> : conv_wgrad_split<S, false>;
+        cudaError_t e = raise_dynamic_smem_once(kernel, ctx->device, ctx->max_smem_optin, nullptr);
+        if (e != cudaSuccess) return e;
+        const long long gx = (p.I + S::BM - 1) / S::BM, gy = (p.g.OC + S::BN - 1) / S::BN;
+        if (gy > 65535 || c.splits > 65535) return cudaErrorInvalidConfiguration;
+        e = launch_dep(ctx, kernel, dim3((unsigned)gx, (unsigned)gy, (unsigned)c.splits), dim3(S::NT), (size_t)S::kSmem, p, ctx->d_status);
+        return e == cudaSuccess ? cudaGetLastError() : e;
+    });
+}
+
+}  // namespace cb

@@ -293,7 +293,7 @@ static int gemm_zero_output(cb_ctx* ctx, const GemmCall& g) {
     return clear_output(ctx, g.C, g.out_mode == 0 ? g.I : g.J, g.ldc, g.out_mode == 0 ? g.J : g.I, g.strideC, g.batch, "clear of a split product");
 }
 
-int launch_simt_gemm(cb_ctx* ctx, const GemmCall& g_in) {
+static int launch_simt_gemm(cb_ctx* ctx, const GemmCall& g_in) {
     GemmCall g = g_in;
     if (g.J <= 16 && g.I > 16) {  // put the thin extent on the I side: D'[j][i] with the operands' roles swapped
         std::swap(g.I, g.J);
@@ -359,6 +359,16 @@ int launch_simt_gemm(cb_ctx* ctx, const GemmCall& g_in) {
     ctx->launches += 1;
     ctx->last_kernel = "simt_fp32";
     return CB_OK;
+}
+
+// Products of CB_MATH_FP32 and those TMA cannot address. In the passes of a model they stay on the CUDA cores: one rounding in an
+// activation moves the gradients of a deep model by percents, and a run could not be compared with one of an earlier version.
+int launch_fp32_gemm(cb_ctx* ctx, const GemmCall& g) {
+    if (!ctx->model_pass) {
+        const int rc = launch_split_gemm(ctx, g);
+        if (rc != CB_EUNSUPPORTED) return rc;
+    }
+    return launch_simt_gemm(ctx, g);
 }
 
 }  // namespace cb

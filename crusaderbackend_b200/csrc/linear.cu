@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(256) colsum_add_kernel(const float* __restrict
 
 int run_gemm(cb_ctx* ctx, const GemmCall& g) {
     if (ctx->math != CB_MATH_FP32 && umma_gemm_eligible(g)) return launch_umma_gemm(ctx, g, ctx->math == CB_MATH_3XTF32);
-    return launch_simt_gemm(ctx, g);
+    return launch_fp32_gemm(ctx, g);
 }
 
 }  // namespace

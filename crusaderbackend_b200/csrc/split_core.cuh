@@ -1,0 +1,414 @@
+// fp32 products on the tensor cores: D[i][j] = sum_k P(i, k) * Q(j, k) at the accuracy of fp32 FMAs, for CB_MATH_FP32 and for
+// operands the TMA-fed kernels cannot address, where the product is large enough to pay for it. One kernel body serves the GEMM
+// forms and the three convolution passes; an operand source (below) says where element (i, k) lies.
+//
+// Every fp32 value is the sum of three bf16 values: x = x1 + x2 + x3 with x1 = x cut off, x2 = x - x1 rounded, x3 the rest, all of it
+// exact (8 + 8 + 8 significant bits, the exponent range is that of fp32). Six of the nine products of two such sums leave out less
+// than 2^-23 of the product (x2 y3 + x3 y2, of either sign: x2 is rounded for that; 2^-26 on average): x2 y2, x1 y3, x3 y1, x1 y2,
+// x2 y1, x1 y1, issued smallest first. What the tensor
+// core does not give is fp32's rounding of sums (TMEM truncates every addition), so no chain of additions there is longer than two
+// k-blocks of 32: their sum is read back and added to the running total in a register, by ordinary fp32 additions.
+//
+// What bounds it: shared-memory bandwidth, were both operands read from there (a 128 x 128 x 16 UMMA reads 8 KB in its 64 clocks;
+// with the loaders' own accesses a k-block of 32 took 1800 clocks, 12 UMMAs 768). So the pieces of P go to TMEM, straight from the
+// registers they are formed in, and only those of Q to shared memory. fp32 FMAs would need 4096 clocks.
+//
+// Roles: loader warps (global memory -> registers, a block ahead -> pieces: P's in TMEM, 48 columns a stage, Q's as three bf16 tiles
+// of K-major rows of 64 bytes under the 64-byte swizzle) and summing warps, which own the output and of which the first issues
+// the UMMAs.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "cb_internal.h"
+#include "cb_ptx.cuh"
+
+namespace cb {
+namespace split {
+
+constexpr int kBK = 32;             // k of a block
+constexpr uint32_t kPieceRow = 64;  // bytes: 32 bf16
+constexpr int kAcc = 2;             // accumulators in TMEM
+constexpr int kStages = 4;
+constexpr int kChunk = 2;           // k-blocks a sum in TMEM runs over
+constexpr uint32_t kPCols = 48;     // TMEM columns of a stage of P: three pieces of 32 k, two a column
+
+// What a loader does is a chain of latencies (fetch, three dependent steps of a split, store, fences): with eight loader warps an SM a
+// block of 128 x 128 took 1780 clocks, 1550 of them the loaders'. With sixteen the CTA's registers no longer divide evenly, so the
+// summing warps take some of theirs (setmaxnreg; the shares add up to what the CTA is launched with).
+template <int BN_>
+struct Shape {
+    static constexpr int BM = 128, BN = BN_;
+    static constexpr int kLoaders = BN == 32 ? 256 : 512;  // loader threads
+    static constexpr int kSumWarps = BN == 32 ? 4 : 8;
+    static constexpr int kCols = BN / (kSumWarps / 4);     // columns a summing thread holds
+    static constexpr int NT = 32 * kSumWarps + kLoaders;
+    static constexpr int kCtas = BN == 32 ? 2 : 1;         // an SM
+    static constexpr int kSumRegs = 112, kLoaderRegs = 64; // of 80 at launch, where there are 768 threads
+    static_assert(NT != 768 || 32 * kSumWarps * kSumRegs + kLoaders * kLoaderRegs <= 80 * NT, "setmaxnreg would wait for ever");
+    static constexpr uint32_t kPieceQ = BN * kPieceRow, kStageBytes = 3 * kPieceQ;
+    static constexpr uint32_t kTmemCols = BN == 32 ? 256 : 512;
+    static constexpr int kSmem = kStages * (int)kStageBytes + 1024;
+    static_assert(kAcc * BN + kStages * kPCols <= kTmemCols && kStages * (int)kStageBytes >= BN * 512, "");
+};
+
+// How the loader threads share an operand's block of 32 k. P: warp w takes kValues k (part w / 4) of the 32 rows of TMEM lane quarter
+// w % 4, and must end up with one row a lane: at once where rows are contiguous in memory (MN), by way of a patch of shared memory
+// of its own where k is (K: a load is these k of a few rows). Q: MN: 8 k of one row; K: two neighbouring k of several rows; KV (k on
+// 16 bytes): 8 k of a row in two 16-byte loads.
+enum Kind { MN, K, KV };
+template <class S, Kind KIND>
+struct ShareP {
+    static_assert(KIND != KV, "");
+    static constexpr int kValues = S::BM * kBK / S::kLoaders;
+    static constexpr int kPatchRow = kValues + 1;                    // words: read by columns
+    static constexpr int kPatch = 32 * kPatchRow;                    // words of a warp
+    static constexpr int kPatches = KIND == K ? S::kLoaders / 32 * kPatch : 1;
+    // row and k of value x
+    static __device__ __forceinline__ int row(int tid, int x) {
+        return 32 * ((tid >> 5) & 3) + (KIND == MN ? (tid & 31) : (tid & 31) / kValues + 32 / kValues * x);
+    }
+    static __device__ __forceinline__ int k(int tid, int x) { return kValues * (tid >> 7) + (KIND == MN ? x : tid % kValues); }
+};
+template <class S, Kind KIND>
+struct ShareQ {
+    static constexpr int ROWS = S::BN, kLoaders = S::kLoaders;
+    static constexpr int kUnit = KIND == K ? 2 : 8;
+    static constexpr int kUnits = KIND == K ? ROWS * 16 / kLoaders : (ROWS * 4 >= kLoaders ? ROWS * 4 / kLoaders : 1);  // a thread's
+    static constexpr int kValues = kUnits * kUnit;
+    static __device__ __forceinline__ bool active(int tid) { return KIND == K || ROWS * 4 >= kLoaders || tid < ROWS * 4; }
+    static __device__ __forceinline__ int row(int tid, int u) {
+        if (KIND == MN) return tid % ROWS;
+        if (KIND == KV) return (tid >> 2) + kLoaders / 4 * u;
+        return (tid >> 4) + kLoaders / 16 * u;
+    }
+    static __device__ __forceinline__ int k(int tid, int u) {  // first of the unit's k
+        if (KIND == MN) return 8 * (tid / ROWS + u * (kLoaders / ROWS));
+        if (KIND == KV) return 8 * (tid & 3);
+        return 2 * (tid & 15);
+    }
+};
+
+// Pairs of fp32 in one instruction each: the loaders and the summing warps are bound by issue slots.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {  // a - b, exact where it is used
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(b), "l"(0xbf800000bf800000ull), "l"(a));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// (x0, x1) as three pairs of bf16, x0 in the low halves
+__device__ __forceinline__ void split2(float x0, float x1, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
+    const uint32_t a0 = __float_as_uint(x0), a1 = __float_as_uint(x1);
+    const uint64_t r = sub2(pack2(x0, x1), pack2(__uint_as_float(a0 & 0xffff0000u), __uint_as_float(a1 & 0xffff0000u)));
+    float r0, r1, c0, c1;
+    unpack2(r, r0, r1);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p2) : "f"(r1), "f"(r0));
+    unpack2(sub2(r, pack2(__uint_as_float(p2 << 16), __uint_as_float(p2 & 0xffff0000u))), c0, c1);
+    p1 = __byte_perm(a0, a1, 0x7632);
+    p3 = __byte_perm(__float_as_uint(c0), __float_as_uint(c1), 0x7632);
+}
+// Address of 16-byte chunk q of a row of a piece: the 64-byte swizzle exchanges chunks by bits 1 and 2 of the row.
+__device__ __forceinline__ uint32_t piece_chunk(uint32_t piece, int row, int q) {
+    return piece + (uint32_t)row * kPieceRow + (uint32_t)((q ^ (row >> 1)) & 3) * 16u;
+}
+// Splits a thread's values of Q's block and stores the pieces. Free of bank conflicts in all three kinds: eight lanes with
+// neighbouring rows and one chunk, or two rows and four chunks, cover 128 bytes.
+template <class Sh, Kind KIND>
+__device__ __forceinline__ void put_q(const float (&v)[ShareQ<Sh, KIND>::kValues], uint32_t pieces, int tid) {
+    typedef ShareQ<Sh, KIND> S;
+    constexpr uint32_t kPiece = Sh::kPieceQ;
+    if (!S::active(tid)) return;
+#pragma unroll
+    for (int u = 0; u < S::kUnits; ++u) {
+        const int row = S::row(tid, u), k = S::k(tid, u);
+        const uint32_t dst = piece_chunk(pieces, row, k >> 3) + (uint32_t)(k & 7) * 2u;
+        uint32_t p[3][4];
+#pragma unroll
+        for (int x = 0; x < S::kUnit; x += 2) split2(v[u * S::kUnit + x], v[u * S::kUnit + x + 1], p[0][x / 2], p[1][x / 2], p[2][x / 2]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            if (KIND == K) asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + i * kPiece), "r"(p[i][0]) : "memory");
+            else asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + i * kPiece), "r"(p[i][0]), "r"(p[i][1]), "r"(p[i][2]), "r"(p[i][3]) : "memory");
+        }
+    }
+}
+// The same for P, into the TMEM columns of a stage (`at`: this warp's lanes and part).
+template <class Sh, Kind KIND>
+__device__ __forceinline__ void put_p(float (&v)[ShareP<Sh, KIND>::kValues], uint32_t at, uint32_t patch, int lane) {
+    typedef ShareP<Sh, KIND> S;
+    constexpr int V = S::kValues;
+    if (KIND == K) {
+        const uint32_t mine = patch + (uint32_t)(lane / V * S::kPatchRow + lane % V) * 4u;
+#pragma unroll
+        for (int x = 0; x < V; ++x) asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + x * (32u / V * S::kPatchRow * 4u)), "f"(v[x]) : "memory");
+        __syncwarp();
+#pragma unroll
+        for (int x = 0; x < V; ++x) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[x]) : "r"(patch + (uint32_t)(lane * S::kPatchRow + x) * 4u) : "memory");
+        __syncwarp();
+    }
+    uint32_t p[3][V / 2];
+#pragma unroll
+    for (int x = 0; x < V; x += 2) split2(v[x], v[x + 1], p[0][x / 2], p[1][x / 2], p[2][x / 2]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) tmem_st(at + 16u * i, p[i]);
+    tmem_st_wait();
+}
+
+// base + n * stride in one instruction
+__device__ __forceinline__ const float* step(const float* base, uint32_t stride_bytes, uint32_t n) {
+    const float* r;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(stride_bytes), "r"(n), "l"(base));
+    return r;
+}
+
+// *src, or 0: one predicated load (a branch around each load cost more than the loads).
+__device__ __forceinline__ float load_if(const float* src, bool ok) {
+    float v;
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}" : "=f"(v) : "l"(src), "r"((int)ok));
+    return v;
+}
+
+// The loader threads alone (named barrier 1).
+template <class S>
+__device__ __forceinline__ void loader_sync() { asm volatile("bar.sync 1, %0;" ::"n"(S::kLoaders) : "memory"); }
+
+struct __align__(8) Barriers {
+    uint64_t full[kStages], empty[kStages], tfull[kAcc], tempty[kAcc], drain;
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+// Value of column c (of a summing thread's own) where it left its sums.
+__device__ __forceinline__ float staged(uint32_t mine, int c) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(mine + (uint32_t)c * 512u));
+    return v;
+}
+
+// The whole kernel behind its index arithmetic: `blocks` k-blocks of the tile through `src`.
+// Source: kP, kQ (Kind); prepare(t, tid), when kTable: entry tid of the table that load() of block t and the kLoaders / 32 - 1 after it
+// may read;
+// load(t, tid, p, q): this thread's values of block t; store(row, first, n, mine): outputs (row, first .. first + n - 1) of the tile,
+// to be read by staged(); covers(row, column), plain(row, column, blocks): whether the tile has the output, its value by fp32 FMAs.
+// patches: ShareP::kPatches floats of shared memory.
+template <class S, class Src>
+__device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Barriers& b, float* patches, int* status) {
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const uint32_t st_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    volatile int* abort_flag = &b.abort_flag;
+    if (threadIdx.x == 0) {
+        b.abort_flag = 0;
+        for (int s = 0; s < kStages; ++s) {
+            mbar_init(smem_u32(&b.full[s]), S::kLoaders / 32);
+            mbar_init(smem_u32(&b.empty[s]), 1);
+        }
+        for (int a = 0; a < kAcc; ++a) {
+            mbar_init(smem_u32(&b.tfull[a]), 1);
+            mbar_init(smem_u32(&b.tempty[a]), S::kSumWarps);
+        }
+        mbar_init(smem_u32(&b.drain), 1);
+        mbar_fence_init();
+    }
+    if (warp == 0) {
+        tmem_alloc(smem_u32(&b.tmem_base), S::kTmemCols);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    griddep_wait();
+    griddep_launch();
+    const uint32_t tmem_base = b.tmem_base;
+
+    if (warp >= S::kSumWarps) {
+        if (S::NT == 768) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(S::kLoaderRegs));
+        const int tid = (int)threadIdx.x - 32 * S::kSumWarps;
+        uint32_t s = 0, ph = 0;
+        typedef ShareP<S, Src::kP> SP;
+        typedef ShareQ<S, Src::kQ> SQ;
+        const uint32_t lw = (uint32_t)(warp - S::kSumWarps);
+        const uint32_t p_at = tmem_base + kAcc * S::BN + SP::kValues / 2u * (lw >> 2) + ((32u * (lw & 3u)) << 16);
+        const uint32_t patch = smem_u32(patches) + lw * (SP::kPatch * 4u);
+        auto store_block = [&](float (&vp)[SP::kValues], const float (&vq)[SQ::kValues]) {
+            if (!mbar_wait_uniform(smem_u32(&b.empty[s]), ph ^ 1u, abort_flag, status, CBK_TIMEOUT_EMPTY)) return false;
+            tc_fence_after();
+            put_q<S, Src::kQ>(vq, st_base + s * S::kStageBytes, tid);
+            put_p<S, Src::kP>(vp, p_at + s * kPCols, patch, lane);
+            fence_proxy_async_smem();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&b.full[s]));
+            if (++s == kStages) { s = 0; ph ^= 1u; }
+            return true;
+        };
+        // A table of the source serves kLoaders / 32 blocks, an entry a loader: its divisions would take longer than a block. A loader
+        // that gave up keeps to the barriers, so that none of the others waits there for it.
+        bool ok = true;
+        auto fetch = [&](int t, float (&vp)[SP::kValues], float (&vq)[SQ::kValues]) {
+            if (t >= blocks) return;
+            if (Src::kTable && t % (S::kLoaders / kBK) == 0) {
+                if (t) loader_sync<S>();
+                src.prepare(t, tid);
+                loader_sync<S>();
+            }
+            src.load(t, tid, vp, vq);
+        };
+        float p[2][SP::kValues], q[2][SQ::kValues];
+        fetch(0, p[0], q[0]);
+        for (int t = 0; t < blocks; t += 2) {
+            fetch(t + 1, p[1], q[1]);
+            ok = ok && store_block(p[0], q[0]);
+            fetch(t + 2, p[0], q[0]);
+            if (t + 1 < blocks) ok = ok && store_block(p[1], q[1]);
+        }
+    } else {
+        if (S::NT == 768) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(S::kSumRegs));
+        const int quarter = warp & 3, first = (warp >> 2) * S::kCols;
+        uint64_t sum[S::kCols / 2];
+#pragma unroll
+        for (int c = 0; c < S::kCols / 2; ++c) sum[c] = 0ull;
+        // Warp 0 issues too: chunk c + 1 before it adds chunk c, whose successor's UMMAs then run behind its additions.
+        uint32_t s = 0, ph = 0;
+        const int chunks = (blocks + kChunk - 1) / kChunk;
+        auto issue = [&](int c) {
+            const uint32_t a = (uint32_t)c % kAcc;
+            if (!mbar_wait_uniform(smem_u32(&b.tempty[a]), (((uint32_t)c / kAcc) & 1u) ^ 1u, abort_flag, status, CBK_TIMEOUT_TMEM_EMPTY)) return false;
+            const uint32_t d = tmem_base + a * S::BN, idesc = umma_idesc_bf16(128, (uint32_t)S::BN);
+            const int n = min(kChunk, blocks - c * kChunk);
+            for (int leading = 0; leading < 2; ++leading) {  // x1 y1 of the whole chunk comes last
+                uint32_t at = s;
+                for (int t = 0; t < n; ++t) {
+                    if (!leading && !mbar_wait_uniform(smem_u32(&b.full[at]), ph ^ (at < s ? 1u : 0u), abort_flag, status, CBK_TIMEOUT_FULL)) return false;
+                    tc_fence_after();
+                    const uint64_t dq = umma_smem_desc(st_base + at * S::kStageBytes, 16u, 512u, UMMA_SW_64B);
+                    const uint32_t dp = tmem_base + kAcc * S::BN + at * kPCols;
+                    // 16 k each: 8 columns, 32 bytes apart
+                    if (leading) {
+                        umma_bf16_ts_elect(d, dp, dq, idesc, 1u);
+                        umma_bf16_ts_elect(d, dp + 8u, dq + 2u, idesc, 1u);
+                        tc_commit_elect(smem_u32(&b.empty[at]));
+                    } else {
+                        constexpr int pp[5] = {1, 0, 2, 0, 1}, qq[5] = {1, 2, 0, 1, 0};
+#pragma unroll
+                        for (int x = 0; x < 5; ++x)
+#pragma unroll
+                            for (uint32_t ks = 0; ks < 2; ++ks)
+                                umma_bf16_ts_elect(d, dp + 16u * pp[x] + 8u * ks, dq + (uint64_t)((qq[x] * S::kPieceQ >> 4) + 2 * ks), idesc, t + x + ks ? 1u : 0u);
+                    }
+                    if (++at == kStages) at = 0;
+                }
+                if (leading) {
+                    if (at < s) ph ^= 1u;
+                    s = at;
+                }
+            }
+            tc_commit_elect(smem_u32(&b.tfull[a]));
+            return true;
+        };
+        bool ok = warp != 0 || issue(0);
+        for (int c = 0; c < chunks && ok; ++c) {
+            if (warp == 0 && c + 1 < chunks && !issue(c + 1)) { ok = false; break; }
+            const uint32_t a = (uint32_t)c % kAcc;
+            ok = mbar_wait_uniform(smem_u32(&b.tfull[a]), ((uint32_t)c / kAcc) & 1u, abort_flag, status, CBK_TIMEOUT_TMEM_FULL);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t at = tmem_base + a * S::BN + (uint32_t)first + ((uint32_t)(32 * quarter) << 16);
+#pragma unroll
+            for (int col = 0; col < S::kCols; col += 32) {
+                uint32_t v[32];
+                tmem_ld32(at + (uint32_t)col, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 32; e += 2)
+                    sum[(col + e) / 2] = add2(sum[(col + e) / 2], pack2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])));
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&b.tempty[a]));
+        }
+        if (ok) {
+            // Every UMMA has read its operands: the stages take the sums, so that what follows is a loop (unrolled over registers, its
+            // branches took longer to fetch than a small product to compute).
+            // A value the three pieces cannot carry (an infinity, a NaN) or a sum that left the range on the way shows as a result that is not finite: it is formed again by fp32 FMAs in k order.
+            const int row = 32 * quarter + lane;
+            const uint32_t mine = st_base + (uint32_t)(first * 128 + row) * 4u;
+            bool all = true;
+#pragma unroll
+            for (int c = 0; c < S::kCols; c += 2) {
+                float lo, hi;
+                unpack2(sum[c / 2], lo, hi);
+                all = all && fabsf(lo) <= 3.402823466e38f && fabsf(hi) <= 3.402823466e38f;
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + c * 512u), "f"(lo) : "memory");
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + c * 512u + 512u), "f"(hi) : "memory");
+            }
+            if (!all)
+                for (int c = 0; c < S::kCols; ++c)
+                    if (!(fabsf(staged(mine, c)) <= 3.402823466e38f) && src.covers(row, first + c))
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + c * 512u), "f"(src.plain(row, first + c, blocks)) : "memory");
+            src.store(row, first, S::kCols, mine);
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        if (b.abort_flag) {  // issued UMMAs may still run: a bounded chance to finish before TMEM and shared memory go
+            tc_commit_elect(smem_u32(&b.drain));
+            if (lane == 0) mbar_drain(smem_u32(&b.drain), 0, status);
+            __syncwarp();
+        }
+        tc_fence_after();
+        tmem_dealloc(tmem_base, S::kTmemCols);
+    }
+}
+
+// Whether a product comes here rather than to the CUDA cores. Contractions of less than 16: the rounding of a few fp32 FMAs is less
+// than what the six products leave out (2-norm error at K = 2: 1.8e-8 .. 3.4e-8 against 2.1e-8 .. 5.7e-8; at K = 16 7.5e-8 against
+// 5.4e-8, at 1501 3.5e-7 against 1.1e-7). Small products: bound by their launch on either path.
+inline bool worth_it(long long I, long long J, long long K, long long copies, long long least_fmas) {
+    return K >= 16 && (double)I * (double)J * (double)K * (double)copies >= (double)least_fmas;
+}
+
+// Columns of the CTA tile and how many CTAs share the contraction (their sums then meet in memory through atomic adds): the cheapest by
+// a model in SM clocks fitted to a sweep of all of them over 25 products, where it is within 5 % of the best everywhere (0.2 % on
+// average). block_scale: how much longer than a matrix's the loads of a block take.
+struct Choice {
+    int bn, splits, per_split;
+};
+inline Choice choose_shape(int sm_count, long long I, long long J, long long blocks, long long copies, bool may_split, double block_scale = 1.0) {
+    static const int bns[3] = {128, 64, 32};
+    static const int pieces[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128};
+    Choice best{64, 1, (int)blocks};
+    double best_cost = 1e300;
+    for (int bn : bns) {
+        const long long tiles = (I + 127) / 128 * ((J + bn - 1) / bn) * copies;
+        for (int want : pieces) {
+            if (want > 1 && (!may_split || blocks < 4LL * want || tiles * want > 16LL * sm_count)) break;
+            const long long per = (blocks + want - 1) / want, splits = (blocks + per - 1) / per, ctas = tiles * splits;
+            // two CTAs of 32 columns share an SM, and then take 1.6 times as long as one after the other would
+            const bool pairs = bn == 32 && ctas > sm_count;
+            const long long slots = pairs ? 2LL * sm_count : sm_count;
+            const double load = pairs ? 3.25 : 1.0, rounds = (double)((ctas + slots - 1) / slots);
+            double cost = rounds * (2650.0 + (double)per * (bn == 128 ? 900.0 : 870.0) * block_scale * load);
+            if (splits > 1) cost += rounds * 128.0 * bn / 6.2 * load + 2000.0;
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = Choice{bn, (int)splits, (int)per};
+            }
+        }
+    }
+    return best;
+}
+
+}  // namespace split
+}  // namespace cb

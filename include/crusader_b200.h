@@ -98,7 +98,7 @@ int cb_gemm_batch_reduce(cb_ctx* ctx, int transA, int transB, int M, int N, int 
 int cb_measure_umma_peak(cb_ctx* ctx, int n, int p_mn, int q_mn, int iters, float* tflops);
 
 /* Name of the kernel family the last cb_gemm / cb_conv_* call dispatched to ("umma_tf32",
- * "umma_3xtf32", "simt_fp32"); for tests and launch accounting. */
+ * "umma_3xtf32", "umma_fp32": fp32 accuracy on the tensor cores, "simt_fp32"); for tests and launch accounting. */
 const char* cb_last_kernel(const cb_ctx* ctx);
 
 /* ---- convolution (NCHW fp32) ------------------------------------------------------------------ */

@@ -1,0 +1,123 @@
+"""Products at fp32 accuracy on the tensor cores (three bf16 values a factor) against the fp64 CPU oracle.
+
+Tolerance: that of the fp32 CUDA-core kernels, 2e-6 of max|c - c64| / max|c64|. The six products leave out 2^-26 of a term on
+average, a chain of 64 k in the tensor core is truncated by four additions (4 x 2^-24 of the chain), the chains are added in fp32.
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+TOL = 2e-6
+FORMS = {"NN": (False, False), "NT": (False, True), "TN": (True, False), "TT": (True, True)}
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import torch
+    assert torch.cuda.is_available(), "GPU tests need a CUDA device"
+    from crusaderbackend_b200.api import Context
+    c = Context(0, math="fp32", sync=True)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("M,N,K", [(130, 1030, 130), (129, 65, 2049), (2049, 130, 64), (1000, 17, 1000), (127, 2049, 65), (33, 512, 1024), (1500, 1400, 95)])
+@pytest.mark.parametrize("pad", [0, 1, 4])
+def test_product(ctx, M, N, K, form, pad):
+    """Tiles of 128 x 128, 64 and 32 and blocks of 32 k one element below, at and above their sizes; rows on 16 bytes and not;
+    contraction whole (deterministic context) or split; overwrite and accumulate; what lies between the rows of C stays."""
+    import torch
+    tA, tB = FORMS[form]
+    A = orc.uniform_pm1((K, M + pad) if tA else (M, K + pad), "split", M, N, K, "A")
+    B = orc.uniform_pm1((N, K + pad) if tB else (K, N + pad), "split", M, N, K, "B")
+    a, b = A[:, :M if tA else K], B[:, :K if tB else N]
+    ref = orc.gemm_f64(np.ascontiguousarray(a), np.ascontiguousarray(b), tA, tB)
+    dA, dB = torch.from_numpy(A).cuda()[:, :a.shape[1]], torch.from_numpy(B).cuda()[:, :b.shape[1]]
+    whole = torch.full((M, N + 3), 7.0, device="cuda")
+    for det in (False, True):
+        ctx.set_deterministic(det)
+        ctx.gemm(dA, dB, whole[:, :N], transA=tA, transB=tB)
+        assert ctx.last_kernel == "umma_fp32"
+        assert orc.max_err_norm(whole[:, :N].cpu().numpy(), ref) <= TOL
+        ctx.gemm(dA, dB, whole[:, :N], transA=tA, transB=tB, accumulate=True)
+        assert orc.max_err_norm(whole[:, :N].cpu().numpy(), 2 * ref) <= TOL
+        ctx.set_deterministic(False)
+    assert bool((whole[:, N:] == 7).all())
+
+
+def test_batches_and_dense_layers(ctx):
+    import torch
+    A, B = orc.uniform_pm1((150, 99), "split", "sA"), orc.uniform_pm1((9, 99, 131), "split", "sB")
+    C = torch.zeros(9, 150, 131, device="cuda")
+    ctx.sgemm(torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda(), C)
+    assert ctx.last_kernel == "umma_fp32"
+    assert orc.max_err_norm(C.cpu().numpy(), np.stack([orc.gemm_f64(A, x) for x in B])) <= TOL
+    A, B = orc.uniform_pm1((7, 130, 225), "split", "fA"), orc.uniform_pm1((7, 101, 225), "split", "fB")
+    C = torch.zeros(130, 101, device="cuda")
+    ctx.sgemmNTA(torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda(), C)
+    assert ctx.last_kernel == "umma_fp32"
+    assert orc.max_err_norm(C.cpu().numpy(), sum(orc.gemm_f64(x, y, False, True) for x, y in zip(A, B))) <= TOL
+    X, W, b, dY = (orc.normal(s, "split", "lin", i) for i, s in enumerate([(130, 777), (200, 777), (200,), (130, 200)]))
+    tX, tW, tb, tdY = (torch.from_numpy(v).cuda() for v in (X, W, b, dY))
+    Y, dX, dW, db = torch.zeros(130, 200, device="cuda"), torch.zeros(130, 777, device="cuda"), torch.zeros(200, 777, device="cuda"), torch.zeros(200, device="cuda")
+    ctx.linear(tX, tW, tb, Y)
+    assert ctx.last_kernel == "umma_fp32"
+    assert orc.max_err_norm(Y.cpu().numpy(), X.astype(np.float64) @ W.T + b) <= TOL
+    ctx.linearXGrad(tdY, tW, dX)
+    ctx.linearParamGrad(tdY, tX, dW, db)
+    assert orc.max_err_norm(dX.cpu().numpy(), dY.astype(np.float64) @ W) <= TOL
+    assert orc.max_err_norm(dW.cpu().numpy(), dY.T.astype(np.float64) @ X) <= TOL
+
+
+def test_values_the_pieces_cannot_carry(ctx):
+    """Infinities, NaNs and sums that leave the range: such outputs are formed again by fp32 FMAs. Values down to where the last
+    piece is a bf16 subnormal keep their accuracy."""
+    import torch
+    A, B = orc.uniform_pm1((300, 200), "split", "nA"), orc.uniform_pm1((200, 300), "split", "nB")
+    A[3, 5], A[9, 2], A[100, 1], B[7, 11] = np.inf, np.nan, 3.4e38, -np.inf
+    C = torch.zeros(300, 300, device="cuda")
+    ctx.gemm(torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda(), C)
+    assert ctx.last_kernel == "umma_fp32"
+    got = C.cpu().numpy()
+    with np.errstate(invalid="ignore", over="ignore"):
+        want = np.zeros((300, 300), np.float32)
+        for k in range(200):
+            want = want + A[:, k:k + 1] * B[k:k + 1]
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
+    rows, cols = np.setdiff1d(np.arange(300), [3, 9, 100]), np.setdiff1d(np.arange(300), [11])
+    plain = orc.gemm_f64(np.ascontiguousarray(A[rows]), np.ascontiguousarray(B[:, cols]))
+    assert orc.max_err_norm(got[np.ix_(rows, cols)], plain) <= TOL
+    for sa, sb in [(1e-30, 1.0), (3e38, 1e-3), (1e-25, 1e-10)]:
+        A, B = (orc.uniform_pm1((300, 200), "split", "tA") * sa).astype(np.float32), (orc.uniform_pm1((200, 300), "split", "tB") * sb).astype(np.float32)
+        ctx.gemm(torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda(), C)
+        assert orc.max_err_norm(C.cpu().numpy(), orc.gemm_f64(A, B)) <= TOL, (sa, sb)
+
+
+@pytest.mark.parametrize("geo", [(9, 17, 28, 28, 33, 3, 1, 1), (3, 16, 31, 45, 64, 3, 2, 1), (2, 40, 21, 23, 70, 5, 1, 2), (40, 64, 9, 9, 130, 1, 1, 0),
+                                 (2, 16, 45, 44, 20, 17, 1, 8), (33, 20, 13, 13, 100, 3, 3, 1), (5, 130, 14, 14, 31, 3, 1, 1)])
+@pytest.mark.parametrize("det", [False, True])
+def test_convolution(ctx, geo, det):
+    """All passes with odd maps, channels around the tiles, strides whose phases have different taps, and filters on both sides of
+    the 15-tap limit of the tap masks; a bias, an accumulating weight gradient, an accumulating data gradient."""
+    import torch
+    N, IC, H, W_, OC, F, s, p = geo
+    OH, OW = orc.conv_out_hw(H, W_, F, F, s, s, p, p)
+    W, X, dY = orc.he_normal_filter(OC, IC, F, F, ("split", geo)), orc.normal((N, IC, H, W_), "split", geo, "X"), orc.normal((N, OC, OH, OW), "split", geo, "dY")
+    bias, dW0 = orc.normal((OC,), "split", geo, "b"), orc.normal((OC, IC, F, F), "split", geo, "dW0")
+    tW, tX, tdY, tb = (torch.from_numpy(v).cuda() for v in (W, X, dY, bias))
+    Y, dX, dW = torch.full_like(tdY, float("nan")), torch.full_like(tX, float("nan")), torch.from_numpy(dW0).cuda()
+    ctx.set_deterministic(det)
+    kern = []
+    for call in (lambda: ctx.conv(tW, tX, Y, s, s, p, p, tb), lambda: ctx.convDerive(tW, tdY, dX, s, s, p, p),
+                 lambda: ctx.convError(tdY, tX, dW, s, s, p, p)):
+        call()
+        kern.append(ctx.last_kernel)
+    ctx.set_deterministic(False)
+    assert kern == ["umma_fp32"] * 3
+    assert orc.max_err_norm(Y.cpu().numpy(), orc.conv_fwd(W, X, bias, (s, s), (p, p))) <= TOL
+    assert orc.max_err_norm(dX.cpu().numpy(), orc.conv_dgrad(W, dY, X.shape, (s, s), (p, p))) <= TOL
+    assert orc.max_err_norm(dW.cpu().numpy(), orc.conv_wgrad(dY, X, W.shape, (s, s), (p, p), dW_init=dW0)) <= TOL
