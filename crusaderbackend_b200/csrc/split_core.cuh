@@ -380,8 +380,9 @@ inline bool worth_it(long long I, long long J, long long K, long long copies, lo
 }
 
 // Columns of the CTA tile and how many CTAs share the contraction (their sums then meet in memory through atomic adds): the cheapest by
-// a model in SM clocks fitted to a sweep of all of them over 25 products, where it is within 5 % of the best everywhere (0.2 % on
-// average). block_scale: how much longer than a matrix's the loads of a block take.
+// a model in SM clocks fitted to a sweep of all of them over 25 products and 48 convolution passes, where what it takes is 2 % from
+// the best on average (24 % at most, 99 x 4001 x 399). block_scale: how much longer a block takes than that of a matrix
+// (convolutions: 1.9 for the gathers, 2.5 for the weight gradient).
 struct Choice {
     int bn, splits, per_split;
 };
@@ -393,14 +394,14 @@ inline Choice choose_shape(int sm_count, long long I, long long J, long long blo
     for (int bn : bns) {
         const long long tiles = (I + 127) / 128 * ((J + bn - 1) / bn) * copies;
         for (int want : pieces) {
-            if (want > 1 && (!may_split || blocks < 4LL * want || tiles * want > 16LL * sm_count)) break;
+            if (want > 1 && (!may_split || blocks < 2LL * want || tiles * want > 16LL * sm_count)) break;
             const long long per = (blocks + want - 1) / want, splits = (blocks + per - 1) / per, ctas = tiles * splits;
-            // two CTAs of 32 columns share an SM, and then take 1.6 times as long as one after the other would
+            // two CTAs of 32 columns share an SM, a block of both takes 1.8 times one's
             const bool pairs = bn == 32 && ctas > sm_count;
             const long long slots = pairs ? 2LL * sm_count : sm_count;
-            const double load = pairs ? 3.25 : 1.0, rounds = (double)((ctas + slots - 1) / slots);
-            double cost = rounds * (2650.0 + (double)per * (bn == 128 ? 900.0 : 870.0) * block_scale * load);
-            if (splits > 1) cost += rounds * 128.0 * bn / 6.2 * load + 2000.0;
+            const double load = pairs ? 1.77 : 1.0, rounds = (double)((ctas + slots - 1) / slots);
+            double cost = rounds * (2300.0 + (double)per * (bn == 128 ? 690.0 : bn == 64 ? 630.0 : 440.0) * block_scale * load);
+            if (splits > 1) cost += rounds * 128.0 * bn / 3.94 * load + 1030.0;
             if (cost < best_cost) {
                 best_cost = cost;
                 best = Choice{bn, (int)splits, (int)per};
