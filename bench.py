@@ -394,8 +394,8 @@ def resnet56_3xtf32_section(torch, local):
     tr.close()
     ctx.close()
     return {"ms_per_step": round(ms, 3), "images_per_s": round(GLOBAL_BATCH / ms * 1e3, 1),
-            "note": "3xTF32: convolutions in one tensor-core pass over [x_lo; x; x] x [w; w_lo; w], three passes where the filter "
-                    "needs a four-way split of the output channels on a large map"}
+            "note": "3xTF32: convolutions in one tensor-core pass over [x_lo; x; x] x [w; w_lo; w]; filters that pass does not take run "
+                    "at fp32 accuracy on the tensor cores"}
 
 
 def densenet_section(torch, local):

@@ -180,6 +180,7 @@ int umma_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const C
 int umma_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, int N, int IC, int IH, int IW, int OC,
                     int FH, int FW, int sH, int sW, int pH, int pW, int accumulate, long long dy_batch, long long x_batch,
                     bool x3 = false);
+int umma_wgrad_launches(int IC, int OC, int FH, int FW);  // of a stride-1 layer
 // Packed-filter cache of a context (conv_sm100.cu).
 int filter_cache_repack_all(cb_ctx* ctx);
 bool filter_cache_fresh(const cb_ctx* ctx);  // no convolution would re-pack a filter it has seen before

@@ -182,10 +182,10 @@ __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_wgrad_simt(const Wgra
 constexpr long long kLeastConv = 1LL << 22;
 
 // One launch for up to four pixel sets. In the passes of a model the two that later layers read stay on the CUDA cores (see
-// launch_fp32_gemm). The contraction is split over CTAs where the output alone does not fill the GPU and the
+// launch_fp32_gemm), except the 3xTF32 ones that never ran there (in_models). The contraction is split over CTAs where the output alone does not fill the GPU and the
 // epilogue is a plain sum (the output is then cleared first), except in the passes of a model: atomic sums come in any order, and
 // one rounding more or less in an activation moves the gradients of a deep model by percents from one run to the next.
-int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, const char* who) {
+int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, bool in_models, const char* who) {
     const long long out_elems = (long long)p.OUTC * p.OHH * p.OWW;
     if ((long long)p.C * p.H * p.W >= (1LL << 29) || out_elems >= (1LL << 31) || (long long)p.C * p.w_ch >= (1LL << 31))
         return fail(ctx, CB_EUNSUPPORTED, std::string(who) + ": an image or filter of more than 2^29 values");
@@ -193,7 +193,7 @@ int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, 
     int most = 0;
     for (int i = 0; i < nsets; ++i) most = sets[i].K > most ? sets[i].K : most;
     const long long I = (long long)p.N * sets[0].UH * sets[0].UW * nsets;
-    const bool on_tensor_cores = !ctx->model_pass && split::worth_it(I, p.OUTC, most, 1, kLeastConv);
+    const bool on_tensor_cores = (!ctx->model_pass || in_models) && split::worth_it(I, p.OUTC, most, 1, kLeastConv);
     simt::Choice c{};
     split::Choice sc{};
     if (on_tensor_cores) sc = split::choose_shape(ctx->sm_count, I, p.OUTC, (most + split::kBK - 1) / split::kBK, 1, may_split, 1.9);
@@ -233,17 +233,17 @@ int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, 
     return CB_OK;
 }
 
-int simt_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const ConvGeo& g, const ConvEpilogue& ep, const char* who) {
+int fp32_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const ConvGeo& g, const ConvEpilogue& ep, bool in_models, const char* who) {
     GatherParams p{};
     p.In = X; p.in_batch = g.x_batch; p.C = g.IC; p.H = g.IH; p.W = g.IW;
     p.Wt = W; p.w_ch = g.FH * g.FW; p.w_out = g.IC * g.FH * g.FW; p.FW = g.FW;
     p.Out = Y; p.out_batch = g.y_batch; p.OUTC = g.OC; p.OHH = g.OH; p.OWW = g.OW;
     p.N = g.N; p.sgn = 1; p.ep = ep;
     const PixelSet s{g.OH, g.OW, g.sH, -g.pH, g.sW, -g.pW, 0, 1, 0, 1, g.FH, g.FW, 0, 1, 0, 1, g.IC * g.FH * g.FW};
-    return launch_gather(ctx, p, &s, 1, who);
+    return launch_gather(ctx, p, &s, 1, in_models, who);
 }
 
-int simt_conv_dgrad(cb_ctx* ctx, const float* W, const float* dY, float* dX, const ConvGeo& g, int accumulate, const char* who) {
+int fp32_conv_dgrad(cb_ctx* ctx, const float* W, const float* dY, float* dX, const ConvGeo& g, int accumulate, bool in_models, const char* who) {
     GatherParams p{};
     p.In = dY; p.in_batch = g.y_batch; p.C = g.OC; p.H = g.OH; p.W = g.OW;
     p.Wt = W; p.w_ch = g.IC * g.FH * g.FW; p.w_out = g.FH * g.FW; p.FW = g.FW;
@@ -265,10 +265,10 @@ int simt_conv_dgrad(cb_ctx* ctx, const float* W, const float* dY, float* dX, con
             s.K = g.OC * s.TH * s.TW;
             sets.push_back(s);
         }
-    return launch_gather(ctx, p, sets.data(), (int)sets.size(), who);
+    return launch_gather(ctx, p, sets.data(), (int)sets.size(), in_models, who);
 }
 
-int simt_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, const ConvGeo& g, int accumulate, const char* who) {
+int fp32_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, const ConvGeo& g, int accumulate, const char* who) {
     WgradParams p{};
     p.X = X; p.dY = dY; p.dW = dW; p.g = g;
     const long long I = (long long)g.IC * g.FH * g.FW, pixels = (long long)g.N * g.OH * g.OW;
@@ -276,7 +276,9 @@ int simt_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, con
         return fail(ctx, CB_EUNSUPPORTED, std::string(who) + ": more than 2^31 pixels or filter values");
     const bool mask = g.FH <= kMaskTaps && g.FW <= kMaskTaps;
     p.I = (int)I; p.pixels = (int)pixels;
-    const bool on_tensor_cores = split::worth_it(I, g.OC, pixels, 1, kLeastConv);
+    // a CTA of conv_wgrad_split holds an SM, which a stream beside this one would miss (ResNet-50 on 16 x 16 images, batch 78: 2300 us
+    // a step against 2263)
+    const bool on_tensor_cores = ctx->wgrad_grid_cap == 0 && split::worth_it(I, g.OC, pixels, 1, kLeastConv);
     simt::Choice c{};
     split::Choice sc{};
     if (on_tensor_cores) sc = split::choose_shape(ctx->sm_count, I, g.OC, (pixels + split::kBK - 1) / split::kBK, 1, !ctx->deterministic, 2.5);
@@ -319,91 +321,27 @@ int make_geo(cb_ctx* ctx, ConvGeo& g, int N, int IC, int IH, int IW, int OC, int
     return CB_OK;
 }
 
-// ---- 3xTF32 composition: x = hi + lo with hi = the 19 bits the tensor core reads, lo = rna_tf32(x - hi).
-// lo[n][i] = lo part of x[n*x_batch + i], written densely (per elements per image)
-__global__ void tf32_lo_kernel(const float* __restrict__ x, float* __restrict__ lo, long long n, long long per,
-                               long long x_batch) {
-    griddep_wait();
-    griddep_launch();
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const long long img = i / per;
-        const float v = x[img * x_batch + (i - img * per)];
-        const float hi = __uint_as_float(__float_as_uint(v) & 0xFFFFE000u);
-        uint32_t r;
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v - hi));
-        lo[i] = __uint_as_float(r);
-    }
-}
-// out = epilogue((a + b) + c): the sum of the three tensor-core passes (the two small cross terms first), dense
-// temporaries in, (possibly strided) output tensor out
-__global__ void sum3_kernel(float* __restrict__ out, const float* __restrict__ lead, const float* __restrict__ a,
-                            const float* __restrict__ b, const ConvEpilogue ep, long long n, long long per, long long plane,
-                            long long out_batch) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const long long img = i / per, r = i - img * per;
-        float* dst = out + img * out_batch + r;
-        const float v = (a[i] + b[i]) + lead[i];
-        *dst = apply_epilogue(ep, v, (int)(r / plane), r, ep.accumulate ? *dst : 0.f);
-    }
-}
-
-int grid_el(const cb_ctx* ctx, long long n) {
-    long long g = (n + 255) / 256;
-    const long long cap = (long long)ctx->sm_count * 16;
-    return (int)(g > cap ? cap : (g < 1 ? 1 : g));
-}
-
 }  // namespace
-
-// 3xTF32 forward / data gradient on the tensor cores: out = pass(W_hi, In_lo) + pass(W_lo, In_hi) + pass(W_hi, In_hi),
-// where every pass is the TF32 kernel (it reads the hi parts by truncation). The dropped lo*lo term is < 2^-20 relative.
-// Scratch (workspace3): In_lo, W_lo and the three partial outputs, all densely packed; the last kernel adds them and
-// applies the epilogue while writing the caller's output. Returns CB_EUNSUPPORTED when the TF32 kernel does not cover the
-// geometry, before any work was queued.
-static int conv_3xtf32(cb_ctx* ctx, const float* W, const float* In, float* Out, const ConvEpilogue& ep, int N, int IC,
-                       int IH, int IW, int OC, int FH, int FW, int sH, int sW, int pH, int pW, bool dgrad_of,
-                       long long in_per, long long out_per, long long out_plane, long long in_batch, long long out_batch) {
-    // one pass of the tensor-core kernel over three channel groups, when the doubled filter fits
-    const int rc1 = umma_conv_fwd(ctx, W, In, Out, ep, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, dgrad_of, in_batch, out_batch, true);
-    if (rc1 != CB_EUNSUPPORTED) return rc1;
-    const long long w_elems = (long long)OC * IC * FH * FW;
-    const long long in_elems = in_per * N, out_elems = out_per * N;
-    auto up = [](long long n) { return (n + 63) & ~63LL; };
-    const size_t need = (size_t)(up(in_elems) + up(w_elems) + 3 * up(out_elems)) * sizeof(float);
-    int rc = ensure_workspace3(ctx, need);
-    if (rc != CB_OK) return rc;
-    float* in_lo = static_cast<float*>(ctx->workspace3);
-    float* w_lo = in_lo + up(in_elems);
-    float* t0 = w_lo + up(w_elems);
-    float* t1 = t0 + up(out_elems);
-    float* t2 = t1 + up(out_elems);
-    const ConvEpilogue plain{};
-    // leading term first: it also tells whether the geometry is covered
-    rc = umma_conv_fwd(ctx, W, In, t0, plain, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, dgrad_of, in_batch, 0);
-    if (rc != CB_OK) return rc;
-    tf32_lo_kernel<<<grid_el(ctx, in_elems), 256, 0, ctx->stream>>>(In, in_lo, in_elems, in_per, in_batch ? in_batch : in_per);
-    tf32_lo_kernel<<<grid_el(ctx, w_elems), 256, 0, ctx->stream>>>(W, w_lo, w_elems, w_elems, w_elems);
-    rc = umma_conv_fwd(ctx, W, in_lo, t1, plain, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, dgrad_of, 0, 0);
-    if (rc == CB_OK) {
-        // w_lo is a temporary whose address recurs with different contents: it must not enter the packed-filter cache
-        const int cache_on = ctx->filter_cache_on;
-        ctx->filter_cache_on = 0;
-        rc = umma_conv_fwd(ctx, w_lo, In, t2, plain, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, dgrad_of, in_batch, 0);
-        ctx->filter_cache_on = cache_on;
-    }
-    if (rc != CB_OK) return rc;
-    sum3_kernel<<<grid_el(ctx, out_elems), 256, 0, ctx->stream>>>(Out, t0, t1, t2, ep, out_elems, out_per, out_plane,
-                                                                 out_batch ? out_batch : out_per);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return check_cuda(ctx, e, "3xTF32 convolution");
-    ctx->launches += 3;
-    ctx->last_kernel = "umma_3xtf32";
-    return CB_OK;
-}
 
 }  // namespace cb
 
 using namespace cb;
+
+// Whether the TF32 kernels take the maps' width. Filters their one-pass 3xTF32 form does not take run at fp32 accuracy on the tensor
+// cores, in models too: three TF32 passes into temporaries took 137 us where that takes 14 (64 -> 128, stride 2, 64 maps of 16 x 16),
+// 41 against 11 (96 -> 96, 9 of 16 x 16).
+static bool tf32_width(const ConvGeo& g) {
+    const int w = g.sW == 2 ? g.IW / 2 : g.IW;
+    return g.FH <= 3 && g.FW <= 3 && (w == 8 || w == 16 || w == 32);
+}
+// Stride-2 3x3 layers of 3xTF32 whose forward pass and weight gradient run at fp32 accuracy: the one-pass form pays for a phase split and
+// lo parts through memory. Forward, then weight gradient, us, one pass / fp32: 32 -> 64 at 32 x 32, batch 128: 38 / 23, 34 / 30; 64 -> 32, batch 118:
+// 72 / 27, 44 / 34 (data gradient 31 / 38 and 38 / 52: stays). Below 2^27 multiplications both are a few launches, 10 to 14 us against 6 to 10.
+static bool x3_at_fp32(const ConvGeo& g) {
+    if ((double)g.N * g.OH * g.OW >= (double)(1LL << 30) || (double)g.IC * g.IH * g.IW >= (double)(1LL << 28) || (double)g.OC * g.OH * g.OW >= (double)(1LL << 28))
+        return false;  // 32-bit indexes
+    return g.sH == 2 && g.sW == 2 && g.FH == 3 && g.FW == 3 && (double)g.N * g.OH * g.OW * g.OC * g.IC * 9.0 >= (double)(1LL << 27);
+}
 
 static int conv_fwd_impl(cb_ctx* ctx, const float* W, const float* X, float* Y, int N, int IC, int IH, int IW, int OC, int FH,
                          int FW, int sH, int sW, int pH, int pW, const cb_epilogue* cep, const char* who) {
@@ -422,15 +360,12 @@ static int conv_fwd_impl(cb_ctx* ctx, const float* W, const float* X, float* Y, 
     const long long npix = (long long)N * g.OH * g.OW;
     if (npix == 0 || OC == 0) return CB_OK;
     if (!W || !X || !Y) return fail(ctx, CB_EINVAL, std::string(who) + ": null operand");
-    if (ctx->math == CB_MATH_TF32) {  // tensor cores; 3xTF32: conv_3xtf32; FP32 and uncovered geometries: CUDA cores
-        rc = umma_conv_fwd(ctx, W, X, Y, ep, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, false, xb, yb);
-        if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;
-    } else if (ctx->math == CB_MATH_3XTF32) {
-        rc = conv_3xtf32(ctx, W, X, Y, ep, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, false, (long long)IC * IH * IW,
-                         (long long)OC * g.OH * g.OW, (long long)g.OH * g.OW, xb, yb);
+    const bool x3 = ctx->math == CB_MATH_3XTF32;
+    if (ctx->math != CB_MATH_FP32 && !(x3 && !ctx->model_pass && x3_at_fp32(g))) {
+        rc = umma_conv_fwd(ctx, W, X, Y, ep, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, false, xb, yb, x3);
         if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;
     }
-    rc = simt_conv_fwd(ctx, W, X, Y, g, ep, who);
+    rc = fp32_conv_fwd(ctx, W, X, Y, g, ep, x3 && tf32_width(g), who);
     return rc == CB_OK ? finish(ctx, who) : rc;
 }
 
@@ -446,15 +381,12 @@ static int conv_dgrad_impl(cb_ctx* ctx, const float* W, const float* dY, float* 
     if (!W || !dY || !dX) return fail(ctx, CB_EINVAL, std::string(who) + ": null operand");
     ConvEpilogue ep{};
     ep.accumulate = accumulate ? 1 : 0;
-    if (ctx->math == CB_MATH_TF32) {
-        rc = umma_conv_fwd(ctx, W, dY, dX, ep, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, true, dy_batch, dx_batch);
-        if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;
-    } else if (ctx->math == CB_MATH_3XTF32) {
-        rc = conv_3xtf32(ctx, W, dY, dX, ep, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, true, (long long)OC * g.OH * g.OW,
-                         (long long)IC * IH * IW, (long long)IH * IW, dy_batch, dx_batch);
+    const bool x3 = ctx->math == CB_MATH_3XTF32;
+    if (ctx->math != CB_MATH_FP32) {
+        rc = umma_conv_fwd(ctx, W, dY, dX, ep, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, true, dy_batch, dx_batch, x3);
         if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;
     }
-    rc = simt_conv_dgrad(ctx, W, dY, dX, g, accumulate ? 1 : 0, who);
+    rc = fp32_conv_dgrad(ctx, W, dY, dX, g, accumulate ? 1 : 0, x3 && tf32_width(g), who);
     return rc == CB_OK ? finish(ctx, who) : rc;
 }
 
@@ -500,6 +432,16 @@ int cb_filters_changed(cb_ctx* ctx) {
 
 }  // extern "C"
 
+// Weight gradients that the TF32 kernel would cut into several launches (filters beyond its accumulator) run in one at fp32 accuracy
+// where that takes less: 6 us + 45 us for 10^9 multiplications against 6.5 us a launch (TF32) or 8 us and 9 for the lo parts (3xTF32).
+// 128 -> 128 3x3, 4 maps of 16 x 16: 25.9 us TF32, 32.5 3xTF32, 7.9 here; 330 -> 48 1x1, 64 of 8 x 8: 14.6 TF32, 7.9 here;
+// 288 -> 48 1x1, 64 of 16 x 16: 14.1 TF32, 18.0 here.
+static bool wgrad_at_fp32(const ConvGeo& g, bool x3) {
+    const int launches = umma_wgrad_launches(g.IC, g.OC, g.FH, g.FW);
+    const double fmas = (double)g.N * g.OH * g.OW * g.OC * g.IC * g.FH * g.FW;
+    return g.sH == 1 && g.sW == 1 && launches > 1 && fmas >= (double)kLeastConv && 6.0 + 45e-9 * fmas < (x3 ? 9.0 + 8.0 * launches : 6.5 * launches);
+}
+
 static int conv_wgrad_impl(cb_ctx* ctx, const float* dY, const float* X, float* dW, int N, int IC, int IH, int IW, int OC,
                            int FH, int FW, int sH, int sW, int pH, int pW, int accumulate, long long dy_batch, long long x_batch,
                            const char* who) {
@@ -518,16 +460,16 @@ static int conv_wgrad_impl(cb_ctx* ctx, const float* dY, const float* X, float* 
         return finish(ctx, who);
     }
     if (!dY || !X) return fail(ctx, CB_EINVAL, std::string(who) + ": null operand");
-    if (ctx->math == CB_MATH_TF32) {
-        rc = umma_conv_wgrad(ctx, dY, X, dW, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, accumulate, dy_batch, x_batch);
-        if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;
-    } else if (ctx->math == CB_MATH_3XTF32) {
-        // the products dY_hi X_hi, dY_hi X_lo, dY_lo X_hi in one launch that walks the pixels three times
-        rc = umma_conv_wgrad(ctx, dY, X, dW, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, accumulate, dy_batch, x_batch, true);
-        if (rc == CB_OK) ctx->last_kernel = "umma_3xtf32";
+    // 3xTF32: the products dY_hi X_hi, dY_hi X_lo, dY_lo X_hi in one launch that walks the pixels three times
+    const bool x3 = ctx->math == CB_MATH_3XTF32;
+    // (contexts whose weight gradients run beside another stream keep the kernel that leaves it half the SMs: a DenseNet-100 step took
+    // 3571 us with its widest layers here, 3561 without)
+    if (ctx->math != CB_MATH_FP32 && (ctx->deterministic || ctx->wgrad_grid_cap > 0 || !((x3 && x3_at_fp32(g)) || wgrad_at_fp32(g, x3)))) {
+        rc = umma_conv_wgrad(ctx, dY, X, dW, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, accumulate, dy_batch, x_batch, x3);
+        if (rc == CB_OK && x3) ctx->last_kernel = "umma_3xtf32";
         if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;
     }
-    rc = simt_conv_wgrad(ctx, dY, X, dW, g, accumulate ? 1 : 0, who);
+    rc = fp32_conv_wgrad(ctx, dY, X, dW, g, accumulate ? 1 : 0, who);
     return rc == CB_OK ? finish(ctx, who) : rc;
 }
 

@@ -690,6 +690,32 @@ static int wgrad_core(cb_ctx* ctx, const float* dY, const float* X, float* dW, i
     return CB_OK;
 }
 
+// How the filter of a stride-1 layer is cut into blocks of input x output channels, a launch each (c_blocks 0: not at all).
+struct WgradBlocks {
+    int oc_blocks, oc_step, c_blocks, c_step;
+};
+static WgradBlocks wgrad_blocks(int IC, int OC, int FH, int FW) {
+    const int OCp_all = (OC + 15) / 16 * 16;
+    int oc_max = (256 / FW) & ~15;
+    if (oc_max > 128) oc_max = 128;
+    WgradBlocks b{};
+    if (oc_max < 16) return b;
+    b.oc_blocks = (OCp_all + oc_max - 1) / oc_max;
+    b.oc_step = ((OC + b.oc_blocks - 1) / b.oc_blocks + 15) & ~15;
+    const int nq = FW * (b.oc_blocks > 1 ? b.oc_step : OCp_all);
+    int c_max = ((512 / nq) * 128 / FH) & ~7;
+    if (c_max > 256) c_max = 256;
+    if (c_max < 8) return b;
+    b.c_blocks = (IC + c_max - 1) / c_max;
+    b.c_step = ((IC + b.c_blocks - 1) / b.c_blocks + 7) & ~7;
+    return b;
+}
+int umma_wgrad_launches(int IC, int OC, int FH, int FW) {
+    if (FH > 3 || FW > 3) return 0;
+    const WgradBlocks b = wgrad_blocks(IC, OC, FH, FW);
+    return b.oc_blocks * b.c_blocks;
+}
+
 int umma_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, int N, int IC, int IH, int IW, int OC,
                     int FH, int FW, int sH, int sW, int pH, int pW, int accumulate, long long dy_batch, long long x_batch,
                     bool x3) {
@@ -715,17 +741,9 @@ int umma_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, int
         // Filters wider than one launch covers (256 input channels, 128 output channels, 512 accumulator columns) are
         // cut into blocks of input x output channels: each block is its own launch pair on channel slices of X and dY
         // (same batch strides) that writes its block of dW.
-        const int OCp_all = (OC + 15) / 16 * 16;
-        int oc_max = (256 / FW) & ~15;
-        if (oc_max > 128) oc_max = 128;
-        const int oc_blocks = (OCp_all + oc_max - 1) / oc_max;
-        const int oc_step = ((OC + oc_blocks - 1) / oc_blocks + 15) & ~15;
-        const int nq = FW * (oc_blocks > 1 ? oc_step : OCp_all);
-        int c_max = ((512 / nq) * 128 / FH) & ~7;
-        if (c_max > 256) c_max = 256;
-        if (c_max < 8) return CB_EUNSUPPORTED;
-        const int c_blocks = (IC + c_max - 1) / c_max;
-        const int c_step = ((IC + c_blocks - 1) / c_blocks + 7) & ~7;
+        const WgradBlocks bl = wgrad_blocks(IC, OC, FH, FW);
+        if (bl.c_blocks == 0) return CB_EUNSUPPORTED;
+        const int oc_blocks = bl.oc_blocks, oc_step = bl.oc_step, c_blocks = bl.c_blocks, c_step = bl.c_step;
         if (IW != 8 && IW != 16 && IW != 32) return CB_EUNSUPPORTED;  // before the lo parts are queued
         const long long plane = (long long)IH * IW;
         LoParts lo;

@@ -121,3 +121,31 @@ def test_convolution(ctx, geo, det):
     assert orc.max_err_norm(Y.cpu().numpy(), orc.conv_fwd(W, X, bias, (s, s), (p, p))) <= TOL
     assert orc.max_err_norm(dX.cpu().numpy(), orc.conv_dgrad(W, dY, X.shape, (s, s), (p, p))) <= TOL
     assert orc.max_err_norm(dW.cpu().numpy(), orc.conv_wgrad(dY, X, W.shape, (s, s), (p, p), dW_init=dW0)) <= TOL
+
+
+@pytest.mark.parametrize("math,geo,kern", [("3xtf32", (9, 96, 16, 96, 3, 1), ["umma_fp32"] * 3), ("3xtf32", (64, 64, 16, 128, 3, 2), ["umma_fp32", "umma_3xtf32", "umma_fp32"]),
+                                           ("3xtf32", (128, 16, 32, 32, 3, 2), ["umma_fp32", "umma_3xtf32", "umma_fp32"]), ("tf32", (64, 330, 8, 48, 1, 1), [None, None, "umma_fp32"]),
+                                           ("tf32", (4, 128, 16, 128, 3, 1), [None, None, "umma_fp32"])])
+def test_passes_of_the_other_modes_that_run_at_fp32_accuracy(math, geo, kern):
+    """Wide filters and large stride-2 layers of 3xTF32, weight gradients the TF32 kernel would cut into several launches."""
+    import torch
+    from crusaderbackend_b200.api import Context
+    N, IC, H, OC, F, s = geo
+    p = F // 2
+    c = Context(0, math=math, sync=True)
+    O = (H + 2 * p - F) // s + 1
+    W, X, dY = orc.he_normal_filter(OC, IC, F, F, ("other", geo)), orc.normal((N, IC, H, H), "other", geo, "X"), orc.normal((N, OC, O, O), "other", geo, "dY")
+    tW, tX, tdY = (torch.from_numpy(v).cuda() for v in (W, X, dY))
+    Y, dX, dW = torch.empty_like(tdY), torch.empty_like(tX), torch.zeros_like(tW)
+    got = []
+    for call in (lambda: c.conv(tW, tX, Y, s, s, p, p), lambda: c.convDerive(tW, tdY, dX, s, s, p, p), lambda: c.convError(tdY, tX, dW, s, s, p, p)):
+        call()
+        got.append(c.last_kernel)
+    c.close()
+    assert all(k is None or k == g for k, g in zip(kern, got)), got
+    tol = [TOL if g == "umma_fp32" else {"tf32": 2e-3, "3xtf32": 1e-5}[math] for g in got]
+    n = min(N, 4)  # a few images of the maps, the whole batch of the weight gradient
+    assert orc.max_err_norm(Y[:n].cpu().numpy(), orc.conv_fwd(W, X[:n], None, (s, s), (p, p))) <= tol[0]
+    assert orc.max_err_norm(dX[:n].cpu().numpy(), orc.conv_dgrad(W, dY[:n], X[:n].shape, (s, s), (p, p))) <= tol[1]
+    ref = torch.nn.grad.conv2d_weight(tX.double(), W.shape, tdY.double(), stride=s, padding=p)
+    assert orc.max_err_norm(dW.cpu().numpy(), ref.cpu().numpy()) <= tol[2]
