@@ -158,6 +158,7 @@ struct GemmCall {
     float* C = nullptr; long long ldc = 0, strideC = 0; int out_mode = 0;
     int accumulate = 0;
     Epilogue ep;
+    float* q_sum = nullptr;  // += sum over k of Q[j][k], J values, where the kernel that runs can do it on the way (launch_fp32_gemm)
     int kfold = 1;  // > 1 (with batch == 1): C (+)= sum over kfold operand pairs, strideP / strideQ apart, of P Q^T
 };
 // Per-element tail of a convolution, applied in this order while the accumulator is written out:
@@ -192,7 +193,8 @@ bool umma_gemm_eligible(const GemmCall& g);
 int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3);
 // fp32 accuracy: on the CUDA cores, or (launch_split_gemm: CB_EUNSUPPORTED, before any work is queued, where it is not worth it) on the
 // tensor cores.
-int launch_fp32_gemm(cb_ctx* ctx, const GemmCall& g);
+// *summed is set where g.q_sum has been added to.
+int launch_fp32_gemm(cb_ctx* ctx, const GemmCall& g, bool* summed = nullptr);
 int launch_split_gemm(cb_ctx* ctx, const GemmCall& g);
 // Clears the output matrices of a call whose partial products are added into them with atomics.
 int clear_output(cb_ctx* ctx, float* p, long long width, long long ld, long long rows, long long stride, long long batch, const char* who);

@@ -15,22 +15,28 @@ __global__ void __launch_bounds__(256) colsum_add_kernel(const float* __restrict
     griddep_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int m = blockIdx.x * 32 + lane;
+    // a chain of latencies in few blocks: what is added to and sixteen rows a warp are on their way at once
+    const float old = warp == 0 && m < OUT ? db[m] : 0.f;
     float s = 0.f;
-    if (m < OUT)
-#pragma unroll 8
-        for (int n = warp; n < batch; n += 8) s += dY[(long long)n * OUT + m];
+    for (int n0 = warp; n0 < batch; n0 += 128) {
+        float v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) v[u] = m < OUT && n0 + 8 * u < batch ? dY[(long long)(n0 + 8 * u) * OUT + m] : 0.f;
+#pragma unroll
+        for (int u = 0; u < 16; ++u) s += v[u];
+    }
     part[warp][lane] = s;
     __syncthreads();
     if (warp == 0 && m < OUT) {
         float v = 0.f;
         for (int w = 0; w < 8; ++w) v += part[w][lane];
-        db[m] += v;
+        db[m] = old + v;
     }
 }
 
-int run_gemm(cb_ctx* ctx, const GemmCall& g) {
+int run_gemm(cb_ctx* ctx, const GemmCall& g, bool* summed = nullptr) {
     if (ctx->math != CB_MATH_FP32 && umma_gemm_eligible(g)) return launch_umma_gemm(ctx, g, ctx->math == CB_MATH_3XTF32);
-    return launch_fp32_gemm(ctx, g);
+    return launch_fp32_gemm(ctx, g, summed);
 }
 
 }  // namespace
@@ -87,8 +93,11 @@ int cb_linear_paramgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW,
         g.Q = dY; g.ldq = OUT; g.q_mn = 1;
         g.C = dW; g.ldc = IN; g.out_mode = 0;
         g.accumulate = 1;
-        int rc = run_gemm(ctx, g);
+        g.q_sum = db;
+        bool summed = false;
+        int rc = run_gemm(ctx, g, &summed);
         if (rc != CB_OK) return rc;
+        if (summed) db = nullptr;
     }
     if (db) {
         cudaError_t e = launch_dep(ctx, colsum_add_kernel, dim3((unsigned)((OUT + 31) / 32)), dim3(256), 0, dY, db, batch, OUT);
