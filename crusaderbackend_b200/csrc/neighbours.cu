@@ -243,13 +243,16 @@ __device__ __forceinline__ void st4(float* row, long long p, long long P, float4
 // Block = T / G float4 position vectors x G rows of threads; thread (x, g) keeps samples n = g, g + G, ... (SPT of them) in
 // registers. Sample n counts to batch group n mod R G, whose members are added in ascending order, then the groups: the order,
 // and with it every bit of the statistics, depends on R G alone, so the launchers below choose G by speed.
-template <int T, int G, int SPT, int R, bool V>
+// S: a model's BatchNorm-(add-)ReLU, which writes Y and what its backward pass needs (BnSaved). A form of its own, as in the backward
+// kernel: the tests of both in one cost registers (DenseNet-100 step 3590 -> 3690 us).
+template <int T, int G, int SPT, int R, bool V, bool S>
 __global__ void __launch_bounds__(T) bn_fwd_par_kernel(const float* __restrict__ X, const float* __restrict__ beta,
                                                          const float* __restrict__ gamma, float* __restrict__ mean,
                                                          float* __restrict__ var, float* __restrict__ Y,
                                                          float* __restrict__ xhat, const float* __restrict__ res, int N,
-                                                         long long P, int relu, long long xs) {
+                                                         long long P, int relu, long long xs, uint8_t* __restrict__ passes) {
     // xs: floats between consecutive samples of X (P when dense; larger for a channel-prefix view of a wider tensor)
+    // passes: a byte for four consecutive elements of Y, whose low bits say which of them are > 0 (BnSaved)
     constexpr int PB = T / G;
     __shared__ __align__(16) float red[R * 4 * T];
     __shared__ __align__(16) float tot[PB * 4];
@@ -287,7 +290,8 @@ __global__ void __launch_bounds__(T) bn_fwd_par_kernel(const float* __restrict__
         if (r + 1 < R) bn_put<1, G, R, T>(q, red);
     }
     bn_block_sums<1, G, R, T>(q, red, tot);
-    const float4 v = make_float4(q[0].x * invN, q[0].y * invN, q[0].z * invN, q[0].w * invN);
+    // rounded on its own, in every form of the kernel: contracted with the addition below, it would give statistics of other bits
+    const float4 v = make_float4(__fmul_rn(q[0].x, invN), __fmul_rn(q[0].y, invN), __fmul_rn(q[0].z, invN), __fmul_rn(q[0].w, invN));
     if (!live) return;
     const float4 inv = make_float4(1.0f / sqrtf(v.x + 1e-8f), 1.0f / sqrtf(v.y + 1e-8f), 1.0f / sqrtf(v.z + 1e-8f),
                                    1.0f / sqrtf(v.w + 1e-8f));
@@ -299,83 +303,128 @@ __global__ void __launch_bounds__(T) bn_fwd_par_kernel(const float* __restrict__
                                          (x[i].w - m.w) * inv.w);
             float4 y = make_float4(h.x * ga.x + be.x, h.y * ga.y + be.y, h.z * ga.z + be.z, h.w * ga.w + be.w);
             if (res) y = f4_add(y, ld4<V>(res + (long long)n * P, p, P));  // shortcut add
-            if (relu) y = make_float4(fmaxf(y.x, 0.f), fmaxf(y.y, 0.f), fmaxf(y.z, 0.f), fmaxf(y.w, 0.f));
+            if (S || relu) y = make_float4(fmaxf(y.x, 0.f), fmaxf(y.y, 0.f), fmaxf(y.z, 0.f), fmaxf(y.w, 0.f));
             st4<V>(Y + (long long)n * P, p, P, y);
-            if (xhat) st4<V>(xhat + (long long)n * P, p, P, h);
+            if (!S && xhat) st4<V>(xhat + (long long)n * P, p, P, h);
+            if (S) passes[(n * P + p) >> 2] = (uint8_t)((y.x > 0.f ? 1 : 0) | (y.y > 0.f ? 2 : 0) | (y.z > 0.f ? 4 : 0) | (y.w > 0.f ? 8 : 0));
         }
     }
     if (g == 0) {
-        if (mean) st4<V>(mean, p, P, m);
-        if (var) st4<V>(var, p, P, v);
+        if (S || mean) st4<V>(mean, p, P, m);
+        if (!S && var) st4<V>(var, p, P, v);
     }
 }
 
 // Data gradient (statistics recomputed from X as seblas::batchNormGrad does) and, when dgamma / dbeta are given, the
 // parameter gradients dbeta = sum dy, dgamma = sum dy * xhat of seblas::batchNormParamGrads in the same pass.
-template <int T, int G, int SPT, int R, bool V>
+template <int T, int G, int SPT, int R, bool V, bool S>
 __global__ void __launch_bounds__(T, SPT <= 4 ? 1024 / T : 1) bn_bwd_par_kernel(const float* __restrict__ dY, const float* __restrict__ gamma,
                                                          const float* __restrict__ X, float* __restrict__ dX,
                                                          float* __restrict__ dgamma, float* __restrict__ dbeta,
                                                          const float* __restrict__ relu_out, float* __restrict__ dres,
                                                          int dres_add, int pg_add, int N, long long P, long long xs,
-                                                         long long dxs, int dx_add) {
+                                                         long long dxs, int dx_add, const BnSaved saved) {
     // xs / dxs: floats between consecutive samples of X / dX (P when dense); dx_add: dX += instead of dX =
+    // S: `saved` is what the forward kernel left: relu_out is not read, and the mean is not summed again
     constexpr int PB = T / G;
     __shared__ __align__(16) float red[R * 16 * T];
     __shared__ __align__(16) float tot[4 * PB * 4];
-    griddep_wait();
-    griddep_launch();
     const long long p = ((long long)blockIdx.x * PB + threadIdx.x) * 4;
     const bool live = p < P;
     const int g = threadIdx.y;
-    const float4 ga = live ? ld4<V>(gamma, p, P) : f4_zero();
+    const float invN = 1.0f / (float)N;
     float4 x[SPT], dy[SPT];
-    float4 s[1] = {f4_zero()}, s0[1] = {f4_zero()};
+    float4 m, sq[R], sxc[R];  // mean, and per batch group of this thread the sums of xc^2 and xc
+    unsigned passes[SPT];
+    if (!S) {
+        griddep_wait();
+        griddep_launch();
+    }
+    const float4 ga = live ? ld4<V>(gamma, p, P) : f4_zero();
+    if (S) {
+        // All this was written at least two kernels ago (a forward pass, and the update before it), so it is complete although the kernel
+        // before this one may still run: its reads from HBM, and the sums over X alone, are done by the time dY is there.
+        m = live ? ld4<V>(saved.mean, p, P) : f4_zero();
+#pragma unroll
+        for (int i = 0; i < SPT; ++i) {
+            const int n = g + G * i;
+            const bool on = live && n < N;
+            x[i] = on ? ld4<V>(X + (long long)n * xs, p, P) : f4_zero();
+            passes[i] = on ? saved.passes[((long long)n * P + p) >> 2] : 0u;
+        }
+    } else {
+        float4 s[1] = {f4_zero()}, s0[1] = {f4_zero()};
+#pragma unroll
+        for (int i = 0; i < SPT; ++i) {
+            const int n = g + G * i;
+            const bool on = live && n < N;
+            x[i] = on ? ld4<V>(X + (long long)n * xs, p, P) : f4_zero();
+            dy[i] = on ? ld4<V>(dY + (long long)n * P, p, P) : f4_zero();
+            if (relu_out && on) {  // the ReLU that followed this layer in the forward pass: dy passes where its output is > 0
+                const float4 r = ld4<V>(relu_out + (long long)n * P, p, P);
+                dy[i] = make_float4(r.x > 0.f ? dy[i].x : 0.f, r.y > 0.f ? dy[i].y : 0.f, r.z > 0.f ? dy[i].z : 0.f,
+                                    r.w > 0.f ? dy[i].w : 0.f);
+            }
+            if (dres && on) {  // the shortcut that was added before that ReLU receives the same masked gradient
+                float* d = dres + (long long)n * P;
+                st4<V>(d, p, P, dres_add ? f4_add(ld4<V>(d, p, P), dy[i]) : dy[i]);
+            }
+            if (R == 2 && i % 2 == 0) s0[0] = f4_add(s0[0], x[i]);
+            else s[0] = f4_add(s[0], x[i]);
+        }
+        if (R == 2) bn_put<1, G, R, T>(s0, red);
+        bn_block_sums<1, G, R, T>(s, red, tot);
+        m = make_float4(s[0].x * invN, s[0].y * invN, s[0].z * invN, s[0].w * invN);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) sq[r] = sxc[r] = f4_zero();
 #pragma unroll
     for (int i = 0; i < SPT; ++i) {
-        const int n = g + G * i;
-        const bool on = live && n < N;
-        x[i] = on ? ld4<V>(X + (long long)n * xs, p, P) : f4_zero();
-        dy[i] = on ? ld4<V>(dY + (long long)n * P, p, P) : f4_zero();
-        if (relu_out && on) {  // the ReLU that followed this layer in the forward pass: dy passes where its output is > 0
-            const float4 r = ld4<V>(relu_out + (long long)n * P, p, P);
-            dy[i] = make_float4(r.x > 0.f ? dy[i].x : 0.f, r.y > 0.f ? dy[i].y : 0.f, r.z > 0.f ? dy[i].z : 0.f,
-                                r.w > 0.f ? dy[i].w : 0.f);
+        if (g + G * i < N) {
+            const float4 xc = make_float4(x[i].x - m.x, x[i].y - m.y, x[i].z - m.z, x[i].w - m.w);
+            x[i] = xc;  // keep the centred value
+            sq[i % R] = f4_add(sq[i % R], make_float4(xc.x * xc.x, xc.y * xc.y, xc.z * xc.z, xc.w * xc.w));
+            sxc[i % R] = f4_add(sxc[i % R], xc);
         }
-        if (dres && on) {  // the shortcut that was added before that ReLU receives the same masked gradient
-            float* d = dres + (long long)n * P;
-            st4<V>(d, p, P, dres_add ? f4_add(ld4<V>(d, p, P), dy[i]) : dy[i]);
-        }
-        if (R == 2 && i % 2 == 0) s0[0] = f4_add(s0[0], x[i]);
-        else s[0] = f4_add(s[0], x[i]);
     }
-    if (R == 2) bn_put<1, G, R, T>(s0, red);
-    const float invN = 1.0f / (float)N;
-    bn_block_sums<1, G, R, T>(s, red, tot);
-    const float4 m = make_float4(s[0].x * invN, s[0].y * invN, s[0].z * invN, s[0].w * invN);
+    if (S) {
+        griddep_wait();
+        griddep_launch();
+#pragma unroll
+        for (int i = 0; i < SPT; ++i) {
+            const int n = g + G * i;
+            const bool on = live && n < N;
+            dy[i] = on ? ld4<V>(dY + (long long)n * P, p, P) : f4_zero();
+            dy[i] = make_float4(passes[i] & 1 ? dy[i].x : 0.f, passes[i] & 2 ? dy[i].y : 0.f, passes[i] & 4 ? dy[i].z : 0.f,
+                                passes[i] & 8 ? dy[i].w : 0.f);
+            if (dres && on) {
+                float* d = dres + (long long)n * P;
+                st4<V>(d, p, P, dres_add ? f4_add(ld4<V>(d, p, P), dy[i]) : dy[i]);
+            }
+        }
+    }
     // sums of xc^2, dy * xc (dxhat = dy * gamma is factored out below), dy and xc, in one exchange
-    float4 sums[4] = {f4_zero(), f4_zero(), f4_zero(), f4_zero()};
+    float4 sums[4];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
+        sums[0] = sq[r];
+        sums[1] = sums[2] = f4_zero();
+        sums[3] = sxc[r];
 #pragma unroll
         for (int i = 0; i < SPT; ++i) {
             if (i % R == r && g + G * i < N) {
-                const float4 xc = make_float4(x[i].x - m.x, x[i].y - m.y, x[i].z - m.z, x[i].w - m.w);
-                x[i] = xc;  // keep the centred value
-                sums[0] = f4_add(sums[0], make_float4(xc.x * xc.x, xc.y * xc.y, xc.z * xc.z, xc.w * xc.w));
-                sums[1] = f4_add(sums[1], make_float4(dy[i].x * xc.x, dy[i].y * xc.y, dy[i].z * xc.z, dy[i].w * xc.w));
+                sums[1] = f4_add(sums[1], make_float4(dy[i].x * x[i].x, dy[i].y * x[i].y, dy[i].z * x[i].z, dy[i].w * x[i].w));
                 sums[2] = f4_add(sums[2], dy[i]);
-                sums[3] = f4_add(sums[3], xc);
             }
         }
         if (r + 1 < R) bn_put<4, G, R, T>(sums, red);
     }
     bn_block_sums<4, G, R, T>(sums, red, tot);
-    const float4 sq = sums[0], sdx = sums[1], sd = sums[2], sxc = sums[3];
+    const float4 sdx = sums[1], sd = sums[2];
     if (!live) return;
     float o_inv[4], o_dvar[4], o_dmean[4];
-    const float sqv[4] = {sq.x, sq.y, sq.z, sq.w}, sdxv[4] = {sdx.x, sdx.y, sdx.z, sdx.w}, sdv[4] = {sd.x, sd.y, sd.z, sd.w},
-                sxcv[4] = {sxc.x, sxc.y, sxc.z, sxc.w}, gav[4] = {ga.x, ga.y, ga.z, ga.w};
+    const float sqv[4] = {sums[0].x, sums[0].y, sums[0].z, sums[0].w}, sdxv[4] = {sdx.x, sdx.y, sdx.z, sdx.w}, sdv[4] = {sd.x, sd.y, sd.z, sd.w},
+                sxcv[4] = {sums[3].x, sums[3].y, sums[3].z, sums[3].w}, gav[4] = {ga.x, ga.y, ga.z, ga.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const float inv = 1.0f / sqrtf(sqv[e] * invN + 1e-8f);
@@ -396,10 +445,10 @@ __global__ void __launch_bounds__(T, SPT <= 4 ? 1024 / T : 1) bn_bwd_par_kernel(
             st4<V>(dst, p, P, dx_add ? f4_add(ld4<V>(dst, p, P), o) : o);
         }
     }
-    if (g == 0 && dgamma && dbeta) {
+    if (g == 0 && (S || (dgamma && dbeta))) {
         float4 gb = sd;
         float4 gg = make_float4(sdx.x * o_inv[0], sdx.y * o_inv[1], sdx.z * o_inv[2], sdx.w * o_inv[3]);  // sum dy * xhat
-        if (pg_add) {  // a later group of a batch whose statistics are taken per group
+        if (!S && pg_add) {  // a later group of a batch whose statistics are taken per group
             gb = f4_add(gb, ld4<V>(dbeta, p, P));
             gg = f4_add(gg, ld4<V>(dgamma, p, P));
         }
@@ -457,11 +506,11 @@ void launch_bn(cb_ctx* ctx, void (*kernel)(KArgs...), long long P, Args... args)
 // 128, 131072 24.4 / 31.4; 173, 111616 38.2 / 34.4. 512 threads in 32 rows: N 64, P 135168 18.0.
 inline bool bn_narrow(const cb_ctx* ctx, int N, long long P) { return N >= 128 && (P / 4 + 7) / 8 < ctx->sm_count; }
 void launch_bn_fwd_par(cb_ctx* ctx, const float* X, const float* beta, const float* gamma, float* mean, float* var, float* Y,
-                       float* xhat, const float* res, int N, long long P, int relu, long long xs = 0, bool vec = true) {
+                       float* xhat, const float* res, int N, long long P, int relu, long long xs = 0, bool vec = true, uint8_t* passes = nullptr) {
     if (xs == 0) xs = P;
 #define CB_BN(T, G, SPT, R)                                                                                                      \
-    launch_bn<T, G>(ctx, vec ? bn_fwd_par_kernel<T, G, SPT, R, true> : bn_fwd_par_kernel<T, G, SPT, R, false>, P, X, beta, gamma, \
-                      mean, var, Y, xhat, res, N, P, relu, xs)
+    launch_bn<T, G>(ctx, passes ? bn_fwd_par_kernel<T, G, SPT, R, true, true> : vec ? bn_fwd_par_kernel<T, G, SPT, R, true, false> : bn_fwd_par_kernel<T, G, SPT, R, false, false>, P, X, beta, gamma, \
+                      mean, var, Y, xhat, res, N, P, relu, xs, passes)
     if (N <= 16) CB_BN(256, 16, 1, 1);
     else if (N <= 32) CB_BN(256, 16, 2, 1);
     else if (N < 64) CB_BN(256, 16, 4, 1);
@@ -482,12 +531,12 @@ void launch_bn_fwd_par(cb_ctx* ctx, const float* X, const float* beta, const flo
 // behind a flushed L2, 16 against 32 rows: P 49152 25.5 / 22.6, 135168 49.2 / 47.1, 270336 81.9 / 84.0; without dX += 26.6 / 25.8.
 void launch_bn_bwd_par(cb_ctx* ctx, const float* dY, const float* gamma, const float* X, float* dX, float* dgamma,
                        float* dbeta, const float* relu_out, float* dres, int dres_add, int pg_add, int N, long long P,
-                       long long xs = 0, long long dxs = 0, int dx_add = 0, bool vec = true) {
+                       long long xs = 0, long long dxs = 0, int dx_add = 0, bool vec = true, BnSaved saved = BnSaved()) {
     if (xs == 0) xs = P;
     if (dxs == 0) dxs = P;
 #define CB_BN(T, G, SPT, R)                                                                                                          \
-    launch_bn<T, G>(ctx, vec ? bn_bwd_par_kernel<T, G, SPT, R, true> : bn_bwd_par_kernel<T, G, SPT, R, false>, P, dY, gamma, X, dX, dgamma, dbeta, relu_out, dres, dres_add, pg_add, N, P, xs, \
-                    dxs, dx_add)
+    launch_bn<T, G>(ctx, saved.passes ? bn_bwd_par_kernel<T, G, SPT, R, true, true> : vec ? bn_bwd_par_kernel<T, G, SPT, R, true, false> : bn_bwd_par_kernel<T, G, SPT, R, false, false>, P, dY, gamma, X, dX, dgamma, dbeta, relu_out, dres, dres_add, pg_add, N, P, xs, \
+                    dxs, dx_add, saved)
     if (N <= 16) CB_BN(256, 16, 1, 1);
     else if (N <= 32) CB_BN(256, 16, 2, 1);
     else if (N < 64) CB_BN(256, 16, 4, 1);
@@ -1003,7 +1052,7 @@ int cb_bn_paramgrad(cb_ctx* ctx, const float* dY, const float* xhat, float* dgam
 
 static int bn_bwd_fused_impl(cb_ctx* ctx, const float* dY, const float* gamma, const float* X, float* dX, float* dgamma,
                              float* dbeta, const float* relu_out, float* dres, int dres_add, int pg_add, int N, long long P,
-                             long long xs = 0, long long dxs = 0, int dx_add = 0) {
+                             long long xs = 0, long long dxs = 0, int dx_add = 0, BnSaved saved = BnSaved()) {
     if (int rc_enter = enter(ctx)) return rc_enter;
     if (N < 0 || P < 0) return fail(ctx, CB_EINVAL, "cb_bn_bwd_fused: negative extent");
     if (N == 0 || P == 0) return CB_OK;
@@ -1014,7 +1063,7 @@ static int bn_bwd_fused_impl(cb_ctx* ctx, const float* dY, const float* gamma, c
     if (!ok) return fail(ctx, CB_EUNSUPPORTED, "cb_bn_bwd_fused: needs N <= 256, P % 4 == 0 and 16-byte aligned tensors");
     if ((xs && (xs < P || (xs & 3))) || (dxs && (dxs < P || (dxs & 3))))
         return fail(ctx, CB_EINVAL, "cb_bn_bwd_fused: a batch stride must be at least P and a multiple of 4 floats");
-    launch_bn_bwd_par(ctx, dY, gamma, X, dX, dgamma, dbeta, relu_out, dres, dres_add, pg_add, N, P, xs, dxs, dx_add);
+    launch_bn_bwd_par(ctx, dY, gamma, X, dX, dgamma, dbeta, relu_out, dres, dres_add, pg_add, N, P, xs, dxs, dx_add, true, saved);
     return done(ctx, "cb_bn_bwd_fused");
 }
 int cb_bn_bwd_fused_ex(cb_ctx* ctx, const float* dY, const float* gamma, const float* X, float* dX, float* dgamma,
@@ -1036,7 +1085,7 @@ int cb_bn_bwd_fused_res(cb_ctx* ctx, const float* dY, const float* gamma, const 
 
 extern "C" {
 static int bn_fwd_relu_impl(cb_ctx* ctx, const float* X, const float* beta, const float* gamma, const float* R, float* Y, int N,
-                            long long P, long long xs = 0);
+                            long long P, long long xs = 0, BnSaved saved = BnSaved());
 }
 
 namespace cb {
@@ -1046,6 +1095,14 @@ namespace cb {
 int bn_bwd_group(cb_ctx* ctx, const float* dY, const float* gamma, const float* X, float* dX, float* dgamma, float* dbeta,
                  const float* relu_out, float* dR, int accumulate_dR, int add_param_grads, int N, long long P) {
     return bn_bwd_fused_impl(ctx, dY, gamma, X, dX, dgamma, dbeta, relu_out, dR, accumulate_dR, add_param_grads, N, P);
+}
+int bn_fwd_model(cb_ctx* ctx, const float* X, const float* beta, const float* gamma, const float* R, float* Y, int N, long long P, long long xs,
+                 const BnSaved& saved) {
+    return bn_fwd_relu_impl(ctx, X, beta, gamma, R, Y, N, P, xs, saved);
+}
+int bn_bwd_model(cb_ctx* ctx, const float* dY, const float* gamma, const float* X, float* dX, float* dgamma, float* dbeta, float* dR,
+                 int accumulate_dR, int N, long long P, long long xs, long long dxs, int accumulate_dX, const BnSaved& saved) {
+    return bn_bwd_fused_impl(ctx, dY, gamma, X, dX, dgamma, dbeta, nullptr, dR, accumulate_dR, 0, N, P, xs, dxs, accumulate_dX, saved);
 }
 int bn_fwd_group(cb_ctx* ctx, const float* X, const float* beta, const float* gamma, const float* R, float* Y, int relu, int N,
                  long long P) {
@@ -1057,7 +1114,7 @@ int bn_fwd_group(cb_ctx* ctx, const float* X, const float* beta, const float* ga
 extern "C" {
 
 static int bn_fwd_relu_impl(cb_ctx* ctx, const float* X, const float* beta, const float* gamma, const float* R, float* Y, int N,
-                            long long P, long long xs) {
+                            long long P, long long xs, BnSaved saved) {
     if (int rc_enter = enter(ctx)) return rc_enter;
     if (N < 0 || P < 0) return fail(ctx, CB_EINVAL, "cb_bn_fwd_relu: negative extent");
     if (N == 0 || P == 0) return CB_OK;
@@ -1066,7 +1123,7 @@ static int bn_fwd_relu_impl(cb_ctx* ctx, const float* X, const float* beta, cons
     if (!((P % 4 == 0) && spt > 0 && aligned16(X) && aligned16(Y) && aligned16(beta) && aligned16(gamma) && (!R || aligned16(R))))
         return fail(ctx, CB_EUNSUPPORTED, "cb_bn_fwd_relu: needs N <= 256, P % 4 == 0 and 16-byte aligned tensors");
     if (xs && (xs < P || (xs & 3))) return fail(ctx, CB_EINVAL, "cb_bn_fwd_relu: the batch stride must be at least P and a multiple of 4 floats");
-    launch_bn_fwd_par(ctx, X, beta, gamma, nullptr, nullptr, Y, nullptr, R, N, P, 1, xs);
+    launch_bn_fwd_par(ctx, X, beta, gamma, saved.mean, nullptr, Y, nullptr, R, N, P, 1, xs, true, saved.passes);
     return done(ctx, "cb_bn_fwd_relu");
 }
 int cb_bn_fwd_relu_ex(cb_ctx* ctx, const float* X, const float* beta, const float* gamma, float* Y, int N, long long P,

@@ -50,6 +50,7 @@ struct Op {
     bool in0_grad_accumulate = false;   // backward adds into in0's gradient instead of overwriting it
     bool in1_grad_accumulate = false;   // likewise for the second input (shortcut of a fused BatchNorm-add-ReLU)
     bool relu = false;                  // BN / ADD: a ReLU is folded into this op (out is the activated tensor)
+    cb::BnSaved saved;                  // BN with a ReLU: what its forward kernel leaves for the backward one
     int pooled = -1, logits = -1, probs = -1;  // HEAD: tensors holding the pooled features, logits and softmax
 };
 
@@ -105,11 +106,11 @@ struct ParamEntry {
 // they lie in a 16-byte word (floats past it): kernels are chosen by alignment, and the buffers a recording reads lie likewise.
 struct PassKey {
     int images_at, labels_at;
-    int backward, math, deterministic, bn_grad_swap, bn_groups, pdl;
+    int backward, math, deterministic, bn_grad_swap, bn_groups, bn_saved, pdl;
     long long scratch_epoch;
     bool operator==(const PassKey& o) const {
         return images_at == o.images_at && labels_at == o.labels_at && backward == o.backward && math == o.math && deterministic == o.deterministic &&
-               bn_grad_swap == o.bn_grad_swap && bn_groups == o.bn_groups && pdl == o.pdl && scratch_epoch == o.scratch_epoch;
+               bn_grad_swap == o.bn_grad_swap && bn_groups == o.bn_groups && bn_saved == o.bn_saved && pdl == o.pdl && scratch_epoch == o.scratch_epoch;
     }
 };
 struct RecordedPass {
@@ -172,6 +173,7 @@ struct cbt_model {
     std::string err;
     void* mom_table = nullptr;     // device descriptor table of the Momentum step, built by cbt_bind
     int bn_grad_swap = 0;          // 1: BatchNorm's two parameter gradients land in each other's slot, as in the reference
+    bool bn_saved = false;         // the last forward pass left what Op::saved holds (it does unless it took statistics per group)
     int bn_groups = 1;             // BatchNorm statistics are taken per group of batch / bn_groups consecutive samples
     // data-parallel state (cbt_dp_init)
     void* comm = nullptr;
@@ -425,6 +427,15 @@ int finalize_model(cbt_model* m, int x, int classes) {
         b.d = par.d + (long long)b.c_off * b.h * b.w;
     }
     m->scratch_elems = biggest;
+    for (Op& o : m->ops) {
+        if (o.kind != OP_BN || !o.relu || o.xhat >= 0 || m->batch < cb::kLeastSaved || m->batch > cb::kMostSaved) continue;
+        const TensorBuf& y = m->t[o.out];
+        float* bytes = nullptr;  // size / 4 of them
+        int rc = dev_alloc(m, &bytes, (y.size() / 4 + 3) / 4);
+        if (rc == CB_OK) rc = dev_alloc(m, &o.saved.mean, y.sample());
+        if (rc != CB_OK) return rc;
+        o.saved.passes = reinterpret_cast<uint8_t*>(bytes);
+    }
     int rc = dev_alloc(m, &m->scratch, biggest);
     if (rc == CB_OK) rc = dev_alloc(m, &m->loss_dev, 4);
     if (rc == CB_OK) rc = dev_alloc(m, &m->loss_n, m->batch);
@@ -913,7 +924,7 @@ int run_recorded(cbt_model* m, bool backward, F ops) {
     if (cap != cudaStreamCaptureStatusNone) return pass();
     float*& input = m->t[m->input].a;
     PassKey key{floats_past_16(input), floats_past_16(m->labels), backward ? 1 : 0, ctx->math, ctx->deterministic, m->bn_grad_swap,
-                m->bn_groups, ctx->pdl, ctx->scratch_epoch};
+                m->bn_groups, m->bn_saved ? 1 : 0, ctx->pdl, ctx->scratch_epoch};
     for (const cb_ctx* c : m->side) key.scratch_epoch += c->scratch_epoch;  // only ever grow: the sum changes with any of them
     RecordedPass* r = nullptr;
     for (RecordedPass& e : m->recorded)
@@ -1009,6 +1020,7 @@ int cbt_forward(cbt_model* m, const float* images, const float* labels) {
     m->t[m->input].a = const_cast<float*>(images);
     m->labels = const_cast<float*>(labels);
     m->input_own = false;
+    m->bn_saved = m->bn_groups == 1;
     return run_recorded(m, false, [&] { return forward_ops(m); });
 }
 static int forward_ops(cbt_model* m) {
@@ -1049,6 +1061,11 @@ static int forward_ops(cbt_model* m) {
                         CBT_TRY(cb::bn_fwd_group(ctx, x.a + off, m->P + o.b_off, m->P + o.w_off,
                                                  o.in1 >= 0 ? m->t[o.in1].a + off : nullptr, y.a + off, o.relu ? 1 : 0, ng, P));
                     }
+                    break;
+                }
+                if (o.saved.passes) {
+                    CBT_TRY(cb::bn_fwd_model(ctx, x.a, m->P + o.b_off, m->P + o.w_off, o.in1 >= 0 ? m->t[o.in1].a : nullptr, y.a, x.n,
+                                             (long long)x.c * x.h * x.w, x.bstride, o.saved));
                     break;
                 }
                 if (o.in1 >= 0) {
@@ -1220,6 +1237,10 @@ static int backward_ops(cbt_model* m) {
                                                  o.relu ? y.a + off : nullptr, o.in1 >= 0 ? m->t[o.in1].d + off : nullptr,
                                                  o.in1_grad_accumulate ? 1 : 0, g > 0 ? 1 : 0, ng, P));
                     }
+                } else if (o.saved.passes && m->bn_saved) {
+                    CBT_TRY(cb::bn_bwd_model(ctx, y.d, m->P + o.w_off, x.a, dx, dgamma, dbeta, o.in1 >= 0 ? m->t[o.in1].d : nullptr,
+                                             o.in1_grad_accumulate ? 1 : 0, x.n, P, x.bstride, x.bstride,
+                                             o.in1 < 0 && o.in0_grad_accumulate ? 1 : 0, o.saved));
                 } else if (o.in1 >= 0) {
                     CBT_TRY(cb_bn_bwd_fused_res(ctx, y.d, m->P + o.w_off, x.a, dx, dgamma, dbeta, y.a, m->t[o.in1].d,
                                                 o.in1_grad_accumulate ? 1 : 0, x.n, P));
