@@ -312,8 +312,11 @@ __global__ void __launch_bounds__(96 + 32 * kEpiWarps + (X3 ? 32 * kSplitWarps :
                 const bool plain = p.bias_i == nullptr && p.bias_j == nullptr && !relu_now;
                 for (int m = 0; m < p.mi && ok; ++m, ++sub) {
                     const uint32_t a = sub & 1u;
+                    // Waiting warps sleep between their looks only where a tile takes long (2048 k, ~5 us): there they would take issue
+                    // slots from the other roles all the time; before, the sleep is most of what a short tile waits (256^3 6.2 -> 5.4 us,
+                    // 512^3 8.1 -> 7.7, 1024^2 with K 64 6.2 -> 5.5; 1024^3 and up the same).
                     ok = mbar_wait_warp(smem_u32(&ps.tfull[a]), (sub >> 1) & 1u, lane, abort_flag, p.status,
-                                        CBK_TIMEOUT_TMEM_FULL, kCluster ? 0 : 512);
+                                        CBK_TIMEOUT_TMEM_FULL, kCluster || p.kb_per_split <= 64 ? 0 : 512);
                     if (!ok) break;
                     tc_fence_after();
                     const int i = it.i0 + 128 * m + 32 * quarter + lane;
