@@ -68,6 +68,7 @@ struct __align__(8) PipeSmem {
     uint64_t xf[kMaxStages];
     uint64_t tfull[2];
     uint64_t tempty[2];
+    uint64_t lo_empty[2];  // umma_gemm_x3_kernel: lo tiles of Q
     uint64_t drain;
     uint32_t tmem_base;
     int abort_flag;
@@ -482,6 +483,270 @@ __global__ void __launch_bounds__(96 + 32 * kEpiWarps + (X3 ? 32 * kSplitWarps :
     }
 }
 
+// 3xTF32 with P in TMEM, for contractions that are not split over a cluster. In the kernel above both operands and their lo parts lie in
+// shared memory: 96 KB a stage of a 128 x 256 tile, so two stages, and 12 KB of operands for every UMMA besides the split's own traffic
+// (2890 clocks a k-block of 32, of which the 12 UMMAs are 1650; 2048^3 TN 115 us). Here the split warps put P, as it is and its lo part,
+// into TMEM (64 columns a stage) and only the lo part of Q into shared memory, in a ring of its own: the UMMAs read 8 KB, three
+// stages of raw tiles are in flight, and the tensor core (12 x 160 clocks: one with A in TMEM starts ~23 late) is what a k-block waits
+// for. TMEM then holds one accumulator, which the epilogue warps add to their registers every `kX3Chunk` blocks at most (in the
+// kernel above: to C, every 16). 2048^3 TN: 72 us, 1950 clocks a k-block.
+constexpr int kX3Raw = 3, kX3Lo = 2, kX3Chunk = 8;  // stages of raw tiles (and of P in TMEM), lo tiles of Q, k-blocks of an accumulation
+constexpr int kX3SplitWarps = 8, kX3EpiWarps = 16, kX3Threads = 128 + 32 * (kX3SplitWarps + kX3EpiWarps);
+constexpr int kX3Regs[3] = {40, 56, 88};          // a thread: producers and issuer, split warps, epilogue warps; 72 at launch
+static_assert(128 * kX3Regs[0] + 32 * kX3SplitWarps * kX3Regs[1] + 32 * kX3EpiWarps * kX3Regs[2] <= 72 * kX3Threads, "setmaxnreg would wait for ever");
+
+template <bool P_MN, bool Q_MN>
+__global__ void __launch_bounds__(kX3Threads, 1)
+    umma_gemm_x3_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmQ, const GemmParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ PipeSmem ps;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    volatile int* abort_flag = &ps.abort_flag;
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t q_bytes = (uint32_t)p.bn * kBK * 4, stage_bytes = (uint32_t)kPTileBytes + q_bytes, lo_base = base + kX3Raw * stage_bytes;
+    if (threadIdx.x == 0) {
+        ps.abort_flag = 0;
+        for (int s = 0; s < kX3Raw; ++s) {
+            mbar_init(smem_u32(&ps.full[s]), 2);
+            mbar_init(smem_u32(&ps.empty[s]), 1);
+            mbar_init(smem_u32(&ps.xf[s]), kX3SplitWarps);
+        }
+        for (int s = 0; s < kX3Lo; ++s) mbar_init(smem_u32(&ps.lo_empty[s]), 1);
+        for (int h = 0; h < 2; ++h) {
+            mbar_init(smem_u32(&ps.tfull[h]), 1);
+            mbar_init(smem_u32(&ps.tempty[h]), kX3EpiWarps / 2);
+        }
+        mbar_init(smem_u32(&ps.drain), 1);
+        mbar_fence_init();
+        tma_prefetch_desc(&tmP);
+        tma_prefetch_desc(&tmQ);
+    }
+    __syncthreads();
+    if (warp == 1) {
+        tmem_alloc(smem_u32(&ps.tmem_base), 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    griddep_wait();
+    griddep_launch();
+    const uint32_t tmem_base = ps.tmem_base, p_cols = tmem_base + 256u;  // P: [raw 32 k][lo 32 k] a stage
+    const int total_work = p.batch * p.tiles_i * p.tiles_j * p.kgroups;
+    uint32_t fills = 0;
+
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kX3Regs[0]));
+        if (warp == 0) {
+            fills = produce<P_MN>(p, &tmP, ps, base, stage_bytes, (uint32_t)kPTileBytes, true, total_work);
+        } else if (warp == 2) {
+            fills = produce<Q_MN>(p, &tmQ, ps, base + kPTileBytes, stage_bytes, q_bytes, false, total_work);
+        } else if (warp == 1) {
+            // The first and the last k-block of a chunk go half a tile at a time, so that the epilogue takes one half while the
+            // tensor core is at the other (2 x 12 UMMAs of 128 columns take ~310 clocks more than 12 of 256; waiting for all of
+            // the accumulator took ~1650 a chunk).
+            const int halves = (p.bn & 63) == 0 ? 2 : 1;
+            const uint32_t idesc = umma_idesc_tf32(128, (uint32_t)p.bn, 0u, Q_MN ? 1u : 0u);
+            const uint32_t part_n = (uint32_t)(p.bn / halves), part_idesc = umma_idesc_tf32(128, part_n, 0u, Q_MN ? 1u : 0u);
+            constexpr uint64_t kStepQ = Q_MN ? (1024u >> 4) : (32u >> 4);
+            const uint64_t descQ0 = Q_MN ? desc_mn(0) : desc_k(0);
+            uint32_t s = 0, ph = 0, l = 0, chunk = 0;
+            bool ok = true;
+            for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
+                const WorkItem it = decode_work(p, w);
+                int kc_pos = 0;
+                for (int kb = it.kb0; kb < it.kb1; ++kb) {
+                    ok = mbar_wait_uniform(smem_u32(&ps.xf[s]), ph, abort_flag, p.status, CBK_TIMEOUT_XFORM);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const bool begin = kc_pos == 0, last = kc_pos == p.kc - 1 || kb == it.kb1 - 1;
+                    const uint32_t a = p_cols + s * 64u;
+                    const uint64_t hi = descQ0 + (uint64_t)((base + s * stage_bytes + kPTileBytes) >> 4), lo = descQ0 + (uint64_t)((lo_base + l * q_bytes) >> 4);
+                    if (begin || last) {
+                        for (int h = 0; h < halves && ok; ++h) {
+                            if (begin)  // the epilogue must have taken the chunk before
+                                for (int x = h; x < (halves == 2 ? h + 1 : 2) && ok; ++x) {
+                                    ok = mbar_wait_uniform(smem_u32(&ps.tempty[x]), (chunk & 1u) ^ 1u, abort_flag, p.status, CBK_TIMEOUT_TMEM_EMPTY);
+                                }
+                            if (!ok) break;
+                            tc_fence_after();
+                            const uint32_t d = tmem_base + (uint32_t)h * part_n;
+                            const uint64_t at = (uint64_t)((uint32_t)h * part_n * 8u);  // rows, or columns, of 128 bytes
+#pragma unroll
+                            for (uint32_t kk = 0; kk < kBK / 8; ++kk) {
+                                umma_tf32_ts_elect(d, a + 8 * kk, lo + at + kk * kStepQ, part_idesc, kk == 0 && begin ? 0u : 1u);
+                                umma_tf32_ts_elect(d, a + 32 + 8 * kk, hi + at + kk * kStepQ, part_idesc, 1u);
+                                umma_tf32_ts_elect(d, a + 8 * kk, hi + at + kk * kStepQ, part_idesc, 1u);
+                            }
+                            if (last)
+                                for (int x = h; x < (halves == 2 ? h + 1 : 2); ++x) tc_commit_elect(smem_u32(&ps.tfull[x]));
+                        }
+                        if (!ok) break;
+                    } else {
+#pragma unroll
+                        for (uint32_t kk = 0; kk < kBK / 8; ++kk) {
+                            umma_tf32_ts_elect(tmem_base, a + 8 * kk, lo + kk * kStepQ, idesc, 1u);
+                            umma_tf32_ts_elect(tmem_base, a + 32 + 8 * kk, hi + kk * kStepQ, idesc, 1u);
+                            umma_tf32_ts_elect(tmem_base, a + 8 * kk, hi + kk * kStepQ, idesc, 1u);
+                        }
+                    }
+                    tc_commit_elect(smem_u32(&ps.empty[s]));
+                    tc_commit_elect(smem_u32(&ps.lo_empty[l]));
+                    kc_pos = last ? 0 : kc_pos + 1;
+                    chunk += last ? 1u : 0u;
+                    if (++s == kX3Raw) { s = 0; ph ^= 1u; }
+                    l ^= 1u;
+                }
+            }
+        }
+    } else if (warp < 4 + kX3SplitWarps) {
+        // ------------------------------------------------------------ split warps: two a lane quarter, 16 k each of P; all of Q together
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kX3Regs[1]));
+        const int quarter = warp & 3, half = (warp - 4) >> 2, row = 32 * quarter + lane;
+        const uint32_t t = threadIdx.x - 128u, n_vec = q_bytes >> 4;
+        constexpr uint32_t kT = 32 * kX3SplitWarps;
+        uint32_t s = 0, ph = 0, l = 0, lph = 0;
+        bool ok = true;
+        for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
+            const WorkItem it = decode_work(p, w);
+            for (int kb = it.kb0; kb < it.kb1; ++kb) {
+                // (the raw stage was refilled after the UMMAs that read this stage of P had retired)
+                ok = mbar_wait_uniform(smem_u32(&ps.full[s]), ph, abort_flag, p.status, CBK_TIMEOUT_XFORM_FULL) &&
+                     mbar_wait_uniform(smem_u32(&ps.lo_empty[l]), lph ^ 1u, abort_flag, p.status, CBK_TIMEOUT_EMPTY);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t raw = base + s * stage_bytes;
+                uint32_t x[16], lo[16];
+                if (P_MN) {  // [32 k][32 rows] boxes, one a lane quarter, 32-byte chunks swizzled by k
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) {
+                        const uint32_t k = (uint32_t)(16 * half + e);
+                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(x[e]) : "r"(raw + (uint32_t)quarter * 4096u + k * 128u + ((((uint32_t)lane >> 3) ^ (k & 3u)) << 5) + ((uint32_t)lane & 7u) * 4u));
+                    }
+                } else {     // rows of 128 bytes, 16-byte chunks swizzled by row
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                                     : "=r"(x[4 * q]), "=r"(x[4 * q + 1]), "=r"(x[4 * q + 2]), "=r"(x[4 * q + 3])
+                                     : "r"(raw + (uint32_t)row * 128u + ((uint32_t)((4 * half + q) ^ (row & 7)) << 4)));
+                }
+#pragma unroll
+                for (int e = 0; e < 16; ++e) lo[e] = tf32_lo(__uint_as_float(x[e]));
+                const uint32_t at = p_cols + s * 64u + 16u * half + ((uint32_t)(32 * quarter) << 16);
+                tmem_st(at, x);
+                tmem_st(at + 32u, lo);
+                const uint32_t src = raw + kPTileBytes + t * 16u, dst = lo_base + l * q_bytes + t * 16u;
+                for (uint32_t v = 0; v < n_vec; v += 4 * kT) {
+                    float4 y[4];
+#pragma unroll
+                    for (uint32_t u = 0; u < 4; ++u)
+                        if (v + u * kT + t < n_vec)
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(y[u].x), "=f"(y[u].y), "=f"(y[u].z), "=f"(y[u].w) : "r"(src + (v + u * kT) * 16u));
+#pragma unroll
+                    for (uint32_t u = 0; u < 4; ++u)
+                        if (v + u * kT + t < n_vec)
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (v + u * kT) * 16u), "r"(tf32_lo(y[u].x)),
+                                         "r"(tf32_lo(y[u].y)), "r"(tf32_lo(y[u].z)), "r"(tf32_lo(y[u].w)) : "memory");
+                }
+                tmem_st_wait();
+                fence_proxy_async_smem();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&ps.xf[s]));
+                if (++s == kX3Raw) { s = 0; ph ^= 1u; }
+                l ^= 1u;
+                if (l == 0) lph ^= 1u;
+            }
+        }
+    } else {
+        // ------------------------------------------------------------ epilogue: four warps a lane quarter, up to 64 columns each
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kX3Regs[2]));
+        const int quarter = warp & 3, slot = (warp - 4 - kX3SplitWarps) >> 2, per = (p.bn + 63) / 64 * 16, first = slot * per, mine = min(per, p.bn - first);
+        uint32_t chunk = 0;
+        bool ok = true;
+        for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
+            const WorkItem it = decode_work(p, w);
+            const int nchunks = (it.kb1 - it.kb0 + p.kc - 1) / p.kc, i = it.i0 + 32 * quarter + lane;
+            float sum[4][16];
+            for (int ch = 0; ch < nchunks; ++ch, ++chunk) {
+                ok = mbar_wait_uniform(smem_u32(&ps.tfull[slot >> 1]), chunk & 1u, abort_flag, p.status, CBK_TIMEOUT_TMEM_FULL);
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (16 * q >= mine) break;
+                    uint32_t r[16];
+                    tmem_ld16(tmem_base + (uint32_t)(first + 16 * q) + ((uint32_t)(32 * quarter) << 16), r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) sum[q][e] = ch == 0 ? __uint_as_float(r[e]) : sum[q][e] + __uint_as_float(r[e]);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&ps.tempty[slot >> 1]));
+            }
+            if (!ok || i >= p.I) continue;
+            // One short pass over the sums for each thing to do: the code of a launch is fetched cold.
+            const int n = min(p.J - it.j0 - first, mine);  // columns of this warp that exist
+            float* dst = p.C + (long long)it.b * p.strideC + (long long)(it.j0 + first) * p.ldc + i;
+            if (it.kgroup == 0 && p.bias_i) {
+                const float bi = p.bias_i[i];
+#pragma unroll
+                for (int e = 0; e < 64; ++e) sum[e >> 4][e & 15] += bi;
+            }
+            if (it.kgroup == 0 && p.bias_j) {
+                const float* bj = p.bias_j + it.j0 + first;
+#pragma unroll
+                for (int e = 0; e < 64; ++e)
+                    if (e < n) sum[e >> 4][e & 15] += bj[e];
+            }
+            if (p.kgroups > 1) {
+#pragma unroll
+                for (int e = 0; e < 64; ++e, dst += p.ldc)
+                    if (e < n) atomicAdd(dst, sum[e >> 4][e & 15]);
+                continue;
+            }
+            if (p.accumulate) {
+                const float* from = dst;
+#pragma unroll
+                for (int q = 0; q < 64; q += 8) {  // loads in flight together
+                    float old[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e, from += p.ldc) old[e] = q + e < n ? *from : 0.f;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) sum[(q + e) >> 4][(q + e) & 15] += old[e];
+                }
+            }
+            if (p.relu)
+#pragma unroll
+                for (int e = 0; e < 64; ++e) sum[e >> 4][e & 15] = fmaxf(sum[e >> 4][e & 15], 0.f);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (16 * q >= n) break;
+#pragma unroll
+                for (int e = 0; e < 16; ++e, dst += p.ldc)
+                    if (16 * q + e < n) *dst = sum[q][e];
+            }
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (ps.abort_flag) {  // as in the kernel above
+        if ((warp == 0 || warp == 2) && lane == 0)
+            for (uint32_t st = 0; st < kX3Raw && st < fills; ++st) mbar_drain(smem_u32(&ps.full[st]), ((fills - 1 - st) / kX3Raw) & 1u, p.status);
+        if (warp == 1) {
+            tc_commit_elect(smem_u32(&ps.drain));
+            if (lane == 0) mbar_drain(smem_u32(&ps.drain), 0, p.status);
+        }
+        __syncthreads();
+    }
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, 512);
+    }
+}
+
 typedef void (*GemmKernel)(const CUtensorMap, const CUtensorMap, const GemmParams);
 template <bool X3, bool kCluster>
 GemmKernel kernel_for(bool p_mn, bool q_mn) {
@@ -489,8 +754,14 @@ GemmKernel kernel_for(bool p_mn, bool q_mn) {
     return q_mn ? umma_gemm_kernel<false, true, X3, kCluster> : umma_gemm_kernel<false, false, X3, kCluster>;
 }
 
+GemmKernel x3_kernel_for(bool p_mn, bool q_mn) {
+    if (p_mn) return q_mn ? umma_gemm_x3_kernel<true, true> : umma_gemm_x3_kernel<true, false>;
+    return q_mn ? umma_gemm_x3_kernel<false, true> : umma_gemm_x3_kernel<false, false>;
+}
+
 struct TileChoice {
     int mi, bn, stages, splits, kgroups;
+    int chunk;  // k-blocks an accumulator of umma_gemm_x3_kernel takes; 0: the general kernel
 };
 // How many clusters of 2 / 4 / 8 CTAs of this kernel the device holds at once. An SM holds one CTA and a cluster lies within
 // one GPC, so this is less than SMs / size; a grid beyond it runs its last clusters as a second wave (512^3 as 16 clusters
@@ -527,8 +798,8 @@ const ClusterRoom& cluster_room(const cb_ctx* ctx) {
 
 // Tile and contraction split by a model in SM clocks. Splits are the CTAs of one cluster, which add their partial tiles
 // through each other's shared memory: reproducible, no clearing launch, no atomics, any epilogue.
-TileChoice search_tile(int sm_count, const ClusterRoom& room, int smem_cap, const GemmCall& g, int num_kb, bool x3, bool may_add) {
-    TileChoice best{0, 16, 2, 1, 1};
+TileChoice search_tile(int sm_count, const ClusterRoom& room, int smem_cap, const GemmCall& g, int num_kb, bool x3, bool may_add, bool may_keep_p) {
+    TileChoice best{0, 16, 2, 1, 1, 0};
     double best_cost = 1e300;
     const int j_gran = g.q_mn ? 32 : 16;
     const bool full = !x3 && (double)g.batch * g.I * g.J > (double)sm_count * 128 * 256;
@@ -567,7 +838,7 @@ TileChoice search_tile(int sm_count, const ClusterRoom& room, int smem_cap, cons
                 if (splits > 1) cost += 4300.0 + 10.0 * bn_eff;  // two cluster barriers, the partial tiles' way through memory
                 if (cost < best_cost) {
                     best_cost = cost;
-                    best = TileChoice{mi, bn_eff, stages, splits, 1};
+                    best = TileChoice{mi, bn_eff, stages, splits, 1, 0};
                 }
             }
             // From about a thousand k on (a batch folded into K, mostly) several clusters on a tile, or single CTAs, which spare
@@ -584,9 +855,37 @@ TileChoice search_tile(int sm_count, const ClusterRoom& room, int smem_cap, cons
                     const double cost = per * kb_cyc + 5000.0 + 13.0 * bn_eff + 43.0 * bn_eff / size + (size > 1 ? 4300.0 + 10.0 * bn_eff : 0.0);
                     if (cost < best_cost) {
                         best_cost = cost;
-                        best = TileChoice{1, bn_eff, stages, size, groups};
+                        best = TileChoice{1, bn_eff, stages, size, groups, 0};
                     }
                 }
+        }
+    }
+    if (!x3 || !may_keep_p || best.mi == 0) return best;
+    // umma_gemm_x3_kernel, by clocks fitted to 31 shapes with every width and 1 to 4 shares: the choice was within 5 % of the best of
+    // them on all. Shares of a contraction may run one after the other in a CTA, whose tile leaves while the next is computed.
+    // Against the general kernel, us: 2048^3 110 -> 72; 2048 x 4096 x 1024 110 -> 72; 4096^2, K 64, 25 -> 21; 8192 x 256 x 1024 41 -> 29
+    // (two shares); 1024 x 1024 x 4096 59 -> 44 (four); 4096 x 128 x 4096 47 -> 27 (four); 512^3 10.8 -> 9.7; 300^3 stays with it.
+    // It stays the better one for reproducible sums of few tiles (clusters: 1024 x 1024 x 4096 81, here 81; 512^3 10.8, 12.8), to
+    // whose cost the model of it adds too little (the factor). A chunk is no longer than that kernel's, so the error
+    // against fp64 does not grow (K 2048: 3.8e-6 -> 1.9e-6 of the norm). Passes of models keep their sums.
+    best_cost = 1.12 * best_cost + 1000.0;
+    const int share = (num_kb + best.splits * best.kgroups - 1) / (best.splits * best.kgroups), chunk = share < kX3Chunk ? share : kX3Chunk;
+    for (int bn = 256; bn >= 32; bn >>= 1) {
+        const int bn_eff = bn < g.J ? bn : (g.J + j_gran - 1) / j_gran * j_gran;
+        if (bn_eff > 256 || bn_eff < j_gran || (bn >= 2 * g.J && bn > j_gran)) continue;
+        if (kX3Raw * (kPTileBytes + bn_eff * kBK * 4) + kX3Lo * bn_eff * kBK * 4 > smem_cap) continue;
+        const long long tiles = (long long)g.batch * ((g.I + 127) / 128) * ((g.J + bn_eff - 1) / bn_eff);
+        for (int groups = 1; groups == 1 || (may_add && (groups <= 4 || tiles * groups <= sm_count)); ++groups) {
+            const int per = (num_kb + groups - 1) / groups;
+            if (groups > 1 && (num_kb < 16 || per < 4)) break;
+            if ((groups - 1) * per >= num_kb) continue;  // an empty share
+            const double waves = (double)((tiles * groups + sm_count - 1) / sm_count), drains = (double)((per + chunk - 1) / chunk);
+            const double block = bn_eff > 68 ? 780.0 + 4.4 * bn_eff : 1080.0;
+            const double cost = waves * (per * block + 600.0 * drains + 1200.0 + 7.0 * bn_eff) + (groups > 1 ? 3500.0 + 20.0 * bn_eff : 0.0);
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = TileChoice{1, bn_eff, kX3Raw, 1, groups, chunk};
+            }
         }
     }
     return best;
@@ -611,7 +910,7 @@ int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3) {
     const int smem_cap = ctx->max_smem_optin - 2048;  // static barriers + 1 KB alignment slack
     // the search takes about a microsecond and depends on these numbers only: a thread keeps the last shapes' answers
     struct Known {
-        int I, J, batch, num_kb, q_mn, x3, sm_count, smem_cap, may_add;
+        int I, J, batch, num_kb, q_mn, x3, sm_count, smem_cap, may_add, model_pass;
         TileChoice choice;
     };
     static thread_local Known table[64];
@@ -619,10 +918,11 @@ int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3) {
     const uint32_t h = ((uint32_t)g.I * 0x9E3779B1u) ^ ((uint32_t)g.J * 0x85EBCA77u) ^ ((uint32_t)num_kb * 0xC2B2AE3Du) ^ (uint32_t)g.batch * 31u;
     Known& known = table[(h >> 20) & 63u];
     if (known.I != g.I || known.J != g.J || known.batch != g.batch || known.num_kb != num_kb || known.q_mn != g.q_mn ||
-        known.x3 != (int)x3 || known.sm_count != ctx->sm_count || known.smem_cap != smem_cap || known.may_add != (int)may_add)
-        known = Known{g.I, g.J, g.batch, num_kb, g.q_mn, x3 ? 1 : 0, ctx->sm_count, smem_cap, may_add ? 1 : 0,
-                      search_tile(ctx->sm_count, cluster_room(ctx), smem_cap, g, num_kb, x3, may_add)};
+        known.x3 != (int)x3 || known.sm_count != ctx->sm_count || known.smem_cap != smem_cap || known.may_add != (int)may_add || known.model_pass != (int)ctx->model_pass)
+        known = Known{g.I, g.J, g.batch, num_kb, g.q_mn, x3 ? 1 : 0, ctx->sm_count, smem_cap, may_add ? 1 : 0, ctx->model_pass ? 1 : 0,
+                      search_tile(ctx->sm_count, cluster_room(ctx), smem_cap, g, num_kb, x3, may_add, !ctx->model_pass)};
     const TileChoice choice = known.choice;
+    const bool p_tmem = choice.chunk > 0;
     if (choice.mi == 0) return fail(ctx, CB_EUNSUPPORTED, "umma gemm: no tile configuration fits");
 
     GemmParams gp{};
@@ -637,8 +937,8 @@ int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3) {
     if (gp.kgroups == 1) gp.splits = (num_kb + gp.kb_per_split - 1) / gp.kb_per_split;  // no empty split
     const bool cluster = gp.splits > 1;
     // 3xTF32: the tensor core's fp32 accumulation error grows with the number of accumulated products, so the
-    // accumulator is drained into C (round-to-nearest fp32 adds) every 512 k
-    gp.kc = x3 ? kChunk3x : (1 << 30);
+    // accumulator is drained with round-to-nearest fp32 adds: into C every 512 k, into registers at least every 256
+    gp.kc = x3 ? (p_tmem ? choice.chunk : kChunk3x) : (1 << 30);
     int cols = 32;
     while (cols < 2 * gp.bn) cols <<= 1;
     gp.tmem_cols = cols;
@@ -699,7 +999,7 @@ int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3) {
 
     const long long work = (long long)gp.batch * gp.tiles_i * gp.tiles_j * gp.kgroups * gp.splits;
     const int hi = gp.mi * kPTileBytes + gp.bn * kBK * 4;
-    const int stage = x3 ? 2 * hi : hi;
+    const int stage = x3 && !p_tmem ? 2 * hi : hi;
     int tile_bytes = 0;
     if (cluster) {
         // The partial tile goes over the stages once they are idle; a 3xTF32 share of more than one accumulation chunk adds
@@ -712,9 +1012,9 @@ int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3) {
     }
     gp.split_groups = gp.stages >= 4 ? 2 : 1;
     const int grid = cluster ? (int)work : (int)(work < ctx->sm_count ? work : ctx->sm_count);
-    size_t smem = (size_t)gp.stages * stage + 1024;
+    size_t smem = (size_t)gp.stages * stage + 1024 + (p_tmem ? kX3Lo * gp.bn * kBK * 4 : 0);
     if (smem < gp.tile_offset + (size_t)tile_bytes + 1024) smem = gp.tile_offset + (size_t)tile_bytes + 1024;
-    const GemmKernel kernel = x3 ? (cluster ? kernel_for<true, true>(g.p_mn, g.q_mn) : kernel_for<true, false>(g.p_mn, g.q_mn))
+    const GemmKernel kernel = p_tmem ? x3_kernel_for(g.p_mn, g.q_mn) : x3 ? (cluster ? kernel_for<true, true>(g.p_mn, g.q_mn) : kernel_for<true, false>(g.p_mn, g.q_mn))
                                  : (cluster ? kernel_for<false, true>(g.p_mn, g.q_mn) : kernel_for<false, false>(g.p_mn, g.q_mn));
     if (gp.kgroups > 1 && !g.accumulate) {
         const int rc = clear_output(ctx, g.C, g.I, g.ldc, g.J, g.strideC, g.batch, "clear of a split product");
@@ -724,7 +1024,7 @@ int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3) {
     cudaError_t e = raise_dynamic_smem_once(kernel, ctx->device, ctx->max_smem_optin, &bound);
     if (e == cudaSuccess && (int)smem > bound) e = cudaErrorInvalidValue;
     if (e == cudaSuccess)
-        e = launch_dep_on(ctx->stream, ctx->pdl != 0, kernel, dim3((unsigned)grid), dim3(96 + 32 * kEpiWarps + (x3 ? 32 * kSplitWarps : 0)), smem,
+        e = launch_dep_on(ctx->stream, ctx->pdl != 0, kernel, dim3((unsigned)grid), dim3(p_tmem ? kX3Threads : 96 + 32 * kEpiWarps + (x3 ? 32 * kSplitWarps : 0)), smem,
                           cluster ? gp.splits : 1, tp, tq, gp);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return check_cuda(ctx, e, "umma_gemm_kernel launch");
