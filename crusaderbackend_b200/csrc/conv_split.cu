@@ -42,13 +42,16 @@ struct SplitGather {
     const GatherParams& p;
     const PixelSet& s;
     TapK* table;             // [kLoaders]
+    int* woffs;              // [kLoaders]: TapK::woff, two neighbours in one load without bank conflicts
     const float* img;        // a loader thread's pixel: its image, its taps, offset of the first tap
     Position at;
     int base;
     long long i0, pixels;
     int j0, block0, part;
     __device__ __forceinline__ void prepare(int t, int tid) {
-        table[tid] = tap_of<MASK>(p, s, (block0 + t) * kBK + tid);
+        const TapK e = tap_of<MASK>(p, s, (block0 + t) * kBK + tid);
+        table[tid] = e;
+        woffs[tid] = e.woff;
     }
     __device__ __forceinline__ void load(int t, int tid, float (&vp)[SP::kValues], float (&vq)[SQ::kValues]) {
         const TapK* tab = table + t % (S::kLoaders / kBK) * kBK;
@@ -58,7 +61,8 @@ struct SplitGather {
             const bool ok = tap_inside<MASK>(at, q.bits, p.H, p.W) && (MASK || q.woff >= 0);
             vp[x] = split::load_if(img + (base + q.off), ok);
         }
-        const int w0 = tab[SQ::k(tid, 0)].woff, w1 = tab[SQ::k(tid, 0) + 1].woff;
+        const int2 w = *reinterpret_cast<const int2*>(woffs + t % (S::kLoaders / kBK) * kBK + SQ::k(tid, 0));
+        const int w0 = w.x, w1 = w.y;
 #pragma unroll
         for (int u = 0; u < SQ::kUnits; ++u) {
             const float* row = p.Wt + (long long)min(j0 + SQ::row(tid, u), p.OUTC - 1) * p.w_out;
@@ -97,9 +101,10 @@ __global__ void __launch_bounds__(S::NT, S::kCtas) conv_gather_split(const __gri
     extern __shared__ uint8_t smem[];
     __shared__ split::Barriers bars;
     __shared__ TapK table[S::kLoaders];
+    __shared__ __align__(8) int woffs[S::kLoaders];
     const int set = blockIdx.z / p.splits, part = blockIdx.z - set * p.splits;
     const PixelSet& s = p.sets[set];
-    SplitGather<S, MASK> src{p, s, table, p.In, Position{-(1 << 29), 0, 0u}, 0, (long long)blockIdx.x * S::BM, (long long)p.N * s.UH * s.UW,
+    SplitGather<S, MASK> src{p, s, table, woffs, p.In, Position{-(1 << 29), 0, 0u}, 0, (long long)blockIdx.x * S::BM, (long long)p.N * s.UH * s.UW,
                              (int)blockIdx.y * S::BN, part * p.per_split, part};
     const int blocks = min(p.per_split, (s.K + kBK - 1) / kBK - src.block0);
     // the grid is sized for the largest set; a share without a block has nothing to add, but a set without any product is still stored
@@ -123,23 +128,35 @@ struct SplitWgrad {
     typedef split::ShareP<S, kP> SP;
     typedef split::ShareQ<S, kQ> SQ;
     const WgradParams& p;
-    PixelK* table;           // [kLoaders]
+    // PixelK of kLoaders pixels, field by field: lanes read neighbouring pixels, entries of 32 bytes were 2- to 8-way bank conflicts
+    // (shared memory was busy 1440 clocks of a block's 2640). 32 -> 64 channels, 32 x 32, stride 2, batch 128: 29.3 -> 24.0 us, with the
+    // patches of put_p; 64 -> 64, 32 x 32, batch 128: 230 -> 208.
+    longlong2* ys;           // [kLoaders / 2]
+    long long* xs;           // [kLoaders]
+    Position* at;            // [kLoaders]; MASK: only the masks, as words
     const TapI* rows;        // [BM]
     int i0, j0, block0, opix;
     __device__ __forceinline__ void prepare(int t, int tid) {
-        table[tid] = pixel_of<MASK>(p, (block0 + t) * kBK + tid);
+        const PixelK e = pixel_of<MASK>(p, (block0 + t) * kBK + tid);
+        xs[tid] = e.x;
+        reinterpret_cast<long long*>(ys)[tid] = e.y;
+        if (MASK) reinterpret_cast<uint32_t*>(at)[tid] = e.at.mask;
+        else at[tid] = e.at;
     }
     __device__ __forceinline__ void load(int t, int tid, float (&vp)[SP::kValues], float (&vq)[SQ::kValues]) {
-        const PixelK* tab = table + t % (S::kLoaders / kBK) * kBK;
-        const PixelK q = tab[SP::k(tid, 0)];
-        const float* first = p.X + q.x;
+        const int tab = t % (S::kLoaders / kBK) * kBK, k = tab + SP::k(tid, 0);
+        const float* first = p.X + xs[k];
+        Position here{0, 0, 0u};
+        if (MASK) here.mask = reinterpret_cast<const uint32_t*>(at)[k];
+        else here = at[k];
 #pragma unroll
         for (int x = 0; x < SP::kValues; ++x) {
             const TapI w = rows[SP::row(tid, x)];
-            const bool ok = tap_inside<MASK>(q.at, w.bits, p.g.IH, p.g.IW) && (MASK || w.off >= 0);
+            const bool ok = tap_inside<MASK>(here, w.bits, p.g.IH, p.g.IW) && (MASK || w.off >= 0);
             vp[x] = split::load_if(first + w.off, ok);
         }
-        const long long y0 = tab[SQ::k(tid, 0)].y, y1 = tab[SQ::k(tid, 0) + 1].y;
+        const longlong2 y = ys[(tab + SQ::k(tid, 0)) / 2];
+        const long long y0 = y.x, y1 = y.y;
 #pragma unroll
         for (int u = 0; u < SQ::kUnits; ++u) {
             const float* row = p.dY + (long long)min(j0 + SQ::row(tid, u), p.g.OC - 1) * opix;
@@ -169,12 +186,14 @@ template <class S, bool MASK>
 __global__ void __launch_bounds__(S::NT, S::kCtas) conv_wgrad_split(const __grid_constant__ WgradParams p, int* status) {
     extern __shared__ uint8_t smem[];
     __shared__ split::Barriers bars;
-    __shared__ float patches[split::ShareP<S, split::K>::kPatches];
-    __shared__ PixelK table[S::kLoaders];
+    __shared__ __align__(16) float patches[split::ShareP<S, split::K>::kPatches];
+    __shared__ longlong2 ys[S::kLoaders / 2];
+    __shared__ long long xs[S::kLoaders];
+    __shared__ Position at[MASK ? (S::kLoaders + 2) / 3 : S::kLoaders];
     __shared__ TapI rows[S::BM];
     const int i0 = blockIdx.x * S::BM;
     for (int e = threadIdx.x; e < S::BM; e += S::NT) rows[e] = row_of<MASK>(p, i0 + e);  // read behind the barrier of run()
-    SplitWgrad<S, MASK> src{p, table, rows, i0, (int)blockIdx.y * S::BN, (int)blockIdx.z * p.per_split, p.g.OH * p.g.OW};
+    SplitWgrad<S, MASK> src{p, ys, xs, at, rows, i0, (int)blockIdx.y * S::BN, (int)blockIdx.z * p.per_split, p.g.OH * p.g.OW};
     split::run<S>(src, min(p.per_split, (p.pixels + kBK - 1) / kBK - src.block0), smem, bars, patches, status);
 }
 

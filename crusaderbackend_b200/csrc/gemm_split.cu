@@ -147,7 +147,7 @@ template <class S, Kind KP, Kind KQ>
 __global__ void __launch_bounds__(S::NT, S::kCtas) split_gemm_kernel(const __grid_constant__ SplitParams p) {
     extern __shared__ uint8_t smem[];
     __shared__ split::Barriers bars;
-    __shared__ float patches[split::ShareP<S, KP>::kPatches];
+    __shared__ __align__(16) float patches[split::ShareP<S, KP>::kPatches];
     const int b = blockIdx.z / p.splits, part = blockIdx.z - b * p.splits;
     GemmSource<S, KP, KQ> src{p, b, part, (int)blockIdx.x * S::BM, (int)blockIdx.y * S::BN, part * p.per_split};
     split::run<S>(src, min(p.per_split, p.blocks - src.block0), smem, bars, patches, p.status);

@@ -61,8 +61,7 @@ template <class S, Kind KIND>
 struct ShareP {
     static_assert(KIND != KV, "");
     static constexpr int kValues = S::BM * kBK / S::kLoaders;
-    static constexpr int kPatchRow = kValues + 1;                    // words: read by columns
-    static constexpr int kPatch = 32 * kPatchRow;                    // words of a warp
+    static constexpr int kPatch = 32 * kValues;                      // words of a warp
     static constexpr int kPatches = KIND == K ? S::kLoaders / 32 * kPatch : 1;
     // row and k of value x
     static __device__ __forceinline__ int row(int tid, int x) {
@@ -148,12 +147,18 @@ __device__ __forceinline__ void put_p(float (&v)[ShareP<Sh, KIND>::kValues], uin
     typedef ShareP<Sh, KIND> S;
     constexpr int V = S::kValues;
     if (KIND == K) {
-        const uint32_t mine = patch + (uint32_t)(lane / V * S::kPatchRow + lane % V) * 4u;
+        // [32 rows][V k], 16-byte chunks exchanged by row * V / 32: a store is 32 words in a row, eight lanes read eight chunks of
+        // different banks (rows of V + 1 words read word by word: two conflicts a store, four times the loads)
+        constexpr int kChunks = V / 4;
 #pragma unroll
-        for (int x = 0; x < V; ++x) asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + x * (32u / V * S::kPatchRow * 4u)), "f"(v[x]) : "memory");
+        for (int x = 0; x < V; ++x)  // row lane / V + 32 / V * x, k lane % V
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(patch + (uint32_t)(32 * x + (lane ^ (x % kChunks * 4))) * 4u), "f"(v[x]) : "memory");
         __syncwarp();
 #pragma unroll
-        for (int x = 0; x < V; ++x) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[x]) : "r"(patch + (uint32_t)(lane * S::kPatchRow + x) * 4u) : "memory");
+        for (int c = 0; c < kChunks; ++c)
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v[4 * c]), "=f"(v[4 * c + 1]), "=f"(v[4 * c + 2]), "=f"(v[4 * c + 3])
+                         : "r"(patch + (uint32_t)(lane * V + 4 * (c ^ (lane * V / 32 % kChunks))) * 4u) : "memory");
         __syncwarp();
     }
     uint32_t p[3][V / 2];
