@@ -29,7 +29,7 @@
 //
 // Covered geometry: stride 1, filter 1x1 (pad 0) or 3x3 (pad 1) per axis, W in {8,16,32}, (32/W) | H,
 // FW * OC(rounded to 16) <= 256 per CTA, packed filter slice <= ~150 KB; stride 2 through the phase split below.
-// Everything else is served by the CUDA-core kernels in conv_simt.cu.
+// Everything else is served by the gathers of conv_simt.cu (CUDA cores) and conv_split.cu (tensor cores at fp32 accuracy).
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>

@@ -1,5 +1,5 @@
-// CUDA-core fp32 GEMM: CB_MATH_FP32 and every operand pair TMA cannot address, on the shared main loop of simt_core.cuh,
-// and split-K kernels for thin products.
+// CUDA-core fp32 GEMM: CB_MATH_FP32 and operand pairs TMA cannot address, as far as gemm_split.cu does not take them, on the shared
+// main loop of simt_core.cuh; kernels for thin products and short contractions.
 #include <utility>
 
 #include "cb_ptx.cuh"

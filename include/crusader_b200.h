@@ -33,7 +33,8 @@ enum {
 enum {
     CB_MATH_TF32 = 0,   /* operands truncated to TF32 by the tensor core, fp32 accumulate */
     CB_MATH_3XTF32 = 1, /* hi/lo split, three tensor-core products per term: fp32-class accuracy */
-    CB_MATH_FP32 = 2    /* CUDA-core fp32 FMA kernels (exact fp32; used for shapes TMA cannot address) */
+    CB_MATH_FP32 = 2    /* fp32 accuracy (also where TMA cannot address an operand): FMAs on the CUDA cores, or, where a product is
+                           large enough, six bf16 tensor-core products of three-way split values, summed in fp32 */
 };
 
 /* ---- context ------------------------------------------------------------------------------- */
