@@ -27,7 +27,7 @@ struct cb_ctx {
     int math = CB_MATH_TF32;
     int sync = 0;
     int deterministic = 0;
-    bool model_pass = false;  // set while a model's forward or backward pass is queued
+    bool model_pass = false;  // set while a model's forward or backward pass is queued; always on the contexts of its weight-gradient streams
     int* d_status = nullptr;       // device status word (0 = ok, CBK_* otherwise)
     void* workspace = nullptr;     // scratch: split-K partials, packed filters
     size_t workspace_bytes = 0;

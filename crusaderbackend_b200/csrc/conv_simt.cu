@@ -276,9 +276,9 @@ int fp32_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, con
         return fail(ctx, CB_EUNSUPPORTED, std::string(who) + ": more than 2^31 pixels or filter values");
     const bool mask = g.FH <= kMaskTaps && g.FW <= kMaskTaps;
     p.I = (int)I; p.pixels = (int)pixels;
-    // a CTA of conv_wgrad_split holds an SM, which a stream beside this one would miss (ResNet-50 on 16 x 16 images, batch 78: 2300 us
-    // a step against 2263)
-    const bool on_tensor_cores = ctx->wgrad_grid_cap == 0 && split::worth_it(I, g.OC, pixels, 1, kLeastConv);
+    // Not in a model's backward pass, on whichever stream (cbt_set_wgrad_streams moves launches, it does not choose kernels): a CTA of
+    // conv_wgrad_split holds an SM, which the stream beside it would miss (ResNet-50 on 16 x 16 images, batch 78: 2300 us a step against 2263)
+    const bool on_tensor_cores = !ctx->model_pass && split::worth_it(I, g.OC, pixels, 1, kLeastConv);
     simt::Choice c{};
     split::Choice sc{};
     if (on_tensor_cores) sc = split::choose_shape(ctx->sm_count, I, g.OC, (pixels + split::kBK - 1) / split::kBK, 1, !ctx->deterministic, 2.5);
@@ -462,9 +462,9 @@ static int conv_wgrad_impl(cb_ctx* ctx, const float* dY, const float* X, float* 
     if (!dY || !X) return fail(ctx, CB_EINVAL, std::string(who) + ": null operand");
     // 3xTF32: the products dY_hi X_hi, dY_hi X_lo, dY_lo X_hi in one launch that walks the pixels three times
     const bool x3 = ctx->math == CB_MATH_3XTF32;
-    // (contexts whose weight gradients run beside another stream keep the kernel that leaves it half the SMs: a DenseNet-100 step took
-    // 3571 us with its widest layers here, 3561 without)
-    if (ctx->math != CB_MATH_FP32 && (ctx->deterministic || ctx->wgrad_grid_cap > 0 || !((x3 && x3_at_fp32(g)) || wgrad_at_fp32(g, x3)))) {
+    // (models keep the kernel that leaves half the SMs to the stream beside it: a DenseNet-100 step took 3571 us with its widest layers
+    // here, 3561 without; without such streams too, or a gradient's accuracy would depend on their number)
+    if (ctx->math != CB_MATH_FP32 && (ctx->deterministic || ctx->model_pass || !((x3 && x3_at_fp32(g)) || wgrad_at_fp32(g, x3)))) {
         rc = umma_conv_wgrad(ctx, dY, X, dW, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, accumulate, dy_batch, x_batch, x3);
         if (rc == CB_OK && x3) ctx->last_kernel = "umma_3xtf32";
         if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;

@@ -204,6 +204,33 @@ def test_wgrad_streams_do_not_change_results(torch_cuda):
     assert results[3][2] <= results[0][2]   # the default context adds into the gradient directly: no second kernel
 
 
+@pytest.mark.parametrize("math", ["tf32", "fp32"])
+def test_wide_layers_take_one_route_whatever_the_streams(torch_cuda, math):
+    """Filters of more output channels than the weight-gradient kernel's accumulator holds (1x1 to 160): on a default context too the
+    gradients of an inline pass and of one on side streams differ by the order of fp32 sums alone (1e-5; TF32 products against
+    fp32 ones part by 2e-3)."""
+    torch = torch_cuda
+    from crusaderbackend_b200.api import Context
+    from crusaderbackend_b200.train import DenseNetTrainer
+    _, _, dimg, dlab = make_batch(torch, 16, 16, 10, "wide")
+    grads = []
+    for n in (0, 2):
+        ctx = Context(0, math=math)
+        tr = DenseNetTrainer(ctx, batch=16, growth=40, layers=2, image_hw=16)
+        tr.set_wgrad_streams(n)
+        tr.init_params("wide")
+        tr.forward(dimg, dlab)
+        tr.backward()
+        ctx.synchronize()
+        grads.append(tr.grads.cpu().numpy())
+        entries = tr.entries
+        tr.close()
+        ctx.close()
+    for e in entries:
+        inline, aside = (g[e["offset"]:e["offset"] + e["size"]] for g in grads)
+        assert orc.max_err_norm(inline, aside) <= 1e-5, (e["kind"], e["dims"])
+
+
 def test_resnet56_loss_tracks_fp32_run(torch_cuda):
     """ResNet-56, batch 128 of N(0,1) CIFAR-shaped images, uniform labels, He init, momentum 0.9, lr 0.01/128, 200 steps
     on a repeated batch: the loss of the TF32 and of the 3xTF32 tensor-core run stays within 1 % (of the curve's largest
