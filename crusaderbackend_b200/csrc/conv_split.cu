@@ -70,18 +70,6 @@ struct SplitGather {
             vq[2 * u + 1] = split::load_if(row + w1, w1 >= 0);
         }
     }
-    __device__ __forceinline__ bool covers(int row, int col) const { return i0 + row < pixels && j0 + col < p.OUTC; }
-    __device__ __noinline__ float plain(int row, int col, int blocks) const {
-        const float* image;
-        const Position where = input_of<MASK>(p, s, i0 + row, image);
-        float sum = 0.f;
-        for (int k = block0 * kBK; k < min(s.K, (block0 + blocks) * kBK); ++k) {
-            const TapK q = tap_of<MASK>(p, s, k);
-            const float x = tap_inside<MASK>(where, q.bits, p.H, p.W) ? image[where.h0 * p.W + where.w0 + q.off] : 0.f;
-            sum = fmaf(x, p.Wt[(long long)(j0 + col) * p.w_out + q.woff], sum);
-        }
-        return sum;
-    }
     __device__ __forceinline__ void store(int row, int first, int n, uint32_t mine) const {
         if (i0 + row >= pixels) return;
         float* out;
@@ -163,17 +151,6 @@ struct SplitWgrad {
             vq[2 * u] = split::load_if(row + y0, y0 >= 0);
             vq[2 * u + 1] = split::load_if(row + y1, y1 >= 0);
         }
-    }
-    __device__ __forceinline__ bool covers(int row, int col) const { return i0 + row < p.I && j0 + col < p.g.OC; }
-    __device__ __noinline__ float plain(int row, int col, int blocks) const {
-        const TapI w = row_of<MASK>(p, i0 + row);
-        float sum = 0.f;
-        for (int k = block0 * kBK; k < min(p.pixels, (block0 + blocks) * kBK); ++k) {
-            const PixelK q = pixel_of<MASK>(p, k);
-            const float x = tap_inside<MASK>(q.at, w.bits, p.g.IH, p.g.IW) ? p.X[q.x + w.off] : 0.f;
-            sum = fmaf(x, p.dY[q.y + (long long)(j0 + col) * opix], sum);
-        }
-        return sum;
     }
     __device__ __forceinline__ void store(int row, int first, int n, uint32_t mine) const {
         const int i = i0 + row, j = j0 + first;

@@ -95,18 +95,6 @@ struct GemmSource {
         load_p<S, kP>(vp, p.P + pair * p.strideP, p.ldp, i0, p.I, k, p.K, tid);
         load_q<S, kQ>(vq, p.Q + pair * p.strideQ, p.ldq, j0, p.J, k, p.K, tid);
     }
-    __device__ __forceinline__ bool covers(int row, int col) const { return i0 + row < p.I && j0 + col < p.J; }
-    __device__ __noinline__ float plain(int row, int col, int blocks) const {
-        float sum = 0.f;
-        for (int t = block0; t < block0 + blocks; ++t) {
-            int pair, k;
-            where(t, pair, k);
-            const float *P = p.P + pair * p.strideP, *Q = p.Q + pair * p.strideQ;
-            for (const int end = min(p.K, k + kBK); k < end; ++k)
-                sum = fmaf(*element<kP>(P, p.ldp, i0 + row, k), *element<kQ>(Q, p.ldq, j0 + col, k), sum);
-        }
-        return sum;
-    }
     __device__ __forceinline__ void store(int row, int first, int n, uint32_t mine) const {
         const int i = i0 + row;
         n = min(n, p.J - j0 - first);

@@ -183,14 +183,64 @@ __device__ __forceinline__ float load_if(const float* src, bool ok) {
     return v;
 }
 
-// The loader threads alone (named barrier 1).
+// The loader threads alone (named barrier 1); all threads, from within their roles (2).
 template <class S>
 __device__ __forceinline__ void loader_sync() { asm volatile("bar.sync 1, %0;" ::"n"(S::kLoaders) : "memory"); }
+template <class S>
+__device__ __forceinline__ void all_sync() { asm volatile("bar.sync 2, %0;" ::"n"(S::NT) : "memory"); }
 
 struct __align__(8) Barriers {
     uint64_t full[kStages], empty[kStages], tfull[kAcc], tempty[kAcc], drain;
     uint32_t tmem_base;
     int abort_flag;
+    int again;  // the tile has outputs that fp32 FMAs have to form
+};
+
+// The second pass over the contraction, by fp32 FMAs in k order, for the outputs of a tile that the pieces cannot give. The loaders
+// fetch the blocks once more and leave them as they are in shared memory, kSliceK at a time behind the sums: [k][128 rows],
+// [k][BN columns]; the summing threads multiply. An infinity or a NaN in one operand makes whole rows of outputs need this, so it is a
+// product like any other: 64 FMAs a thread and k at BN = 128, 4096 clocks a block as on the CUDA cores. us, finite values / a NaN in
+// every output / the latter with one thread an output, whose every step waits for its loads: 256 x 256 x 8192 in one share
+// 190 / 750 / 10190, 1000 x 777 x 1501 36 / 187 / 2330, weight gradient 16 -> 64 of 8 maps of 28 x 28 in one share 180 / 770 / 60300.
+template <class S>
+struct Again {
+    static constexpr int kSliceK = S::BN / 4;
+    static_assert(kBK % kSliceK == 0 && S::BN * 512 + kSliceK * (S::BM + S::BN) * 4 <= kStages * (int)S::kStageBytes, "");
+    template <Kind KP, Kind KQ>
+    static __device__ __forceinline__ void put(const float (&vp)[ShareP<S, KP>::kValues], const float (&vq)[ShareQ<S, KQ>::kValues], int first, uint32_t slice, int tid) {
+        typedef ShareP<S, KP> P;
+        typedef ShareQ<S, KQ> Q;
+#pragma unroll
+        for (int x = 0; x < P::kValues; ++x) {
+            const int k = P::k(tid, x) - first;
+            if ((unsigned)k < (unsigned)kSliceK)
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(slice + (uint32_t)(k * S::BM + P::row(tid, x)) * 4u), "f"(vp[x]) : "memory");
+        }
+        if (!Q::active(tid)) return;
+#pragma unroll
+        for (int x = 0; x < Q::kValues; ++x) {
+            const int k = Q::k(tid, x / Q::kUnit) + x % Q::kUnit - first;
+            if ((unsigned)k < (unsigned)kSliceK)
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(slice + (uint32_t)((kSliceK * S::BM + k * S::BN) + Q::row(tid, x / Q::kUnit)) * 4u), "f"(vq[x]) : "memory");
+        }
+    }
+    // row, first: the thread's outputs
+    static __device__ __forceinline__ void add(float (&sum)[S::kCols], uint32_t slice, int row, int first) {
+        for (int k = 0; k < kSliceK; ++k) {
+            float p;
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(p) : "r"(slice + (uint32_t)(k * S::BM + row) * 4u) : "memory");
+#pragma unroll
+            for (int c = 0; c < S::kCols; c += 4) {
+                float q0, q1, q2, q3;
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q0), "=f"(q1), "=f"(q2), "=f"(q3)
+                             : "r"(slice + (uint32_t)(kSliceK * S::BM + k * S::BN + first + c) * 4u) : "memory");
+                sum[c] = fmaf(p, q0, sum[c]);
+                sum[c + 1] = fmaf(p, q1, sum[c + 1]);
+                sum[c + 2] = fmaf(p, q2, sum[c + 2]);
+                sum[c + 3] = fmaf(p, q3, sum[c + 3]);
+            }
+        }
+    }
 };
 
 // Value of column c (of a summing thread's own) where it left its sums.
@@ -203,8 +253,8 @@ __device__ __forceinline__ float staged(uint32_t mine, int c) {
 // The whole kernel behind its index arithmetic: `blocks` k-blocks of the tile through `src`.
 // Source: kP, kQ (Kind); prepare(t, tid), when kTable: entry tid of the table that load() of block t and the kLoaders / 32 - 1 after it
 // may read;
-// load(t, tid, p, q): this thread's values of block t; store(row, first, n, mine): outputs (row, first .. first + n - 1) of the tile,
-// to be read by staged(); covers(row, column), plain(row, column, blocks): whether the tile has the output, its value by fp32 FMAs.
+// load(t, tid, p, q): this thread's values of block t, asked for in ascending order from 0 on, at most twice over;
+// store(row, first, n, mine): outputs (row, first .. first + n - 1) of the tile, to be read by staged().
 // patches: ShareP::kPatches floats of shared memory.
 template <class S, class Src>
 __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Barriers& b, float* patches, int* status) {
@@ -213,6 +263,7 @@ __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Bar
     volatile int* abort_flag = &b.abort_flag;
     if (threadIdx.x == 0) {
         b.abort_flag = 0;
+        b.again = 0;
         for (int s = 0; s < kStages; ++s) {
             mbar_init(smem_u32(&b.full[s]), S::kLoaders / 32);
             mbar_init(smem_u32(&b.empty[s]), 1);
@@ -234,6 +285,7 @@ __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Bar
     griddep_wait();
     griddep_launch();
     const uint32_t tmem_base = b.tmem_base;
+    const uint32_t slice = st_base + S::BN * 512u;  // of a second pass, behind the sums
 
     if (warp >= S::kSumWarps) {
         if (S::NT == 768) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(S::kLoaderRegs));
@@ -276,6 +328,16 @@ __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Bar
             fetch(t + 2, p[0], q[0]);
             if (t + 1 < blocks) ok = ok && store_block(p[1], q[1]);
         }
+        all_sync<S>();
+        if (b.again && !b.abort_flag)
+            for (int t = 0; t < blocks; ++t) {
+                fetch(t, p[0], q[0]);
+                for (int k = 0; k < kBK; k += Again<S>::kSliceK) {
+                    all_sync<S>();  // the slice before this one has been read
+                    Again<S>::template put<Src::kP, Src::kQ>(p[0], q[0], k, slice, tid);
+                    all_sync<S>();
+                }
+            }
     } else {
         if (S::NT == 768) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(S::kSumRegs));
         const int quarter = warp & 3, first = (warp >> 2) * S::kCols;
@@ -341,13 +403,14 @@ __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Bar
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&b.tempty[a]));
         }
+        // Every UMMA has read its operands: the stages take the sums, so that what follows is a loop (unrolled over registers, its
+        // branches took longer to fetch than a small product to compute).
+        // A value the three pieces cannot carry (an infinity, a NaN) or a sum that left the range on the way shows as a result that is
+        // not finite: such outputs are formed again.
+        const int row = 32 * quarter + lane;
+        const uint32_t mine = st_base + (uint32_t)(first * 128 + row) * 4u;
+        bool all = true;
         if (ok) {
-            // Every UMMA has read its operands: the stages take the sums, so that what follows is a loop (unrolled over registers, its
-            // branches took longer to fetch than a small product to compute).
-            // A value the three pieces cannot carry (an infinity, a NaN) or a sum that left the range on the way shows as a result that is not finite: it is formed again by fp32 FMAs in k order.
-            const int row = 32 * quarter + lane;
-            const uint32_t mine = st_base + (uint32_t)(first * 128 + row) * 4u;
-            bool all = true;
 #pragma unroll
             for (int c = 0; c < S::kCols; c += 2) {
                 float lo, hi;
@@ -356,11 +419,28 @@ __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Bar
                 asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + c * 512u), "f"(lo) : "memory");
                 asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + c * 512u + 512u), "f"(hi) : "memory");
             }
-            if (!all)
+        }
+        const bool wanted = __any_sync(0xffffffffu, !all);
+        if (wanted) b.again = 1;
+        else if (ok) src.store(row, first, S::kCols, mine);
+        all_sync<S>();
+        if (b.again && !b.abort_flag) {
+            float plain[S::kCols];
+#pragma unroll
+            for (int c = 0; c < S::kCols; ++c) plain[c] = 0.f;
+            for (int t = 0; t < blocks; ++t)
+                for (int k = 0; k < kBK; k += Again<S>::kSliceK) {
+                    all_sync<S>();
+                    all_sync<S>();
+                    if (wanted) Again<S>::add(plain, slice, row, first);
+                }
+            if (wanted) {
+#pragma unroll
                 for (int c = 0; c < S::kCols; ++c)
-                    if (!(fabsf(staged(mine, c)) <= 3.402823466e38f) && src.covers(row, first + c))
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + c * 512u), "f"(src.plain(row, first + c, blocks)) : "memory");
-            src.store(row, first, S::kCols, mine);
+                    if (!(fabsf(staged(mine, c)) <= 3.402823466e38f))
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + c * 512u), "f"(plain[c]) : "memory");
+                src.store(row, first, S::kCols, mine);
+            }
         }
     }
 

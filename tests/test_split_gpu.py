@@ -149,3 +149,104 @@ def test_passes_of_the_other_modes_that_run_at_fp32_accuracy(math, geo, kern):
     assert orc.max_err_norm(dX[:n].cpu().numpy(), orc.conv_dgrad(W, dY[:n], X[:n].shape, (s, s), (p, p))) <= tol[1]
     ref = torch.nn.grad.conv2d_weight(tX.double(), W.shape, tdY.double(), stride=s, padding=p)
     assert orc.max_err_norm(dW.cpu().numpy(), ref.cpu().numpy()) <= tol[2]
+
+
+def _elapsed_us(call, reps=3):
+    import torch
+    call()
+    best = float("inf")
+    for _ in range(reps):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        call()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b) * 1e3)
+    return best
+
+
+def _same_bad_places(got, want, tol=TOL):
+    """NaN where the reference has NaN, its infinities where it has them, and its finite values elsewhere."""
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    inf = np.isinf(want)
+    assert np.array_equal(np.isinf(got), inf) and np.array_equal(got[inf], want[inf].astype(np.float32))
+    ok = np.isfinite(want)
+    assert not ok.any() or np.abs(got[ok] - want[ok]).max() <= tol * np.abs(want[ok]).max()
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("M,N,K", [(1030, 1030, 95), (300, 260, 1000), (70, 2049, 513), (2049, 40, 256)])
+@pytest.mark.parametrize("pad", [1, 4])
+def test_products_with_whole_rows_that_are_not_finite(ctx, M, N, K, form, pad):
+    """Tiles of every shape in which some outputs, or all, are formed again: an infinity in every row of one factor, NaNs in single
+    columns of the other, on both sides of the tiles' edges and in the contraction's first, middle and ragged last block."""
+    import torch
+    tA, tB = FORMS[form]
+    A, B = orc.uniform_pm1((M, K), "again", M, N, K, "A"), orc.uniform_pm1((K, N), "again", M, N, K, "B")
+    for i in (0, 31, M - 1):
+        A[i, (i * 7) % K] = np.inf if i % 2 else -np.inf
+    B[K - 1, N - 1], B[K // 2, 3] = np.nan, np.inf
+    every = A.copy()
+    every[:, K // 3] = np.inf
+    for a in (A, every):
+        with np.errstate(invalid="ignore"):
+            want = a.astype(np.float64) @ B
+        sA, sB = np.ascontiguousarray(a.T if tA else a), np.ascontiguousarray(B.T if tB else B)
+        dA, dB = (torch.from_numpy(np.pad(s, ((0, 0), (0, pad)))).cuda()[:, :s.shape[1]] for s in (sA, sB))
+        C = torch.full((M, N), 7.0, device="cuda")
+        for det in (False, True):
+            ctx.set_deterministic(det)
+            ctx.gemm(dA, dB, C, transA=tA, transB=tB)
+            ctx.set_deterministic(False)
+            assert ctx.last_kernel == "umma_fp32"
+            _same_bad_places(C.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("geo", [(9, 17, 28, 28, 33, 3, 1, 1), (3, 16, 31, 45, 64, 3, 2, 1), (33, 20, 13, 13, 100, 3, 3, 1), (2, 16, 45, 44, 20, 17, 1, 8)])
+@pytest.mark.parametrize("det", [False, True])
+def test_convolutions_with_values_that_are_not_finite(ctx, geo, det):
+    """Infinities in the input and NaNs in the output gradient: all three passes against the same sums as matrix products in fp64."""
+    import torch
+    N, IC, H, W_, OC, F, s, p = geo
+    W = torch.from_numpy(orc.he_normal_filter(OC, IC, F, F, ("bad", geo)))
+    X = torch.from_numpy(orc.normal((N, IC, H, W_), "bad", geo, "X"))
+    OH, OW = orc.conv_out_hw(H, W_, F, F, s, s, p, p)
+    dY = torch.from_numpy(orc.normal((N, OC, OH, OW), "bad", geo, "dY"))
+    X[0, 2, 5, 7], X[N - 1, IC - 1, H - 1, W_ - 1] = float("inf"), float("-inf")
+    dY[0, 1, 2, 3], dY[N - 1, OC - 1, OH - 1, OW - 1] = float("nan"), float("inf")
+    cols = torch.nn.functional.unfold(X.double(), F, padding=p, stride=s)
+    fwd = (W.double().reshape(OC, -1) @ cols).reshape(dY.shape)
+    wgrad = torch.einsum("nop,nkp->ok", dY.double().reshape(N, OC, -1), cols).reshape(W.shape)
+    dgrad = torch.nn.functional.fold(W.double().reshape(OC, -1).T @ dY.double().reshape(N, OC, -1), (H, W_), F, padding=p, stride=s)
+    tW, tX, tdY = W.cuda(), X.cuda(), dY.cuda()
+    Y, dX, dW = torch.empty_like(tdY), torch.empty_like(tX), torch.zeros_like(tW)
+    ctx.set_deterministic(det)
+    kern = []
+    for call in (lambda: ctx.conv(tW, tX, Y, s, s, p, p), lambda: ctx.convDerive(tW, tdY, dX, s, s, p, p), lambda: ctx.convError(tdY, tX, dW, s, s, p, p)):
+        call()
+        kern.append(ctx.last_kernel)
+    ctx.set_deterministic(False)
+    assert kern == ["umma_fp32"] * 3
+    for got, want in ((Y, fwd), (dX, dgrad), (dW, wgrad)):
+        _same_bad_places(got.cpu().numpy(), want.numpy())
+
+
+def test_values_that_are_not_finite_cost_a_second_pass(ctx):
+    """A program whose training has diverged: a NaN in every output. Forming them again takes a pass over the contraction by fp32 FMAs,
+    four times the clocks of a pass on the tensor cores and as many blocks to fetch: bounded by ten times the time of finite values (one
+    thread an output, one product after the other, took hundreds)."""
+    import torch
+    A, B = torch.randn(256, 8192, device="cuda"), torch.randn(8192, 256, device="cuda")
+    C = torch.empty(256, 256, device="cuda")
+    X, dY, dW = torch.randn(8, 16, 28, 28, device="cuda"), torch.randn(8, 64, 28, 28, device="cuda"), torch.zeros(64, 16, 3, 3, device="cuda")
+    for det in (False, True):
+        ctx.set_deterministic(det)
+        for call, bad in ((lambda: ctx.gemm(A, B, C), A[:, 4000]), (lambda: ctx.convError(dY, X, dW, 1, 1, 1, 1), dY[0, :, 0, 0])):
+            finite = _elapsed_us(call)
+            assert ctx.last_kernel == "umma_fp32"
+            keep = bad.clone()
+            bad.fill_(float("nan"))
+            again = _elapsed_us(call)
+            bad.copy_(keep)
+            assert again <= 10 * finite, (det, finite, again)
+        ctx.set_deterministic(False)
