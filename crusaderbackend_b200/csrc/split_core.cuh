@@ -2,8 +2,8 @@
 // operands the TMA-fed kernels cannot address, where the product is large enough to pay for it. One kernel body serves the GEMM
 // forms and the three convolution passes; an operand source (below) says where element (i, k) lies.
 //
-// Every fp32 value is the sum of three bf16 values: x = x1 + x2 + x3 with x1 = x cut off, x2 = x - x1 rounded, x3 the rest, all of it
-// exact (8 + 8 + 8 significant bits, the exponent range is that of fp32). Six of the nine products of two such sums leave out less
+// Every fp32 value from 2^-110 on is the sum of three bf16 values: x = x1 + x2 + x3 with x1 = x cut off, x2 = x - x1 rounded, x3 the rest,
+// all of it exact (8 + 8 + 8 significant bits; below, the third runs into bf16's least subnormal, 2^-133: see kLow). Six of the nine products of two such sums leave out less
 // than 2^-23 of the product (x2 y3 + x3 y2, of either sign: x2 is rounded for that; 2^-26 on average): x2 y2, x1 y3, x3 y1, x1 y2,
 // x2 y1, x1 y1, issued smallest first. What the tensor
 // core does not give is fp32's rounding of sums (TMEM truncates every addition), so no chain of additions there is longer than two
@@ -31,6 +31,7 @@ constexpr uint32_t kPieceRow = 64;  // bytes: 32 bf16
 constexpr int kAcc = 2;             // accumulators in TMEM
 constexpr int kStages = 4;
 constexpr int kChunk = 2;           // k-blocks a sum in TMEM runs over
+constexpr float kFinite = 3.402823466e38f, kWhole = 0x1p-110f, kLow = 0x1p-70f;  // see where the sums are checked
 constexpr uint32_t kPCols = 48;     // TMEM columns of a stage of P: three pieces of 32 k, two a column
 
 // What a loader does is a chain of latencies (fetch, three dependent steps of a split, store, fences): with eight loader warps an SM a
@@ -193,10 +194,24 @@ struct __align__(8) Barriers {
     uint64_t full[kStages], empty[kStages], tfull[kAcc], tempty[kAcc], drain;
     uint32_t tmem_base;
     int abort_flag;
-    int again;  // the tile has outputs that fp32 FMAs have to form
+    int again;    // the tile has outputs that fp32 FMAs have to form
+    int cut;      // found on the way: factors below 2^-110; the largest factor's magnitude, as bits
+    unsigned largest;
 };
 
-// The second pass over the contraction, by fp32 FMAs in k order, for the outputs of a tile that the pieces cannot give. The loaders
+__device__ __forceinline__ float word(uint32_t at) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+    return v;
+}
+// Value of column c (of a summing thread's own) where it left its sums.
+__device__ __forceinline__ float staged(uint32_t mine, int c) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(mine + (uint32_t)c * 512u));
+    return v;
+}
+
+// The second pass over the contraction, by fp32 FMAs in k order, for the outputs of a tile that the pieces do not give. The loaders
 // fetch the blocks once more and leave them as they are in shared memory, kSliceK at a time behind the sums: [k][128 rows],
 // [k][BN columns]; the summing threads multiply. An infinity or a NaN in one operand makes whole rows of outputs need this, so it is a
 // product like any other: 64 FMAs a thread and k at BN = 128, 4096 clocks a block as on the CUDA cores. us, finite values / a NaN in
@@ -224,31 +239,50 @@ struct Again {
                 asm volatile("st.shared.f32 [%0], %1;" ::"r"(slice + (uint32_t)((kSliceK * S::BM + k * S::BN) + Q::row(tid, x / Q::kUnit)) * 4u), "f"(vq[x]) : "memory");
         }
     }
-    // row, first: the thread's outputs
-    static __device__ __forceinline__ void add(float (&sum)[S::kCols], uint32_t slice, int row, int first) {
-        for (int k = 0; k < kSliceK; ++k) {
-            float p;
-            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(p) : "r"(slice + (uint32_t)(k * S::BM + row) * 4u) : "memory");
+    // The summing threads': (row, first ...) are a thread's outputs, staged from `mine` on; wanted: whether its warp has some to form.
+    static __device__ __noinline__ void sum(Barriers& b, int blocks, uint32_t slice, uint32_t mine, int row, int first, bool wanted) {
+        float plain[S::kCols];
 #pragma unroll
-            for (int c = 0; c < S::kCols; c += 4) {
-                float q0, q1, q2, q3;
-                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q0), "=f"(q1), "=f"(q2), "=f"(q3)
-                             : "r"(slice + (uint32_t)(kSliceK * S::BM + k * S::BN + first + c) * 4u) : "memory");
-                sum[c] = fmaf(p, q0, sum[c]);
-                sum[c + 1] = fmaf(p, q1, sum[c + 1]);
-                sum[c + 2] = fmaf(p, q2, sum[c + 2]);
-                sum[c + 3] = fmaf(p, q3, sum[c + 3]);
+        for (int c = 0; c < S::kCols; ++c) plain[c] = 0.f;
+        for (int s = 0; s < blocks * (kBK / kSliceK); ++s) {
+            all_sync<S>();
+            all_sync<S>();
+            // whether the slice holds factors below kWhole, and its largest finite factor (what an infinity touches is not finite)
+            unsigned largest = 0;
+#pragma unroll 1
+            for (int i = threadIdx.x; i < kSliceK * (S::BM + S::BN); i += 32 * S::kSumWarps) {
+                const float v = fabsf(word(slice + (uint32_t)i * 4u));
+                if (v > 0.f && v < kWhole) b.cut = 1;
+                if (v <= kFinite) largest = max(largest, __float_as_uint(v));
             }
+            largest = __reduce_max_sync(0xffffffffu, largest);
+            if ((threadIdx.x & 31) == 0) atomicMax(&b.largest, largest);
+            if (!wanted) continue;
+            for (int k = 0; k < kSliceK; ++k) {
+                const float p = word(slice + (uint32_t)(k * S::BM + row) * 4u);
+#pragma unroll
+                for (int c = 0; c < S::kCols; c += 4) {
+                    float q0, q1, q2, q3;
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q0), "=f"(q1), "=f"(q2), "=f"(q3)
+                                 : "r"(slice + (uint32_t)(kSliceK * S::BM + k * S::BN + first + c) * 4u) : "memory");
+                    plain[c] = fmaf(p, q0, plain[c]);
+                    plain[c + 1] = fmaf(p, q1, plain[c + 1]);
+                    plain[c + 2] = fmaf(p, q2, plain[c + 2]);
+                    plain[c + 3] = fmaf(p, q3, plain[c + 3]);
+                }
+            }
+        }
+        asm volatile("bar.sync 3, %0;" ::"n"(32 * S::kSumWarps) : "memory");  // the loaders are through with theirs
+        if (!wanted) return;
+        // magnitude from which on what was lost is less than 2^-24 of an output
+        const float least = b.cut ? __uint_as_float(b.largest) * 0x1p-60f * (float)(blocks * kBK) * 0x1p-49f : 0.f;
+#pragma unroll
+        for (int c = 0; c < S::kCols; ++c) {
+            const float v = fabsf(staged(mine, c));
+            if (!(v <= kFinite) || v < least) asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + c * 512u), "f"(plain[c]) : "memory");
         }
     }
 };
-
-// Value of column c (of a summing thread's own) where it left its sums.
-__device__ __forceinline__ float staged(uint32_t mine, int c) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(mine + (uint32_t)c * 512u));
-    return v;
-}
 
 // The whole kernel behind its index arithmetic: `blocks` k-blocks of the tile through `src`.
 // Source: kP, kQ (Kind); prepare(t, tid), when kTable: entry tid of the table that load() of block t and the kLoaders / 32 - 1 after it
@@ -263,7 +297,8 @@ __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Bar
     volatile int* abort_flag = &b.abort_flag;
     if (threadIdx.x == 0) {
         b.abort_flag = 0;
-        b.again = 0;
+        b.again = b.cut = 0;
+        b.largest = 0;
         for (int s = 0; s < kStages; ++s) {
             mbar_init(smem_u32(&b.full[s]), S::kLoaders / 32);
             mbar_init(smem_u32(&b.empty[s]), 1);
@@ -329,7 +364,7 @@ __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Bar
             if (t + 1 < blocks) ok = ok && store_block(p[1], q[1]);
         }
         all_sync<S>();
-        if (b.again && !b.abort_flag)
+        if (b.again && !b.abort_flag) {
             for (int t = 0; t < blocks; ++t) {
                 fetch(t, p[0], q[0]);
                 for (int k = 0; k < kBK; k += Again<S>::kSliceK) {
@@ -338,6 +373,7 @@ __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Bar
                     all_sync<S>();
                 }
             }
+        }
     } else {
         if (S::NT == 768) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(S::kSumRegs));
         const int quarter = warp & 3, first = (warp >> 2) * S::kCols;
@@ -405,42 +441,34 @@ __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Bar
         }
         // Every UMMA has read its operands: the stages take the sums, so that what follows is a loop (unrolled over registers, its
         // branches took longer to fetch than a small product to compute).
-        // A value the three pieces cannot carry (an infinity, a NaN) or a sum that left the range on the way shows as a result that is
-        // not finite: such outputs are formed again.
+        // Outputs that are formed again. A value that has no pieces (an infinity, a NaN) or a sum that left the range on the way shows as a
+        // result that is not finite. A factor below kWhole loses up to 2^-133, what lies under bf16's least subnormal, so outputs are off by
+        // up to K 2^-133 times the largest factor. Asking every factor cost the loaders 1 to 4 % of a launch; so an output below kLow
+        // (but not 0) brings the second pass, which looks at the factors. Outputs above it may be off by more than 2^-24 of
+        // themselves only where K times the largest factor exceeds 2^39.
         const int row = 32 * quarter + lane;
         const uint32_t mine = st_base + (uint32_t)(first * 128 + row) * 4u;
-        bool all = true;
+        uint64_t zeros = 0;
+        unsigned smallest = 0xffffffffu;
         if (ok) {
 #pragma unroll
             for (int c = 0; c < S::kCols; c += 2) {
                 float lo, hi;
                 unpack2(sum[c / 2], lo, hi);
-                all = all && fabsf(lo) <= 3.402823466e38f && fabsf(hi) <= 3.402823466e38f;
+                // a product with 0 is a NaN for what is not finite; the bits without their sign, less one, put 0 above everything
+                asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(zeros) : "l"(sum[c / 2]), "l"(0ull));
+                smallest = min(smallest, min(2u * __float_as_uint(lo) - 1u, 2u * __float_as_uint(hi) - 1u));
                 asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + c * 512u), "f"(lo) : "memory");
                 asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + c * 512u + 512u), "f"(hi) : "memory");
             }
         }
-        const bool wanted = __any_sync(0xffffffffu, !all);
+        const bool wanted = __any_sync(0xffffffffu, (zeros & 0x7fffffff7fffffffull) != 0 || smallest < 2u * __float_as_uint(kLow) - 1u);
         if (wanted) b.again = 1;
         else if (ok) src.store(row, first, S::kCols, mine);
         all_sync<S>();
         if (b.again && !b.abort_flag) {
-            float plain[S::kCols];
-#pragma unroll
-            for (int c = 0; c < S::kCols; ++c) plain[c] = 0.f;
-            for (int t = 0; t < blocks; ++t)
-                for (int k = 0; k < kBK; k += Again<S>::kSliceK) {
-                    all_sync<S>();
-                    all_sync<S>();
-                    if (wanted) Again<S>::add(plain, slice, row, first);
-                }
-            if (wanted) {
-#pragma unroll
-                for (int c = 0; c < S::kCols; ++c)
-                    if (!(fabsf(staged(mine, c)) <= 3.402823466e38f))
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + c * 512u), "f"(plain[c]) : "memory");
-                src.store(row, first, S::kCols, mine);
-            }
+            Again<S>::sum(b, blocks, slice, mine, row, first, wanted);
+            if (wanted) src.store(row, first, S::kCols, mine);
         }
     }
 

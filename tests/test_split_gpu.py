@@ -74,8 +74,7 @@ def test_batches_and_dense_layers(ctx):
 
 
 def test_values_the_pieces_cannot_carry(ctx):
-    """Infinities, NaNs and sums that leave the range: such outputs are formed again by fp32 FMAs. Values down to where the last
-    piece is a bf16 subnormal keep their accuracy."""
+    """Infinities, NaNs and sums that leave the range: such outputs are formed again by fp32 FMAs."""
     import torch
     A, B = orc.uniform_pm1((300, 200), "split", "nA"), orc.uniform_pm1((200, 300), "split", "nB")
     A[3, 5], A[9, 2], A[100, 1], B[7, 11] = np.inf, np.nan, 3.4e38, -np.inf
@@ -250,3 +249,60 @@ def test_values_that_are_not_finite_cost_a_second_pass(ctx):
             bad.copy_(keep)
             assert again <= 10 * finite, (det, finite, again)
         ctx.set_deterministic(False)
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("scale", [1e-30, 8e-34, 4e-34, 1e-35, 5e-38, 1e-40])
+@pytest.mark.parametrize("other", [1.0, 1e6])
+def test_factors_below_the_range_of_three_pieces(ctx, form, scale, other):
+    """Below 2^-110 the third piece is cut off. A factor of that size, all over or in some rows beside ordinary ones, keeps fp32
+    accuracy: TOL of the row's largest output, plus the rounding of subnormal sums, 2^-150 an FMA. Shares of a contraction meet in
+    memory by atomic adds, which take a subnormal for 0: 2^-126 each."""
+    import torch
+    tA, tB = FORMS[form]
+    M, N, K = 300, 330, 257
+    A = orc.uniform_pm1((M, K), "low", scale, "A")
+    A *= np.where((np.arange(M) % 3 == 0) | (M - 1 == np.arange(M)), scale, 1.0 if other == 1.0 else scale)[:, None]
+    A = (A * (orc.uniform_pm1((M, K), "low", "mask") > 0)).astype(np.float32)
+    B = (orc.uniform_pm1((K, N), "low", scale, "B") * other).astype(np.float32)
+    B[:, 17] = 0
+    for a, b in ((A, B), (np.ascontiguousarray(B.T), np.ascontiguousarray(A.T))):
+        want = a.astype(np.float64) @ b
+        dA, dB = torch.from_numpy(np.ascontiguousarray(a.T if tA else a)).cuda(), torch.from_numpy(np.ascontiguousarray(b.T if tB else b)).cuda()
+        C = torch.full(want.shape, 7.0, device="cuda")
+        for det in (False, True):
+            ctx.set_deterministic(det)
+            ctx.gemm(dA, dB, C, transA=tA, transB=tB)
+            ctx.set_deterministic(False)
+            assert ctx.last_kernel == "umma_fp32"
+            axis = 1 if a is A else 0
+            worst = np.abs(want).max(axis=axis, keepdims=True)
+            assert (np.abs(C.cpu().numpy() - want) <= TOL * worst + K * 2.0 ** -150 + (0 if det else 128 * 2.0 ** -126)).all()
+
+
+@pytest.mark.parametrize("geo", [(9, 17, 28, 28, 33, 3, 1, 1), (3, 16, 31, 45, 64, 3, 2, 1), (33, 20, 13, 13, 100, 3, 3, 1), (2, 16, 45, 44, 20, 17, 1, 8)])
+def test_convolutions_of_factors_below_the_range_of_three_pieces(ctx, geo):
+    """The output gradient of a saturated loss: some channels and images around 1e-36, the others ordinary. Relative to the largest output of
+    an image, or of a filter: a sum of K FMAs is a random walk of K roundings by up to 2^-24 of it, 2^-24 sqrt(K / 3) of standard
+    deviation, seven of them allowed; atomic adds of shares take a subnormal for 0, 2^-126 each."""
+    import torch
+    N, IC, H, W_, OC, F, s, p = geo
+    OH, OW = orc.conv_out_hw(H, W_, F, F, s, s, p, p)
+    W, X, dY = orc.he_normal_filter(OC, IC, F, F, ("low", geo)), orc.normal((N, IC, H, W_), "low", geo, "X"), orc.normal((N, OC, OH, OW), "low", geo, "dY")
+    X[0] *= np.float32(3e-36)
+    dY[0] *= np.float32(1e-36)
+    dY[:, 1] *= np.float32(2e-36)
+    tW, tX, tdY = (torch.from_numpy(v).cuda() for v in (W, X, dY))
+    Y, dX, dW = torch.empty_like(tdY), torch.empty_like(tX), torch.zeros_like(tW)
+    for det in (False, True):
+        ctx.set_deterministic(det)
+        dW.zero_()
+        for call in (lambda: ctx.conv(tW, tX, Y, s, s, p, p), lambda: ctx.convDerive(tW, tdY, dX, s, s, p, p), lambda: ctx.convError(tdY, tX, dW, s, s, p, p)):
+            call()
+            assert ctx.last_kernel == "umma_fp32"
+        ctx.set_deterministic(False)
+        for K, got, want in ((IC * F * F, Y, orc.conv_fwd(W, X, None, (s, s), (p, p))), (OC * F * F, dX, orc.conv_dgrad(W, dY, X.shape, (s, s), (p, p))),
+                             (N * OH * OW, dW, orc.conv_wgrad(dY, X, W.shape, (s, s), (p, p)))):
+            g, w = (v.reshape(v.shape[0], v.shape[1], -1) if got is not dW else v.reshape(v.shape[0], 1, -1) for v in (got.cpu().numpy(), np.asarray(want, dtype=np.float64)))
+            scale = np.abs(w).max(axis=(1, 2), keepdims=True)  # an image's, or an output channel's
+            assert (np.abs(g - w) <= 4 * 2.0 ** -24 * K ** 0.5 * scale + (0 if det else 128 * 2.0 ** -126)).all()
