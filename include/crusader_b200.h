@@ -34,7 +34,14 @@ enum {
     CB_MATH_TF32 = 0,   /* operands truncated to TF32 by the tensor core, fp32 accumulate */
     CB_MATH_3XTF32 = 1, /* hi/lo split, three tensor-core products per term: fp32-class accuracy */
     CB_MATH_FP32 = 2    /* fp32 accuracy (also where TMA cannot address an operand): FMAs on the CUDA cores, or, where a product is
-                           large enough, six bf16 tensor-core products of three-way split values, summed in fp32 */
+                           large enough, six bf16 tensor-core products of three-way split values, summed in fp32. The errors
+                           of the latter against fp64 are smaller than the FMAs' in dense dot products (2-norm, 512 terms:
+                           1.0e-7 against 4.1e-7) and larger where all but some 16 terms are 0, as with diagonal or masked
+                           factors: one term 5.5e-8, 2.9e-7 at most, against 2.5e-8 and 6.0e-8; four 6.6e-8 against 4.0e-8 (a
+                           term with a power of two is exact). Factors below 2^-110 count whole in outputs below 2^-70, and
+                           in all of them where the number of terms times the largest factor is below 2^39; elsewhere what
+                           lies under 2^-133 in them is cut off. Outputs that are not finite, or below 2^-70 but not 0, take
+                           a second pass, by FMAs: up to five times the time of the first. */
 };
 
 /* ---- context ------------------------------------------------------------------------------- */

@@ -251,6 +251,31 @@ def test_values_that_are_not_finite_cost_a_second_pass(ctx):
         ctx.set_deterministic(False)
 
 
+@pytest.mark.parametrize("terms", [1, 2, 4])
+def test_dot_products_of_few_terms(ctx, terms):
+    """Rows with one to four values that are not 0 in a contraction of 512 (a diagonal, a mask). Of a term the three products left out
+    are at most 2 x 2^-7 2^-16 = 2^-22 (the pieces: 8 bits cut off, so x2 < 2^-7, x3 < 2^-16); a term's largest product is truncated by up to
+    2^-23 when it is added, its five small ones together by as much at most, and its chain's sum is rounded by 2^-24 once: (1.5 terms +
+    3) 2^-23 of the sum of the terms' magnitudes. A term with a power of two is exact."""
+    import torch
+    M, N, K = 512, 320, 512
+    rng = np.random.default_rng(terms)
+    A, B = np.zeros((M, K), np.float32), orc.normal((K, N), "few", terms)
+    for i in range(M):
+        A[i, rng.choice(K, terms, replace=False)] = rng.standard_normal(terms)
+    for a, b in ((A, B), (np.ascontiguousarray(B.T), np.ascontiguousarray(A.T))):
+        C = torch.empty(a.shape[0], b.shape[1], device="cuda")
+        ctx.gemm(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), C)
+        assert ctx.last_kernel == "umma_fp32"
+        want, size = a.astype(np.float64) @ b, np.abs(a).astype(np.float64) @ np.abs(b)
+        assert (np.abs(C.cpu().numpy() - want) <= (1.5 * terms + 3) * 2.0 ** -23 * size).all()
+        if terms == 1:
+            two = np.where(a == 0, 0, np.copysign(2.0 ** np.floor(np.log2(np.abs(a) + (a == 0))), a)).astype(np.float32) if a is A else a
+            other = b if a is A else np.where(b == 0, 0, np.copysign(2.0 ** np.floor(np.log2(np.abs(b) + (b == 0))), b)).astype(np.float32)
+            ctx.gemm(torch.from_numpy(two).cuda(), torch.from_numpy(other).cuda(), C)
+            assert np.array_equal(C.cpu().numpy(), two.astype(np.float64) @ other)
+
+
 @pytest.mark.parametrize("form", list(FORMS))
 @pytest.mark.parametrize("scale", [1e-30, 8e-34, 4e-34, 1e-35, 5e-38, 1e-40])
 @pytest.mark.parametrize("other", [1.0, 1e6])
