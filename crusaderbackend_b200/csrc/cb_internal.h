@@ -47,7 +47,7 @@ struct cb_ctx {
     long long filter_version = 0;  // bumped by every call that may have changed a filter's values
     void* filter_cache = nullptr;  // the cache itself (conv_sm100.cu)
     std::vector<std::pair<const float*, const float*>> bound_params;  // parameter buffers of the models on this context
-    int pdl = 1;                   // launch kernels that call griddep_wait with programmatic stream serialization
+    int pdl = 1;                   // launch kernels that call griddep_wait_then_launch with programmatic stream serialization
     void* wgrad_acc = nullptr;     // weight-gradient accumulator [column][row], all zero between calls (wgrad_sm100.cu)
     size_t wgrad_acc_bytes = 0;
     int wgrad_grid_cap = 0;        // > 0: most CTAs a weight-gradient kernel uses (contexts that run beside another stream)
@@ -83,8 +83,8 @@ const char* status_name(int s);
 // Returns after an optional sync; maps a non-zero device status word to CB_ETIMEOUT.
 int finish(cb_ctx* ctx, const char* what);
 // Launches `kernel` on the context's stream; with ctx->pdl the launch carries the programmatic-stream-serialization
-// attribute, so ONLY for kernels whose every thread calls griddep_wait() before its first access to global memory
-// that an earlier kernel may have written or may still read.
+// attribute, so ONLY for kernels whose every thread calls griddep_wait_then_launch() before its first access to global memory that
+// an earlier kernel may have written or may still read (cb_ptx.cuh has the one exception and what it rests on).
 template <typename... KArgs, typename... Args>
 cudaError_t launch_dep_on(cudaStream_t stream, bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                           int cluster, Args&&... args) {

@@ -97,15 +97,21 @@ enum : int {
     CBK_TIMEOUT_DRAIN = 107       // drain of in-flight copies after an abort
 };
 
+// Programmatic dependent launch. A kernel launched with the programmatic-serialization attribute may start while the kernel before
+// it on the stream is still running. griddepcontrol.wait returns once that kernel has completed and its writes are visible
+// (immediately for a kernel launched without the attribute); griddepcontrol.launch_dependents lets the kernel after this one begin the
+// same way, once every block has issued it or exited. Both are one call here, always in this order, because of what rests on it:
+// when a kernel starts, a block of its predecessor has come back from the wait, so the kernel BEFORE the predecessor has completed.
+// (So no kernel may end all its blocks without this call, and none may issue launch_dependents ahead of the wait.) Ahead of the call a
+// kernel may thus read what was written at least two kernels ago on its stream, or what its stream waited for then; it must
+// not read what the kernel just before it may have written, nor write anything. bn_bwd_par_kernel reads ahead, no other.
+__device__ __forceinline__ void griddep_wait_then_launch() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Bounded wait: gives up after CB_WAIT_LIMIT_NS of wall time (or when another role raised the abort
 // flag). Returns true when the phase completed, false on abort/timeout.
-// Programmatic dependent launch. A kernel launched with the programmatic-serialization attribute may start while
-// the kernel before it on the stream is still running: griddep_wait returns once that kernel has completed and its
-// writes are visible (immediately for a kernel launched without the attribute), so everything before it must touch
-// no global memory another kernel produces; griddep_launch lets the kernel after this one begin the same way.
-__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 __device__ __forceinline__ bool mbar_wait_for(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
                                               int code, uint64_t limit_ns) {
     // Reading %globaltimer costs ~600 clocks: a wait that looked at it whenever its first poll failed bound every pipeline

@@ -63,8 +63,7 @@ template <class T, bool MASK>
 __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_gather_simt(const __grid_constant__ GatherParams p) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ TapK table[2 * simt::kBK];
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const int set = blockIdx.z / p.splits, split = blockIdx.z - set * p.splits;
     const PixelSet& s = p.sets[set];
     const long long pixels = (long long)p.N * s.UH * s.UW;
@@ -157,8 +156,7 @@ __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_wgrad_simt(const Wgra
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ PixelK table[2 * simt::kBK];
     __shared__ TapI rows[T::BM];
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const int i0 = blockIdx.x * T::BM;
     for (int e = threadIdx.x; e < T::BM; e += T::NT) rows[e] = row_of<MASK>(p, i0 + e);
     WgradSource<T, MASK> src{p, table, rows, (int)blockIdx.y * T::BN, (int)blockIdx.z * p.per_split, p.g.OH * p.g.OW};

@@ -234,8 +234,7 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, kEpiWarps == 8 ? 2 : 1)
     // Up to here nothing has touched global memory (barriers, descriptor prefetch of kernel parameters, TMEM): the
     // kernel before this one may still be running. From here on its results are complete, and the kernel after this
     // one may begin its own preamble.
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const uint32_t tmem_base = cs.tmem_base;
     const uint32_t acc_stride = (uint32_t)p.tmem_cols >> 1;
     uint32_t fills = 0;  // producer: stages filled so far
@@ -492,14 +491,12 @@ __device__ __forceinline__ float pack_value(const PackJob& j, unsigned i) {
 }
 
 __global__ void pack_filter_kernel(const PackJob j) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < j.total; i += gridDim.x * blockDim.x) j.Wp[i] = pack_value(j, i);
 }
 // Every cached filter of a context in one launch: blockIdx.y indexes a device table of jobs.
 __global__ void pack_filter_table_kernel(const PackJob* __restrict__ jobs) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const PackJob j = jobs[blockIdx.y];
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < j.total; i += gridDim.x * blockDim.x) j.Wp[i] = pack_value(j, i);
 }
@@ -508,8 +505,7 @@ __global__ void pack_filter_table_kernel(const PackJob* __restrict__ jobs) {
 // Xs[n][phase*C + c][i][j] = X[n][c][2i + (phase >> 1)][2j + (phase & 1)]
 __global__ void space_to_depth2_kernel(const float* __restrict__ X, float* __restrict__ Xs, int C, int H, int W,
                                        long long total) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const int H2 = H / 2, W2 = W / 2;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
@@ -526,8 +522,7 @@ __global__ void space_to_depth2_kernel(const float* __restrict__ X, float* __res
 // dX[n][c][y][x] (+)= dXs[group][n][o][y/2][x/2] with phase*C + c = group*per_group + o
 __global__ void depth_to_space2_kernel(const float* __restrict__ dXs, float* __restrict__ dX, int N, int C, int H, int W,
                                        int per_group, long long total, int accumulate) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const int H2 = H / 2, W2 = W / 2;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
@@ -546,8 +541,7 @@ __global__ void depth_to_space2_kernel(const float* __restrict__ dXs, float* __r
 // Xsub[nc][i][j] = X[nc][2i][2j]
 __global__ void subsample2_kernel(const float* __restrict__ X, float* __restrict__ Xsub, long long NC, int H, int W,
                                   long long total) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const int H2 = H / 2, W2 = W / 2;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
@@ -561,8 +555,7 @@ __global__ void subsample2_kernel(const float* __restrict__ X, float* __restrict
 // dX[nc][y][x] (+)= (y, x both even) ? dXsub[nc][y/2][x/2] : 0
 __global__ void upsample2_zero_kernel(const float* __restrict__ dXsub, float* __restrict__ dX, int H, int W,
                                       long long total, int accumulate) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const int H2 = H / 2, W2 = W / 2;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
@@ -588,8 +581,7 @@ struct PlaneIndex {      // item -> (plane n * C + c, row y, quad q)
 constexpr int kRelayoutItems = 4;
 __global__ void __launch_bounds__(256) space_to_depth2_vec_kernel(const float* __restrict__ X, float* __restrict__ Xs, const PlaneIndex ix,
                                                                   int W2, long long plane2, uint32_t items) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < items; i0 += kRelayoutItems * stride) {
         float4 v[kRelayoutItems];
@@ -610,8 +602,7 @@ __global__ void __launch_bounds__(256) space_to_depth2_vec_kernel(const float* _
 __global__ void __launch_bounds__(256) depth_to_space2_vec_kernel(const float* __restrict__ dXs, float* __restrict__ dX, const PlaneIndex ix,
                                                                   int N, int W2, long long plane2, const FastDiv group, uint32_t items,
                                                                   int accumulate) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < items; i0 += kRelayoutItems * stride) {
         float4 v[kRelayoutItems];
@@ -641,8 +632,7 @@ __global__ void __launch_bounds__(256) depth_to_space2_vec_kernel(const float* _
 // item: four pixels of an even row
 __global__ void __launch_bounds__(256) subsample2_vec_kernel(const float* __restrict__ X, float* __restrict__ Xsub, const FastDiv wq, int W,
                                                              uint32_t items) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < items; i += gridDim.x * blockDim.x) {
         uint32_t q;
         const uint32_t row = wq.split(i, q);  // plane * H/2 + output row: H is even, so input row 2 * row of the stack of planes
@@ -652,8 +642,7 @@ __global__ void __launch_bounds__(256) subsample2_vec_kernel(const float* __rest
 }
 __global__ void __launch_bounds__(256) upsample2_zero_vec_kernel(const float* __restrict__ dXsub, float* __restrict__ dX, const FastDiv wq,
                                                                  uint32_t items, int accumulate) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < items; i += gridDim.x * blockDim.x) {
         uint32_t q;
         const uint32_t row = wq.split(i, q);  // row of the stack of planes
@@ -683,8 +672,7 @@ static bool vec_ok(const void* a, const void* b, int W) {
 __device__ __forceinline__ float4 lo4(float4 v) { return make_float4(tf32_lo(v.x), tf32_lo(v.y), tf32_lo(v.z), tf32_lo(v.w)); }
 __global__ void __launch_bounds__(256) tf32_split2_kernel(const float* __restrict__ X, float* __restrict__ X2, long long per4,
                                                           const FastDiv perp4, long long x_batch, uint32_t items) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < items; i0 += kRelayoutItems * stride) {
         float4 v[kRelayoutItems];
@@ -708,8 +696,7 @@ __global__ void __launch_bounds__(256) tf32_split2_kernel(const float* __restric
 // of X and, Cp planes later, their lo parts (Cp: 4 C rounded up to a multiple of 8, the planes between zeroed).
 __global__ void __launch_bounds__(256) space_to_depth2_split_kernel(const float* __restrict__ X, float* __restrict__ X2, const PlaneIndex ix,
                                                                     int Cp, int W2, long long plane2, uint32_t items) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const uint32_t stride = gridDim.x * blockDim.x, C = ix.c.d;
     const long long half = Cp * plane2, pad = (Cp - 4LL * C) * plane2;
     for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < items; i0 += kRelayoutItems * stride) {

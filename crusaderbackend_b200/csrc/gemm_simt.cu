@@ -68,8 +68,7 @@ struct GemmSource {
 template <class T, bool P_MN, bool Q_MN>
 __global__ void __launch_bounds__(T::NT, T::kMinCtas) simt_gemm_kernel(const SimtParams p) {
     extern __shared__ __align__(16) uint8_t smem[];
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const int b = blockIdx.z / p.splits, split = blockIdx.z - b * p.splits;
     const int i0 = blockIdx.x * T::BM, j0 = blockIdx.y * T::BN;
     GemmSource<T, P_MN, Q_MN> src{p, b, i0, j0, split * p.k_per_split};
@@ -134,8 +133,7 @@ template <int IT>
 __global__ void __launch_bounds__(256) thin_gemm_k_kernel(const SimtParams p) {
     __shared__ float sP[IT][kThinK];
     constexpr int NV = 4 * IT;
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int j0 = blockIdx.x * 32 + warp * 4;
     const int k_begin = blockIdx.y * p.k_per_split, k_end = min(p.K, k_begin + p.k_per_split);
@@ -195,8 +193,7 @@ template <int IT>
 __global__ void __launch_bounds__(256) thin_gemm_mn_kernel(const SimtParams p) {
     __shared__ float sP[IT][kThinK];
     __shared__ float part[IT][8][32];
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int j = blockIdx.x * 32 + lane;
     const int k_begin = blockIdx.y * p.k_per_split, k_end = min(p.K, k_begin + p.k_per_split);
@@ -260,8 +257,7 @@ constexpr int kShortRows = 2, kShortGroups = 8;  // rows a thread, rows of threa
 template <int KT, bool V>
 __global__ void __launch_bounds__(32 * kShortGroups) short_gemm_kernel(const SimtParams p) {
     __shared__ float sQ[kShortRows * kShortGroups][KT];
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;
     const int i = (blockIdx.x * 32 + lane) * 4, j0 = blockIdx.y * kShortRows * kShortGroups, b = blockIdx.z;
     const float* P = p.P + (long long)b * p.strideP;
@@ -343,8 +339,7 @@ cudaError_t launch_tile(cb_ctx* ctx, const SimtParams& sp, dim3 grid) {
 template <bool V>
 __global__ void __launch_bounds__(256) clear_kernel(float* __restrict__ p, const FastDiv width, const FastDiv rows, long long ld,
                                                     long long stride, uint32_t items) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < items; i += gridDim.x * blockDim.x) {
         if (V) {
             reinterpret_cast<float4*>(p)[i] = make_float4(0.f, 0.f, 0.f, 0.f);

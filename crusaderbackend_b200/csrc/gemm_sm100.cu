@@ -206,8 +206,7 @@ __global__ void __launch_bounds__(96 + 32 * kEpiWarps + (X3 ? 32 * kSplitWarps :
     __syncthreads();
     tc_fence_after();
     // nothing so far touched global memory: the kernel before this one may still be running up to here
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const uint32_t tmem_base = ps.tmem_base;
     const uint32_t acc_stride = (uint32_t)p.tmem_cols >> 1;  // column offset of accumulator 1
 
@@ -529,8 +528,7 @@ __global__ void __launch_bounds__(kX3Threads, 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const uint32_t tmem_base = ps.tmem_base, p_cols = tmem_base + 256u;  // P: [raw 32 k][lo 32 k] a stage
     const int total_work = p.batch * p.tiles_i * p.tiles_j * p.kgroups;
     uint32_t fills = 0;

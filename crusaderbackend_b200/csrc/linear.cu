@@ -11,8 +11,7 @@ namespace {
 __global__ void __launch_bounds__(256) colsum_add_kernel(const float* __restrict__ dY, float* __restrict__ db,
                                                          int batch, int OUT) {
     __shared__ float part[8][32];
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int m = blockIdx.x * 32 + lane;
     // a chain of latencies in few blocks: what is added to and sixteen rows a warp are on their way at once

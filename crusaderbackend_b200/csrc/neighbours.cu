@@ -256,8 +256,7 @@ __global__ void __launch_bounds__(T) bn_fwd_par_kernel(const float* __restrict__
     constexpr int PB = T / G;
     __shared__ __align__(16) float red[R * 4 * T];
     __shared__ __align__(16) float tot[PB * 4];
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const long long p = ((long long)blockIdx.x * PB + threadIdx.x) * 4;
     const bool live = p < P;
     const int g = threadIdx.y;
@@ -337,8 +336,7 @@ __global__ void __launch_bounds__(T, SPT <= 4 ? 1024 / T : 1) bn_bwd_par_kernel(
     float4 m, sq[R], sxc[R];  // mean, and per batch group of this thread the sums of xc^2 and xc
     unsigned passes[SPT];
     if (!S) {
-        griddep_wait();
-        griddep_launch();
+        griddep_wait_then_launch();
     }
     const float4 ga = live ? ld4<V>(gamma, p, P) : f4_zero();
     if (S) {
@@ -389,8 +387,7 @@ __global__ void __launch_bounds__(T, SPT <= 4 ? 1024 / T : 1) bn_bwd_par_kernel(
 #pragma unroll
         for (int i = 0; i < SPT; ++i)
             if (g + G * i < N) centre(i, sq[i % R], sxc[i % R]);
-        griddep_wait();
-        griddep_launch();
+        griddep_wait_then_launch();
 #pragma unroll
         for (int i = 0; i < SPT; ++i) {
             const int n = g + G * i;
@@ -465,8 +462,7 @@ __global__ void __launch_bounds__(256) bn_paramgrad_par_kernel(const float* __re
                                                                float* __restrict__ dgamma, float* __restrict__ dbeta,
                                                                int N, long long P) {
     __shared__ float4 red[16][16];
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const long long p = ((long long)blockIdx.x * 16 + threadIdx.x) * 4;
     const bool live = p < P;
     float4 sg = f4_zero(), sb = f4_zero();
@@ -577,8 +573,7 @@ __device__ __forceinline__ float ew(float a, float b, float c, float s) {
 template <int OP, bool VEC>
 __global__ void __launch_bounds__(kThreads) eltwise_kernel(const float* __restrict__ a, float* __restrict__ b, float* __restrict__ out,
                                                            float s, long long n) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const long long stride = (long long)gridDim.x * blockDim.x;
     if (VEC) {
         constexpr int U = 4;
@@ -676,8 +671,7 @@ struct PoolIndex {
 };
 __global__ void __launch_bounds__(kThreads) avgpool2_kernel(const float* __restrict__ X, float* __restrict__ Y, const PoolIndex ix,
                                                             long long ys, uint32_t items) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const uint32_t stride = gridDim.x * blockDim.x, wq = ix.wq.d;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < items; i += stride) {
         uint32_t q, oh, c;
@@ -691,8 +685,7 @@ __global__ void __launch_bounds__(kThreads) avgpool2_kernel(const float* __restr
 }
 __global__ void __launch_bounds__(kThreads) avgpool2_back_kernel(float* __restrict__ dX, const float* __restrict__ dY, const PoolIndex ix,
                                                                  long long ys, uint32_t items) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const uint32_t stride = gridDim.x * blockDim.x, wq = ix.wq.d;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < items; i += stride) {
         uint32_t q, oh, c;
@@ -798,8 +791,7 @@ struct MomentumTensor {
 };
 // blockIdx.y = tensor. w *= (1 - l2) for weight tensors, m = beta m + (1 - beta) g, w -= lr m, g = 0.
 __global__ void momentum_multi_kernel(const MomentumTensor* __restrict__ ts, float lr, float beta, float l2) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const MomentumTensor t = ts[blockIdx.y];
     const float decay = t.is_weight ? (1.0f - l2) : 1.0f;
     const float omb = 1.0f - beta;
@@ -857,8 +849,7 @@ __global__ void __launch_bounds__(1024) head_fwd_kernel(const float* __restrict_
                                                        float* __restrict__ pooled, float* __restrict__ logits,
                                                        float* __restrict__ probs, float* __restrict__ dlogits,
                                                        float* __restrict__ loss_n, int C, int HW, int M) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     extern __shared__ float sh[];  // pooled[C], then logits[32]
     float* shl = sh + C;
     const int n = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -920,8 +911,7 @@ __global__ void __launch_bounds__(256) head_bwd_kernel(const float* __restrict__
                                                        float* __restrict__ dW, float* __restrict__ db,
                                                        const float* __restrict__ loss_n, float* __restrict__ loss_sum, int N,
                                                        int C, int HW, int M) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     extern __shared__ float sh[];  // dpooled[C]
     const int n = blockIdx.x;
     if (n < N) {

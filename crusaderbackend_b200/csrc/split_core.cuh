@@ -317,8 +317,7 @@ __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Bar
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const uint32_t tmem_base = b.tmem_base;
     const uint32_t slice = st_base + S::BN * 512u;  // of a second pass, behind the sums
 

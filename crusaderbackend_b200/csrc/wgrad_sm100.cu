@@ -146,8 +146,7 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
     __syncthreads();
     tc_fence_after();
     // nothing above touches global memory: the kernel before this one may still be running until here
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const uint32_t tmem_base = ws.tmem_base;
     if (threadIdx.x == 0) CB_TRACE_EVENT(p.trace, 2);
 
@@ -404,8 +403,7 @@ __global__ void __launch_bounds__(32 * kReduceGroups) wgrad_reduce_kernel(float*
     // a fixed summation order (deterministic). One shared accumulator tile (clear != 0): every thread row of the block
     // takes its own 32 rows, reads the sum and leaves zero behind for the next call.
     __shared__ float red[kReduceGroups][33];
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     const long long total = (long long)rows_tot * NQ;
     const int row_blocks = (rowsA + 31) / 32;
     const int grp = threadIdx.y;
@@ -453,8 +451,7 @@ __global__ void __launch_bounds__(32 * kReduceGroups) wgrad_reduce_kernel(float*
 // thread, lo dense with `per4` float4 per image.
 __global__ void __launch_bounds__(256) tf32_lo4_kernel(const float* __restrict__ x, float* __restrict__ lo, const FastDiv per4,
                                                        long long x_batch, uint32_t items) {
-    griddep_wait();
-    griddep_launch();
+    griddep_wait_then_launch();
     constexpr int U = 4;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < items; i0 += U * stride) {

@@ -69,3 +69,14 @@ def test_compat_shim_compiles_against_the_library():
            "-lcrusader_b200", "-Xlinker", "-rpath", "-Xlinker", "$ORIGIN/../../crusaderbackend_b200/lib"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
+
+
+def test_kernels_wait_for_their_predecessor_before_they_let_a_successor_start():
+    """That one kernel reads ahead of its wait (bn_bwd_par_kernel) rests on this order in every kernel, so there is one call for both
+    instructions, and the trigger is issued nowhere else."""
+    found = {}
+    for p in sorted((cb_build.CSRC).glob("*.cu*")):
+        text = re.sub(r"//[^\n]*", "", p.read_text())
+        found.update({(p.name, m.start()): m.group(0) for m in re.finditer(r"griddepcontrol\.\w+|cudaTriggerProgrammaticLaunchCompletion|cudaGridDependencySynchronize", text)})
+    assert [found[k] for k in sorted(found)] == ["griddepcontrol.wait", "griddepcontrol.launch_dependents"]
+    assert {name for name, _ in found} == {"cb_ptx.cuh"}
