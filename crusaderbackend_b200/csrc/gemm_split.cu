@@ -95,6 +95,7 @@ struct GemmSource {
         load_p<S, kP>(vp, p.P + pair * p.strideP, p.ldp, i0, p.I, k, p.K, tid);
         load_q<S, kQ>(vq, p.Q + pair * p.strideQ, p.ldq, j0, p.J, k, p.K, tid);
     }
+    template <bool LOW>
     __device__ __forceinline__ void store(int row, int first, int n, uint32_t mine) const {
         const int i = i0 + row;
         n = min(n, p.J - j0 - first);
@@ -109,7 +110,7 @@ struct GemmSource {
             // output is what a read, an addition and a write are, without waiting for the read.
             if (p.atomic_out || p.accumulate)
 #pragma unroll 8
-                for (int c = 0; c < n; ++c, dst += step) atomicAdd(dst, split::staged(mine, c));
+                for (int c = 0; c < n; ++c, dst += step) split::add_to<LOW>(dst, split::staged(mine, c));
             else
 #pragma unroll 8
                 for (int c = 0; c < n; ++c, dst += step) *dst = split::staged(mine, c);
@@ -121,7 +122,7 @@ struct GemmSource {
             if (biased) y += bias;
             if (bias_j) y += bias_j[c];
             if (p.atomic_out) {
-                atomicAdd(dst, y);
+                split::add_to<LOW>(dst, y);
             } else {
                 if (p.accumulate) y += *dst;
                 if (p.relu) y = fmaxf(y, 0.f);

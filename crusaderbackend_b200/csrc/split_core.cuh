@@ -211,6 +211,21 @@ __device__ __forceinline__ float staged(uint32_t mine, int c) {
     return v;
 }
 
+// *dst += y among other CTAs. The atomic add of memory takes subnormals, its own result too, for 0; LOW: an addition that keeps them, for
+// outputs of the second pass.
+template <bool LOW>
+__device__ __forceinline__ void add_to(float* dst, float y) {
+    if (!LOW) {
+        atomicAdd(dst, y);
+        return;
+    }
+    unsigned* word = reinterpret_cast<unsigned*>(dst);
+    for (unsigned old = 0u, seen;; old = seen) {
+        seen = atomicCAS(word, old, __float_as_uint(__uint_as_float(old) + y));
+        if (seen == old) return;
+    }
+}
+
 // The second pass over the contraction, by fp32 FMAs in k order, for the outputs of a tile that the pieces do not give. The loaders
 // fetch the blocks once more and leave them as they are in shared memory, kSliceK at a time behind the sums: [k][128 rows],
 // [k][BN columns]; the summing threads multiply. An infinity or a NaN in one operand makes whole rows of outputs need this, so it is a
@@ -288,7 +303,7 @@ struct Again {
 // Source: kP, kQ (Kind); prepare(t, tid), when kTable: entry tid of the table that load() of block t and the kLoaders / 32 - 1 after it
 // may read;
 // load(t, tid, p, q): this thread's values of block t, asked for in ascending order from 0 on, at most twice over;
-// store(row, first, n, mine): outputs (row, first .. first + n - 1) of the tile, to be read by staged().
+// store<LOW>(row, first, n, mine): outputs (row, first .. first + n - 1) of the tile, to be read by staged(), added by add_to<LOW>.
 // patches: ShareP::kPatches floats of shared memory.
 template <class S, class Src>
 __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Barriers& b, float* patches, int* status) {
@@ -463,11 +478,11 @@ __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Bar
         }
         const bool wanted = __any_sync(0xffffffffu, (zeros & 0x7fffffff7fffffffull) != 0 || smallest < 2u * __float_as_uint(kLow) - 1u);
         if (wanted) b.again = 1;
-        else if (ok) src.store(row, first, S::kCols, mine);
+        else if (ok) src.template store<false>(row, first, S::kCols, mine);
         all_sync<S>();
         if (b.again && !b.abort_flag) {
             Again<S>::sum(b, blocks, slice, mine, row, first, wanted);
-            if (wanted) src.store(row, first, S::kCols, mine);
+            if (wanted) src.template store<true>(row, first, S::kCols, mine);
         }
     }
 
