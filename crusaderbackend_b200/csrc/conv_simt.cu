@@ -194,7 +194,7 @@ int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, 
     const bool on_tensor_cores = (!ctx->model_pass || in_models) && split::worth_it(I, p.OUTC, most, 1, kLeastConv);
     simt::Choice c{};
     split::Choice sc{};
-    if (on_tensor_cores) sc = split::choose_shape(ctx->sm_count, I, p.OUTC, (most + split::kBK - 1) / split::kBK, 1, may_split, 1.9);
+    if (on_tensor_cores) sc = split::choose_shape(ctx->sm_count, I, p.OUTC, (most + split::kBK - 1) / split::kBK, 1, may_split, split::kGather);
     else c = simt::choose_tile(ctx->sm_count, I, p.OUTC, (most + simt::kBK - 1) / simt::kBK, 1, may_split);
     p.splits = on_tensor_cores ? sc.splits : c.splits;
     p.per_split = on_tensor_cores ? sc.per_split : c.per_split;
@@ -279,7 +279,7 @@ int fp32_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, con
     const bool on_tensor_cores = !ctx->model_pass && split::worth_it(I, g.OC, pixels, 1, kLeastConv);
     simt::Choice c{};
     split::Choice sc{};
-    if (on_tensor_cores) sc = split::choose_shape(ctx->sm_count, I, g.OC, (pixels + split::kBK - 1) / split::kBK, 1, !ctx->deterministic, 2.5);
+    if (on_tensor_cores) sc = split::choose_shape(ctx->sm_count, I, g.OC, (pixels + split::kBK - 1) / split::kBK, 1, !ctx->deterministic, split::kWgrad);
     else c = simt::choose_tile(ctx->sm_count, I, g.OC, (pixels + simt::kBK - 1) / simt::kBK, 1, !ctx->deterministic);
     p.splits = on_tensor_cores ? sc.splits : c.splits;
     p.per_split = on_tensor_cores ? sc.per_split : c.per_split;

@@ -189,7 +189,7 @@ int launch_split_gemm(cb_ctx* ctx, const GemmCall& g) {
     sp.per_fold = (g.K + kBK - 1) / kBK;
     if ((long long)sp.per_fold * fold > (1LL << 30) || g.ldp >= (1LL << 30) || g.ldq >= (1LL << 30)) return CB_EUNSUPPORTED;
     sp.blocks = sp.per_fold * fold;
-    const split::Choice c = split::choose_shape(ctx->sm_count, g.I, g.J, sp.blocks, g.batch, may_split);
+    const split::Choice c = split::choose_shape(ctx->sm_count, g.I, g.J, sp.blocks, g.batch, may_split, split::kMatrix);
     sp.splits = c.splits; sp.per_split = c.per_split;
     sp.atomic_out = c.splits > 1 ? 1 : 0;
     const long long gy = ((long long)g.J + c.bn - 1) / c.bn, gz = (long long)g.batch * c.splits;

@@ -501,34 +501,45 @@ __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Bar
 
 // Whether a product comes here rather than to the CUDA cores. Contractions of less than 16: the rounding of a few fp32 FMAs is less
 // than what the six products leave out (2-norm error at K = 2: 1.8e-8 .. 3.4e-8 against 2.1e-8 .. 5.7e-8; at K = 16 7.5e-8 against
-// 5.4e-8, at 1501 3.5e-7 against 1.1e-7). Small products: bound by their launch on either path.
+// 5.4e-8, at 1501 3.5e-7 against 1.1e-7). Small products: bound by their launch on either path. Whether the contraction may be shared
+// does not matter: with one share on each side (deterministic contexts, a ReLU, models) this kernel takes less in all of 57
+// products from 64 x 64 x 4096 (90 us against 151) to 20000 x 32 x 64 (11.1 and 12.2) and in 43 convolution passes (1.75 to 2.9 times).
 inline bool worth_it(long long I, long long J, long long K, long long copies, long long least_fmas) {
     return K >= 16 && (double)I * (double)J * (double)K * (double)copies >= (double)least_fmas;
 }
 
-// Columns of the CTA tile and how many CTAs share the contraction (their sums then meet in memory through atomic adds): the cheapest by
-// a model in SM clocks fitted to a sweep of all of them over 25 products and 48 convolution passes, where what it takes is 2 % from
-// the best on average (24 % at most, 99 x 4001 x 399). block_scale: how much longer a block takes than that of a matrix
-// (convolutions: 1.9 for the gathers, 2.5 for the weight gradient).
+// What a tile costs, in SM clocks of a model: a round of CTAs; a block of 128, 64 and 32 columns; how much longer two CTAs of 32 columns
+// on an SM take; values an SM adds into memory a clock; the launch that clears the output before. Fitted to sweeps of all tiles and shares.
+struct Costs {
+    double round, block[3], pair, flush, clear;
+};
+// 515 products (17 to 4600 rows and columns, K 64 to 5500, all forms): what it takes is 0.8 % from the best on average, 13 % at most. A fit
+// to 25 larger ones gave outputs of few columns too few shares: 6 % on average, 59 % at most, 16 products slower than on the CUDA cores,
+// where now none is. 2048 x 32 x 512: 10.9 us, 8.9 on the CUDA cores, 8.5 now; 4096 x 20 x 512 16.6, 13.3, 10.6.
+constexpr Costs kMatrix{2880.0, {710.0, 665.0, 610.0}, 1.29, 11.8, 1120.0};
+// 48 convolution passes; over 178 others the gathers are 1.6 % from the best on average, 24 % at most, the weight gradient 0.7 and 14 %.
+constexpr Costs kGather{2300.0, {690.0 * 1.9, 630.0 * 1.9, 440.0 * 1.9}, 1.77, 3.94, 1030.0}, kWgrad{2300.0, {690.0 * 2.5, 630.0 * 2.5, 440.0 * 2.5}, 1.77, 3.94, 1030.0};
+
+// Columns of the CTA tile and how many CTAs share the contraction (their sums then meet in memory through atomic adds): the cheapest.
 struct Choice {
     int bn, splits, per_split;
 };
-inline Choice choose_shape(int sm_count, long long I, long long J, long long blocks, long long copies, bool may_split, double block_scale = 1.0) {
+inline Choice choose_shape(int sm_count, long long I, long long J, long long blocks, long long copies, bool may_split, const Costs& costs) {
     static const int bns[3] = {128, 64, 32};
     static const int pieces[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128};
     Choice best{64, 1, (int)blocks};
     double best_cost = 1e300;
-    for (int bn : bns) {
+    for (int b = 0; b < 3; ++b) {
+        const int bn = bns[b];
         const long long tiles = (I + 127) / 128 * ((J + bn - 1) / bn) * copies;
         for (int want : pieces) {
             if (want > 1 && (!may_split || blocks < 2LL * want || tiles * want > 16LL * sm_count)) break;
             const long long per = (blocks + want - 1) / want, splits = (blocks + per - 1) / per, ctas = tiles * splits;
-            // two CTAs of 32 columns share an SM, a block of both takes 1.8 times one's
             const bool pairs = bn == 32 && ctas > sm_count;
             const long long slots = pairs ? 2LL * sm_count : sm_count;
-            const double load = pairs ? 1.77 : 1.0, rounds = (double)((ctas + slots - 1) / slots);
-            double cost = rounds * (2300.0 + (double)per * (bn == 128 ? 690.0 : bn == 64 ? 630.0 : 440.0) * block_scale * load);
-            if (splits > 1) cost += rounds * 128.0 * bn / 3.94 * load + 1030.0;
+            const double load = pairs ? costs.pair : 1.0, rounds = (double)((ctas + slots - 1) / slots);
+            double cost = rounds * (costs.round + (double)per * costs.block[b] * load);
+            if (splits > 1) cost += rounds * 128.0 * bn / costs.flush * load + costs.clear;
             if (cost < best_cost) {
                 best_cost = cost;
                 best = Choice{bn, (int)splits, (int)per};
