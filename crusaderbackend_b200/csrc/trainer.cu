@@ -600,7 +600,8 @@ int cbt_densenet_create(cbt_model** out, cb_ctx* ctx, int batch, int growth, int
     for (int block = 0; block < 3; ++block) {
         for (int l = 0; l < layers; ++l) {
             int y = add_conv(m, add_bn_relu(m, x), 4 * growth, 1, 1, 0);
-            add_conv(m, add_bn_relu(m, y), growth, 3, 1, 1, new_view(m, block_buf, ch, growth));
+            y = add_bn_relu(m, y);  // before the view: as arguments of one call their order, and with it the ids, would be the compiler's
+            add_conv(m, y, growth, 3, 1, 1, new_view(m, block_buf, ch, growth));
             ch += growth;
             x = new_view(m, block_buf, 0, ch);  // for the last layer: the whole buffer
         }

@@ -231,6 +231,127 @@ def test_wide_layers_take_one_route_whatever_the_streams(torch_cuda, math):
         assert orc.max_err_norm(inline, aside) <= 1e-5, (e["kind"], e["dims"])
 
 
+def _bn_calls(torch, ctx):
+    """BatchNorm + (add +) ReLU by the public calls, which keep nothing between the passes; x and dx may be prefixes of wider tensors."""
+    p = lambda t: t.data_ptr()
+
+    def forward(x, wide, gamma, beta, shortcut=None):
+        n, P = x.shape[0], gamma.numel()
+        y = torch.empty((n,) + tuple(gamma.shape), device="cuda")
+        if shortcut is None:
+            ctx._check(ctx.lib.cb_bn_fwd_relu_ex(ctx.h, p(x), p(beta), p(gamma), p(y), n, P, wide))
+        else:
+            ctx._check(ctx.lib.cb_bn_fwd_add_relu(ctx.h, p(x), p(beta), p(gamma), p(shortcut), p(y), n, P))
+        return y
+
+    def backward(dy, gamma, x, wide, y, dx, add, dshortcut=None):
+        n, P = x.shape[0], gamma.numel()
+        dg, db = torch.empty_like(gamma), torch.empty_like(gamma)
+        if dshortcut is None:
+            ctx._check(ctx.lib.cb_bn_bwd_fused_ex(ctx.h, p(dy), p(gamma), p(x), p(dx), p(dg), p(db), p(y), n, P, wide, wide, add))
+        else:
+            ctx._check(ctx.lib.cb_bn_bwd_fused_res(ctx.h, p(dy), p(gamma), p(x), p(dx), p(dg), p(db), p(y), p(dshortcut), 0, n, P))
+        return dg, db
+
+    return forward, backward
+
+
+def _model_after_one_pass(torch, cls, batch, key, **shape):
+    from crusaderbackend_b200.api import Context
+    _, _, dimg, dlab = make_batch(torch, batch, 32, 10, key)
+    ctx = Context(0, math="tf32")
+    tr = cls(ctx, batch=batch, image_hw=32, **shape)
+    host = tr.init_params(key)
+    for i, e in enumerate(tr.entries):
+        if e["kind"].startswith("bn"):
+            host[e["offset"]:e["offset"] + e["size"]] += 0.1 * orc.uniform_pm1((e["size"],), key, "bnp", i)
+    tr.set_params(host)
+    tr.forward(dimg, dlab)
+    tr.backward()
+    ctx.synchronize()
+    entry = lambda flat, i: flat[tr.entries[i]["offset"]:tr.entries[i]["offset"] + tr.entries[i]["size"]].clone()
+    return ctx, tr, lambda i: entry(tr.params, i), lambda i: entry(tr.grads, i)
+
+
+BN_BATCHES = [16, 17, 24, 32, 33, 48, 64, 65, 96, 128, 129]  # what the passes keep begins at 16 and ends at 128; 1, 2, 4 and 8 samples a thread
+
+
+@pytest.mark.parametrize("batch", BN_BATCHES)
+def test_batchnorm_of_a_residual_model_has_the_bits_of_the_calls(torch_cuda, batch):
+    """ResNet-8: every BatchNorm's output, data gradient and parameter gradients, and a projection's shortcut gradient, from the model's
+    own inputs of that layer, against cb_bn_fwd_relu / cb_bn_fwd_add_relu and cb_bn_bwd_fused / _res."""
+    torch = torch_cuda
+    from crusaderbackend_b200.train import ResNetTrainer
+    ctx, tr, param, grad = _model_after_one_pass(torch, ResNetTrainer, batch, "bnr", blocks_per_stage=1)
+    forward, backward = _bn_calls(torch, ctx)
+
+    def check(x, y, shape, entry, shortcut=None, projected=False):
+        dims = (batch,) + shape
+        X, Y, dY = tr.tensor(x, dims), tr.tensor(y, dims), tr.tensor(y, dims, grad=True)
+        gamma, beta = param(entry).view(shape), param(entry + 1).view(shape)
+        R = None if shortcut is None else tr.tensor(shortcut, dims)
+        assert torch.equal(forward(X, 0, gamma, beta, R), Y)
+        dX, dR = torch.empty_like(X), None if R is None else torch.empty_like(X)
+        dg, db = backward(dY, gamma, X, 0, Y, dX, 0, dR)
+        assert torch.equal(dX, tr.tensor(x, dims, grad=True))
+        assert torch.equal(dg.ravel(), grad(entry)) and torch.equal(db.ravel(), grad(entry + 1))
+        if projected:  # (an identity's gradient goes on to take the first convolution's)
+            assert torch.equal(dR, tr.tensor(shortcut, dims, grad=True))
+
+    check(1, 2, (16, 32, 32), 1)
+    x, entry = 2, 3
+    for c, hw in ((16, 32), (32, 16), (64, 8)):
+        projected = c > 16
+        # filter, gamma, beta, filter, gamma, beta, [filter]; convolution, BatchNorm, convolution, [projection,] BatchNorm + add
+        check(x + 1, x + 2, (c, hw, hw), entry + 1)
+        check(x + 3, x + 5 if projected else x + 4, (c, hw, hw), entry + 4, x + 4 if projected else x, projected)
+        x, entry = (x + 5, entry + 7) if projected else (x + 4, entry + 6)
+    tr.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("batch", BN_BATCHES)
+def test_batchnorm_of_a_dense_model_has_the_bits_of_the_calls(torch_cuda, batch):
+    """DenseNet, growth 16, two layers a block: inputs that are channel prefixes of a block's buffer, and gradients of that buffer summed over the
+    layers in backward order. 32 to 64 channels at 32 x 32, 16 x 16 and 8 x 8: both forms of two batch groups and the narrow one."""
+    torch = torch_cuda
+    from crusaderbackend_b200.train import DenseNetTrainer
+    growth, layers = 16, 2
+    ctx, tr, param, grad = _model_after_one_pass(torch, DenseNetTrainer, batch, "bnd", growth=growth, layers=layers)
+    forward, backward = _bn_calls(torch, ctx)
+    ch, hw, buf, entry = 2 * growth, 32, 1, 1
+    nxt = 3  # image 0, buffer 1, its first channels 2
+    for block in range(3):
+        wide = (batch, ch + layers * growth, hw, hw)
+        X, dX, want = tr.tensor(buf, wide), tr.tensor(buf, wide, grad=True), torch.empty(wide, device="cuda")
+        stride = wide[1] * hw * hw
+        layer_bns = []
+        for _ in range(layers):
+            layer_bns.append((nxt, ch, entry))                 # on the prefix
+            c = 4 * growth                                     # on the 1x1 convolution's output
+            dims, shape = (batch, c, hw, hw), (c, hw, hw)
+            x, y, dy = tr.tensor(nxt + 1, dims), tr.tensor(nxt + 2, dims), tr.tensor(nxt + 2, dims, grad=True)
+            gamma, beta = param(entry + 3).view(shape), param(entry + 4).view(shape)
+            assert torch.equal(forward(x, 0, gamma, beta), y)
+            dx = torch.empty_like(x)
+            dg, db = backward(dy, gamma, x, 0, y, dx, 0)
+            assert torch.equal(dx, tr.tensor(nxt + 1, dims, grad=True))
+            assert torch.equal(dg.ravel(), grad(entry + 3)) and torch.equal(db.ravel(), grad(entry + 4))
+            ch, nxt, entry = ch + growth, nxt + 5, entry + 6   # BN, conv, BN, conv's view, the next prefix
+        layer_bns.append((nxt, ch, entry))                     # transition or head, on the whole buffer
+        for add, (y_id, c, e) in enumerate(reversed(layer_bns)):
+            dims, shape = (batch, c, hw, hw), (c, hw, hw)
+            y, dy, gamma, beta = tr.tensor(y_id, dims), tr.tensor(y_id, dims, grad=True), param(e).view(shape), param(e + 1).view(shape)
+            assert torch.equal(forward(X, stride, gamma, beta), y)
+            dg, db = backward(dy, gamma, X, stride, y, want, 1 if add else 0)
+            assert torch.equal(dg.ravel(), grad(e)) and torch.equal(db.ravel(), grad(e + 1))
+        assert torch.equal(want, dX)
+        if block < 2:  # BN, conv; the next buffer and its first channels
+            ch, hw, buf, entry, nxt = ch // 2, hw // 2, nxt + 2, entry + 3, nxt + 4
+    tr.close()
+    ctx.close()
+
+
 def test_resnet56_loss_tracks_fp32_run(torch_cuda):
     """ResNet-56, batch 128 of N(0,1) CIFAR-shaped images, uniform labels, He init, momentum 0.9, lr 0.01/128, 200 steps
     on a repeated batch: the loss of the TF32 and of the 3xTF32 tensor-core run stays within 1 % (of the curve's largest
