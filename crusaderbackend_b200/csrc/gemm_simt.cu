@@ -252,8 +252,21 @@ __global__ void __launch_bounds__(256) thin_gemm_mn_kernel(const SimtParams p) {
 
 // Short contractions (K <= KT, the input gradient of a classifier layer): bound by writing the output. A thread keeps the K values of
 // four columns of P in registers and forms kShortRows rows of the output, whose Q values are shared-memory broadcasts; products are
-// added in k order by FMAs, as everywhere here. 4096 x 128 x 10: 5.5 us on the 64 x 64 tiles, one slice of 16 k each, 2.9 here.
+// added in k order by FMAs, as everywhere here. us, 64 x 64 tiles (one slice of 16 k) / here: 128 x 4096 x 10 6.8 / 2.9, x 15 6.8 / 3.9.
 constexpr int kShortRows = 2, kShortGroups = 8;  // rows a thread, rows of threads
+// Whether it reads and writes 16 bytes at a time.
+template <class T>
+bool short_vec(const T& p) {
+    return ((p.I | p.ldp | p.strideP | p.ldc | p.strideC) & 3) == 0 && ((reinterpret_cast<uintptr_t>(p.P) | reinterpret_cast<uintptr_t>(p.C)) & 15u) == 0;
+}
+// Which products it takes: every sixteen rows read P's columns again, so where there are many the tiles are faster. us, tiles / here: K = 10 on
+// 16 bytes 2000 x 4096 28.1 / 14.8, off them 1000 x 4095 16.9 / 16.9, 8000 x 4095 97 / 114 (K = 3 97 / 57, 7 97 / 98); K = 11 to 15
+// 256 x 4095 7.4 / 8.0 to 9.0, 8000 x 4095 97 / 173 to 190, 2000 x 4096 28.2 / 32.4 to 34.7 (60 x 40000 13.9 / 11.8 to 12.5).
+bool short_pays(const GemmCall& g) {
+    const double outputs = (double)g.I * g.J * g.batch;
+    if (g.K > 10) return outputs <= (double)(1 << 19) || (g.J <= 64 && short_vec(g));
+    return g.K <= 4 || short_vec(g) || outputs <= (double)(1 << 22);
+}
 template <int KT, bool V>
 __global__ void __launch_bounds__(32 * kShortGroups) short_gemm_kernel(const SimtParams p) {
     __shared__ float sQ[kShortRows * kShortGroups][KT];
@@ -305,8 +318,7 @@ __global__ void __launch_bounds__(32 * kShortGroups) short_gemm_kernel(const Sim
     }
 }
 cudaError_t launch_short(cb_ctx* ctx, const SimtParams& p) {
-    const bool vec = ((p.I | p.ldp | p.strideP | p.ldc | p.strideC) & 3) == 0 &&
-                     ((reinterpret_cast<uintptr_t>(p.P) | reinterpret_cast<uintptr_t>(p.C)) & 15u) == 0;
+    const bool vec = short_vec(p);
     typedef void (*Kernel)(const SimtParams);
     static const Kernel kernels[2][3] = {{short_gemm_kernel<4, false>, short_gemm_kernel<10, false>, short_gemm_kernel<16, false>},
                                          {short_gemm_kernel<4, true>, short_gemm_kernel<10, true>, short_gemm_kernel<16, true>}};
@@ -387,7 +399,8 @@ static int gemm_zero_output(cb_ctx* ctx, const GemmCall& g) {
 static int launch_simt_gemm(cb_ctx* ctx, const GemmCall& g_in, bool* summed) {
     GemmCall g = g_in;
     const int fold = g.kfold > 1 ? g.kfold : 1;
-    const bool short_k = g.K <= 16 && g.p_mn && g.out_mode == 0 && fold == 1 && g.I >= 128 && g.J <= 65535 * kShortRows * kShortGroups && g.batch <= 65535;
+    const bool short_k = g.K <= 16 && g.p_mn && g.out_mode == 0 && fold == 1 && g.I >= 128 && g.J <= 65535 * kShortRows * kShortGroups && g.batch <= 65535 &&
+                         short_pays(g);
     const bool swapped = !short_k && g.J <= 16 && g.I > 16;
     if (swapped) {  // put the thin extent on the I side: D'[j][i] with the operands' roles swapped
         std::swap(g.I, g.J);

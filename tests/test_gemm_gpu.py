@@ -347,3 +347,27 @@ def test_split_products_clear_their_output(torch_cuda, ctxs, batch, M, N, K, pad
     want = np.stack([orc.gemm_f64(A.cpu().numpy(), b) for b in B.cpu().numpy()])
     assert orc.max_err_norm(whole[:, :M, :N].cpu().numpy(), want) <= TOL["fp32"]
     assert bool((whole[:, M:, :] == 7).all()) and bool((whole[:, :, N:] == 7).all())
+
+
+@pytest.mark.parametrize("M,N", [(1, 128), (15, 132), (16, 128), (17, 131), (33, 516), (130, 257), (512, 1025), (1025, 513), (2050, 2047)])
+@pytest.mark.parametrize("K", [1, 4, 5, 10, 11, 15, 16])
+@pytest.mark.parametrize("pad", [0, 1, 4])
+def test_short_contractions(torch_cuda, ctxs, M, N, K, pad):
+    """Contractions of up to 16 at the edges of their kernel: rows of sixteen, columns of 128 and of four, its three lengths of K in 16-byte
+    and in 4-byte form, outputs on both sides of where the tiles take them; overwrite, accumulate and batches. K + 1 roundings, each by
+    2^-24 of a sum that is at most K (2 K)."""
+    torch, ctx = torch_cuda, ctxs["fp32"]
+    A, B = orc.uniform_pm1((M, K + pad), "short", M, N, K, "A"), orc.uniform_pm1((K, N + pad), "short", M, N, K, "B")
+    a, b = torch.from_numpy(A).cuda()[:, :K], torch.from_numpy(B).cuda()[:, :N]
+    ref = A[:, :K].astype(np.float64) @ B[:, :N]
+    C = torch.full((M, N + pad), 7.0, device="cuda")
+    for again in (1, 2):
+        ctx.gemm(a, b, C[:, :N], accumulate=again == 2)
+        assert ctx.last_kernel == "simt_fp32"
+        assert np.abs(C[:, :N].cpu().numpy() - again * ref).max() <= again * (K + 1) * 2.0 ** -24 * K
+    assert bool((C[:, N:] == 7).all())
+    if pad == 0 and M * N < 100000:
+        B3 = orc.uniform_pm1((3, K, N), "short", M, N, K, "B3")
+        C3 = torch.empty(3, M, N, device="cuda")
+        ctx.sgemm(a, torch.from_numpy(B3).cuda(), C3)
+        assert np.abs(C3.cpu().numpy() - A.astype(np.float64) @ B3).max() <= (K + 1) * 2.0 ** -24 * K
