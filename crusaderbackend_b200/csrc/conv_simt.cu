@@ -333,11 +333,15 @@ static bool tf32_width(const ConvGeo& g) {
     return g.FH <= 3 && g.FW <= 3 && (w == 8 || w == 16 || w == 32);
 }
 // Stride-2 3x3 layers of 3xTF32 whose forward pass and weight gradient run at fp32 accuracy: the one-pass form pays for a phase split and
-// lo parts through memory. Forward, then weight gradient, us, one pass / fp32: 32 -> 64 at 32 x 32, batch 128: 38 / 23, 34 / 30; 64 -> 32, batch 118:
-// 72 / 27, 44 / 34 (data gradient 31 / 38 and 38 / 52: stays). Below 2^27 multiplications both are a few launches, 10 to 14 us against 6 to 10.
-static bool x3_at_fp32(const ConvGeo& g) {
+// lo parts through memory. Forward, then weight gradient, us, one pass / fp32: 32 -> 64 at 32 x 32, batch 128: 37 / 21, 34 / 24; 64 -> 32, batch 118:
+// 71 / 25, 44 / 29 (data gradient 31 / 38 and 38 / 52: stays). Below 2^27 multiplications both are a few launches, 10 to 14 us against 6 to 10.
+// 145 layers of 4 to 147 channels, 16 x 16 to 64 x 64: forward 1.0 to 3.6 times as fast, except for few input channels on many pixels, where
+// each of the gather's outputs has little to sum: 16 channels, more than 2^15 pixels, 0.70 to 1.06 (to 48, 191 of 64 x 64: 61 / 86), or
+// 1.1 to 1.6 for the 17 to 32 outputs that fill its narrowest tile; weight gradient 1.0 to 3.1, two 16 -> 48 layers 0.8 and 0.9.
+static bool x3_at_fp32(const ConvGeo& g, bool forward) {
     if ((double)g.N * g.OH * g.OW >= (double)(1LL << 30) || (double)g.IC * g.IH * g.IW >= (double)(1LL << 28) || (double)g.OC * g.OH * g.OW >= (double)(1LL << 28))
         return false;  // 32-bit indexes
+    if (forward && g.IC <= 16 && (long long)g.N * g.OH * g.OW > (1 << 15) && (g.OC <= 16 || g.OC > 32)) return false;
     return g.sH == 2 && g.sW == 2 && g.FH == 3 && g.FW == 3 && (double)g.N * g.OH * g.OW * g.OC * g.IC * 9.0 >= (double)(1LL << 27);
 }
 
@@ -359,7 +363,7 @@ static int conv_fwd_impl(cb_ctx* ctx, const float* W, const float* X, float* Y, 
     if (npix == 0 || OC == 0) return CB_OK;
     if (!W || !X || !Y) return fail(ctx, CB_EINVAL, std::string(who) + ": null operand");
     const bool x3 = ctx->math == CB_MATH_3XTF32;
-    if (ctx->math != CB_MATH_FP32 && !(x3 && !ctx->model_pass && x3_at_fp32(g))) {
+    if (ctx->math != CB_MATH_FP32 && !(x3 && !ctx->model_pass && x3_at_fp32(g, true))) {
         rc = umma_conv_fwd(ctx, W, X, Y, ep, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, false, xb, yb, x3);
         if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;
     }
@@ -433,7 +437,8 @@ int cb_filters_changed(cb_ctx* ctx) {
 // Weight gradients that the TF32 kernel would cut into several launches (filters beyond its accumulator) run in one at fp32 accuracy
 // where that takes less: 6 us + 45 us for 10^9 multiplications against 6.5 us a launch (TF32) or 8 us and 9 for the lo parts (3xTF32).
 // 128 -> 128 3x3, 4 maps of 16 x 16: 25.9 us TF32, 32.5 3xTF32, 7.9 here; 330 -> 48 1x1, 64 of 8 x 8: 14.6 TF32, 7.9 here;
-// 288 -> 48 1x1, 64 of 16 x 16: 14.1 TF32, 18.0 here.
+// 288 -> 48 1x1, 64 of 16 x 16: 14.1 TF32, 18.0 here. Of 140 other layers of either mode one is slower for it (16 -> 176 1x1, 15 of 32 x 32:
+// 11.3 TF32, 12.9 here).
 static bool wgrad_at_fp32(const ConvGeo& g, bool x3) {
     const int launches = umma_wgrad_launches(g.IC, g.OC, g.FH, g.FW);
     const double fmas = (double)g.N * g.OH * g.OW * g.OC * g.IC * g.FH * g.FW;
@@ -462,7 +467,7 @@ static int conv_wgrad_impl(cb_ctx* ctx, const float* dY, const float* X, float* 
     const bool x3 = ctx->math == CB_MATH_3XTF32;
     // (models keep the kernel that leaves half the SMs to the stream beside it: a DenseNet-100 step took 3571 us with its widest layers
     // here, 3561 without; without such streams too, or a gradient's accuracy would depend on their number)
-    if (ctx->math != CB_MATH_FP32 && (ctx->deterministic || ctx->model_pass || !((x3 && x3_at_fp32(g)) || wgrad_at_fp32(g, x3)))) {
+    if (ctx->math != CB_MATH_FP32 && (ctx->deterministic || ctx->model_pass || !((x3 && x3_at_fp32(g, false)) || wgrad_at_fp32(g, x3)))) {
         rc = umma_conv_wgrad(ctx, dY, X, dW, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, accumulate, dy_batch, x_batch, x3);
         if (rc == CB_OK && x3) ctx->last_kernel = "umma_3xtf32";
         if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;

@@ -123,7 +123,8 @@ def test_convolution(ctx, geo, det):
 
 
 @pytest.mark.parametrize("math,geo,kern", [("3xtf32", (9, 96, 16, 96, 3, 1), ["umma_fp32"] * 3), ("3xtf32", (64, 64, 16, 128, 3, 2), ["umma_fp32", "umma_3xtf32", "umma_fp32"]),
-                                           ("3xtf32", (128, 16, 32, 32, 3, 2), ["umma_fp32", "umma_3xtf32", "umma_fp32"]), ("tf32", (64, 330, 8, 48, 1, 1), [None, None, "umma_fp32"]),
+                                           ("3xtf32", (128, 16, 32, 32, 3, 2), ["umma_fp32", "umma_3xtf32", "umma_fp32"]), ("3xtf32", (34, 16, 64, 64, 3, 2), ["umma_3xtf32", "umma_3xtf32", "umma_fp32"]),
+                                           ("3xtf32", (34, 16, 64, 32, 3, 2), ["umma_fp32", "umma_3xtf32", "umma_fp32"]), ("tf32", (64, 330, 8, 48, 1, 1), [None, None, "umma_fp32"]),
                                            ("tf32", (4, 128, 16, 128, 3, 1), [None, None, "umma_fp32"])])
 def test_passes_of_the_other_modes_that_run_at_fp32_accuracy(math, geo, kern):
     """Wide filters and large stride-2 layers of 3xTF32, weight gradients the TF32 kernel would cut into several launches."""
