@@ -529,11 +529,11 @@ def bench_reference(args):
 def run_case(args):
     """`--case NAME`: a few launches of ONE kernel on a small, larger-than-L2-irrelevant case, for profiler captures of
     that kernel (prints a one-line summary, not the benchmark line). NAME is conv_fwd | conv_dgrad | conv_wgrad
-    (with --shape N,IC,H,OC,F,stride), bn_fwd | bn_bwd (--shape N,C,H), momentum, head, gemm (--shape M,N,K,form)."""
+    (with --shape N,IC,H,OC,F,stride), bn_fwd | bn_bwd (--shape N,C,H), momentum, head, gemm (--shape M,N,K,form); --math sets the mode."""
     import torch
     from crusaderbackend_b200.api import Context
     torch.cuda.set_device(0)
-    ctx = Context(0, math="tf32", sync=False)
+    ctx = Context(0, math=args.math, sync=False)
     name = args.case
     shp = args.shape.split(",") if args.shape else []
     reps = max(1, args.steps)
@@ -706,6 +706,7 @@ def main():
     ap.add_argument("--quick", action="store_true", help="headline and convolution table only (profiling runs)")
     ap.add_argument("--case", default=None, help="run a few launches of one kernel instead of the benchmark (profiler captures)")
     ap.add_argument("--shape", default=None, help="comma-separated extents of --case")
+    ap.add_argument("--math", default="tf32", choices=["tf32", "3xtf32", "fp32"], help="math mode of --case")
     args = ap.parse_args()
     if args.case:
         run_case(args)

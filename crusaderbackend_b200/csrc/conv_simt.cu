@@ -180,9 +180,10 @@ __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_wgrad_simt(const Wgra
 constexpr long long kLeastConv = 1LL << 22;
 
 // One launch for up to four pixel sets. In the passes of a model the two that later layers read stay on the CUDA cores (see
-// launch_fp32_gemm), except the 3xTF32 ones that never ran there (in_models). The contraction is split over CTAs where the output alone does not fill the GPU and the
-// epilogue is a plain sum (the output is then cleared first), except in the passes of a model: atomic sums come in any order, and
-// one rounding more or less in an activation moves the gradients of a deep model by percents from one run to the next.
+// launch_fp32_gemm), except the 3xTF32 ones that never ran there (in_models). The contraction is split over CTAs where the output alone
+// does not fill the GPU and the epilogue is a plain sum (the output is then cleared first), except in the passes of a model: atomic
+// sums come in any order, and one rounding more or less in an activation moves the gradients of a deep model by percents from one run
+// to the next.
 int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, bool in_models, const char* who) {
     const long long out_elems = (long long)p.OUTC * p.OHH * p.OWW;
     if ((long long)p.C * p.H * p.W >= (1LL << 29) || out_elems >= (1LL << 31) || (long long)p.C * p.w_ch >= (1LL << 31))
@@ -275,7 +276,8 @@ int fp32_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, con
     const bool mask = g.FH <= kMaskTaps && g.FW <= kMaskTaps;
     p.I = (int)I; p.pixels = (int)pixels;
     // Not in a model's backward pass, on whichever stream (cbt_set_wgrad_streams moves launches, it does not choose kernels): a CTA of
-    // conv_wgrad_split holds an SM, which the stream beside it would miss (ResNet-50 on 16 x 16 images, batch 78: 2300 us a step against 2263)
+    // conv_wgrad_split holds an SM, which the stream beside it would miss (ResNet-50 on 16 x 16 images, batch 78: 2300 us a step
+    // against 2263)
     const bool on_tensor_cores = !ctx->model_pass && split::worth_it(I, g.OC, pixels, 1, kLeastConv);
     simt::Choice c{};
     split::Choice sc{};
@@ -333,11 +335,12 @@ static bool tf32_width(const ConvGeo& g) {
     return g.FH <= 3 && g.FW <= 3 && (w == 8 || w == 16 || w == 32);
 }
 // Stride-2 3x3 layers of 3xTF32 whose forward pass and weight gradient run at fp32 accuracy: the one-pass form pays for a phase split and
-// lo parts through memory. Forward, then weight gradient, us, one pass / fp32: 32 -> 64 at 32 x 32, batch 128: 37 / 21, 34 / 24; 64 -> 32, batch 118:
-// 71 / 25, 44 / 29 (data gradient 31 / 38 and 38 / 52: stays). Below 2^27 multiplications both are a few launches, 10 to 14 us against 6 to 10.
-// 145 layers of 4 to 147 channels, 16 x 16 to 64 x 64: forward 1.0 to 3.6 times as fast, except for few input channels on many pixels, where
-// each of the gather's outputs has little to sum: 16 channels, more than 2^15 pixels, 0.70 to 1.06 (to 48, 191 of 64 x 64: 61 / 86), or
-// 1.1 to 1.6 for the 17 to 32 outputs that fill its narrowest tile; weight gradient 1.0 to 3.1, two 16 -> 48 layers 0.8 and 0.9.
+// lo parts through memory. Forward, then weight gradient, us, one pass / fp32: 32 -> 64 at 32 x 32, batch 128: 37 / 21, 34 / 24; 64 ->
+// 32, batch 118: 71 / 25, 44 / 29 (data gradient 31 / 38 and 38 / 52: stays). Below 2^27 multiplications both are a few launches, 10 to
+// 14 us against 6 to 10. 145 layers of 4 to 147 channels, 16 x 16 to 64 x 64: forward 1.0 to 3.6 times as fast, except for few input
+// channels on many pixels, where each of the gather's outputs has little to sum: 16 channels, more than 2^15 pixels, 0.70 to 1.06 (to
+// 48, 191 of 64 x 64: 61 / 86), or 1.1 to 1.6 for the 17 to 32 outputs that fill its narrowest tile; weight gradient 1.0 to 3.1, two 16
+// -> 48 layers 0.8 and 0.9.
 static bool x3_at_fp32(const ConvGeo& g, bool forward) {
     if ((double)g.N * g.OH * g.OW >= (double)(1LL << 30) || (double)g.IC * g.IH * g.IW >= (double)(1LL << 28) || (double)g.OC * g.OH * g.OW >= (double)(1LL << 28))
         return false;  // 32-bit indexes

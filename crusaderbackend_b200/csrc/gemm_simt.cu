@@ -259,9 +259,9 @@ template <class T>
 bool short_vec(const T& p) {
     return ((p.I | p.ldp | p.strideP | p.ldc | p.strideC) & 3) == 0 && ((reinterpret_cast<uintptr_t>(p.P) | reinterpret_cast<uintptr_t>(p.C)) & 15u) == 0;
 }
-// Which products it takes: every sixteen rows read P's columns again, so where there are many the tiles are faster. us, tiles / here: K = 10 on
-// 16 bytes 2000 x 4096 28.1 / 14.8, off them 1000 x 4095 16.9 / 16.9, 8000 x 4095 97 / 114 (K = 3 97 / 57, 7 97 / 98); K = 11 to 15
-// 256 x 4095 7.4 / 8.0 to 9.0, 8000 x 4095 97 / 173 to 190, 2000 x 4096 28.2 / 32.4 to 34.7 (60 x 40000 13.9 / 11.8 to 12.5).
+// Which products it takes: every sixteen rows read P's columns again, so where there are many the tiles are faster. us, tiles / here: K
+// = 10 on 16 bytes 2000 x 4096 28.1 / 14.8, off them 1000 x 4095 16.9 / 16.9, 8000 x 4095 97 / 114 (K = 3 97 / 57, 7 97 / 98); K = 11
+// to 15 256 x 4095 7.4 / 8.0 to 9.0, 8000 x 4095 97 / 173 to 190, 2000 x 4096 28.2 / 32.4 to 34.7 (60 x 40000 13.9 / 11.8 to 12.5).
 bool short_pays(const GemmCall& g) {
     const double outputs = (double)g.I * g.J * g.batch;
     if (g.K > 10) return outputs <= (double)(1 << 19) || (g.J <= 64 && short_vec(g));
@@ -478,8 +478,9 @@ static int launch_simt_gemm(cb_ctx* ctx, const GemmCall& g_in, bool* summed) {
     return CB_OK;
 }
 
-// Products of CB_MATH_FP32 and those TMA cannot address. In the passes of a model they stay on the CUDA cores: one rounding in an
-// activation moves the gradients of a deep model by percents, and a run could not be compared with one of an earlier version.
+// Products of CB_MATH_FP32 and those TMA cannot address. In the passes of a model they stay on the CUDA cores, where they take two to three
+// times as long: their sums are then those that models have always had. (One rounding in an activation moves the gradients of a deep
+// model by percents, whatever code computed it; neither path is the better one in that.)
 int launch_fp32_gemm(cb_ctx* ctx, const GemmCall& g, bool* summed) {
     if (!ctx->model_pass) {
         const int rc = launch_split_gemm(ctx, g);

@@ -171,8 +171,8 @@ Kind kind_of(const float* base, long long ld, long long stride, int mn) {
 }  // namespace
 
 // Thin products stay on the kernels that stream the long operand once, contractions of one or two blocks on the CUDA cores. The least
-// multiplications: where a launch of gemm_simt.cu and one of these take the same time (257^3: 9.4 us against 8.6 to 10.2, 513 x 65 x 257: 10.2
-// against 9.7; 515^3 17.8 against 10.6, 2047^3 421 against 123).
+// multiplications: where a launch of gemm_simt.cu and one of these take the same time (257^3: 9.4 us against 8.6 to 10.2, 513 x 65 x
+// 257: 10.2 against 9.7; 515^3 17.8 against 10.6, 2047^3 421 against 123).
 constexpr long long kLeastGemm = 1LL << 24;
 
 int launch_split_gemm(cb_ctx* ctx, const GemmCall& g) {

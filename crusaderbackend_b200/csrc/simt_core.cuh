@@ -1,7 +1,7 @@
 // fp32 products on the CUDA cores: D[i][j] = sum_k P(i, k) * Q(j, k) with exact fp32 FMAs in k order, for CB_MATH_FP32
 // and for operands the TMA-fed kernels cannot address (rows TMA cannot start at, convolution geometries outside conv_sm100.cu),
-// where a product is too small for split_core.cuh or belongs to a model's pass. One kernel body serves the GEMM forms and the three convolution passes; an operand source (below) says
-// where element (i, k) lies.
+// where a product is too small for split_core.cuh or belongs to a model's pass. One kernel body serves the GEMM forms and the three
+// convolution passes; an operand source (below) says where element (i, k) lies.
 //
 // What bounds it: the fp32 pipe (128 FMA per SM and clock) as long as the extents are large, so everything is laid out to
 // leave the issue slots to FMAs: 8 x 8 (or 8 x 4) outputs per thread, packed two-wide FMAs (fma.rn.f32x2, each half an

@@ -914,7 +914,8 @@ struct StageInputs {
 // model's own (its node is given the new addresses before a launch), and the passes read those. Eager, and reading the caller's
 // buffers: the first calls, streams that are being captured, sync mode, data-parallel models (their collectives are ordered call
 // by call), calls that find a filter's packed copy stale or the filter cache switched off, passes whose recording fails, and a
-// backward pass whose forward pass was eager. A recording is keyed by everything it has baked in, scratch blocks included; at most kMostRecorded are kept.
+// backward pass whose forward pass was eager. A recording is keyed by everything it has baked in, scratch blocks included; at most
+// kMostRecorded are kept.
 template <class F>
 int run_recorded(cbt_model* m, bool backward, F ops) {
     constexpr size_t kMostRecorded = 8;
@@ -1023,8 +1024,8 @@ int run_recorded(cbt_model* m, bool backward, F ops) {
 extern "C" {
 
 // Forward pass on `images` (batch x 3 x H x W, device) with one-hot `labels` (batch x classes, device). The images are
-// read in place unless the pass runs as a recording: they must stay unchanged until cbt_backward has run. Leaves the softmax in the last tensor
-// and the summed loss in the model's device loss word (after cbt_backward for models with the fused head).
+// read in place unless the pass runs as a recording: they must stay unchanged until cbt_backward has run. Leaves the softmax in the
+// last tensor and the summed loss in the model's device loss word (after cbt_backward for models with the fused head).
 static int forward_ops(cbt_model* m);
 int cbt_forward(cbt_model* m, const float* images, const float* labels) {
     if (!m || !m->P || !images || !labels) return CB_EINVAL;
@@ -1345,8 +1346,8 @@ int cbt_dp_unique_id(char* id128) {
 }
 
 // Joins the communicator (collective over all ranks) and splits the flat gradient buffer into `buckets` ranges (1..8)
-// that double in size from the first layers' end (1 : 2 : 4 ...). From then on cbt_backward sum-allreduces each range over the ranks on a communication
-// stream as soon as its last gradient has been produced, and the gradients are the sums over all ranks when
+// that double in size from the first layers' end (1 : 2 : 4 ...). From then on cbt_backward sum-allreduces each range over the ranks on
+// a communication stream as soon as its last gradient has been produced, and the gradients are the sums over all ranks when
 // cbt_backward's work is done. Call before capturing the step in a CUDA graph.
 int cbt_dp_init(cbt_model* m, const char* id128, int world, int rank, int buckets) {
     if (const char* e = std::getenv("CBT_DP_BUCKETS")) buckets = std::atoi(e);  // development override
