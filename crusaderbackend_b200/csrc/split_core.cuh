@@ -2,13 +2,13 @@
 // operands the TMA-fed kernels cannot address, where the product is large enough to pay for it. One kernel body serves the GEMM
 // forms and the three convolution passes; an operand source (below) says where element (i, k) lies.
 //
-// Every fp32 value from 2^-110 on is the sum of three bf16 values: x = x1 + x2 + x3 with x1 = x cut off, x2 = x - x1 rounded, x3 the rest,
-// all of it exact (8 + 8 + 8 significant bits; below, the third runs into bf16's least subnormal, 2^-133: see kLow). Six of the nine
-// products of two such sums leave out up to 2^-22 of the product (x2 y3 + x3 y2, of either sign: x2 is rounded for that; 2^-26 on
-// average): x2 y2, x1 y3, x3 y1, x1 y2, x2 y1, x1 y1, issued smallest first. (The splitting is that of G. Henry, P. T. P. Tang and
-// A. Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations", 2019.) What the tensor core does not give is fp32's rounding of
-// sums (TMEM truncates every addition), so no chain of additions there is longer than two k-blocks of 32: their sum is read back and
-// added to the running total in a register, by ordinary fp32 additions.
+// Every fp32 value from 2^-110 on is the sum of three bf16 values: x = x1 + x2 + x3 with x1 = x cut off, x2 = x - x1 rounded, x3 the
+// rest, all of it exact (8 + 8 + 8 significant bits; below, the third runs into bf16's least subnormal, 2^-133: see kLow). Six of the
+// nine products of two such sums leave out up to 2^-22 of the product (x2 y3 + x3 y2, of either sign: x2 is rounded for that; 2^-26 on
+// average): x2 y2, x1 y3, x3 y1, x1 y2, x2 y1, x1 y1, issued smallest first. (The splitting is that of G. Henry, P. T. P. Tang and A.
+// Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations", 2019.) What the tensor core
+// does not give is fp32's rounding of sums (TMEM truncates every addition), so no chain of additions there is longer than two k-blocks
+// of 32: their sum is read back and added to the running total in a register, by ordinary fp32 additions.
 //
 // What bounds it: shared-memory bandwidth, were both operands read from there (a 128 x 128 x 16 UMMA reads 8 KB in its 64 clocks;
 // with the loaders' own accesses a k-block of 32 took 1800 clocks, 12 UMMAs 768). So the pieces of P go to TMEM, straight from the
