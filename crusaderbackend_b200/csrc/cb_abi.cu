@@ -58,6 +58,19 @@ int finish(cb_ctx* ctx, const char* what) {
 // on a stream the context used earlier may still read it), and never while the workspace is frozen or the stream is
 // being captured: a captured graph keeps the addresses of the blocks it was recorded with, so a later free would leave
 // it reading released memory.
+// Scratch for the pieces of a convolution's filter (conv_patch.cu), or null: where it is too small, and where work that the context cannot
+// order against its own may use it too: on another stream than the one the context was created with (cb_set_stream does not wait for the old one),
+// and in a graph that is being captured (it may be replayed beside later calls).
+void* filter_pieces(const cb_ctx* ctx, size_t bytes) {
+    if (bytes > kFilterPieces || ctx->stream != ctx->home_stream) return nullptr;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return ctx->d_status + 64;
+}
+
 static int grow_block(cb_ctx* ctx, void** block, size_t* have, size_t bytes, size_t ahead) {
     if (bytes <= *have) return CB_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -246,7 +259,8 @@ int cb_create(cb_ctx** out, int device, void* cuda_stream) {
     ctx->sm_count = prop.multiProcessorCount;
     ctx->max_smem_optin = (int)prop.sharedMemPerBlockOptin;
     if (const char* e = std::getenv("CB_PDL")) ctx->pdl = std::atoi(e) != 0;  // development switch, default on
-    if (cudaMalloc(&ctx->d_status, sizeof(int)) != cudaSuccess || cudaMemset(ctx->d_status, 0, sizeof(int)) != cudaSuccess) {
+    ctx->home_stream = ctx->stream;
+    if (cudaMalloc(&ctx->d_status, 256 + kFilterPieces) != cudaSuccess || cudaMemset(ctx->d_status, 0, sizeof(int)) != cudaSuccess) {
         delete ctx;
         return CB_ENOMEM;
     }

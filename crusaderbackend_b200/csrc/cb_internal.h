@@ -29,6 +29,7 @@ struct cb_ctx {
     int deterministic = 0;
     bool model_pass = false;  // set while a model's forward or backward pass is queued; always on the contexts of its weight-gradient streams
     int* d_status = nullptr;       // device status word (0 = ok, CBK_* otherwise)
+    cudaStream_t home_stream = nullptr;  // the one the context was created with
     void* workspace = nullptr;     // scratch: split-K partials, packed filters
     size_t workspace_bytes = 0;
     void* workspace2 = nullptr;    // scratch: re-laid-out activations / gradients of the stride-2 convolutions
@@ -129,6 +130,8 @@ int enter(cb_ctx* ctx);
 // block is freed, and is refused (CB_ENOMEM) while the workspace is frozen or the stream is being captured. A block that has to
 // grow gets `ahead` bytes if it can: what the caller knows will be asked for next. A growth takes 0.3 ms whatever its size.
 int ensure_workspace(cb_ctx* ctx, size_t bytes);
+constexpr size_t kFilterPieces = (size_t(1) << 20) - 256;  // of 128 -> 128 channels, 3x3: 0.9 MB
+void* filter_pieces(const cb_ctx* ctx, size_t bytes);
 int ensure_workspace2(cb_ctx* ctx, size_t bytes, size_t ahead = 0);
 int ensure_workspace3(cb_ctx* ctx, size_t bytes, size_t ahead = 0);
 // The zero-filled accumulator of the weight-gradient kernels, at least `bytes` large (same growth rules).

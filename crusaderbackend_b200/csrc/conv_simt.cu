@@ -3,9 +3,11 @@
 // exact fp32 FMAs. Index maps follow seblas/operations/cuConv.cu:105-115 (forward) and the adjoint of it for the
 // two gradients (the reference's weight-gradient map at :570-571 is wrong for stride > 1 and is not reproduced).
 #include <cstdlib>
+#include <cstring>
 
 #include "cb_ptx.cuh"
 #include "conv_gather.cuh"
+#include "conv_patch.h"
 #include "simt_core.cuh"
 #include "split_core.cuh"
 
@@ -179,6 +181,21 @@ __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_wgrad_simt(const Wgra
 // Multiplications from which a pass runs at fp32 accuracy on the tensor cores (conv_split.cu).
 constexpr long long kLeastConv = 1LL << 22;
 
+// us a launch of conv_gather_split takes, by a model fitted to 555 passes (7.5 % off on average). conv_patch.cu is taken where its own model
+// is 12 % below: over these passes 1.14 times as fast as without it (1.16 with the faster of the two each time), 2 % of them slower, by
+// 10 % on average. us without / with: forward 32 -> 32 at 28 x 28, batch 32 14.4 / 10.6, its data gradient 17.3 / 10.4; 32 -> 64 at 32 x 32,
+// stride 2, batch 128 20.9 / 16.9; 16 -> 32 5x5 at 46 x 46, batch 23 28.5 / 18.6 and 60.7 / 25.9; few channels at stride 2 stay: 5 -> 38 at
+// 32 x 32, batch 18 4.8 / 6.8.
+double gather_us(int sm_count, long long I, int OUTC, long long blocks, bool may_split, const GatherParams& p, const PixelSet* sets) {
+    const split::Choice c = split::choose_shape(sm_count, I, OUTC, blocks, 1, may_split, split::kGather);
+    const long long ctas = (I + 127) / 128 * ((OUTC + c.bn - 1) / c.bn) * c.splits;
+    const bool pairs = c.bn == 32 && ctas > sm_count, dgrad = p.sgn < 0, strided = dgrad && sets[0].ohs == 2;
+    const double block = (c.bn == 128 ? 1.303 : c.bn == 64 ? 0.756 : 0.621) * (dgrad ? 1.263 : 1.0) * (strided ? 0.833 : 1.0), load = pairs ? 1.6 : 1.0;
+    const double rounds = (double)((ctas + (pairs ? 2 : 1) * sm_count - 1) / ((pairs ? 2 : 1) * sm_count));
+    const double us = 1.0 + rounds * (2.76 + c.per_split * block * load) + (c.splits > 1 ? rounds * 128.0 * c.bn * 0.00017 * load + 0.98 : 0.0);
+    return us;
+}
+
 // One launch for up to four pixel sets. In the passes of a model the two that later layers read stay on the CUDA cores (see
 // launch_fp32_gemm), except the 3xTF32 ones that never ran there (in_models). The contraction is split over CTAs where the output alone
 // does not fill the GPU and the epilogue is a plain sum (the output is then cleared first), except in the passes of a model: atomic
@@ -193,6 +210,19 @@ int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, 
     for (int i = 0; i < nsets; ++i) most = sets[i].K > most ? sets[i].K : most;
     const long long I = (long long)p.N * sets[0].UH * sets[0].UW * nsets;
     const bool on_tensor_cores = (!ctx->model_pass || in_models) && split::worth_it(I, p.OUTC, most, 1, kLeastConv);
+    if (on_tensor_cores && !ctx->model_pass && nsets <= kMaxSets) {
+        std::memcpy(p.sets, sets, nsets * sizeof(PixelSet));
+        PatchPlan plan{};
+        void* pieces = plan_patch(ctx, p, nsets, may_split, plan) && plan.us < 0.88 * gather_us(ctx->sm_count, I, p.OUTC, (most + split::kBK - 1) / split::kBK, may_split, p, sets)
+                           ? filter_pieces(ctx, plan.filter_bytes) : nullptr;
+        if (pieces) {
+            const cudaError_t e = launch_patch(ctx, plan, pieces);
+            if (e != cudaSuccess) return check_cuda(ctx, e, who);
+            ctx->launches += 2;
+            ctx->last_kernel = "umma_fp32";
+            return CB_OK;
+        }
+    }
     simt::Choice c{};
     split::Choice sc{};
     if (on_tensor_cores) sc = split::choose_shape(ctx->sm_count, I, p.OUTC, (most + split::kBK - 1) / split::kBK, 1, may_split, split::kGather);

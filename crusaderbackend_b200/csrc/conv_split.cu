@@ -11,27 +11,6 @@ namespace {
 
 using split::kBK;
 
-// A summing thread's n outputs into memory `step` floats apart. plain: stored, or (add) added to what is there, one atomic add being
-// a read, an addition and a write without the wait for the read. Otherwise value(c, y, old place) is what is stored, or added.
-template <bool LOW, class F>
-__device__ __forceinline__ void store_columns(float* dst, long long step, int n, uint32_t mine, bool plain, bool add, F value) {
-    if (plain) {  // without a branch in the loop: reads of several columns are in flight together
-        if (add)
-#pragma unroll 8
-            for (int c = 0; c < n; ++c, dst += step) split::add_to<LOW>(dst, split::staged(mine, c));
-        else
-#pragma unroll 8
-            for (int c = 0; c < n; ++c, dst += step) *dst = split::staged(mine, c);
-        return;
-    }
-#pragma unroll 4
-    for (int c = 0; c < n; ++c, dst += step) {
-        const float y = value(c, split::staged(mine, c), dst);
-        if (add) split::add_to<LOW>(dst, y);
-        else *dst = y;
-    }
-}
-
 // Forward and data gradient: rows are pixels, columns output channels.
 template <class S, bool MASK>
 struct SplitGather {
@@ -76,7 +55,7 @@ struct SplitGather {
         float* out;
         const int place = output_of(p, s, i0 + row, out), plane = p.OHH * p.OWW, j = j0 + first;
         const bool bias = p.ep.bias && part == 0;
-        store_columns<LOW>(out + (long long)j * plane, plane, min(n, p.OUTC - j), mine,
+        split::store_columns<LOW>(out + (long long)j * plane, plane, min(n, p.OUTC - j), mine,
                       p.atomic_out ? !bias : !p.ep.scale && !p.ep.bias && !p.ep.relu, p.atomic_out || (p.ep.accumulate && !p.ep.relu && !p.ep.scale && !p.ep.bias),
                       [&](int c, float y, const float* dst) {
                           if (p.atomic_out) return y + p.ep.bias[j + c];
@@ -157,7 +136,7 @@ struct SplitWgrad {
     __device__ __forceinline__ void store(int row, int first, int n, uint32_t mine) const {
         const int i = i0 + row, j = j0 + first;
         if (i >= p.I) return;
-        store_columns<LOW>(p.dW + (long long)j * p.I + i, p.I, min(n, p.g.OC - j), mine, true, p.mode != 0, [](int, float y, const float*) { return y; });
+        split::store_columns<LOW>(p.dW + (long long)j * p.I + i, p.I, min(n, p.g.OC - j), mine, true, p.mode != 0, [](int, float y, const float*) { return y; });
     }
 };
 

@@ -500,6 +500,27 @@ __device__ __forceinline__ void run(Src& src, int blocks, uint8_t* smem_raw, Bar
     }
 }
 
+// A summing thread's n outputs into memory `step` floats apart. plain: stored, or (add) added to what is there, one atomic add being
+// a read, an addition and a write without the wait for the read. Otherwise value(c, y, old place) is what is stored, or added.
+template <bool LOW, class F>
+__device__ __forceinline__ void store_columns(float* dst, long long step, int n, uint32_t mine, bool plain, bool add, F value) {
+    if (plain) {  // without a branch in the loop: reads of several columns are in flight together
+        if (add)
+#pragma unroll 8
+            for (int c = 0; c < n; ++c, dst += step) add_to<LOW>(dst, staged(mine, c));
+        else
+#pragma unroll 8
+            for (int c = 0; c < n; ++c, dst += step) *dst = staged(mine, c);
+        return;
+    }
+#pragma unroll 4
+    for (int c = 0; c < n; ++c, dst += step) {
+        const float y = value(c, staged(mine, c), dst);
+        if (add) add_to<LOW>(dst, y);
+        else *dst = y;
+    }
+}
+
 // Whether a product comes here rather than to the CUDA cores. Contractions of less than 16: the rounding of a few fp32 FMAs is less
 // than what the six products leave out (2-norm error at K = 2: 1.8e-8 .. 3.4e-8 against 2.1e-8 .. 5.7e-8; at K = 16 7.5e-8 against
 // 5.4e-8, at 1501 3.5e-7 against 1.1e-7). Small products: bound by their launch on either path. Whether the contraction may be shared
