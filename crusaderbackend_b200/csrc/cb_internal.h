@@ -199,6 +199,8 @@ int launch_umma_gemm(cb_ctx* ctx, const GemmCall& g, bool x3);
 // *summed is set where g.q_sum has been added to.
 int launch_fp32_gemm(cb_ctx* ctx, const GemmCall& g, bool* summed = nullptr);
 int launch_split_gemm(cb_ctx* ctx, const GemmCall& g);
+// Up to 16 rows or columns, both operands with k contiguous, small: fp32 FMAs, any mode (CB_EUNSUPPORTED otherwise).
+int launch_thin_rows(cb_ctx* ctx, const GemmCall& g);
 // Clears the output matrices of a call whose partial products are added into them with atomics.
 int clear_output(cb_ctx* ctx, float* p, long long width, long long ld, long long rows, long long stride, long long batch, const char* who);
 

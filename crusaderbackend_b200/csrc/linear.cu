@@ -34,6 +34,10 @@ __global__ void __launch_bounds__(256) colsum_add_kernel(const float* __restrict
 }
 
 int run_gemm(cb_ctx* ctx, const GemmCall& g, bool* summed = nullptr) {
+    if (ctx->math != CB_MATH_FP32) {
+        const int rc = launch_thin_rows(ctx, g);
+        if (rc != CB_EUNSUPPORTED) return rc;
+    }
     if (ctx->math != CB_MATH_FP32 && umma_gemm_eligible(g)) return launch_umma_gemm(ctx, g, ctx->math == CB_MATH_3XTF32);
     return launch_fp32_gemm(ctx, g, summed);
 }
