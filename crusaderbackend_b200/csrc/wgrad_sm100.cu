@@ -37,7 +37,9 @@ struct WgradParams {
     // (X, dY) — the tensor core reads the hi part of whatever it is given — and all of it lands in one accumulator
     int vgroups;                     // groups, or 3 * groups
     int stages, tmem_cols;
-    uint32_t line_bytes, stage_bytes, a_bytes;  // one line slot of a stage / lps of them / the A part of a line slot
+    // In a stage: from a line's A rows to the next line's, to the first line's B rows, from a line's B rows to the next line's; what the
+    // copies of a stage bring of X
+    uint32_t stage_bytes, a_step, b_at, b_step, x_bytes;
     float* partial;                  // [gridDim.x][NQ][mtiles * 128]; with `atomic`: ONE such tile that every CTA adds into
     int atomic;
     // direct != 0: no second kernel. The CTA lays its tile out in the idle pipeline stages in the order of the filter
@@ -48,6 +50,11 @@ struct WgradParams {
     // FH consecutive image rows and arrive as ONE 4-D box [channel][fh][32 px]: the accumulator rows are then ordered
     // (c, fh) instead of (fh, c), and a line costs two TMA boxes instead of FH + 1.
     int rows_cf;
+    // rows_shared != 0 (the same maps, several lines a stage): the FH blocks of one line are those of the next moved by one, so a stage
+    // holds lps + FH - 1 image rows, [row][channel][32 px], as ONE box, and a line's A rows, ordered (fh, c), start one row further on. X
+    // comes 1.5 times (lps 4) or twice (2) in place of FH times, and a stage takes less room: 48 -> 12, batch 64 10.5 -> 9.7 us, 24 -> 40, batch 33
+    // 9.8 -> 9.4, 16 -> 16, batch 128 10.7 -> 10.6 (bound by the shift warps then).
+    int rows_shared;
     long long oc_stride, base_off;
     float* dW;
     int* status;
@@ -64,34 +71,22 @@ struct __align__(8) WgradSmem {
     int abort_flag;
 };
 
-// 16-byte chunk q of the 128-byte row at row_addr under the standard 128-byte swizzle (chunk ^= row index mod 8)
-__device__ __forceinline__ uint32_t sw128_chunk(uint32_t row_addr, int q) {
-    return row_addr + ((((uint32_t)q) ^ ((row_addr >> 7) & 7u)) << 4);
-}
-
 constexpr int kShiftWarps = 8;  // one scheduler cannot hide the shared-memory latencies of a single warp
 
-// One 16-byte chunk (pixels 4q .. 4q+3) of the horizontally shifted copies of a dY row: row_m1 (tap offset -1: pairs
-// X[px] with dY[px + 1]) and row_p1 (tap offset +1: pairs X[px] with dY[px - 1]); zeros enter at the edges of the
-// W-wide image rows packed in the line; an address of 0 skips that copy.
-__device__ __forceinline__ void shift_dy_chunk(uint32_t src_row, uint32_t row_m1, uint32_t row_p1, int q, int W) {
+// One 16-byte chunk (pixels 4q .. 4q+3, eight neighbouring lanes a row) of a dY row and of its horizontally shifted copies: tap offset -1 pairs
+// X[px] with dY[px + 1], tap offset +1 with dY[px - 1]. Image rows are whole chunks, so zeros enter in a chunk's last or first pixel alone.
+struct ShiftChunk {
     float4 v;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(sw128_chunk(src_row, q)));
-    float left = 0.f, right = 0.f;
-    if (q > 0) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(left) : "r"(sw128_chunk(src_row, q - 1) + 12u));
-    if (q < 7) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(right) : "r"(sw128_chunk(src_row, q + 1)));
-    const int x0 = 4 * q, wm = W - 1;
-    if (row_m1) {
-        const float a0 = ((x0 & wm) < wm) ? v.y : 0.f, a1 = (((x0 + 1) & wm) < wm) ? v.z : 0.f;
-        const float a2 = (((x0 + 2) & wm) < wm) ? v.w : 0.f, a3 = (((x0 + 3) & wm) < wm) ? right : 0.f;
-        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(sw128_chunk(row_m1, q)), "f"(a0), "f"(a1), "f"(a2), "f"(a3) : "memory");
+    __device__ __forceinline__ void load(uint32_t at) {
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
     }
-    if (row_p1) {
-        const float b0 = ((x0 & wm) >= 1) ? left : 0.f, b1 = (((x0 + 1) & wm) >= 1) ? v.x : 0.f;
-        const float b2 = (((x0 + 2) & wm) >= 1) ? v.y : 0.f, b3 = (((x0 + 3) & wm) >= 1) ? v.z : 0.f;
-        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(sw128_chunk(row_p1, q)), "f"(b0), "f"(b1), "f"(b2), "f"(b3) : "memory");
+    // m1, p1: bytes from the row to its copies, 0: there is no such tap; whole warp
+    __device__ __forceinline__ void store(uint32_t at, uint32_t m1, uint32_t p1, bool row_begins, bool row_ends, bool ok) const {
+        const float right = __shfl_down_sync(0xffffffffu, v.x, 1, 8), left = __shfl_up_sync(0xffffffffu, v.w, 1, 8);
+        if (ok && m1) asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at + m1), "f"(v.y), "f"(v.z), "f"(v.w), "f"(row_ends ? 0.f : right) : "memory");
+        if (ok && p1) asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at + p1), "f"(row_begins ? 0.f : left), "f"(v.x), "f"(v.y), "f"(v.z) : "memory");
     }
-}
+};
 
 // The four K steps (8 pixels each) of one line on one M tile; b_units: from the A tile to the line's B rows.
 __device__ __forceinline__ void issue_line(uint32_t d_tmem, uint64_t dA, uint32_t b_units, uint32_t idesc, uint32_t accumulate) {
@@ -162,7 +157,7 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
             const uint32_t s1 = s + 1 == (uint32_t)p.stages ? 0u : s + 1, ph1 = s1 ? ph : ph ^ 1u;
             ahead = mbar_test(smem_u32(&ws.empty[s1]), ph1 ^ 1u);
             const uint32_t full = smem_u32(&ws.full[s]);
-            mbar_expect_tx_elect(full, (uint32_t)p.lps * (p.a_bytes + set_bytes));
+            mbar_expect_tx_elect(full, p.x_bytes + (uint32_t)p.lps * set_bytes);
             // 3xTF32 form: the two small cross terms first, while the accumulator is small (the tensor core's
             // fp32 accumulation error is relative to what the accumulator holds), the hi x hi products last
             const int pass = x3 ? g / p.groups : 0, gg = g - pass * p.groups;
@@ -171,16 +166,19 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
             // lines past the end use an image index >= N: their boxes are zero-filled and add nothing
             const int g0 = gg * p.lps;  // total_lines < 2^29 (checked on the host)
             int n = g0 / p.LPI, line = g0 - n * p.LPI;
+            const uint32_t stage = st_base + s * p.stage_bytes;
+            if (p.rows_shared) tma_load_4d_elect(stage, mx, full, 0, 0, line - p.pH, n);
             for (int l = 0; l < p.lps; ++l) {
-                const uint32_t stg = st_base + s * p.stage_bytes + (uint32_t)l * p.line_bytes;
+                const uint32_t stg = stage + (uint32_t)l * p.a_step;
                 const int h0 = line * p.L;
-                if (p.rows_cf) {
+                if (p.rows_shared) {
+                } else if (p.rows_cf) {
                     tma_load_4d_elect(stg, mx, full, 0, h0 - p.pH, 0, n);
                 } else {
                     for (int fh = 0; fh < p.FH; ++fh)
                         tma_load_3d_elect(stg + (uint32_t)fh * p.Cp * kRowBytes, mx, full, (h0 + fh - p.pH) * p.W, 0, n);
                 }
-                tma_load_3d_elect(stg + p.a_bytes + (uint32_t)centre * set_bytes, my, full, h0 * p.W, oc_first, n);
+                tma_load_3d_elect(stage + p.b_at + (uint32_t)l * p.b_step + (uint32_t)centre * set_bytes, my, full, h0 * p.W, oc_first, n);
                 if (++line == p.LPI) {
                     line = 0;
                     ++n;
@@ -197,7 +195,7 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
         // The whole warp runs the loop with the same values (waits go through votes) and one elected lane issues: the
         // descriptors stay in uniform registers (see umma_tf32_elect).
         const bool shifted = p.FW > 1;
-        const uint32_t line_units = p.line_bytes >> 4, a_units = p.a_bytes >> 4;  // descriptor address units
+        const uint32_t a_units = p.a_step >> 4, b_units = p.b_at >> 4, ba_units = (p.b_step >> 4) - (p.a_step >> 4);  // descriptor address units
         uint32_t s = 0, ph = 0, ahead = 0;
         bool first_line = true;
         for (int g = cta; g < p.vgroups; g += ctas) {
@@ -215,12 +213,12 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
             if (p.lps == 4 && p.mtiles == 1) {  // the narrow layers: 16 small UMMAs, whose loop would cost as much as they do
 #pragma unroll
                 for (uint32_t l = 0; l < 4; ++l)
-                    issue_line(tmem_base, stg + (uint64_t)(l * line_units), a_units, idesc, first_line && l == 0 ? 0u : 1u);
+                    issue_line(tmem_base, stg + (uint64_t)(l * a_units), b_units + l * ba_units, idesc, first_line && l == 0 ? 0u : 1u);
             } else {
                 for (uint32_t l = 0; l < (uint32_t)p.lps; ++l)
                     for (uint32_t m = 0; m < (uint32_t)p.mtiles; ++m) {
                         const uint32_t shift = m * (16384u >> 4);
-                        issue_line(tmem_base + m * (uint32_t)p.NQ, stg + (uint64_t)(l * line_units + shift), a_units - shift, idesc,
+                        issue_line(tmem_base + m * (uint32_t)p.NQ, stg + (uint64_t)(l * a_units + shift), b_units + l * ba_units - shift, idesc,
                                    first_line && l == 0 ? 0u : 1u);
                     }
             }
@@ -235,23 +233,38 @@ __global__ void __launch_bounds__(192 + 32 * kShiftWarps, 1)
     } else {
         // ------------------------------------------------------------ shift warps (6..): fw = 0 and fw = 2 copies of dY
         if (warp >= 6 && p.FW > 1) {
-            const int t = threadIdx.x - 192;
+            // A thread takes one chunk of every 32nd row (a multiple of the swizzle's eight, so its place in the row is the same in all of them);
+            // where those lie in a stage is worked out once, and a stage's reads are all under way before the first is used. Reading the
+            // neighbours' pixels from shared memory too, four-way bank conflicts, one row after the other, these warps were the bound of
+            // most launches: 16 -> 16 at 32 x 32, batch 128 10.6 -> 8.6 us, 64 -> 64 30.9 -> 25.7.
+            constexpr int kRows = 4;  // of a thread at a time
+            const int t = threadIdx.x - 192, rows = p.lps * p.OCp, q = t & 7, row0 = t >> 3;
+            const uint32_t chunk = (uint32_t)(q ^ (row0 & 7)) << 4;
+            auto place = [&](int row) {
+                uint32_t at = chunk;
+                for (; row >= p.OCp; row -= p.OCp) at += p.b_step;
+                return at + (uint32_t)row * kRowBytes;
+            };
+            uint32_t at[kRows];
+#pragma unroll
+            for (int u = 0; u < kRows; ++u) at[u] = place(min(row0 + 32 * u, rows - 1));
+            const uint32_t m1 = centre >= 1 ? 0u - set_bytes : 0u, p1 = centre + 1 < p.FW ? set_bytes : 0u;  // taps fw = pW - 1, pW + 1
+            const bool row_begins = ((4 * q) & (p.W - 1)) == 0, row_ends = ((4 * q + 4) & (p.W - 1)) == 0;
             uint32_t s = 0, ph = 0;
-            // item = (row, 16-byte chunk) of a line; a thread's items keep their chunk (32 * kShiftWarps is a multiple of 8)
-            const int rows = p.lps * p.OCp, q = t & 7;
             for (int g = cta; g < p.vgroups; g += ctas) {
                 if (!mbar_wait_uniform(smem_u32(&ws.full[s]), ph, abort_flag, p.status, CBK_TIMEOUT_XFORM_FULL)) break;
-                const uint32_t base = st_base + s * p.stage_bytes + p.a_bytes + (uint32_t)centre * set_bytes;
-                int l = 0, row = t >> 3;
-                for (int r = t >> 3; r < rows; r += 4 * kShiftWarps, row += 4 * kShiftWarps) {
-                    while (row >= p.OCp) {
-                        row -= p.OCp;
-                        ++l;
-                    }
-                    const uint32_t src = base + (uint32_t)l * p.line_bytes + (uint32_t)row * kRowBytes;
-                    const uint32_t m1 = centre >= 1 ? src - set_bytes : 0u;             // tap fw = pW - 1
-                    const uint32_t p1 = centre + 1 < p.FW ? src + set_bytes : 0u;       // tap fw = pW + 1
-                    shift_dy_chunk(src, m1, p1, q, p.W);
+                const uint32_t base = st_base + s * p.stage_bytes + p.b_at + (uint32_t)centre * set_bytes;
+                ShiftChunk c[kRows];
+#pragma unroll
+                for (int u = 0; u < kRows; ++u)
+                    if (32 * u < rows) c[u].load(base + at[u]);
+#pragma unroll
+                for (int u = 0; u < kRows; ++u)
+                    if (32 * u < rows) c[u].store(base + at[u], m1, p1, row_begins, row_ends, row0 + 32 * u < rows);
+                for (int r = 32 * kRows; r < rows; r += 32) {
+                    const uint32_t more = base + place(min(row0 + r, rows - 1));
+                    c[0].load(more);
+                    c[0].store(more, m1, p1, row_begins, row_ends, row0 + r < rows);
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
@@ -568,8 +581,23 @@ static int wgrad_core(cb_ctx* ctx, const float* dY, const float* X, float* dW, i
     }
     if (sh.nsplit == 0) return CB_EUNSUPPORTED;
     const int OCp = sh.OCp, NQ = sh.NQ, lps = sh.lps, grid = sh.grid;
-    const uint32_t line_bytes = sh.line_bytes, stage_bytes = (uint32_t)lps * line_bytes;
-    const long long stages = sh.stages;
+    // The choice above, by lines of their own, stays: which lines a CTA sums is part of a gradient's last bits.
+    long long stages = sh.stages;
+    uint32_t a_step = sh.line_bytes, b_at = (uint32_t)rowsA * kRowBytes, b_step = sh.line_bytes, stage_bytes = (uint32_t)lps * sh.line_bytes;
+    uint32_t x_bytes = (uint32_t)lps * (uint32_t)rowsA * kRowBytes;
+    bool rows_shared = false;
+    if (IW == 32 && FH == 3 && !s2 && lps > 1 && IH % lps == 0) {
+        const uint32_t row = (uint32_t)Cp * kRowBytes, rows = (uint32_t)(lps + FH - 1) * row, set = (uint32_t)NQ * kRowBytes;
+        // an M tile's 128 rows may begin in the last line's few and must end in the stage
+        const uint32_t reach = (uint32_t)(lps - 1) * row + (uint32_t)mtiles * 128u * kRowBytes, bytes = rows + (uint32_t)lps * set;
+        const uint32_t whole = ((bytes < reach ? reach : bytes) + 1023u) & ~1023u;
+        const long long fit = smem_cap / whole < kConvMaxStages ? smem_cap / whole : kConvMaxStages, tile = 4LL * OCp * run;
+        rows_shared = tile <= fit * whole || tile > stages * (long long)stage_bytes;  // the tile leaves as it would have
+        if (rows_shared) {
+            a_step = row; b_at = x_bytes = rows; b_step = set; stage_bytes = whole;
+            stages = fit;
+        }
+    }
 
     WgradParams p{};
     p.N = N; p.Cin = Cin; p.H = IH; p.W = IW; p.OC = OC;
@@ -582,9 +610,8 @@ static int wgrad_core(cb_ctx* ctx, const float* dY, const float* X, float* dW, i
     int cols = 32;
     while (cols < mtiles * NQ) cols <<= 1;
     p.tmem_cols = cols;
-    p.line_bytes = line_bytes;
     p.stage_bytes = stage_bytes;
-    p.a_bytes = (uint32_t)rowsA * kRowBytes;
+    p.a_step = a_step; p.b_at = b_at; p.b_step = b_step; p.x_bytes = x_bytes;
     p.lps = lps;
     p.groups = (int)((p.total_lines + lps - 1) / lps);
     p.vgroups = lo.x ? 3 * p.groups : p.groups;
@@ -594,7 +621,8 @@ static int wgrad_core(cb_ctx* ctx, const float* dY, const float* X, float* dW, i
     // zero-filled tile that every CTA adds into with atomics and the second kernel moves into dW and clears again.
     p.atomic = ctx->deterministic ? 0 : 1;
     p.s2 = s2; p.IC_src = IC_src;
-    p.rows_cf = (IW == 32 && FH > 1 && !s2) ? 1 : 0;
+    p.rows_shared = rows_shared ? 1 : 0;
+    p.rows_cf = (IW == 32 && FH > 1 && !s2 && !rows_shared) ? 1 : 0;
     p.run = run;
     p.oc_stride = s2 ? (long long)IC_src * 9 : (long long)IC_total * FH * FW;
     p.base_off = s2 ? 0 : ((long long)oc_off * IC_total + c_off) * FH * FW;
@@ -623,6 +651,12 @@ static int wgrad_core(cb_ctx* ctx, const float* dY, const float* X, float* dW, i
     auto encode_x = [&](CUtensorMap* tm, const float* base, long long batch) -> int {
         const uint64_t bstride = (uint64_t)(batch ? batch : (long long)Cin * IH * IW) * 4;
         if (bstride & 15u) return CB_EUNSUPPORTED;
+        if (rows_shared) {
+            uint64_t dims[4] = {32u, (uint64_t)Cin, (uint64_t)IH, (uint64_t)N};
+            uint64_t str[3] = {(uint64_t)IH * IW * 4, 128u, bstride};
+            uint32_t box[4] = {32u, (uint32_t)Cp, (uint32_t)(lps + FH - 1), 1u};
+            return encode_tmap(ctx, tm, base, 4, dims, str, box, nullptr, 128);
+        }
         if (p.rows_cf) {
             uint64_t dims[4] = {32u, (uint64_t)IH, (uint64_t)Cin, (uint64_t)N};
             uint64_t str[3] = {128u, (uint64_t)IH * IW * 4, bstride};
