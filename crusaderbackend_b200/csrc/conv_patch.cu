@@ -6,7 +6,8 @@
 // reach beyond the tensor; those read 0. A tap is then one constant distance on that line. Shared memory holds, per piece and group of
 // 8 channels, 16 bytes (8 bf16) a position: K-major core matrices without swizzle whose 8 rows are 8 neighbouring positions, so a UMMA's
 // A operand for a tap is the same memory from another first position on. A stride of 2 splits the input into the four planes of even and odd
-// rows and columns, each a line of its own; the data gradient of stride 2 is four sets of pixels (conv_gather.cuh) with 1, 2, 2 and 4 taps.
+// rows and columns, each a line of its own; the data gradient of stride 2 is two sets of pixels, of even and odd rows, with the even and odd
+// columns side by side in the product (plan_patch).
 //
 // A UMMA of few columns is bound by reading its 128 rows of A, so the pieces of the filter are stacked in N: x1 meets [y1 y2 y3], x2
 // [y1 y2] and x3 [y1], in three groups of accumulator columns for products of the orders 1, 2^-8 and 2^-16: 3 UMMAs a step instead of 6
@@ -16,7 +17,7 @@
 // pack_patch_filter has made before, and summing warps, which help with the first patch.
 //
 // us, conv_split.cu's gather / here: 32 -> 32 3x3, 28 x 28, batch 32, forward 14.4 / 10.6, data gradient 17.3 / 10.4; 32 -> 64 3x3 stride 2, 32 x
-// 32, batch 128 20.9 / 16.9; 128 -> 128 3x3, 4 maps of 56 x 56 37.7 / 30.8 and 64.1 / 30.8; 16 -> 32 5x5, 46 x 46, batch 23 28.5 / 18.6 and
+// 32, batch 128 20.9 / 17.5, its data gradient 36.3 / 24.9; 128 -> 128 3x3, 4 maps of 56 x 56 37.7 / 30.8 and 64.1 / 30.8; 16 -> 32 5x5, 46 x 46, batch 23 28.5 / 18.6 and
 // 60.7 / 25.9. What bounds it now: in the first of these 3.2 us are pack_patch_filter's, 2.6 a CTA's start until its first patch is there; then
 // UMMAs, 60 clocks each whatever their width, and between blocks of them the hand-over of accumulators (a second issuing warp, a
 // second CTA on the SM). One CTA an SM that walks over tiles, fetching ahead, took 12.7 us there: what a patch warp executes for a run of
@@ -36,6 +37,7 @@ namespace {
 constexpr int kMaxRing = 4;   // slots of the patch and the filter ring at most
 constexpr int kChain = 5;     // steps of 16 k whose sum stays in TMEM
 constexpr int kGroup = 8;     // blocks whose sums are added one after another
+constexpr unsigned kAbsent = 0x7fc0abe5u;  // in a slice of the second pass: a tap that a phase of the output does not have
 constexpr int kPackCols = 8;  // columns of a block of pack_patch_filter
 
 // Two CTAs an SM, so that one computes while the other starts, adds or stores. Each has 256 columns of TMEM: two accumulators of 3 x 32
@@ -59,6 +61,11 @@ struct __align__(8) PatchBarriers {
     int cut;           // of the second pass: factors below split::kWhole; the largest factor's magnitude, as bits
     unsigned largest;
 };
+
+// The parameters arrive 64 bytes a miss: every warp asks for a part, or the misses come one after the other as the code gets to them.
+__device__ __forceinline__ void fetch_parameters(const PatchParams& q, int warp, int warps) {
+    for (int at = warp * 16; at < (int)(sizeof(PatchParams) / 4); at += warps * 16) asm volatile("" ::"r"(reinterpret_cast<const int*>(&q)[at]));
+}
 
 // What a CTA does at a time: a tile of pixels of a set, a column tile, a share of the contraction.
 struct PatchItem {
@@ -153,7 +160,7 @@ __device__ __forceinline__ void fetch_patch(const PatchParams& q, const PatchIte
 
 // The second pass of split::Again, by the summing warps alone: the share's products once more by fp32 FMAs in the CUDA cores' order, for the
 // outputs of warps that want it; (row, first ...) are a thread's.
-template <class S>
+template <class S, bool FOLD>
 __device__ __noinline__ void sum_again(const PatchParams& q, const PatchItem& it, PatchBarriers& b, uint32_t slice, uint32_t mine, int row, int first, bool wanted) {
     const GatherParams& p = q.p;
     const PixelSet& s = p.sets[it.set];
@@ -196,11 +203,11 @@ __device__ __noinline__ void sum_again(const PatchParams& q, const PatchItem& it
         for (int i = tid; i < S::kSlice * S::BN; i += kThreads) {
             const int k = i / S::BN, j = it.j0 + i % S::BN;
             float y = 0.f;
-            if (k0 + k < K && j < p.OUTC) {
+            if (k0 + k < K && j < q.cols) {
                 int tap, c;
                 place(k0 + k, tap, c);
-                const int th = tap / s.TW, tw = tap - th * s.TW;
-                y = __ldg(p.Wt + (long long)j * p.w_out + (long long)c * p.w_ch + (s.wt0 + s.wts * th) * p.FW + s.wu0 + s.wus * tw);
+                const int th = tap / s.TW, at = q.filter_of<FOLD>(it.set, th, tap - th * s.TW, j);
+                y = at < 0 ? __uint_as_float(kAbsent) : __ldg(p.Wt + (long long)(FOLD ? j >> 1 : j) * p.w_out + (long long)c * p.w_ch + at);
             }
             put(S::kSlice * S::BM + i, y);
         }
@@ -215,10 +222,11 @@ __device__ __noinline__ void sum_again(const PatchParams& q, const PatchItem& it
                 float y0, y1, y2, y3;
                 asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(y0), "=f"(y1), "=f"(y2), "=f"(y3)
                              : "r"(slice + (uint32_t)(S::kSlice * S::BM + k * S::BN + first + c) * 4u) : "memory");
-                plain[c] = fmaf(x, y0, plain[c]);
-                plain[c + 1] = fmaf(x, y1, plain[c + 1]);
-                plain[c + 2] = fmaf(x, y2, plain[c + 2]);
-                plain[c + 3] = fmaf(x, y3, plain[c + 3]);
+                // (0 in place of a tap that a phase does not have would make a NaN of an infinity)
+                if (!FOLD || __float_as_uint(y0) != kAbsent) plain[c] = fmaf(x, y0, plain[c]);
+                if (!FOLD || __float_as_uint(y1) != kAbsent) plain[c + 1] = fmaf(x, y1, plain[c + 1]);
+                if (!FOLD || __float_as_uint(y2) != kAbsent) plain[c + 2] = fmaf(x, y2, plain[c + 2]);
+                if (!FOLD || __float_as_uint(y3) != kAbsent) plain[c + 3] = fmaf(x, y3, plain[c + 3]);
             }
         }
     }
@@ -235,7 +243,7 @@ __device__ __noinline__ void sum_again(const PatchParams& q, const PatchItem& it
     asm volatile("bar.sync 3, %0;" ::"n"(kThreads) : "memory");  // b.cut is the next tile's
 }
 
-template <class S>
+template <class S, bool FOLD>
 __global__ void __launch_bounds__(S::NT, S::kCtas) conv_patch_kernel(const __grid_constant__ PatchParams q, int* status) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ PatchBarriers b;
@@ -243,9 +251,7 @@ __global__ void __launch_bounds__(S::NT, S::kCtas) conv_patch_kernel(const __gri
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t base = (smem_u32(smem_raw) + 127u) & ~127u;
     const uint32_t fbase = base + q.pslots * q.pslot_bytes, staging = base;  // what the sums are staged in has been read by then
-    // The parameters arrive 64 bytes a miss: every warp asks for a part, or the misses come one after the other as the code gets to them.
-    for (int at = warp * 16; at < (int)(sizeof(PatchParams) / 4); at += S::NT / 32 * 16)
-        asm volatile("" ::"r"(reinterpret_cast<const int*>(&q)[at]));
+    fetch_parameters(q, warp, S::NT / 32);
     volatile int* abort_flag = &b.abort_flag;
     const PatchItem it(q, blockIdx.x, S::BN);
     const PatchSet& ps = q.sets[it.set];
@@ -442,17 +448,39 @@ __global__ void __launch_bounds__(S::NT, S::kCtas) conv_patch_kernel(const __gri
         const bool wanted = __any_sync(0xffffffffu, live && ok && ((zeros & 0x7fffffff7fffffffull) != 0 || smallest < 2u * __float_as_uint(split::kLow) - 1u));
         uint32_t again;  // any warp's
         asm volatile("{\n\t.reg .pred w, r;\n\tsetp.ne.b32 w, %1, 0;\n\tbarrier.cta.red.or.pred r, 3, %2, w;\n\tselp.b32 %0, 1, 0, r;\n\t}" : "=r"(again) : "r"((int)wanted), "n"(32 * S::kSumWarps) : "memory");
-        if (again) sum_again<S>(q, it, b, slice, mine, row, first, wanted);
+        if (again) sum_again<S, FOLD>(q, it, b, slice, mine, row, first, wanted);
         if (live && ok) {
             const int plane = p.OHH * p.OWW, place = (s.oh0 + s.ohs * u) * p.OWW + s.ow0 + s.ows * v, j = it.j0 + first;
-            float* out = p.Out + (long long)n * p.out_batch + place + (long long)j * plane;
+            float* out = p.Out + (long long)n * p.out_batch + place + (long long)(FOLD ? j >> 1 : j) * plane;
             const bool bias = p.ep.bias && it.part == 0, plain = p.atomic_out ? !bias : !p.ep.scale && !p.ep.bias && !p.ep.relu;
             const bool add = p.atomic_out || (p.ep.accumulate && !p.ep.relu && !p.ep.scale && !p.ep.bias);
             auto value = [&](int c, float y, const float* dst) {
                 if (p.atomic_out) return y + p.ep.bias[j + c];
                 return apply_epilogue(p.ep, y, j + c, (long long)(j + c) * plane + place, p.ep.accumulate ? *dst : 0.f);
             };
-            if (wanted) split::store_columns<true>(out, plane, min(S::kCols, p.OUTC - j), mine, plain, add, value);
+            if (FOLD) {  // two neighbouring columns of a channel; a data gradient has no epilogue but the addition
+                const int count = min(S::kCols, q.cols - j) / 2;
+                const bool both = v < ps.phase_UW[1];
+                const bool pairs = both && !add && ((plane | p.OWW) & 1) == 0 && (p.out_batch & 1) == 0 && (reinterpret_cast<uintptr_t>(p.Out) & 7u) == 0;
+#pragma unroll 4
+                for (int c = 0; c < count; ++c, out += plane) {
+                    const float y0 = split::staged(mine, 2 * c), y1 = split::staged(mine, 2 * c + 1);
+                    if (pairs) {
+                        *reinterpret_cast<float2*>(out) = make_float2(y0, y1);
+                    } else if (add) {
+                        if (wanted) {
+                            split::add_to<true>(out, y0);
+                            if (both) split::add_to<true>(out + 1, y1);
+                        } else {
+                            atomicAdd(out, y0);
+                            if (both) atomicAdd(out + 1, y1);
+                        }
+                    } else {
+                        out[0] = y0;
+                        if (both) out[1] = y1;
+                    }
+                }
+            } else if (wanted) split::store_columns<true>(out, plane, min(S::kCols, p.OUTC - j), mine, plain, add, value);
             else split::store_columns<false>(out, plane, min(S::kCols, p.OUTC - j), mine, plain, add, value);
         }
     }
@@ -478,7 +506,8 @@ __global__ void __launch_bounds__(S::NT, S::kCtas) conv_patch_kernel(const __gri
 // [piece][BN columns][8 bf16], steps as in ChunkSteps (16 channels, the taps of those, ...). A block takes the 16 channels of 8
 // columns, all taps: its values are runs of consecutive floats, of a column or of a channel. Splitting the filter in every CTA took
 // four times as long as the patches (128 -> 128, 4 maps of 56 x 56: 88 us).
-__global__ void __launch_bounds__(128, 16) pack_patch_filter(const __grid_constant__ PatchParams q, uint8_t* out, int bn, int packing, uint32_t clear) {
+template <bool FOLD>
+__global__ void __launch_bounds__(128, 8) pack_patch_filter(const __grid_constant__ PatchParams q, uint8_t* out, int bn, int packing, uint32_t clear) {
     extern __shared__ float raw[];
     griddep_wait_then_launch();
     const GatherParams& p = q.p;
@@ -494,10 +523,10 @@ __global__ void __launch_bounds__(128, 16) pack_patch_filter(const __grid_consta
     const int c16 = (int)blockIdx.x % groups, column = (int)blockIdx.x / groups % columns, set = (int)blockIdx.x / groups / columns;
     const PixelSet& s = p.sets[set];
     const int F = q.filter_plane, c0 = c16 * 16, j0 = column * kPackCols, taps = s.TH * s.TW;
-    const int runs = q.run_out ? kPackCols : 16, len = (q.run_out ? 16 : kPackCols) * F, pitch = len | 1;
-    const int channels = min(16, p.C - c0), here = max(0, min(kPackCols, p.OUTC - j0));
+    const int runs = q.run_out ? kPackCols >> (FOLD ? 1 : 0) : 16, len = (q.run_out ? 16 : kPackCols >> (FOLD ? 1 : 0)) * F, pitch = len | 1;
+    const int channels = min(16, p.C - c0), here = max(0, min(kPackCols >> (FOLD ? 1 : 0), p.OUTC - (j0 >> (FOLD ? 1 : 0))));
     const int real_runs = q.run_out ? here : channels, real_len = (q.run_out ? channels : here) * F;
-    const float* src = p.Wt + (long long)c0 * p.w_ch + (long long)j0 * p.w_out;
+    const float* src = p.Wt + (long long)c0 * p.w_ch + (long long)(j0 >> (FOLD ? 1 : 0)) * p.w_out;
     const long long step = q.run_out ? p.w_out : p.w_ch;
     for (int i0 = threadIdx.x; i0 < runs * len; i0 += 9 * 128) {  // a 3x3 filter's loads all at once
         float v[9];
@@ -518,12 +547,12 @@ __global__ void __launch_bounds__(128, 16) pack_patch_filter(const __grid_consta
     uint8_t* dst = out + q.sets[set].filter_at + ((long long)tile * steps + (long long)c16 * taps) * (2u * group);
     for (int i = threadIdx.x; i < taps * 2 * kPackCols; i += 128) {
         const int n = i % kPackCols, g = i / kPackCols % 2, t = i / (2 * kPackCols), th = t / s.TW, tw = t - th * s.TW;
-        const int at = (s.wt0 + s.wts * th) * p.FW + s.wu0 + s.wus * tw;
+        const int at = q.filter_of<FOLD>(set, th, tw, n), col = n >> (FOLD ? 1 : 0);
         uint32_t y[3][4];
 #pragma unroll
         for (int e = 0; e < 8; e += 2) {
             float v[2];
-            for (int x = 0; x < 2; ++x) v[x] = raw[q.run_out ? n * pitch + (8 * g + e + x) * F + at : (8 * g + e + x) * pitch + n * F + at];
+            for (int x = 0; x < 2; ++x) v[x] = at < 0 ? 0.f : raw[q.run_out ? col * pitch + (8 * g + e + x) * F + at : (8 * g + e + x) * pitch + col * F + at];
             split::split2(v[0], v[1], y[0][e / 2], y[1][e / 2], y[2][e / 2]);
         }
 #pragma unroll
@@ -589,11 +618,37 @@ bool fit(const cb_ctx* ctx, const GatherParams& p, int nsets, PatchPlan& plan) {
 }  // namespace
 
 // Whether the launch can come here, and how. Shares of the contraction are whole chunks of channels.
-bool plan_patch(const cb_ctx* ctx, const GatherParams& p, int nsets, bool may_split, PatchPlan& best) {
-    if (nsets < 1 || nsets > kMaxSets || p.N < 1) return false;
+bool plan_patch(const cb_ctx* ctx, const GatherParams& given, int nsets, bool may_split, PatchPlan& best) {
+    if (nsets < 1 || nsets > kMaxSets || given.N < 1) return false;
     PatchPlan plan{};
     PatchParams& q = plan.q;
-    q.p = p;
+    q.p = given;
+    GatherParams& p = q.p;
+    // The four sets of a stride-2 data gradient as two, of even and odd rows, whose column phases lie side by side in the product: the patch of
+    // a distance serves both, and pairs of columns leave together. 32 -> 64 at 32 x 32, batch 128: 34.5 us as
+    // four sets, 26.0.
+    q.fold = nsets == 4 && p.sgn < 0 && p.sets[0].ohs == 2 && p.sets[0].ows == 2 ? 1 : 0;
+    if (q.fold) {
+        for (int a = 0; a < 2; ++a) {
+            const PixelSet even = p.sets[2 * a], odd = p.sets[2 * a + 1];
+            PixelSet s = even;
+            PatchSet& ps = q.sets[a];
+            int lo = 1 << 20, hi = -(1 << 20);  // columns the taps of either phase reach
+            const PixelSet* phases[2] = {&even, &odd};
+            for (int b = 0; b < 2; ++b) {
+                ps.f0[b] = phases[b]->wu0; ps.phase_wb[b] = phases[b]->wb; ps.phase_UW[b] = phases[b]->UW;
+                if (phases[b]->TW == 0) continue;
+                hi = phases[b]->wb > hi ? phases[b]->wb : hi;
+                lo = phases[b]->wb - phases[b]->TW + 1 < lo ? phases[b]->wb - phases[b]->TW + 1 : lo;
+            }
+            s.wb = hi >= lo ? hi : 0;
+            s.TW = hi >= lo ? hi - lo + 1 : 0;
+            s.UW = even.UW > odd.UW ? even.UW : odd.UW;
+            p.sets[a] = s;
+        }
+        nsets = 2;
+    }
+    q.cols = p.OUTC << q.fold;
     int GH = 1, GW = 1, px = 128;
     long long useful = 0;
     struct Reach {
@@ -666,13 +721,13 @@ bool plan_patch(const cb_ctx* ctx, const GatherParams& p, int nsets, bool may_sp
         ps.segs = FastDiv(((ps.planes * px >> ps.pairs) + 31) / 32);
     }
     q.run_out = p.w_ch < p.w_out || (p.w_ch == p.w_out && p.C == 1) ? 1 : 0;
-    q.run = FastDiv((q.run_out ? 16 : kPackCols) * q.filter_plane);
+    q.run = FastDiv((q.run_out ? 16 : kPackCols >> q.fold) * q.filter_plane);
     double best_cost = 1e300;
     for (int bn = 64; bn >= 32; bn /= 2) {
         PatchPlan c = plan;
         c.bn = bn;
         if (!(bn == 64 ? fit<64>(ctx, c.q.p, nsets, c) : fit<32>(ctx, c.q.p, nsets, c))) continue;
-        const long long groups = (long long)((p.OUTC + bn - 1) / bn) * nsets;
+        const long long groups = (long long)((q.cols + bn - 1) / bn) * nsets;
         double steps = 0, runs = 0;  // of a set: steps, and runs of 32 positions x 8 channels of a chunk's patch
         for (int i = 0; i < nsets; ++i) {
             steps += (double)c.q.sets[i].steps / nsets;
@@ -701,7 +756,7 @@ bool plan_patch(const cb_ctx* ctx, const GatherParams& p, int nsets, bool may_sp
                 best.q.p.per_split = per;
                 best.q.items = (uint32_t)items;
                 best.q.tiles = FastDiv(tiles);
-                best.q.columns = FastDiv((p.OUTC + bn - 1) / bn);
+                best.q.columns = FastDiv((q.cols + bn - 1) / bn);
                 best.q.splits = FastDiv(splits);
                 best.q.image_out = FastDiv((long long)p.OUTC * p.OHH * p.OWW);
             }
@@ -711,7 +766,7 @@ bool plan_patch(const cb_ctx* ctx, const GatherParams& p, int nsets, bool may_sp
     best.nsets = nsets;
     best.q.p.atomic_out = best.q.p.splits > 1 ? 1 : 0;
     long long bytes = 0;
-    const long long columns = (p.OUTC + best.bn - 1) / best.bn;
+    const long long columns = (q.cols + best.bn - 1) / best.bn;
     for (int i = 0; i < nsets; ++i) {
         best.q.sets[i].filter_at = bytes;
         bytes += columns * ((p.C + 15) / 16) * p.sets[i].TH * p.sets[i].TW * 96LL * best.bn;
@@ -722,21 +777,22 @@ bool plan_patch(const cb_ctx* ctx, const GatherParams& p, int nsets, bool may_sp
 
 cudaError_t launch_patch(cb_ctx* ctx, PatchPlan& plan, void* scratch) {
     plan.q.filter = static_cast<const uint8_t*>(scratch);
-    const int cols = (plan.q.p.OUTC + plan.bn - 1) / plan.bn * plan.bn;
-    const int F = plan.q.filter_plane, raw = (plan.q.run_out ? kPackCols * (16 * F | 1) : 16 * (kPackCols * F | 1)) * 4;
+    const int cols = (plan.q.cols + plan.bn - 1) / plan.bn * plan.bn;
+    const int F = plan.q.filter_plane, raw = (plan.q.run_out ? kPackCols * (16 * F | 1) : 16 * (kPackCols * F | 1)) * 4;  // (half of it with fold)
     // further blocks clear the output where shares of the contraction are added up in it
     const uint32_t clear = plan.q.p.atomic_out && !plan.q.p.ep.accumulate ? plan.q.image_out.d * (uint32_t)plan.q.p.N : 0u;
     const long long packing = (plan.q.p.C + 15LL) / 16 * (cols / kPackCols) * plan.nsets;
     const long long clearing = ((long long)clear + 1023) / 1024 < 8LL * ctx->sm_count ? ((long long)clear + 1023) / 1024 : 8LL * ctx->sm_count;
-    cudaError_t ep = launch_dep(ctx, pack_patch_filter, dim3((unsigned)(packing + clearing)), dim3(128), (size_t)raw, plan.q, static_cast<uint8_t*>(scratch), plan.bn,
+    cudaError_t ep = launch_dep(ctx, plan.q.fold ? pack_patch_filter<true> : pack_patch_filter<false>, dim3((unsigned)(packing + clearing)), dim3(128), (size_t)raw, plan.q, static_cast<uint8_t*>(scratch), plan.bn,
                                 (int)packing, clear);
     if (ep == cudaSuccess) ep = cudaGetLastError();
     if (ep != cudaSuccess) return ep;
     auto go = [&](auto shape) {
         typedef decltype(shape) S;
-        cudaError_t e = raise_dynamic_smem_once(conv_patch_kernel<S>, ctx->device, ctx->max_smem_optin, nullptr);
+        auto kernel = plan.q.fold ? conv_patch_kernel<S, true> : conv_patch_kernel<S, false>;
+        cudaError_t e = raise_dynamic_smem_once(kernel, ctx->device, ctx->max_smem_optin, nullptr);
         if (e != cudaSuccess) return e;
-        e = launch_dep(ctx, conv_patch_kernel<S>, dim3(plan.q.items), dim3(S::NT), plan.smem, plan.q, ctx->d_status);
+        e = launch_dep(ctx, kernel, dim3(plan.q.items), dim3(S::NT), plan.smem, plan.q, ctx->d_status);
         return e == cudaSuccess ? cudaGetLastError() : e;
     };
     return plan.bn == 64 ? go(PatchShape<64>{}) : go(PatchShape<32>{});

@@ -14,6 +14,9 @@ struct ChunkSteps {
 struct PatchSet {
     int planes;          // input planes the taps read: 1, or up to four of even / odd rows and columns
     int ph[4], pw[4];    // row and column phase of each
+    // fold: the set holds the even and odd output columns of a stride-2 data gradient; column 2c + b of the product is phase b of channel c.
+    // Tap tw of the set, distance wb - tw, is filter column f0[b] + 2 (phase_wb[b] - wb + tw) of phase b, where the filter has that.
+    int f0[2], phase_wb[2], phase_UW[2];
     int distance[kPatchTaps];  // of each tap in a patch, planes one behind the other: where its first row of A lies
     int taps, steps;     // of the set; steps of its whole contraction
     int pairs;           // planes 2k and 2k + 1 are even and odd columns of the same rows and are read together
@@ -29,6 +32,7 @@ struct PatchParams {
     uint32_t items;                      // tiles x column tiles x shares x sets
     FastDiv tiles = FastDiv(1), columns = FastDiv(1), splits = FastDiv(1);
     int chunks;                          // of cw channels
+    int fold, cols;                      // every set's; columns of the product: output channels, twice as many with fold
     FastDiv image_out = FastDiv(1);      // by the values of an output image (pack_patch_filter clears it)
     FastDiv run = FastDiv(1);            // by a run of the filter's values (pack_patch_filter)
     FastDiv image = FastDiv(1), row = FastDiv(1);  // by GH * GW, by GW
@@ -38,6 +42,16 @@ struct PatchParams {
     int pslots, fslots;                  // ring slots of patches and of filter blocks
     uint32_t pslot_bytes, fslot_bytes;
     const uint8_t* filter;               // packed (pack_patch_filter)
+    // Offset in a filter plane of tap (th, tw) for column j of the product, -1 where that phase has no such tap.
+    template <bool FOLD>
+    __device__ __forceinline__ int filter_of(int set, int th, int tw, int j) const {
+        const gather::PixelSet& s = p.sets[set];
+        const PatchSet& ps = sets[set];
+        const int row = (s.wt0 + s.wts * th) * p.FW;
+        if (!FOLD) return row + s.wu0 + s.wus * tw;
+        const int fw = ps.f0[j & 1] + 2 * (ps.phase_wb[j & 1] - s.wb + tw);
+        return fw >= 0 && fw < p.FW ? row + fw : -1;
+    }
     // Pixel at a position of the line: its image and place; false where there is none.
     __device__ __forceinline__ bool pixel_of(const gather::PixelSet& s, int N, int at, int& n, int& u, int& v) const {
         uint32_t in, col;

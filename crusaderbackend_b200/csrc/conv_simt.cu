@@ -197,11 +197,12 @@ double gather_us(int sm_count, long long I, int OUTC, long long blocks, bool may
 }
 
 // One launch for up to four pixel sets. In the passes of a model the two that later layers read stay on the CUDA cores (see
-// launch_fp32_gemm), except the 3xTF32 ones that never ran there (in_models). The contraction is split over CTAs where the output alone
+// launch_fp32_gemm), except the 3xTF32 ones that never ran there. The contraction is split over CTAs where the output alone
 // does not fill the GPU and the epilogue is a plain sum (the output is then cleared first), except in the passes of a model: atomic
 // sums come in any order, and one rounding more or less in an activation moves the gradients of a deep model by percents from one run
 // to the next.
-int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, bool in_models, const char* who) {
+enum class Route { Any, TensorCores, PatchesOnly };  // by the rules below; on the tensor cores in models too; conv_patch.cu or CB_EUNSUPPORTED
+int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, Route route, const char* who) {
     const long long out_elems = (long long)p.OUTC * p.OHH * p.OWW;
     if ((long long)p.C * p.H * p.W >= (1LL << 29) || out_elems >= (1LL << 31) || (long long)p.C * p.w_ch >= (1LL << 31))
         return fail(ctx, CB_EUNSUPPORTED, std::string(who) + ": an image or filter of more than 2^29 values");
@@ -209,7 +210,7 @@ int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, 
     int most = 0;
     for (int i = 0; i < nsets; ++i) most = sets[i].K > most ? sets[i].K : most;
     const long long I = (long long)p.N * sets[0].UH * sets[0].UW * nsets;
-    const bool on_tensor_cores = (!ctx->model_pass || in_models) && split::worth_it(I, p.OUTC, most, 1, kLeastConv);
+    const bool on_tensor_cores = (!ctx->model_pass || route == Route::TensorCores) && split::worth_it(I, p.OUTC, most, 1, kLeastConv);
     if (on_tensor_cores && !ctx->model_pass && nsets <= kMaxSets) {
         std::memcpy(p.sets, sets, nsets * sizeof(PixelSet));
         PatchPlan plan{};
@@ -223,6 +224,7 @@ int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, 
             return CB_OK;
         }
     }
+    if (route == Route::PatchesOnly) return CB_EUNSUPPORTED;
     simt::Choice c{};
     split::Choice sc{};
     if (on_tensor_cores) sc = split::choose_shape(ctx->sm_count, I, p.OUTC, (most + split::kBK - 1) / split::kBK, 1, may_split, split::kGather);
@@ -262,17 +264,17 @@ int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, 
     return CB_OK;
 }
 
-int fp32_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const ConvGeo& g, const ConvEpilogue& ep, bool in_models, const char* who) {
+int fp32_conv_fwd(cb_ctx* ctx, const float* W, const float* X, float* Y, const ConvGeo& g, const ConvEpilogue& ep, Route route, const char* who) {
     GatherParams p{};
     p.In = X; p.in_batch = g.x_batch; p.C = g.IC; p.H = g.IH; p.W = g.IW;
     p.Wt = W; p.w_ch = g.FH * g.FW; p.w_out = g.IC * g.FH * g.FW; p.FW = g.FW;
     p.Out = Y; p.out_batch = g.y_batch; p.OUTC = g.OC; p.OHH = g.OH; p.OWW = g.OW;
     p.N = g.N; p.sgn = 1; p.ep = ep;
     const PixelSet s{g.OH, g.OW, g.sH, -g.pH, g.sW, -g.pW, 0, 1, 0, 1, g.FH, g.FW, 0, 1, 0, 1, g.IC * g.FH * g.FW};
-    return launch_gather(ctx, p, &s, 1, in_models, who);
+    return launch_gather(ctx, p, &s, 1, route, who);
 }
 
-int fp32_conv_dgrad(cb_ctx* ctx, const float* W, const float* dY, float* dX, const ConvGeo& g, int accumulate, bool in_models, const char* who) {
+int fp32_conv_dgrad(cb_ctx* ctx, const float* W, const float* dY, float* dX, const ConvGeo& g, int accumulate, Route route, const char* who) {
     GatherParams p{};
     p.In = dY; p.in_batch = g.y_batch; p.C = g.OC; p.H = g.OH; p.W = g.OW;
     p.Wt = W; p.w_ch = g.IC * g.FH * g.FW; p.w_out = g.FH * g.FW; p.FW = g.FW;
@@ -294,7 +296,7 @@ int fp32_conv_dgrad(cb_ctx* ctx, const float* W, const float* dY, float* dX, con
             s.K = g.OC * s.TH * s.TW;
             sets.push_back(s);
         }
-    return launch_gather(ctx, p, sets.data(), (int)sets.size(), in_models, who);
+    return launch_gather(ctx, p, sets.data(), (int)sets.size(), route, who);
 }
 
 int fp32_conv_wgrad(cb_ctx* ctx, const float* dY, const float* X, float* dW, const ConvGeo& g, int accumulate, const char* who) {
@@ -364,18 +366,21 @@ static bool tf32_width(const ConvGeo& g) {
     const int w = g.sW == 2 ? g.IW / 2 : g.IW;
     return g.FH <= 3 && g.FW <= 3 && (w == 8 || w == 16 || w == 32);
 }
-// Stride-2 3x3 layers of 3xTF32 whose forward pass and weight gradient run at fp32 accuracy: the one-pass form pays for a phase split and
-// lo parts through memory. Forward, then weight gradient, us, one pass / fp32: 32 -> 64 at 32 x 32, batch 128: 37 / 21, 34 / 24; 64 ->
-// 32, batch 118: 71 / 25, 44 / 29 (data gradient 31 / 38 and 38 / 52: stays). Below 2^27 multiplications both are a few launches, 10 to
-// 14 us against 6 to 10. 145 layers of 4 to 147 channels, 16 x 16 to 64 x 64: forward 1.0 to 3.6 times as fast, except for few input
-// channels on many pixels, where each of the gather's outputs has little to sum: 16 channels, more than 2^15 pixels, 0.70 to 1.06 (to
-// 48, 191 of 64 x 64: 61 / 86), or 1.1 to 1.6 for the 17 to 32 outputs that fill its narrowest tile; weight gradient 1.0 to 3.1, two 16
-// -> 48 layers 0.8 and 0.9.
-static bool x3_at_fp32(const ConvGeo& g, bool forward) {
+// Stride-2 3x3 layers of 3xTF32 whose passes run at fp32 accuracy: the one-pass form pays for a phase split and lo parts through memory. us,
+// one pass / fp32: 32 -> 64 at 32 x 32, batch 128: forward 37 / 17, data gradient 30.2 / 26.0, weight gradient 34 / 24. Over 53 layers of 3 to 128
+// channels, 16 x 16 to 64 x 64, 1.38, 1.76 and 1.46 times as fast with every layer of 2^22 multiplications on there; below 2^26 both are a few
+// launches. What stays in the one-pass form: few input channels on many pixels forward, where each of the gather's outputs has little to
+// sum (16 channels, more than 2^15 pixels: 0.81 to 0.97, or 1.1 to 1.6 for the 17 to 32 outputs that fill its narrowest tile); data
+// gradients of up to 16 channels (0.81 to 1.22), from many pixels (2^15 on: 0.45 to 1.09; 2^14 on from up to 16 channels to more than 32:
+// 0.98), and those that conv_patch.cu does not take.
+enum class Pass { Forward, DataGradient, WeightGradient };
+static bool x3_at_fp32(const ConvGeo& g, Pass pass) {
     if ((double)g.N * g.OH * g.OW >= (double)(1LL << 30) || (double)g.IC * g.IH * g.IW >= (double)(1LL << 28) || (double)g.OC * g.OH * g.OW >= (double)(1LL << 28))
         return false;  // 32-bit indexes
-    if (forward && g.IC <= 16 && (long long)g.N * g.OH * g.OW > (1 << 15) && (g.OC <= 16 || g.OC > 32)) return false;
-    return g.sH == 2 && g.sW == 2 && g.FH == 3 && g.FW == 3 && (double)g.N * g.OH * g.OW * g.OC * g.IC * 9.0 >= (double)(1LL << 27);
+    const long long pixels = (long long)g.N * g.OH * g.OW;
+    if (pass == Pass::Forward && g.IC <= 16 && pixels > (1 << 15) && (g.OC <= 16 || g.OC > 32)) return false;
+    if (pass == Pass::DataGradient && (g.IC <= 16 || pixels > (1 << 15) || (pixels > (1 << 14) && g.IC > 32 && g.OC <= 16))) return false;
+    return g.sH == 2 && g.sW == 2 && g.FH == 3 && g.FW == 3 && (double)pixels * g.OC * g.IC * 9.0 >= (double)(1LL << 26);
 }
 
 static int conv_fwd_impl(cb_ctx* ctx, const float* W, const float* X, float* Y, int N, int IC, int IH, int IW, int OC, int FH,
@@ -396,11 +401,11 @@ static int conv_fwd_impl(cb_ctx* ctx, const float* W, const float* X, float* Y, 
     if (npix == 0 || OC == 0) return CB_OK;
     if (!W || !X || !Y) return fail(ctx, CB_EINVAL, std::string(who) + ": null operand");
     const bool x3 = ctx->math == CB_MATH_3XTF32;
-    if (ctx->math != CB_MATH_FP32 && !(x3 && !ctx->model_pass && x3_at_fp32(g, true))) {
+    if (ctx->math != CB_MATH_FP32 && !(x3 && !ctx->model_pass && x3_at_fp32(g, Pass::Forward))) {
         rc = umma_conv_fwd(ctx, W, X, Y, ep, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, false, xb, yb, x3);
         if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;
     }
-    rc = fp32_conv_fwd(ctx, W, X, Y, g, ep, x3 && tf32_width(g), who);
+    rc = fp32_conv_fwd(ctx, W, X, Y, g, ep, x3 && tf32_width(g) ? Route::TensorCores : Route::Any, who);
     return rc == CB_OK ? finish(ctx, who) : rc;
 }
 
@@ -417,11 +422,15 @@ static int conv_dgrad_impl(cb_ctx* ctx, const float* W, const float* dY, float* 
     ConvEpilogue ep{};
     ep.accumulate = accumulate ? 1 : 0;
     const bool x3 = ctx->math == CB_MATH_3XTF32;
+    if (x3 && !ctx->model_pass && x3_at_fp32(g, Pass::DataGradient)) {
+        rc = fp32_conv_dgrad(ctx, W, dY, dX, g, accumulate ? 1 : 0, Route::PatchesOnly, who);
+        if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;
+    }
     if (ctx->math != CB_MATH_FP32) {
         rc = umma_conv_fwd(ctx, W, dY, dX, ep, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, true, dy_batch, dx_batch, x3);
         if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;
     }
-    rc = fp32_conv_dgrad(ctx, W, dY, dX, g, accumulate ? 1 : 0, x3 && tf32_width(g), who);
+    rc = fp32_conv_dgrad(ctx, W, dY, dX, g, accumulate ? 1 : 0, x3 && tf32_width(g) ? Route::TensorCores : Route::Any, who);
     return rc == CB_OK ? finish(ctx, who) : rc;
 }
 
@@ -500,7 +509,7 @@ static int conv_wgrad_impl(cb_ctx* ctx, const float* dY, const float* X, float* 
     const bool x3 = ctx->math == CB_MATH_3XTF32;
     // (models keep the kernel that leaves half the SMs to the stream beside it: a DenseNet-100 step took 3571 us with its widest layers
     // here, 3561 without; without such streams too, or a gradient's accuracy would depend on their number)
-    if (ctx->math != CB_MATH_FP32 && (ctx->deterministic || ctx->model_pass || !((x3 && x3_at_fp32(g, false)) || wgrad_at_fp32(g, x3)))) {
+    if (ctx->math != CB_MATH_FP32 && (ctx->deterministic || ctx->model_pass || !((x3 && x3_at_fp32(g, Pass::WeightGradient)) || wgrad_at_fp32(g, x3)))) {
         rc = umma_conv_wgrad(ctx, dY, X, dW, N, IC, IH, IW, OC, FH, FW, sH, sW, pH, pW, accumulate, dy_batch, x_batch, x3);
         if (rc == CB_OK && x3) ctx->last_kernel = "umma_3xtf32";
         if (rc != CB_EUNSUPPORTED) return rc == CB_OK ? finish(ctx, who) : rc;

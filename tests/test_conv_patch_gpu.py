@@ -20,7 +20,7 @@ TOL = 2e-6
 GEOS = [(32, 32, 28, 28, 32, 3, 1, 1), (9, 17, 47, 45, 33, 3, 1, 1), (20, 40, 33, 29, 70, 3, 1, 0), (64, 32, 32, 32, 64, 3, 2, 1), (24, 64, 61, 47, 31, 3, 2, 1),
         (12, 30, 40, 38, 65, 5, 1, 2), (7, 96, 54, 54, 16, 3, 2, 1), (40, 64, 40, 40, 64, 1, 1, 0), (30, 80, 42, 44, 96, 1, 2, 0), (30, 1, 56, 57, 64, 5, 1, 2),
         (30, 64, 41, 41, 1, 5, 1, 2), (6, 129, 30, 31, 48, 3, 1, 1), (16, 16, 50, 50, 16, 5, 1, 1), (25, 16, 40, 40, 40, 4, 2, 1)]
-PATCHES = set(GEOS) - {(30, 80, 42, 44, 96, 1, 2, 0), (25, 16, 40, 40, 40, 4, 2, 1)}  # the gathers' own model says less for these
+PATCHES = set(GEOS) - {(30, 80, 42, 44, 96, 1, 2, 0)}  # the gathers' own model says less for this one
 
 
 @pytest.fixture(scope="module")
@@ -181,6 +181,24 @@ def test_values_the_pieces_cannot_carry(ctx, geo, det):
     assert np.isnan(a[:, 4]).any() and not np.isfinite(a[1]).all()
     fine = np.isfinite(a)
     assert orc.max_err_norm(a[fine], b[fine]) <= 2 * TOL
+    # what does not reach a phase of a stride-2 data gradient must not reach its outputs: the same pattern by both routes
+    for grad_geo in [(64, 32, 32, 32, 64, 3, 2, 1), (24, 64, 61, 47, 31, 3, 2, 1)]:
+        gW, gX, gdY = tensors(grad_geo)
+        gdY[1, 2, 3, 4], gdY[0, 0, 0, 0], gW[5, 1, 2, 2] = float("inf"), float("nan"), float("inf")
+        ref = []
+        for stream in (None, other.cuda_stream):
+            dX = torch.empty_like(gX)
+            torch.cuda.synchronize()
+            ctx.lib.cb_set_stream(ctx.h, stream)
+            n = launches(ctx, lambda: ctx.convDerive(gW, gdY, dX, 2, 2, 1, 1))
+            assert n == (2 if stream is None else n)
+            torch.cuda.synchronize()
+            ref.append(dX.cpu().numpy())
+        ctx.lib.cb_set_stream(ctx.h, None)
+        a, b = ref
+        assert np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(np.isposinf(a), np.isposinf(b)) and np.array_equal(np.isneginf(a), np.isneginf(b))
+        fine = np.isfinite(a)
+        assert 0.5 < fine.mean() < 1 and orc.max_err_norm(a[fine], b[fine]) <= 2 * TOL
     for scale in (1e-36, 1e-30, 1e37):
         a, b = both(W, X * scale)
         y, _ = reference(W, X * scale, dY, s, p)
