@@ -107,7 +107,7 @@ enum : int {
 // when a kernel starts, a block of its predecessor has come back from the wait, so the kernel BEFORE the predecessor has completed.
 // (So no kernel may end all its blocks without this call, and none may issue launch_dependents ahead of the wait.) Ahead of the call a
 // kernel may thus read what was written at least two kernels ago on its stream, or what its stream waited for then; it must
-// not read what the kernel just before it may have written, nor write anything. bn_bwd_par_kernel reads ahead, no other.
+// not read what the kernel just before it may have written, nor write anything. bn_bwd_par_kernel and conv_patch_kernel read ahead, no other.
 __device__ __forceinline__ void griddep_wait_then_launch() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
