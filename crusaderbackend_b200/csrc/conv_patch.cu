@@ -25,7 +25,6 @@
 // 1152, in one share: 0.90, 0.98, 1.02e-7 of the norm; the gathers' 0.94, 1.02, 1.16e-7 (1.03e-7 in two shares).
 #include "conv_gather.cuh"
 #include "conv_patch.h"
-#include "simt_core.cuh"
 #include "split_core.cuh"
 
 namespace cb {
