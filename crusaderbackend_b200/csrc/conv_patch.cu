@@ -323,8 +323,11 @@ __global__ void __launch_bounds__(S::NT, S::kCtas) conv_patch_kernel(const __gri
                 const int n = min(cs.per_block, left);
                 left -= n;
                 if (turn == a) {
-                    ok = mbar_wait_uniform(smem_u32(&b.ffull[f_slot]), f_ph, abort_flag, status, CBK_TIMEOUT_FULL) &&
-                         mbar_wait_uniform(smem_u32(&b.tempty[a]), a_ph ^ 1u, abort_flag, status, CBK_TIMEOUT_TMEM_EMPTY);
+                    // In this order: a ring of three slots gives a slot's fills to the two warps in turn, and a barrier that is still in the
+                    // phase of the fill before this block's (block i - 3, the other warp's) passes a test for this one's parity. With the
+                    // accumulator free, block i - 2 has been added up, and i - 3 before it: that fill has landed, the phase is right.
+                    ok = mbar_wait_uniform(smem_u32(&b.tempty[a]), a_ph ^ 1u, abort_flag, status, CBK_TIMEOUT_TMEM_EMPTY) &&
+                         mbar_wait_uniform(smem_u32(&b.ffull[f_slot]), f_ph, abort_flag, status, CBK_TIMEOUT_FULL);
                     if (!ok) break;
                     tc_fence_after();
                     a_ph ^= 1u;
