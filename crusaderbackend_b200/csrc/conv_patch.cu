@@ -54,7 +54,7 @@ struct PatchShape {
 };
 
 struct __align__(8) PatchBarriers {
-    uint64_t pfull[kMaxRing], pempty[kMaxRing], ffull[kMaxRing], fempty[kMaxRing], tfull[2], tempty[2], ready, drain;
+    uint64_t pfull[kMaxRing], pempty[kMaxRing], ffull[kMaxRing], fempty[kMaxRing], tfull[2], tempty[2], drain;
     uint32_t tmem_base;
     int abort_flag;
     int cut;           // of the second pass: factors below split::kWhole; the largest factor's magnitude, as bits
@@ -269,10 +269,18 @@ __global__ void __launch_bounds__(S::NT, S::kCtas) conv_patch_kernel(const __gri
             mbar_init(smem_u32(&b.tempty[a]), S::kSumWarps);
         }
         mbar_init(smem_u32(&b.drain), S::kAcc);
-        mbar_init(smem_u32(&b.ready), 1);
         mbar_fence_init();
     }
+    // Ahead of every griddep_wait_then_launch: a kernel that may start after that call could take the columns that another stream's kernel
+    // gives back on this SM, and wait for this kernel's end while this kernel waits for them.
+    if (warp == S::kIssuer) {
+        tmem_alloc(smem_u32(&b.tmem_base), S::kTmemCols);
+        tmem_relinquish();
+    }
+    tc_fence_before();
     __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = b.tmem_base;
     uint32_t fills = 0;  // filter blocks asked for
 
     if (warp == S::kCopier) {
@@ -302,15 +310,9 @@ __global__ void __launch_bounds__(S::NT, S::kCtas) conv_patch_kernel(const __gri
         // its own. What one does between two blocks (barriers, commits, addresses: 500 to 1000 clocks) is then behind the other's
         // UMMAs. Descriptors come from parameters alone: one that comes from memory is not in uniform registers, at ~110 clocks a UMMA.
         const uint32_t a = (uint32_t)(warp - S::kIssuer);
-        if (a == 0) {
-            tmem_alloc(smem_u32(&b.tmem_base), S::kTmemCols);
-            tmem_relinquish();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&b.ready));
-        }
         griddep_wait_then_launch();
-        bool ok = mbar_wait_uniform(smem_u32(&b.ready), 0, abort_flag, status, CBK_TIMEOUT_TMEM_EMPTY);
-        const uint32_t d = *reinterpret_cast<volatile uint32_t*>(&b.tmem_base) + a * (3u * S::BN);
+        bool ok = true;
+        const uint32_t d = tmem_base + a * (3u * S::BN);
         uint32_t p_slot = 0, p_ph = 0, f_slot = 0, f_ph = 0, a_ph = 0, turn = 0;
         const uint32_t row_bytes = (uint32_t)(ps.planes * q.px) * 16u, piece = (uint32_t)(q.cw >> 3) * row_bytes;
         for (int chunk = it.chunk0; chunk < it.chunk1 && ok; ++chunk) {
@@ -374,8 +376,7 @@ __global__ void __launch_bounds__(S::NT, S::kCtas) conv_patch_kernel(const __gri
             if (lane == 0) mbar_arrive(smem_u32(&b.pfull[0]));
         }
         griddep_wait_then_launch();
-        bool ok = mbar_wait_uniform(smem_u32(&b.ready), 0, abort_flag, status, CBK_TIMEOUT_TMEM_EMPTY);
-        const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&b.tmem_base);
+        bool ok = true;
         const int quarter = warp & 3, first = (warp >> 2) * S::kCols, row = 32 * quarter + lane;
         const uint32_t mine = staging + (uint32_t)(first * 128 + row) * 4u, slice = staging + S::BN * 512u;
         uint32_t a = 0, a_ph = 0;
@@ -500,7 +501,7 @@ __global__ void __launch_bounds__(S::NT, S::kCtas) conv_patch_kernel(const __gri
     }
     if (warp == S::kIssuer) {
         tc_fence_after();
-        tmem_dealloc(b.tmem_base, S::kTmemCols);
+        tmem_dealloc(tmem_base, S::kTmemCols);
     }
 }
 
