@@ -36,7 +36,6 @@ namespace {
 constexpr int kMaxRing = 4;   // slots of the patch and the filter ring at most
 constexpr int kChain = 5;     // steps of 16 k whose sum stays in TMEM
 constexpr int kGroup = 8;     // blocks whose sums are added one after another
-constexpr unsigned kAbsent = 0x7fc0abe5u;  // in a slice of the second pass: a tap that a phase of the output does not have
 constexpr int kPackCols = 8;  // columns of a block of pack_patch_filter
 
 // Two CTAs an SM, so that one computes while the other starts, adds or stores. Each has 256 columns of TMEM: two accumulators of 3 x 32
@@ -206,7 +205,7 @@ __device__ __noinline__ void sum_again(const PatchParams& q, const PatchItem& it
                 int tap, c;
                 place(k0 + k, tap, c);
                 const int th = tap / s.TW, at = q.filter_of<FOLD>(it.set, th, tap - th * s.TW, j);
-                y = at < 0 ? __uint_as_float(kAbsent) : __ldg(p.Wt + (long long)(FOLD ? j >> 1 : j) * p.w_out + (long long)c * p.w_ch + at);
+                if (at >= 0) y = __ldg(p.Wt + (long long)(FOLD ? j >> 1 : j) * p.w_out + (long long)c * p.w_ch + at);
             }
             put(S::kSlice * S::BM + i, y);
         }
@@ -214,18 +213,32 @@ __device__ __noinline__ void sum_again(const PatchParams& q, const PatchItem& it
         if ((tid & 31) == 0) atomicMax(&b.largest, largest);
         asm volatile("bar.sync 3, %0;" ::"n"(kThreads) : "memory");
         if (!wanted) continue;
+        // Bit 2k + b: phase b of the output has the tap of k. 0 in place of one that it does not have would make a NaN of an infinity, and
+        // any other value may be the filter's own.
+        uint32_t has = ~0u;
+        if (FOLD) {
+            int tap = 0, c;
+            const int k = k0 + ((tid & 31) >> 1);
+            if (k < K) place(k, tap, c);
+            const int th = tap / s.TW;
+            has = __ballot_sync(0xffffffffu, k < K && q.filter_of<FOLD>(it.set, th, tap - th * s.TW, tid & 1) >= 0);
+        }
         for (int k = 0; k < S::kSlice; ++k) {
+            const bool even = (has >> (2 * k)) & 1u, odd = (has >> (2 * k + 1)) & 1u;
             const float x = split::word(slice + (uint32_t)(k * S::BM + row) * 4u);
 #pragma unroll
             for (int c = 0; c < S::kCols; c += 4) {
                 float y0, y1, y2, y3;
                 asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(y0), "=f"(y1), "=f"(y2), "=f"(y3)
                              : "r"(slice + (uint32_t)(S::kSlice * S::BM + k * S::BN + first + c) * 4u) : "memory");
-                // (0 in place of a tap that a phase does not have would make a NaN of an infinity)
-                if (!FOLD || __float_as_uint(y0) != kAbsent) plain[c] = fmaf(x, y0, plain[c]);
-                if (!FOLD || __float_as_uint(y1) != kAbsent) plain[c + 1] = fmaf(x, y1, plain[c + 1]);
-                if (!FOLD || __float_as_uint(y2) != kAbsent) plain[c + 2] = fmaf(x, y2, plain[c + 2]);
-                if (!FOLD || __float_as_uint(y3) != kAbsent) plain[c + 3] = fmaf(x, y3, plain[c + 3]);
+                if (!FOLD || even) {
+                    plain[c] = fmaf(x, y0, plain[c]);
+                    plain[c + 2] = fmaf(x, y2, plain[c + 2]);
+                }
+                if (!FOLD || odd) {
+                    plain[c + 1] = fmaf(x, y1, plain[c + 1]);
+                    plain[c + 3] = fmaf(x, y3, plain[c + 3]);
+                }
             }
         }
     }
