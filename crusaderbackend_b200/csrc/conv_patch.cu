@@ -122,7 +122,7 @@ __device__ __forceinline__ void load_patch(const PatchParams& q, const PatchItem
         if (pairs) {
 #pragma unroll
             for (int e = 0; e < 8; ++e)
-                asm("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %3, 0;\n\tmov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t@q ld.global.nc.v2.f32 {%0, %1}, [%2];\n\t}"
+                asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %3, 0;\n\tmov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t@q ld.global.nc.v2.f32 {%0, %1}, [%2];\n\t}"
                     : "=f"(l.v[0][e]), "=f"(l.v[1][e]) : "l"(split::step(src, (uint32_t)plane_in * 4u, e)), "r"((int)(e < channels)));
             l.dst[1] = here ? l.dst[0] + (uint32_t)q.px * 16u : ~0u;
         } else {

@@ -178,10 +178,11 @@ __device__ __forceinline__ const float* step(const float* base, uint32_t stride_
     return r;
 }
 
-// *src, or 0: one predicated load (a branch around each load cost more than the loads).
+// *src, or 0: one predicated load (a branch around each load cost more than the loads). Volatile: the compiler must not move it ahead of
+// griddep_wait_then_launch, up to which the kernel before may still write what it reads.
 __device__ __forceinline__ float load_if(const float* src, bool ok) {
     float v;
-    asm("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}" : "=f"(v) : "l"(src), "r"((int)ok));
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}" : "=f"(v) : "l"(src), "r"((int)ok));
     return v;
 }
 
