@@ -176,17 +176,6 @@ __global__ void bn_bwd_kernel(const float* __restrict__ dY, const float* __restr
 __device__ __forceinline__ float4 f4_add(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 __device__ __forceinline__ float4 f4_zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
 
-// sum over the 16 batch groups of the block; every thread returns the total of its position vector
-__device__ __forceinline__ float4 bn_group_sum(float4 v, float4 (*red)[16]) {
-    red[threadIdx.y][threadIdx.x] = v;
-    __syncthreads();
-    float4 t = f4_zero();
-#pragma unroll
-    for (int g = 0; g < 16; ++g) t = f4_add(t, red[g][threadIdx.x]);
-    __syncthreads();
-    return t;
-}
-
 // Sums, over the R * G batch groups of a block (R a thread), of Q float4 quantities per position vector; every thread returns
 // the totals of its position. The values go through shared memory once: thread (x, g) with g < 4 Q adds component g & 3 of
 // quantity g >> 2 over the groups in group order (a fixed order: deterministic), and everyone reads the totals back.
