@@ -859,16 +859,18 @@ __global__ void __launch_bounds__(1024) head_fwd_kernel(const float* __restrict_
     const float* Xn = X + (long long)n * C * HW;
     const int warps = blockDim.x >> 5;
     // The first class's weights, the bias and the label are on their way while the planes are read: behind the barriers below each would be a
-    // round trip to memory on its own. With sixteen warps in place of eight, a ResNet-8 step of batch 16 154.5 -> 152.7 us.
+    // round trip to memory on its own. With sixteen warps in place of eight, 16 samples of 64 channels of 8 x 8 5.7 -> 3.2 us.
     constexpr int kAhead = 4;
     float w[kAhead];
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) w[u] = warp < M && lane + 32 * u < C ? W[(long long)warp * C + lane + 32 * u] : 0.f;
     const float bias = b && warp < M ? b[warp] : 0.f, lab = warp == 0 && lane < M ? labels[(long long)n * M + lane] : 0.f;
     // pooling: a warp takes four channels at a time so that their loads are in flight together; each channel is summed
-    // lane-strided, then across the lanes
+    // lane-strided, then across the lanes. Four positions of each at a time: with those weights in registers the compiler unrolls no
+    // further by itself, and large planes came one position after the other (16 samples of 256 channels of 14 x 14 6.9 us, 11.4 so).
     for (int c0 = warp * 4; c0 < C; c0 += 4 * warps) {
         float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
         for (int i = lane; i < HW; i += 32) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
