@@ -445,10 +445,13 @@ __global__ void __launch_bounds__(T, SPT <= 4 ? 1024 / T : 1) bn_bwd_par_kernel(
     }
 }
 
-// Parameter gradients alone (seblas::batchNormParamGrads): one pass over dY and xhat, batch-parallel. A thread's samples go to memory eight at
-// a time, and the two sums of a position cross shared memory once, a component a thread: 16 channels of 32 x 32, batch 128 3.8 -> 3.2 us, behind the other kernels of a BatchNorm 5.5 -> 2.4.
-template <bool V>
-__global__ void __launch_bounds__(256) bn_paramgrad_par_kernel(const float* __restrict__ dY, const float* __restrict__ xhat,
+// Parameter gradients alone (seblas::batchNormParamGrads): one pass over dY and xhat, batch-parallel. U of a thread's samples go to memory at a
+// time, and the two sums of a position cross shared memory once, a component a thread: 16 channels of 32 x 32, batch 128 3.8 -> 3.2 us, behind
+// the other kernels of a BatchNorm 5.5 -> 2.4. Four samples leave room for four blocks on an SM, eight (98 registers) for two, which large grids wait
+// for: 291 x 65536 33 us a loop of single samples, 32 with eight, 25 with four; 200 x 28000 5.9 / 7.0 / 4.6. Positions read one by one want eight in
+// small grids (200 x 17: 4.3 / 2.8 / 3.2).
+template <bool V, int U>
+__global__ void __launch_bounds__(256, U == 4 ? 4 : 2) bn_paramgrad_par_kernel(const float* __restrict__ dY, const float* __restrict__ xhat,
                                                                float* __restrict__ dgamma, float* __restrict__ dbeta,
                                                                int N, long long P) {
     __shared__ __align__(16) float red[2][16][16 * 4];
@@ -456,7 +459,6 @@ __global__ void __launch_bounds__(256) bn_paramgrad_par_kernel(const float* __re
     const long long p = ((long long)blockIdx.x * 16 + threadIdx.x) * 4;
     float4 sg = f4_zero(), sb = f4_zero();
     if (p < P) {
-        constexpr int U = 8;
         for (int n0 = threadIdx.y; n0 < N; n0 += 16 * U) {
             float4 h[U], d[U];
 #pragma unroll
@@ -1053,8 +1055,9 @@ int cb_bn_paramgrad(cb_ctx* ctx, const float* dY, const float* xhat, float* dgam
     if (P == 0) return CB_OK;
     if (!dY || !xhat || !dgamma || !dbeta) return fail(ctx, CB_EINVAL, "cb_bn_paramgrad: null operand");
     const bool vec = (P % 4 == 0) && aligned16(xhat) && aligned16(dY) && aligned16(dgamma) && aligned16(dbeta);
-    launch_dep(ctx, vec ? bn_paramgrad_par_kernel<true> : bn_paramgrad_par_kernel<false>, dim3((unsigned)(((P + 3) / 4 + 15) / 16)), dim3(16, 16), 0,
-               dY, xhat, dgamma, dbeta, N, P);
+    const unsigned blocks = (unsigned)(((P + 3) / 4 + 15) / 16);
+    auto* kernel = vec ? bn_paramgrad_par_kernel<true, 4> : blocks > 2u * ctx->sm_count ? bn_paramgrad_par_kernel<false, 4> : bn_paramgrad_par_kernel<false, 8>;
+    launch_dep(ctx, kernel, dim3(blocks), dim3(16, 16), 0, dY, xhat, dgamma, dbeta, N, P);
     return done(ctx, "cb_bn_paramgrad");
 }
 
