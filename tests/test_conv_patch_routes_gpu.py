@@ -21,7 +21,9 @@ pytestmark = pytest.mark.gpu
 ROUTES = {(32, 32, 28, 28, 32, 3, 1, 1): (False, False), (9, 17, 47, 45, 33, 3, 1, 1): (None, False), (20, 40, 33, 29, 70, 3, 1, 0): (None, True),
           (64, 32, 32, 32, 64, 3, 2, 1): (None, False), (24, 64, 61, 47, 31, 3, 2, 1): (None, False), (12, 30, 40, 38, 65, 5, 1, 2): (False, True),
           (40, 64, 40, 40, 64, 1, 1, 0): (False, False), (30, 80, 42, 44, 96, 1, 2, 0): (None, None), (30, 64, 41, 41, 1, 5, 1, 2): (False, None),
-          (6, 129, 30, 31, 48, 3, 1, 1): (True, False)}
+          (6, 129, 30, 31, 48, 3, 1, 1): (True, False),
+          # a CTA for every SM (75 to 148 of them) and two
+          (5, 48, 40, 40, 80, 5, 2, 2): (True, True), (16, 32, 28, 28, 32, 3, 1, 1): (None, True)}
 
 
 @pytest.mark.parametrize("geo", ROUTES)
