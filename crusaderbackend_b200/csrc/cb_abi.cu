@@ -54,10 +54,6 @@ int finish(cb_ctx* ctx, const char* what) {
     return read_status(ctx, what);
 }
 
-// Growth of one of the three scratch blocks. The old block is released only after the whole device is idle (work queued
-// on a stream the context used earlier may still read it), and never while the workspace is frozen or the stream is
-// being captured: a captured graph keeps the addresses of the blocks it was recorded with, so a later free would leave
-// it reading released memory.
 // Scratch for the pieces of a convolution's filter (conv_patch.cu), or null: where it is too small, and where work that the context cannot
 // order against its own may use it too: on another stream than the one the context was created with (cb_set_stream does not wait for the old one),
 // and in a graph that is being captured (it may be replayed beside later calls).
@@ -71,6 +67,10 @@ void* filter_pieces(const cb_ctx* ctx, size_t bytes) {
     return ctx->d_status + 64;
 }
 
+// Growth of one of the three scratch blocks. The old block is released only after the whole device is idle (work queued
+// on a stream the context used earlier may still read it), and never while the workspace is frozen or the stream is
+// being captured: a captured graph keeps the addresses of the blocks it was recorded with, so a later free would leave
+// it reading released memory.
 static int grow_block(cb_ctx* ctx, void** block, size_t* have, size_t bytes, size_t ahead) {
     if (bytes <= *have) return CB_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -79,7 +79,7 @@ static int grow_block(cb_ctx* ctx, void** block, size_t* have, size_t bytes, siz
                                     "before the capture so that the scratch is already large enough");
     if (ctx->workspace_frozen)
         return fail(ctx, CB_ENOMEM, "workspace is frozen (cb_freeze_workspace) and this call needs a larger scratch block");
-    cudaError_t e = cudaDeviceSynchronize();
+    cudaError_t e = *block || block == &ctx->wgrad_acc ? cudaDeviceSynchronize() : cudaSuccess;  // (that one is cleared on the legacy stream)
     if (e != cudaSuccess) return check_cuda(ctx, e, "workspace growth sync");
     if (*block) cudaFree(*block);
     *block = nullptr;
@@ -245,7 +245,7 @@ int cb_create(cb_ctx** out, int device, void* cuda_stream) {
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0) return CB_ECUDA;
     if (device < 0 || device >= ndev) return CB_EINVAL;
     if (cudaSetDevice(device) != cudaSuccess) return CB_ECUDA;
-    // three attributes: all the properties together take 2.5 ms, most of what a context costs
+    // four attributes: all the properties together take 2.5 ms, most of what a context costs
     int major = 0, minor = 0, sms = 0, smem = 0;
     if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
         cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device) != cudaSuccess ||

@@ -214,8 +214,14 @@ int launch_gather(cb_ctx* ctx, GatherParams p, const PixelSet* sets, int nsets, 
     if (on_tensor_cores && !ctx->model_pass && nsets <= kMaxSets) {
         std::memcpy(p.sets, sets, nsets * sizeof(PixelSet));
         PatchPlan plan{};
-        void* pieces = plan_patch(ctx, p, nsets, may_split, plan) && plan.us < 0.88 * gather_us(ctx->sm_count, I, p.OUTC, (most + split::kBK - 1) / split::kBK, may_split, p, sets)
-                           ? filter_pieces(ctx, plan.filter_bytes) : nullptr;
+        void* pieces = nullptr;
+        if (plan_patch(ctx, p, nsets, may_split, plan) && plan.us < 0.88 * gather_us(ctx->sm_count, I, p.OUTC, (most + split::kBK - 1) / split::kBK, may_split, p, sets)) {
+            // In place of the one-pass form pieces lie in the workspace, where that would pack its filter: on every stream, and in a capture whose
+            // call was made before. (Elsewhere than on the context's own stream it would go to that form, whose blocks no call has grown.) The
+            // gathers need no scratch, so what could go there must not depend on the workspace.
+            if (route != Route::PatchesOnly) pieces = filter_pieces(ctx, plan.filter_bytes);
+            else if (plan.filter_bytes <= kFilterPieces && ensure_workspace(ctx, plan.filter_bytes) == CB_OK) pieces = ctx->workspace;
+        }
         if (pieces) {
             const cudaError_t e = launch_patch(ctx, plan, pieces);
             if (e != cudaSuccess) return check_cuda(ctx, e, who);
