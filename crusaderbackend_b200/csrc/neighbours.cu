@@ -447,9 +447,9 @@ __global__ void __launch_bounds__(T, SPT <= 4 ? 1024 / T : 1) bn_bwd_par_kernel(
 
 // Parameter gradients alone (seblas::batchNormParamGrads): one pass over dY and xhat, batch-parallel. U of a thread's samples go to memory at a
 // time, and the two sums of a position cross shared memory once, a component a thread: 16 channels of 32 x 32, batch 128 3.8 -> 3.2 us, behind
-// the other kernels of a BatchNorm 5.5 -> 2.4. Four samples leave room for four blocks on an SM, eight (98 registers) for two, which large grids wait
-// for: 291 x 65536 33 us a loop of single samples, 32 with eight, 25 with four; 200 x 28000 5.9 / 7.0 / 4.6. Positions read one by one want eight in
-// small grids (200 x 17: 4.3 / 2.8 / 3.2).
+// the other kernels of a BatchNorm 5.5 -> 2.4. Four samples leave room for four blocks on an SM, eight (98 registers) for two, which larger grids wait
+// for: 291 x 65536 33 us a loop of single samples, 32 with eight, 25 with four; 200 x 28000 5.9 / 7.0 / 4.6. Grids of up to two blocks an SM have
+// eight: 200 x 17 4.3 / 2.8 / 3.2, and behind the other kernels 75 samples of 16 channels of 26 x 26 are 0.5 us ahead of four.
 template <bool V, int U>
 __global__ void __launch_bounds__(256, U == 4 ? 4 : 2) bn_paramgrad_par_kernel(const float* __restrict__ dY, const float* __restrict__ xhat,
                                                                float* __restrict__ dgamma, float* __restrict__ dbeta,
@@ -1056,7 +1056,8 @@ int cb_bn_paramgrad(cb_ctx* ctx, const float* dY, const float* xhat, float* dgam
     if (!dY || !xhat || !dgamma || !dbeta) return fail(ctx, CB_EINVAL, "cb_bn_paramgrad: null operand");
     const bool vec = (P % 4 == 0) && aligned16(xhat) && aligned16(dY) && aligned16(dgamma) && aligned16(dbeta);
     const unsigned blocks = (unsigned)(((P + 3) / 4 + 15) / 16);
-    auto* kernel = vec ? bn_paramgrad_par_kernel<true, 4> : blocks > 2u * ctx->sm_count ? bn_paramgrad_par_kernel<false, 4> : bn_paramgrad_par_kernel<false, 8>;
+    auto* kernel = blocks > 2u * ctx->sm_count ? (vec ? bn_paramgrad_par_kernel<true, 4> : bn_paramgrad_par_kernel<false, 4>)
+                                               : (vec ? bn_paramgrad_par_kernel<true, 8> : bn_paramgrad_par_kernel<false, 8>);
     launch_dep(ctx, kernel, dim3(blocks), dim3(16, 16), 0, dY, xhat, dgamma, dbeta, N, P);
     return done(ctx, "cb_bn_paramgrad");
 }
