@@ -609,24 +609,24 @@ bool fit(const cb_ctx* ctx, const GatherParams& p, int nsets, PatchPlan& plan) {
                         if (bytes < (long long)S::kStaging) bytes = S::kStaging;
                         bytes += 128;
                         if (bytes > (ctas == 2 ? half : whole)) continue;
-                            q.cw = cw; q.pslots = pslots; q.fslots = fslots; q.chunks = chunks;
-                            plan.smem = (size_t)bytes;
+                        q.cw = cw; q.pslots = pslots; q.fslots = fslots; q.chunks = chunks;
+                        plan.smem = (size_t)bytes;
                         plan.ctas_sm = ctas;
-                            for (int i = 0; i < nsets; ++i) {
-                                q.sets[i].taps = p.sets[i].TH * p.sets[i].TW;
-                                q.sets[i].steps = (p.C + 15) / 16 * q.sets[i].taps;
-                                for (int end = 0; end < 2; ++end) {
-                                    ChunkSteps& cs = end ? q.sets[i].last : q.sets[i].full;
-                                    cs.channels16 = end ? (p.C - (chunks - 1) * cw + 15) / 16 : cw / 16;
-                                    cs.steps = cs.channels16 * q.sets[i].taps;
-                                    cs.blocks = (cs.steps + block - 1) / block;
-                                    cs.per_block = cs.blocks ? (cs.steps + cs.blocks - 1) / cs.blocks : 0;
-                                    if (cs.per_block) cs.blocks = (cs.steps + cs.per_block - 1) / cs.per_block;
-                                }
+                        for (int i = 0; i < nsets; ++i) {
+                            q.sets[i].taps = p.sets[i].TH * p.sets[i].TW;
+                            q.sets[i].steps = (p.C + 15) / 16 * q.sets[i].taps;
+                            for (int end = 0; end < 2; ++end) {
+                                ChunkSteps& cs = end ? q.sets[i].last : q.sets[i].full;
+                                cs.channels16 = end ? (p.C - (chunks - 1) * cw + 15) / 16 : cw / 16;
+                                cs.steps = cs.channels16 * q.sets[i].taps;
+                                cs.blocks = (cs.steps + block - 1) / block;
+                                cs.per_block = cs.blocks ? (cs.steps + cs.blocks - 1) / cs.blocks : 0;
+                                if (cs.per_block) cs.blocks = (cs.steps + cs.per_block - 1) / cs.per_block;
                             }
-                            return true;
                         }
+                        return true;
                     }
+                }
     }
     return false;
 }

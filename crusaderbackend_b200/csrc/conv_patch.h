@@ -6,7 +6,7 @@ namespace cb {
 
 constexpr int kPatchTaps = 32;  // taps of a filter at most
 
-// A chunk of channels as every role of the kernel walks it: steps (16 channels, one tap each; taps fastest) in blocks of at most four.
+// A chunk of channels as every role of the kernel walks it: steps (16 channels, one tap each; taps fastest) in blocks of at most kChain.
 struct ChunkSteps {
     int channels16, steps, blocks, per_block;
     __device__ __forceinline__ int in_block(int b) const { return min(per_block, steps - b * per_block); }

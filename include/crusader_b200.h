@@ -50,6 +50,11 @@ enum {
  * stream every reference seblas kernel is launched on). */
 int cb_create(cb_ctx** out, int device, void* cuda_stream);
 int cb_destroy(cb_ctx* ctx);
+/* Later calls go to `cuda_stream`; the context does not wait for what it has queued on the former one. Convolutions that run at
+ * fp32 accuracy (CB_MATH_FP32, and layers of the other modes whose shape calls for it) keep the pieces of their filters in scratch
+ * that belongs to the stream the context was created with. On any other stream, and while a stream is being captured, such a
+ * call runs a kernel that needs none: the same error bounds, other last bits and another time (stride-2 data gradients of
+ * CB_MATH_3XTF32 use the workspace instead and are the same everywhere). */
 int cb_set_stream(cb_ctx* ctx, void* cuda_stream);
 int cb_set_math(cb_ctx* ctx, int mode);
 int cb_get_math(const cb_ctx* ctx);
@@ -60,7 +65,8 @@ int cb_set_sync(cb_ctx* ctx, int sync_every_call);
  * freeze the workspace after the warm-up calls and before (or right after) the capture, and keep it frozen for as long
  * as the graph is replayed. Growth is also refused while the context's stream is being captured. */
 int cb_freeze_workspace(cb_ctx* ctx, int on);
-/* 1: never split a reduction across CTAs with atomics (bit-reproducible results). Default 0. */
+/* 1: never split a reduction across CTAs with atomics (bit-reproducible results: the same call gives the same bits every time on
+ * the context's own stream, and every time on other streams or in captures; cb_set_stream says where the two differ). Default 0. */
 int cb_set_deterministic(cb_ctx* ctx, int on);
 /* Waits for the stream, then reads and clears the device status word. CB_OK or CB_ETIMEOUT/CB_ECUDA. */
 int cb_synchronize(cb_ctx* ctx);
