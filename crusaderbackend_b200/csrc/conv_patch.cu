@@ -16,9 +16,9 @@
 // Roles: patch warps (global memory -> registers -> pieces), one or two issuing warps, one that copies the filter's pieces, which
 // pack_patch_filter has made before, and summing warps, which help with the first patch.
 //
-// us, conv_split.cu's gather / here: 32 -> 32 3x3, 28 x 28, batch 32, forward 14.4 / 10.6, data gradient 17.3 / 10.4; 32 -> 64 3x3 stride 2, 32 x
-// 32, batch 128 20.9 / 17.5, its data gradient 36.3 / 24.9; 128 -> 128 3x3, 4 maps of 56 x 56 37.7 / 30.8 and 64.1 / 30.8; 16 -> 32 5x5, 46 x 46, batch 23 28.5 / 18.6 and
-// 60.7 / 25.9. What bounds it now: in the first of these 3.2 us are pack_patch_filter's, 2.6 a CTA's start until its first patch is there; then
+// us, conv_split.cu's gather / here: 32 -> 32 3x3, 28 x 28, batch 32, forward 14.6 / 10.9, data gradient 17.6 / 10.9; 32 -> 64 3x3 stride 2, 32 x
+// 32, batch 128 21.1 / 18.2, its data gradient 37.2 / 25.7; 128 -> 128 3x3, 4 maps of 56 x 56 37.7 / 32.4 and 65.6 / 32.6; 16 -> 32 5x5, 46 x 46,
+// batch 23 29.0 / 19.0 and 61.2 / 26.0. What bounds it now: in the first of these 3.2 us are pack_patch_filter's, 2.6 a CTA's start until its first patch is there; then
 // UMMAs, 60 clocks each whatever their width, and between blocks of them the hand-over of accumulators (a second issuing warp, a
 // second CTA on the SM). One CTA an SM that walks over tiles, fetching ahead, took 12.7 us there: what a patch warp executes for a run of
 // 32 positions x 8 channels, ~150 instructions a chain of 1500 clocks, was then the bound. Error against fp64 at K = 288, 576,
@@ -39,7 +39,8 @@ constexpr int kGroup = 8;     // blocks whose sums are added one after another
 constexpr int kPackCols = 8;  // columns of a block of pack_patch_filter
 
 // Two CTAs an SM, so that one computes while the other starts, adds or stores. Each has 256 columns of TMEM: two accumulators of 3 x 32
-// columns, each with an issuing warp of its own, or one of 3 x 64.
+// columns, each with an issuing warp of its own, or one of 3 x 64. Twice 512 threads leave 64 registers a thread: 4 to 60 bytes of
+// spill stores (ptxas), the price of the second CTA.
 template <int BN_>
 struct PatchShape {
     static constexpr int BM = 128, BN = BN_, NT = 512, kCtas = 2;
@@ -642,7 +643,7 @@ bool plan_patch(const cb_ctx* ctx, const GatherParams& given, int nsets, bool ma
     GatherParams& p = q.p;
     // The four sets of a stride-2 data gradient as two, of even and odd rows, whose column phases lie side by side in the product: the patch of
     // a distance serves both, and pairs of columns leave together. 32 -> 64 at 32 x 32, batch 128: 34.5 us as
-    // four sets, 26.0.
+    // four sets, 25.7.
     q.fold = nsets == 4 && p.sgn < 0 && p.sets[0].ohs == 2 && p.sets[0].ows == 2 ? 1 : 0;
     if (q.fold) {
         for (int a = 0; a < 2; ++a) {

@@ -182,10 +182,10 @@ __global__ void __launch_bounds__(T::NT, T::kMinCtas) conv_wgrad_simt(const Wgra
 constexpr long long kLeastConv = 1LL << 22;
 
 // us a launch of conv_gather_split takes, by a model fitted to 555 passes (7.5 % off on average). conv_patch.cu is taken where its own model
-// is 12 % below: over these passes 1.14 times as fast as without it (1.16 with the faster of the two each time), 2 % of them slower, by
-// 10 % on average. us without / with: forward 32 -> 32 at 28 x 28, batch 32 14.4 / 10.6, its data gradient 17.3 / 10.4; 32 -> 64 at 32 x 32,
-// stride 2, batch 128 20.9 / 16.9; 16 -> 32 5x5 at 46 x 46, batch 23 28.5 / 18.6 and 60.7 / 25.9; few channels at stride 2 stay: 5 -> 38 at
-// 32 x 32, batch 18 4.8 / 6.8.
+// is 12 % below: 6400 passes of drawn layers that go there are 1.43 times as fast as without it, 3 % of them slower by more than 4 %, by 12 % on
+// average and 1.41 to 1.56 times at most (5x5 filters, grids of just under two CTAs an SM). us without / with: forward 32 -> 32 at 28 x 28, batch
+// 32 14.6 / 10.9, its data gradient 17.6 / 10.9; 32 -> 64 at 32 x 32, stride 2, batch 128 21.1 / 18.2; 16 -> 32 5x5 at 46 x 46, batch 23 29.0 /
+// 19.0 and 61.2 / 26.0; few channels at stride 2 stay: 5 -> 38 at 32 x 32, batch 18 4.8 / 6.8.
 double gather_us(int sm_count, long long I, int OUTC, long long blocks, bool may_split, const GatherParams& p, const PixelSet* sets) {
     const split::Choice c = split::choose_shape(sm_count, I, OUTC, blocks, 1, may_split, split::kGather);
     const long long ctas = (I + 127) / 128 * ((OUTC + c.bn - 1) / c.bn) * c.splits;
@@ -373,7 +373,7 @@ static bool tf32_width(const ConvGeo& g) {
     return g.FH <= 3 && g.FW <= 3 && (w == 8 || w == 16 || w == 32);
 }
 // Stride-2 3x3 layers of 3xTF32 whose passes run at fp32 accuracy: the one-pass form pays for a phase split and lo parts through memory. us,
-// one pass / fp32: 32 -> 64 at 32 x 32, batch 128: forward 37 / 17, data gradient 30.2 / 26.0, weight gradient 34 / 24. Over 53 layers of 3 to 128
+// one pass / fp32: 32 -> 64 at 32 x 32, batch 128: forward 37 / 18, data gradient 30.2 / 25.8, weight gradient 34 / 26. Over 53 layers of 3 to 128
 // channels, 16 x 16 to 64 x 64, 1.38, 1.76 and 1.46 times as fast with every layer of 2^22 multiplications on there; below 2^26 both are a few
 // launches. What stays in the one-pass form: few input channels on many pixels forward, where each of the gather's outputs has little to
 // sum (16 channels, more than 2^15 pixels: 0.81 to 0.97, or 1.1 to 1.6 for the 17 to 32 outputs that fill its narrowest tile); data
